@@ -162,11 +162,19 @@ def ensure_qmap(device):
     _QMAP_DEVICES.add(device)
 
 
+# Pinned buffers of rings that were dropped while a copy out of them was still queued, each with
+# the event behind that copy.  The library's copies are unknown to torch's pinned-memory cache,
+# which would hand a freed block to the next ring at once: the queued copy would then read the
+# new ring's table.  Entries whose event has passed are let go when the next ring is made.
+_RETIRED = []
+
+
 class _PinnedRing:
     """A small ring of pinned host buffers.  A buffer is reused only after the
-    copy that read it has completed on the device."""
+    copy that read it has completed on the device, also when the ring itself is gone."""
 
     def __init__(self, nbytes, depth=3):
+        _RETIRED[:] = [x for x in _RETIRED if not x[1].query()]
         self.bufs = [torch.empty(max(nbytes, 16), dtype=torch.uint8, pin_memory=True) for _ in range(depth)]
         self.events = [None] * depth
         self.i = 0
@@ -184,6 +192,12 @@ class _PinnedRing:
             ev = torch.cuda.Event()
             self.events[self.i] = ev
         ev.record(stream)
+
+    def __del__(self, retired=_RETIRED):
+        try:
+            retired.extend(x for x in zip(self.bufs, self.events) if x[1] is not None and not x[1].query())
+        except Exception:      # (a ring that was never built, or a context that is gone)
+            pass
 
 
 class FullrankKey(tuple):

@@ -773,7 +773,10 @@ class Adafactor8Bit(Optimizer):
                 if self._cfg_seen.get(id(p)) != sig:     # first step after a load, or an option was edited
                     state = self._sync_state(p, g, group, state)
                     self._cfg_seen[id(p)] = sig
-                    self._plans.clear()                  # launch plans cache state pointers and formats
+                    # the group's launch plans cache state pointers and formats (other groups' plans, whose
+                    # launches of this step may be queued already, stay)
+                    for k in [k for k in self._plans if k[0] == gi]:
+                        del self._plans[k]
             states[j] = state
             if group.get("stochastic_round_writeback", False) and p.dtype in (torch.bfloat16, torch.float16):
                 self._sr_seed(state, p)     # seeds follow the parameter order of the step (optimizer.py:1889-1892)

@@ -229,6 +229,7 @@ apollo_project_umma_kernel(const UmmaTask *__restrict__ tasks, int n_tasks, int 
     // consumer of use n waits for phase parity n & 1, the producer of use n >= 1 for (n-1) & 1.
     int fills = 0, gchunk = 0;
     int issued = 0;                 // producer only: stage fills issued so far
+    int mapped = -1;                // producer only: task whose tensor maps it has acquired
 
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
         if (volatile_load(&s_abort)) break;
@@ -365,6 +366,11 @@ apollo_project_umma_kernel(const UmmaTask *__restrict__ tasks, int n_tasks, int 
         } else if (warp == UM_TMA_WARP && lane == 0) {
             // ---------------- copies ----------------
             const uint32_t bytes = (uint32_t)(UM_A_BYTES + 3 * plane_bytes);
+            if (lo != mapped) {
+                tensormap_acquire(&U->map_a);
+                tensormap_acquire(&U->map_b);
+                mapped = lo;
+            }
             for (int ks = 0; ks < ksteps; ++ks) {
                 const int f = fills + ks, slot = f % UM_STAGES, use = f / UM_STAGES;
                 if (use >= 1 && !mbar_wait_bounded(&s_empty[slot], (uint32_t)(use - 1) & 1u)) { failed = true; break; }

@@ -1028,6 +1028,7 @@ factored_stats_vec_kernel(const FactoredLaunch L, const int use_ring, const CUte
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int cur_t = -1;
     uint32_t cons = 0;                           // row slices this warp has taken from its ring
+    [[maybe_unused]] int mapped = -1;            // tensor whose maps this warp's lane 0 has acquired
     if (use_ring) {
         if (lane == 0) {
             for (int k = 0; k < sring_stages<GradT>(); ++k) mbar_init(&s_full[warp][k], 1);
@@ -1082,6 +1083,7 @@ factored_stats_vec_kernel(const FactoredLaunch L, const int use_ring, const CUte
                 if (use_ring == 2) {                                             // boxes of rows through tensor maps
                     boxes = true;
                     const CUtensorMap *mp = maps + 2 * t;
+                    if (lane == 0 && t != mapped) { tensormap_acquire(mp); tensormap_acquire(mp + 1); mapped = t; }
                     if (one) ok = small ? residual_rows_box<true, true>(L, sT, mp, r0, c0, pre_div, ic, cacc, ring, s_full[warp], cons)
                                         : residual_rows_box<true, false>(L, sT, mp, r0, c0, pre_div, ic, cacc, ring, s_full[warp], cons);
                     else ok = small ? residual_rows_box<false, true>(L, sT, mp, r0, c0, pre_div, ic, cacc, ring, s_full[warp], cons)

@@ -26,6 +26,13 @@ inline EncodeTiledFn encode_tiled_fn()
     return fn;
 }
 
+// Orders the uses of a tensor map by the calling thread behind the host's copy that wrote it: a map that lives in
+// global memory is read through a proxy of its own, which may still hold what was at that address before.
+__device__ __forceinline__ void tensormap_acquire(const CUtensorMap *map)
+{
+    asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
+}
+
 // global -> shared, completion as transaction bytes on `bar`
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar)
 {
