@@ -155,13 +155,13 @@ inline int persistent_grid(K kernel, int threads, size_t smem, int64_t total_blo
     return AF8_OK;
 }
 
-template <typename GradT, typename ParamT, int MODE>
+template <typename GradT, typename ParamT, int VB, int MF, bool SR, bool LAG>
 inline int launch_fast(const FullrankLaunch &L, cudaStream_t st)
 {
-    using Ring = FastRing<GradT, ParamT, MODE>;
-    auto kernel = fullrank_fast_kernel<GradT, ParamT, MODE>;
-    // the ring lives in dynamic shared memory (up to 48-60 KB per CTA): opt in and ask for
-    // the large shared-memory carve-out
+    using Ring = FastRing<GradT, ParamT, VB, MF>;
+    auto kernel = fullrank_fast_kernel<GradT, ParamT, VB, MF, SR, LAG>;
+    // the ring lives in dynamic shared memory (up to 44 KB per CTA): opt in and ask for the large
+    // shared-memory carve-out
     AF8_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring::SMEM_BYTES));
     AF8_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                       (int)cudaSharedmemCarveoutMaxShared));
@@ -173,10 +173,10 @@ inline int launch_fast(const FullrankLaunch &L, cudaStream_t st)
     return AF8_OK;
 }
 
-template <typename GradT>
+template <typename GradT, int VB, int MF>
 inline int launch_stat(const FullrankLaunch &L, cudaStream_t st)
 {
-    auto kernel = fullrank_stat_kernel<GradT>;
+    auto kernel = fullrank_stat_kernel<GradT, VB, MF>;
     int per_sm = 0;
     AF8_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, STAT_THREADS, 0));
     if (per_sm < 1) return fail(AF8_ERR_CUDA, "statistic kernel does not fit on an SM");
@@ -217,16 +217,52 @@ inline int dispatch_generic(int mode, const FullrankLaunch &L, const GenericCfg 
     }
 }
 
-// the specialised kernels (AdamW UF8/AL8 layout): statistic pass, or the update pass for ParamT
-template <typename GradT, typename ParamT>
-inline int dispatch_fast(int mode, const FullrankLaunch &L, cudaStream_t st)
+// The specialised kernels cover the Adam denominator with AL8 or AL16 second moments in blocks of 2048 and
+// UF8 / UF4 momentum in blocks of 256 or none, for fp32 parameters with fp32 or bf16 gradients and for bf16
+// parameters with bf16 gradients: the formats that large tensors are trained with.  What is left to the
+// general kernel are the formats with a codebook (d8, d4), fp16, other block sizes and the small
+// binary32-state tensors.  The lag mode exists for UF8 / AL8.
+inline bool fast_covers(const af8_fullrank_cfg &c)
 {
-    switch (mode) {
-    case AF8_MODE_NOCLIP: return launch_fast<GradT, ParamT, AF8_MODE_NOCLIP>(L, st);
-    case AF8_MODE_SUMSQ: return launch_stat<GradT>(L, st);
-    case AF8_MODE_LAG: return launch_fast<GradT, ParamT, AF8_MODE_LAG>(L, st);
-    default: return launch_fast<GradT, ParamT, AF8_MODE_APPLY>(L, st);
+    if (!c.use_adam_denom || c.momentum_only || c.block != FAST_VBLOCK || c.mode == AF8_MODE_SUMSQ_M) return false;
+    if (c.v_fmt != AF8_V_AL8 && c.v_fmt != AF8_V_AL16) return false;
+    if (c.m_fmt != AF8_M_NONE && (c.m_block != FAST_MBLOCK || (c.m_fmt != AF8_M_UF8 && c.m_fmt != AF8_M_UF4))) return false;
+    if (c.mode == AF8_MODE_LAG && !(c.v_fmt == AF8_V_AL8 && c.m_fmt == AF8_M_UF8)) return false;
+    return (c.param_dtype == AF8_F32 && (c.grad_dtype == AF8_F32 || c.grad_dtype == AF8_BF16)) ||
+           (c.param_dtype == AF8_BF16 && c.grad_dtype == AF8_BF16);
+}
+
+template <typename GradT, typename ParamT, bool SR, int VB, int MF>
+inline int dispatch_fast_mode(int mode, FullrankLaunch L, cudaStream_t st)
+{
+    if (mode == AF8_MODE_SUMSQ) return launch_stat<GradT, VB, MF>(L, st);
+    if constexpr (VB == 8 && MF == AF8_M_UF8) {
+        if (mode == AF8_MODE_LAG) return launch_fast<GradT, ParamT, VB, MF, SR, true>(L, st);
     }
+    if (mode == AF8_MODE_NOCLIP) L.dyn = nullptr;        // the step size is the table's
+    return launch_fast<GradT, ParamT, VB, MF, SR, false>(L, st);
+}
+
+template <typename GradT, typename ParamT, bool SR>
+inline int dispatch_fast_formats(const af8_fullrank_cfg &c, const FullrankLaunch &L, cudaStream_t st)
+{
+    if (c.v_fmt == AF8_V_AL8) {
+        if (c.m_fmt == AF8_M_UF8) return dispatch_fast_mode<GradT, ParamT, SR, 8, AF8_M_UF8>(c.mode, L, st);
+        if (c.m_fmt == AF8_M_UF4) return dispatch_fast_mode<GradT, ParamT, SR, 8, AF8_M_UF4>(c.mode, L, st);
+        return dispatch_fast_mode<GradT, ParamT, SR, 8, AF8_M_NONE>(c.mode, L, st);
+    }
+    if (c.m_fmt == AF8_M_UF8) return dispatch_fast_mode<GradT, ParamT, SR, 16, AF8_M_UF8>(c.mode, L, st);
+    if (c.m_fmt == AF8_M_UF4) return dispatch_fast_mode<GradT, ParamT, SR, 16, AF8_M_UF4>(c.mode, L, st);
+    return dispatch_fast_mode<GradT, ParamT, SR, 16, AF8_M_NONE>(c.mode, L, st);
+}
+
+// c must satisfy fast_covers
+inline int dispatch_fast(const af8_fullrank_cfg &c, const FullrankLaunch &L, cudaStream_t st)
+{
+    if (c.param_dtype == AF8_BF16)
+        return c.stochastic_round ? dispatch_fast_formats<bf16_tag, bf16_tag, true>(c, L, st) : dispatch_fast_formats<bf16_tag, bf16_tag, false>(c, L, st);
+    if (c.grad_dtype == AF8_BF16) return dispatch_fast_formats<bf16_tag, float, false>(c, L, st);
+    return dispatch_fast_formats<float, float, false>(c, L, st);
 }
 
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -312,13 +348,7 @@ extern "C" int af8_fullrank_step(const af8_fullrank_cfg *cfg, const af8_fullrank
     L.sr = c.stochastic_round ? 1 : 0;
     GenericCfg C{c.v_fmt, c.m_fmt, c.block, c.m_block, c.use_adam_denom ? 1 : 0, c.momentum_only ? 1 : 0};
 
-    const bool fast = c.v_fmt == AF8_V_AL8 && c.m_fmt == AF8_M_UF8 && c.block == FAST_VBLOCK &&
-                      c.m_block == FAST_MBLOCK && c.use_adam_denom && !c.momentum_only &&
-                      c.mode != AF8_MODE_SUMSQ_M;
-    // specialised kernels: fp32 parameters with fp32 / bf16 gradients, bf16 parameters with bf16 gradients
-    if (fast && c.param_dtype == AF8_F32 && c.grad_dtype == AF8_BF16) return dispatch_fast<bf16_tag, float>(c.mode, L, st);
-    if (fast && c.param_dtype == AF8_F32 && c.grad_dtype == AF8_F32) return dispatch_fast<float, float>(c.mode, L, st);
-    if (fast && c.param_dtype == AF8_BF16 && c.grad_dtype == AF8_BF16) return dispatch_fast<bf16_tag, bf16_tag>(c.mode, L, st);
+    if (fast_covers(c)) return dispatch_fast(c, L, st);
     if (c.grad_dtype == AF8_BF16) return dispatch_generic<bf16_tag>(c.mode, L, C, st);
     if (c.grad_dtype == AF8_F16) return dispatch_generic<f16_tag>(c.mode, L, C, st);
     return dispatch_generic<float>(c.mode, L, C, st);

@@ -1,52 +1,62 @@
-// Full-rank fused step, specialised kernel: AdamW-style update with UF8
-// momentum (M block 256) and AL8 second moment (V block 2048), fp32
-// parameters with fp32 or bf16 gradients, or bf16 parameters (rounded to
-// nearest or stochastically) with bf16 gradients.
+// Full-rank fused step, specialised kernel: AdamW- / RMSprop-style update (Adam denominator) with an
+// AL8 or AL16 second moment (V block 2048) and a UF8 or UF4 momentum (M block 256) or none, fp32
+// parameters with fp32 or bf16 gradients, or bf16 parameters (rounded to nearest or stochastically)
+// with bf16 gradients.
 //
 // Reference semantics: _update_param_8bit full-rank branch with the Adam
 // denominator (optimizer.py:2115-2123), _fallback_1d_update
 // (optimizer.py:903-910), _m_ema_pytorch (optimizer.py:690-700), the AL codec
-// (optimizer.py:299-353) and the UF8 codec (optimizer.py:504-532).
+// (optimizer.py:299-353) and the uniform codecs (optimizer.py:504-532).
 //
 // Work decomposition.  The launch covers a table of tensors; the unit of work
 // is one V block (2048 consecutive elements of one tensor).  A persistent grid
-// walks the flat block space with a grid stride.  One CTA of 256 threads owns a
-// block; warp w owns elements [256w, 256w+256), i.e. exactly M block w, so the
-// momentum absmax is a pure warp reduction.  Lane l of the warp owns the two
-// 4-element groups at 256w+4l and 256w+128+4l: every shared-memory read and
-// every global store of a warp is one contiguous 128/256/512-byte run.
+// walks the flat block space with a grid stride.  One CTA of 128 threads owns a
+// block; warp w owns elements [512w, 512w+512), i.e. two M blocks, so a
+// momentum absmax is a pure warp reduction.  Lane l owns the 4-element groups at
+// 512w+4l, +128, +256 and +384: every shared-memory read and every global store
+// of a warp is one contiguous run.  Sixteen elements per thread halve what a
+// block costs besides its elements against eight (256 threads): 69 -> 54
+// instructions per parameter, and a block-wide barrier joins four warps instead
+// of eight.
 //
-// Data movement.  The parameter, gradient and both code arrays of a full block
+// Data movement.  The parameter, gradient and code arrays of a full block
 // are brought into a two-stage shared-memory ring by bulk asynchronous copies
 // (cp.async.bulk, completion on an mbarrier).  While block i is being processed
 // the copies of block i+1 of the same tensor are already in flight, and the
 // 256-entry AL8 decode table of block i+1 is computed while warp 0 derives the
-// range of block i.  Tail blocks (fewer than 2048 real elements) and the first
-// block a CTA touches in a tensor take a plain-load path.  Every wait on an
+// range of block i.  A tail block (fewer than 2048 real elements) is copied into
+// its slot by the threads.  Every wait on an
 // mbarrier is bounded; a wait that runs out raises the device error flag that
 // af8_device_status() reports, the threads skip the stores of that block and
 // the CTA stops at its next block-wide barrier.
 //
-// Instruction count.  At 14-16 bytes per parameter the HBM roofline leaves
-// roughly 60 issue slots per parameter, so exact IEEE arithmetic is spent only
-// where it decides a stored bit:
+// What bounds it: instruction issue and the latency between dependent
+// instructions (57 % of the issue slots at 24 warps per SM; DRAM 63 % busy), so
+// the hot loop is kept small (about 14 KB of code): what is rare - tail blocks, uncommon
+// scalars, codes in doubt - is rolled up or handled by a compact general branch.  Inlined
+// between the parts of the loop those copies had put instruction fetches at the top of the
+// stall list.  Exact IEEE arithmetic is spent only where it decides a stored bit:
 //   * the EMAs, the dequantisation and both requantisations are bit-exact
 //     restatements of the torch ops;
 //   * the block extrema are reduced on v itself (log2 is monotone) and the
 //     exactly rounded log2 is taken of the two extreme values only;
-//   * a second-moment code is first computed from the hardware log2
+//   * an AL8 code is first computed from the hardware log2
 //     approximation; only when that estimate lies closer to a rounding
 //     boundary than its own error bound is the exact sequence (binary64 log2,
 //     IEEE division) evaluated, so the stored code is always the exact one;
+//     AL16 codes, 257 times finer, are always computed exactly;
 //   * the momentum division m/absmax uses the correctly rounded reciprocal of
 //     the block's absmax with one residual correction, which yields the IEEE
 //     quotient;
 //   * the parameter update u = m / (sqrt(v) + eps) feeds nothing but the fp32
 //     parameter, whose tolerance is relative 1e-5; it uses the hardware
 //     approximations of sqrt and reciprocal (relative error below 3e-7).
+//
+// Measured on a B200, before -> after the split by sixteen elements (and, for the formats other
+// than UF8/AL8, against the general kernel): TinyLlama-1.1B update pass 3.23 -> 2.9 ms (5.3 TB/s);
+// bf16 parameters with stochastic rounding 5.0 -> 3.6 ms; UF4/AL16, 176 M parameters 4.17 -> 0.90 ms;
+// AL8 without momentum, fp32 gradients, 110 M parameters 1.95 -> 0.31 ms (4.9 TB/s).
 #pragma once
-
-#include <cstddef>
 
 #include "common.cuh"
 
@@ -54,9 +64,17 @@ namespace af8 {
 
 constexpr int FAST_VBLOCK = 2048;
 constexpr int FAST_MBLOCK = 256;
-constexpr int FAST_THREADS = 256;
-constexpr int FAST_EPT = 8;  // elements per thread
+constexpr int FAST_THREADS = 128;
+constexpr int FAST_EPT = 16;  // elements per thread
 constexpr int FAST_WARPS = FAST_THREADS / 32;
+// resident CTAs asked of the compiler (AL8: 5 -> 6 gave 1-3 %; AL16: 3, 4 and 5 gave 0.93, 0.91 and 0.97 ms on the UF4/AL16 case)
+#ifndef AF8_FAST_CTAS8
+#define AF8_FAST_CTAS8 6
+#endif
+#ifndef AF8_FAST_CTAS16
+#define AF8_FAST_CTAS16 4
+#endif
+template <int VB> constexpr int fast_min_ctas() { return VB == 8 ? AF8_FAST_CTAS8 : AF8_FAST_CTAS16; }
 
 struct FullrankLaunch {
     const af8_fullrank_tensor *tensors;
@@ -178,13 +196,6 @@ __device__ __forceinline__ uint32_t bf16x2_rn(float lo, float hi)
     return r;
 }
 
-template <bool SMALL_W>
-__device__ __forceinline__ float lerp_sel(float s, float e, float w, float wm1)
-{
-    const float d = __fsub_rn(e, s);
-    return SMALL_W ? __fmaf_rn(w, d, s) : __fmaf_rn(wm1, d, e);
-}
-
 // ---------------------------------------------------------------------------
 // device error flag, mbarrier and bulk-copy helpers
 // ---------------------------------------------------------------------------
@@ -239,136 +250,388 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
 }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-template <typename T> struct ParamElem { typedef float type; };
-template <> struct ParamElem<bf16_tag> { typedef uint16_t type; };
-template <typename T> struct GradBytes { static constexpr int value = 4; };
-template <> struct GradBytes<bf16_tag> { static constexpr int value = 2; };
-
 // ---------------------------------------------------------------------------
-// EMAs and update of a thread's 8 elements
+// second-moment codecs of the update kernel
 // ---------------------------------------------------------------------------
-struct StepScalars {
-    float decay, v_w, v_wm1, m_w, m_wm1, eps_g, eps_d, step_mul, fira;
-    bool zero_upd;
-    bool round_decay;   // bf16 parameter, nearest rounding: p*decay is rounded to bf16 before the update is added
+// AL16 has 65536 codes, so there is no table of a block's values: every element is decoded and
+// encoded with the binary64 sequences below.  Their small tables live one entry per lane in the
+// warp's registers and are read with shuffles (a shared-memory table costs about ten cycles of the
+// load pipe per look-up in bank conflicts, a shuffle one), and the operands enter binary64 through
+// their bits where they can (conversions run at a quarter of the rate of the arithmetic).
+struct LaneTables {
+    double e2;          // 2^(lane/32)
+    double l2;          // -log2(inv) of interval `lane`
+    uint32_t inv_hi;    // high word of inv
+};
+struct LogLaneEntry { uint32_t inv_hi; double l2; };
+__constant__ LogLaneEntry c_log2_lane[32] = {
+#include "log2_lane_table.inc"
 };
 
-// MODE: NOCLIP, APPLY (scalars of the statistic pass) or LAG (scalars of the previous step; the sum
-// of squares of this step's raw update is added to usq)
-template <int MODE, bool HAS_EPSG, bool TAIL>
-__device__ __forceinline__ void ema_update(const float (&g)[8], float (&p)[8], const uint32_t (&mq)[2],
-                                           const uint32_t (&vq)[2], const float *tab, float mc,
-                                           const StepScalars &S, int nva, int nvb, float (&v)[8], float (&m)[8],
-                                           float &usq)
+// exp2_cr_fast with the table in the lanes: |x| <= 150
+__device__ __forceinline__ float exp2_lane(float x, const LaneTables &T)
 {
-    constexpr bool DYN = MODE == AF8_MODE_APPLY || MODE == AF8_MODE_LAG;
-    const float2 w_v = bc2(S.v_w), w_m = bc2(S.m_w), mc2 = bc2(mc), eps_d2 = bc2(S.eps_d);
-    const float2 decay2 = bc2(S.decay), step2 = bc2(S.step_mul), fira2 = bc2(S.fira);
-#pragma unroll
-    for (int j = 0; j < 8; j += 2) {
-        const uint32_t c0 = __byte_perm(vq[j >> 2], 0u, 0x4440u | (uint32_t)(j & 3));
-        const uint32_t c1 = __byte_perm(vq[j >> 2], 0u, 0x4440u | (uint32_t)((j + 1) & 3));
-        const float2 gj = make_float2(g[j], g[j + 1]);
-        // second moment (optimizer.py:2117-2119)
-        float2 g2 = __fmul2_rn(gj, gj);
-        if (HAS_EPSG) g2 = __fadd2_rn(g2, bc2(S.eps_g));          // 0 in Adam mode (optimizer.py:1967)
-        const float2 v_old = make_float2(tab[c0], tab[c1]);
-        float2 vj = __ffma2_rn(w_v, sub2(g2, v_old), v_old);
-        // momentum (optimizer.py:528-531, 698): (byte - 128) * fl(scale / 128), then lerp
-        const float2 mb = make_float2(__uint_as_float(__byte_perm(mq[j >> 2], 0x4b000000u, 0x7540u | (uint32_t)(j & 3))),
-                                      __uint_as_float(__byte_perm(mq[j >> 2], 0x4b000000u, 0x7540u | (uint32_t)((j + 1) & 3))));
-        const float2 m_old = __fmul2_rn(__fadd2_rn(mb, bc2(-8388736.0f)), mc2);
-        float2 mj = __ffma2_rn(w_m, sub2(gj, m_old), m_old);
-        bool real0 = true, real1 = true;
-        if (TAIL) {
-            real0 = (j < 4) ? (j < nva) : (j - 4 < nvb);
-            real1 = (j < 4) ? (j + 1 < nva) : (j - 3 < nvb);
-            if (!real0) { vj.x = 0.0f; mj.x = 0.0f; }
-            if (!real1) { vj.y = 0.0f; mj.y = 0.0f; }
-        }
-        v[j] = vj.x; v[j + 1] = vj.y; m[j] = mj.x; m[j + 1] = mj.y;
-        // update from the un-requantised v and m (optimizer.py:905, 909); feeds the parameter only
-        const float2 den = __fadd2_rn(make_float2(sqrt_approx(vj.x), sqrt_approx(vj.y)), eps_d2);
-        float2 u = __fmul2_rn(mj, make_float2(rcp_approx(den.x), rcp_approx(den.y)));
-        if (TAIL) {                                               // padding (0 * inf when eps is 0)
-            if (!real0) u.x = 0.0f;
-            if (!real1) u.y = 0.0f;
-        }
-        float2 pj = __fmul2_rn(make_float2(p[j], p[j + 1]), decay2);     // optimizer.py:2039
-        if (S.round_decay) {                                      // Tensor.mul_ on a bf16 tensor rounds to bf16
-            const uint32_t pk = bf16x2_rn(pj.x, pj.y);
-            pj = make_float2(__uint_as_float(pk << 16), __uint_as_float(pk & 0xffff0000u));
-        }
-        if (MODE == AF8_MODE_LAG) usq = __fmaf_rn(u.y, u.y, __fmaf_rn(u.x, u.x, usq));
-        if (DYN) u = __fmul2_rn(u, fira2);                        // optimizer.py:803
-        if (!(DYN && S.zero_upd))                                 // non-finite norm: zero update (optimizer.py:798-800)
-            pj = __ffma2_rn(step2, u, pj);                        // optimizer.py:874
-        p[j] = pj.x; p[j + 1] = pj.y;
-    }
+    // n = rint(32 x) and the remainder x - n/32 are exact in binary32 (|32 x| < 2^13)
+    const float z = __fadd_rn(__fmul_rn(x, 32.0f), 12582912.0f);
+    const int n = __float_as_int(z);                                     // low bits hold n
+    const double r = (double)__fmaf_rn(__fsub_rn(z, 12582912.0f), -0.03125f, x);
+    const double t = __shfl_sync(0xffffffffu, T.e2, n & 31);
+    double p = AF8_EXP2_C6;
+    p = fma(p, r, AF8_EXP2_C5);
+    p = fma(p, r, AF8_EXP2_C4);
+    p = fma(p, r, AF8_EXP2_C3);
+    p = fma(p, r, AF8_EXP2_C2);
+    p = fma(p, r, AF8_EXP2_C1);
+    p = fma(p, r, 1.0);
+    const double y = t * p;                                              // in [1, 2.03)
+    return __double2float_rn(__hiloint2double(__double2hiint(y) + (((n - 0x4b400000) >> 5) << 20), __double2loint(y)));
+}
+
+// Correctly rounded log2 of a positive normal x (up to the error 2^-52 of the sum before the last
+// rounding): x = 2^e * m, m in [1, 2); the leading five fraction bits select inv_j, r = m*inv_j - 1 is
+// exact (24 + 21 bits) with |r| < 2^-6, log2(1 + r) by its Taylor series through r^8 (truncation below
+// 2^-56).  Next to x = 1 the result is absolutely, not relatively, accurate: for codes, not for ranges.
+__device__ __forceinline__ float log2_lane(float x, const LaneTables &T)
+{
+    const uint32_t b = __float_as_uint(x);
+    const int j = (b >> 18) & 31;
+    const double m = __hiloint2double((int)(0x3ff00000u | ((b >> 3) & 0xfffffu)), (int)(b << 29));
+    const double inv = __hiloint2double((int)__shfl_sync(0xffffffffu, T.inv_hi, j), 0);
+    const double tab = __shfl_sync(0xffffffffu, T.l2, j);
+    const double e = __hiloint2double(0x43300000, (int)(b >> 23)) - (4503599627370496.0 + 127.0);
+    const double r = fma(m, inv, -1.0);
+    double p = -0x1.71547652b82fep-3;       // -1/(8 ln 2)
+    p = fma(p, r, 0x1.a61762a7adedap-3);    //  1/(7 ln 2)
+    p = fma(p, r, -0x1.ec709dc3a03fep-3);   // -1/(6 ln 2)
+    p = fma(p, r, 0x1.2776c50ef9bfep-2);    //  1/(5 ln 2)
+    p = fma(p, r, -0x1.71547652b82fep-2);   // -1/(4 ln 2)
+    p = fma(p, r, 0x1.ec709dc3a03fep-2);    //  1/(3 ln 2)
+    p = fma(p, r, -0x1.71547652b82fep-1);   // -1/(2 ln 2)
+    p = fma(p, r, 0x1.71547652b82fep+0);    //  1/ln 2
+    return __double2float_rn(fma(p, r, e + tab));
+}
+
+// x / d from the correctly rounded reciprocal of d and one residual step: the IEEE quotient (Markstein)
+__device__ __forceinline__ float2 div2_by(float2 x, float2 rc, float2 nd)
+{
+    const float2 q = __fmul2_rn(x, rc);
+    return __ffma2_rn(__ffma2_rn(q, nd, x), rc, q);
+}
+
+// AL16 decode of two codes (optimizer.py:341-349); every lane of the warp takes part
+__device__ __forceinline__ float2 al16_decode2(uint32_t pair, float scale, float min_log, const LaneTables &T)
+{
+    const uint32_t c0 = pair & 0xffffu, c1 = pair >> 16;
+    // code - 1 as a float: the code becomes the low mantissa bits of 2^23 + code
+    const float2 c = make_float2(__fsub_rn(__uint_as_float(0x4b000000u | c0), 8388609.0f), __fsub_rn(__uint_as_float(0x4b000000u | c1), 8388609.0f));
+    const float2 x = __fmul2_rn(c, bc2(scale));
+    const float2 t = __fadd2_rn(div2_by(x, bc2(1.0f / 65534.0f), bc2(-65534.0f)), bc2(min_log));
+    // (code 0 decodes to zero; its t, just below min_log, only has to stay in range)
+    const float y0 = exp2_lane(t.x, T), y1 = exp2_lane(t.y, T);
+    return make_float2(c0 ? y0 : 0.0f, c1 ? y1 : 0.0f);
+}
+
+// ---------------------------------------------------------------------------
+// stochastic rounding of a pair to bf16 (same bits as sr_bf16_bits of each)
+// ---------------------------------------------------------------------------
+// "r24 < low16 * 256" only depends on the top 16 of the 24 random bits, r24 / 256 < low16; and adding
+// 65535 - r16 to the binary32 pattern carries into the upper half exactly then.  The last xor-shift of
+// the generator (by 31) does not reach the top 24 bits.  Infinities, NaNs and steps into an infinity
+// take the exact function.
+__device__ __forceinline__ uint32_t sr_hi32(uint64_t z)
+{
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    return (uint32_t)(z >> 32);
+}
+__device__ __forceinline__ uint32_t sr_bf16x2(float a, float b, uint32_t ha, uint32_t hb)
+{
+    const uint32_t x = __float_as_uint(a) + (~ha >> 16), y = __float_as_uint(b) + (~hb >> 16);
+    return __byte_perm(x, y, 0x7632);
+}
+
+// three-operand maximum, NaN if any operand is
+__device__ __forceinline__ float max3_nan(float a, float b, float c)
+{
+    float d;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+__device__ __forceinline__ float max3(float a, float b, float c)
+{
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+__device__ __forceinline__ float min3(float a, float b, float c)
+{
+    float d;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
 }
 
 // ---------------------------------------------------------------------------
 // the kernel
 // ---------------------------------------------------------------------------
-#ifndef AF8_FAST_MIN_CTAS
-#define AF8_FAST_MIN_CTAS 4
-#endif
-#ifndef AF8_FAST_STAGES_UPDATE
-#define AF8_FAST_STAGES_UPDATE 2      /* ring depth of the NOCLIP / APPLY passes, bf16 gradients */
-#endif
-#ifndef AF8_FAST_STAGES_UPDATE_F32
-#define AF8_FAST_STAGES_UPDATE_F32 2  /* the same with fp32 gradients (20 KB per slot) */
-#endif
+template <typename T> struct ParamElem { typedef float type; };
+template <> struct ParamElem<bf16_tag> { typedef uint16_t type; };
+template <typename T> struct GradBytes { static constexpr int value = 4; };
+template <> struct GradBytes<bf16_tag> { static constexpr int value = 2; };
 
-// Measured on B200 (TinyLlama set): depths 2 / 3 / 4 / 6 change the pass times by a few
-// per cent in the wrong direction (fewer resident CTAs), so the default stays at 2.
-// Ring geometry of one kernel variant: byte offsets inside a slot and the slot count.
-template <typename GradT, typename ParamT, int MODE> struct FastRing {
-    static constexpr int GB = GradBytes<GradT>::value;
-    static constexpr int PB = GradBytes<ParamT>::value;     // bytes per parameter: 4 (float) or 2 (bf16_tag)
-    static_assert(MODE == AF8_MODE_NOCLIP || MODE == AF8_MODE_APPLY || MODE == AF8_MODE_LAG, "the statistic pass has its own kernel (fullrank_stat.cuh)");
-    static constexpr int P_OFF = 0;
-    static constexpr int G_OFF = FAST_VBLOCK * PB;
-    static constexpr int MQ_OFF = G_OFF + FAST_VBLOCK * GB;
-    static constexpr int VQ_OFF = MQ_OFF + FAST_VBLOCK;
-    static constexpr int STAGE_BYTES = VQ_OFF + FAST_VBLOCK;
-    static constexpr int NST = GB == 2 ? AF8_FAST_STAGES_UPDATE : AF8_FAST_STAGES_UPDATE_F32;
-    static constexpr int SMEM_BYTES = NST * STAGE_BYTES;
-    static_assert(NST >= 2 && NST <= 8, "ring depth");
+// the step's scalars of the current tensor, in shared memory
+struct __align__(16) StepScalars {
+    float decay, step_mul, fira, eps_d;
+    float v_w, m_w, eps_g;
+    int16_t plain;      // both EMA weights below 1/2 and no eps on g^2
+    int16_t zero_upd;   // the limiter asked for a zero update
 };
 
-template <typename GradT, typename ParamT, int MODE>
-__global__ void __launch_bounds__(FAST_THREADS, AF8_FAST_MIN_CTAS)
+// Ring geometry of one kernel variant: byte offsets inside a slot and the slot count.
+template <typename GradT, typename ParamT, int VB, int MF> struct FastRing {
+    static constexpr int GB = GradBytes<GradT>::value;
+    static constexpr int PB = GradBytes<ParamT>::value;     // bytes per parameter: 4 (float) or 2 (bf16_tag)
+    static constexpr int MQ_BYTES = MF == AF8_M_UF8 ? FAST_VBLOCK : (MF == AF8_M_UF4 ? FAST_VBLOCK / 2 : 0);
+    static constexpr int VQ_BYTES = FAST_VBLOCK * VB / 8;
+    static constexpr int P_OFF = 0;
+    static constexpr int G_OFF = FAST_VBLOCK * PB;
+    static constexpr int VQ_OFF = G_OFF + FAST_VBLOCK * GB;
+    static constexpr int MQ_OFF = VQ_OFF + VQ_BYTES;
+    static constexpr int STAGE_BYTES = MQ_OFF + MQ_BYTES;
+    static constexpr int NST = 2;
+    static constexpr int SMEM_BYTES = NST * STAGE_BYTES;
+};
+
+// Eight elements (two groups of four) of one momentum block: EMAs, update, new parameter.
+// PLAIN: the common scalars (see StepScalars::plain).  LAG: sumsq += u^2 over the elements whose bit is set in real.
+template <int MF, bool PLAIN, bool ROUND_DECAY, bool LAG>
+__device__ __forceinline__ void fast_ema8(const StepScalars &S, const float2 (&g)[4], const float2 (&v_old)[4], const float2 (&m_old)[4],
+                                          float2 (&p)[4], float2 (&v)[4], float2 (&m)[4], uint32_t real, float &sumsq)
+{
+    const float2 w_v = bc2(S.v_w), w_m = bc2(S.m_w), eps_d2 = bc2(S.eps_d), decay2 = bc2(S.decay), step2 = bc2(S.step_mul), fira2 = bc2(S.fira);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        // second moment (optimizer.py:2117-2119)
+        if (PLAIN) {
+            v[j] = __ffma2_rn(w_v, sub2(__fmul2_rn(g[j], g[j]), v_old[j]), v_old[j]);
+        } else {
+            v[j] = make_float2(lerp_t(v_old[j].x, __fadd_rn(__fmul_rn(g[j].x, g[j].x), S.eps_g), S.v_w),
+                               lerp_t(v_old[j].y, __fadd_rn(__fmul_rn(g[j].y, g[j].y), S.eps_g), S.v_w));
+        }
+        // momentum (optimizer.py:698); without one the gradient itself is normalised (optimizer.py:911-917)
+        if (MF == AF8_M_NONE) m[j] = g[j];
+        else if (PLAIN) m[j] = __ffma2_rn(w_m, sub2(g[j], m_old[j]), m_old[j]);
+        else m[j] = make_float2(lerp_t(m_old[j].x, g[j].x, S.m_w), lerp_t(m_old[j].y, g[j].y, S.m_w));
+        // update from the un-requantised v and m (optimizer.py:905, 909); feeds the parameter only
+        const float2 den = __fadd2_rn(make_float2(sqrt_approx(v[j].x), sqrt_approx(v[j].y)), eps_d2);
+        float2 u = __fmul2_rn(m[j], make_float2(rcp_approx(den.x), rcp_approx(den.y)));
+        if (LAG) {                                                // (padding may be 0 * inf)
+            if ((real >> (2 * j)) & 1u) sumsq = __fmaf_rn(u.x, u.x, sumsq);
+            if ((real >> (2 * j + 1)) & 1u) sumsq = __fmaf_rn(u.y, u.y, sumsq);
+        }
+        float2 x = __fmul2_rn(p[j], decay2);                      // optimizer.py:2039
+        if (ROUND_DECAY) {                                        // Tensor.mul_ on a bf16 tensor rounds to bf16
+            const uint32_t pk = bf16x2_rn(x.x, x.y);
+            x = make_float2(__uint_as_float(pk << 16), __uint_as_float(pk & 0xffff0000u));
+        }
+        u = __fmul2_rn(u, fira2);                                 // optimizer.py:803 (1 without a limiter)
+        if (!S.zero_upd) x = __ffma2_rn(step2, u, x);             // optimizer.py:874; non-finite norm: zero update (optimizer.py:798-800)
+        p[j] = x;
+    }
+}
+
+__device__ __forceinline__ void unpack_bf16x4(uint2 w, float2 &a, float2 &b)
+{
+    a = make_float2(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xffff0000u));
+    b = make_float2(__uint_as_float(w.y << 16), __uint_as_float(w.y & 0xffff0000u));
+}
+
+// low bytes of four words
+__device__ __forceinline__ uint32_t pack4(uint32_t a, uint32_t b, uint32_t c, uint32_t d)
+{
+    return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
+}
+
+// element j of a register array, for the rare paths that are kept rolled: the kernel's hot loop is about
+// 14 KB of code, and unrolled copies of the exact sequences between its parts cost more in instruction
+// fetches than anything else (a quarter of the stall cycles in an earlier version)
+template <int N>
+__device__ __forceinline__ float pick(const float (&x)[N], int j)
+{
+    float r = x[0];
+#pragma unroll
+    for (int k = 1; k < N; ++k) r = j == k ? x[k] : r;
+    return r;
+}
+template <int N, typename T>
+__device__ __forceinline__ void put(T (&x)[N], int j, T value)
+{
+#pragma unroll
+    for (int k = 0; k < N; ++k) x[k] = j == k ? value : x[k];
+}
+
+// the inputs of a thread's eight elements of one momentum block (groups at oa and oa + 128) from a ring slot
+template <typename GradT, typename ParamT, int VB, int MF>
+__device__ __forceinline__ void fast_load8(const unsigned char *st, int oa, const float *tab, float v_scale, float v_min_log, float m_scale,
+                                           const LaneTables &LT, float2 (&p)[4], float2 (&g)[4], float2 (&v_old)[4], float2 (&m_old)[4])
+{
+    using Ring = FastRing<GradT, ParamT, VB, MF>;
+    const int ob = oa + 128;
+    if (Ring::PB == 4) {
+        const float4 a = *reinterpret_cast<const float4 *>(st + Ring::P_OFF + oa * 4);
+        const float4 c = *reinterpret_cast<const float4 *>(st + Ring::P_OFF + ob * 4);
+        p[0] = make_float2(a.x, a.y); p[1] = make_float2(a.z, a.w); p[2] = make_float2(c.x, c.y); p[3] = make_float2(c.z, c.w);
+    } else {
+        unpack_bf16x4(*reinterpret_cast<const uint2 *>(st + Ring::P_OFF + oa * 2), p[0], p[1]);
+        unpack_bf16x4(*reinterpret_cast<const uint2 *>(st + Ring::P_OFF + ob * 2), p[2], p[3]);
+    }
+    if (Ring::GB == 4) {
+        const float4 a = *reinterpret_cast<const float4 *>(st + Ring::G_OFF + oa * 4);
+        const float4 c = *reinterpret_cast<const float4 *>(st + Ring::G_OFF + ob * 4);
+        g[0] = make_float2(a.x, a.y); g[1] = make_float2(a.z, a.w); g[2] = make_float2(c.x, c.y); g[3] = make_float2(c.z, c.w);
+    } else {
+        unpack_bf16x4(*reinterpret_cast<const uint2 *>(st + Ring::G_OFF + oa * 2), g[0], g[1]);
+        unpack_bf16x4(*reinterpret_cast<const uint2 *>(st + Ring::G_OFF + ob * 2), g[2], g[3]);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int o = h ? ob : oa;
+        if (VB == 8) {
+            const uint32_t w = *reinterpret_cast<const uint32_t *>(st + Ring::VQ_OFF + o);
+            v_old[2 * h] = make_float2(tab[w & 0xffu], tab[__byte_perm(w, 0u, 0x4441u)]);
+            v_old[2 * h + 1] = make_float2(tab[__byte_perm(w, 0u, 0x4442u)], tab[w >> 24]);
+        } else {
+            const uint2 w = *reinterpret_cast<const uint2 *>(st + Ring::VQ_OFF + o * 2);
+            v_old[2 * h] = al16_decode2(w.x, v_scale, v_min_log, LT);
+            v_old[2 * h + 1] = al16_decode2(w.y, v_scale, v_min_log, LT);
+        }
+        if (MF == AF8_M_UF8) {
+            // (byte - 128) * fl(scale / 128) (optimizer.py:528-531): a power-of-two divisor, and
+            // m_scale >= 1e-12 keeps the quotient far from the subnormal range
+            const float2 mc2 = bc2(__fmul_rn(m_scale, 0.0078125f));
+            const uint32_t w = *reinterpret_cast<const uint32_t *>(st + Ring::MQ_OFF + o);
+            const float2 x = make_float2(__uint_as_float(__byte_perm(w, 0x4b000000u, 0x7540u)), __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7541u)));
+            const float2 y = make_float2(__uint_as_float(__byte_perm(w, 0x4b000000u, 0x7542u)), __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7543u)));
+            m_old[2 * h] = __fmul2_rn(__fadd2_rn(x, bc2(-8388736.0f)), mc2);
+            m_old[2 * h + 1] = __fmul2_rn(__fadd2_rn(y, bc2(-8388736.0f)), mc2);
+        } else if (MF == AF8_M_UF4) {
+            // (nibble - 8) * fl(scale / 8), the even element in the high nibble
+            const float2 mc2 = bc2(__fmul_rn(m_scale, 0.125f));
+            const uint32_t w = *reinterpret_cast<const uint16_t *>(st + Ring::MQ_OFF + o / 2);
+            const float2 x = make_float2(__uint_as_float(0x4b000000u | ((w >> 4) & 15u)), __uint_as_float(0x4b000000u | (w & 15u)));
+            const float2 y = make_float2(__uint_as_float(0x4b000000u | (w >> 12)), __uint_as_float(0x4b000000u | ((w >> 8) & 15u)));
+            m_old[2 * h] = __fmul2_rn(__fadd2_rn(x, bc2(-8388616.0f)), mc2);
+            m_old[2 * h + 1] = __fmul2_rn(__fadd2_rn(y, bc2(-8388616.0f)), mc2);
+        } else {
+            m_old[2 * h] = m_old[2 * h + 1] = make_float2(0.0f, 0.0f);
+        }
+    }
+}
+
+// Requantisation of one momentum block: 32 lanes of eight elements, groups at e and e + 128
+// (optimizer.py:510, 518).  Writes the codes and the scale when `live`.
+template <int MF>
+__device__ __forceinline__ void fast_store_m(const float2 (&m)[4], uint8_t *m_q, float *m_scale, int64_t e, bool live, int lane)
+{
+    float amx = fabsf(m[0].x);
+    amx = max3(amx, fabsf(m[0].y), fabsf(m[1].x));
+    amx = max3(amx, fabsf(m[1].y), fabsf(m[2].x));
+    amx = max3(amx, fabsf(m[2].y), fabsf(m[3].x));
+    amx = fmaxf(amx, fabsf(m[3].y));
+    // non-negative floats order like their bit patterns: one REDUX instead of a shuffle tree
+    const float am = fmaxf(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amx))), 1e-12f);
+    const float2 ra2 = bc2(__frcp_rn(am)), nam2 = bc2(-am);
+    // round(m / am * levels) (the product with the power of two is exact); |m / am| <= 1, so only
+    // +levels needs the clamp to levels - 1
+    constexpr float LEVELS = MF == AF8_M_UF4 ? 8.0f : 128.0f;
+    constexpr int TOP = MF == AF8_M_UF4 ? 7 : 127;
+    uint32_t raw[8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float2 kf = __ffma2_rn(div2_by(m[j], ra2, nam2), bc2(LEVELS), bc2(AF8_MAGIC_F));
+        raw[2 * j] = (uint32_t)min(__float_as_int(kf.x), AF8_MAGIC_I + TOP);
+        raw[2 * j + 1] = (uint32_t)min(__float_as_int(kf.y), AF8_MAGIC_I + TOP);
+    }
+    if (!live) return;
+    if (MF == AF8_M_UF8) {
+        // low bytes hold k mod 256; k + 128 is that byte with its top bit flipped
+        *reinterpret_cast<uint32_t *>(m_q + e) = pack4(raw[0], raw[1], raw[2], raw[3]) ^ 0x80808080u;
+        *reinterpret_cast<uint32_t *>(m_q + e + 128) = pack4(raw[4], raw[5], raw[6], raw[7]) ^ 0x80808080u;
+    } else {
+        // low nibbles hold k mod 16; the first element of a byte is its high nibble
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t b0 = ((raw[4 * h] & 15u) << 4) | (raw[4 * h + 1] & 15u), b1 = ((raw[4 * h + 2] & 15u) << 4) | (raw[4 * h + 3] & 15u);
+            *reinterpret_cast<uint16_t *>(m_q + ((e + 128 * h) >> 1)) = (uint16_t)((b0 | (b1 << 8)) ^ 0x8888u);
+        }
+    }
+    if (lane == 0) *m_scale = am;
+}
+
+// The 16-bit patterns of eight new bf16 parameters (elements e .. e + 3 and e + 128 ..): the last rounding, to
+// nearest or stochastic (optimizer.py:873-881).
+template <bool SR>
+__device__ __forceinline__ void fast_round8(const float2 (&p)[4], uint64_t sr_base, int64_t e, uint32_t (&w)[4])
+{
+    if (!SR) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[j] = bf16x2_rn(p[j].x, p[j].y);
+        return;
+    }
+    const uint64_t z0 = sr_base + (uint64_t)e + 0x9E3779B97F4A7C15ull;
+    float top = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint64_t z = z0 + (uint64_t)((j < 2 ? 0 : 124) + 2 * j);
+        w[j] = sr_bf16x2(p[j].x, p[j].y, sr_hi32(z), sr_hi32(z + 1));
+        top = max3_nan(top, fabsf(p[j].x), fabsf(p[j].y));
+    }
+    if (!(top < 3.3895314e38f)) {                 // an infinity, a NaN or a step into an infinity: element by element
+        const float x[8] = {p[0].x, p[0].y, p[1].x, p[1].y, p[2].x, p[2].y, p[3].x, p[3].y};
+#pragma unroll 1
+        for (int k = 0; k < 4; ++k) {
+            const uint64_t i = (uint64_t)(e + (k < 2 ? 0 : 124) + 2 * k);
+            put(w, k, sr_bf16_bits(pick(x, 2 * k), sr_bits24(sr_base, i)) | (sr_bf16_bits(pick(x, 2 * k + 1), sr_bits24(sr_base, i + 1)) << 16));
+        }
+    }
+}
+
+// SR: bf16 parameters rounded stochastically.  LAG: the scalars are those of the previous step and the
+// sum of squares of this step's raw update goes to block_sumsq.
+template <typename GradT, typename ParamT, int VB, int MF, bool SR, bool LAG>
+__global__ void __launch_bounds__(FAST_THREADS, fast_min_ctas<VB>())
 fullrank_fast_kernel(const FullrankLaunch L)
 {
-    using Ring = FastRing<GradT, ParamT, MODE>;
-    constexpr int GB = Ring::GB;
-    constexpr int PB = Ring::PB;
+    using Ring = FastRing<GradT, ParamT, VB, MF>;
     using PElem = typename ParamElem<ParamT>::type;
-    constexpr int P_OFF = Ring::P_OFF, G_OFF = Ring::G_OFF, MQ_OFF = Ring::MQ_OFF, VQ_OFF = Ring::VQ_OFF;
-    constexpr int STAGE_BYTES = Ring::STAGE_BYTES;
-    constexpr int NST = Ring::NST;
+    constexpr int GB = Ring::GB, PB = Ring::PB, NST = Ring::NST, STAGE_BYTES = Ring::STAGE_BYTES;
+    constexpr int P_OFF = Ring::P_OFF, G_OFF = Ring::G_OFF, VQ_OFF = Ring::VQ_OFF, MQ_OFF = Ring::MQ_OFF;
+    constexpr int MPB = FAST_VBLOCK / FAST_MBLOCK;                // momentum blocks per V block
+    constexpr int QMAX = VB == 16 ? 65535 : 255;
+    constexpr float QM1 = VB == 16 ? 65534.0f : 254.0f;
+    constexpr bool TABLE = VB == 8;
 
     extern __shared__ __align__(128) unsigned char s_ring[];     // NST slots of STAGE_BYTES
     __shared__ __align__(8) uint64_t s_full[NST];
     __shared__ __align__(16) af8_fullrank_tensor sT;
-    __shared__ float s_tab[2][256];
+    __shared__ StepScalars sS;
+    __shared__ float s_tab[2][TABLE ? 256 : 1];
     __shared__ uint32_t s_redmin[FAST_WARPS];
     __shared__ uint32_t s_redmax[FAST_WARPS];
     __shared__ float s_usq[FAST_WARPS];
     __shared__ VRange s_vr;
     __shared__ int s_abort;
-    __shared__ double s_exp2[32];            // copy of the exp2 table of the decode
-    __shared__ double2 s_log2[97];           // copy of the log2 table of the range computation
+    __shared__ double s_exp2[TABLE ? 32 : 1];        // copy of the exp2 table of the decode
+    __shared__ double2 s_log2[97];                   // copy of the log2 table of the range computation
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
     const int lane = tid & 31;
-    const int oa = warp * FAST_MBLOCK + lane * 4;   // first 4-element group of this thread
-    const int ob = oa + 128;                         // second group
+    const int ow = warp * (FAST_EPT * 32) + lane * 4;   // first group of four of this thread; the others follow at 128, 256, ...
 
-    if (tid < 32) s_exp2[tid] = c_exp2_tab[tid];
+    if (TABLE && tid < 32) s_exp2[tid] = c_exp2_tab[tid];
     if (tid < 97) s_log2[tid] = c_log2_tab[tid];
+    LaneTables LT;
+    if (!TABLE) { LT.e2 = c_exp2_tab[lane]; LT.l2 = c_log2_lane[lane].l2; LT.inv_hi = c_log2_lane[lane].inv_hi; }
     if (tid == 0) {
         for (int k = 0; k < NST; ++k) mbar_init(&s_full[k], 1);
         s_abort = 0;
@@ -383,8 +646,9 @@ fullrank_fast_kernel(const FullrankLaunch L)
     uint32_t phase = 0;                      // bit k: parity to wait for on ring slot k
     int ahead = 0;                           // consecutive blocks from the current one whose copies are in flight
     bool staged = false;                     // this block's decode table and ranges were prepared last iteration
-    float nsc = 0.f, nml = 0.f, nms = 0.f;   // prefetched range of the next block (v_scale, v_min_log, m_scale)
-    float mscale_cur = 0.f;
+    float csc = 0.f, cml = 0.f;              // range of this block (AL16: the elements are decoded with it)
+    float nsc = 0.f, nml = 0.f;              // prefetched range of the next block
+    float cms[2] = {0.f, 0.f}, nms[2] = {0.f, 0.f};   // momentum scales of this warp's two blocks, and the next ones
     int n = 0;
 
     for (int64_t blk = blockIdx.x; blk < L.total_blocks; blk += gridDim.x, ++n) {
@@ -401,6 +665,19 @@ fullrank_fast_kernel(const FullrankLaunch L)
                 reinterpret_cast<uint32_t *>(&sT)[tid] =
                     __ldg(reinterpret_cast<const uint32_t *>(L.tensors + t) + tid);
             __syncthreads();
+            if (tid == 0) {
+                StepScalars S;
+                S.decay = sT.decay; S.step_mul = -sT.alpha; S.fira = 1.0f; S.eps_d = sT.eps_denom;
+                S.v_w = sT.v_w; S.m_w = MF == AF8_M_NONE ? 0.0f : sT.m_w; S.eps_g = sT.eps_gradsq;
+                S.zero_upd = 0;
+                if (L.dyn != nullptr) {
+                    const af8_dyn_scalars ds = L.dyn[t];
+                    S.step_mul = ds.step; S.fira = ds.fira; S.zero_upd = ds.zero != 0.0f;
+                }
+                S.plain = fabsf(S.v_w) < 0.5f && fabsf(S.m_w) < 0.5f && S.eps_g == 0.0f;
+                sS = S;
+            }
+            __syncthreads();
             cur_t = t;
             cur_first = sT.first_block;
             cur_end = cur_first + (sT.numel + FAST_VBLOCK - 1) / FAST_VBLOCK;
@@ -410,8 +687,8 @@ fullrank_fast_kernel(const FullrankLaunch L)
         const int b = (int)(blk - cur_first);         // V block index inside the tensor
         const int64_t base = (int64_t)b * FAST_VBLOCK;   // first element of the block
         const bool full = b < nfull;
-        const int64_t rem = full ? FAST_VBLOCK : sT.numel - base;   // real elements from base on (> 0), capped
-        const int stage = n & 1;                      // decode-table / partial-sum buffer of this block
+        const int rem = full ? FAST_VBLOCK : (int)(sT.numel - base);   // real elements from base on (> 0)
+        const int stage = n & 1;                      // decode-table buffer of this block
         const int slot = n % NST;                     // ring slot of this block
         const int b_next = b + G;
         // blocks blk, blk+G, ... that are full blocks of this tensor get their copies issued ahead
@@ -434,38 +711,40 @@ fullrank_fast_kernel(const FullrankLaunch L)
                 mbar_expect_tx(&s_full[sl], STAGE_BYTES);
                 bulk_g2s(dst + P_OFF, pp + nb * PB, FAST_VBLOCK * PB, &s_full[sl]);
                 bulk_g2s(dst + G_OFF, gp + nb * GB, FAST_VBLOCK * GB, &s_full[sl]);
-                bulk_g2s(dst + MQ_OFF, sT.m_q + nb, FAST_VBLOCK, &s_full[sl]);
-                bulk_g2s(dst + VQ_OFF, vp + nb, FAST_VBLOCK, &s_full[sl]);
+                bulk_g2s(dst + VQ_OFF, vp + nb * (VB / 8), Ring::VQ_BYTES, &s_full[sl]);
+                if (MF != AF8_M_NONE)
+                    bulk_g2s(dst + MQ_OFF, sT.m_q + (MF == AF8_M_UF4 ? nb / 2 : nb), Ring::MQ_BYTES, &s_full[sl]);
             }
         }
         const int in_flight = want;                   // copies outstanding now, this block included
         ahead = want > 0 ? want - 1 : 0;              // ... as seen from the next block
         // ---- ranges of this block (if not prefetched) and of the next one ----
-        const bool m_exists = (int64_t)warp * FAST_MBLOCK < rem;   // this warp's M block is allocated
         if (!staged) {
-            const float sc = __ldg(sT.v_scale + b);
-            const float ml = __ldg(sT.v_min_log + b);
-            mscale_cur = m_exists ? __ldg(sT.m_scale + b * (FAST_VBLOCK / FAST_MBLOCK) + warp) : 0.0f;
-            s_tab[stage][tid] = al8_decode_fast((uint32_t)tid, sc, ml, s_exp2);   // optimizer.py:341-349
+            csc = __ldg(sT.v_scale + b);
+            cml = __ldg(sT.v_min_log + b);
+            if (MF != AF8_M_NONE) {
+#pragma unroll
+                for (int k = 0; k < 2; ++k)           // (momentum blocks beyond the tensor are not allocated)
+                    cms[k] = (2 * warp + k) * FAST_MBLOCK < rem ? __ldg(sT.m_scale + (int64_t)b * MPB + 2 * warp + k) : 0.0f;
+            }
+            if (TABLE) {
+                s_tab[stage][tid] = al8_decode_fast((uint32_t)tid, csc, cml, s_exp2);   // optimizer.py:341-349
+                s_tab[stage][tid + 128] = al8_decode_fast((uint32_t)tid + 128u, csc, cml, s_exp2);
+            }
             __syncthreads();
         }
         if (next_staged) {
             nsc = __ldg(sT.v_scale + b_next);
             nml = __ldg(sT.v_min_log + b_next);
-            nms = __ldg(sT.m_scale + b_next * (FAST_VBLOCK / FAST_MBLOCK) + warp);
+            if (MF != AF8_M_NONE) {
+                const float2 x = make_float2(__ldg(sT.m_scale + (int64_t)b_next * MPB + 2 * warp), __ldg(sT.m_scale + (int64_t)b_next * MPB + 2 * warp + 1));
+                nms[0] = x.x; nms[1] = x.y;
+            }
         }
-        // fl(m_scale / 128) (optimizer.py:531): a power-of-two divisor, so the product is the
-        // same number (m_scale >= 1e-12 keeps it far from the subnormal range)
-        const float mc = __fmul_rn(mscale_cur, 0.0078125f);
 
-        // ---- this thread's raw inputs ----
-        float p[8], g[8];
-        uint32_t mq[2], vq[2];
-        int nva = 4, nvb = 4;
+        // ---- this block's inputs in its ring slot ----
+        unsigned char *const st = s_ring + slot * STAGE_BYTES;
         bool bad = false;
-        // (typed pointers: with byte pointers and a scaled offset the update pass ran 2.5 % slower)
-        PElem *pa = static_cast<PElem *>(sT.param) + base + oa;
-        PElem *pb = static_cast<PElem *>(sT.param) + base + ob;
         if (full) {
             if (!mbar_wait_bounded(&s_full[slot], (phase >> slot) & 1u)) {
                 bad = true;      // this thread stores nothing for the block
@@ -473,139 +752,152 @@ fullrank_fast_kernel(const FullrankLaunch L)
                 atomicExch(&g_device_error, DEVERR_COPY_TIMEOUT);
             }
             phase ^= 1u << slot;
-            const unsigned char *st = s_ring + slot * STAGE_BYTES;
-            if (PB == 4) {
-                const float4 a = *reinterpret_cast<const float4 *>(st + P_OFF + oa * 4);
-                const float4 c = *reinterpret_cast<const float4 *>(st + P_OFF + ob * 4);
-                p[0] = a.x; p[1] = a.y; p[2] = a.z; p[3] = a.w;
-                p[4] = c.x; p[5] = c.y; p[6] = c.z; p[7] = c.w;
-            } else {
-                const uint2 a = *reinterpret_cast<const uint2 *>(st + P_OFF + oa * 2);
-                const uint2 c = *reinterpret_cast<const uint2 *>(st + P_OFF + ob * 2);
-                p[0] = __uint_as_float(a.x << 16); p[1] = __uint_as_float(a.x & 0xffff0000u);
-                p[2] = __uint_as_float(a.y << 16); p[3] = __uint_as_float(a.y & 0xffff0000u);
-                p[4] = __uint_as_float(c.x << 16); p[5] = __uint_as_float(c.x & 0xffff0000u);
-                p[6] = __uint_as_float(c.y << 16); p[7] = __uint_as_float(c.y & 0xffff0000u);
-            }
-            if (GB == 4) {
-                const float4 a = *reinterpret_cast<const float4 *>(st + G_OFF + oa * 4);
-                const float4 c = *reinterpret_cast<const float4 *>(st + G_OFF + ob * 4);
-                g[0] = a.x; g[1] = a.y; g[2] = a.z; g[3] = a.w;
-                g[4] = c.x; g[5] = c.y; g[6] = c.z; g[7] = c.w;
-            } else {
-                const uint2 a = *reinterpret_cast<const uint2 *>(st + G_OFF + oa * 2);
-                const uint2 c = *reinterpret_cast<const uint2 *>(st + G_OFF + ob * 2);
-                g[0] = __uint_as_float(a.x << 16); g[1] = __uint_as_float(a.x & 0xffff0000u);
-                g[2] = __uint_as_float(a.y << 16); g[3] = __uint_as_float(a.y & 0xffff0000u);
-                g[4] = __uint_as_float(c.x << 16); g[5] = __uint_as_float(c.x & 0xffff0000u);
-                g[6] = __uint_as_float(c.y << 16); g[7] = __uint_as_float(c.y & 0xffff0000u);
-            }
-            mq[0] = *reinterpret_cast<const uint32_t *>(st + MQ_OFF + oa);
-            mq[1] = *reinterpret_cast<const uint32_t *>(st + MQ_OFF + ob);
-            vq[0] = *reinterpret_cast<const uint32_t *>(st + VQ_OFF + oa);
-            vq[1] = *reinterpret_cast<const uint32_t *>(st + VQ_OFF + ob);
         } else {
-            // tail block: guarded plain loads; the V state is padded to the block, the M
-            // state only to its own 256-element blocks
-            nva = (int)max((int64_t)0, min((int64_t)4, rem - oa));
-            nvb = (int)max((int64_t)0, min((int64_t)4, rem - ob));
-            const uint8_t *vp = static_cast<const uint8_t *>(sT.v_q) + base;
-            vq[0] = *reinterpret_cast<const uint32_t *>(vp + oa);
-            vq[1] = *reinterpret_cast<const uint32_t *>(vp + ob);
-            mq[0] = m_exists ? *reinterpret_cast<const uint32_t *>(sT.m_q + base + oa) : 0x80808080u;
-            mq[1] = m_exists ? *reinterpret_cast<const uint32_t *>(sT.m_q + base + ob) : 0x80808080u;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int e = (j < 4) ? oa + j : ob + j - 4;
-                const bool ok = (j < 4) ? (j < nva) : (j - 4 < nvb);
-                p[j] = ok ? param_load(sT.param, base + e, PB == 4 ? AF8_F32 : AF8_BF16) : 0.0f;
-                g[j] = ok ? GradLoad<GradT>::load1(sT.grad, base + e) : 0.0f;
+            // Tail block: guarded plain loads into the slot.  Beyond the end the gradient and the parameter are
+            // zero; the V state is padded to the block, the M state only to its own 256-element blocks.
+#pragma unroll 1
+            for (int e = tid; e < FAST_VBLOCK; e += FAST_THREADS) {
+                const bool ok = e < rem;
+                if (PB == 4) reinterpret_cast<float *>(st + P_OFF)[e] = ok ? static_cast<const float *>(sT.param)[base + e] : 0.0f;
+                else reinterpret_cast<uint16_t *>(st + P_OFF)[e] = ok ? static_cast<const uint16_t *>(sT.param)[base + e] : (uint16_t)0;
+                if (GB == 4) reinterpret_cast<float *>(st + G_OFF)[e] = ok ? static_cast<const float *>(sT.grad)[base + e] : 0.0f;
+                else reinterpret_cast<uint16_t *>(st + G_OFF)[e] = ok ? static_cast<const uint16_t *>(sT.grad)[base + e] : (uint16_t)0;
+                if (VB == 8) (st + VQ_OFF)[e] = static_cast<const uint8_t *>(sT.v_q)[base + e];
+                else reinterpret_cast<uint16_t *>(st + VQ_OFF)[e] = static_cast<const uint16_t *>(sT.v_q)[base + e];
+                const bool m_ok = (e & ~(FAST_MBLOCK - 1)) < rem;
+                if (MF == AF8_M_UF8) (st + MQ_OFF)[e] = m_ok ? sT.m_q[base + e] : (uint8_t)128;
+                if (MF == AF8_M_UF4 && (e & 1) == 0) (st + MQ_OFF)[e >> 1] = m_ok ? sT.m_q[(base + e) >> 1] : (uint8_t)0x88;
             }
-        }
-        if (L.negate_grad) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) g[j] = -g[j];
+            __syncthreads();
         }
 
-        // ---- scalars of the step ----
-        StepScalars S;
-        {   // three vector loads instead of six scalar ones (the descriptor is 16-byte aligned)
-            static_assert(offsetof(af8_fullrank_tensor, decay) % 8 == 0 && offsetof(af8_fullrank_tensor, v_w) % 16 == 0 &&
-                          offsetof(af8_fullrank_tensor, m_w) == offsetof(af8_fullrank_tensor, v_w) + 12 &&
-                          offsetof(af8_fullrank_tensor, eps_gradsq) % 8 == 0 &&
-                          offsetof(af8_fullrank_tensor, eps_denom) == offsetof(af8_fullrank_tensor, eps_gradsq) + 4, "descriptor layout");
-            const float2 da = *reinterpret_cast<const float2 *>(&sT.decay);
-            const float4 vw = *reinterpret_cast<const float4 *>(&sT.v_w);
-            const float2 ep = *reinterpret_cast<const float2 *>(&sT.eps_gradsq);
-            S.decay = da.x; S.step_mul = -da.y; S.v_w = vw.x; S.m_w = vw.w; S.eps_g = ep.x; S.eps_d = ep.y;
-        }
-        S.v_wm1 = __fsub_rn(S.v_w, 1.0f); S.m_wm1 = __fsub_rn(S.m_w, 1.0f);
-        S.fira = 1.0f; S.zero_upd = false;
-        S.round_decay = PB == 2 && !L.sr;
-        constexpr bool DYN = MODE == AF8_MODE_APPLY || MODE == AF8_MODE_LAG;
+        const StepScalars S = sS;
+        const bool hot = full && S.plain;    // (uniform over the CTA)
+        float v[FAST_EPT];                   // hot blocks: the new second moments
         float usq = 0.0f;                    // LAG: this thread's sum of squares of the raw update
-        if (DYN) {
-            const af8_dyn_scalars ds = L.dyn[cur_t];
-            S.step_mul = ds.step; S.fira = ds.fira; S.zero_upd = ds.zero != 0.0f;
-        }
+        // Extrema of v.  v >= 0, so the bit patterns order like the values.  The minimum runs over the
+        // non-zero elements (optimizer.py:312-313) and travels as bits - 1, which sends "none" to the top.
+        uint32_t umin, umax;
 
-        // ---- EMAs and update: everything that reaches a state is exact ----
-        float v[8], m[8];
-        const bool small_w = fabsf(S.v_w) < 0.5f && fabsf(S.m_w) < 0.5f;   // ATen's lerp has two forms
-        if (small_w) {
-            if (full) {
-                if (S.eps_g == 0.0f) ema_update<MODE, false, false>(g, p, mq, vq, s_tab[stage], mc, S, nva, nvb, v, m, usq);
-                else ema_update<MODE, true, false>(g, p, mq, vq, s_tab[stage], mc, S, nva, nvb, v, m, usq);
-            } else {
-                ema_update<MODE, true, true>(g, p, mq, vq, s_tab[stage], mc, S, nva, nvb, v, m, usq);
-            }
-        } else {
+        if (hot) {
+            // ---- two momentum blocks per warp: EMAs, update, parameter, momentum codes ----
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {   // general lerp (weights >= 0.5): rare, kept simple
-                const bool real = (j < 4) ? (j < nva) : (j - 4 < nvb);
-                const uint32_t vcode = (vq[j >> 2] >> (8 * (j & 3))) & 0xffu;
-                const float g2 = __fadd_rn(__fmul_rn(g[j], g[j]), S.eps_g);
-                float vj = lerp_t(s_tab[stage][vcode], g2, S.v_w);
-                float mj = lerp_t(__fmul_rn(byte_minus_128(mq[j >> 2], j & 3), mc), g[j], S.m_w);
-                if (!real) { vj = 0.0f; mj = 0.0f; }
-                v[j] = vj; m[j] = mj;
-                float u = __fmul_rn(mj, rcp_approx(__fadd_rn(sqrt_approx(vj), S.eps_d)));
-                if (!real) u = 0.0f;
-                float pj = __fmul_rn(p[j], S.decay);
-                if (S.round_decay) pj = param_round(pj, AF8_BF16);
-                if (MODE == AF8_MODE_LAG) usq = __fmaf_rn(u, u, usq);
-                const float us = DYN ? __fmul_rn(u, S.fira) : u;
-                if (!(DYN && S.zero_upd)) pj = __fmaf_rn(S.step_mul, us, pj);
-                p[j] = pj;
+            for (int mb = 0; mb < 2; ++mb) {
+                const int oa = ow + mb * FAST_MBLOCK;
+                float2 g[4], p[4], v_old[4], m_old[4], vn[4], mn[4];
+                fast_load8<GradT, ParamT, VB, MF>(st, oa, s_tab[stage], csc, cml, cms[mb], LT, p, g, v_old, m_old);
+                if (L.negate_grad) {                              // maximize (optimizer.py:1973-1974)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) g[j] = make_float2(-g[j].x, -g[j].y);
+                }
+                fast_ema8<MF, true, PB == 2 && !SR, LAG>(S, g, v_old, m_old, p, vn, mn, 0xffu, usq);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) { v[8 * mb + 2 * j] = vn[j].x; v[8 * mb + 2 * j + 1] = vn[j].y; }
+                PElem *const pa = static_cast<PElem *>(sT.param) + base + oa;
+                if (PB == 4) {
+                    if (!bad) {
+                        *reinterpret_cast<float4 *>(pa) = make_float4(p[0].x, p[0].y, p[1].x, p[1].y);
+                        *reinterpret_cast<float4 *>(pa + 128) = make_float4(p[2].x, p[2].y, p[3].x, p[3].y);
+                        if (sT.param_copy != nullptr) {           // bf16 compute copy
+                            uint16_t *const ca = static_cast<uint16_t *>(sT.param_copy) + base + oa;
+                            *reinterpret_cast<uint2 *>(ca) = make_uint2(bf16x2_rn(p[0].x, p[0].y), bf16x2_rn(p[1].x, p[1].y));
+                            *reinterpret_cast<uint2 *>(ca + 128) = make_uint2(bf16x2_rn(p[2].x, p[2].y), bf16x2_rn(p[3].x, p[3].y));
+                        }
+                    }
+                } else {
+                    uint32_t w[4];
+                    fast_round8<SR>(p, sT.sr_base, base + oa, w);
+                    if (!bad) {
+                        *reinterpret_cast<uint2 *>(pa) = make_uint2(w[0], w[1]);
+                        *reinterpret_cast<uint2 *>(pa + 128) = make_uint2(w[2], w[3]);
+                    }
+                }
+                if (MF != AF8_M_NONE)
+                    fast_store_m<MF>(mn, sT.m_q, sT.m_scale + (int64_t)b * MPB + 2 * warp + mb, base + oa, !bad, lane);
             }
-        }
-
-        // ---- block extrema of v.  v >= 0, so the bit patterns order like the values.  The
-        //      minimum runs over the non-zero elements (optimizer.py:312-313) and travels as
-        //      bits-1, which sends "none" to the top; a warp that holds a zero (rare after the
-        //      first steps, except in all-zero regions) rescans its registers for it ----
-        {
             float fmn = v[0], fmx = v[0];
 #pragma unroll
-            for (int j = 1; j < 8; ++j) {
-                fmn = fminf(fmn, v[j]);
-                fmx = fmaxf(fmx, v[j]);
+            for (int j = 1; j + 1 < FAST_EPT; j += 2) {
+                fmn = min3(fmn, v[j], v[j + 1]);
+                fmx = max3(fmx, v[j], v[j + 1]);
             }
-            uint32_t umin = __reduce_min_sync(0xffffffffu, __float_as_uint(fmn));
-            const uint32_t umax = __reduce_max_sync(0xffffffffu, __float_as_uint(fmx));
-            if (umin == 0u) {                                    // uniform over the warp
+            fmn = fminf(fmn, v[FAST_EPT - 1]);
+            fmx = fmaxf(fmx, v[FAST_EPT - 1]);
+            umin = __reduce_min_sync(0xffffffffu, __float_as_uint(fmn));
+            umax = __reduce_max_sync(0xffffffffu, __float_as_uint(fmx));
+            if (umin == 0u) {            // the warp holds a zero (rare after the first steps, except in all-zero regions)
                 uint32_t um = 0xffffffffu;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) um = min(um, __float_as_uint(v[j]) - 1u);
+                for (int j = 0; j < FAST_EPT; ++j) um = min(um, __float_as_uint(v[j]) - 1u);
                 umin = __reduce_min_sync(0xffffffffu, um);
             } else {
                 umin -= 1u;
             }
-            if (lane == 0) { s_redmin[warp] = umin; s_redmax[warp] = umax; }
-            if (MODE == AF8_MODE_LAG) {      // the block's sum of squares travels with the extrema
-                const float ws = warp_sum(usq);
-                if (lane == 0) s_usq[warp] = ws;
+        } else {
+            // ---- a tail block, or uncommon scalars: the general forms, rolled, the new second moments in place of
+            //      the consumed inputs in the ring slot ----
+            umin = 0xffffffffu;
+            umax = 0u;
+#pragma unroll 1
+            for (int mb = 0; mb < 2; ++mb) {
+                const int oa = ow + mb * FAST_MBLOCK;
+                float2 g[4], p[4], v_old[4], m_old[4], vn[4], mn[4];
+                fast_load8<GradT, ParamT, VB, MF>(st, oa, s_tab[stage], csc, cml, mb ? cms[1] : cms[0], LT, p, g, v_old, m_old);
+                if (L.negate_grad) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) g[j] = make_float2(-g[j].x, -g[j].y);
+                }
+                uint32_t real = 0u;                               // bit j: element j exists
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if ((j < 4 ? oa : oa + 124) + j < rem) real |= 1u << j;
+                fast_ema8<MF, false, PB == 2 && !SR, LAG>(S, g, v_old, m_old, p, vn, mn, real, usq);
+                float x[8], q[8];
+                uint32_t w[4] = {0u, 0u, 0u, 0u};
+                if (PB == 2) fast_round8<SR>(p, sT.sr_base, base + oa, w);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {                     // padding re-enters both states as zero
+                    if (!((real >> (2 * j)) & 1u)) { vn[j].x = 0.0f; mn[j].x = 0.0f; }
+                    if (!((real >> (2 * j + 1)) & 1u)) { vn[j].y = 0.0f; mn[j].y = 0.0f; }
+                    x[2 * j] = vn[j].x; x[2 * j + 1] = vn[j].y;
+                    q[2 * j] = p[j].x; q[2 * j + 1] = p[j].y;
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    umin = min(umin, __float_as_uint(x[j]) - 1u);
+                    umax = max(umax, __float_as_uint(x[j]));
+                    const int e = (j < 4 ? oa : oa + 124) + j;
+                    if (((real >> j) & 1u) && !bad) {
+                        if (PB == 4) {
+                            static_cast<float *>(sT.param)[base + e] = q[j];
+                            if (sT.param_copy != nullptr) static_cast<uint16_t *>(sT.param_copy)[base + e] = (uint16_t)f32_to_bf16_rn_bits(q[j]);
+                        } else {
+                            static_cast<uint16_t *>(sT.param)[base + e] = (uint16_t)(w[j >> 1] >> (16 * (j & 1)));
+                        }
+                    }
+                }
+                if (MF != AF8_M_NONE)
+                    fast_store_m<MF>(mn, sT.m_q, sT.m_scale + (int64_t)b * MPB + 2 * warp + mb, base + oa,
+                                     (2 * warp + mb) * FAST_MBLOCK < rem && !bad, lane);
+                // (this thread's own inputs: 16 bytes of fp32 parameters, or 8 of bf16 parameters and 8 of gradients, per group)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int o = oa + 128 * h;
+                    if (PB == 4) {
+                        *reinterpret_cast<float4 *>(st + P_OFF + o * 4) = make_float4(x[4 * h], x[4 * h + 1], x[4 * h + 2], x[4 * h + 3]);
+                    } else {
+                        *reinterpret_cast<float2 *>(st + P_OFF + o * 2) = make_float2(x[4 * h], x[4 * h + 1]);
+                        *reinterpret_cast<float2 *>(st + G_OFF + o * 2) = make_float2(x[4 * h + 2], x[4 * h + 3]);
+                    }
+                }
             }
+            umin = __reduce_min_sync(0xffffffffu, umin);
+            umax = __reduce_max_sync(0xffffffffu, umax);
+        }
+        if (lane == 0) { s_redmin[warp] = umin; s_redmax[warp] = umax; }
+        if (LAG) {                           // the block's sum of squares travels with the extrema
+            const float ws = warp_sum(usq);
+            if (lane == 0) s_usq[warp] = ws;
         }
         // ---- D: only warp 0 consumes the extrema; the other warps signal and move on ----
         if (warp == 0) asm volatile("bar.sync 1, %0;" ::"n"(FAST_THREADS) : "memory");
@@ -613,8 +905,8 @@ fullrank_fast_kernel(const FullrankLaunch L)
 
         // ---- warp 0: exact log2 of the two extreme values only (optimizer.py:308-318) ----
         if (warp == 0) {
-            uint32_t umin = lane < FAST_WARPS ? s_redmin[lane] : 0xffffffffu;
-            uint32_t umax = lane < FAST_WARPS ? s_redmax[lane] : 0u;
+            umin = lane < FAST_WARPS ? s_redmin[lane] : 0xffffffffu;
+            umax = lane < FAST_WARPS ? s_redmax[lane] : 0u;
             umin = __reduce_min_sync(0xffffffffu, umin);
             umax = __reduce_max_sync(0xffffffffu, umax);
             // lane 0 takes the log of the minimum, lane 1 of the maximum
@@ -626,21 +918,26 @@ fullrank_fast_kernel(const FullrankLaunch L)
                 const float mx = mx_l;
                 VRange r;
                 al_range(mn, mx, L.v_floor, r.min_log, r.scale);
-                r.k = __fdiv_rn(254.0f, r.scale);
-                r.c = -__fmul_rn(r.min_log, r.k);
-                // error bound of the estimate in code units: the hardware log2, the roundings
-                // of the estimate and those of the exact sequence it must agree with
-                const float lmax = fmaxf(fmaxf(fabsf(r.min_log), fabsf(mx)), 1.0f);
-                const float err = __fmaf_rn(__fmul_rn(lmax, LG2_REL_BOUND), r.k, 2.0e-4f);
-                r.thr = 0.5f - err;
-                // Exact path for every element of the block when the range is absurd (NaN / inf)
-                // or when some non-zero element lies below the floor (subnormal values with the
-                // default floor): the estimate path has no lower clamp and flushes subnormals.
-                if (!(r.k >= 1.0f) || L.v_floor < -126.0f || mn < L.v_floor) r.thr = -1.0f;
+                if (VB == 8) {
+                    r.k = __fdiv_rn(254.0f, r.scale);
+                    r.c = -__fmul_rn(r.min_log, r.k);
+                    // error bound of the estimate in code units: the hardware log2, the roundings
+                    // of the estimate and those of the exact sequence it must agree with
+                    const float lmax = fmaxf(fmaxf(fabsf(r.min_log), fabsf(mx)), 1.0f);
+                    const float err = __fmaf_rn(__fmul_rn(lmax, LG2_REL_BOUND), r.k, 2.0e-4f);
+                    r.thr = 0.5f - err;
+                    // Exact path for every element of the block when the range is absurd (NaN / inf)
+                    // or when some non-zero element lies below the floor (subnormal values with the
+                    // default floor): the estimate path has no lower clamp and flushes subnormals.
+                    if (!(r.k >= 1.0f) || L.v_floor < -126.0f || mn < L.v_floor) r.thr = -1.0f;
+                } else {
+                    r.k = __frcp_rn(r.scale);                    // for the quotient by the scale
+                    r.c = 0.0f; r.thr = 0.0f;
+                }
                 s_vr = r;
                 sT.v_scale[b] = r.scale;
                 sT.v_min_log[b] = r.min_log;
-                if (MODE == AF8_MODE_LAG) {
+                if (LAG) {
                     float s = 0.0f;
 #pragma unroll
                     for (int w = 0; w < FAST_WARPS; ++w) s = __fadd_rn(s, s_usq[w]);
@@ -649,94 +946,26 @@ fullrank_fast_kernel(const FullrankLaunch L)
             }
         }
 
-        // ---- parameter store ----
-        if (bad) {
-        } else if (PB == 4 && full) {
-            *reinterpret_cast<float4 *>(pa) = make_float4(p[0], p[1], p[2], p[3]);
-            *reinterpret_cast<float4 *>(pb) = make_float4(p[4], p[5], p[6], p[7]);
-        } else if (PB == 4) {
+        // ---- what does not need the range: the next block's decode table, or (AL16) this block's log2 ----
+        if (TABLE && next_staged) {
+            s_tab[stage ^ 1][tid] = al8_decode_fast((uint32_t)tid, nsc, nml, s_exp2);
+            s_tab[stage ^ 1][tid + 128] = al8_decode_fast((uint32_t)tid + 128u, nsc, nml, s_exp2);
+        }
+        float lv[TABLE ? 1 : FAST_EPT];
+        if (!TABLE && hot) {
+            uint32_t odd = 0u;                                   // subnormal second moments above the floor of 1e-38
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if (j < nva) pa[j] = p[j];
-                if (j < nvb) pb[j] = p[j + 4];
+            for (int j = 0; j < FAST_EPT; ++j) {
+                const float l = log2_lane(v[j], LT);             // (shuffles: every lane takes part)
+                lv[TABLE ? 0 : j] = v[j] > AF8_TINY ? l : AF8_LOG2_TINY;
+                if (v[j] > AF8_TINY && v[j] < 1.17549435e-38f) odd |= 1u << j;
             }
-        } else {
-            // bf16 parameters: the last rounding, to nearest or stochastic (optimizer.py:873-881)
-            uint32_t w[4];
-            if (L.sr) {
-                uint32_t h[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    h[j] = sr_bf16_bits(p[j], sr_bits24(sT.sr_base, (uint64_t)(base + ((j < 4) ? oa + j : ob + j - 4))));
-#pragma unroll
-                for (int j = 0; j < 4; ++j) w[j] = h[2 * j] | (h[2 * j + 1] << 16);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) w[j] = bf16x2_rn(p[2 * j], p[2 * j + 1]);
-            }
-            if (full) {
-                *reinterpret_cast<uint2 *>(pa) = make_uint2(w[0], w[1]);
-                *reinterpret_cast<uint2 *>(pb) = make_uint2(w[2], w[3]);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const uint32_t ha = (j & 1) ? (w[j >> 1] >> 16) : (w[j >> 1] & 0xffffu);
-                    const uint32_t hb = (j & 1) ? (w[2 + (j >> 1)] >> 16) : (w[2 + (j >> 1)] & 0xffffu);
-                    if (j < nva) pa[j] = (PElem)ha;
-                    if (j < nvb) pb[j] = (PElem)hb;
-                }
+#pragma unroll 1
+            for (; odd; odd &= odd - 1u) {
+                const int j = __ffs((int)odd) - 1;
+                put(lv, j, log2_cr_fast(pick(v, j), s_log2));
             }
         }
-
-        // ---- optional bf16 compute copy of the fp32 parameter (round to nearest) ----
-        if (PB == 4 && !bad && sT.param_copy != nullptr) {
-            uint16_t *ca = static_cast<uint16_t *>(sT.param_copy) + base + oa;
-            uint16_t *cb = static_cast<uint16_t *>(sT.param_copy) + base + ob;
-            if (full) {
-                *reinterpret_cast<uint2 *>(ca) = make_uint2(bf16x2_rn(p[0], p[1]), bf16x2_rn(p[2], p[3]));
-                *reinterpret_cast<uint2 *>(cb) = make_uint2(bf16x2_rn(p[4], p[5]), bf16x2_rn(p[6], p[7]));
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if (j < nva) ca[j] = (uint16_t)f32_to_bf16_rn_bits(p[j]);
-                    if (j < nvb) cb[j] = (uint16_t)f32_to_bf16_rn_bits(p[j + 4]);
-                }
-            }
-        }
-
-        // ---- momentum requantisation: one warp = one M block (optimizer.py:510, 518) ----
-        {
-            float amx = 0.0f;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) amx = fmaxf(amx, fabsf(m[j]));
-            // non-negative floats order like their bit patterns: one REDUX instead of a shuffle tree
-            const float am = fmaxf(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amx))), 1e-12f);
-            const float2 ra2 = bc2(__frcp_rn(am)), nam2 = bc2(-am);
-            uint32_t raw[8];
-#pragma unroll
-            for (int j = 0; j < 8; j += 2) {
-                // IEEE m / am from the correctly rounded reciprocal and one residual step
-                const float2 mj = make_float2(m[j], m[j + 1]);
-                float2 q = __fmul2_rn(mj, ra2);
-                const float2 r = __ffma2_rn(q, nam2, mj);
-                q = __ffma2_rn(r, ra2, q);
-                // round(q * 128) (the product is exact); |q| <= 1, so only +128 needs the clamp to 127
-                const float2 kf = __ffma2_rn(q, bc2(128.0f), bc2(AF8_MAGIC_F));
-                raw[j] = (uint32_t)min(__float_as_int(kf.x), AF8_MAGIC_I + 127);
-                raw[j + 1] = (uint32_t)min(__float_as_int(kf.y), AF8_MAGIC_I + 127);
-            }
-            // low bytes hold k mod 256; k + 128 is that byte with its top bit flipped
-            const uint32_t o0 = __byte_perm(__byte_perm(raw[0], raw[1], 0x0040), __byte_perm(raw[2], raw[3], 0x0040), 0x5410) ^ 0x80808080u;
-            const uint32_t o1 = __byte_perm(__byte_perm(raw[4], raw[5], 0x0040), __byte_perm(raw[6], raw[7], 0x0040), 0x5410) ^ 0x80808080u;
-            if (m_exists && !bad) {
-                *reinterpret_cast<uint32_t *>(sT.m_q + base + oa) = o0;
-                *reinterpret_cast<uint32_t *>(sT.m_q + base + ob) = o1;
-                if (lane == 0) sT.m_scale[b * (FAST_VBLOCK / FAST_MBLOCK) + warp] = am;
-            }
-        }
-
-        // ---- decode table of the next block, while warp 0 finishes the range ----
-        if (next_staged) s_tab[stage ^ 1][tid] = al8_decode_fast((uint32_t)tid, nsc, nml, s_exp2);
         __syncthreads();                     // ---- E ----
         if (s_abort) {       // a copy never completed: give the ones still in flight a bounded chance, then stop
             for (int k = 1; k < in_flight; ++k) mbar_wait_bounded(&s_full[(n + k) % NST], (phase >> ((n + k) % NST)) & 1u);
@@ -744,45 +973,85 @@ fullrank_fast_kernel(const FullrankLaunch L)
         }
 
         // ---- second-moment codes ----
-        {
-            const VRange r = s_vr;
-            int kk[8];
-            float dd[8];
-            float dmax = 0.0f;
+        const VRange r = s_vr;
+        if (!hot) {
+            // the exact sequence for every element, from the values left in the ring slot
+#pragma unroll 1
+            for (int q = 0; q < FAST_EPT; ++q) {
+                const int o = ow + (q >> 2) * 128, k = q & 3;
+                const float x = PB == 4 ? reinterpret_cast<const float *>(st + P_OFF)[o + k]
+                                        : reinterpret_cast<const float *>(st + (k < 2 ? P_OFF : G_OFF) + o * 2)[k & 1];
+                const uint32_t c = al_encode(x, al_log2_fast(x, s_log2), r.min_log, r.scale, QM1, QMAX);
+                if (VB == 8) static_cast<uint8_t *>(sT.v_q)[base + o + k] = (uint8_t)c;
+                else static_cast<uint16_t *>(sT.v_q)[base + o + k] = (uint16_t)c;
+            }
+            __syncthreads();             // the slot may be refilled from the next iteration on
+        } else if (VB == 8) {
+            uint8_t *const vp = static_cast<uint8_t *>(sT.v_q) + base;
             const float2 k2 = bc2(r.k), c2 = bc2(r.c), mg2 = bc2(AF8_MAGIC_F + 1.0f), nmg2 = bc2(-(AF8_MAGIC_F + 1.0f));
 #pragma unroll
-            for (int j = 0; j < 8; j += 2) {
-                // An exact zero estimates as -inf: te and sm are -inf, whose low byte is 0, the
-                // reserved code, and d is NaN, which the tests below ignore.  Every other element
-                // of a block that takes this path is a normal number at or above min_log, so
-                // 0 <= t <= 254 up to the estimate's error and no clamp is needed.
-                const float2 le = make_float2(lg2_approx(v[j]), lg2_approx(v[j + 1]));
-                const float2 te = __ffma2_rn(le, k2, c2);
-                const float2 sm = __fadd2_rn(te, mg2);             // rint(te) + 1 in the low bits
-                const float2 rf = __fadd2_rn(sm, nmg2);
-                const float2 d = sub2(te, rf);                     // distance to the chosen integer
-                dd[j] = d.x; dd[j + 1] = d.y;
-                dmax = fmaxf(dmax, fmaxf(fabsf(d.x), fabsf(d.y)));   // fmaxf drops NaN
-                kk[j] = __float_as_int(sm.x); kk[j + 1] = __float_as_int(sm.y);
-            }
-            if (__any_sync(0xffffffffu, dmax > r.thr)) {
-                // rare: redo the codes in doubt (and the zeros of this thread) with the exact sequence
+            for (int mb = 0; mb < 2; ++mb) {
+                float x[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    if (!(fabsf(dd[j]) <= r.thr))
-                        kk[j] = AF8_MAGIC_I + (int)al_encode(v[j], al_log2_fast(v[j], s_log2), r.min_log, r.scale, 254.0f, 255);
-            }
-            uint32_t raw[8];
+                for (int j = 0; j < 8; ++j) x[j] = v[8 * mb + j];
+                uint32_t kk[8];
+                float dd[8];
+                float dmax = 0.0f;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) raw[j] = (uint32_t)kk[j];
-            const uint32_t o0 = __byte_perm(__byte_perm(raw[0], raw[1], 0x0040), __byte_perm(raw[2], raw[3], 0x0040), 0x5410);
-            const uint32_t o1 = __byte_perm(__byte_perm(raw[4], raw[5], 0x0040), __byte_perm(raw[6], raw[7], 0x0040), 0x5410);
-            uint8_t *vp = static_cast<uint8_t *>(sT.v_q) + base;
-            *reinterpret_cast<uint32_t *>(vp + oa) = o0;       // (not reached after a failed wait: the CTA left at E)
-            *reinterpret_cast<uint32_t *>(vp + ob) = o1;
+                for (int j = 0; j < 8; j += 2) {
+                    // An exact zero estimates as -inf: te and sm are -inf, whose low byte is 0, the
+                    // reserved code, and d is NaN, which the tests below ignore.  Every other element
+                    // of a block that takes this path is a normal number at or above min_log, so
+                    // 0 <= t <= 254 up to the estimate's error and no clamp is needed.
+                    const float2 le = make_float2(lg2_approx(x[j]), lg2_approx(x[j + 1]));
+                    const float2 te = __ffma2_rn(le, k2, c2);
+                    const float2 sm = __fadd2_rn(te, mg2);             // rint(te) + 1 in the low bits
+                    const float2 rf = __fadd2_rn(sm, nmg2);
+                    const float2 d = sub2(te, rf);                     // distance to the chosen integer
+                    dd[j] = d.x; dd[j + 1] = d.y;
+                    dmax = max3(dmax, fabsf(d.x), fabsf(d.y));         // (drops NaN)
+                    kk[j] = __float_as_uint(sm.x); kk[j + 1] = __float_as_uint(sm.y);
+                }
+                if (dmax > r.thr) {
+                    // rare: redo the codes in doubt with the exact sequence (an exact zero's distance is NaN and its code 0)
+                    uint32_t odd = 0u;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (!(fabsf(dd[j]) <= r.thr)) odd |= 1u << j;
+#pragma unroll 1
+                    for (; odd; odd &= odd - 1u) {
+                        const int j = __ffs((int)odd) - 1;
+                        const float y = pick(x, j);
+                        put(kk, j, (uint32_t)AF8_MAGIC_I + al_encode(y, al_log2_fast(y, s_log2), r.min_log, r.scale, QM1, QMAX));
+                    }
+                }
+                *reinterpret_cast<uint32_t *>(vp + ow + mb * FAST_MBLOCK) = pack4(kk[0], kk[1], kk[2], kk[3]);       // (not reached after a failed wait: the CTA left at E)
+                *reinterpret_cast<uint32_t *>(vp + ow + mb * FAST_MBLOCK + 128) = pack4(kk[4], kk[5], kk[6], kk[7]);
+            }
+        } else {
+            uint16_t *const vp = static_cast<uint16_t *>(sT.v_q) + base;
+            const float2 nml2 = bc2(-r.min_log), rc2 = bc2(r.k), nd2 = bc2(-r.scale);
+#pragma unroll
+            for (int q = 0; q < FAST_EPT / 4; ++q) {
+                uint32_t kk[4];
+#pragma unroll
+                for (int j = 0; j < 4; j += 2) {
+                    // al_encode on a pair: (l - min_log) / scale * 65534, rounded, plus one (optimizer.py:320-321)
+                    const int i = TABLE ? 0 : 4 * q + j;
+                    const float2 d = __fadd2_rn(make_float2(lv[i], lv[TABLE ? 0 : i + 1]), nml2);
+                    const float2 t = div2_by(d, rc2, nd2);
+                    // (scalar: the compiler fuses a packed product into a packed sum, which loses the rounding in between)
+                    const int k0 = __float_as_int(__fadd_rn(__fmul_rn(t.x, QM1), AF8_MAGIC_F)) - (AF8_MAGIC_I - 1);
+                    const int k1 = __float_as_int(__fadd_rn(__fmul_rn(t.y, QM1), AF8_MAGIC_F)) - (AF8_MAGIC_I - 1);
+                    kk[j] = v[4 * q + j] == 0.0f ? 0u : (uint32_t)max(1, min(k0, QMAX));
+                    kk[j + 1] = v[4 * q + j + 1] == 0.0f ? 0u : (uint32_t)max(1, min(k1, QMAX));
+                }
+                *reinterpret_cast<uint2 *>(vp + ow + q * 128) = make_uint2(kk[0] | (kk[1] << 16), kk[2] | (kk[3] << 16));
+            }
         }
         staged = next_staged;
-        mscale_cur = nms;
+        csc = nsc; cml = nml;
+        cms[0] = nms[0]; cms[1] = nms[1];
     }
 }
 

@@ -1,5 +1,5 @@
-// Statistic pass of the AdamW UF8/AL8 configuration: per V block, the sum of squares of
-// the update u = m_new / (sqrt(v_new) + eps) that the APPLY pass is going to use
+// Statistic pass of the specialised full-rank configurations (fullrank_fast.cuh): per V block, the
+// sum of squares of the update u = m_new / (sqrt(v_new) + eps) that the APPLY pass is going to use
 // (first pass of the NORM -> APPLY structure, optimizer.py:1048-1077).
 //
 // Nothing computed here reaches a stored state: the sums only produce the norm that
@@ -14,7 +14,9 @@
 // Per element: 2 special-function operations (sqrt, reciprocal) plus 1/8 for the table; the
 // special-function pipe was the busiest unit with the decode per element (3 operations,
 // 70 % busy): the table took the pass from 1.04 to 0.93 ms on the TinyLlama set.
-// (Replacing the reciprocal by rsqrt and a short series was measured slower.)
+// (Replacing the reciprocal by rsqrt and a short series was measured slower; so were requests for the
+// next block's lines in L2, 0.972 against 0.955 ms.)  AL16 has too many codes for a table: an element
+// costs one exp2 more.
 #pragma once
 
 #include "common.cuh"
@@ -28,9 +30,6 @@ constexpr int STAT_THREADS = 256;
 #endif
 #ifndef AF8_STAT_UNROLL
 #define AF8_STAT_UNROLL 4
-#endif
-#ifndef AF8_STAT_PREFETCH
-#define AF8_STAT_PREFETCH 0      /* measured on the TinyLlama set: 0.972 ms with the requests, 0.955 ms without */
 #endif
 #define AF8_PRAGMA_(x) _Pragma(#x)
 #define AF8_UNROLL_(n) AF8_PRAGMA_(unroll n)
@@ -63,13 +62,15 @@ __device__ __forceinline__ void stat_load_g<bf16_tag>(const void *grad, int64_t 
     g[6] = __uint_as_float(a.w << 16); g[7] = __uint_as_float(a.w & 0xffff0000u);
 }
 
-template <typename GradT>
+template <typename GradT, int VB, int MF>
 __global__ void __launch_bounds__(STAT_THREADS, AF8_STAT_MIN_CTAS)
 fullrank_stat_kernel(const FullrankLaunch L)
 {
     // per-warp decode table of the block's 256 second-moment codes: 8 exponentials per lane and block
     // instead of 64 (the special-function pipe is the busiest unit of this pass); entry 0 is exact zero
-    __shared__ float s_dec[STAT_THREADS / 32][256];
+    constexpr bool TABLE = VB == 8;
+    constexpr float M_UNIT = MF == AF8_M_UF4 ? 0.125f : 0.0078125f;
+    __shared__ float s_dec[STAT_THREADS / 32][TABLE ? 256 : 1];
     const int lane = threadIdx.x & 31;
     float *const dec = s_dec[threadIdx.x >> 5];
     const int64_t warps = (int64_t)gridDim.x * (STAT_THREADS / 32);
@@ -80,7 +81,7 @@ fullrank_stat_kernel(const FullrankLaunch L)
     const void *grad = nullptr;
     const uint8_t *mq = nullptr, *vq = nullptr;
     const float *m_scale = nullptr, *v_scale = nullptr, *v_min_log = nullptr;
-    float v_w = 0.f, m_w = 0.f, eps_d = 0.f, eps_g = 0.f, v_wm1 = 0.f, m_wm1 = 0.f;
+    float v_w = 0.f, m_w = 0.f, eps_d = 0.f, eps_g = 0.f;
     bool small_w = true;
 
     for (int64_t blk = w0; blk < L.total_blocks; blk += warps) {
@@ -94,44 +95,29 @@ fullrank_stat_kernel(const FullrankLaunch L)
             grad = T->grad;
             mq = T->m_q; vq = static_cast<const uint8_t *>(T->v_q);
             m_scale = T->m_scale; v_scale = T->v_scale; v_min_log = T->v_min_log;
-            v_w = __ldg(&T->v_w); m_w = __ldg(&T->m_w);
+            v_w = __ldg(&T->v_w); m_w = MF == AF8_M_NONE ? 0.0f : __ldg(&T->m_w);
             eps_d = __ldg(&T->eps_denom); eps_g = __ldg(&T->eps_gradsq);
-            v_wm1 = __fsub_rn(v_w, 1.0f); m_wm1 = __fsub_rn(m_w, 1.0f);
             small_w = fabsf(v_w) < 0.5f && fabsf(m_w) < 0.5f;
         }
         const int64_t b = blk - cur_first;
         const int64_t base = b * FAST_VBLOCK;
         const int64_t rem = numel - base;
-#if AF8_STAT_PREFETCH
-        // Optional: ask L2 for this warp's next block (same tensor, a full block) while this one is worked
-        // on: the gradient is 32 lines of 128 bytes (one per lane), the two code arrays 16 lines each.
-        {
-            const int64_t nb = b + warps;
-            if (blk + warps < cur_end && (nb + 1) * FAST_VBLOCK <= numel) {
-                const int64_t nbase = nb * FAST_VBLOCK;
-                constexpr int GBYTES = std::is_same<GradT, float>::value ? 4 : 2;
-                const char *gp = static_cast<const char *>(grad) + nbase * GBYTES;
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(gp + lane * 128));
-                if (GBYTES == 4) asm volatile("prefetch.global.L2 [%0];" ::"l"(gp + 4096 + lane * 128));
-                const uint8_t *cp = (lane < 16 ? mq : vq) + nbase + (lane & 15) * 128;
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(cp));
-            }
-        }
-#endif
-        // decode v = 2^((code-1)*scale/254 + min_log) as 2^(code*a + c)
+        // decode v = 2^((code-1)*scale/levels + min_log) as 2^(code*a + c)
         const float sc = __ldg(v_scale + b), ml = __ldg(v_min_log + b);
-        const float a = sc * (1.0f / 254.0f);
+        const float a = sc * (VB == 16 ? 1.0f / 65534.0f : 1.0f / 254.0f);
         const float c = ml - a;
         float acc = 0.0f;
 
         if (rem >= FAST_VBLOCK && small_w) {
-            __syncwarp();                                   // the previous block's look-ups are done
+            if (TABLE) {
+                __syncwarp();                                   // the previous block's look-ups are done
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const int code = lane + 32 * k;
-                dec[code] = code ? ex2_approx(__fmaf_rn((float)code, a, c)) : 0.0f;
+                for (int k = 0; k < 8; ++k) {
+                    const int code = lane + 32 * k;
+                    dec[code] = code ? ex2_approx(__fmaf_rn((float)code, a, c)) : 0.0f;
+                }
+                __syncwarp();
             }
-            __syncwarp();
             const float2 wv2 = bc2(v_w), wm2 = bc2(m_w), ed2 = bc2(eps_d);
             float2 acc2 = make_float2(0.0f, 0.0f);
 AF8_UNROLL_(AF8_STAT_UNROLL)
@@ -143,22 +129,46 @@ AF8_UNROLL_(AF8_STAT_UNROLL)
 #pragma unroll
                     for (int j = 0; j < 8; ++j) g[j] = -g[j];
                 }
-                const uint2 mw = __ldcs(reinterpret_cast<const uint2 *>(mq + off));
-                const uint2 vw = __ldcs(reinterpret_cast<const uint2 *>(vq + off));
-                const float2 mc2 = bc2(__ldg(m_scale + b * (FAST_VBLOCK / FAST_MBLOCK) + s) * 0.0078125f);
+                uint2 mw = make_uint2(0u, 0u);
+                uint32_t vw[VB / 4];
+                if (MF == AF8_M_UF8) mw = __ldcs(reinterpret_cast<const uint2 *>(mq + off));
+                if (MF == AF8_M_UF4) mw.x = __ldcs(reinterpret_cast<const uint32_t *>(mq + off / 2));
+                if (VB == 8) {
+                    const uint2 w = __ldcs(reinterpret_cast<const uint2 *>(vq + off));
+                    vw[0] = w.x; vw[1] = w.y;
+                } else {
+                    const uint4 w = __ldcs(reinterpret_cast<const uint4 *>(vq + off * 2));
+                    vw[0] = w.x; vw[1] = w.y; vw[VB / 4 - 2] = w.z; vw[VB / 4 - 1] = w.w;
+                }
+                const float2 mc2 = bc2(MF == AF8_M_NONE ? 0.0f : __ldg(m_scale + b * (FAST_VBLOCK / FAST_MBLOCK) + s) * M_UNIT);
 #pragma unroll
                 for (int j = 0; j < 8; j += 2) {
-                    const uint32_t mword = (j < 4) ? mw.x : mw.y, vword = (j < 4) ? vw.x : vw.y;
                     const float2 gj = make_float2(g[j], g[j + 1]);
                     float2 g2 = __fmul2_rn(gj, gj);
                     if (eps_g != 0.0f) g2 = __fadd2_rn(g2, bc2(eps_g));
-                    const float2 v_old = make_float2(dec[__byte_perm(vword, 0u, 0x4440u | (uint32_t)(j & 3))],
-                                                     dec[__byte_perm(vword, 0u, 0x4440u | (uint32_t)((j + 1) & 3))]);
+                    float2 v_old;
+                    if (VB == 8) {
+                        v_old = make_float2(dec[TABLE ? __byte_perm(vw[j >> 2], 0u, 0x4440u | (uint32_t)(j & 3)) : 0u],
+                                            dec[TABLE ? __byte_perm(vw[j >> 2], 0u, 0x4440u | (uint32_t)((j + 1) & 3)) : 0u]);
+                    } else {
+                        const uint32_t w = vw[(j >> 1) & (VB / 4 - 1)];
+                        const float2 cd = __fadd2_rn(make_float2(__uint_as_float(0x4b000000u | (w & 0xffffu)), __uint_as_float(0x4b000000u | (w >> 16))), bc2(-8388608.0f));
+                        const float2 tt = __ffma2_rn(cd, bc2(a), bc2(c));
+                        v_old = make_float2((w & 0xffffu) ? ex2_approx(tt.x) : 0.0f, (w >> 16) ? ex2_approx(tt.y) : 0.0f);
+                    }
                     const float2 vj = __ffma2_rn(wv2, sub2(g2, v_old), v_old);
-                    const float2 mb = make_float2(__uint_as_float(__byte_perm(mword, 0x4b000000u, 0x7540u | (uint32_t)(j & 3))),
-                                                  __uint_as_float(__byte_perm(mword, 0x4b000000u, 0x7540u | (uint32_t)((j + 1) & 3))));
-                    const float2 m_old = __fmul2_rn(__fadd2_rn(mb, bc2(-8388736.0f)), mc2);
-                    const float2 mj = __ffma2_rn(wm2, sub2(gj, m_old), m_old);
+                    float2 mj = gj;
+                    if (MF == AF8_M_UF8) {
+                        const uint32_t mword = (j < 4) ? mw.x : mw.y;
+                        const float2 mb = make_float2(__uint_as_float(__byte_perm(mword, 0x4b000000u, 0x7540u | (uint32_t)(j & 3))),
+                                                      __uint_as_float(__byte_perm(mword, 0x4b000000u, 0x7540u | (uint32_t)((j + 1) & 3))));
+                        const float2 m_old = __fmul2_rn(__fadd2_rn(mb, bc2(-8388736.0f)), mc2);
+                        mj = __ffma2_rn(wm2, sub2(gj, m_old), m_old);
+                    } else if (MF == AF8_M_UF4) {                      // byte j / 2, the even element in its high nibble
+                        const float2 mb = make_float2(__uint_as_float(0x4b000000u | ((mw.x >> (4 * j + 4)) & 15u)), __uint_as_float(0x4b000000u | ((mw.x >> (4 * j)) & 15u)));
+                        const float2 m_old = __fmul2_rn(__fadd2_rn(mb, bc2(-8388616.0f)), mc2);
+                        mj = __ffma2_rn(wm2, sub2(gj, m_old), m_old);
+                    }
                     const float2 den = __fadd2_rn(make_float2(sqrt_approx(vj.x), sqrt_approx(vj.y)), ed2);
                     const float2 u = __fmul2_rn(mj, make_float2(rcp_approx(den.x), rcp_approx(den.y)));
                     acc2 = __ffma2_rn(u, u, acc2);
@@ -173,11 +183,14 @@ AF8_UNROLL_(AF8_STAT_UNROLL)
                 float gj = GradLoad<GradT>::load1(grad, e);
                 if (L.negate_grad) gj = -gj;
                 const float g2 = __fadd_rn(__fmul_rn(gj, gj), eps_g);
-                const uint32_t code = vq[e];
+                const uint32_t code = VB == 16 ? reinterpret_cast<const uint16_t *>(vq)[e] : vq[e];
                 const float v_old = code ? ex2_approx(__fmaf_rn((float)code, a, c)) : 0.0f;
                 const float vj = lerp_t(v_old, g2, v_w);
-                const float m_old = __fmul_rn((float)((int)mq[e] - 128), __ldg(m_scale + e / FAST_MBLOCK) * 0.0078125f);
-                const float mj = lerp_t(m_old, gj, m_w);
+                float mj = gj;
+                if (MF != AF8_M_NONE) {
+                    const int k = MF == AF8_M_UF8 ? (int)mq[e] - 128 : (int)((e & 1) ? (mq[e >> 1] & 15u) : (mq[e >> 1] >> 4)) - 8;
+                    mj = lerp_t(__fmul_rn((float)k, __ldg(m_scale + e / FAST_MBLOCK) * M_UNIT), gj, m_w);
+                }
                 const float u = __fmul_rn(mj, rcp_approx(__fadd_rn(sqrt_approx(vj), eps_d)));
                 acc = __fmaf_rn(u, u, acc);
             }
@@ -185,7 +198,6 @@ AF8_UNROLL_(AF8_STAT_UNROLL)
         acc = warp_sum(acc);
         if (lane == 0) L.block_sumsq[blk] = acc;
     }
-    (void)v_wm1; (void)m_wm1;
 }
 
 }  // namespace af8

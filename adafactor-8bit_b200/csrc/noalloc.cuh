@@ -159,12 +159,14 @@ extern "C" int af8_fullrank_limited_step_noalloc(const af8_fullrank_cfg *cfg, co
     L.param_dtype = AF8_F32;
     L.sr = 0;
     GenericCfg C{c.v_fmt, c.m_fmt, c.block, c.m_block, c.use_adam_denom ? 1 : 0, 0};
-    const bool fast = c.v_fmt == AF8_V_AL8 && c.m_fmt == AF8_M_UF8 && c.block == FAST_VBLOCK &&
-                      c.m_block == FAST_MBLOCK && c.use_adam_denom;
     const bool bf16 = c.grad_dtype == AF8_BF16;
 
     auto pass = [&](int mode) {
-        if (fast) return bf16 ? dispatch_fast<bf16_tag, float>(mode, L, st) : dispatch_fast<float, float>(mode, L, st);
+        af8_fullrank_cfg cm = c;
+        cm.mode = mode;
+        cm.param_dtype = AF8_F32;
+        cm.stochastic_round = 0;
+        if (fast_covers(cm)) return dispatch_fast(cm, L, st);
         return bf16 ? dispatch_generic<bf16_tag>(mode, L, C, st) : dispatch_generic<float>(mode, L, C, st);
     };
     rc = pass(AF8_MODE_SUMSQ);
