@@ -624,8 +624,11 @@ class FactoredPlan:
         self.numel = self.rows * self.cols
         self.full_numel = self.full_rows * self.cols
         self.total_numel = int(self.numel.sum())
-        # (batches of matrices take the general kernels; the optimizer keeps them in plans of their own)
+        # 1: whole vectors of 8; else 2 (batches of matrices, rows of any length >= 8) where a step's arrays lie on
+        # 16-byte boundaries, 0 (the general kernels) where they do not (see stages)
         self.cfg.aligned8 = int(bool((self.cols % 8 == 0).all()) and not bool((self.batch > 1).any()))
+        self._any_rows = (self.cfg.aligned8 == 0 and bool((self.cols >= 8).all()) and bool((self.rows < 1 << 31).all())
+                          and (m_fmt in (None, "fp32") or self.cfg.m_block == 256) and grad_dtype != torch.float16)
         lib = N.lib()
         m_quant = m_fmt not in (None, "fp32")
         self.chunk = lib.af8_factored_chunk(self.cfg.m_block if m_quant else 0)
@@ -734,6 +737,7 @@ class FactoredPlan:
             if k == self.n_tables - 1:
                 self.small_units = int(units.sum())
         self._sums_off = self._running(self._vec_len)
+        self._static_aligned = not any((t[0][name] & np.uint64(15)).any() for name in ("param", "m_q", "m_f32", "param_copy"))
         return t
 
     def kernel_name(self, what):
@@ -846,6 +850,8 @@ class FactoredPlan:
         tables[:] = self._static
         table = tables[0]
         table["grad"] = [g.data_ptr() for g in grads]
+        if self._any_rows:
+            self.cfg.aligned8 = 2 if self._static_aligned and not (table["grad"] & np.uint64(15)).any() else 0
         for k in ("decay", "alpha", "v_w", "m_w", "c_w", "eps1", "eps_came"):
             table[k] = scalars[k]
         table["sr_base"] = scalars.get("sr_base", 0)

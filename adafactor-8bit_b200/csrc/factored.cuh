@@ -45,6 +45,7 @@ struct FactoredLaunch {
     int32_t grad_dtype, m_fmt, m_block, came, negate_grad, mode;
     float v_floor;
     int32_t param_dtype, sr;
+    int32_t split;               // tile kernels: a unit is the (1 << split)-th part of a tile (see tile_split)
 };
 
 __device__ __forceinline__ int find_factored_tile(const af8_factored_tensor *t, int n, int64_t id)
@@ -77,6 +78,42 @@ __host__ __device__ __forceinline__ int64_t fact_tiles(const af8_factored_tensor
 __device__ __forceinline__ int64_t fact_col_base(const af8_factored_tensor &t, int64_t row)
 {
     return t.batch_rows > 0 ? (row / t.batch_rows) * t.cols : 0;
+}
+
+// Unit `id` of a launch over the tiles (L.split applied) of tensor T: its rows r0 .. r_end - 1 (of the flattened
+// batch), its first column and the first entry of its matrix's part of the column arrays.
+struct TilePos { int64_t r0, r_end, c0, cb; };
+__device__ __forceinline__ TilePos tile_pos(const FactoredLaunch &L, const af8_factored_tensor &T, int64_t id)
+{
+    TilePos p;
+    const int64_t ntc = (T.cols + FSTAT_COLS - 1) / FSTAT_COLS;
+    int64_t local = (id >> L.split) - T.first_tile, first = 0, end = T.rows;
+    p.cb = 0;
+    if (T.batch_rows > 0) {                                          // a tile lies inside one matrix of a batch
+        const int64_t tpm = ((T.batch_rows + FSTAT_ROWS - 1) / FSTAT_ROWS) * ntc;
+        const int64_t mat = local / tpm;
+        local -= mat * tpm;
+        first = mat * T.batch_rows;
+        end = first + T.batch_rows;
+        p.cb = mat * T.cols;
+    }
+    const int64_t tr = local / ntc;
+    const int part_rows = FSTAT_ROWS >> L.split, part = (int)(id & (((int64_t)1 << L.split) - 1));
+    p.c0 = (local - tr * ntc) * FSTAT_COLS;
+    p.r0 = first + tr * FSTAT_ROWS + part * part_rows;
+    p.r_end = min(end, p.r0 + (int64_t)part_rows);                   // (an empty part: r_end <= r0)
+    return p;
+}
+
+// Parts per tile, as a power of two: a 512-row tile is 131072 elements, so a small table has fewer tiles than the
+// chip has resident CTAs (444 to 592) and its last wave is most of its time.  Tiles are halved, down to 64 rows,
+// while they give less than about eight waves of half-used SMs; smaller parts only add column atomics (256 per part).
+// 8 layers of 512 x 1376 with CAME, 256 tiles: see factored_stats_vec_kernel for the times.
+inline int tile_split(int64_t tiles)
+{
+    int sh = 0;
+    while (sh < 3 && (tiles << sh) < 1776) ++sh;
+    return sh;
 }
 
 __device__ __forceinline__ float load_grad_any(const void *g, int dtype, int64_t i)
@@ -252,6 +289,18 @@ factored_stats_kernel(const FactoredLaunch L)
         __syncthreads();
         if (c0 + tid < C) atomicAdd(sT.col_sum + cb + c0 + tid, s_col[tid]);
     }
+}
+
+// grid (n_tensors, slices): zero the row and column sums of every tensor
+__global__ void __launch_bounds__(256)
+factored_clear_kernel(const af8_factored_tensor *tensors)
+{
+    const af8_factored_tensor &T = tensors[blockIdx.x];
+    const int64_t stride = (int64_t)blockDim.x * gridDim.y, first = (int64_t)blockIdx.y * blockDim.x + threadIdx.x;
+    const int64_t nr = T.rows, nc = fact_batch(T) * T.cols;
+    double *const rs = T.row_sum, *const cs = T.col_sum;
+    for (int64_t i = first; i < nr; i += stride) rs[i] = 0.0;
+    for (int64_t i = first; i < nc; i += stride) cs[i] = 0.0;
 }
 
 // ---------------------------------------------------------------------------
@@ -556,6 +605,14 @@ template <> struct GradRaw8<float> {
         const float4 *p = reinterpret_cast<const float4 *>(static_cast<const float *>(grad) + off);
         a = __ldcs(p); b = __ldcs(p + 1);
     }
+    __device__ __forceinline__ void load_part(const void *grad, int64_t off, int n)       // the first n (< 8), zeros after them
+    {
+        const float *p = static_cast<const float *>(grad) + off;
+        float x[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j] = j < n ? p[j] : 0.0f;
+        a = make_float4(x[0], x[1], x[2], x[3]); b = make_float4(x[4], x[5], x[6], x[7]);
+    }
     __device__ __forceinline__ void from_shared(const unsigned char *p)
     {
         a = *reinterpret_cast<const float4 *>(p); b = *reinterpret_cast<const float4 *>(p + 16);
@@ -575,6 +632,14 @@ template <> struct GradRaw8<bf16_tag> {
     __device__ __forceinline__ void load(const void *grad, int64_t off)
     {
         a = __ldcs(reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(grad) + off));
+    }
+    __device__ __forceinline__ void load_part(const void *grad, int64_t off, int n)       // the first n (< 8), zeros after them
+    {
+        const uint16_t *p = static_cast<const uint16_t *>(grad) + off;
+        uint32_t x[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j] = j < n ? p[j] : 0u;
+        a = make_uint4(x[0] | (x[1] << 16), x[2] | (x[3] << 16), x[4] | (x[5] << 16), x[6] | (x[7] << 16));
     }
     __device__ __forceinline__ void from_shared(const unsigned char *p) { a = *reinterpret_cast<const uint4 *>(p); }
     __device__ __forceinline__ void unpack(int negate, float (&g)[8]) const
@@ -622,27 +687,163 @@ __device__ __forceinline__ void m_old8(const af8_factored_tensor &T, int m_fmt, 
     }
 }
 
+// 8 consecutive gradient elements from an offset of any alignment, for rows whose length is no multiple of 8.  A lane's
+// columns stay the same from row to row, so the offset moves by the row length; bf16: the two aligned 16-byte vectors
+// around the elements are loaded (the lanes' vectors overlap: the second comes from L1) and shifted when they are
+// used, so that the loads of several rows are in flight together.  Nothing at or beyond element `numel` is read.
+template <typename GradT> struct GradAny8;
+template <> struct GradAny8<bf16_tag> {
+    uint4 a, b;
+    int s;
+    __device__ __forceinline__ static uint4 vec(const uint16_t *p, int64_t off, int64_t numel)
+    {
+        if (off + 8 <= numel) return __ldg(reinterpret_cast<const uint4 *>(p + off));
+        GradRaw8<bf16_tag> t;
+        t.load_part(p, off, (int)(numel - off));                 // (none for a negative count)
+        return t.a;
+    }
+    __device__ __forceinline__ void zero() { a = b = make_uint4(0u, 0u, 0u, 0u); s = 0; }
+    __device__ __forceinline__ void load(const void *grad, int64_t off, int64_t numel)
+    {
+        const uint16_t *p = static_cast<const uint16_t *>(grad);
+        s = (int)(off & 7);
+        a = vec(p, off - s, numel);
+        b = s ? vec(p, off - s + 8, numel) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    __device__ __forceinline__ void unpack(int negate, float (&g)[8]) const
+    {
+        uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        if (s & 4) {
+#pragma unroll
+            for (int i = 0; i < 6; ++i) w[i] = w[i + 2];
+        }
+        if (s & 2) {
+#pragma unroll
+            for (int i = 0; i < 5; ++i) w[i] = w[i + 1];
+        }
+        GradRaw8<bf16_tag> t;
+        const uint32_t sh = (s & 1) * 16;
+        t.a = make_uint4(__funnelshift_r(w[0], w[1], sh), __funnelshift_r(w[1], w[2], sh), __funnelshift_r(w[2], w[3], sh), __funnelshift_r(w[3], w[4], sh));
+        t.unpack(negate, g);
+    }
+};
+template <> struct GradAny8<float> {
+    float v[8];
+    __device__ __forceinline__ void zero()
+    {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = 0.0f;
+    }
+    __device__ __forceinline__ void load(const void *grad, int64_t off, int64_t numel)
+    {
+        const float *p = static_cast<const float *>(grad) + off;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = off + j < numel ? __ldg(p + j) : 0.0f;
+    }
+    __device__ __forceinline__ void unpack(int negate, float (&g)[8]) const
+    {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) g[j] = negate ? -v[j] : v[j];
+    }
+};
+
+// old momentum of 8 consecutive elements at any offset: the run may end one momentum block and begin the next
+__device__ __forceinline__ void m_old8_any(const af8_factored_tensor &T, int m_fmt, int m_block, int64_t flat, int64_t numel, float (&m)[8])
+{
+    if (m_fmt == AF8_M_UF8 && m_block == 256) {
+        const int64_t b = flat >> 8, last = (numel - 1) >> 8;
+        const int left = 256 - (int)(flat & 255);                // elements of the first block
+        const float s0 = __fmul_rn(__ldg(T.m_scale + b), 0.0078125f), s1 = __fmul_rn(__ldg(T.m_scale + min(b + 1, last)), 0.0078125f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t code = flat + j < numel ? (uint32_t)T.m_q[flat + j] : 128u;
+            m[j] = __fmul_rn(byte_minus_128(code, 0), j < left ? s0 : s1);
+        }
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) m[j] = flat + j < numel ? m_old_at(T, m_fmt, m_block, flat + j) : 0.0f;
+}
+
+// values col .. col + 7 of a column vector, 0 from column C on
+__device__ __forceinline__ void load_cols_any(const float *p, int64_t col, int64_t C, float (&x)[8])
+{
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] = col + j < C ? __ldg(p + col + j) : 0.0f;
+}
+
+// stats_rows for rows of any length: elements beyond the row's end count as zeros, all loads through GradAny8
+template <typename GradT, int NB, bool RESIDUAL>
+__device__ __forceinline__ void stats_rows_any(const FactoredLaunch &L, const af8_factored_tensor &sT, int64_t r0, int64_t r_end, int64_t c,
+                                               float pre_div, const float (&ic)[8], double (&cacc)[8])
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t C = sT.cols, numel = sT.rows * C;
+    const int nc = (int)max((int64_t)0, min((int64_t)8, C - c));     // this lane's columns
+    for (int k0 = 0; r0 + warp + 8 * k0 < r_end; k0 += NB) {         // (uniform over the warp)
+        GradAny8<GradT> cur[NB];
+#pragma unroll
+        for (int k = 0; k < NB; ++k) {
+            const int64_t r = r0 + warp + 8 * (k0 + k);
+            if (nc > 0 && r < r_end) cur[k].load(sT.grad, r * C + c, numel);
+            else cur[k].zero();
+        }
+#pragma unroll
+        for (int k = 0; k < NB; ++k) {
+            const int64_t r = r0 + warp + 8 * (k0 + k);
+            float g[8], x[8];
+            cur[k].unpack(L.negate_grad, g);
+            if (!RESIDUAL) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x[j] = __fmul_rn(g[j], g[j]);
+            } else if (nc > 0 && r < r_end) {
+                const float ir = sT.inv_row[r];
+                const DivBy D = make_div(pre_div);
+                const LerpW LW = make_lerp(sT.m_w);
+                float mo[8];
+                m_old8_any(sT, L.m_fmt, L.m_block, r * C + c, numel, mo);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const float u = u_clipped_fast(g[j], ir, ic[j], D);
+                    const float df = __fsub_rn(u, lerp_w(mo[j], u, LW));
+                    x[j] = __fadd_rn(__fmul_rn(df, df), sT.eps_came);
+                }
+            }
+            double racc = 0.0;
+            const bool live = r < r_end;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const double xd = (live && j < nc) ? (double)x[j] : 0.0;
+                racc += xd;
+                cacc[j] += xd;
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) racc += __shfl_xor_sync(0xffffffffu, racc, o);
+            if (lane == 0 && live) atomicAdd(sT.row_sum + r, racc);
+        }
+    }
+}
+
 // Rows r0 + warp + 8k of the tile, NB at a time so that NB independent 128-bit loads per lane
 // are in flight.  Column partials go to a per-warp shared array (no shared-memory atomics).
 template <typename GradT, int NB, bool PREFETCH, bool RESIDUAL>
-__device__ __forceinline__ void stats_rows(const FactoredLaunch &L, const af8_factored_tensor &sT, int64_t r0, int64_t row_end, int64_t c,
+__device__ __forceinline__ void stats_rows(const FactoredLaunch &L, const af8_factored_tensor &sT, int64_t r0, int64_t r_end, int64_t c,
                                            bool col_ok, float pre_div, const float (&ic)[8], double (&cacc)[8])
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t R = row_end, C = sT.cols;          // row_end: end of the tile's matrix (the tensor's rows unless it is a batch)
+    const int64_t R = r_end, C = sT.cols;            // r_end: end of the unit's rows
     // PREFETCH: the loads of the next NB rows are issued before the current ones are processed
     GradRaw8<GradT> cur[NB], nxt[NB];
     auto fetch = [&](GradRaw8<GradT> (&dst)[NB], int k0) {
 #pragma unroll
         for (int k = 0; k < NB; ++k) {
             const int64_t r = r0 + warp + 8 * (k0 + k);
-            if (col_ok && r < R && k0 + k < FSTAT_ROWS / 8) dst[k].load(sT.grad, r * C + c);
+            if (col_ok && r < R) dst[k].load(sT.grad, r * C + c);
             else dst[k].zero();
         }
     };
     if (PREFETCH) fetch(cur, 0);
-    for (int k0 = 0; k0 < FSTAT_ROWS / 8; k0 += NB) {
-        if (r0 + warp + 8 * k0 >= R) break;                       // uniform over the warp
+    for (int k0 = 0; r0 + warp + 8 * k0 < R; k0 += NB) {          // (uniform over the warp)
         if (PREFETCH) fetch(nxt, k0 + NB);
         else fetch(cur, k0);
         float g[NB][8];
@@ -710,7 +911,7 @@ __device__ __forceinline__ void stats_rows(const FactoredLaunch &L, const af8_fa
             for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
             if ((lane & 7) == 0) {
                 const int64_t r = r0 + warp + 8 * (k0 + (lane >> 3));
-                if (r < R && k0 + (lane >> 3) < FSTAT_ROWS / 8) atomicAdd(sT.row_sum + r, v);
+                if (r < R) atomicAdd(sT.row_sum + r, v);
             }
         } else {
             const bool hi = lane & 16;
@@ -719,7 +920,7 @@ __device__ __forceinline__ void stats_rows(const FactoredLaunch &L, const af8_fa
             for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
             if ((lane & 15) == 0) {
                 const int64_t r = r0 + warp + 8 * (k0 + (lane >> 4));
-                if (r < R && k0 + (lane >> 4) < FSTAT_ROWS / 8) atomicAdd(sT.row_sum + r, v);
+                if (r < R) atomicAdd(sT.row_sum + r, v);
             }
         }
     }
@@ -781,7 +982,7 @@ __device__ __forceinline__ void residual_x8(const float (&g)[8], uint2 codes, fl
 // next iteration are loaded while the current one computes; the sign of a negated gradient rides on the row
 // factor ((-g) * r == g * (-r) bit for bit).  Returns false after a time-out.
 template <typename GradT, int NB, bool ONE, bool SMALL>
-__device__ __forceinline__ bool residual_rows_ring(const FactoredLaunch &L, const af8_factored_tensor &sT, int64_t r0, int64_t c0,
+__device__ __forceinline__ bool residual_rows_ring(const FactoredLaunch &L, const af8_factored_tensor &sT, int64_t r0, int64_t r_end, int64_t c0,
                                                    float pre_div, const float (&ic)[8], double (&cacc)[8],
                                                    unsigned char *ring, uint64_t *full, uint32_t &cons)
 {
@@ -790,7 +991,6 @@ __device__ __forceinline__ bool residual_rows_ring(const FactoredLaunch &L, cons
     static_assert(NB == 2 || NB == 4, "row-sum reduction is written for 2 or 4 rows");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t C = sT.cols;
-    const int64_t r_end = min(sT.rows, r0 + (int64_t)FSTAT_ROWS);
     const int64_t row0 = r0 + warp;
     const int nrows = row0 < r_end ? (int)((r_end - row0 + 7) / 8) : 0;          // rows row0 + 8 k of this warp
     // lanes 0 and 1 request the next slice: lane 0 its gradients (and the bytes to expect), lane 1 its codes,
@@ -903,7 +1103,7 @@ __device__ __forceinline__ bool residual_rows_ring(const FactoredLaunch &L, cons
 // 256-column slices of the gradient (tensor map maps[0]: bf16 [rows][cols], box 256 x FBOX_ROWS), one their UF8 codes
 // (maps[1]: bytes, same box) into a stage of the warp's two-stage ring, so that the instructions of a request -
 // about 57 issue slots with one lane active - are spent once per FBOX_ROWS rows instead of once per row.  Warp w
-// takes the row groups r0 + FBOX_ROWS (w + 8 k); rows past the end of the tensor arrive as zeros and are skipped.
+// takes the row groups r0 + FBOX_ROWS (w + 8 k); rows past the end of the unit are skipped (past the end of the tensor they arrive as zeros).
 // bf16 gradients only (a stage is 3 KB; the two stages fill the ring's 6 KB per warp).
 constexpr int FBOX_ROWS = 4, FBOX_STAGES = 2;
 constexpr int FBOX_G_BYTES = FBOX_ROWS * 512, FBOX_STAGE_BYTES = FBOX_G_BYTES + FBOX_ROWS * 256;
@@ -912,13 +1112,13 @@ static_assert(FSTAT_ROWS % (8 * FBOX_ROWS) == 0, "whole row groups per warp and 
 
 template <bool ONE, bool SMALL>
 __device__ __forceinline__ bool residual_rows_box(const FactoredLaunch &L, const af8_factored_tensor &sT, const CUtensorMap *maps,
-                                                  int64_t r0, int64_t c0, float pre_div, const float (&ic)[8], double (&cacc)[8],
+                                                  int64_t r0, int64_t row_end, int64_t c0, float pre_div, const float (&ic)[8], double (&cacc)[8],
                                                   unsigned char *ring, uint64_t *full, uint32_t &cons)
 {
     constexpr int BR = FBOX_ROWS, NS = FBOX_STAGES;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t C = sT.cols;
-    const int r_end = (int)min(sT.rows, r0 + (int64_t)FSTAT_ROWS);
+    const int r_end = (int)row_end;
     const int row0 = (int)r0 + BR * warp;                        // first row of this warp's group 0; group g: + 8 * BR * g
     const int ngroups = row0 < r_end ? (r_end - row0 + 8 * BR - 1) / (8 * BR) : 0;
     auto issue = [&](int g) {                                    // lane 0: group g into its stage
@@ -1017,8 +1217,9 @@ __device__ __forceinline__ bool residual_rows_box(const FactoredLaunch &L, const
 #ifndef AF8_FSTAT_MIN_CTAS_RES
 #define AF8_FSTAT_MIN_CTAS_RES 3
 #endif
-template <typename GradT, bool RESIDUAL>
-__global__ void __launch_bounds__(256, RESIDUAL ? AF8_FSTAT_MIN_CTAS_RES : AF8_FSTAT_MIN_CTAS)
+// ANY: the table has batches of matrices or rows whose length is no multiple of 8 (tensor by tensor)
+template <typename GradT, bool RESIDUAL, bool ANY>
+__global__ void __launch_bounds__(256, ANY && (RESIDUAL || std::is_same<GradT, float>::value) ? 2 : RESIDUAL ? AF8_FSTAT_MIN_CTAS_RES : AF8_FSTAT_MIN_CTAS)
 factored_stats_vec_kernel(const FactoredLaunch L, const int use_ring, const CUtensorMap *__restrict__ maps)
 {
     __shared__ double s_col[8][FSTAT_COLS];      // [warp][j * 32 + lane]
@@ -1039,8 +1240,9 @@ factored_stats_vec_kernel(const FactoredLaunch L, const int use_ring, const CUte
 
     for (int64_t id = blockIdx.x; id < L.total_units; id += gridDim.x) {
         int t = cur_t;
-        if (t < 0) t = find_factored_tile(L.tensors, L.n_tensors, id);
-        else while (t + 1 < L.n_tensors && __ldg(&L.tensors[t + 1].first_tile) <= id) ++t;
+        const int64_t tile = id >> L.split;
+        if (t < 0) t = find_factored_tile(L.tensors, L.n_tensors, tile);
+        else while (t + 1 < L.n_tensors && __ldg(&L.tensors[t + 1].first_tile) <= tile) ++t;
         __syncthreads();                                           // s_col of the previous tile was read
         if (t != cur_t) {
             if (tid < (int)(sizeof(af8_factored_tensor) / 4))
@@ -1049,11 +1251,9 @@ factored_stats_vec_kernel(const FactoredLaunch L, const int use_ring, const CUte
             __syncthreads();
         }
         const int64_t C = sT.cols;
-        const int64_t ntc = (C + FSTAT_COLS - 1) / FSTAT_COLS;
-        const int64_t local = id - sT.first_tile;                  // (batches of matrices take the general kernel)
-        const int64_t r0 = (local / ntc) * FSTAT_ROWS;
-        const int64_t row_end = sT.rows;
-        const int64_t c0 = (local % ntc) * FSTAT_COLS;
+        const TilePos P = tile_pos(L, sT, id);
+        const int64_t r0 = P.r0, row_end = P.r_end, c0 = P.c0;
+        if (r0 >= row_end) continue;                               // an empty part of a split tile
         const int64_t c = c0 + lane * 8;                           // this lane's 8 columns
         const bool col_ok = c < C;                                 // C % 8 == 0: all 8 or none
         float pre_div = 1.0f;
@@ -1062,7 +1262,8 @@ factored_stats_vec_kernel(const FactoredLaunch L, const int use_ring, const CUte
         for (int j = 0; j < 8; ++j) ic[j] = 0.0f;
         if (RESIDUAL) {
             pre_div = L.dyn[t].pre_div;
-            if (col_ok) load_f8_ro(sT.inv_col + c, ic);
+            if (ANY && (C & 7) != 0) load_cols_any(sT.inv_col + P.cb, c, C, ic);
+            else if (col_ok) load_f8_ro(sT.inv_col + P.cb + c, ic);
         }
         double cacc[8];
 #pragma unroll
@@ -1072,7 +1273,12 @@ factored_stats_vec_kernel(const FactoredLaunch L, const int use_ring, const CUte
         // gradient, were slower through a ring - 3.0 -> 4.3 ms and 4.6 -> 5.9 ms - and load directly)
         // (the ring's quotient wants a clip divisor >= 1 or NaN, which is what the RMS clip produces)
         bool done = false;
-        if constexpr (RESIDUAL) {
+        if constexpr (ANY) {
+            if ((C & 7) != 0) {
+                done = true;
+                stats_rows_any<GradT, 4, RESIDUAL>(L, sT, r0, row_end, c, pre_div, ic, cacc);
+            }
+        } else if constexpr (RESIDUAL) {
             if (use_ring && (C % FSTAT_COLS) == 0 && L.m_fmt == AF8_M_UF8 && L.m_block == 256 && !(pre_div < 1.0f)) {
                 done = true;
                 unsigned char *ring = sr_smem + (size_t)warp * sring_stages<GradT>() * sring_stage_bytes<GradT, true>();
@@ -1084,24 +1290,25 @@ factored_stats_vec_kernel(const FactoredLaunch L, const int use_ring, const CUte
                     boxes = true;
                     const CUtensorMap *mp = maps + 2 * t;
                     if (lane == 0 && t != mapped) { tensormap_acquire(mp); tensormap_acquire(mp + 1); mapped = t; }
-                    if (one) ok = small ? residual_rows_box<true, true>(L, sT, mp, r0, c0, pre_div, ic, cacc, ring, s_full[warp], cons)
-                                        : residual_rows_box<true, false>(L, sT, mp, r0, c0, pre_div, ic, cacc, ring, s_full[warp], cons);
-                    else ok = small ? residual_rows_box<false, true>(L, sT, mp, r0, c0, pre_div, ic, cacc, ring, s_full[warp], cons)
-                                    : residual_rows_box<false, false>(L, sT, mp, r0, c0, pre_div, ic, cacc, ring, s_full[warp], cons);
+                    if (one) ok = small ? residual_rows_box<true, true>(L, sT, mp, r0, row_end, c0, pre_div, ic, cacc, ring, s_full[warp], cons)
+                                        : residual_rows_box<true, false>(L, sT, mp, r0, row_end, c0, pre_div, ic, cacc, ring, s_full[warp], cons);
+                    else ok = small ? residual_rows_box<false, true>(L, sT, mp, r0, row_end, c0, pre_div, ic, cacc, ring, s_full[warp], cons)
+                                    : residual_rows_box<false, false>(L, sT, mp, r0, row_end, c0, pre_div, ic, cacc, ring, s_full[warp], cons);
                 }
                 }
                 if (boxes) { }
-                else if (one) ok = small ? residual_rows_ring<GradT, NB, true, true>(L, sT, r0, c0, pre_div, ic, cacc, ring, s_full[warp], cons)
-                                    : residual_rows_ring<GradT, NB, true, false>(L, sT, r0, c0, pre_div, ic, cacc, ring, s_full[warp], cons);
-                else ok = small ? residual_rows_ring<GradT, NB, false, true>(L, sT, r0, c0, pre_div, ic, cacc, ring, s_full[warp], cons)
-                                : residual_rows_ring<GradT, NB, false, false>(L, sT, r0, c0, pre_div, ic, cacc, ring, s_full[warp], cons);
+                else if (one) ok = small ? residual_rows_ring<GradT, NB, true, true>(L, sT, r0, row_end, c0, pre_div, ic, cacc, ring, s_full[warp], cons)
+                                    : residual_rows_ring<GradT, NB, true, false>(L, sT, r0, row_end, c0, pre_div, ic, cacc, ring, s_full[warp], cons);
+                else ok = small ? residual_rows_ring<GradT, NB, false, true>(L, sT, r0, row_end, c0, pre_div, ic, cacc, ring, s_full[warp], cons)
+                                : residual_rows_ring<GradT, NB, false, false>(L, sT, r0, row_end, c0, pre_div, ic, cacc, ring, s_full[warp], cons);
                 if (!ok) {
                     atomicExch(&g_device_error, DEVERR_SRING_TIMEOUT);
                     return;                      // (the whole warp; the others finish their rows and leave at the next barrier)
                 }
             }
         }
-        if (!RESIDUAL) stats_rows<GradT, 4, true, false>(L, sT, r0, row_end, c, col_ok, pre_div, ic, cacc);
+        if (ANY && done) { }
+        else if (!RESIDUAL) stats_rows<GradT, 4, true, false>(L, sT, r0, row_end, c, col_ok, pre_div, ic, cacc);
         else if (!done) stats_rows<GradT, AF8_FSTAT_RES_NB, AF8_FSTAT_RES_PREFETCH, true>(L, sT, r0, row_end, c, col_ok, pre_div, ic, cacc);
 #pragma unroll
         for (int j = 0; j < 8; ++j) s_col[warp][j * 32 + lane] = cacc[j];
@@ -1111,7 +1318,7 @@ factored_stats_vec_kernel(const FactoredLaunch L, const int use_ring, const CUte
             double sum = 0.0;
 #pragma unroll
             for (int w = 0; w < 8; ++w) sum += s_col[w][(tid & 7) * 32 + (tid >> 3)];
-            atomicAdd(sT.col_sum + c0 + tid, sum);
+            atomicAdd(sT.col_sum + P.cb + c0 + tid, sum);
         }
     }
 }
@@ -1122,7 +1329,12 @@ factored_stats_vec_kernel(const FactoredLaunch L, const int use_ring, const CUte
 // CTAS: resident CTAs per SM asked of the compiler.  Measured on B200: 4 for the sum passes; for the
 // writing passes 3 with momentum (CAME, 0.78 ms per Llama-2-7B layer) and 2 without (Adafactor on the
 // TinyLlama set: 2.51 -> 2.21 ms, no register spills).
-template <typename GradT, int PASS, int CTAS>
+// ANY: tensors with batches of matrices or with rows of any length >= 8.  The flat vectors of 8 stay aligned; a vector
+// crosses at most one row end, so its elements take one of two row factors and column factors that are loaded one by
+// one (for rows of a multiple of 8: as vectors).  Only a tensor's last vector may be partial.  The squares of the sum
+// passes enter binary64 one by one, as in factored_update_kernel, which such tensors took before: 59 M parameters of
+// odd sizes, UF8 momentum: see the figures there.
+template <typename GradT, int PASS, int CTAS, bool ANY>
 __global__ void __launch_bounds__(FUPD_THREADS, CTAS)
 factored_update_vec_kernel(const FactoredLaunch L)
 {
@@ -1212,6 +1424,8 @@ factored_update_vec_kernel(const FactoredLaunch L)
         (void)t;
         const int64_t numel = sT.rows * sT.cols;
         const bool ok = flat < numel;                                // numel % 8 == 0: all 8 or none
+        const bool partial = ANY && ok && flat + 8 > numel;          // (the tensor's last elements)
+        const int nval = partial ? (int)(numel - flat) : 8;
         // this chunk's streams, loaded one iteration ahead when the chunk is in the same tensor
         GradRaw8<GradT> cg;
         float4 cp0 = make_float4(0.f, 0.f, 0.f, 0.f), cp1 = cp0;
@@ -1221,7 +1435,22 @@ factored_update_vec_kernel(const FactoredLaunch L)
         const bool lowp = L.param_dtype != AF8_F32;                  // 16-bit parameters: 8 of them in cp0
         const uint16_t *const hbase = static_cast<const uint16_t *>(sT.param);
         if (have) { cg = ng; cp0 = np0; cp1 = np1; cm = nm; }
-        else if (ok) {
+        else if (partial) {
+            cg.load_part(sT.grad, flat, nval);
+            if (writes && lowp) {
+                uint32_t x[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (j < nval) x[j >> 1] |= (uint32_t)hbase[flat + j] << (16 * (j & 1));
+                cp0 = make_float4(__uint_as_float(x[0]), __uint_as_float(x[1]), __uint_as_float(x[2]), __uint_as_float(x[3]));
+            } else if (writes) {
+                float x[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x[j] = j < nval ? pbase[flat + j] : 0.0f;
+                cp0 = make_float4(x[0], x[1], x[2], x[3]); cp1 = make_float4(x[4], x[5], x[6], x[7]);
+            }
+            if (pre_m) cm = *reinterpret_cast<const uint2 *>(sT.m_q + flat);     // (codes are stored in whole blocks)
+        } else if (ok) {
             cg.load(sT.grad, flat);
             if (writes) {
                 if (lowp) cp0 = *reinterpret_cast<const float4 *>(hbase + flat);
@@ -1246,7 +1475,7 @@ factored_update_vec_kernel(const FactoredLaunch L)
 #endif
         {
             const int64_t nf = flat + 2048;                          // the next chunk of this CTA, if it is in this tensor
-            have = id + 1 < id_end && nf < numel;
+            have = id + 1 < id_end && (ANY ? nf + 8 <= numel : nf < numel);
             if (have) {
                 ng.load(sT.grad, nf);
                 if (writes) {
@@ -1262,47 +1491,85 @@ factored_update_vec_kernel(const FactoredLaunch L)
             float g[8], ic[8], u[8];
             const LerpW LW = make_lerp(sT.m_w);
             cg.unpack(L.negate_grad, g);
-            load_f8_ro(sT.inv_col + col, ic);
-            const float ir = __ldg(sT.inv_row + row);
+            // ANY: elements j >= wrap belong to the next row; cb0 / cb1: first entries of the two rows' matrices in the
+            // column arrays, irow1: index of the next row (clamped: nothing valid follows the last)
+            int wrap = 8;
+            int64_t cb0 = 0, cb1 = 0, irow1 = row;
+            bool whole = true;                                       // the columns come as vectors
+            if constexpr (ANY) {
+                whole = (sT.cols & 7) == 0;
+                if (!whole) {
+                    wrap = (int)min((int64_t)8, sT.cols - col);
+                    irow1 = min(row + 1, sT.rows - 1);
+                }
+                if (sT.batch_rows > 0) {                             // (rows < 2^31)
+                    cb0 = (int64_t)((uint32_t)row / (uint32_t)sT.batch_rows) * sT.cols;
+                    cb1 = (int64_t)((uint32_t)irow1 / (uint32_t)sT.batch_rows) * sT.cols;
+                }
+            }
+            auto cols8 = [&](const float *v, float (&x)[8]) {
+                if (!ANY || whole) { load_f8_ro(v + cb0 + col, x); return; }
+                const float *va = v + cb0 + col, *vb = v + cb1 - wrap;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x[j] = __ldg((j < wrap ? va : vb) + j);
+            };
+            auto row2 = [&](float a, float b, int j) {               // the row factors of elements j, j + 1
+                return ANY ? make_float2(j < wrap ? a : b, j + 1 < wrap ? a : b) : bc2(a);
+            };
+            cols8(sT.inv_col, ic);
+            const float ir = __ldg(sT.inv_row + row), irb = ANY ? __ldg(sT.inv_row + irow1) : 0.0f;
             // pairs of elements in packed binary32 arithmetic (bit-identical to the element-wise form)
-            const float2 ir2 = bc2(ir);
             if (L.came) {
                 if (L.mode == AF8_FUPD_SUMSQ_U) {
 #pragma unroll
                     for (int j = 0; j < 8; j += 2) {
-                        const float2 uj = __fmul2_rn(__fmul2_rn(make_float2(g[j], g[j + 1]), ir2), make_float2(ic[j], ic[j + 1]));
+                        const float2 uj = __fmul2_rn(__fmul2_rn(make_float2(g[j], g[j + 1]), row2(ir, irb, j)), make_float2(ic[j], ic[j + 1]));
                         u[j] = uj.x; u[j + 1] = uj.y;
                     }
                 } else {
                     float mo[8], icc[8];
-                    m_old8(sT, L.m_fmt, L.m_block, flat, mo, pre_m, cm);
-                    load_f8_ro(sT.inv_col_conf + col, icc);
-                    const float2 irc2 = bc2(__ldg(sT.inv_row_conf + row));
+                    if (partial && !m_quant) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) mo[j] = j < nval ? sT.m_f32[flat + j] : 0.0f;
+                    } else m_old8(sT, L.m_fmt, 256, flat, mo, pre_m, cm);
+                    cols8(sT.inv_col_conf, icc);
+                    const float irc = __ldg(sT.inv_row_conf + row), ircb = ANY ? __ldg(sT.inv_row_conf + irow1) : 0.0f;
 #pragma unroll
                     for (int j = 0; j < 8; j += 2) {
-                        const float2 ut = div_by2(__fmul2_rn(__fmul2_rn(make_float2(g[j], g[j + 1]), ir2), make_float2(ic[j], ic[j + 1])), D);
+                        const float2 ut = div_by2(__fmul2_rn(__fmul2_rn(make_float2(g[j], g[j + 1]), row2(ir, irb, j)), make_float2(ic[j], ic[j + 1])), D);
                         const float2 mm = lerp_w2(make_float2(mo[j], mo[j + 1]), ut, LW);
-                        const float2 uj = __fmul2_rn(__fmul2_rn(mm, irc2), make_float2(icc[j], icc[j + 1]));
+                        const float2 uj = __fmul2_rn(__fmul2_rn(mm, row2(irc, ircb, j)), make_float2(icc[j], icc[j + 1]));
                         mj[j] = mm.x; mj[j + 1] = mm.y; u[j] = uj.x; u[j + 1] = uj.y;
                     }
                 }
             } else if (has_m) {
                 float mo[8];
-                m_old8(sT, L.m_fmt, L.m_block, flat, mo, pre_m, cm);
+                if (partial && !m_quant) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) mo[j] = j < nval ? sT.m_f32[flat + j] : 0.0f;
+                    } else m_old8(sT, L.m_fmt, 256, flat, mo, pre_m, cm);
 #pragma unroll
                 for (int j = 0; j < 8; j += 2) {
                     const float2 mm = lerp_w2(make_float2(mo[j], mo[j + 1]), make_float2(g[j], g[j + 1]), LW);
-                    const float2 uj = __fmul2_rn(__fmul2_rn(mm, ir2), make_float2(ic[j], ic[j + 1]));
+                    const float2 uj = __fmul2_rn(__fmul2_rn(mm, row2(ir, irb, j)), make_float2(ic[j], ic[j + 1]));
                     mj[j] = mm.x; mj[j + 1] = mm.y; u[j] = uj.x; u[j + 1] = uj.y;
                 }
             } else {
 #pragma unroll
                 for (int j = 0; j < 8; j += 2) {
-                    const float2 uj = __fmul2_rn(__fmul2_rn(make_float2(g[j], g[j + 1]), ir2), make_float2(ic[j], ic[j + 1]));
+                    const float2 uj = __fmul2_rn(__fmul2_rn(make_float2(g[j], g[j + 1]), row2(ir, irb, j)), make_float2(ic[j], ic[j + 1]));
                     u[j] = uj.x; u[j + 1] = uj.y;
                 }
             }
-            if (SUMS) {
+            if (partial) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (j >= nval) { u[j] = 0.0f; mj[j] = 0.0f; }
+            }
+            if (SUMS && ANY) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) part += (double)__fmul_rn(u[j], u[j]);
+            } else if (SUMS) {
                 // The thread's eight squares are added in binary32 (two packed chains) and enter the binary64
                 // partial as one number: the sum only feeds a norm (clip divisor, limiter), where a relative
                 // 1e-7 is far below what the parameters can show, and it saves seven conversions and seven
@@ -1326,6 +1593,11 @@ factored_update_vec_kernel(const FactoredLaunch L)
                         const uint32_t r = param_step_bits(pv, sT.decay, step_mul, uu, L.param_dtype, L.sr, sT.sr_base, flat + j);
                         if (j & 1) o[j >> 1] |= r << 16; else o[j >> 1] = r;
                     }
+                    if (partial) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            if (j < nval) const_cast<uint16_t *>(hbase)[flat + j] = (uint16_t)(o[j >> 1] >> (16 * (j & 1)));
+                    } else
                     *reinterpret_cast<uint4 *>(const_cast<uint16_t *>(hbase) + flat) = make_uint4(o[0], o[1], o[2], o[3]);
                 } else {
                     float *pp = pbase + flat;
@@ -1337,13 +1609,26 @@ factored_update_vec_kernel(const FactoredLaunch L)
                         if (!zero_upd) pj = __ffma2_rn(step2, __fmul2_rn(make_float2(u[j], u[j + 1]), fira2), pj);
                         p[j] = pj.x; p[j + 1] = pj.y;
                     }
+                    if (partial) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            if (j < nval) {
+                                pp[j] = p[j];
+                                if (sT.param_copy != nullptr) static_cast<uint16_t *>(sT.param_copy)[flat + j] = (uint16_t)f32_to_bf16_rn_bits(p[j]);
+                            }
+                    } else {
                     *reinterpret_cast<float4 *>(pp) = make_float4(p[0], p[1], p[2], p[3]);
                     *reinterpret_cast<float4 *>(pp + 4) = make_float4(p[4], p[5], p[6], p[7]);
                     if (sT.param_copy != nullptr)                                    // bf16 compute copy
                         *reinterpret_cast<uint4 *>(static_cast<uint16_t *>(sT.param_copy) + flat) =
                             make_uint4(bf16x2_rn(p[0], p[1]), bf16x2_rn(p[2], p[3]), bf16x2_rn(p[4], p[5]), bf16x2_rn(p[6], p[7]));
+                    }
                 }
-                if (has_m && !m_quant) {
+                if (partial && has_m && !m_quant) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (j < nval) sT.m_f32[flat + j] = mj[j];
+                } else if (has_m && !m_quant) {
                     *reinterpret_cast<float4 *>(sT.m_f32 + flat) = make_float4(mj[0], mj[1], mj[2], mj[3]);
                     *reinterpret_cast<float4 *>(sT.m_f32 + flat + 4) = make_float4(mj[4], mj[5], mj[6], mj[7]);
                 }
@@ -1368,7 +1653,7 @@ factored_update_vec_kernel(const FactoredLaunch L)
                     const DivBy A = make_div(am);
                     const uint32_t o0 = uf8_encode_fast2(make_float2(mj[0], mj[1]), A) | (uf8_encode_fast2(make_float2(mj[2], mj[3]), A) << 16);
                     const uint32_t o1 = uf8_encode_fast2(make_float2(mj[4], mj[5]), A) | (uf8_encode_fast2(make_float2(mj[6], mj[7]), A) << 16);
-                    if (ok) *reinterpret_cast<uint2 *>(sT.m_q + flat) = make_uint2(o0, o1);
+                    if (ANY || ok) *reinterpret_cast<uint2 *>(sT.m_q + flat) = make_uint2(o0, o1);
                 } else if (L.m_fmt == AF8_M_D8) {
                     uint32_t o0 = 0, o1 = 0;
 #pragma unroll
@@ -1376,13 +1661,13 @@ factored_update_vec_kernel(const FactoredLaunch L)
                         o0 |= m_encode(mj[j], am, L.m_fmt) << (8 * j);
                         o1 |= m_encode(mj[j + 4], am, L.m_fmt) << (8 * j);
                     }
-                    if (ok) *reinterpret_cast<uint2 *>(sT.m_q + flat) = make_uint2(o0, o1);
+                    if (ANY || ok) *reinterpret_cast<uint2 *>(sT.m_q + flat) = make_uint2(o0, o1);
                 } else {
                     uint32_t o = 0;
 #pragma unroll
                     for (int j = 0; j < 8; j += 2)
                         o |= ((m_encode(mj[j], am, L.m_fmt) << 4) | m_encode(mj[j + 1], am, L.m_fmt)) << (4 * j);
-                    if (ok) *reinterpret_cast<uint32_t *>(sT.m_q + (flat >> 1)) = o;
+                    if (ANY || ok) *reinterpret_cast<uint32_t *>(sT.m_q + (flat >> 1)) = o;
                 }
                 if (lane == 0) sT.m_scale[w0 / 256] = am;
             }
@@ -1618,8 +1903,9 @@ factored_apply_tile_kernel(const FactoredLaunch L)
 
     for (int64_t id = blockIdx.x; id < L.total_units; id += gridDim.x) {
         int t = cur_t;
-        if (t < 0) t = find_factored_tile(L.tensors, L.n_tensors, id);
-        else while (t + 1 < L.n_tensors && __ldg(&L.tensors[t + 1].first_tile) <= id) ++t;
+        const int64_t tile = id >> L.split;
+        if (t < 0) t = find_factored_tile(L.tensors, L.n_tensors, tile);
+        else while (t + 1 < L.n_tensors && __ldg(&L.tensors[t + 1].first_tile) <= tile) ++t;
         if (t != cur_t) {
             __syncthreads();                                         // every warp has left the previous tensor
             if (tid < (int)(sizeof(af8_factored_tensor) / 4))
@@ -1634,17 +1920,14 @@ factored_apply_tile_kernel(const FactoredLaunch L)
             }
             D = make_div(pre_div);
         }
-        const int64_t R = sT.rows, C = sT.cols;
-        const int64_t ntc = C / FSTAT_COLS;                          // (cols % 256 == 0)
-        const int64_t local = id - sT.first_tile;
-        const int64_t r0 = (local / ntc) * FSTAT_ROWS;
-        const int64_t c0 = (local % ntc) * FSTAT_COLS;
+        const int64_t C = sT.cols;                                   // (a multiple of 256)
+        const TilePos P = tile_pos(L, sT, id);
+        const int64_t r0 = P.r0, r_end = P.r_end, c0 = P.c0;
         const int64_t c = c0 + lane * 8;                             // this lane's 8 columns
-        const int64_t r_end = min(R, r0 + (int64_t)FSTAT_ROWS);
         const int nrows = r0 + warp < r_end ? (int)((r_end - (r0 + warp) + 7) / 8) : 0;
         float ic[8], icc[8];
-        load_f8_ro(sT.inv_col + c, ic);
-        if (L.came) load_f8_ro(sT.inv_col_conf + c, icc);
+        load_f8_ro(sT.inv_col + P.cb + c, ic);
+        if (L.came) load_f8_ro(sT.inv_col_conf + P.cb + c, icc);
         float *const pbase = static_cast<float *>(sT.param);
         const unsigned char *gp = static_cast<const unsigned char *>(sT.grad);
         const LerpW LW = make_lerp(sT.m_w);
@@ -1840,8 +2123,9 @@ factored_sumsq_wide_kernel(const FactoredLaunch L)
 // its 8 columns in registers while its warp walks the tile's rows (the flat kernel above re-reads them for
 // every element, twice the bytes of the gradient itself through L1), four rows' loads in flight.  A CTA adds
 // its tile's sum to the slot of the tensor's first chunk; the caller clears the slots first.
-template <typename GradT>
-__global__ void __launch_bounds__(256, 4)
+// ANY: batches of matrices and rows of any length; the squares enter binary64 one by one (see factored_update_vec_kernel).
+template <typename GradT, bool ANY>
+__global__ void __launch_bounds__(256, ANY ? 3 : 4)
 factored_sumsq_tile_kernel(const FactoredLaunch L)
 {
     constexpr int NB = 4;
@@ -1851,8 +2135,9 @@ factored_sumsq_tile_kernel(const FactoredLaunch L)
     int cur_t = -1;
     for (int64_t id = blockIdx.x; id < L.total_units; id += gridDim.x) {
         int t = cur_t;
-        if (t < 0) t = find_factored_tile(L.tensors, L.n_tensors, id);
-        else while (t + 1 < L.n_tensors && __ldg(&L.tensors[t + 1].first_tile) <= id) ++t;
+        const int64_t tile = id >> L.split;
+        if (t < 0) t = find_factored_tile(L.tensors, L.n_tensors, tile);
+        else while (t + 1 < L.n_tensors && __ldg(&L.tensors[t + 1].first_tile) <= tile) ++t;
         __syncthreads();                                           // s_acc2 of the previous tile was read
         if (t != cur_t) {
             if (tid < (int)(sizeof(af8_factored_tensor) / 4))
@@ -1860,29 +2145,54 @@ factored_sumsq_tile_kernel(const FactoredLaunch L)
             cur_t = t;
             __syncthreads();
         }
-        const int64_t R = sT.rows, C = sT.cols;
-        const int64_t ntc = (C + FSTAT_COLS - 1) / FSTAT_COLS;
-        const int64_t local = id - sT.first_tile;
-        const int64_t r0 = (local / ntc) * FSTAT_ROWS;
-        const int64_t c = (local % ntc) * FSTAT_COLS + lane * 8;   // this lane's 8 columns
+        const int64_t C = sT.cols;
+        const TilePos P = tile_pos(L, sT, id);
+        const int64_t r0 = P.r0, R = P.r_end;
+        if (r0 >= R) continue;                                     // an empty part of a split tile
+        const int64_t c = P.c0 + lane * 8;                         // this lane's 8 columns
         const bool col_ok = c < C;                                 // C % 8 == 0: all 8 or none
         float ic[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) ic[j] = 0.0f;
-        if (col_ok) load_f8_ro(sT.inv_col + c, ic);
         double acc = 0.0;
+        if (ANY && (C & 7) != 0) {
+            const int nc = (int)max((int64_t)0, min((int64_t)8, C - c));
+            const int64_t numel = sT.rows * C;
+            load_cols_any(sT.inv_col + P.cb, c, C, ic);
+            for (int k0 = 0; r0 + warp + 8 * k0 < R; k0 += NB) {   // (uniform over the warp)
+                GradAny8<GradT> any[NB];
+#pragma unroll
+                for (int k = 0; k < NB; ++k) {
+                    const int64_t r = r0 + warp + 8 * (k0 + k);
+                    if (nc > 0 && r < R) any[k].load(sT.grad, r * C + c, numel);
+                    else any[k].zero();
+                }
+#pragma unroll
+                for (int k = 0; k < NB; ++k) {
+                    const int64_t r = min(r0 + warp + 8 * (int64_t)(k0 + k), R - 1);     // (a row beyond the end carries zeros)
+                    const float ir = __ldg(sT.inv_row + r);
+                    float g[8];
+                    any[k].unpack(0, g);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const float uj = __fmul_rn(__fmul_rn(g[j], ir), ic[j]);
+                        if (j < nc) acc += (double)__fmul_rn(uj, uj);
+                    }
+                }
+            }
+        } else {
+        if (col_ok) load_f8_ro(sT.inv_col + P.cb + c, ic);
         GradRaw8<GradT> cur[NB], nxt[NB];
         auto fetch = [&](GradRaw8<GradT> (&dst)[NB], int k0) {
 #pragma unroll
             for (int k = 0; k < NB; ++k) {
                 const int64_t r = r0 + warp + 8 * (k0 + k);
-                if (col_ok && r < R && k0 + k < FSTAT_ROWS / 8) dst[k].load(sT.grad, r * C + c);
+                if (col_ok && r < R) dst[k].load(sT.grad, r * C + c);
                 else dst[k].zero();
             }
         };
         fetch(cur, 0);
-        for (int k0 = 0; k0 < FSTAT_ROWS / 8; k0 += NB) {
-            if (r0 + warp + 8 * k0 >= R) break;                    // uniform over the warp
+        for (int k0 = 0; r0 + warp + 8 * k0 < R; k0 += NB) {       // (uniform over the warp)
             fetch(nxt, k0 + NB);
 #pragma unroll
             for (int k = 0; k < NB; ++k) {
@@ -1894,11 +2204,13 @@ factored_sumsq_tile_kernel(const FactoredLaunch L)
 #pragma unroll
                 for (int j = 0; j < 8; j += 2) {
                     const float2 uj = __fmul2_rn(__fmul2_rn(make_float2(g[j], g[j + 1]), ir2), make_float2(ic[j], ic[j + 1]));
-                    a2 = j == 0 ? __fmul2_rn(uj, uj) : __ffma2_rn(uj, uj, a2);
+                    if (ANY) { const float2 q = __fmul2_rn(uj, uj); acc += (double)q.x; acc += (double)q.y; }
+                    else a2 = j == 0 ? __fmul2_rn(uj, uj) : __ffma2_rn(uj, uj, a2);
                 }
-                acc += (double)__fadd_rn(a2.x, a2.y);
+                if (!ANY) acc += (double)__fadd_rn(a2.x, a2.y);
                 cur[k] = nxt[k];
             }
+        }
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
@@ -1930,7 +2242,8 @@ inline int validate_factored(const af8_factored_cfg &c, const af8_factored_tenso
         const af8_factored_tensor &t = T[i];
         if (t.rows <= 0 || t.cols <= 0) return fail(AF8_ERR_INVALID, "factored tensor %d: empty shape", i);
         if (c.aligned8) {
-            if (t.cols % 8 != 0) return fail(AF8_ERR_INVALID, "factored tensor %d: aligned8 needs cols %% 8 == 0", i);
+            if (c.aligned8 != 2 && t.cols % 8 != 0) return fail(AF8_ERR_INVALID, "factored tensor %d: aligned8 needs cols %% 8 == 0", i);
+            if (c.aligned8 == 2 && t.cols < 8) return fail(AF8_ERR_INVALID, "factored tensor %d: aligned8 = 2 needs cols >= 8", i);
             const void *ptrs[] = {t.param, t.grad, t.m_q, t.m_f32, t.inv_col, t.inv_col_conf, t.param_copy};
             for (const void *q : ptrs)
                 if (q && (reinterpret_cast<uintptr_t>(q) & 15u)) return fail(AF8_ERR_INVALID, "factored tensor %d: aligned8 needs 16-byte aligned arrays", i);
@@ -1947,8 +2260,9 @@ inline int validate_factored(const af8_factored_cfg &c, const af8_factored_tenso
         next_chunk += (t.rows * t.cols + chunk - 1) / chunk;
         if (t.batch_rows < 0 || (t.batch_rows > 0 && t.rows % t.batch_rows != 0))
             return fail(AF8_ERR_INVALID, "factored tensor %d: batch_rows %lld does not divide rows %lld", i, (long long)t.batch_rows, (long long)t.rows);
-        if (t.batch_rows > 0 && c.aligned8)
-            return fail(AF8_ERR_INVALID, "factored tensor %d: a batch of matrices takes the general kernels (cfg.aligned8 = 0)", i);
+        if (t.batch_rows > 0 && c.aligned8 && c.aligned8 != 2)
+            return fail(AF8_ERR_INVALID, "factored tensor %d: a batch of matrices needs cfg.aligned8 = 0 or 2", i);
+        if (c.aligned8 == 2 && t.rows >= ((int64_t)1 << 31)) return fail(AF8_ERR_UNSUPPORTED, "factored tensor %d: too many rows for aligned8 = 2", i);
         next_tile += fact_tiles(t);
         const af8_small_state *ss[4] = {&t.row_var, &t.col_var, &t.conf_row, &t.conf_col};
         const int sb = t.row_var.block;
@@ -1992,7 +2306,7 @@ inline FactoredLaunch make_factored_launch(const af8_factored_cfg &c, const af8_
     L.tensors = dev; L.dyn = dyn; L.block_sumsq = sumsq; L.total_units = units; L.n_tensors = n;
     L.grad_dtype = c.grad_dtype; L.m_fmt = c.m_fmt; L.m_block = c.m_block > 0 ? c.m_block : 256;
     L.came = c.came ? 1 : 0; L.negate_grad = c.negate_grad ? 1 : 0; L.mode = c.mode; L.v_floor = c.v_floor;
-    L.param_dtype = c.param_dtype; L.sr = c.stochastic_round ? 1 : 0;
+    L.param_dtype = c.param_dtype; L.sr = c.stochastic_round ? 1 : 0; L.split = 0;
     return L;
 }
 
@@ -2050,29 +2364,39 @@ static int af8_factored_stats_impl(const af8_factored_cfg *cfg, const af8_factor
     if (cfg->mode == AF8_FSTAT_RESIDUAL && (!cfg->came || !dyn)) return fail(AF8_ERR_INVALID, "af8_factored_stats: the residual needs CAME and dyn");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int64_t tiles = 0;
-    // clear the accumulators; ranges that follow one another in memory share one memset
-    char *run_begin = nullptr, *run_end = nullptr;
+    // clear the accumulators: ranges that follow one another in memory form a run; one or two runs take a memset each
+    // (3 us of copy engine and gap apiece), more of them one launch over the table
+    // (29 tensors of odd sizes: 58 memsets, 93 us of a step)
+    struct { char *begin, *end; } run[2] = {};
+    int runs = 0;
     for (int i = 0; i < n_tensors; ++i) {
         const af8_factored_tensor &t = host_tensors[i];
         char *const ptr[2] = {reinterpret_cast<char *>(t.row_sum), reinterpret_cast<char *>(t.col_sum)};
         const size_t len[2] = {sizeof(double) * (size_t)t.rows, sizeof(double) * (size_t)(fact_batch(t) * t.cols)};
         for (int k = 0; k < 2; ++k) {
-            if (ptr[k] == run_end) { run_end += len[k]; continue; }
-            if (run_end != run_begin) AF8_CUDA_TRY(cudaMemsetAsync(run_begin, 0, (size_t)(run_end - run_begin), st));
-            run_begin = ptr[k];
-            run_end = ptr[k] + len[k];
+            if (runs > 0 && runs <= 2 && ptr[k] == run[runs - 1].end) { run[runs - 1].end += len[k]; continue; }
+            if (runs < 2) { run[runs].begin = ptr[k]; run[runs].end = ptr[k] + len[k]; }
+            if (runs < 3) ++runs;
         }
         tiles += fact_tiles(t);
     }
-    if (run_end != run_begin) AF8_CUDA_TRY(cudaMemsetAsync(run_begin, 0, (size_t)(run_end - run_begin), st));
-    FactoredLaunch L = make_factored_launch(*cfg, dev_tensors, n_tensors, tiles, dyn, nullptr);
-    int64_t grid = (int64_t)sm_count() * 6;
-    if (grid > tiles) grid = tiles;
+    if (runs <= 2) {
+        for (int k = 0; k < runs; ++k) AF8_CUDA_TRY(cudaMemsetAsync(run[k].begin, 0, (size_t)(run[k].end - run[k].begin), st));
+    } else {
+        factored_clear_kernel<<<dim3((unsigned)n_tensors, 4), 256, 0, st>>>(dev_tensors);
+        AF8_CUDA_TRY(cudaGetLastError());
+    }
     const bool bf = cfg->grad_dtype == AF8_BF16, res = cfg->mode == AF8_FSTAT_RESIDUAL;
     const bool vec = cfg->aligned8 && cfg->grad_dtype != AF8_F16;      // fp16 gradients take the general kernels
+    FactoredLaunch L = make_factored_launch(*cfg, dev_tensors, n_tensors, tiles, dyn, nullptr);
+    L.split = vec ? tile_split(tiles) : 0;
+    L.total_units = tiles << L.split;
+    int64_t grid = (int64_t)sm_count() * 6;
+    if (grid > L.total_units) grid = L.total_units;
     static const bool ring_off = getenv("AF8_NO_FACTORED_RING") != nullptr;
     static const bool box_off = getenv("AF8_NO_FACTORED_BOXES") != nullptr;
-    int ring = (ring_off || !res) ? 0 : 1;
+    const bool any = cfg->aligned8 == 2;
+    int ring = (ring_off || !res || any) ? 0 : 1;
     // residual pass over bf16 gradients and UF8 codes of tensors with cols % 256 == 0: boxes of rows through
     // tensor maps, when the caller has given room for the maps
     const CUtensorMap *maps = nullptr;
@@ -2096,8 +2420,9 @@ static int af8_factored_stats_impl(const af8_factored_cfg *cfg, const af8_factor
     }
 #define AF8_LAUNCH_FSTAT(G, RES) do { \
         const size_t sm = ring ? sring_smem_bytes<G, RES>() : 0; \
-        if (sm > 0) AF8_CUDA_TRY(cudaFuncSetAttribute(factored_stats_vec_kernel<G, RES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)); \
-        factored_stats_vec_kernel<G, RES><<<(int)grid, 256, sm, st>>>(L, ring, maps); } while (0)
+        if (sm > 0) AF8_CUDA_TRY(cudaFuncSetAttribute(factored_stats_vec_kernel<G, RES, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)); \
+        if (any) factored_stats_vec_kernel<G, RES, true><<<(int)grid, 256, 0, st>>>(L, 0, nullptr); \
+        else factored_stats_vec_kernel<G, RES, false><<<(int)grid, 256, sm, st>>>(L, ring, maps); } while (0)
     if (vec && bf && res) AF8_LAUNCH_FSTAT(bf16_tag, true);
     else if (vec && bf) AF8_LAUNCH_FSTAT(bf16_tag, false);
     else if (vec && res) AF8_LAUNCH_FSTAT(float, true);
@@ -2172,19 +2497,22 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
     static const bool wide_off = getenv("AF8_NO_WIDE_SUMS") != nullptr;
     static const bool tile_off = getenv("AF8_NO_TILE_SUMS") != nullptr;
     const int64_t total_tiles = cfg->total_tiles;
+    const bool any = cfg->aligned8 == 2;         // batches of matrices, rows of any length >= 8
     if (vec && !apply && !tile_off && total_tiles > 0 && cfg->grad_dtype != AF8_F16 && ((cfg->came && cfg->mode == AF8_FUPD_SUMSQ_U) || no_m)) {
         // the sum only needs the gradient: over the statistic tiles, column factors in registers
         AF8_CUDA_TRY(cudaMemsetAsync(block_sumsq, 0, sizeof(double) * (size_t)total_chunks, cst));
         FactoredLaunch LT = L;
-        LT.total_units = total_tiles;
-        int64_t tg = (int64_t)sm_count() * 8;
-        if (tg > total_tiles) tg = total_tiles;
-        if (bf) factored_sumsq_tile_kernel<bf16_tag><<<(int)tg, 256, 0, cst>>>(LT);
-        else factored_sumsq_tile_kernel<float><<<(int)tg, 256, 0, cst>>>(LT);
+        LT.split = tile_split(total_tiles);
+        LT.total_units = total_tiles << LT.split;
+        const int64_t tg = std::min<int64_t>((int64_t)sm_count() * 8, LT.total_units);
+        if (bf && any) factored_sumsq_tile_kernel<bf16_tag, true><<<(int)tg, 256, 0, cst>>>(LT);
+        else if (any) factored_sumsq_tile_kernel<float, true><<<(int)tg, 256, 0, cst>>>(LT);
+        else if (bf) factored_sumsq_tile_kernel<bf16_tag, false><<<(int)tg, 256, 0, cst>>>(LT);
+        else factored_sumsq_tile_kernel<float, false><<<(int)tg, 256, 0, cst>>>(LT);
         AF8_CUDA_TRY(cudaGetLastError());
         return AF8_OK;
     }
-    if (vec && !apply && !wide_off && cfg->grad_dtype != AF8_F16 && ((cfg->came && cfg->mode == AF8_FUPD_SUMSQ_U) || no_m)) {
+    if (vec && !any && !apply && !wide_off && cfg->grad_dtype != AF8_F16 && ((cfg->came && cfg->mode == AF8_FUPD_SUMSQ_U) || no_m)) {
         // the sum only needs the gradient: 16 elements per thread, next step's loads in flight
         if (bf) factored_sumsq_wide_kernel<bf16_tag><<<(int)grid, FUPD_THREADS, 0, cst>>>(L);
         else factored_sumsq_wide_kernel<float><<<(int)grid, FUPD_THREADS, 0, cst>>>(L);
@@ -2196,20 +2524,21 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
         cfg->total_tiles > 0 && cfg->cols_mult256) {
         // every row slice of 256 columns is one momentum block: tile order, column factors in registers
         FactoredLaunch LT = L;
-        LT.total_units = cfg->total_tiles;
+        LT.split = tile_split(cfg->total_tiles);
+        LT.total_units = cfg->total_tiles << LT.split;
         if (bf) {
-            int64_t tg = std::min<int64_t>((int64_t)sm_count() * 3, cfg->total_tiles);
+            int64_t tg = std::min<int64_t>((int64_t)sm_count() * 3, LT.total_units);
             AF8_CUDA_TRY(cudaFuncSetAttribute(factored_apply_tile_kernel<bf16_tag, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fring_smem_bytes<bf16_tag>()));
             factored_apply_tile_kernel<bf16_tag, 3><<<(int)tg, FUPD_THREADS, fring_smem_bytes<bf16_tag>(), cst>>>(LT);
         } else {
-            int64_t tg = std::min<int64_t>((int64_t)sm_count() * 2, cfg->total_tiles);
+            int64_t tg = std::min<int64_t>((int64_t)sm_count() * 2, LT.total_units);
             AF8_CUDA_TRY(cudaFuncSetAttribute(factored_apply_tile_kernel<float, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fring_smem_bytes<float>()));
             factored_apply_tile_kernel<float, 2><<<(int)tg, FUPD_THREADS, fring_smem_bytes<float>(), cst>>>(LT);
         }
         AF8_CUDA_TRY(cudaGetLastError());
         return AF8_OK;
     }
-    if (vec && cfg->mode == AF8_FUPD_APPLY && cfg->m_fmt == AF8_M_UF8 && cfg->param_dtype == AF8_F32 && !ring_off) {
+    if (vec && !any && cfg->mode == AF8_FUPD_APPLY && cfg->m_fmt == AF8_M_UF8 && cfg->param_dtype == AF8_F32 && !ring_off) {
         // fp32 parameters, UF8 momentum: inputs through per-warp rings of bulk copies
         if (bf) {
             AF8_CUDA_TRY(cudaFuncSetAttribute(factored_apply_ring_kernel<bf16_tag, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fring_smem_bytes<bf16_tag>()));
@@ -2222,7 +2551,16 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
         AF8_CUDA_TRY(cudaGetLastError());
         return AF8_OK;
     }
-#define AF8_LAUNCH_FUPD(G, P, C) factored_update_vec_kernel<G, P, C><<<(int)grid, FUPD_THREADS, 0, cst>>>(L)
+    if (vec && any) {                            // (writing: 2 resident CTAs; the sum pass: 3)
+        grid = std::min<int64_t>((int64_t)sm_count() * (apply ? 2 : 3), total_chunks);
+#define AF8_LAUNCH_FUPD(G, P, C) factored_update_vec_kernel<G, P, C, true><<<(int)grid, FUPD_THREADS, 0, cst>>>(L)
+        if (bf) { if (lag) AF8_LAUNCH_FUPD(bf16_tag, 2, 2); else if (apply) AF8_LAUNCH_FUPD(bf16_tag, 1, 2); else AF8_LAUNCH_FUPD(bf16_tag, 0, 3); }
+        else { if (lag) AF8_LAUNCH_FUPD(float, 2, 2); else if (apply) AF8_LAUNCH_FUPD(float, 1, 2); else AF8_LAUNCH_FUPD(float, 0, 3); }
+#undef AF8_LAUNCH_FUPD
+        AF8_CUDA_TRY(cudaGetLastError());
+        return AF8_OK;
+    }
+#define AF8_LAUNCH_FUPD(G, P, C) factored_update_vec_kernel<G, P, C, false><<<(int)grid, FUPD_THREADS, 0, cst>>>(L)
     if (vec && bf && lag) { if (no_m) AF8_LAUNCH_FUPD(bf16_tag, 2, 2); else AF8_LAUNCH_FUPD(bf16_tag, 2, 3); }
     else if (vec && lag) { if (no_m) AF8_LAUNCH_FUPD(float, 2, 2); else AF8_LAUNCH_FUPD(float, 2, 3); }
     else if (vec && bf && apply) { if (no_m) AF8_LAUNCH_FUPD(bf16_tag, 1, 2); else AF8_LAUNCH_FUPD(bf16_tag, 1, 3); }

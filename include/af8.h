@@ -297,7 +297,7 @@ typedef struct af8_small_state {
  * factored over its last two: optimizer.py:2203-2207).  For a batch the row arrays (row_sum, inv_row*, the row
  * states) still hold `rows` values, the column arrays (col_sum, inv_col*, the column states) hold
  * (rows / batch_rows) * cols values, matrix after matrix, and the mean that normalises the row factor is
- * taken per matrix.  Batches run through the general kernels: launch them with cfg.aligned8 = 0. */
+ * taken per matrix.  Launch batches with cfg.aligned8 = 0 or 2. */
 typedef struct af8_factored_tensor {
     void *param;                /* rows*cols elements of cfg.param_dtype */
     const void *grad;           /* fp32 or bf16 */
@@ -355,7 +355,9 @@ typedef struct af8_factored_cfg {
     int32_t mode;           /* AF8_FSTAT_* for af8_factored_stats, AF8_FUPD_* for af8_factored_update */
     float v_floor;          /* min_log floor of the AL requantisation (-126) */
     int32_t aligned8;       /* 1: every tensor has cols % 8 == 0 and 16-byte aligned arrays
-                               (checked by af8_factored_upload); selects the 128-bit kernels */
+                               (checked by af8_factored_upload); selects the 128-bit kernels.  2: every tensor has
+                               cols >= 8 and 16-byte aligned arrays; rows of any length and batches of matrices
+                               through the 128-bit kernels.  0: the general kernels */
     int32_t stochastic_round; /* as af8_fullrank_cfg.stochastic_round */
     int64_t total_tiles;    /* optional: the table's number of statistic tiles (the last tensor's first_tile plus its
                                own tiles).  With it the sum-of-squares passes that only read the gradient

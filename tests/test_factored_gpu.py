@@ -64,6 +64,33 @@ EXTRA_CASES.update({
                         hp=cases.CASES["came_al16"]["hp"]),
 })
 
+# rows of any length and batches of matrices through the 128-bit kernels: a row end inside a vector, the shortest
+# rows (8, 9), a partial last vector, a partial last momentum block, several chunks, fp32 gradients, one matrix of the
+# table with whole vectors; columns of a multiple of 256 in a batch (the write pass over the tiles).  (7, 5) and
+# (3, 7): fewer than 8 columns take the whole table to the general kernels.
+_ANY = [(9, 9), (5, 8), (131, 273), (700, 257), (64, 264)]
+_ANY3 = [(3, 70, 40), (2, 33, 131), (2, 600, 72)]
+_F32 = dict(cases.CASES["adafactor_factored"]["grad"], dtype="f32")
+EXTRA_CASES.update({
+    "adafactor_any": dict(shapes=_ANY, steps=3, seed=51, grad=cases.CASES["adafactor_factored"]["grad"],
+                          hp=cases.CASES["adafactor_factored"]["hp"]),
+    "adafactor_any_f32": dict(shapes=_ANY, steps=3, seed=52, grad=_F32, hp=cases.CASES["adafactor_factored"]["hp"]),
+    "adafactor_m_any": dict(shapes=_ANY, steps=3, seed=53, grad=cases.CASES["adafactor_factored_m"]["grad"],
+                            hp=cases.CASES["adafactor_factored_m"]["hp"]),
+    "adafactor_mf32_any": dict(shapes=_ANY, steps=3, seed=54, grad=_F32,
+                               hp=dict(cases.CASES["adafactor_factored_m"]["hp"], m_quant_type="fp32")),
+    "adafactor_m_any_lag": dict(shapes=_ANY, steps=4, seed=55, grad=cases.CASES["adafactor_factored_m"]["grad"],
+                                hp=dict(cases.CASES["adafactor_factored_m"]["hp"], lag_norm=True)),
+    "came_any": dict(shapes=_ANY, steps=3, seed=56, grad=cases.CASES["came_al16"]["grad"], hp=cases.CASES["came_al16"]["hp"]),
+    "adafactor_any_short": dict(shapes=[(7, 5), (3, 7), (40, 33)], steps=3, seed=57,
+                                grad=cases.CASES["adafactor_factored"]["grad"], hp=cases.CASES["adafactor_factored"]["hp"]),
+    "adafactor_any_3d": dict(shapes=_ANY3, steps=3, seed=58, grad=cases.CASES["adafactor_factored"]["grad"],
+                             hp=cases.CASES["adafactor_factored"]["hp"]),
+    "came_any_3d": dict(shapes=_ANY3, steps=3, seed=59, grad=cases.CASES["came_al16"]["grad"], hp=cases.CASES["came_al16"]["hp"]),
+    "adafactor_m_256_3d": dict(shapes=[(3, 40, 256), (2, 530, 512)], steps=3, seed=60,
+                               grad=cases.CASES["adafactor_factored_m"]["grad"], hp=cases.CASES["adafactor_factored_m"]["hp"]),
+})
+
 # lag_norm=True (one pass with the previous step's norm; optimizer.py:1056-1071): the vector kernels, the
 # element-wise kernels (odd column counts) and the limiter on top of the clip
 EXTRA_CASES.update({
