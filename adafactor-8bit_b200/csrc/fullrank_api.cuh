@@ -189,19 +189,27 @@ inline int launch_stat(const FullrankLaunch &L, cudaStream_t st)
     return AF8_OK;
 }
 
-template <typename GradT, int MODE>
-inline int launch_generic(const FullrankLaunch &L, const GenericCfg &C, cudaStream_t st)
+template <typename GradT, int MODE, int THREADS>
+inline int launch_generic_threads(const FullrankLaunch &L, const GenericCfg &C, bool plain, cudaStream_t st)
 {
-    const size_t smem = (size_t)2 * C.block * sizeof(float);
-    auto kernel = fullrank_generic_kernel<GradT, MODE>;
+    const size_t smem = plain ? 0 : (size_t)2 * C.block * sizeof(float);       // (only quantised states are staged)
+    auto kernel = fullrank_generic_kernel<GradT, MODE, THREADS>;
     if (smem > 48 * 1024)
         AF8_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int grid = 0;
-    int rc = persistent_grid(kernel, GEN_THREADS, smem, L.total_blocks, &grid);
+    int rc = persistent_grid(kernel, THREADS, smem, L.total_blocks, &grid);
     if (rc) return rc;
-    kernel<<<grid, GEN_THREADS, smem, st>>>(L, C);
+    kernel<<<grid, THREADS, smem, st>>>(L, C);
     AF8_CUDA_TRY(cudaGetLastError());
     return AF8_OK;
+}
+
+template <typename GradT, int MODE>
+inline int launch_generic(const FullrankLaunch &L, const GenericCfg &C, cudaStream_t st)
+{
+    const bool plain = (C.v_fmt == AF8_V_FP32 || C.v_fmt == AF8_V_NONE) && (C.m_fmt == AF8_M_NONE || C.m_fmt == AF8_M_FP32);
+    return plain && L.total_blocks <= 2 * (int64_t)sm_count() ? launch_generic_threads<GradT, MODE, 1024>(L, C, plain, st)
+                                                              : launch_generic_threads<GradT, MODE, GEN_THREADS>(L, C, plain, st);
 }
 
 // the general kernel in any mode

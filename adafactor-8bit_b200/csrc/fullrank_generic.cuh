@@ -83,15 +83,18 @@ __device__ __forceinline__ uint32_t m_encode(float m, float a, int fmt)
 // MODE: AF8_MODE_NOCLIP / SUMSQ / APPLY, plus 3 = SUMSQ of the momentum update
 // on the momentum-only path (reads dyn.pre_div like APPLY, writes nothing but
 // the partial sums).
-template <typename GradT, int MODE>
-__global__ void __launch_bounds__(GEN_THREADS)
+// THREADS: 256, or 1024 where neither state is quantised and there are at most two blocks per SM (the norm vectors and
+// biases of a model, tensors of a few thousand elements): each of the few CTAs walked its block in eight dependent rounds
+// of loads.  45 vectors of 2048 elements: 23 -> 9 us in one pass, 19 + 16 -> 9 + 8 us in two.
+template <typename GradT, int MODE, int THREADS>
+__global__ void __launch_bounds__(THREADS)
 fullrank_generic_kernel(const FullrankLaunch L, const GenericCfg C)
 {
     extern __shared__ float s_dyn[];
     float *s_l = s_dyn;                 // log2 of the new v, -inf marks exact zero
     float *s_m = s_dyn + C.block;       // new momentum
     __shared__ af8_fullrank_tensor sT;
-    __shared__ float s_red[3][GEN_THREADS / 32];
+    __shared__ float s_red[3][THREADS / 32];
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
@@ -142,7 +145,7 @@ fullrank_generic_kernel(const FullrankLaunch L, const GenericCfg C)
 
         float acc = 0.0f, mn = INFINITY, mx = -INFINITY;
 
-        for (int i = tid; i < C.block; i += GEN_THREADS) {
+        for (int i = tid; i < C.block; i += THREADS) {
             const bool real = i < valid;
             float vj = 0.0f, mj = 0.0f;
             if (real) {
@@ -237,7 +240,7 @@ fullrank_generic_kernel(const FullrankLaunch L, const GenericCfg C)
             __syncthreads();
             if (tid == 0) {
                 float s = 0.0f;
-                for (int w = 0; w < GEN_THREADS / 32; ++w) s = __fadd_rn(s, s_red[2][w]);
+                for (int w = 0; w < THREADS / 32; ++w) s = __fadd_rn(s, s_red[2][w]);
                 L.block_sumsq[blk] = s;
             }
             if (!writes) continue;
@@ -250,13 +253,13 @@ fullrank_generic_kernel(const FullrankLaunch L, const GenericCfg C)
         }
         __syncthreads();   // s_l, s_m and the warp extrema are visible
         if (v_quant) {
-            for (int w = 0; w < GEN_THREADS / 32; ++w) {
+            for (int w = 0; w < THREADS / 32; ++w) {
                 mn = fminf(mn, s_red[0][w]);
                 mx = fmaxf(mx, s_red[1][w]);
             }
             float min_log, scale;
             al_range(mn, mx, L.v_floor, min_log, scale);
-            for (int i = tid; i < C.block; i += GEN_THREADS) {
+            for (int i = tid; i < C.block; i += THREADS) {
                 const float l = s_l[i];
                 const bool zero = (l == -INFINITY);
                 const uint32_t code = zero ? 0u : al_encode(1.0f, l, min_log, scale, qm1, qmax);
@@ -269,7 +272,7 @@ fullrank_generic_kernel(const FullrankLaunch L, const GenericCfg C)
             // the M state is padded to a multiple of m_block only: sub-blocks that
             // start at or beyond numel do not exist
             const bool four_bit = (C.m_fmt == AF8_M_UF4 || C.m_fmt == AF8_M_D4);
-            for (int sb = warp; sb < subs_per_block; sb += GEN_THREADS / 32) {
+            for (int sb = warp; sb < subs_per_block; sb += THREADS / 32) {
                 const int s0 = sb * C.m_block;
                 if (s0 >= valid) break;
                 float am = 0.0f;
