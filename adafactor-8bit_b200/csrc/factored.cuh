@@ -105,14 +105,16 @@ __device__ __forceinline__ TilePos tile_pos(const FactoredLaunch &L, const af8_f
     return p;
 }
 
-// Parts per tile, as a power of two: a 512-row tile is 131072 elements, so a small table has fewer tiles than the
-// chip has resident CTAs (444 to 592) and its last wave is most of its time.  Tiles are halved, down to 64 rows,
-// while they give less than about eight waves of half-used SMs; smaller parts only add column atomics (256 per part).
-// 8 layers of 512 x 1376 with CAME, 256 tiles: see factored_stats_vec_kernel for the times.
-inline int tile_split(int64_t tiles)
+// Parts per tile, as a power of two: a 512-row tile is 131072 elements, so a table of fewer than about 40 M parameters
+// has fewer tiles than CTAs that are resident together (3 per SM in the kernels with the most registers).  Tiles are
+// halved, down to 64 rows, while the parts still run in one wave: a part costs a fixed 4 us or so (pipeline fill, the
+// reduction over the warps, 256 column atomics), so that more waves of smaller parts lose - 256 tiles of an 8-layer
+// 512 x 1376 model: statistic pass 23 us whole, 42 us in eighths; sum pass 21 and 27 us.  CAME's residual pass spends
+// several times as long on a row, so that up to five waves of parts still gain there: 126 us whole, 98 us in eighths.
+inline int tile_split(int64_t tiles, int waves = 1)
 {
     int sh = 0;
-    while (sh < 3 && (tiles << sh) < 1776) ++sh;
+    while (sh < 3 && (tiles << (sh + 1)) <= 3 * waves * (int64_t)sm_count()) ++sh;
     return sh;
 }
 
@@ -306,11 +308,12 @@ factored_clear_kernel(const af8_factored_tensor *tensors)
 // ---------------------------------------------------------------------------
 // small states
 // ---------------------------------------------------------------------------
+constexpr int SMALL_MAX_THREADS = 512;
 // EMA + requantisation of block b of one small state of n elements (optimizer.py:2232-2238,
 // 937-946, 2248-2251).  `out` receives the un-requantised values.  Returns this thread's partial
 // sum of the block's values (binary64) for the mean of the row state.
 __device__ double small_state_block(const af8_small_state &S, const double *sums, double count, int64_t n, int64_t b,
-                                    float eps_add, float w, float floor_log, float *out, float *s_l, float (*s_red)[8])
+                                    float eps_add, float w, float floor_log, float *out, float *s_l, float (*s_red)[SMALL_MAX_THREADS / 32])
 {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int block = S.block;
@@ -350,7 +353,7 @@ __device__ double small_state_block(const af8_small_state &S, const double *sums
     mx = warp_max(mx);
     if (lane == 0) { s_red[0][warp] = mn; s_red[1][warp] = mx; }
     __syncthreads();
-    for (int w8 = 0; w8 < 8; ++w8) { mn = fminf(mn, s_red[0][w8]); mx = fmaxf(mx, s_red[1][w8]); }
+    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) { mn = fminf(mn, s_red[0][k]); mx = fmaxf(mx, s_red[1][k]); }
     float min_log, scale;
     al_range(mn, mx, floor_log, min_log, scale);
     for (int i = tid; i < block; i += blockDim.x) {
@@ -376,12 +379,14 @@ __device__ __forceinline__ int find_factored_small(const af8_factored_tensor *t,
 
 // One CTA per quantisation block of a row or column state: every block of every tensor in
 // parallel (a 32000-row state has 125 blocks of 256; one CTA per tensor walked them in turn).
-__global__ void __launch_bounds__(256)
+// A thread walks block / THREADS elements with binary64 logarithms.
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS)
 factored_small_kernel(const af8_factored_tensor *tensors, int n_tensors, int conf, float floor_log)
 {
     extern __shared__ float s_l[];
-    __shared__ float s_red[2][8];
-    __shared__ double s_acc[8];
+    __shared__ float s_red[2][SMALL_MAX_THREADS / 32];
+    __shared__ double s_acc[SMALL_MAX_THREADS / 32];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int t = find_factored_small(tensors, n_tensors, (int)blockIdx.x);
     const af8_factored_tensor T = tensors[t];
@@ -409,7 +414,7 @@ factored_small_kernel(const af8_factored_tensor *tensors, int n_tensors, int con
     __syncthreads();                                            // (also: every thread has read its row sums)
     if (tid == 0) {
         double s = 0.0;
-        for (int k = 0; k < 8; ++k) s += s_acc[k];
+        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) s += s_acc[k];
         T.row_sum[b * block] = s;
     }
 }
@@ -770,6 +775,23 @@ __device__ __forceinline__ void load_cols_any(const float *p, int64_t col, int64
 {
 #pragma unroll
     for (int j = 0; j < 8; ++j) x[j] = col + j < C ? __ldg(p + col + j) : 0.0f;
+}
+
+// values i .. i + 7 of a 16-byte aligned array, i of any alignment: the two or three aligned vectors around them, shifted
+// (24 cache-line accesses a warp instead of 64 for eight scalar loads).  The last vector holds value i + 7; arrays are
+// allocated in multiples of 4 values.
+__device__ __forceinline__ void load_cols8_shifted(const float *v, int64_t i, float (&x)[8])
+{
+    const int s = (int)(i & 3);
+    const float4 *p = reinterpret_cast<const float4 *>(v + (i - s));
+    const float4 a = __ldg(p), b = __ldg(p + 1);
+    float4 c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (s) c = __ldg(p + 2);
+    float w[11] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z};
+#pragma unroll
+    for (int j = 0; j < 9; ++j) w[j] = (s & 2) ? w[j + 2] : w[j];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] = (s & 1) ? w[j + 1] : w[j];
 }
 
 // stats_rows for rows of any length: elements beyond the row's end count as zeros, all loads through GradAny8
@@ -1329,12 +1351,14 @@ factored_stats_vec_kernel(const FactoredLaunch L, const int use_ring, const CUte
 // CTAS: resident CTAs per SM asked of the compiler.  Measured on B200: 4 for the sum passes; for the
 // writing passes 3 with momentum (CAME, 0.78 ms per Llama-2-7B layer) and 2 without (Adafactor on the
 // TinyLlama set: 2.51 -> 2.21 ms, no register spills).
-// ANY: tensors with batches of matrices or with rows of any length >= 8.  The flat vectors of 8 stay aligned; a vector
-// crosses at most one row end, so its elements take one of two row factors and column factors that are loaded one by
-// one (for rows of a multiple of 8: as vectors).  Only a tensor's last vector may be partial.  The squares of the sum
-// passes enter binary64 one by one, as in factored_update_kernel, which such tensors took before: 59 M parameters of
-// odd sizes, UF8 momentum: see the figures there.
-template <typename GradT, int PASS, int CTAS, bool ANY>
+// ANY = 1: batches of matrices, rows of a multiple of 8.  ANY = 2: rows of any length >= 8 as well.  The flat vectors of
+// 8 stay aligned; a vector crosses at most one row end, so its elements take one of two row factors, and column factors
+// from three aligned vectors that are shifted (one by one in a lane with a row end).  Only a tensor's last vector may be
+// partial.  The squares of the sum
+// passes enter binary64 one by one, as in factored_update_kernel, which such tensors took before.  Write pass with bf16
+// gradients: 59 M parameters of odd sizes with a UF8 momentum 1 ms -> 252 us (issue and latency bound, 500 instructions
+// per 256 elements), 138 M in batches without momentum 1.55 ms -> 245 us (325 us with the tests of ANY = 2).
+template <typename GradT, int PASS, int CTAS, int ANY>
 __global__ void __launch_bounds__(FUPD_THREADS, CTAS)
 factored_update_vec_kernel(const FactoredLaunch L)
 {
@@ -1424,7 +1448,7 @@ factored_update_vec_kernel(const FactoredLaunch L)
         (void)t;
         const int64_t numel = sT.rows * sT.cols;
         const bool ok = flat < numel;                                // numel % 8 == 0: all 8 or none
-        const bool partial = ANY && ok && flat + 8 > numel;          // (the tensor's last elements)
+        const bool partial = ANY == 2 && ok && flat + 8 > numel;          // (the tensor's last elements)
         const int nval = partial ? (int)(numel - flat) : 8;
         // this chunk's streams, loaded one iteration ahead when the chunk is in the same tensor
         GradRaw8<GradT> cg;
@@ -1475,7 +1499,7 @@ factored_update_vec_kernel(const FactoredLaunch L)
 #endif
         {
             const int64_t nf = flat + 2048;                          // the next chunk of this CTA, if it is in this tensor
-            have = id + 1 < id_end && (ANY ? nf + 8 <= numel : nf < numel);
+            have = id + 1 < id_end && (ANY == 2 ? nf + 8 <= numel : nf < numel);
             if (have) {
                 ng.load(sT.grad, nf);
                 if (writes) {
@@ -1496,28 +1520,31 @@ factored_update_vec_kernel(const FactoredLaunch L)
             int wrap = 8;
             int64_t cb0 = 0, cb1 = 0, irow1 = row;
             bool whole = true;                                       // the columns come as vectors
-            if constexpr (ANY) {
+            if constexpr (ANY == 2) {
                 whole = (sT.cols & 7) == 0;
                 if (!whole) {
                     wrap = (int)min((int64_t)8, sT.cols - col);
                     irow1 = min(row + 1, sT.rows - 1);
                 }
+            }
+            if constexpr (ANY != 0) {
                 if (sT.batch_rows > 0) {                             // (rows < 2^31)
                     cb0 = (int64_t)((uint32_t)row / (uint32_t)sT.batch_rows) * sT.cols;
-                    cb1 = (int64_t)((uint32_t)irow1 / (uint32_t)sT.batch_rows) * sT.cols;
+                    if (ANY == 2) cb1 = (int64_t)((uint32_t)irow1 / (uint32_t)sT.batch_rows) * sT.cols;
                 }
             }
             auto cols8 = [&](const float *v, float (&x)[8]) {
-                if (!ANY || whole) { load_f8_ro(v + cb0 + col, x); return; }
+                if (ANY != 2 || whole) { load_f8_ro(v + cb0 + col, x); return; }
+                if (wrap == 8) { load_cols8_shifted(v, cb0 + col, x); return; }
                 const float *va = v + cb0 + col, *vb = v + cb1 - wrap;
 #pragma unroll
                 for (int j = 0; j < 8; ++j) x[j] = __ldg((j < wrap ? va : vb) + j);
             };
             auto row2 = [&](float a, float b, int j) {               // the row factors of elements j, j + 1
-                return ANY ? make_float2(j < wrap ? a : b, j + 1 < wrap ? a : b) : bc2(a);
+                return ANY == 2 ? make_float2(j < wrap ? a : b, j + 1 < wrap ? a : b) : bc2(a);
             };
             cols8(sT.inv_col, ic);
-            const float ir = __ldg(sT.inv_row + row), irb = ANY ? __ldg(sT.inv_row + irow1) : 0.0f;
+            const float ir = __ldg(sT.inv_row + row), irb = ANY == 2 ? __ldg(sT.inv_row + irow1) : 0.0f;
             // pairs of elements in packed binary32 arithmetic (bit-identical to the element-wise form)
             if (L.came) {
                 if (L.mode == AF8_FUPD_SUMSQ_U) {
@@ -1533,7 +1560,7 @@ factored_update_vec_kernel(const FactoredLaunch L)
                         for (int j = 0; j < 8; ++j) mo[j] = j < nval ? sT.m_f32[flat + j] : 0.0f;
                     } else m_old8(sT, L.m_fmt, 256, flat, mo, pre_m, cm);
                     cols8(sT.inv_col_conf, icc);
-                    const float irc = __ldg(sT.inv_row_conf + row), ircb = ANY ? __ldg(sT.inv_row_conf + irow1) : 0.0f;
+                    const float irc = __ldg(sT.inv_row_conf + row), ircb = ANY == 2 ? __ldg(sT.inv_row_conf + irow1) : 0.0f;
 #pragma unroll
                     for (int j = 0; j < 8; j += 2) {
                         const float2 ut = div_by2(__fmul2_rn(__fmul2_rn(make_float2(g[j], g[j + 1]), row2(ir, irb, j)), make_float2(ic[j], ic[j + 1])), D);
@@ -1566,7 +1593,7 @@ factored_update_vec_kernel(const FactoredLaunch L)
                 for (int j = 0; j < 8; ++j)
                     if (j >= nval) { u[j] = 0.0f; mj[j] = 0.0f; }
             }
-            if (SUMS && ANY) {
+            if (SUMS && ANY != 0) {
 #pragma unroll
                 for (int j = 0; j < 8; ++j) part += (double)__fmul_rn(u[j], u[j]);
             } else if (SUMS) {
@@ -1653,7 +1680,7 @@ factored_update_vec_kernel(const FactoredLaunch L)
                     const DivBy A = make_div(am);
                     const uint32_t o0 = uf8_encode_fast2(make_float2(mj[0], mj[1]), A) | (uf8_encode_fast2(make_float2(mj[2], mj[3]), A) << 16);
                     const uint32_t o1 = uf8_encode_fast2(make_float2(mj[4], mj[5]), A) | (uf8_encode_fast2(make_float2(mj[6], mj[7]), A) << 16);
-                    if (ANY || ok) *reinterpret_cast<uint2 *>(sT.m_q + flat) = make_uint2(o0, o1);
+                    if (ANY != 0 || ok) *reinterpret_cast<uint2 *>(sT.m_q + flat) = make_uint2(o0, o1);
                 } else if (L.m_fmt == AF8_M_D8) {
                     uint32_t o0 = 0, o1 = 0;
 #pragma unroll
@@ -1661,13 +1688,13 @@ factored_update_vec_kernel(const FactoredLaunch L)
                         o0 |= m_encode(mj[j], am, L.m_fmt) << (8 * j);
                         o1 |= m_encode(mj[j + 4], am, L.m_fmt) << (8 * j);
                     }
-                    if (ANY || ok) *reinterpret_cast<uint2 *>(sT.m_q + flat) = make_uint2(o0, o1);
+                    if (ANY != 0 || ok) *reinterpret_cast<uint2 *>(sT.m_q + flat) = make_uint2(o0, o1);
                 } else {
                     uint32_t o = 0;
 #pragma unroll
                     for (int j = 0; j < 8; j += 2)
                         o |= ((m_encode(mj[j], am, L.m_fmt) << 4) | m_encode(mj[j + 1], am, L.m_fmt)) << (4 * j);
-                    if (ANY || ok) *reinterpret_cast<uint32_t *>(sT.m_q + (flat >> 1)) = o;
+                    if (ANY != 0 || ok) *reinterpret_cast<uint32_t *>(sT.m_q + (flat >> 1)) = o;
                 }
                 if (lane == 0) sT.m_scale[w0 / 256] = am;
             }
@@ -2243,6 +2270,7 @@ inline int validate_factored(const af8_factored_cfg &c, const af8_factored_tenso
         if (t.rows <= 0 || t.cols <= 0) return fail(AF8_ERR_INVALID, "factored tensor %d: empty shape", i);
         if (c.aligned8) {
             if (c.aligned8 != 2 && t.cols % 8 != 0) return fail(AF8_ERR_INVALID, "factored tensor %d: aligned8 needs cols %% 8 == 0", i);
+            if (c.aligned8 == 2 && c.cols_mult8 && t.cols % 8) return fail(AF8_ERR_INVALID, "factored tensor %d: cols_mult8 needs cols %% 8 == 0", i);
             if (c.aligned8 == 2 && t.cols < 8) return fail(AF8_ERR_INVALID, "factored tensor %d: aligned8 = 2 needs cols >= 8", i);
             const void *ptrs[] = {t.param, t.grad, t.m_q, t.m_f32, t.inv_col, t.inv_col_conf, t.param_copy};
             for (const void *q : ptrs)
@@ -2389,7 +2417,7 @@ static int af8_factored_stats_impl(const af8_factored_cfg *cfg, const af8_factor
     const bool bf = cfg->grad_dtype == AF8_BF16, res = cfg->mode == AF8_FSTAT_RESIDUAL;
     const bool vec = cfg->aligned8 && cfg->grad_dtype != AF8_F16;      // fp16 gradients take the general kernels
     FactoredLaunch L = make_factored_launch(*cfg, dev_tensors, n_tensors, tiles, dyn, nullptr);
-    L.split = vec ? tile_split(tiles) : 0;
+    L.split = vec ? tile_split(tiles, res ? 5 : 1) : 0;
     L.total_units = tiles << L.split;
     int64_t grid = (int64_t)sm_count() * 6;
     if (grid > L.total_units) grid = L.total_units;
@@ -2457,7 +2485,10 @@ extern "C" int af8_factored_small(const af8_factored_cfg *cfg, const af8_factore
     if (conf && !cfg->came) return fail(AF8_ERR_INVALID, "af8_factored_small: confidence states exist only with CAME");
     const size_t smem = sizeof(float) * GEN_MAX_BLOCK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    factored_small_kernel<<<total_units, 256, smem, st>>>(dev_tensors, n_tensors, conf, cfg->v_floor);
+    // at most one unit per SM (blocks of 2048, few tensors): the launch lasts as long as one CTA, so more threads
+    // (8 layers of 512 x 1376 with CAME: 12.3 -> 10 us a launch; 480 units of 256 elements: 6.2 us with 256, 14 with 512)
+    if (total_units <= sm_count()) factored_small_kernel<SMALL_MAX_THREADS><<<total_units, SMALL_MAX_THREADS, smem, st>>>(dev_tensors, n_tensors, conf, cfg->v_floor);
+    else factored_small_kernel<256><<<total_units, 256, smem, st>>>(dev_tensors, n_tensors, conf, cfg->v_floor);
     AF8_CUDA_TRY(cudaGetLastError());
     factored_inv_kernel<<<dim3((unsigned)n_tensors, 8), 256, 0, st>>>(dev_tensors, conf);
     AF8_CUDA_TRY(cudaGetLastError());
@@ -2553,14 +2584,15 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
     }
     if (vec && any) {                            // (writing: 2 resident CTAs; the sum pass: 3)
         grid = std::min<int64_t>((int64_t)sm_count() * (apply ? 2 : 3), total_chunks);
-#define AF8_LAUNCH_FUPD(G, P, C) factored_update_vec_kernel<G, P, C, true><<<(int)grid, FUPD_THREADS, 0, cst>>>(L)
+#define AF8_LAUNCH_FUPD(G, P, C) do { if (cfg->cols_mult8) factored_update_vec_kernel<G, P, C, 1><<<(int)grid, FUPD_THREADS, 0, cst>>>(L); \
+        else factored_update_vec_kernel<G, P, C, 2><<<(int)grid, FUPD_THREADS, 0, cst>>>(L); } while (0)
         if (bf) { if (lag) AF8_LAUNCH_FUPD(bf16_tag, 2, 2); else if (apply) AF8_LAUNCH_FUPD(bf16_tag, 1, 2); else AF8_LAUNCH_FUPD(bf16_tag, 0, 3); }
         else { if (lag) AF8_LAUNCH_FUPD(float, 2, 2); else if (apply) AF8_LAUNCH_FUPD(float, 1, 2); else AF8_LAUNCH_FUPD(float, 0, 3); }
 #undef AF8_LAUNCH_FUPD
         AF8_CUDA_TRY(cudaGetLastError());
         return AF8_OK;
     }
-#define AF8_LAUNCH_FUPD(G, P, C) factored_update_vec_kernel<G, P, C, false><<<(int)grid, FUPD_THREADS, 0, cst>>>(L)
+#define AF8_LAUNCH_FUPD(G, P, C) factored_update_vec_kernel<G, P, C, 0><<<(int)grid, FUPD_THREADS, 0, cst>>>(L)
     if (vec && bf && lag) { if (no_m) AF8_LAUNCH_FUPD(bf16_tag, 2, 2); else AF8_LAUNCH_FUPD(bf16_tag, 2, 3); }
     else if (vec && lag) { if (no_m) AF8_LAUNCH_FUPD(float, 2, 2); else AF8_LAUNCH_FUPD(float, 2, 3); }
     else if (vec && bf && apply) { if (no_m) AF8_LAUNCH_FUPD(bf16_tag, 1, 2); else AF8_LAUNCH_FUPD(bf16_tag, 1, 3); }

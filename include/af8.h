@@ -357,7 +357,8 @@ typedef struct af8_factored_cfg {
     int32_t aligned8;       /* 1: every tensor has cols % 8 == 0 and 16-byte aligned arrays
                                (checked by af8_factored_upload); selects the 128-bit kernels.  2: every tensor has
                                cols >= 8 and 16-byte aligned arrays; rows of any length and batches of matrices
-                               through the 128-bit kernels.  0: the general kernels */
+                               through the 128-bit kernels (inv_col and inv_col_conf are then allocated in
+                               multiples of 4 values).  0: the general kernels */
     int32_t stochastic_round; /* as af8_fullrank_cfg.stochastic_round */
     int64_t total_tiles;    /* optional: the table's number of statistic tiles (the last tensor's first_tile plus its
                                own tiles).  With it the sum-of-squares passes that only read the gradient
@@ -365,7 +366,8 @@ typedef struct af8_factored_cfg {
                                factors in registers; 0: over the flat chunks */
     int32_t cols_mult256;   /* 1: every tensor of the table has cols % 256 == 0 (with total_tiles: the write pass with a
                                UF8 momentum then also runs over the tiles, a row slice being one momentum block) */
-    int32_t reserved;
+    int32_t cols_mult8;     /* with aligned8 = 2: 1 if every tensor of the table has cols % 8 == 0 (batches of matrices
+                               whose rows come as whole vectors) */
 } af8_factored_cfg;
 
 /* Number of flattened elements per work unit of af8_factored_update for a
