@@ -177,6 +177,8 @@ class _PinnedRing:
         _RETIRED[:] = [x for x in _RETIRED if not x[1].query()]
         self.bufs = [torch.empty(max(nbytes, 16), dtype=torch.uint8, pin_memory=True) for _ in range(depth)]
         self.events = [None] * depth
+        self.views = [b.numpy() for b in self.bufs]
+        self.tables = {}
         self.i = 0
 
     def next(self):
@@ -185,6 +187,13 @@ class _PinnedRing:
         if ev is not None:
             ev.synchronize()
         return self.bufs[self.i]
+
+    def table(self, dtype, n):
+        """The current buffer's first n records of dtype."""
+        t = self.tables.get((self.i, dtype.itemsize, n))
+        if t is None:
+            t = self.tables[self.i, dtype.itemsize, n] = self.views[self.i][: n * dtype.itemsize].view(dtype)
+        return t
 
     def mark(self, stream):
         ev = self.events[self.i]
@@ -251,7 +260,7 @@ class FullrankPlan:
 
         self.d_table = torch.empty(n * N.FULLRANK_TENSOR.itemsize, dtype=torch.uint8, device=self.device)
         self.d_dyn = torch.zeros(n * N.DYN_SCALARS.itemsize, dtype=torch.uint8, device=self.device)
-        self.d_norm = torch.empty(n * N.NORM_TENSOR.itemsize, dtype=torch.uint8, device=self.device)
+        self._norm_tables = {}       # (pre_div_mode, exchange) -> (inputs, limiter pointers, device table) of norm_finalize
         self.d_sumsq = None
         self.h_table = _PinnedRing(n * N.FULLRANK_TENSOR.itemsize)
         self.h_norm = _PinnedRing(n * N.NORM_TENSOR.itemsize)
@@ -306,7 +315,7 @@ class FullrankPlan:
             self._static = self._static_fields()
             self._ptr_sig = sig
         buf = self.h_table.next()
-        table = buf.numpy()[: self.n * N.FULLRANK_TENSOR.itemsize].view(N.FULLRANK_TENSOR)
+        table = self.h_table.table(N.FULLRANK_TENSOR, self.n)
         table[:] = self._static
         table["grad"] = [g.data_ptr() for g in grads]
         for k in ("decay", "alpha", "v_w", "v_keep", "v_eps_add", "m_w", "eps_gradsq", "eps_denom", "eps_sq"):
@@ -349,40 +358,9 @@ class FullrankPlan:
             a = int(first[i])
             _add_to_slot(self.pieces[i].slots[x], k, partials[a:a + int(count[i])])
 
-    def _finalize(self, table, pre_div_mode, d, fira, fira_margin, stream, x=None, k=1):
+    def _finalize(self, pre_div_mode, d, fira, fira_margin, stream, x=None, k=1):
         """x, k: exchange index and scalar index where the whole sums of the cut entries are."""
-        buf = self.h_norm.next()
-        nt = buf.numpy()[: self.n * N.NORM_TENSOR.itemsize].view(N.NORM_TENSOR)
-        nt["first_block"] = self.first_block
-        nt["n_blocks"] = self.nblocks
-        if x is not None:
-            for i in self.cut:
-                nt["n_blocks"][i] = -1
-                nt["first_block"][i] = self.pieces[i].slots[x].data_ptr() + 8 * k
-        nt["pre_div_mode"] = pre_div_mode
-        nt["partials_f64"] = 0
-        nt["alpha"] = table["alpha"]
-        if self._alpha_on_device:
-            nt["alpha_dev"] = (self.d_table.data_ptr() + np.arange(self.n, dtype=np.uint64) * np.uint64(N.FULLRANK_TENSOR.itemsize)
-                               + np.uint64(N.FULLRANK_TENSOR.fields["alpha"][1]))
-        else:
-            nt["alpha_dev"] = 0
-        sqrt_n = np.sqrt(self.full_numel.astype(np.float64))
-        nt["sqrt_n"] = sqrt_n.astype(np.float32)
-        nt["d"] = np.float32(d)
-        use_clip = d > 0 and pre_div_mode == 0
-        nt["clip_div"] = (sqrt_n * d).astype(np.float32) if use_clip else np.float32(0.0)
-        nt["fira_margin1"] = np.float32(1.0 + fira_margin)
-        if fira and pre_div_mode != 1:
-            nt["fira_prev"], nt["fira_has_prev"] = fira_state_pointers(self)
-        else:
-            nt["fira_prev"] = 0
-            nt["fira_has_prev"] = 0
-        self.d_norm.copy_(buf[: self.d_norm.numel()], non_blocking=True)
-        self.h_norm.mark(stream)
-        rc = N.lib().af8_norm_finalize(self.d_norm.data_ptr(), self.n, self.d_sumsq.data_ptr(),
-                                       self.d_dyn.data_ptr(), stream.cuda_stream)
-        N.check(rc, "af8_norm_finalize")
+        norm_finalize(self, self.first_block, self.nblocks, 0, N.FULLRANK_TENSOR, pre_div_mode, d, fira, fira_margin, stream, x, k)
 
     def _scale_table(self, buf, scale, stream):
         """Upload the launch table and fill the host table of the parameter-RMS passes
@@ -492,7 +470,7 @@ class FullrankPlan:
             if scale is not None:
                 self._param_finish(stream)
             if need_stat:
-                self._finalize(table, 0, d, fira, fira_margin, stream, x, 1)
+                self._finalize(0, d, fira, fira_margin, stream, x, 1)
                 self._step(N.MODE_APPLY, None, stream)
             else:
                 self._step(N.MODE_NOCLIP, buf, stream)
@@ -512,7 +490,7 @@ class FullrankPlan:
             if scale is not None:
                 self._param_finish(stream)
             if clip_first:
-                self._finalize(table, 1, d, False, fira_margin, stream, x, 1)
+                self._finalize(1, d, False, fira_margin, stream, x, 1)
             x += 1
         if not clip_first:
             self.d_dyn.view(torch.float32).view(self.n, 8)[:, 2] = 1.0   # pre_div
@@ -521,13 +499,51 @@ class FullrankPlan:
             pending = None
             self._sums_to_slots(x, 1, self.d_sumsq, self.first_block, self.nblocks)
             yield
-            self._finalize(table, 2, 0.0, True, fira_margin, stream, x, 1)
+            self._finalize(2, 0.0, True, fira_margin, stream, x, 1)
         self._step(N.MODE_APPLY, pending, stream)
 
     def norms(self):
         """Update norms measured by the last two-pass step (one per tensor)."""
         dyn = self.d_dyn.cpu().numpy().view(N.DYN_SCALARS)
         return dyn["norm"].copy()
+
+
+def norm_finalize(plan, first, count, f64, table_dtype, pre_div_mode, d, fira, fira_margin, stream, x, k):
+    """Enqueue af8_norm_finalize for a plan.  Everything in its table is fixed by the options of the group (the step size
+    is read from the plan's device table), so each kind of table a step needs stays on the device and is rebuilt when
+    one of its inputs differs."""
+    use_fira = bool(fira) and pre_div_mode != 1
+    prev, has = fira_state_pointers(plan) if use_fira else (0, 0)
+    known = type(has) is int                # (an array: some tensor may be at its first limited step)
+    sig, ptrs = (float(d), float(fira_margin), use_fira, k), prev if use_fira else None
+    cached = plan._norm_tables.get((pre_div_mode, x))
+    if cached is None or cached[0] != sig or cached[1] is not ptrs or not known:
+        buf = plan.h_norm.next()
+        nt = plan.h_norm.table(N.NORM_TENSOR, plan.n)
+        nt["first_block"] = first
+        nt["n_blocks"] = count
+        if x is not None:
+            for i in plan.cut:
+                nt["n_blocks"][i] = -1
+                nt["first_block"][i] = plan.pieces[i].slots[x].data_ptr() + 8 * k
+        nt["pre_div_mode"] = pre_div_mode
+        nt["partials_f64"] = f64
+        nt["alpha"] = 0.0
+        nt["alpha_dev"] = (plan.d_table.data_ptr() + np.arange(plan.n, dtype=np.uint64) * np.uint64(table_dtype.itemsize)
+                           + np.uint64(table_dtype.fields["alpha"][1]))
+        sqrt_n = np.sqrt(plan.full_numel.astype(np.float64))
+        nt["sqrt_n"] = sqrt_n.astype(np.float32)
+        nt["d"] = np.float32(d)
+        nt["clip_div"] = (sqrt_n * d).astype(np.float32) if (d > 0 and pre_div_mode == 0) else np.float32(0.0)
+        nt["fira_margin1"] = np.float32(1.0 + fira_margin)
+        nt["fira_prev"], nt["fira_has_prev"] = prev, has
+        dev = cached[2] if cached is not None else torch.empty(plan.n * N.NORM_TENSOR.itemsize, dtype=torch.uint8, device=plan.device)
+        dev.copy_(buf[: dev.numel()], non_blocking=True)
+        plan.h_norm.mark(stream)
+        # (cut entries' slots may be replaced between steps: their tables are not kept)
+        plan._norm_tables[pre_div_mode, x] = cached = (sig if known and not plan.cut else None, ptrs, dev)
+    N.check(N.lib().af8_norm_finalize(cached[2].data_ptr(), plan.n, plan.d_sumsq.data_ptr(),
+                                      plan.d_dyn.data_ptr(), stream.cuda_stream), "af8_norm_finalize")
 
 
 def fira_state_pointers(plan):
@@ -648,7 +664,7 @@ class FactoredPlan:
         self.d_tables = torch.empty(self.n_tables * tb, dtype=torch.uint8, device=self.device)
         self.d_table = self.d_tables[:tb]
         self.d_dyn = torch.zeros(n * N.DYN_SCALARS.itemsize, dtype=torch.uint8, device=self.device)
-        self.d_norm = torch.empty(n * N.NORM_TENSOR.itemsize, dtype=torch.uint8, device=self.device)
+        self._norm_tables = {}       # (pre_div_mode, exchange) -> (inputs, limiter pointers, device table) of norm_finalize
         self.d_sumsq = torch.empty(self.total_chunks, dtype=torch.float64, device=self.device)
         self.h_table = _PinnedRing(self.n_tables * tb)
         self.h_norm = _PinnedRing(n * N.NORM_TENSOR.itemsize)
@@ -801,37 +817,8 @@ class FactoredPlan:
                 a = int(self.first_chunk[i])
                 _add_to_slot(self.pieces[i].slots[x], 1, self.d_sumsq[a:a + int(self.nchunks[i])])
 
-    def _finalize(self, table, pre_div_mode, d, fira, fira_margin, stream, x=None):
-        buf = self.h_norm.next()
-        nt = buf.numpy()[: self.n * N.NORM_TENSOR.itemsize].view(N.NORM_TENSOR)
-        nt["first_block"] = self.first_chunk
-        nt["n_blocks"] = self.nchunks
-        if x is not None:
-            for i in self.cut:
-                nt["n_blocks"][i] = -1
-                nt["first_block"][i] = self.pieces[i].slots[x].data_ptr() + 8
-        nt["pre_div_mode"] = pre_div_mode
-        nt["partials_f64"] = 1
-        nt["alpha"] = table["alpha"]
-        if self._alpha_on_device:
-            nt["alpha_dev"] = (self.d_table.data_ptr() + np.arange(self.n, dtype=np.uint64) * np.uint64(N.FACTORED_TENSOR.itemsize)
-                               + np.uint64(N.FACTORED_TENSOR.fields["alpha"][1]))
-        else:
-            nt["alpha_dev"] = 0
-        sqrt_n = np.sqrt(self.full_numel.astype(np.float64))
-        nt["sqrt_n"] = sqrt_n.astype(np.float32)
-        nt["d"] = np.float32(d)
-        nt["clip_div"] = (sqrt_n * d).astype(np.float32) if (d > 0 and pre_div_mode == 0) else np.float32(0.0)
-        nt["fira_margin1"] = np.float32(1.0 + fira_margin)
-        if fira and pre_div_mode != 1:
-            nt["fira_prev"], nt["fira_has_prev"] = fira_state_pointers(self)
-        else:
-            nt["fira_prev"] = 0
-            nt["fira_has_prev"] = 0
-        self.d_norm.copy_(buf[: self.d_norm.numel()], non_blocking=True)
-        self.h_norm.mark(stream)
-        N.check(N.lib().af8_norm_finalize(self.d_norm.data_ptr(), self.n, self.d_sumsq.data_ptr(),
-                                          self.d_dyn.data_ptr(), stream.cuda_stream), "af8_norm_finalize")
+    def _finalize(self, pre_div_mode, d, fira, fira_margin, stream, x=None):
+        norm_finalize(self, self.first_chunk, self.nchunks, 1, N.FACTORED_TENSOR, pre_div_mode, d, fira, fira_margin, stream, x, 1)
 
     def run(self, grads, scalars, d=0.0, fira=False, fira_margin=0.01, scale=None, stream=None, lag=False):
         """One optimizer step for every tensor of the plan, start to end."""
@@ -847,7 +834,7 @@ class FactoredPlan:
             self._static = self._static_fields()
             self._ptr_sig = sig
         buf = self.h_table.next()
-        tables = buf.numpy()[: self.n_tables * self.n * N.FACTORED_TENSOR.itemsize].view(N.FACTORED_TENSOR).reshape(self.n_tables, self.n)
+        tables = self.h_table.table(N.FACTORED_TENSOR, self.n_tables * self.n).reshape(self.n_tables, self.n)
         tables[:] = self._static
         table = tables[0]
         table["grad"] = [g.data_ptr() for g in grads]
@@ -879,14 +866,14 @@ class FactoredPlan:
             # clip of U (optimizer.py:826-828); d == 0 means no clip: an infinite threshold gives divisor 1
             self._update(N.FUPD_SUMSQ_U, False, stream, 1)
             yield
-            self._finalize(table, 1, d if d > 0 else float("inf"), False, fira_margin, stream, 1)
+            self._finalize(1, d if d > 0 else float("inf"), False, fira_margin, stream, 1)
             self._stats(N.FSTAT_RESIDUAL, buf, stream, 2)
             yield
             self._small(True, stream)
             if fira:                                    # the final update is applied with d = 0 (optimizer.py:953)
                 self._update(N.FUPD_SUMSQ, True, stream, 3)
                 yield
-                self._finalize(table, 2, 0.0, True, fira_margin, stream, 3)
+                self._finalize(2, 0.0, True, fira_margin, stream, 3)
             self._update(N.FUPD_APPLY, True, stream)
         elif need_stat and lag:
             # lag_norm=True: one pass with the previous step's norm (optimizer.py:1056-1071)
@@ -907,7 +894,7 @@ class FactoredPlan:
         elif need_stat:
             self._update(N.FUPD_SUMSQ, False, stream, 1)
             yield
-            self._finalize(table, 0, d, fira, fira_margin, stream, 1)
+            self._finalize(0, d, fira, fira_margin, stream, 1)
             self._update(N.FUPD_APPLY, True, stream)
         else:
             self._update(N.FUPD_APPLY, False, stream)

@@ -665,7 +665,11 @@ class Adafactor8Bit(Optimizer):
                 if self._shard is not None:
                     pending.append((gi, e, dev, gen))
                     continue
-                with torch.cuda.device(dev):             # the whole pass sequence of the plan, now
+                if dev.index == torch.cuda.current_device():
+                    for _ in gen:                        # the whole pass sequence of the plan, now
+                        pass
+                    continue
+                with torch.cuda.device(dev):
                     for _ in gen:
                         pass
             for p, work in copy_back:
@@ -1036,30 +1040,33 @@ class Adafactor8Bit(Optimizer):
             self._plans[pkey] = plan
         n = len(items)
         scale = self._scale_inputs(group, n) if group["scale_parameter"] else None
-        cols = {k: np.empty(n, dtype=f32) for k in ("decay", "alpha", "v_w", "m_w", "c_w", "eps1", "eps_came")}
-        if sr:
-            cols["sr_base"] = np.zeros(n, dtype=np.uint64)
         steps = []
         for _, _, st in items:
             step = st["step"] + 1
             st["step"] = step
             steps.append(step)
+        uniform = steps.count(steps[0]) == n          # the usual case: every tensor of the group is at the same step
+        # (one value per field then, else one per tensor)
+        cols = {} if uniform else {k: np.empty(n, dtype=f32) for k in ("decay", "alpha", "v_w", "m_w", "c_w", "eps1", "eps_came")}
         grads = [g if g.is_contiguous() else g.contiguous() for _, g, _ in items]
         if sr:                      # a part of a tensor draws the counters of its elements in the whole tensor
+            cols["sr_base"] = np.zeros(n, dtype=np.uint64)
             for i, (_, _, st) in enumerate(items):
                 first = pcs[i].elem0 if pcs[i] is not None else 0
                 cols["sr_base"][i] = (sr_base(self._sr_seed(st), steps[i]) + first) & 0xFFFFFFFFFFFFFFFF
-        uniform = steps.count(steps[0]) == n          # the usual case: every tensor of the group is at the same step
         for i in ([0] if uniform else range(n)):
             where = slice(None) if uniform else i
             sc = self._step_scalars(group, steps[i])
             alpha, decay = self._alpha_decay(group, sc)
-            cols["decay"][where], cols["alpha"][where] = decay, alpha
-            cols["v_w"][where] = f32(sc["beta_val"])
-            cols["m_w"][where] = f32(1.0 - group["beta1"]) if group.get("beta1") is not None else f32(0.0)
-            cols["c_w"][where] = f32(1.0 - group["beta3"]) if group.get("beta3") is not None else f32(0.0)
-            cols["eps1"][where] = f32(sc["eps1"])
-            cols["eps_came"][where] = f32(group.get("eps_came", 1e-16))
+            vals = dict(decay=decay, alpha=alpha, v_w=f32(sc["beta_val"]),
+                        m_w=f32(1.0 - group["beta1"]) if group.get("beta1") is not None else f32(0.0),
+                        c_w=f32(1.0 - group["beta3"]) if group.get("beta3") is not None else f32(0.0),
+                        eps1=f32(sc["eps1"]), eps_came=f32(group.get("eps_came", 1e-16)))
+            if uniform:
+                cols.update(vals)
+            else:
+                for k, v in vals.items():
+                    cols[k][i] = v
             if scale is not None:
                 self._fill_scale(scale, where, group, sc)
         d, fira, lag = float(group["d"]), bool(group.get("enable_fira_for_adafactor", False)), bool(group.get("lag_norm", False))
@@ -1069,10 +1076,10 @@ class Adafactor8Bit(Optimizer):
     def _run_fullrank(self, gi, group, key, items):
         device, gdtype, v_fmt, m_fmt, block, m_block, pdtype = key
         sr = bool(group.get("stochastic_round_writeback", False)) and pdtype in (torch.bfloat16, torch.float16)
-        sc0 = self._step_scalars(group, 1)
+        adam = (not group.get("factored", True)) and group["beta2"] is not None and group.get("beta3") is None   # (as _step_scalars)
         momentum_only = group.get("momentum_only_1d")
         if momentum_only is None:
-            momentum_only = not sc0["adam"]
+            momentum_only = not adam
         sgd = v_fmt == "none"
         if sgd:
             momentum_only = False
@@ -1081,7 +1088,7 @@ class Adafactor8Bit(Optimizer):
         plan = self._plans.get(pkey)
         pcs = [self._pieces.get(id(p)) for p, _, _ in items]
         if plan is None or plan.ids != ids:
-            plan = FullrankPlan(device, gdtype, v_fmt, m_fmt, block, m_block, sc0["adam"], momentum_only,
+            plan = FullrankPlan(device, gdtype, v_fmt, m_fmt, block, m_block, adam, momentum_only,
                                 group["maximize"], [p for p, _, _ in items], [s for _, _, s in items],
                                 stochastic_round=sr, pieces=pcs)
             plan.ids = ids
@@ -1092,9 +1099,7 @@ class Adafactor8Bit(Optimizer):
             scale = {k: np.zeros(n, dtype=f32) for k in ("rho", "eps2", "bc", "weight_decay")}
             scale["bc_mode"] = np.zeros(n, dtype=np.int32)
             scale["scale_weight_decay"] = np.full(n, int(bool(group.get("scale_weight_decay", True))), dtype=np.int32)
-        cols = {k: np.empty(n, dtype=f32) for k in _FULLRANK_COLS}
-        if sr:
-            cols["sr_base"] = np.zeros(n, dtype=np.uint64)
+
         def row_values(step):
             sc = self._step_scalars(group, step)
             alpha, decay = self._alpha_decay(group, sc)
@@ -1109,13 +1114,16 @@ class Adafactor8Bit(Optimizer):
             step = st["step"] + 1
             st["step"] = step
             steps.append(step)
+        uniform = steps.count(steps[0]) == n          # the usual case: every tensor of the group is at the same step
+        # (one value per field then, else one per tensor)
+        cols = {} if uniform else {k: np.empty(n, dtype=f32) for k in _FULLRANK_COLS}
         grads = [g if g.is_contiguous() else g.contiguous() for _, g, _ in items]
         if sr:                      # a part of a tensor draws the counters of its elements in the whole tensor
+            cols["sr_base"] = np.zeros(n, dtype=np.uint64)
             for i, (_, _, st) in enumerate(items):
                 first = pcs[i].elem0 if pcs[i] is not None else 0
                 cols["sr_base"][i] = (sr_base(self._sr_seed(st), steps[i]) + first) & 0xFFFFFFFFFFFFFFFF
         cache = {}
-        uniform = steps.count(steps[0]) == n          # the usual case: every tensor of the group is at the same step
         for i in ([0] if uniform else range(n)):
             step = steps[i]
             got = cache.get(step)
@@ -1123,8 +1131,11 @@ class Adafactor8Bit(Optimizer):
                 got = cache[step] = row_values(step)
             sc, vals = got
             where = slice(None) if uniform else i
-            for k, v in zip(_FULLRANK_COLS, vals):
-                cols[k][where] = v
+            if uniform:
+                cols.update(zip(_FULLRANK_COLS, vals))
+            else:
+                for k, v in zip(_FULLRANK_COLS, vals):
+                    cols[k][i] = v
             if scale is not None:
                 scale["rho"][where] = sc["rho"]
                 scale["eps2"][where] = f32(sc["eps2"])
