@@ -711,24 +711,15 @@ inline int apollo_project_exact(const af8_apollo_proj_desc &d, int32_t grad_dtyp
 
 // tensor-core path, per tensor: bf16 planes of Pt (and, for the mma.sync kernel, the non-finite flag and the
 // channel norms; the tcgen05 kernel produces both itself); fills the task
-// true: this projection runs on tcgen05 (right case, rank a multiple of 16 up to 256)
-// bytes of the transposed gradient that a left-case tensor needs on the tcgen05 path
-inline int64_t apollo_transpose_need(const af8_apollo_proj_desc &d)
-{
-    return d.rows >= d.cols ? 0 : (d.rows * d.cols * 2 + 255) / 256 * 256;
-}
-
-// true: this projection runs on tcgen05 (rank a multiple of 16 up to 256; the left case also
-// needs room for the transposed gradient, because the kernel takes both operands K-major)
-inline bool apollo_umma_eligible(const af8_apollo_proj_desc &d, int64_t transpose_bytes)
+// true: this projection runs on tcgen05 (rank a multiple of 16 up to 256)
+inline bool apollo_umma_eligible(const af8_apollo_proj_desc &d)
 {
     static const bool disabled = getenv("AF8_NO_UMMA") != nullptr;
-    return !disabled && d.rank % 16 == 0 && d.rank >= 16 && d.rank <= UM_MAXN && apollo_transpose_need(d) <= transpose_bytes;
+    return !disabled && d.rank % 16 == 0 && d.rank >= 16 && d.rank <= UM_MAXN;
 }
 
-// gt: where the transposed gradient of a left-case tcgen05 task goes (nullptr otherwise)
 inline int apollo_project_prepare(const af8_apollo_proj_desc &d, int32_t grad_dtype, ProjTask &task, int &next_tile, bool umma,
-                                  cudaStream_t st, void *gt = nullptr)
+                                  cudaStream_t st)
 {
     int *flag = static_cast<int *>(d.workspace);
     __nv_bfloat16 *planes = reinterpret_cast<__nv_bfloat16 *>(static_cast<char *>(d.workspace) + APOLLO_WS_HEADER);
@@ -752,13 +743,6 @@ inline int apollo_project_prepare(const af8_apollo_proj_desc &d, int32_t grad_dt
     }
     AF8_CUDA_TRY(cudaGetLastError());
     task.grad = static_cast<const __nv_bfloat16 *>(d.grad);
-    if (umma && !right) {                                    // the kernel reads G^T [cols][rows]
-        dim3 grid((unsigned)((d.cols + 63) / 64), (unsigned)((d.rows + 63) / 64));
-        apollo_transpose_bf16_kernel<<<grid, 256, 0, st>>>(static_cast<const uint16_t *>(d.grad), (int)d.rows, (int)d.cols,
-                                                            static_cast<uint16_t *>(gt));
-        AF8_CUDA_TRY(cudaGetLastError());
-        task.grad = static_cast<const __nv_bfloat16 *>(gt);
-    }
     task.planes = planes;
     task.out = d.g_low;
     task.nonfinite_flag = flag;
@@ -776,18 +760,20 @@ inline int apollo_project_prepare(const af8_apollo_proj_desc &d, int32_t grad_dt
     return AF8_OK;
 }
 
-// the two tensor maps of a tcgen05 task: G as [M][K] with boxes of 128 x 32, the planes as
-// [3][N][K] with boxes of 3 x N x 32, both with the 64-byte swizzle and zero fill outside
+// the two tensor maps of a tcgen05 task: G as [M][K] with boxes of 128 x 32 and the 64-byte swizzle (left: as [K][M] with
+// boxes of 32 x 64 and the 128-byte swizzle), the planes as [3][N][K] with boxes of 3 x N x 32 and the 64-byte swizzle;
+// zero fill outside
 inline int apollo_umma_maps(UmmaTask &u)
 {
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return fail(AF8_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
     const ProjTask &t = u.t;
     {
-        const cuuint64_t dim[2] = {(cuuint64_t)t.K, (cuuint64_t)t.M}, stride[1] = {(cuuint64_t)t.K * 2};
-        const cuuint32_t box[2] = {UM_BK, UM_BM}, es[2] = {1, 1};
+        const int inner = t.right ? t.K : t.M, outer = t.right ? t.M : t.K;
+        const cuuint64_t dim[2] = {(cuuint64_t)inner, (cuuint64_t)outer}, stride[1] = {(cuuint64_t)inner * 2};
+        const cuuint32_t box[2] = {t.right ? (cuuint32_t)UM_BK : (cuuint32_t)UM_LEFT_BOX_M, t.right ? (cuuint32_t)UM_BM : (cuuint32_t)UM_BK}, es[2] = {1, 1};
         const CUresult r = enc(&u.map_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16 *>(t.grad), dim, stride, box, es,
-                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                               CU_TENSOR_MAP_INTERLEAVE_NONE, t.right ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) return fail(AF8_ERR_CUDA, "cuTensorMapEncodeTiled (gradient) failed with %d", (int)r);
     }
@@ -856,7 +842,7 @@ extern "C" int af8_apollo_project_ws(const void *grad, int32_t grad_dtype, int32
     if (!apollo_tc_eligible(d, grad_dtype)) return apollo_project_exact(d, grad_dtype, st);
     ProjTask task;
     int tiles = 0;
-    const bool umma = apollo_umma_eligible(d, 0);            // no room for a transposed gradient here: right case only
+    const bool umma = apollo_umma_eligible(d);
     rc = apollo_project_prepare(d, grad_dtype, task, tiles, umma, st);
     if (rc) return rc;
     // the task lives in the workspace between the flag and the planes; the copy from this
@@ -891,47 +877,25 @@ extern "C" int af8_apollo_project_batch(const af8_apollo_proj_desc *descs, int32
     if ((reinterpret_cast<uintptr_t>(host_scratch) & 63u) || (reinterpret_cast<uintptr_t>(dev_scratch) & 63u))
         return fail(AF8_ERR_INVALID, "af8_apollo_project_batch: scratch buffers must be 64-byte aligned");
     if (transpose_bytes > 0 && (!transpose_scratch || (reinterpret_cast<uintptr_t>(transpose_scratch) & 255u)))
-        return fail(AF8_ERR_INVALID, "af8_apollo_project_batch: transpose_scratch must be 256-byte aligned");
+        return fail(AF8_ERR_INVALID, "af8_apollo_project_batch: transpose_scratch must be 256-byte aligned");      // (no longer used)
     int n_umma = 0, n_mma = 0;
     for (int i = 0; i < n; ++i) {
         int rc = apollo_check_desc(descs[i], grad_dtype);
         if (rc) return rc;
-        if (apollo_tc_eligible(descs[i], grad_dtype)) { if (apollo_umma_eligible(descs[i], transpose_bytes)) ++n_umma; else ++n_mma; }
+        if (apollo_tc_eligible(descs[i], grad_dtype)) { if (apollo_umma_eligible(descs[i])) ++n_umma; else ++n_mma; }
     }
     UmmaTask *host_u = static_cast<UmmaTask *>(host_scratch);
     const UmmaTask *dev_u = static_cast<const UmmaTask *>(dev_scratch);
     ProjTask *host_m = reinterpret_cast<ProjTask *>(host_u + n_umma);
     int iu = 0, im = 0, tiles_u = 0, tiles_m = 0;
-    // The tcgen05 tasks go out in sub-batches: a new one starts when the transposed gradients
-    // of the left-case tensors would no longer fit the scratch (stream order makes its reuse safe).
-    int sub_start = 0;
-    int64_t t_off = 0;
-    auto launch_sub = [&](int end) -> int {
-        if (end > sub_start) {
-            AF8_CUDA_TRY(cudaMemcpyAsync(static_cast<char *>(dev_scratch) + sizeof(UmmaTask) * (size_t)sub_start, host_u + sub_start,
-                                         sizeof(UmmaTask) * (size_t)(end - sub_start), cudaMemcpyHostToDevice, st));
-            int rc = apollo_project_launch_umma(dev_u + sub_start, end - sub_start, tiles_u, st);
-            if (rc) return rc;
-        }
-        sub_start = end;
-        tiles_u = 0;
-        t_off = 0;
-        return AF8_OK;
-    };
     for (int i = 0; i < n; ++i) {
         int rc;
         if (!apollo_tc_eligible(descs[i], grad_dtype)) {
             rc = apollo_project_exact(descs[i], grad_dtype, st);
-        } else if (apollo_umma_eligible(descs[i], transpose_bytes)) {
-            const int64_t need = apollo_transpose_need(descs[i]);
-            if (need > 0 && t_off + need > transpose_bytes) {
-                rc = launch_sub(iu);
-                if (rc) return rc;
-            }
+        } else if (apollo_umma_eligible(descs[i])) {
             UmmaTask &u = host_u[iu++];
             memset(&u, 0, sizeof(u));
-            rc = apollo_project_prepare(descs[i], grad_dtype, u.t, tiles_u, true, st, need > 0 ? static_cast<char *>(transpose_scratch) + t_off : nullptr);
-            t_off += need;
+            rc = apollo_project_prepare(descs[i], grad_dtype, u.t, tiles_u, true, st);
             u.chan_g2 = descs[i].chan_g2;
             if (!rc) rc = apollo_umma_maps(u);
         } else {
@@ -939,8 +903,11 @@ extern "C" int af8_apollo_project_batch(const af8_apollo_proj_desc *descs, int32
         }
         if (rc) return rc;
     }
-    int rc = launch_sub(iu);
-    if (rc) return rc;
+    if (iu) {
+        AF8_CUDA_TRY(cudaMemcpyAsync(dev_scratch, host_u, sizeof(UmmaTask) * (size_t)iu, cudaMemcpyHostToDevice, st));
+        int rc = apollo_project_launch_umma(dev_u, iu, tiles_u, st);
+        if (rc) return rc;
+    }
     if (n_mma) {
         ProjTask *dev_m = reinterpret_cast<ProjTask *>(static_cast<char *>(dev_scratch) + sizeof(UmmaTask) * (size_t)n_umma);
         AF8_CUDA_TRY(cudaMemcpyAsync(dev_m, host_m, sizeof(ProjTask) * (size_t)n_mma, cudaMemcpyHostToDevice, st));

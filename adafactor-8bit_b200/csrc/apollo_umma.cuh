@@ -1,5 +1,7 @@
-// APOLLO projection, "right" case (rows >= cols), on the fifth-generation tensor cores:
+// APOLLO projection on the fifth-generation tensor cores.  "Right" case (rows >= cols):
 //   g_low[M x N] = G[M x K] @ Pt[K x N],   M = rows, K = cols, N = rank
+// "Left" case (rows < cols), as the transposed problem:
+//   g_low^T[M x N] = G^T[M x K] @ P^T[K x N],   M = cols, K = rows
 // with the same three-plane bf16 split of Pt as apollo_mma.cuh.  tcgen05.mma reads both
 // operands from shared memory and accumulates in tensor memory (TMEM).
 //
@@ -9,10 +11,13 @@
 // 8-row groups, and advance by 32 bytes per 16 values of K.  The gradient already has K
 // contiguous; the planes of Pt are written transposed ([3][N][K]) by the split kernel and
 // arrive with one three-dimensional copy per stage.
+// In the left case the gradient has M contiguous: a stage of it is two boxes of 32 rows (K) x 64 columns (128 bytes,
+// 128-byte swizzle), an M-major operand.  (A separate transposition of such gradients, 52 us per Llama-3-8B layer, and
+// their second trip through memory are gone with it.)
 //
 // CTA = 320 threads, one CTA per SM, persistent over (task, M tile) pairs:
 //   warps 0-7  read every gradient tile from shared memory before its MMAs: they add up the
-//              squares of each row (the channel norms ||G_row||^2 that the scaling step needs,
+//              squares of each row of M (the channel norms ||G_row||^2 that the scaling step needs,
 //              so the gradient is read from memory once) and zero non-finite entries; then
 //              drain the accumulator: warp w owns TMEM lanes 32 (w % 4) .. +31 and columns
 //              128 (w / 4) .. +127, 128 totals per thread; then store g_low and the norms.
@@ -48,7 +53,7 @@ constexpr int UM_BM = 128, UM_BK = 32, UM_STAGES = 4, UM_THREADS = 320, UM_WORKE
 constexpr int UM_FLUSH = 8;        // stages (256 values of K) per accumulator chunk
 constexpr int UM_MAXN = 256;
 constexpr int UM_ROW_BYTES = UM_BK * 2;                       // 64
-constexpr int UM_A_BYTES = UM_BM * UM_ROW_BYTES;              // 8 KB
+constexpr int UM_A_BYTES = UM_BM * UM_ROW_BYTES;              // 8 KB (a multiple of 1024, like a stage: the 128-byte swizzle's period)
 constexpr int UM_B_BYTES = UM_MAXN * UM_ROW_BYTES;            // 16 KB per plane at N = 256
 constexpr int UM_STAGE_BYTES = UM_A_BYTES + 3 * UM_B_BYTES;   // 56 KB
 constexpr int UM_SBO = 8 * UM_ROW_BYTES;                      // 512 bytes between 8-row groups
@@ -56,7 +61,7 @@ constexpr int DEVERR_UMMA_TIMEOUT = 2;
 
 // One projection of a tcgen05 launch: the mma.sync task plus the two tensor maps
 struct __align__(64) UmmaTask {
-    CUtensorMap map_a;       // G as [M][K], box 128 x 32
+    CUtensorMap map_a;       // right: G as [M][K], box 128 x 32; left: G as [K][M], box 32 x 64
     CUtensorMap map_b;       // planes as [3][N][K], box 3 x N x 32
     ProjTask t;
     double *chan_g2;         // [M] sums of squares of the rows of G (non-finite entries count as zero)
@@ -71,10 +76,18 @@ __device__ __forceinline__ uint64_t umma_smem_desc(uint32_t smem_addr)
     return (uint64_t)((smem_addr >> 4) & 0x3fffu) | ((uint64_t)1 << 16) | ((uint64_t)(UM_SBO >> 4) << 32) |
            (1ull << 46) | (4ull << 61);
 }
-// kind::f16 instruction descriptor: D = F32, A = B = BF16, both K-major, M = 128, N = n
-__device__ __forceinline__ uint32_t umma_instr_desc(int n)
+// M-major A with the 128-byte swizzle: blocks of 64 values of M x 8 of K (1024 bytes); 4096 bytes to the next 64 values
+// of M (a box), 1024 bytes to the next 8 of K; layout type 2 = 128-byte swizzle
+constexpr int UM_LEFT_BOX_M = 64, UM_LEFT_BOX_BYTES = UM_BK * UM_LEFT_BOX_M * 2;
+__device__ __forceinline__ uint64_t umma_smem_desc_left(uint32_t smem_addr)
 {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(UM_BM >> 4) << 24);
+    return (uint64_t)((smem_addr >> 4) & 0x3fffu) | ((uint64_t)(UM_LEFT_BOX_BYTES >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
+           (1ull << 46) | (2ull << 61);
+}
+// kind::f16 instruction descriptor: D = F32, A = B = BF16, B K-major, A K-major or (bit 15) M-major, M = 128, N = n
+__device__ __forceinline__ uint32_t umma_instr_desc(int n, bool a_m_major)
+{
+    return (1u << 4) | (1u << 7) | (1u << 10) | (a_m_major ? 1u << 15 : 0u) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(UM_BM >> 4) << 24);
 }
 __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
 {
@@ -92,48 +105,6 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar)
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// G[R][C] (bf16) -> G^T[C][R], non-finite entries replaced by zero (optimizer.py:2606).
-// 64 x 64 tiles.  A thread transposes 2 x 2 blocks in registers (two 32-bit loads from neighbouring
-// rows become the two 32-bit words of neighbouring output rows), so shared memory only moves whole
-// words through two 32 x 33 arrays, without bank conflicts; every global access of a warp is a
-// contiguous run of 128 bytes.  R and C even.
-__global__ void __launch_bounds__(256)
-apollo_transpose_bf16_kernel(const uint16_t *__restrict__ in, int R, int C, uint16_t *__restrict__ out)
-{
-    __shared__ uint32_t t0[32][33], t1[32][33];       // [block column][block row]: output rows 2 bc and 2 bc + 1
-    const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    uint32_t a[4], b[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {                      // block (row ty + 8 k, column tx): rows r, r + 1, columns c, c + 1
-        const int r = r0 + 2 * (ty + 8 * k), c = c0 + 2 * tx;
-        a[k] = b[k] = 0u;
-        if (r < R && c < C) {
-            a[k] = __ldg(reinterpret_cast<const uint32_t *>(in + (int64_t)r * C + c));
-            b[k] = __ldg(reinterpret_cast<const uint32_t *>(in + (int64_t)(r + 1) * C + c));
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        uint32_t x = a[k], y = b[k];
-        if ((x & 0x7f80u) == 0x7f80u) x &= 0xffff0000u;
-        if ((x & 0x7f800000u) == 0x7f800000u) x &= 0x0000ffffu;
-        if ((y & 0x7f80u) == 0x7f80u) y &= 0xffff0000u;
-        if ((y & 0x7f800000u) == 0x7f800000u) y &= 0x0000ffffu;
-        t0[tx][ty + 8 * k] = __byte_perm(x, y, 0x5410);          // column c:     (row r, row r + 1)
-        t1[tx][ty + 8 * k] = __byte_perm(x, y, 0x7632);          // column c + 1
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {                      // output rows c, c + 1 of block column ty + 8 k; columns r, r + 1 of block row tx
-        const int c = c0 + 2 * (ty + 8 * k), r = r0 + 2 * tx;
-        if (c < C && r < R) {
-            *reinterpret_cast<uint32_t *>(out + (int64_t)c * R + r) = t0[ty + 8 * k][tx];
-            *reinterpret_cast<uint32_t *>(out + (int64_t)(c + 1) * R + r) = t1[ty + 8 * k][tx];
-        }
-    }
-}
-
 // Pt[K][N] (fp32) -> three bf16 planes stored [N][K]
 __global__ void __launch_bounds__(256)
 apollo_split_transposed_kernel(const float *__restrict__ p, int K, int N, __nv_bfloat16 *__restrict__ planes)
@@ -198,6 +169,38 @@ __device__ __forceinline__ double umma_chunk_sumsq(unsigned char *p, bool &wrote
     return d;
 }
 
+// Left case: the 4 values of half a 16-byte chunk belong to 4 rows of M.  Their squares are added to acc[4] in binary32 (the
+// caller passes the sums on to binary64 after at most 8 values); where a magnitude from 2^60 up makes squares that might
+// leave binary32, they go into wide[4] in binary64, and non-finite entries are zeroed in shared memory as above.
+__device__ __forceinline__ void umma_quad_squares(unsigned char *p, float (&acc)[4], double (&wide)[4], bool &wrote)
+{
+    const uint2 v = *reinterpret_cast<const uint2 *>(p);
+    uint32_t w[2] = {v.x, v.y};
+    const uint32_t top = __vmaxu2(w[0] & 0x7fff7fffu, w[1] & 0x7fff7fffu);
+    if ((top >> 16) < 0x5d80u && (top & 0xffffu) < 0x5d80u) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float lo = __uint_as_float(w[i] << 16), hi = __uint_as_float(w[i] & 0xffff0000u);
+            acc[2 * i] = __fmaf_rn(lo, lo, acc[2 * i]);
+            acc[2 * i + 1] = __fmaf_rn(hi, hi, acc[2 * i + 1]);
+        }
+        return;
+    }
+    bool changed = false;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        if ((w[i] & 0x7f80u) == 0x7f80u) { w[i] &= 0xffff0000u; changed = true; }
+        if ((w[i] & 0x7f800000u) == 0x7f800000u) { w[i] &= 0x0000ffffu; changed = true; }
+        const double lo = (double)__uint_as_float(w[i] << 16), hi = (double)__uint_as_float(w[i] & 0xffff0000u);
+        wide[2 * i] += lo * lo;
+        wide[2 * i + 1] += hi * hi;
+    }
+    if (changed) {
+        *reinterpret_cast<uint2 *>(p) = make_uint2(w[0], w[1]);
+        wrote = true;
+    }
+}
+
 __global__ void __launch_bounds__(UM_THREADS, 1)
 apollo_project_umma_kernel(const UmmaTask *__restrict__ tasks, int n_tasks, int total_tiles)
 {
@@ -245,6 +248,7 @@ apollo_project_umma_kernel(const UmmaTask *__restrict__ tasks, int n_tasks, int 
         const int ksteps = (K + UM_BK - 1) / UM_BK;
         const int nchunks = (ksteps + UM_FLUSH - 1) / UM_FLUSH;
         const int plane_bytes = N * UM_ROW_BYTES;
+        const bool right = __ldg(&T->right) != 0;
         bool failed = false;
 
         if (warp < UM_MMA_WARP) {
@@ -278,10 +282,19 @@ apollo_project_umma_kernel(const UmmaTask *__restrict__ tasks, int n_tasks, int 
                 mbar_arrive(&s_acc_empty[buf]);
                 return true;
             };
-            // The 8 KB gradient tile of a stage is 512 chunks of 16 bytes, two per thread; chunk i lies in
-            // row i / 4 of the tile (the swizzle permutes chunks within a row).  rs0 / rs1: this thread's
-            // share of the squared norms of rows tid / 4 and 64 + tid / 4, over all of K.
-            double rs0 = 0.0, rs1 = 0.0;
+            // The 8 KB gradient tile of a stage is 512 chunks of 16 bytes, two per thread.  rs: this thread's share
+            // of squared norms of rows of M, over all of K.  Right: chunk i lies in row i / 4 of the tile (the swizzle
+            // permutes chunks within a row), rs[0] and rs[1] are of rows tid / 4 and 64 + tid / 4.  Left: warp w has the
+            // 16 rows of M from 16 w on, a lane 4 of them (lane & 3) at 4 values of K: 2 (lane / 4 % 4) and the next one
+            // of two of the four groups of 8.  The 128-byte swizzle puts chunk c of a box row k at c ^ (k & 7): the 16
+            // lanes of an access hit 16 different pairs of banks.
+            double rs[4];
+            float rq[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { rs[i] = 0.0; rq[i] = 0.0f; }
+            const int lk = 2 * ((lane >> 2) & 3), lc = 2 * (warp & 3) + ((lane >> 1) & 1);
+            const int lbase = (warp >> 2) * UM_LEFT_BOX_BYTES + (lane >> 4) * 2048 + (lane & 1) * 8;
+            const int left0 = lbase + lk * 128 + ((lc ^ lk) << 4), left1 = lbase + (lk + 1) * 128 + ((lc ^ (lk + 1)) << 4);
             auto scan = [&](int c) -> bool {
                 const int k_end = min(ksteps, (c + 1) * UM_FLUSH);
                 for (int ks = c * UM_FLUSH; ks < k_end; ++ks) {
@@ -289,8 +302,19 @@ apollo_project_umma_kernel(const UmmaTask *__restrict__ tasks, int n_tasks, int 
                     if (!mbar_wait_bounded(&s_full[slot], (uint32_t)(f / UM_STAGES) & 1u)) return false;
                     unsigned char *st = um_smem + slot * UM_STAGE_BYTES;
                     bool wrote = false;
-                    rs0 += umma_chunk_sumsq(st + tid * 16, wrote);
-                    rs1 += umma_chunk_sumsq(st + (tid + UM_WORKERS) * 16, wrote);
+                    if (right) {
+                        rs[0] += umma_chunk_sumsq(st + tid * 16, wrote);
+                        rs[1] += umma_chunk_sumsq(st + (tid + UM_WORKERS) * 16, wrote);
+                    } else {
+                        umma_quad_squares(st + left0, rq, rs, wrote);
+                        umma_quad_squares(st + left1, rq, rs, wrote);
+                        umma_quad_squares(st + left0 + 1024, rq, rs, wrote);
+                        umma_quad_squares(st + left1 + 1024, rq, rs, wrote);
+                        if ((ks & 1) == 1 || ks + 1 == ksteps) {     // (8 values)
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) { rs[i] += (double)rq[i]; rq[i] = 0.0f; }
+                        }
+                    }
                     if (wrote) fence_proxy_async();              // repaired entries must be visible to the MMAs
                     mbar_arrive(&s_clean[slot]);
                 }
@@ -307,7 +331,7 @@ apollo_project_umma_kernel(const UmmaTask *__restrict__ tasks, int n_tasks, int 
                 const int m = m0 + row;
                 const float sgn = __ldg(&T->negate) ? -1.0f : 1.0f;
                 float *__restrict__ out = T->out;
-                if (m < M && __ldg(&T->right)) {
+                if (m < M && right) {
 #pragma unroll
                     for (int q = 0; q < 32; ++q) {
                         const int n = col_half * 128 + q * 4;
@@ -324,19 +348,29 @@ apollo_project_umma_kernel(const UmmaTask *__restrict__ tasks, int n_tasks, int 
                         if (n < N) out[(int64_t)n * M + m] = sgn * total[e];
                     }
                 }
-                // the four threads that share a row add their parts; one of them stores the norm
-                rs0 += __shfl_xor_sync(0xffffffffu, rs0, 1); rs0 += __shfl_xor_sync(0xffffffffu, rs0, 2);
-                rs1 += __shfl_xor_sync(0xffffffffu, rs1, 1); rs1 += __shfl_xor_sync(0xffffffffu, rs1, 2);
+                // the threads that share a row (four; left: eight) add their parts; one of them stores the norm
                 double *__restrict__ chan = U->chan_g2;
-                if ((tid & 3) == 0 && chan != nullptr) {
-                    const int ra = m0 + (tid >> 2), rb = ra + 64;
-                    if (ra < M) chan[ra] = rs0;
-                    if (rb < M) chan[rb] = rs1;
+                if (right) {
+#pragma unroll
+                    for (int o = 1; o < 4; o <<= 1) { rs[0] += __shfl_xor_sync(0xffffffffu, rs[0], o); rs[1] += __shfl_xor_sync(0xffffffffu, rs[1], o); }
+                    if ((tid & 3) == 0 && chan != nullptr) {
+                        const int ra = m0 + (tid >> 2), rb = ra + 64;
+                        if (ra < M) chan[ra] = rs[0];
+                        if (rb < M) chan[rb] = rs[1];
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+                        for (int o = 4; o < 32; o <<= 1) rs[i] += __shfl_xor_sync(0xffffffffu, rs[i], o);
+                        const int r = m0 + 16 * warp + 4 * lane + i;
+                        if (lane < 4 && r < M && chan != nullptr) chan[r] = rs[i];
+                    }
                 }
             }
         } else if (warp == UM_MMA_WARP && lane == 0) {
             // ---------------- MMA issuer ----------------
-            const uint32_t idesc = umma_instr_desc(N);
+            const uint32_t idesc = umma_instr_desc(N, !right);
             for (int ks = 0; ks < ksteps; ++ks) {
                 const int g = gchunk + ks / UM_FLUSH, buf = g & 1;
                 const bool chunk_start = (ks % UM_FLUSH) == 0;
@@ -353,7 +387,7 @@ apollo_project_umma_kernel(const UmmaTask *__restrict__ tasks, int n_tasks, int 
                 const uint32_t d = tmem + (uint32_t)(buf * UM_MAXN);
 #pragma unroll
                 for (int k16 = 0; k16 < UM_BK / 16; ++k16) {
-                    const uint64_t ad = umma_smem_desc(a0 + k16 * 32);
+                    const uint64_t ad = right ? umma_smem_desc(a0 + k16 * 32) : umma_smem_desc_left(a0 + k16 * 2048);
 #pragma unroll
                     for (int t = 2; t >= 0; --t) {              // smallest plane first
                         const uint64_t bd = umma_smem_desc(a0 + UM_A_BYTES + t * plane_bytes + k16 * 32);
@@ -376,7 +410,11 @@ apollo_project_umma_kernel(const UmmaTask *__restrict__ tasks, int n_tasks, int 
                 if (use >= 1 && !mbar_wait_bounded(&s_empty[slot], (uint32_t)(use - 1) & 1u)) { failed = true; break; }
                 unsigned char *st = um_smem + slot * UM_STAGE_BYTES;
                 mbar_expect_tx(&s_full[slot], bytes);
-                tma_load_2d(st, &U->map_a, ks * UM_BK, m0, &s_full[slot]);
+                if (right) tma_load_2d(st, &U->map_a, ks * UM_BK, m0, &s_full[slot]);
+                else {
+                    tma_load_2d(st, &U->map_a, m0, ks * UM_BK, &s_full[slot]);
+                    tma_load_2d(st + UM_LEFT_BOX_BYTES, &U->map_a, m0 + UM_LEFT_BOX_M, ks * UM_BK, &s_full[slot]);
+                }
                 tma_load_3d(st + UM_A_BYTES, &U->map_b, ks * UM_BK, 0, 0, &s_full[slot]);
                 issued = f + 1;
             }

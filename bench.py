@@ -596,8 +596,8 @@ def run_gpu_arm(args):
             roofline.update({"bound": "tensor", "unit": "TFLOP/s", "peak": peak_tf, "achieved": 3.0 * tf,
                              "frac": 3.0 * tf / peak_tf, "frac_of_8tbs": None, "achieved_as_specified": tf,
                              "flops_note": "achieved = issued bf16 MMA flops (3 planes x 2*rank per parameter); "
-                                           "achieved_as_specified = 2*rank per parameter; the launch also transposes "
-                                           "left-case gradients and sums channel norms",
+                                           "achieved_as_specified = 2*rank per parameter; the launch also sums "
+                                           "channel norms",
                              "traffic": None, "peak_source": peak_kind})
 
     # ---- end to end: gradients in pinned host memory ----

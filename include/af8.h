@@ -474,10 +474,7 @@ AF8_API int af8_apollo_project_ws(const void *grad, int32_t grad_dtype, int32_t 
  * the GPU full when a single matrix has fewer tiles than there are SMs; the others take
  * the exact path one by one.  host_scratch (pinned, valid until the copies have run) and
  * dev_scratch each hold n * af8_apollo_project_task_bytes() bytes, 64-byte aligned.
- * transpose_scratch (device, 256-byte aligned, may be NULL with transpose_bytes 0) lets
- * left-case tensors (rows < cols) use the tcgen05 kernel, which wants both operands with the
- * contracted dimension contiguous: their gradients are transposed into it, as many tensors at
- * a time as fit; a tensor whose transposed gradient does not fit stays on the mma.sync kernel. */
+ * transpose_scratch and transpose_bytes are no longer used (NULL and 0, or a 256-byte aligned buffer as before). */
 typedef struct af8_apollo_proj_desc {
     const void *grad;       /* rows x cols */
     const float *pt;        /* cols x rank (rows >= cols) or rank x rows */
