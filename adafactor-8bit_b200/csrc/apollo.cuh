@@ -18,6 +18,8 @@
 // step 1 are in apollo_umma.cuh (tcgen05 + TMA) and apollo_mma.cuh (mma.sync).
 #pragma once
 
+#include <algorithm>
+
 #include <cstdlib>
 #include <cstring>
 
@@ -904,6 +906,15 @@ extern "C" int af8_apollo_project_batch(const af8_apollo_proj_desc *descs, int32
         if (rc) return rc;
     }
     if (iu) {
+        // The persistent CTAs deal the tiles out in turn and a tile costs its K: long ones first, so that the last round
+        // is one of short ones (four Llama-3-8B layers: 1600 tiles of K = 4096 and 256 of K = 1024 over 148 CTAs:
+        // 1466 -> 1328 us).
+        std::sort(host_u, host_u + iu, [](const UmmaTask &a, const UmmaTask &b) { return a.t.K > b.t.K; });
+        int tile = 0;
+        for (int i = 0; i < iu; ++i) {
+            host_u[i].t.first_tile = tile;
+            tile += (host_u[i].t.M + UM_BM - 1) / UM_BM;
+        }
         AF8_CUDA_TRY(cudaMemcpyAsync(dev_scratch, host_u, sizeof(UmmaTask) * (size_t)iu, cudaMemcpyHostToDevice, st));
         int rc = apollo_project_launch_umma(dev_u, iu, tiles_u, st);
         if (rc) return rc;
