@@ -836,6 +836,15 @@ class Adafactor8Bit(Optimizer):
             v_fmt = st.get("v_quant_type", "al8") if quant else "fp32"
             key = (p.device, g.dtype, v_fmt, m_fmt, st.get("block_size", group.get("block_size", 2048)), m_block, p.dtype)
             fullrank.setdefault(key, []).append(ent)
+        # Without momentum the matrices join the batches' plan where these hold most of the elements: the passes are the
+        # same, and a plan costs nine launches.  (Its sum pass is a third slower per element than the one for matrices
+        # alone, so that a model of matrices with a few batches keeps two plans.)
+        for key in [k for k in factored_items if k[6] and k[2] is None and k[:6] + (False,) in factored_items]:
+            flat = factored_items[key[:6] + (False,)]
+            if (sum(e[1].numel() for e in flat) <= sum(e[1].numel() for e in factored_items[key])
+                    and all(e[1].shape[-1] % 8 == 0 for e in flat + factored_items[key])):
+                factored_items[key] = sorted(flat + factored_items[key], key=lambda e: e[0])
+                del factored_items[key[:6] + (False,)]
         out = [(self._run_fullrank, key, items) for key, items in fullrank.items()]
         out += [(self._run_factored, key, items) for key, items in factored_items.items()]
         if apollo_items:

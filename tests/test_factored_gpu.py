@@ -87,6 +87,12 @@ EXTRA_CASES.update({
     "adafactor_any_3d": dict(shapes=_ANY3, steps=3, seed=58, grad=cases.CASES["adafactor_factored"]["grad"],
                              hp=cases.CASES["adafactor_factored"]["hp"]),
     "came_any_3d": dict(shapes=_ANY3, steps=3, seed=59, grad=cases.CASES["came_al16"]["grad"], hp=cases.CASES["came_al16"]["hp"]),
+    # matrices that join the batches' table (no momentum, batches hold most elements), and a CAME table where only some
+    # tensors have columns of a multiple of 256
+    "adafactor_mixed_3d": dict(shapes=[(3, 70, 40), (64, 264), (2, 600, 72), (9, 8)], steps=3, seed=61,
+                               grad=cases.CASES["adafactor_factored"]["grad"], hp=cases.CASES["adafactor_factored"]["hp"]),
+    "came_mixed_cols": dict(shapes=[(70, 512), (37, 264), (530, 256), (5, 1376)], steps=3, seed=62,
+                            grad=cases.CASES["came_al16"]["grad"], hp=cases.CASES["came_al16"]["hp"]),
     "adafactor_m_256_3d": dict(shapes=[(3, 40, 256), (2, 530, 512)], steps=3, seed=60,
                                grad=cases.CASES["adafactor_factored_m"]["grad"], hp=cases.CASES["adafactor_factored_m"]["hp"]),
 })
