@@ -680,7 +680,7 @@ __device__ __forceinline__ void m_old8(const af8_factored_tensor &T, int m_fmt, 
                                        bool have_pre = false, uint2 pre = make_uint2(0u, 0u))
 {
     if (m_fmt == AF8_M_FP32) { load_f8(T.m_f32 + flat, m); return; }
-    const float sc = __ldg(T.m_scale + flat / m_block);
+    const float sc = __ldg(T.m_scale + (m_block == 256 ? flat >> 8 : flat / m_block));
     if (m_fmt == AF8_M_UF8) {
         const uint2 w = have_pre ? pre : *reinterpret_cast<const uint2 *>(T.m_q + flat);
         const float mc = __fmul_rn(sc, 0.0078125f);      // fl(scale / 128): a power-of-two divisor, scale >= 1e-12
@@ -1483,11 +1483,11 @@ factored_update_vec_kernel(const FactoredLaunch L)
             if (pre_m) cm = *reinterpret_cast<const uint2 *>(sT.m_q + flat);
         } else cg.zero();
 #if AF8_FUPD_PREFETCH_AHEAD > 0
-        if (writes && !has_m) {
+        if (writes && (!has_m || ANY == 2)) {
             // The momentum-free write pass asks L2 for the chunk a few iterations ahead (same tensor), one
             // request per 128-byte line: measured on the TinyLlama set 2.33 -> 1.89 ms (5.8 TB/s).  The
             // passes with momentum and the sum passes were measured slower with it (CAME apply 24.9 ->
-            // 25.6 ms, sums 0.87 -> 0.94 ms), so they go without.
+            // 25.6 ms, sums 0.87 -> 0.94 ms), so they go without; rows of any length, whose loads wait longer, gain with one too (252 -> 238 us, 59 M parameters).
             const int64_t pf = flat + (int64_t)AF8_FUPD_PREFETCH_AHEAD * 2048;
             if (id + AF8_FUPD_PREFETCH_AHEAD < id_end && pf < numel) {
                 constexpr int GB = sizeof_grad<GradT>();
@@ -2426,7 +2426,8 @@ static int af8_factored_stats_impl(const af8_factored_cfg *cfg, const af8_factor
     const bool any = cfg->aligned8 == 2;
     int ring = (ring_off || !res || any) ? 0 : 1;
     // residual pass over bf16 gradients and UF8 codes of tensors with cols % 256 == 0: boxes of rows through
-    // tensor maps, when the caller has given room for the maps
+    // tensor maps, when the caller has given room for the maps.  (In tables where only some tensors qualify they were
+    // slower than row copies: 117 against 97 us on an 8-layer 512 x 1376 model.)
     const CUtensorMap *maps = nullptr;
     if (ring && !box_off && vec && bf && host_maps && dev_maps && cfg->m_fmt == AF8_M_UF8 && cfg->m_block == 256 && cfg->cols_mult256) {
         bool ok = (reinterpret_cast<uintptr_t>(dev_maps) & 63) == 0;
