@@ -321,6 +321,8 @@ class FullrankPlan:
         for k in ("decay", "alpha", "v_w", "v_keep", "v_eps_add", "m_w", "eps_gradsq", "eps_denom", "eps_sq"):
             table[k] = scalars[k]
         table["sr_base"] = scalars.get("sr_base", 0)
+        if self.cfg.use_adam_denom:
+            self.cfg.use_adam_denom = N.ADAM_DENOM_EPS_HIDES if np.min(scalars["eps_denom"]) >= N.EPS_HIDES else 1
         return buf, table
 
     # -- launches ------------------------------------------------------------

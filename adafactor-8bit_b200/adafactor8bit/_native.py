@@ -18,6 +18,7 @@ F32, BF16, F16 = 0, 1, 2
 V_FP32, V_AL8, V_AL16 = 0, 8, 16
 M_NONE, M_UF8, M_UF4, M_D8, M_D4, M_FP32 = 0, 1, 2, 3, 4, 5
 MODE_NOCLIP, MODE_SUMSQ, MODE_APPLY, MODE_SUMSQ_M, MODE_LAG = 0, 1, 2, 3, 4
+ADAM_DENOM_EPS_HIDES, EPS_HIDES = 2, 2.0 ** -38      # FullrankCfg.use_adam_denom; the eps from which it may be set
 
 V_NONE = 1
 V_FMT = {"fp32": V_FP32, "al8": V_AL8, "al16": V_AL16, "none": V_NONE}

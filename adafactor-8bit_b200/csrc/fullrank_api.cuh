@@ -155,11 +155,11 @@ inline int persistent_grid(K kernel, int threads, size_t smem, int64_t total_blo
     return AF8_OK;
 }
 
-template <typename GradT, typename ParamT, int VB, int MF, bool SR, bool LAG>
+template <typename GradT, typename ParamT, int VB, int MF, bool SR, bool LAG, bool FTZ>
 inline int launch_fast(const FullrankLaunch &L, cudaStream_t st)
 {
     using Ring = FastRing<GradT, ParamT, VB, MF>;
-    auto kernel = fullrank_fast_kernel<GradT, ParamT, VB, MF, SR, LAG>;
+    auto kernel = fullrank_fast_kernel<GradT, ParamT, VB, MF, SR, LAG, FTZ>;
     // the ring lives in dynamic shared memory (up to 44 KB per CTA): opt in and ask for the large
     // shared-memory carve-out
     AF8_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring::SMEM_BYTES));
@@ -241,36 +241,36 @@ inline bool fast_covers(const af8_fullrank_cfg &c)
 }
 
 template <typename GradT, typename ParamT, bool SR, int VB, int MF>
-inline int dispatch_fast_mode(int mode, FullrankLaunch L, cudaStream_t st)
+inline int dispatch_fast_mode(int mode, FullrankLaunch L, bool eps_hides, cudaStream_t st)
 {
     if (mode == AF8_MODE_SUMSQ) return launch_stat<GradT, VB, MF>(L, st);
     if constexpr (VB == 8 && MF == AF8_M_UF8) {
-        if (mode == AF8_MODE_LAG) return launch_fast<GradT, ParamT, VB, MF, SR, true>(L, st);
+        if (mode == AF8_MODE_LAG) return launch_fast<GradT, ParamT, VB, MF, SR, true, false>(L, st);
     }
     if (mode == AF8_MODE_NOCLIP) L.dyn = nullptr;        // the step size is the table's
-    return launch_fast<GradT, ParamT, VB, MF, SR, false>(L, st);
+    return eps_hides ? launch_fast<GradT, ParamT, VB, MF, SR, false, true>(L, st) : launch_fast<GradT, ParamT, VB, MF, SR, false, false>(L, st);
 }
 
 template <typename GradT, typename ParamT, bool SR>
-inline int dispatch_fast_formats(const af8_fullrank_cfg &c, const FullrankLaunch &L, cudaStream_t st)
+inline int dispatch_fast_formats(const af8_fullrank_cfg &c, const FullrankLaunch &L, bool eps_hides, cudaStream_t st)
 {
     if (c.v_fmt == AF8_V_AL8) {
-        if (c.m_fmt == AF8_M_UF8) return dispatch_fast_mode<GradT, ParamT, SR, 8, AF8_M_UF8>(c.mode, L, st);
-        if (c.m_fmt == AF8_M_UF4) return dispatch_fast_mode<GradT, ParamT, SR, 8, AF8_M_UF4>(c.mode, L, st);
-        return dispatch_fast_mode<GradT, ParamT, SR, 8, AF8_M_NONE>(c.mode, L, st);
+        if (c.m_fmt == AF8_M_UF8) return dispatch_fast_mode<GradT, ParamT, SR, 8, AF8_M_UF8>(c.mode, L, eps_hides, st);
+        if (c.m_fmt == AF8_M_UF4) return dispatch_fast_mode<GradT, ParamT, SR, 8, AF8_M_UF4>(c.mode, L, eps_hides, st);
+        return dispatch_fast_mode<GradT, ParamT, SR, 8, AF8_M_NONE>(c.mode, L, eps_hides, st);
     }
-    if (c.m_fmt == AF8_M_UF8) return dispatch_fast_mode<GradT, ParamT, SR, 16, AF8_M_UF8>(c.mode, L, st);
-    if (c.m_fmt == AF8_M_UF4) return dispatch_fast_mode<GradT, ParamT, SR, 16, AF8_M_UF4>(c.mode, L, st);
-    return dispatch_fast_mode<GradT, ParamT, SR, 16, AF8_M_NONE>(c.mode, L, st);
+    if (c.m_fmt == AF8_M_UF8) return dispatch_fast_mode<GradT, ParamT, SR, 16, AF8_M_UF8>(c.mode, L, eps_hides, st);
+    if (c.m_fmt == AF8_M_UF4) return dispatch_fast_mode<GradT, ParamT, SR, 16, AF8_M_UF4>(c.mode, L, eps_hides, st);
+    return dispatch_fast_mode<GradT, ParamT, SR, 16, AF8_M_NONE>(c.mode, L, eps_hides, st);
 }
 
-// c must satisfy fast_covers
-inline int dispatch_fast(const af8_fullrank_cfg &c, const FullrankLaunch &L, cudaStream_t st)
+// c must satisfy fast_covers; eps_hides: every eps_denom of the table is at least EPS_HIDES (fullrank_fast.cuh)
+inline int dispatch_fast(const af8_fullrank_cfg &c, const FullrankLaunch &L, bool eps_hides, cudaStream_t st)
 {
     if (c.param_dtype == AF8_BF16)
-        return c.stochastic_round ? dispatch_fast_formats<bf16_tag, bf16_tag, true>(c, L, st) : dispatch_fast_formats<bf16_tag, bf16_tag, false>(c, L, st);
-    if (c.grad_dtype == AF8_BF16) return dispatch_fast_formats<bf16_tag, float, false>(c, L, st);
-    return dispatch_fast_formats<float, float, false>(c, L, st);
+        return c.stochastic_round ? dispatch_fast_formats<bf16_tag, bf16_tag, true>(c, L, eps_hides, st) : dispatch_fast_formats<bf16_tag, bf16_tag, false>(c, L, eps_hides, st);
+    if (c.grad_dtype == AF8_BF16) return dispatch_fast_formats<bf16_tag, float, false>(c, L, eps_hides, st);
+    return dispatch_fast_formats<float, float, false>(c, L, eps_hides, st);
 }
 
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -356,7 +356,14 @@ extern "C" int af8_fullrank_step(const af8_fullrank_cfg *cfg, const af8_fullrank
     L.sr = c.stochastic_round ? 1 : 0;
     GenericCfg C{c.v_fmt, c.m_fmt, c.block, c.m_block, c.use_adam_denom ? 1 : 0, c.momentum_only ? 1 : 0};
 
-    if (fast_covers(c)) return dispatch_fast(c, L, st);
+    if (fast_covers(c)) {
+        bool eps_hides = c.use_adam_denom == AF8_ADAM_DENOM_EPS_HIDES;
+        if (host_tensors) {
+            eps_hides = true;
+            for (int i = 0; i < n_tensors; ++i) eps_hides = eps_hides && host_tensors[i].eps_denom >= EPS_HIDES;
+        }
+        return dispatch_fast(c, L, eps_hides, st);
+    }
     if (c.grad_dtype == AF8_BF16) return dispatch_generic<bf16_tag>(c.mode, L, C, st);
     if (c.grad_dtype == AF8_F16) return dispatch_generic<f16_tag>(c.mode, L, C, st);
     return dispatch_generic<float>(c.mode, L, C, st);

@@ -50,7 +50,8 @@
 //     quotient;
 //   * the parameter update u = m / (sqrt(v) + eps) feeds nothing but the fp32
 //     parameter, whose tolerance is relative 1e-5; it uses the hardware
-//     approximations of sqrt and reciprocal (relative error below 3e-7).
+//     approximations of sqrt and reciprocal (relative error below 3e-7, for subnormal
+//     second moments too: see EPS_HIDES).
 //
 // Measured on a B200, before -> after the split by sixteen elements (and, for the formats other
 // than UF8/AL8, against the general kernel): TinyLlama-1.1B update pass 3.23 -> 2.9 ms (5.3 TB/s);
@@ -139,18 +140,26 @@ template <> struct GradLoad<bf16_tag> {
     }
 };
 
-// hardware approximations (flush-to-zero forms: one MUFU instruction each, no
-// subnormal fix-up code), used only where the result does not reach a stored state
+// Hardware approximations, used only where the result does not reach a stored state.  FTZ: the flush-to-zero
+// forms, one MUFU instruction each; without it subnormal operands and results keep their value, at three more
+// instructions.  A second moment below 2^-126 has a square root below 2^-63, which an eps of 2^-38 (EPS_HIDES)
+// or more absorbs whole; below that eps the square root is the denominator and must not be flushed: with the
+// constructor's eps of 1e-30 a first gradient of 1e-18 would otherwise give an update of 1e12 instead of 31.6.
+constexpr float EPS_HIDES = 0x1p-38f;
+template <bool FTZ>
 __device__ __forceinline__ float sqrt_approx(float x)
 {
     float y;
-    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    if (FTZ) asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    else asm("sqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+template <bool FTZ>
 __device__ __forceinline__ float rcp_approx(float x)
 {
     float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    if (FTZ) asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    else asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
 __device__ __forceinline__ float lg2_approx(float x)
@@ -403,7 +412,8 @@ template <typename GradT, typename ParamT, int VB, int MF> struct FastRing {
 
 // Eight elements (two groups of four) of one momentum block: EMAs, update, new parameter.
 // PLAIN: the common scalars (see StepScalars::plain).  LAG: sumsq += u^2 over the elements whose bit is set in real.
-template <int MF, bool PLAIN, bool ROUND_DECAY, bool LAG>
+// FTZ: see sqrt_approx.
+template <int MF, bool PLAIN, bool ROUND_DECAY, bool LAG, bool FTZ>
 __device__ __forceinline__ void fast_ema8(const StepScalars &S, const float2 (&g)[4], const float2 (&v_old)[4], const float2 (&m_old)[4],
                                           float2 (&p)[4], float2 (&v)[4], float2 (&m)[4], uint32_t real, float &sumsq)
 {
@@ -422,8 +432,8 @@ __device__ __forceinline__ void fast_ema8(const StepScalars &S, const float2 (&g
         else if (PLAIN) m[j] = __ffma2_rn(w_m, sub2(g[j], m_old[j]), m_old[j]);
         else m[j] = make_float2(lerp_t(m_old[j].x, g[j].x, S.m_w), lerp_t(m_old[j].y, g[j].y, S.m_w));
         // update from the un-requantised v and m (optimizer.py:905, 909); feeds the parameter only
-        const float2 den = __fadd2_rn(make_float2(sqrt_approx(v[j].x), sqrt_approx(v[j].y)), eps_d2);
-        float2 u = __fmul2_rn(m[j], make_float2(rcp_approx(den.x), rcp_approx(den.y)));
+        const float2 den = __fadd2_rn(make_float2(sqrt_approx<FTZ>(v[j].x), sqrt_approx<FTZ>(v[j].y)), eps_d2);
+        float2 u = __fmul2_rn(m[j], make_float2(rcp_approx<FTZ>(den.x), rcp_approx<FTZ>(den.y)));
         if (LAG) {                                                // (padding may be 0 * inf)
             if ((real >> (2 * j)) & 1u) sumsq = __fmaf_rn(u.x, u.x, sumsq);
             if ((real >> (2 * j + 1)) & 1u) sumsq = __fmaf_rn(u.y, u.y, sumsq);
@@ -596,8 +606,10 @@ __device__ __forceinline__ void fast_round8(const float2 (&p)[4], uint64_t sr_ba
 }
 
 // SR: bf16 parameters rounded stochastically.  LAG: the scalars are those of the previous step and the
-// sum of squares of this step's raw update goes to block_sumsq.
-template <typename GradT, typename ParamT, int VB, int MF, bool SR, bool LAG>
+// sum of squares of this step's raw update goes to block_sumsq.  FTZ: every eps of the table is at least EPS_HIDES.
+// (A kernel of its own: chosen per tensor or per block inside one kernel, the two forms cost the common one 2 to 15 %
+// in registers and instruction fetches.  TinyLlama-1.1B, UF8/AL8: 2.69 ms with FTZ, 2.94 ms without.)
+template <typename GradT, typename ParamT, int VB, int MF, bool SR, bool LAG, bool FTZ>
 __global__ void __launch_bounds__(FAST_THREADS, fast_min_ctas<VB>())
 fullrank_fast_kernel(const FullrankLaunch L)
 {
@@ -790,7 +802,7 @@ fullrank_fast_kernel(const FullrankLaunch L)
 #pragma unroll
                     for (int j = 0; j < 4; ++j) g[j] = make_float2(-g[j].x, -g[j].y);
                 }
-                fast_ema8<MF, true, PB == 2 && !SR, LAG>(S, g, v_old, m_old, p, vn, mn, 0xffu, usq);
+                fast_ema8<MF, true, PB == 2 && !SR, LAG, FTZ>(S, g, v_old, m_old, p, vn, mn, 0xffu, usq);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) { v[8 * mb + 2 * j] = vn[j].x; v[8 * mb + 2 * j + 1] = vn[j].y; }
                 PElem *const pa = static_cast<PElem *>(sT.param) + base + oa;
@@ -851,7 +863,7 @@ fullrank_fast_kernel(const FullrankLaunch L)
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
                     if ((j < 4 ? oa : oa + 124) + j < rem) real |= 1u << j;
-                fast_ema8<MF, false, PB == 2 && !SR, LAG>(S, g, v_old, m_old, p, vn, mn, real, usq);
+                fast_ema8<MF, false, PB == 2 && !SR, LAG, FTZ>(S, g, v_old, m_old, p, vn, mn, real, usq);
                 float x[8], q[8];
                 uint32_t w[4] = {0u, 0u, 0u, 0u};
                 if (PB == 2) fast_round8<SR>(p, sT.sr_base, base + oa, w);

@@ -166,7 +166,7 @@ extern "C" int af8_fullrank_limited_step_noalloc(const af8_fullrank_cfg *cfg, co
         cm.mode = mode;
         cm.param_dtype = AF8_F32;
         cm.stochastic_round = 0;
-        if (fast_covers(cm)) return dispatch_fast(cm, L, st);
+        if (fast_covers(cm)) return dispatch_fast(cm, L, row.eps_denom >= EPS_HIDES, st);
         return bf16 ? dispatch_generic<bf16_tag>(mode, L, C, st) : dispatch_generic<float>(mode, L, C, st);
     };
     rc = pass(AF8_MODE_SUMSQ);

@@ -158,6 +158,8 @@ typedef struct af8_fullrank_tensor {
                                Only with cfg.param_dtype == AF8_F32.  No counterpart in the reference. */
 } af8_fullrank_tensor;
 
+#define AF8_ADAM_DENOM_EPS_HIDES 2
+
 /* Launch-wide configuration: everything that selects a kernel variant. */
 typedef struct af8_fullrank_cfg {
     int32_t param_dtype;    /* AF8_F32, AF8_BF16 or AF8_F16.  A 16-bit parameter is rounded to nearest
@@ -168,7 +170,10 @@ typedef struct af8_fullrank_cfg {
     int32_t m_fmt;          /* AF8_M_* */
     int32_t block;          /* V block size: multiple of 128, >= 128 */
     int32_t m_block;        /* M block size: multiple of 4, >= 32, divides block */
-    int32_t use_adam_denom; /* 1: u = m/(sqrt(v)+eps); 0: u = m*rsqrt(max(v,eps_sq)) */
+    int32_t use_adam_denom; /* 1: u = m/(sqrt(v)+eps); 0: u = m*rsqrt(max(v,eps_sq)).  AF8_ADAM_DENOM_EPS_HIDES: as
+                               1, and every eps_denom of the table is at least 2^-38, so that the square root of a
+                               subnormal v vanishes in it; a launch without host_tensors may then use the faster
+                               arithmetic that a launch with them finds out by itself */
     int32_t momentum_only;  /* 1: momentum is the EMA of the normalised gradient */
     int32_t negate_grad;    /* maximize */
     int32_t mode;           /* AF8_MODE_* */
