@@ -155,11 +155,11 @@ inline int persistent_grid(K kernel, int threads, size_t smem, int64_t total_blo
     return AF8_OK;
 }
 
-template <typename GradT, typename ParamT, int VB, int MF, bool SR, bool LAG, bool FTZ>
+template <typename GradT, typename ParamT, int VB, int MF, bool SR, bool LAG, int ROOT>
 inline int launch_fast(const FullrankLaunch &L, cudaStream_t st)
 {
     using Ring = FastRing<GradT, ParamT, VB, MF>;
-    auto kernel = fullrank_fast_kernel<GradT, ParamT, VB, MF, SR, LAG, FTZ>;
+    auto kernel = fullrank_fast_kernel<GradT, ParamT, VB, MF, SR, LAG, ROOT>;
     // the ring lives in dynamic shared memory (up to 44 KB per CTA): opt in and ask for the large
     // shared-memory carve-out
     AF8_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring::SMEM_BYTES));
@@ -245,10 +245,11 @@ inline int dispatch_fast_mode(int mode, FullrankLaunch L, bool eps_hides, cudaSt
 {
     if (mode == AF8_MODE_SUMSQ) return launch_stat<GradT, VB, MF>(L, st);
     if constexpr (VB == 8 && MF == AF8_M_UF8) {
-        if (mode == AF8_MODE_LAG) return launch_fast<GradT, ParamT, VB, MF, SR, true, false>(L, st);
+        if (mode == AF8_MODE_LAG) return launch_fast<GradT, ParamT, VB, MF, SR, true, ROOT_FULL>(L, st);
     }
     if (mode == AF8_MODE_NOCLIP) L.dyn = nullptr;        // the step size is the table's
-    return eps_hides ? launch_fast<GradT, ParamT, VB, MF, SR, false, true>(L, st) : launch_fast<GradT, ParamT, VB, MF, SR, false, false>(L, st);
+    constexpr int HIDES = root_exact<VB, MF> ? ROOT_REFINED : ROOT_FTZ, SHOWS = root_exact<VB, MF> ? ROOT_EXACT : ROOT_FULL;
+    return eps_hides ? launch_fast<GradT, ParamT, VB, MF, SR, false, HIDES>(L, st) : launch_fast<GradT, ParamT, VB, MF, SR, false, SHOWS>(L, st);
 }
 
 template <typename GradT, typename ParamT, bool SR>

@@ -48,15 +48,17 @@
 //   * the momentum division m/absmax uses the correctly rounded reciprocal of
 //     the block's absmax with one residual correction, which yields the IEEE
 //     quotient;
-//   * the parameter update u = m / (sqrt(v) + eps) feeds nothing but the fp32
-//     parameter, whose tolerance is relative 1e-5; it uses the hardware
-//     approximations of sqrt and reciprocal (relative error below 3e-7, for subnormal
-//     second moments too: see EPS_HIDES).
+//   * the parameter update u = m / (sqrt(v) + eps) feeds nothing but the
+//     parameter; with UF8/AL8 it uses the hardware approximations of sqrt and
+//     reciprocal (relative error below 3e-7, for subnormal second moments too: see
+//     EPS_HIDES), with every other format the correctly rounded operations.
 //
 // Measured on a B200, before -> after the split by sixteen elements (and, for the formats other
-// than UF8/AL8, against the general kernel): TinyLlama-1.1B update pass 3.23 -> 2.9 ms (5.3 TB/s);
-// bf16 parameters with stochastic rounding 5.0 -> 3.6 ms; UF4/AL16, 176 M parameters 4.17 -> 0.90 ms;
-// AL8 without momentum, fp32 gradients, 110 M parameters 1.95 -> 0.31 ms (4.9 TB/s).
+// than UF8/AL8, against the general kernel): TinyLlama-1.1B update pass 3.23 -> 2.8 ms (5.5 TB/s);
+// bf16 parameters with stochastic rounding 5.0 -> 3.75 ms; UF4/AL16, 176 M parameters 4.17 -> 0.99 ms;
+// AL8 without momentum, fp32 gradients, 110 M parameters 1.95 -> 0.32 ms (4.9 TB/s).  The correctly
+// rounded update of these formats (ROOT_REFINED) costs 5 to 12 % of that against the hardware
+// approximations; with the IEEE functions it cost 30 %.
 #pragma once
 
 #include "common.cuh"
@@ -68,7 +70,7 @@ constexpr int FAST_MBLOCK = 256;
 constexpr int FAST_THREADS = 128;
 constexpr int FAST_EPT = 16;  // elements per thread
 constexpr int FAST_WARPS = FAST_THREADS / 32;
-// resident CTAs asked of the compiler (AL8: 5 -> 6 gave 1-3 %; AL16: 3, 4 and 5 gave 0.93, 0.91 and 0.97 ms on the UF4/AL16 case)
+// resident CTAs asked of the compiler (AL8: 5 -> 6 gave 1-3 %; AL16: 3, 4 and 5 gave 0.93, 0.91 and 0.97 ms on 176 M UF4/AL16 parameters, before ROOT_REFINED)
 #ifndef AF8_FAST_CTAS8
 #define AF8_FAST_CTAS8 6
 #endif
@@ -140,27 +142,65 @@ template <> struct GradLoad<bf16_tag> {
     }
 };
 
-// Hardware approximations, used only where the result does not reach a stored state.  FTZ: the flush-to-zero
-// forms, one MUFU instruction each; without it subnormal operands and results keep their value, at three more
-// instructions.  A second moment below 2^-126 has a square root below 2^-63, which an eps of 2^-38 (EPS_HIDES)
-// or more absorbs whole; below that eps the square root is the denominator and must not be flushed: with the
-// constructor's eps of 1e-30 a first gradient of 1e-18 would otherwise give an update of 1e12 instead of 31.6.
+// How the update m / (sqrt(v) + eps) is formed.  It feeds nothing but the parameter and the norm.
+//   ROOT_EXACT    every operation correctly rounded, as in the general kernel; every format pair but UF8/AL8
+//   ROOT_REFINED  the same numbers from the hardware approximations and one residual step each (Markstein 1990), in packed
+//                 arithmetic: a third of the instructions of the IEEE functions.  Above EPS_HIDES (below) only: a residual
+//                 of v < 2^-100 may be subnormal, but no bit of such a square root survives the addition of eps
+//   ROOT_FTZ      hardware approximations in their flush-to-zero forms, one MUFU instruction each (UF8/AL8; relative error
+//                 below 3e-7).  A second moment below 2^-126 has a square root below 2^-63, which an eps of 2^-38
+//                 (EPS_HIDES) or more absorbs whole; below that eps the square root is the denominator and must not be
+//                 flushed: with the constructor's eps of 1e-30 a first gradient of 1e-18 would otherwise give an update
+//                 of 1e12 instead of 31.6
+//   ROOT_FULL     the approximations without the flush, three more instructions each (UF8/AL8 below EPS_HIDES)
 constexpr float EPS_HIDES = 0x1p-38f;
-template <bool FTZ>
-__device__ __forceinline__ float sqrt_approx(float x)
+constexpr int ROOT_FTZ = 0, ROOT_FULL = 1, ROOT_EXACT = 2, ROOT_REFINED = 3;
+template <int VB, int MF> constexpr bool root_exact = !(VB == 8 && MF == AF8_M_UF8);
+template <int ROOT>
+__device__ __forceinline__ float root_sqrt(float x)
 {
+    if (ROOT == ROOT_EXACT) return __fsqrt_rn(x);
     float y;
-    if (FTZ) asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    if (ROOT == ROOT_FTZ) asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     else asm("sqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-template <bool FTZ>
-__device__ __forceinline__ float rcp_approx(float x)
+template <int ROOT>
+__device__ __forceinline__ float root_rcp(float x)
+{
+    if (ROOT == ROOT_EXACT) return __frcp_rn(x);
+    float y;
+    if (ROOT == ROOT_FULL) asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+    else asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rsqrt_approx(float x)
 {
     float y;
-    if (FTZ) asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    else asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+// the updates of two elements from the un-requantised m and v (optimizer.py:905, 909); without momentum m is the gradient
+// and the reference divides (optimizer.py:911-917)
+template <int MF, int ROOT>
+__device__ __forceinline__ float2 root_update2(float2 m, float2 v, float2 eps)
+{
+    if (ROOT == ROOT_REFINED) {
+        const float2 one = make_float2(1.0f, 1.0f), neg = make_float2(-1.0f, -1.0f);
+        const float2 y = make_float2(rsqrt_approx(fmaxf(v.x, 0x1p-126f)), rsqrt_approx(fmaxf(v.y, 0x1p-126f)));     // (zero: s = 0)
+        const float2 s = __fmul2_rn(v, y);
+        const float2 root = __ffma2_rn(__ffma2_rn(s, s, __fmul2_rn(v, neg)), __fmul2_rn(y, make_float2(-0.5f, -0.5f)), s);
+        float2 den = __fadd2_rn(root, eps);
+        // (an infinite v has made it NaN: its reciprocal is zero, like that of the largest number, which is flushed)
+        den = make_float2(fminf(den.x, 3.402823466e38f), fminf(den.y, 3.402823466e38f));
+        const float2 nd = __fmul2_rn(den, neg), r = make_float2(root_rcp<ROOT>(den.x), root_rcp<ROOT>(den.y));
+        const float2 inv = __ffma2_rn(__ffma2_rn(nd, r, one), r, r);
+        const float2 u = __fmul2_rn(m, inv);
+        return MF == AF8_M_NONE ? __ffma2_rn(__ffma2_rn(nd, u, m), inv, u) : u;
+    }
+    const float2 den = __fadd2_rn(make_float2(root_sqrt<ROOT>(v.x), root_sqrt<ROOT>(v.y)), eps);
+    if (ROOT == ROOT_EXACT && MF == AF8_M_NONE) return make_float2(__fdiv_rn(m.x, den.x), __fdiv_rn(m.y, den.y));
+    return __fmul2_rn(m, make_float2(root_rcp<ROOT>(den.x), root_rcp<ROOT>(den.y)));
 }
 __device__ __forceinline__ float lg2_approx(float x)
 {
@@ -269,7 +309,7 @@ __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.
 // their bits where they can (conversions run at a quarter of the rate of the arithmetic).
 struct LaneTables {
     double e2;          // 2^(lane/32)
-    double l2;          // -log2(inv) of interval `lane`
+    double l2;          // -log2(inv) of centre `lane`
     uint32_t inv_hi;    // high word of inv
 };
 struct LogLaneEntry { uint32_t inv_hi; double l2; };
@@ -296,20 +336,22 @@ __device__ __forceinline__ float exp2_lane(float x, const LaneTables &T)
     return __double2float_rn(__hiloint2double(__double2hiint(y) + (((n - 0x4b400000) >> 5) << 20), __double2loint(y)));
 }
 
-// Correctly rounded log2 of a positive normal x (up to the error 2^-52 of the sum before the last
-// rounding): x = 2^e * m, m in [1, 2); the leading five fraction bits select inv_j, r = m*inv_j - 1 is
-// exact (24 + 21 bits) with |r| < 2^-6, log2(1 + r) by its Taylor series through r^8 (truncation below
-// 2^-56).  Next to x = 1 the result is absolutely, not relatively, accurate: for codes, not for ranges.
+// Correctly rounded log2 of a positive normal x (up to the relative error 2^-52 of the sum before the last
+// rounding): x = 2^e * m with m in [63/64, 127/64); the nearest of the 32 centres 1 + j/32 selects inv_j,
+// r = m*inv_j - 1 is exact (24 + 21 bits) with |r| <= 2^-6, log2(1 + r) by its Taylor series through r^9 (truncation
+// below 2^-57 of r).  Around x = 1 the centre is 1 itself, inv = 1 and the table entry 0, so that the result stays
+// relatively accurate there.
 __device__ __forceinline__ float log2_lane(float x, const LaneTables &T)
 {
-    const uint32_t b = __float_as_uint(x);
-    const int j = (b >> 18) & 31;
-    const double m = __hiloint2double((int)(0x3ff00000u | ((b >> 3) & 0xfffffu)), (int)(b << 29));
+    const uint32_t b = __float_as_uint(x), near = b + 0x20000u;
+    const int j = (near >> 18) & 31;
+    const double m = __hiloint2double((int)((b >> 3) - ((near >> 23) << 20) + 0x3ff00000u), (int)(b << 29));
     const double inv = __hiloint2double((int)__shfl_sync(0xffffffffu, T.inv_hi, j), 0);
     const double tab = __shfl_sync(0xffffffffu, T.l2, j);
-    const double e = __hiloint2double(0x43300000, (int)(b >> 23)) - (4503599627370496.0 + 127.0);
+    const double e = __hiloint2double(0x43300000, (int)(near >> 23)) - (4503599627370496.0 + 127.0);
     const double r = fma(m, inv, -1.0);
-    double p = -0x1.71547652b82fep-3;       // -1/(8 ln 2)
+    double p = 0x1.484b13d7c02a9p-3;        //  1/(9 ln 2)
+    p = fma(p, r, -0x1.71547652b82fep-3);   // -1/(8 ln 2)
     p = fma(p, r, 0x1.a61762a7adedap-3);    //  1/(7 ln 2)
     p = fma(p, r, -0x1.ec709dc3a03fep-3);   // -1/(6 ln 2)
     p = fma(p, r, 0x1.2776c50ef9bfep-2);    //  1/(5 ln 2)
@@ -412,8 +454,8 @@ template <typename GradT, typename ParamT, int VB, int MF> struct FastRing {
 
 // Eight elements (two groups of four) of one momentum block: EMAs, update, new parameter.
 // PLAIN: the common scalars (see StepScalars::plain).  LAG: sumsq += u^2 over the elements whose bit is set in real.
-// FTZ: see sqrt_approx.
-template <int MF, bool PLAIN, bool ROUND_DECAY, bool LAG, bool FTZ>
+// ROOT: see ROOT_EXACT.
+template <int MF, bool PLAIN, bool ROUND_DECAY, bool LAG, int ROOT>
 __device__ __forceinline__ void fast_ema8(const StepScalars &S, const float2 (&g)[4], const float2 (&v_old)[4], const float2 (&m_old)[4],
                                           float2 (&p)[4], float2 (&v)[4], float2 (&m)[4], uint32_t real, float &sumsq)
 {
@@ -431,9 +473,7 @@ __device__ __forceinline__ void fast_ema8(const StepScalars &S, const float2 (&g
         if (MF == AF8_M_NONE) m[j] = g[j];
         else if (PLAIN) m[j] = __ffma2_rn(w_m, sub2(g[j], m_old[j]), m_old[j]);
         else m[j] = make_float2(lerp_t(m_old[j].x, g[j].x, S.m_w), lerp_t(m_old[j].y, g[j].y, S.m_w));
-        // update from the un-requantised v and m (optimizer.py:905, 909); feeds the parameter only
-        const float2 den = __fadd2_rn(make_float2(sqrt_approx<FTZ>(v[j].x), sqrt_approx<FTZ>(v[j].y)), eps_d2);
-        float2 u = __fmul2_rn(m[j], make_float2(rcp_approx<FTZ>(den.x), rcp_approx<FTZ>(den.y)));
+        float2 u = root_update2<MF, ROOT>(m[j], v[j], eps_d2);
         if (LAG) {                                                // (padding may be 0 * inf)
             if ((real >> (2 * j)) & 1u) sumsq = __fmaf_rn(u.x, u.x, sumsq);
             if ((real >> (2 * j + 1)) & 1u) sumsq = __fmaf_rn(u.y, u.y, sumsq);
@@ -606,10 +646,10 @@ __device__ __forceinline__ void fast_round8(const float2 (&p)[4], uint64_t sr_ba
 }
 
 // SR: bf16 parameters rounded stochastically.  LAG: the scalars are those of the previous step and the
-// sum of squares of this step's raw update goes to block_sumsq.  FTZ: every eps of the table is at least EPS_HIDES.
+// sum of squares of this step's raw update goes to block_sumsq.  ROOT_FTZ: every eps of the table is at least EPS_HIDES.
 // (A kernel of its own: chosen per tensor or per block inside one kernel, the two forms cost the common one 2 to 15 %
-// in registers and instruction fetches.  TinyLlama-1.1B, UF8/AL8: 2.69 ms with FTZ, 2.94 ms without.)
-template <typename GradT, typename ParamT, int VB, int MF, bool SR, bool LAG, bool FTZ>
+// in registers and instruction fetches.  TinyLlama-1.1B, UF8/AL8: 2.69 ms with ROOT_FTZ, 2.94 ms with ROOT_FULL.)
+template <typename GradT, typename ParamT, int VB, int MF, bool SR, bool LAG, int ROOT>
 __global__ void __launch_bounds__(FAST_THREADS, fast_min_ctas<VB>())
 fullrank_fast_kernel(const FullrankLaunch L)
 {
@@ -784,7 +824,8 @@ fullrank_fast_kernel(const FullrankLaunch L)
         }
 
         const StepScalars S = sS;
-        const bool hot = full && S.plain;    // (uniform over the CTA)
+        // (uniform over the CTA; a block that decodes to NaN takes the general forms: ROOT_REFINED would lose the NaN)
+        const bool hot = full && S.plain && (ROOT != ROOT_REFINED || csc <= 3.402823466e38f);
         float v[FAST_EPT];                   // hot blocks: the new second moments
         float usq = 0.0f;                    // LAG: this thread's sum of squares of the raw update
         // Extrema of v.  v >= 0, so the bit patterns order like the values.  The minimum runs over the
@@ -802,7 +843,7 @@ fullrank_fast_kernel(const FullrankLaunch L)
 #pragma unroll
                     for (int j = 0; j < 4; ++j) g[j] = make_float2(-g[j].x, -g[j].y);
                 }
-                fast_ema8<MF, true, PB == 2 && !SR, LAG, FTZ>(S, g, v_old, m_old, p, vn, mn, 0xffu, usq);
+                fast_ema8<MF, true, PB == 2 && !SR, LAG, ROOT>(S, g, v_old, m_old, p, vn, mn, 0xffu, usq);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) { v[8 * mb + 2 * j] = vn[j].x; v[8 * mb + 2 * j + 1] = vn[j].y; }
                 PElem *const pa = static_cast<PElem *>(sT.param) + base + oa;
@@ -863,7 +904,7 @@ fullrank_fast_kernel(const FullrankLaunch L)
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
                     if ((j < 4 ? oa : oa + 124) + j < rem) real |= 1u << j;
-                fast_ema8<MF, false, PB == 2 && !SR, LAG, FTZ>(S, g, v_old, m_old, p, vn, mn, real, usq);
+                fast_ema8<MF, false, PB == 2 && !SR, LAG, root_exact<VB, MF> ? ROOT_EXACT : ROOT>(S, g, v_old, m_old, p, vn, mn, real, usq);
                 float x[8], q[8];
                 uint32_t w[4] = {0u, 0u, 0u, 0u};
                 if (PB == 2) fast_round8<SR>(p, sT.sr_base, base + oa, w);

@@ -4,8 +4,10 @@
 //
 // Nothing computed here reaches a stored state: the sums only produce the norm that
 // feeds the Fira limiter and the RMS clip, i.e. fp32 parameters with a 1e-5 tolerance.
-// So, unlike the update kernel, this pass decodes the second moment with the hardware
-// exp2 (relative error 2^-22) instead of the exact sequence.  One WARP owns one V block
+// So with UF8/AL8 this pass, unlike the update kernel, decodes the second moment with the
+// hardware exp2 (relative error 2^-22) instead of the exact sequence; every other format takes
+// the exact decode (AL16: within one unit in the last place) and correctly rounded updates, as
+// in the general kernel, and adds a lane's squares in groups of eight.  One WARP owns one V block
 // (8 sub-steps of 256 elements, 8 per lane), keeps its sum in registers and writes one
 // float: no block-wide barrier, plain coalesced 64/128-bit loads.  The 256 possible values
 // of the block's codes go into a per-warp shared-memory table first (8 exp2 per lane and
@@ -16,7 +18,7 @@
 // 70 % busy): the table took the pass from 1.04 to 0.93 ms on the TinyLlama set.
 // (Replacing the reciprocal by rsqrt and a short series was measured slower; so were requests for the
 // next block's lines in L2, 0.972 against 0.955 ms.)  AL16 has too many codes for a table: an element
-// costs one exp2 more.
+// costs a polynomial more (176 M UF4/AL16 parameters: 0.30 ms; 0.55 with the binary64 sequence of exp2_lane).
 #pragma once
 
 #include "common.cuh"
@@ -28,19 +30,45 @@ constexpr int STAT_THREADS = 256;
 #ifndef AF8_STAT_MIN_CTAS
 #define AF8_STAT_MIN_CTAS 5
 #endif
+#ifndef AF8_STAT_MIN_CTAS16
+#define AF8_STAT_MIN_CTAS16 3
+#endif
 #ifndef AF8_STAT_UNROLL
 #define AF8_STAT_UNROLL 4
 #endif
 #define AF8_PRAGMA_(x) _Pragma(#x)
 #define AF8_UNROLL_(n) AF8_PRAGMA_(unroll n)
 
-template <bool FTZ>
+template <int ROOT>
 __device__ __forceinline__ float ex2_approx(float x)
 {
     float y;
-    if (FTZ) asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    if (ROOT == ROOT_FTZ) asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     else asm("ex2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+
+// AL16 decode of two codes (optimizer.py:341-349) of a block with min_log >= -125 and a finite scale: the exponent as
+// al16_decode2 rounds it, 2^n times the Taylor polynomial of 2^f for f in [-1/2, 1/2] (truncation 2^-27), error below one
+// unit in the last place.
+__device__ __forceinline__ float2 al16_decode2_stat(uint32_t pair, float scale, float min_log)
+{
+    const uint32_t c0 = pair & 0xffffu, c1 = pair >> 16;
+    const float2 c = __fadd2_rn(make_float2(__uint_as_float(0x4b000000u | c0), __uint_as_float(0x4b000000u | c1)), bc2(-8388609.0f));
+    const float2 t = __fadd2_rn(div2_by(__fmul2_rn(c, bc2(scale)), bc2(1.0f / 65534.0f), bc2(-65534.0f)), bc2(min_log));
+    const float2 z = __fadd2_rn(t, bc2(AF8_MAGIC_F));
+    const float2 f = sub2(t, __fadd2_rn(z, bc2(-AF8_MAGIC_F)));
+    float2 p = bc2(1.52527338e-5f);                       // ln(2)^7 / 7!
+    p = __ffma2_rn(p, f, bc2((float)AF8_EXP2_C6));
+    p = __ffma2_rn(p, f, bc2((float)AF8_EXP2_C5));
+    p = __ffma2_rn(p, f, bc2((float)AF8_EXP2_C4));
+    p = __ffma2_rn(p, f, bc2((float)AF8_EXP2_C3));
+    p = __ffma2_rn(p, f, bc2((float)AF8_EXP2_C2));
+    p = __ffma2_rn(p, f, bc2((float)AF8_EXP2_C1));
+    p = __ffma2_rn(p, f, bc2(1.0f));
+    // (the low bits of z hold n; code 0 decodes to zero)
+    return make_float2(c0 ? __int_as_float(__float_as_int(p.x) + (__float_as_int(z.x) << 23)) : 0.0f,
+                       c1 ? __int_as_float(__float_as_int(p.y) + (__float_as_int(z.y) << 23)) : 0.0f);
 }
 
 template <typename GradT>
@@ -65,15 +93,21 @@ __device__ __forceinline__ void stat_load_g<bf16_tag>(const void *grad, int64_t 
 }
 
 template <typename GradT, int VB, int MF>
-__global__ void __launch_bounds__(STAT_THREADS, AF8_STAT_MIN_CTAS)
+__global__ void __launch_bounds__(STAT_THREADS, VB == 16 ? AF8_STAT_MIN_CTAS16 : AF8_STAT_MIN_CTAS)
 fullrank_stat_kernel(const FullrankLaunch L)
 {
     // per-warp decode table of the block's 256 second-moment codes: 8 exponentials per lane and block
     // instead of 64 (the special-function pipe is the busiest unit of this pass); entry 0 is exact zero
     constexpr bool TABLE = VB == 8;
     constexpr float M_UNIT = MF == AF8_M_UF4 ? 0.125f : 0.0078125f;
+    constexpr bool EXACT = root_exact<VB, MF>;
     __shared__ float s_dec[STAT_THREADS / 32][TABLE ? 256 : 1];
+    __shared__ double s_exp2[EXACT && TABLE ? 32 : 1];       // copy of the exp2 table of the exact decode
     const int lane = threadIdx.x & 31;
+    if (EXACT && TABLE) {
+        if (threadIdx.x < 32) s_exp2[threadIdx.x] = c_exp2_tab[threadIdx.x];
+        __syncthreads();
+    }
     float *const dec = s_dec[threadIdx.x >> 5];
     const int64_t warps = (int64_t)gridDim.x * (STAT_THREADS / 32);
     const int64_t w0 = (int64_t)blockIdx.x * (STAT_THREADS / 32) + (threadIdx.x >> 5);
@@ -101,27 +135,32 @@ fullrank_stat_kernel(const FullrankLaunch L)
         eps_d = __ldg(&T->eps_denom); eps_g = __ldg(&T->eps_gradsq);
         small_w = fabsf(v_w) < 0.5f && fabsf(m_w) < 0.5f;
 
-        // The blocks of this warp in this tensor, in one of two copies of the loop (see sqrt_approx; TinyLlama-1.1B: 0.95 and 1.24 ms).
+        // The blocks of this warp in this tensor, in one of two copies of the loop (see ROOT_EXACT; TinyLlama-1.1B with UF8/AL8:
+        // 0.95 and 1.24 ms).
         const int64_t stop = min(cur_end, L.total_blocks);
-        const auto blocks = [&](auto ftz) {
-            constexpr bool FTZ = decltype(ftz)::value;
+        const auto blocks = [&](auto root) {
+            constexpr int ROOT = decltype(root)::value;
             for (; blk < stop; blk += warps) {
                 const int64_t b = blk - cur_first;
                 const int64_t base = b * FAST_VBLOCK;
                 const int64_t rem = numel - base;
                 // decode v = 2^((code-1)*scale/levels + min_log) as 2^(code*a + c)
                 const float sc = __ldg(v_scale + b), ml = __ldg(v_min_log + b);
-                const float a = sc * (VB == 16 ? 1.0f / 65534.0f : 1.0f / 254.0f);
-                const float c = ml - a;
+                [[maybe_unused]] const float a = sc * (VB == 16 ? 1.0f / 65534.0f : 1.0f / 254.0f);
+                [[maybe_unused]] const float c = ml - a;
                 float acc = 0.0f;
 
-                if (rem >= FAST_VBLOCK && small_w) {
+                // (a block that decodes to NaN, or into the subnormals, takes the forms that hold there)
+                const bool regular = !EXACT || (sc <= 3.402823466e38f && (VB == 8 || ml >= -125.0f));
+
+                if (rem >= FAST_VBLOCK && small_w && regular) {
                     if (TABLE) {
                         __syncwarp();                                   // the previous block's look-ups are done
 #pragma unroll
                         for (int k = 0; k < 8; ++k) {
                             const int code = lane + 32 * k;
-                            dec[code] = code ? ex2_approx<FTZ>(__fmaf_rn((float)code, a, c)) : 0.0f;
+                            if (EXACT) dec[code] = al8_decode_fast((uint32_t)code, sc, ml, s_exp2);
+                            else dec[code] = code ? ex2_approx<ROOT>(__fmaf_rn((float)code, a, c)) : 0.0f;
                         }
                         __syncwarp();
                     }
@@ -147,6 +186,7 @@ AF8_UNROLL_(AF8_STAT_UNROLL)
                             const uint4 w = __ldcs(reinterpret_cast<const uint4 *>(vq + off * 2));
                             vw[0] = w.x; vw[1] = w.y; vw[VB / 4 - 2] = w.z; vw[VB / 4 - 1] = w.w;
                         }
+                        float2 sum8 = make_float2(0.0f, 0.0f);
                         const float2 mc2 = bc2(MF == AF8_M_NONE ? 0.0f : __ldg(m_scale + b * (FAST_VBLOCK / FAST_MBLOCK) + s) * M_UNIT);
 #pragma unroll
                         for (int j = 0; j < 8; j += 2) {
@@ -158,10 +198,7 @@ AF8_UNROLL_(AF8_STAT_UNROLL)
                                 v_old = make_float2(dec[TABLE ? __byte_perm(vw[j >> 2], 0u, 0x4440u | (uint32_t)(j & 3)) : 0u],
                                                     dec[TABLE ? __byte_perm(vw[j >> 2], 0u, 0x4440u | (uint32_t)((j + 1) & 3)) : 0u]);
                             } else {
-                                const uint32_t w = vw[(j >> 1) & (VB / 4 - 1)];
-                                const float2 cd = __fadd2_rn(make_float2(__uint_as_float(0x4b000000u | (w & 0xffffu)), __uint_as_float(0x4b000000u | (w >> 16))), bc2(-8388608.0f));
-                                const float2 tt = __ffma2_rn(cd, bc2(a), bc2(c));
-                                v_old = make_float2((w & 0xffffu) ? ex2_approx<FTZ>(tt.x) : 0.0f, (w >> 16) ? ex2_approx<FTZ>(tt.y) : 0.0f);
+                                v_old = al16_decode2_stat(vw[(j >> 1) & (VB / 4 - 1)], sc, ml);
                             }
                             const float2 vj = __ffma2_rn(wv2, sub2(g2, v_old), v_old);
                             float2 mj = gj;
@@ -176,14 +213,15 @@ AF8_UNROLL_(AF8_STAT_UNROLL)
                                 const float2 m_old = __fmul2_rn(__fadd2_rn(mb, bc2(-8388616.0f)), mc2);
                                 mj = __ffma2_rn(wm2, sub2(gj, m_old), m_old);
                             }
-                            const float2 den = __fadd2_rn(make_float2(sqrt_approx<FTZ>(vj.x), sqrt_approx<FTZ>(vj.y)), ed2);
-                            const float2 u = __fmul2_rn(mj, make_float2(rcp_approx<FTZ>(den.x), rcp_approx<FTZ>(den.y)));
-                            acc2 = __ffma2_rn(u, u, acc2);
+                            const float2 u = root_update2<MF, ROOT>(mj, vj, ed2);
+                            if (EXACT) sum8 = __ffma2_rn(u, u, sum8);
+                            else acc2 = __ffma2_rn(u, u, acc2);
                         }
+                        if (EXACT) acc2 = __fadd2_rn(acc2, sum8);
                     }
                     acc = __fadd_rn(acc2.x, acc2.y);
                 } else {
-                    // tail block of a tensor, or EMA weights >= 0.5: element-wise with guards
+                    // tail block of a tensor, EMA weights >= 0.5, or an irregular block: element-wise with guards
                     for (int64_t i = lane; i < FAST_VBLOCK; i += 32) {
                         if (i >= rem) break;
                         const int64_t e = base + i;
@@ -191,14 +229,14 @@ AF8_UNROLL_(AF8_STAT_UNROLL)
                         if (L.negate_grad) gj = -gj;
                         const float g2 = __fadd_rn(__fmul_rn(gj, gj), eps_g);
                         const uint32_t code = VB == 16 ? reinterpret_cast<const uint16_t *>(vq)[e] : vq[e];
-                        const float v_old = code ? ex2_approx<FTZ>(__fmaf_rn((float)code, a, c)) : 0.0f;
+                        const float v_old = EXACT ? al_decode(code, sc, ml, VB == 16 ? 65534.0f : 254.0f) : code ? ex2_approx<ROOT>(__fmaf_rn((float)code, a, c)) : 0.0f;
                         const float vj = lerp_t(v_old, g2, v_w);
                         float mj = gj;
                         if (MF != AF8_M_NONE) {
                             const int k = MF == AF8_M_UF8 ? (int)mq[e] - 128 : (int)((e & 1) ? (mq[e >> 1] & 15u) : (mq[e >> 1] >> 4)) - 8;
                             mj = lerp_t(__fmul_rn((float)k, __ldg(m_scale + e / FAST_MBLOCK) * M_UNIT), gj, m_w);
                         }
-                        const float u = __fmul_rn(mj, rcp_approx<FTZ>(__fadd_rn(sqrt_approx<FTZ>(vj), eps_d)));
+                        const float u = root_update2<MF, EXACT ? ROOT_EXACT : ROOT>(make_float2(mj, 0.0f), make_float2(vj, 0.0f), bc2(eps_d)).x;
                         acc = __fmaf_rn(u, u, acc);
                     }
                 }
@@ -206,8 +244,8 @@ AF8_UNROLL_(AF8_STAT_UNROLL)
                 if (lane == 0) L.block_sumsq[blk] = acc;
             }
         };
-        if (eps_d >= EPS_HIDES) blocks(std::true_type());
-        else blocks(std::false_type());
+        if (eps_d >= EPS_HIDES) blocks(std::integral_constant<int, EXACT ? ROOT_REFINED : ROOT_FTZ>());
+        else blocks(std::integral_constant<int, EXACT ? ROOT_EXACT : ROOT_FULL>());
     }
 }
 

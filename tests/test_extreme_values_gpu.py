@@ -43,3 +43,67 @@ def test_subnormal_second_moments(m, v, limiter, oracle):
             if limiter:
                 a, b = float(opt.state[p]["fira_prev_norm"].item()), float(run.states[i]["fira_prev_norm"])
                 assert abs(a - b) <= 2e-6 * abs(b), f"{m}/{v} t{t} p{i}: norm {a} against {b}"
+
+KEYS = ("variance_q", "variance_scale", "variance_min_log", "m_q", "m_scale", "fira_prev_norm")
+
+
+def bits(x):
+    """The bytes of a tensor, every NaN as the same one."""
+    a = x.detach().cpu().contiguous()
+    if a.is_floating_point():
+        a = torch.where(torch.isnan(a), torch.full_like(a, float("nan")), a)
+        a = a.view(torch.int32 if a.element_size() == 4 else torch.int16)
+    return a
+
+
+def two_kernels(hp, shapes, steps, edit, seed=71):
+    """Steps the same tensors twice, with gradients in binary32 (specialised kernels) and in fp16 (general kernel); edit(t, i, g)
+    changes the fp16 gradient of tensor i in place.  -> ((parameters, optimizer), (parameters, optimizer))"""
+    from adafactor8bit import Adafactor8Bit
+    gen = torch.Generator().manual_seed(seed)
+    start = [torch.randn(s, generator=gen) * 0.02 for s in shapes]
+    grads = []
+    for t in range(1, steps + 1):
+        row = [(torch.randn(s, generator=gen) * 1e-2).half() for s in shapes]
+        for i, g in enumerate(row):
+            edit(t, i, g)
+        grads.append(row)
+    out = []
+    for dtype in (torch.float32, torch.float16):
+        params = [torch.nn.Parameter(x.clone().cuda()) for x in start]
+        for p in params:
+            p.grad_dtype = None
+        opt = Adafactor8Bit(params, **hp)
+        for row in grads:
+            for p, g in zip(params, row):
+                p.grad = g.cuda().to(dtype)
+            opt.step()
+        torch.cuda.synchronize()
+        out.append((params, opt))
+    return out
+
+
+def assert_same_state(a, b, what):
+    (pa, oa), (pb, ob) = a, b
+    for i, (x, y) in enumerate(zip(pa, pb)):
+        for key in KEYS:
+            if key in ob.state[y]:
+                s, r = bits(oa.state[x][key]), bits(ob.state[y][key])
+                assert torch.equal(s, r), f"{what} p{i} {key}: {int((s != r).sum())} of {r.numel()} differ"
+
+
+@pytest.mark.parametrize("limiter", [False, True])
+@pytest.mark.parametrize("m,v", [f for f in FORMATS if f != ("uf8", "al8")])
+def test_updates_are_the_general_kernels(m, v, limiter):
+    """AL16, UF4 and momentum-free states: parameters and states bit for bit as the general kernel gives them.  With the limiter a
+    tensor is one block with one gradient that is not zero, so that its norm is one element's update, whatever the order of the sum."""
+    def edit(t, i, g):
+        if limiter:
+            keep = g[7 + i].clone()
+            g.zero_()
+            g[7 + i] = keep
+    shapes = [(2048,)] * 6 if limiter else [(1 << 22,), (5 * 2048 + 300,), (2049,), (300,)]
+    fast, general = two_kernels(options(m, v, eps=(1e-8, 1e-3), enable_fira_for_adafactor=limiter), shapes, 3, edit)
+    assert_same_state(fast, general, f"{m}/{v}")
+    for i, (x, y) in enumerate(zip(fast[0], general[0])):
+        assert torch.equal(bits(x), bits(y)), f"{m}/{v} p{i}: {int((x != y).sum())} of {x.numel()} parameters differ"
