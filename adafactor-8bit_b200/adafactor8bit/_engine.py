@@ -322,7 +322,9 @@ class FullrankPlan:
             table[k] = scalars[k]
         table["sr_base"] = scalars.get("sr_base", 0)
         if self.cfg.use_adam_denom:
-            self.cfg.use_adam_denom = N.ADAM_DENOM_EPS_HIDES if np.min(scalars["eps_denom"]) >= N.EPS_HIDES else 1
+            eps = scalars["eps_denom"]
+            eps = float(eps.min()) if isinstance(eps, np.ndarray) else float(eps)
+            self.cfg.use_adam_denom = N.ADAM_DENOM_EPS_HIDES if eps >= N.EPS_HIDES else 1
         return buf, table
 
     # -- launches ------------------------------------------------------------
