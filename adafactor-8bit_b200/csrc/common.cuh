@@ -250,8 +250,9 @@ __device__ __forceinline__ float exp2_cr_fast(float x, const double *tab = c_exp
 __device__ __forceinline__ float rsqrt_t(float x) { return __frcp_rn(__fsqrt_rn(x)); }
 
 // log2 of a second-moment value as _log_quantize_nonneg sees it
-// (optimizer.py:308-310): values below 1e-38 (zero included) are lifted to 1e-38.
+// (optimizer.py:308-310): values below 1e-38 (zero included) are lifted to 1e-38, and NaNs with them.
 __device__ __forceinline__ float al_log2(float v) { return (v > AF8_TINY) ? log2_cr(v) : AF8_LOG2_TINY; }
+// (an infinity gives 1024)
 __device__ __forceinline__ float al_log2_fast(float v, const double2 *tab = c_log2_tab) { return (v > AF8_TINY) ? log2_cr_fast(v, tab) : AF8_LOG2_TINY; }
 
 // AL dequantisation of one code (optimizer.py:341-349).  qm1 = levels - 2.
@@ -267,7 +268,10 @@ __device__ __forceinline__ float al_decode(uint32_t code, float scale, float min
 // AL8 dequantisation with the short sequences: x / 254 from the correctly rounded
 // reciprocal and one residual step (equal to the IEEE quotient for every x >= 1e-13,
 // checked exhaustively on the host; (code-1)*scale is 0 or at least 1e-12), then
-// exp2_cr_fast.  min_log >= -127.3 and the block maximum is below 128, so |t| <= 150.
+// exp2_cr_fast.  min_log >= -127.3 and the block maximum is at most 128, so |t| <= 150, but for blocks that held
+// infinities: their range is infinite, and so is what they decode to, or NaN.  STRICT: an exponent of infinity gives
+// infinity (NaN else).
+template <bool STRICT>
 __device__ __forceinline__ float al8_decode_fast(uint32_t code, float scale, float min_log, const double *tab = c_exp2_tab)
 {
     if (code == 0) return 0.0f;
@@ -275,7 +279,8 @@ __device__ __forceinline__ float al8_decode_fast(uint32_t code, float scale, flo
     const float rc = 0x1.020408p-8f;                        // fl(1 / 254)
     const float q0 = __fmul_rn(x, rc);
     const float q = __fmaf_rn(__fmaf_rn(-q0, 254.0f, x), rc, q0);
-    return exp2_cr_fast(__fadd_rn(q, min_log), tab);
+    const float t = __fadd_rn(q, min_log);
+    return STRICT && t > 150.0f ? t : exp2_cr_fast(t, tab);
 }
 
 // Block range of _log_quantize_nonneg from the reduced extrema

@@ -369,7 +369,10 @@ __device__ __forceinline__ float2 div2_by(float2 x, float2 rc, float2 nd)
     return __ffma2_rn(__ffma2_rn(q, nd, x), rc, q);
 }
 
-// AL16 decode of two codes (optimizer.py:341-349); every lane of the warp takes part
+// false: the block held an infinite second moment
+__device__ __forceinline__ bool range_finite(float scale, float min_log) { return scale <= 3.402823466e38f && min_log <= 3.402823466e38f; }
+
+// AL16 decode of two codes (optimizer.py:341-349) of a block with a finite range; every lane of the warp takes part
 __device__ __forceinline__ float2 al16_decode2(uint32_t pair, float scale, float min_log, const LaneTables &T)
 {
     const uint32_t c0 = pair & 0xffffu, c1 = pair >> 16;
@@ -520,7 +523,8 @@ __device__ __forceinline__ void put(T (&x)[N], int j, T value)
 }
 
 // the inputs of a thread's eight elements of one momentum block (groups at oa and oa + 128) from a ring slot
-template <typename GradT, typename ParamT, int VB, int MF>
+// REGULAR: the block's range is finite
+template <typename GradT, typename ParamT, int VB, int MF, bool REGULAR>
 __device__ __forceinline__ void fast_load8(const unsigned char *st, int oa, const float *tab, float v_scale, float v_min_log, float m_scale,
                                            const LaneTables &LT, float2 (&p)[4], float2 (&g)[4], float2 (&v_old)[4], float2 (&m_old)[4])
 {
@@ -553,6 +557,12 @@ __device__ __forceinline__ void fast_load8(const unsigned char *st, int oa, cons
             const uint2 w = *reinterpret_cast<const uint2 *>(st + Ring::VQ_OFF + o * 2);
             v_old[2 * h] = al16_decode2(w.x, v_scale, v_min_log, LT);
             v_old[2 * h + 1] = al16_decode2(w.y, v_scale, v_min_log, LT);
+            if (!REGULAR && !range_finite(v_scale, v_min_log)) {     // code 0 is zero, the others infinity or NaN
+                const float x1 = al_decode(1u, v_scale, v_min_log, 65534.0f), x2 = al_decode(2u, v_scale, v_min_log, 65534.0f);
+                const auto value = [=](uint32_t c) { return c == 0u ? 0.0f : c == 1u ? x1 : x2; };
+                v_old[2 * h] = make_float2(value(w.x & 0xffffu), value(w.x >> 16));
+                v_old[2 * h + 1] = make_float2(value(w.y & 0xffffu), value(w.y >> 16));
+            }
         }
         if (MF == AF8_M_UF8) {
             // (byte - 128) * fl(scale / 128) (optimizer.py:528-531): a power-of-two divisor, and
@@ -578,17 +588,20 @@ __device__ __forceinline__ void fast_load8(const unsigned char *st, int oa, cons
 }
 
 // Requantisation of one momentum block: 32 lanes of eight elements, groups at e and e + 128
-// (optimizer.py:510, 518).  Writes the codes and the scale when `live`.
-template <int MF>
+// (optimizer.py:510, 518).  Writes the codes and the scale when `live`.  STRICT: infinities and NaNs as in the general
+// kernel, which leaves NaNs out of the largest magnitude and gives both the code of zero.
+template <int MF, bool STRICT>
 __device__ __forceinline__ void fast_store_m(const float2 (&m)[4], uint8_t *m_q, float *m_scale, int64_t e, bool live, int lane)
 {
+    const auto top3 = [](float a, float b, float c) { return STRICT ? max3_nan(a, b, c) : max3(a, b, c); };
     float amx = fabsf(m[0].x);
-    amx = max3(amx, fabsf(m[0].y), fabsf(m[1].x));
-    amx = max3(amx, fabsf(m[1].y), fabsf(m[2].x));
-    amx = max3(amx, fabsf(m[2].y), fabsf(m[3].x));
-    amx = fmaxf(amx, fabsf(m[3].y));
+    amx = top3(amx, fabsf(m[0].y), fabsf(m[1].x));
+    amx = top3(amx, fabsf(m[1].y), fabsf(m[2].x));
+    amx = top3(amx, fabsf(m[2].y), fabsf(m[3].x));
+    amx = top3(amx, fabsf(m[3].y), 0.0f);
     // non-negative floats order like their bit patterns: one REDUX instead of a shuffle tree
-    const float am = fmaxf(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amx))), 1e-12f);
+    const uint32_t abits = __reduce_max_sync(0xffffffffu, __float_as_uint(amx));
+    float am = fmaxf(__uint_as_float(abits), 1e-12f);
     const float2 ra2 = bc2(__frcp_rn(am)), nam2 = bc2(-am);
     // round(m / am * levels) (the product with the power of two is exact); |m / am| <= 1, so only
     // +levels needs the clamp to levels - 1
@@ -600,6 +613,15 @@ __device__ __forceinline__ void fast_store_m(const float2 (&m)[4], uint8_t *m_q,
         const float2 kf = __ffma2_rn(div2_by(m[j], ra2, nam2), bc2(LEVELS), bc2(AF8_MAGIC_F));
         raw[2 * j] = (uint32_t)min(__float_as_int(kf.x), AF8_MAGIC_I + TOP);
         raw[2 * j + 1] = (uint32_t)min(__float_as_int(kf.y), AF8_MAGIC_I + TOP);
+    }
+    if (STRICT && abits >= 0x7f800000u) {      // an infinity or a NaN in the block
+        float x[8];
+        amx = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) { x[j] = j & 1 ? m[j >> 1].y : m[j >> 1].x; amx = fmaxf(amx, fabsf(x[j])); }
+        am = fmaxf(warp_max(amx), 1e-12f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) raw[j] = (uint32_t)AF8_MAGIC_I + (MF == AF8_M_UF4 ? uf4_encode(x[j], am) - 8u : uf8_encode(x[j], am) - 128u);
     }
     if (!live) return;
     if (MF == AF8_M_UF8) {
@@ -661,6 +683,9 @@ fullrank_fast_kernel(const FullrankLaunch L)
     constexpr int QMAX = VB == 16 ? 65535 : 255;
     constexpr float QM1 = VB == 16 ? 65534.0f : 254.0f;
     constexpr bool TABLE = VB == 8;
+    // Infinities and NaNs in whole blocks as in the general kernel.  Not with UF8/AL8, where their tests cost 8 % of the
+    // update pass: there a NaN is left out of the range and of the largest magnitude.
+    constexpr bool STRICT = root_exact<VB, MF>;
 
     extern __shared__ __align__(128) unsigned char s_ring[];     // NST slots of STAGE_BYTES
     __shared__ __align__(8) uint64_t s_full[NST];
@@ -780,8 +805,8 @@ fullrank_fast_kernel(const FullrankLaunch L)
                     cms[k] = (2 * warp + k) * FAST_MBLOCK < rem ? __ldg(sT.m_scale + (int64_t)b * MPB + 2 * warp + k) : 0.0f;
             }
             if (TABLE) {
-                s_tab[stage][tid] = al8_decode_fast((uint32_t)tid, csc, cml, s_exp2);   // optimizer.py:341-349
-                s_tab[stage][tid + 128] = al8_decode_fast((uint32_t)tid + 128u, csc, cml, s_exp2);
+                s_tab[stage][tid] = al8_decode_fast<STRICT>((uint32_t)tid, csc, cml, s_exp2);   // optimizer.py:341-349
+                s_tab[stage][tid + 128] = al8_decode_fast<STRICT>((uint32_t)tid + 128u, csc, cml, s_exp2);
             }
             __syncthreads();
         }
@@ -824,8 +849,8 @@ fullrank_fast_kernel(const FullrankLaunch L)
         }
 
         const StepScalars S = sS;
-        // (uniform over the CTA; a block that decodes to NaN takes the general forms: ROOT_REFINED would lose the NaN)
-        const bool hot = full && S.plain && (ROOT != ROOT_REFINED || csc <= 3.402823466e38f);
+        // (uniform over the CTA; a block that decodes to infinities or NaNs takes the general forms: ROOT_REFINED would lose a NaN)
+        const bool hot = full && S.plain && (!root_exact<VB, MF> || range_finite(csc, cml));
         float v[FAST_EPT];                   // hot blocks: the new second moments
         float usq = 0.0f;                    // LAG: this thread's sum of squares of the raw update
         // Extrema of v.  v >= 0, so the bit patterns order like the values.  The minimum runs over the
@@ -838,7 +863,7 @@ fullrank_fast_kernel(const FullrankLaunch L)
             for (int mb = 0; mb < 2; ++mb) {
                 const int oa = ow + mb * FAST_MBLOCK;
                 float2 g[4], p[4], v_old[4], m_old[4], vn[4], mn[4];
-                fast_load8<GradT, ParamT, VB, MF>(st, oa, s_tab[stage], csc, cml, cms[mb], LT, p, g, v_old, m_old);
+                fast_load8<GradT, ParamT, VB, MF, true>(st, oa, s_tab[stage], csc, cml, cms[mb], LT, p, g, v_old, m_old);
                 if (L.negate_grad) {                              // maximize (optimizer.py:1973-1974)
 #pragma unroll
                     for (int j = 0; j < 4; ++j) g[j] = make_float2(-g[j].x, -g[j].y);
@@ -866,23 +891,28 @@ fullrank_fast_kernel(const FullrankLaunch L)
                     }
                 }
                 if (MF != AF8_M_NONE)
-                    fast_store_m<MF>(mn, sT.m_q, sT.m_scale + (int64_t)b * MPB + 2 * warp + mb, base + oa, !bad, lane);
+                    fast_store_m<MF, STRICT>(mn, sT.m_q, sT.m_scale + (int64_t)b * MPB + 2 * warp + mb, base + oa, !bad, lane);
             }
-            float fmn = v[0], fmx = v[0];
+            float fmn = v[0], fmx = v[0];        // (STRICT: a NaN reaches fmx, else neither)
 #pragma unroll
             for (int j = 1; j + 1 < FAST_EPT; j += 2) {
                 fmn = min3(fmn, v[j], v[j + 1]);
-                fmx = max3(fmx, v[j], v[j + 1]);
+                fmx = STRICT ? max3_nan(fmx, v[j], v[j + 1]) : max3(fmx, v[j], v[j + 1]);
             }
             fmn = fminf(fmn, v[FAST_EPT - 1]);
-            fmx = fmaxf(fmx, v[FAST_EPT - 1]);
+            fmx = STRICT ? max3_nan(fmx, v[FAST_EPT - 1], v[FAST_EPT - 1]) : fmaxf(fmx, v[FAST_EPT - 1]);
             umin = __reduce_min_sync(0xffffffffu, __float_as_uint(fmn));
             umax = __reduce_max_sync(0xffffffffu, __float_as_uint(fmx));
-            if (umin == 0u) {            // the warp holds a zero (rare after the first steps, except in all-zero regions)
-                uint32_t um = 0xffffffffu;
+            if (umin == 0u || (STRICT && umax > 0x7f800000u)) {      // the warp holds a zero (rare after the first steps, except in all-zero regions) or a NaN
+                uint32_t um = 0xffffffffu, ux = 0u;
 #pragma unroll
-                for (int j = 0; j < FAST_EPT; ++j) um = min(um, __float_as_uint(v[j]) - 1u);
+                for (int j = 0; j < FAST_EPT; ++j) {
+                    if (STRICT && !(v[j] >= 0.0f)) v[j] = AF8_TINY;      // (see al_log2)
+                    um = min(um, __float_as_uint(v[j]) - 1u);
+                    if (STRICT) ux = max(ux, __float_as_uint(v[j]));
+                }
                 umin = __reduce_min_sync(0xffffffffu, um);
+                if (STRICT) umax = __reduce_max_sync(0xffffffffu, ux);
             } else {
                 umin -= 1u;
             }
@@ -895,7 +925,7 @@ fullrank_fast_kernel(const FullrankLaunch L)
             for (int mb = 0; mb < 2; ++mb) {
                 const int oa = ow + mb * FAST_MBLOCK;
                 float2 g[4], p[4], v_old[4], m_old[4], vn[4], mn[4];
-                fast_load8<GradT, ParamT, VB, MF>(st, oa, s_tab[stage], csc, cml, mb ? cms[1] : cms[0], LT, p, g, v_old, m_old);
+                fast_load8<GradT, ParamT, VB, MF, false>(st, oa, s_tab[stage], csc, cml, mb ? cms[1] : cms[0], LT, p, g, v_old, m_old);
                 if (L.negate_grad) {
 #pragma unroll
                     for (int j = 0; j < 4; ++j) g[j] = make_float2(-g[j].x, -g[j].y);
@@ -912,6 +942,8 @@ fullrank_fast_kernel(const FullrankLaunch L)
                 for (int j = 0; j < 4; ++j) {                     // padding re-enters both states as zero
                     if (!((real >> (2 * j)) & 1u)) { vn[j].x = 0.0f; mn[j].x = 0.0f; }
                     if (!((real >> (2 * j + 1)) & 1u)) { vn[j].y = 0.0f; mn[j].y = 0.0f; }
+                    if (!(vn[j].x >= 0.0f)) vn[j].x = STRICT ? AF8_TINY : 0.0f;      // NaN (see al_log2)
+                    if (!(vn[j].y >= 0.0f)) vn[j].y = STRICT ? AF8_TINY : 0.0f;
                     x[2 * j] = vn[j].x; x[2 * j + 1] = vn[j].y;
                     q[2 * j] = p[j].x; q[2 * j + 1] = p[j].y;
                 }
@@ -930,7 +962,7 @@ fullrank_fast_kernel(const FullrankLaunch L)
                     }
                 }
                 if (MF != AF8_M_NONE)
-                    fast_store_m<MF>(mn, sT.m_q, sT.m_scale + (int64_t)b * MPB + 2 * warp + mb, base + oa,
+                    fast_store_m<MF, STRICT>(mn, sT.m_q, sT.m_scale + (int64_t)b * MPB + 2 * warp + mb, base + oa,
                                      (2 * warp + mb) * FAST_MBLOCK < rem && !bad, lane);
                 // (this thread's own inputs: 16 bytes of fp32 parameters, or 8 of bf16 parameters and 8 of gradients, per group)
 #pragma unroll
@@ -967,8 +999,8 @@ fullrank_fast_kernel(const FullrankLaunch L)
                                    : ((lane == 1) ? al_log2_fast(__uint_as_float(umax), s_log2) : 0.0f);
             const float mx_l = __shfl_sync(0xffffffffu, lg, 1);
             if (lane == 0) {
-                const float mn = lg;
-                const float mx = mx_l;
+                const float mn = lg == 1024.0f ? INFINITY : lg;      // (infinite second moments)
+                const float mx = mx_l == 1024.0f ? INFINITY : mx_l;
                 VRange r;
                 al_range(mn, mx, L.v_floor, r.min_log, r.scale);
                 if (VB == 8) {
@@ -985,7 +1017,7 @@ fullrank_fast_kernel(const FullrankLaunch L)
                     if (!(r.k >= 1.0f) || L.v_floor < -126.0f || mn < L.v_floor) r.thr = -1.0f;
                 } else {
                     r.k = __frcp_rn(r.scale);                    // for the quotient by the scale
-                    r.c = 0.0f; r.thr = 0.0f;
+                    r.c = 0.0f; r.thr = range_finite(r.scale, r.min_log) ? 0.0f : -1.0f;     // (negative: exact path)
                 }
                 s_vr = r;
                 sT.v_scale[b] = r.scale;
@@ -1001,8 +1033,8 @@ fullrank_fast_kernel(const FullrankLaunch L)
 
         // ---- what does not need the range: the next block's decode table, or (AL16) this block's log2 ----
         if (TABLE && next_staged) {
-            s_tab[stage ^ 1][tid] = al8_decode_fast((uint32_t)tid, nsc, nml, s_exp2);
-            s_tab[stage ^ 1][tid + 128] = al8_decode_fast((uint32_t)tid + 128u, nsc, nml, s_exp2);
+            s_tab[stage ^ 1][tid] = al8_decode_fast<STRICT>((uint32_t)tid, nsc, nml, s_exp2);
+            s_tab[stage ^ 1][tid + 128] = al8_decode_fast<STRICT>((uint32_t)tid + 128u, nsc, nml, s_exp2);
         }
         float lv[TABLE ? 1 : FAST_EPT];
         if (!TABLE && hot) {
@@ -1080,6 +1112,12 @@ fullrank_fast_kernel(const FullrankLaunch L)
                 }
                 *reinterpret_cast<uint32_t *>(vp + ow + mb * FAST_MBLOCK) = pack4(kk[0], kk[1], kk[2], kk[3]);       // (not reached after a failed wait: the CTA left at E)
                 *reinterpret_cast<uint32_t *>(vp + ow + mb * FAST_MBLOCK + 128) = pack4(kk[4], kk[5], kk[6], kk[7]);
+            }
+        } else if (r.thr < 0.0f) {
+#pragma unroll 1
+            for (int q = 0; q < FAST_EPT; ++q) {
+                const float x = pick(v, q);
+                static_cast<uint16_t *>(sT.v_q)[base + ow + (q >> 2) * 128 + (q & 3)] = (uint16_t)al_encode(x, al_log2_fast(x, s_log2), r.min_log, r.scale, QM1, QMAX);
             }
         } else {
             uint16_t *const vp = static_cast<uint16_t *>(sT.v_q) + base;

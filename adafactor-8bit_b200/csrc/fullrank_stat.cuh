@@ -159,7 +159,7 @@ fullrank_stat_kernel(const FullrankLaunch L)
 #pragma unroll
                         for (int k = 0; k < 8; ++k) {
                             const int code = lane + 32 * k;
-                            if (EXACT) dec[code] = al8_decode_fast((uint32_t)code, sc, ml, s_exp2);
+                            if (EXACT) dec[code] = al8_decode_fast<true>((uint32_t)code, sc, ml, s_exp2);
                             else dec[code] = code ? ex2_approx<ROOT>(__fmaf_rn((float)code, a, c)) : 0.0f;
                         }
                         __syncwarp();
