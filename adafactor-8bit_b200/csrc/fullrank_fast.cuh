@@ -1130,12 +1130,14 @@ fullrank_fast_kernel(const FullrankLaunch L)
                     // al_encode on a pair: (l - min_log) / scale * 65534, rounded, plus one (optimizer.py:320-321)
                     const int i = TABLE ? 0 : 4 * q + j;
                     const float2 d = __fadd2_rn(make_float2(lv[i], lv[TABLE ? 0 : i + 1]), nml2);
-                    const float2 t = div2_by(d, rc2, nd2);
+                    const float2 q2 = div2_by(d, rc2, nd2);
+                    // (below min_log: code 1, which the rounding constant would not give for a quotient of -2^6 and less)
+                    const float2 t = make_float2(fmaxf(q2.x, 0.0f), fmaxf(q2.y, 0.0f));
                     // (scalar: the compiler fuses a packed product into a packed sum, which loses the rounding in between)
                     const int k0 = __float_as_int(__fadd_rn(__fmul_rn(t.x, QM1), AF8_MAGIC_F)) - (AF8_MAGIC_I - 1);
                     const int k1 = __float_as_int(__fadd_rn(__fmul_rn(t.y, QM1), AF8_MAGIC_F)) - (AF8_MAGIC_I - 1);
-                    kk[j] = v[4 * q + j] == 0.0f ? 0u : (uint32_t)max(1, min(k0, QMAX));
-                    kk[j + 1] = v[4 * q + j + 1] == 0.0f ? 0u : (uint32_t)max(1, min(k1, QMAX));
+                    kk[j] = v[4 * q + j] == 0.0f ? 0u : (uint32_t)min(k0, QMAX);
+                    kk[j + 1] = v[4 * q + j + 1] == 0.0f ? 0u : (uint32_t)min(k1, QMAX);
                 }
                 *reinterpret_cast<uint2 *>(vp + ow + q * 128) = make_uint2(kk[0] | (kk[1] << 16), kk[2] | (kk[3] << 16));
             }

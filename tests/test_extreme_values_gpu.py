@@ -172,3 +172,22 @@ def test_nan_in_a_tail_leaves_the_range(oracle):
     for p, st in zip(params, run.states):
         for key in ("variance_scale", "variance_min_log"):
             assert np.array_equal(opt.state[p][key].cpu().numpy(), st[key]), key
+
+
+@pytest.mark.parametrize("m", ["uf8", "uf4", None])
+def test_al16_codes_far_below_the_floor(m, oracle):
+    """A block whose maximum lies just above the floor of 2^-126 and whose other values lie below it: hundreds of ranges below
+    min_log, where the rounding constant no longer covers the quotient; their code is 1."""
+    hp = options(m, "al16", eps=(1e-8, 1e-3))
+    case = dict(shapes=[(2048,)], steps=1, seed=83, hp=hp, grad=dict(dist="normal", std=1e-3, zero_frac=0.0, dtype="f32"))
+    run = OracleRun("below the floor", case=case)
+    v = np.full(2048, 5e-39)
+    v[::64] = 2.0 ** np.linspace(-126.2, -125.999, 32)
+    run.grads[1][0][:] = np.sqrt(v / 0.001).astype(np.float32)
+    params, opt = make_optimizer(run)
+    params[0].grad = to_cuda_grad(run.grads[1][0], params[0].shape)
+    opt.step()
+    run.step()
+    scale = float(run.states[0]["variance_scale"][0])
+    assert 6e-4 < scale < 1.3e-3
+    assert np.array_equal(opt.state[params[0]]["variance_q"].cpu().numpy().view(np.uint16), run.states[0]["variance_q"])
