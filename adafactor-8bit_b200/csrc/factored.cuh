@@ -218,6 +218,42 @@ __device__ __forceinline__ uint32_t uf8_encode_fast2(float2 m, const DivBy &A)
     return (uint32_t)(k0 - 0x4b400000 + 128) | ((uint32_t)(k1 - 0x4b400000 + 128) << 8);
 }
 
+// Largest magnitude of a momentum block of 256, 8 elements a lane: at least 1e-12, NaNs left out.  odd: the block holds an
+// infinity or a NaN.  (The bit patterns of non-negative floats are ordered: one REDUX instead of a shuffle tree.)
+__device__ __forceinline__ float m_absmax256(const float (&m)[8], bool &odd)
+{
+    float top = max3_nan(fabsf(m[0]), fabsf(m[1]), fabsf(m[2]));
+    top = max3_nan(top, fabsf(m[3]), fabsf(m[4]));
+    top = max3_nan(top, fabsf(m[5]), fabsf(m[6]));
+    top = max3_nan(top, fabsf(m[7]), fabsf(m[7]));
+    const uint32_t bits = __reduce_max_sync(0xffffffffu, __float_as_uint(top));
+    odd = bits >= 0x7f800000u;
+    float am = __uint_as_float(bits);
+    if (odd) {
+        am = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) am = fmaxf(am, fabsf(m[j]));
+        am = warp_max(am);
+    }
+    return fmaxf(am, 1e-12f);
+}
+// its UF8 codes; with an infinity or a NaN by uf8_encode, which gives both the code of zero
+__device__ __forceinline__ uint2 uf8_codes8(const float (&m)[8], float am, bool odd)
+{
+    if (odd) {
+        uint2 o = make_uint2(0u, 0u);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            o.x |= uf8_encode(m[j], am) << (8 * j);
+            o.y |= uf8_encode(m[j + 4], am) << (8 * j);
+        }
+        return o;
+    }
+    const DivBy A = make_div(am);
+    return make_uint2(uf8_encode_fast2(make_float2(m[0], m[1]), A) | (uf8_encode_fast2(make_float2(m[2], m[3]), A) << 16),
+                      uf8_encode_fast2(make_float2(m[4], m[5]), A) | (uf8_encode_fast2(make_float2(m[6], m[7]), A) << 16));
+}
+
 // ---------------------------------------------------------------------------
 // statistics
 // ---------------------------------------------------------------------------
@@ -1671,16 +1707,12 @@ factored_update_vec_kernel(const FactoredLaunch L)
         if (m_quant) {
             // one warp = one momentum block of 256 (the block exists iff its first element does)
             const int64_t w0 = (id - sT.first_chunk) * 2048 + warp * 256;
-            float am = 0.0f;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) am = fmaxf(am, fabsf(mj[j]));
-            am = fmaxf(warp_max(am), 1e-12f);
+            bool odd;
+            const float am = m_absmax256(mj, odd);
             if (w0 < numel) {
                 if (L.m_fmt == AF8_M_UF8) {
-                    const DivBy A = make_div(am);
-                    const uint32_t o0 = uf8_encode_fast2(make_float2(mj[0], mj[1]), A) | (uf8_encode_fast2(make_float2(mj[2], mj[3]), A) << 16);
-                    const uint32_t o1 = uf8_encode_fast2(make_float2(mj[4], mj[5]), A) | (uf8_encode_fast2(make_float2(mj[6], mj[7]), A) << 16);
-                    if (ANY != 0 || ok) *reinterpret_cast<uint2 *>(sT.m_q + flat) = make_uint2(o0, o1);
+                    const uint2 codes = uf8_codes8(mj, am, odd);
+                    if (ANY != 0 || ok) *reinterpret_cast<uint2 *>(sT.m_q + flat) = codes;
                 } else if (L.m_fmt == AF8_M_D8) {
                     uint32_t o0 = 0, o1 = 0;
 #pragma unroll
@@ -1882,15 +1914,11 @@ factored_apply_ring_kernel(const FactoredLaunch L)
         }
         // one warp = one momentum block of 256 (the block exists iff its first element does)
         const int64_t w0 = (id - sT.first_chunk) * 2048 + warp * 256;
-        float am = 0.0f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) am = fmaxf(am, fabsf(mj[j]));
-        am = fmaxf(warp_max(am), 1e-12f);
+        bool odd;
+        const float am = m_absmax256(mj, odd);
         if (w0 < numel) {
-            const DivBy A = make_div(am);
-            const uint32_t o0 = uf8_encode_fast2(make_float2(mj[0], mj[1]), A) | (uf8_encode_fast2(make_float2(mj[2], mj[3]), A) << 16);
-            const uint32_t o1 = uf8_encode_fast2(make_float2(mj[4], mj[5]), A) | (uf8_encode_fast2(make_float2(mj[6], mj[7]), A) << 16);
-            if (ok) *reinterpret_cast<uint2 *>(sT.m_q + flat) = make_uint2(o0, o1);
+            const uint2 codes = uf8_codes8(mj, am, odd);
+            if (ok) *reinterpret_cast<uint2 *>(sT.m_q + flat) = codes;
             if (lane == 0) sT.m_scale[w0 / 256] = am;
         }
     }
@@ -2043,14 +2071,10 @@ factored_apply_tile_kernel(const FactoredLaunch L)
                 *reinterpret_cast<uint4 *>(static_cast<uint16_t *>(sT.param_copy) + flat) =
                     make_uint4(bf16x2_rn(p[0], p[1]), bf16x2_rn(p[2], p[3]), bf16x2_rn(p[4], p[5]), bf16x2_rn(p[6], p[7]));
             // the row slice is one momentum block of 256
-            float am = 0.0f;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) am = fmaxf(am, fabsf(mj[j]));
-            am = fmaxf(warp_max(am), 1e-12f);
-            const DivBy A = make_div(am);
-            const uint32_t o0 = uf8_encode_fast2(make_float2(mj[0], mj[1]), A) | (uf8_encode_fast2(make_float2(mj[2], mj[3]), A) << 16);
-            const uint32_t o1 = uf8_encode_fast2(make_float2(mj[4], mj[5]), A) | (uf8_encode_fast2(make_float2(mj[6], mj[7]), A) << 16);
-            *reinterpret_cast<uint2 *>(sT.m_q + flat) = make_uint2(o0, o1);
+            bool odd;
+            const float am = m_absmax256(mj, odd);
+            const uint2 codes = uf8_codes8(mj, am, odd);
+            *reinterpret_cast<uint2 *>(sT.m_q + flat) = codes;
             if (lane == 0) scp[k * scstep] = am;
         }
         cons += (uint32_t)nrows;

@@ -153,3 +153,30 @@ def test_factored_matches_reference_golden(name, oracle):
             if key in ref:
                 parity.assert_codes(state_np(opt.state[p], key), ref[key], f"{name} final p{i} {key} vs reference",
                                     al16=(ref[key].dtype == np.uint16), zero_reserved=(key != "m_q"))
+
+
+@pytest.mark.parametrize("came", [False, True])
+@pytest.mark.parametrize("shape", [(3, 40, 264), (3, 33, 131), (70, 1001), (3, 40, 256)])
+def test_infinities_and_nans_in_rows_of_any_length(shape, came, oracle):
+    """Batches and rows of any length with a UF8 momentum: momenta, ranges and parameters as the general kernels (fp16 gradients) leave them."""
+    from adafactor8bit import Adafactor8Bit
+    hp = dict(cases.CASES["came_al16" if came else "adafactor_factored_m"]["hp"], m_quant_type="uf8", m_block_size=256, min_8bit_size=1)
+    gen = torch.Generator().manual_seed(31)
+    start = torch.randn(shape, generator=gen) * 0.02
+    grads = [(torch.randn(shape, generator=gen) * 1e-2).half() for _ in range(3)]
+    flat = grads[1].view(-1)
+    flat[7], flat[-1], flat[400] = float("inf"), float("nan"), -float("inf")
+    out = []
+    for dtype in (torch.float32, torch.float16):
+        p = torch.nn.Parameter(start.clone().cuda())
+        p.grad_dtype = None
+        opt = Adafactor8Bit([p], **hp)
+        for g in grads:
+            p.grad = g.cuda().to(dtype)
+            opt.step()
+        torch.cuda.synchronize()
+        out.append((p.detach().cpu(), {k: v.cpu() for k, v in opt.state[p].items() if isinstance(v, torch.Tensor)}))
+    (p, st), (q, ref) = out
+    np.testing.assert_allclose(st["m_scale"].numpy(), ref["m_scale"].numpy(), rtol=1e-5, equal_nan=True)
+    parity.assert_codes(st["m_q"].numpy(), ref["m_q"].numpy(), f"{shape} m_q", zero_reserved=False)
+    np.testing.assert_allclose(p.numpy(), q.numpy(), rtol=1e-4, atol=1e-7, equal_nan=True)
