@@ -48,6 +48,12 @@ struct FactoredLaunch {
     int32_t split;               // tile kernels: a unit is the (1 << split)-th part of a tile (see tile_split)
 };
 
+// Whether a tensor's squares are added eight at a time in binary32 before they enter the binary64 sum: a matrix of whole
+// vectors is, in a table of such matrices and, so that its norm does not depend on its neighbours, in a table that it shares
+// with batches; batches of matrices, and tables with rows of any length, add each square in binary64.
+template <int ANY>
+__device__ __forceinline__ bool sums_by_eight(const af8_factored_tensor &T) { return ANY == 0 || (ANY == 1 && T.batch_rows == 0); }
+
 __device__ __forceinline__ int find_factored_tile(const af8_factored_tensor *t, int n, int64_t id)
 {
     int lo = 0, hi = n - 1;
@@ -1391,7 +1397,7 @@ factored_stats_vec_kernel(const FactoredLaunch L, const int use_ring, const CUte
 // 8 stay aligned; a vector crosses at most one row end, so its elements take one of two row factors, and column factors
 // from three aligned vectors that are shifted (one by one in a lane with a row end).  Only a tensor's last vector may be
 // partial.  The squares of the sum
-// passes enter binary64 one by one, as in factored_update_kernel, which such tensors took before.  Write pass with bf16
+// passes enter binary64 one by one, as in factored_update_kernel, which such tensors took before (but see sums_by_eight).  Write pass with bf16
 // gradients: 59 M parameters of odd sizes with a UF8 momentum 1 ms -> 252 us (issue and latency bound, 500 instructions
 // per 256 elements), 138 M in batches without momentum 1.55 ms -> 245 us (325 us with the tests of ANY = 2).
 template <typename GradT, int PASS, int CTAS, int ANY>
@@ -1629,7 +1635,7 @@ factored_update_vec_kernel(const FactoredLaunch L)
                 for (int j = 0; j < 8; ++j)
                     if (j >= nval) { u[j] = 0.0f; mj[j] = 0.0f; }
             }
-            if (SUMS && ANY != 0) {
+            if (SUMS && !sums_by_eight<ANY>(sT)) {
 #pragma unroll
                 for (int j = 0; j < 8; ++j) part += (double)__fmul_rn(u[j], u[j]);
             } else if (SUMS) {
@@ -2174,8 +2180,8 @@ factored_sumsq_wide_kernel(const FactoredLaunch L)
 // its 8 columns in registers while its warp walks the tile's rows (the flat kernel above re-reads them for
 // every element, twice the bytes of the gradient itself through L1), four rows' loads in flight.  A CTA adds
 // its tile's sum to the slot of the tensor's first chunk; the caller clears the slots first.
-// ANY: batches of matrices and rows of any length; the squares enter binary64 one by one (see factored_update_vec_kernel).
-template <typename GradT, bool ANY>
+// ANY = 1: batches of matrices, whole vectors; 2: rows of any length as well (see sums_by_eight).
+template <typename GradT, int ANY>
 __global__ void __launch_bounds__(256, ANY ? 3 : 4)
 factored_sumsq_tile_kernel(const FactoredLaunch L)
 {
@@ -2206,7 +2212,7 @@ factored_sumsq_tile_kernel(const FactoredLaunch L)
 #pragma unroll
         for (int j = 0; j < 8; ++j) ic[j] = 0.0f;
         double acc = 0.0;
-        if (ANY && (C & 7) != 0) {
+        if (ANY == 2 && (C & 7) != 0) {
             const int nc = (int)max((int64_t)0, min((int64_t)8, C - c));
             const int64_t numel = sT.rows * C;
             load_cols_any(sT.inv_col + P.cb, c, C, ic);
@@ -2233,35 +2239,39 @@ factored_sumsq_tile_kernel(const FactoredLaunch L)
             }
         } else {
         if (col_ok) load_f8_ro(sT.inv_col + P.cb + c, ic);
-        GradRaw8<GradT> cur[NB], nxt[NB];
-        auto fetch = [&](GradRaw8<GradT> (&dst)[NB], int k0) {
+        const auto sum_rows = [&](auto by_eight) {                 // (a copy of the loop for each: the choice inside cost a third)
+            GradRaw8<GradT> cur[NB], nxt[NB];
+            auto fetch = [&](GradRaw8<GradT> (&dst)[NB], int k0) {
 #pragma unroll
-            for (int k = 0; k < NB; ++k) {
-                const int64_t r = r0 + warp + 8 * (k0 + k);
-                if (col_ok && r < R) dst[k].load(sT.grad, r * C + c);
-                else dst[k].zero();
+                for (int k = 0; k < NB; ++k) {
+                    const int64_t r = r0 + warp + 8 * (k0 + k);
+                    if (col_ok && r < R) dst[k].load(sT.grad, r * C + c);
+                    else dst[k].zero();
+                }
+            };
+            fetch(cur, 0);
+            for (int k0 = 0; r0 + warp + 8 * k0 < R; k0 += NB) {   // (uniform over the warp)
+                fetch(nxt, k0 + NB);
+#pragma unroll
+                for (int k = 0; k < NB; ++k) {
+                    const int64_t r = min(r0 + warp + 8 * (int64_t)(k0 + k), R - 1);     // (a row beyond the end carries zeros)
+                    const float2 ir2 = bc2(__ldg(sT.inv_row + r));
+                    float g[8];
+                    cur[k].unpack(0, g);                           // (the sign does not matter for the square)
+                    float2 a2 = make_float2(0.0f, 0.0f);
+#pragma unroll
+                    for (int j = 0; j < 8; j += 2) {
+                        const float2 uj = __fmul2_rn(__fmul2_rn(make_float2(g[j], g[j + 1]), ir2), make_float2(ic[j], ic[j + 1]));
+                        if (!decltype(by_eight)::value) { const float2 q = __fmul2_rn(uj, uj); acc += (double)q.x; acc += (double)q.y; }
+                        else a2 = j == 0 ? __fmul2_rn(uj, uj) : __ffma2_rn(uj, uj, a2);
+                    }
+                    if (decltype(by_eight)::value) acc += (double)__fadd_rn(a2.x, a2.y);
+                    cur[k] = nxt[k];
+                }
             }
         };
-        fetch(cur, 0);
-        for (int k0 = 0; r0 + warp + 8 * k0 < R; k0 += NB) {       // (uniform over the warp)
-            fetch(nxt, k0 + NB);
-#pragma unroll
-            for (int k = 0; k < NB; ++k) {
-                const int64_t r = min(r0 + warp + 8 * (int64_t)(k0 + k), R - 1);     // (a row beyond the end carries zeros)
-                const float2 ir2 = bc2(__ldg(sT.inv_row + r));
-                float g[8];
-                cur[k].unpack(0, g);                               // (the sign does not matter for the square)
-                float2 a2 = make_float2(0.0f, 0.0f);
-#pragma unroll
-                for (int j = 0; j < 8; j += 2) {
-                    const float2 uj = __fmul2_rn(__fmul2_rn(make_float2(g[j], g[j + 1]), ir2), make_float2(ic[j], ic[j + 1]));
-                    if (ANY) { const float2 q = __fmul2_rn(uj, uj); acc += (double)q.x; acc += (double)q.y; }
-                    else a2 = j == 0 ? __fmul2_rn(uj, uj) : __ffma2_rn(uj, uj, a2);
-                }
-                if (!ANY) acc += (double)__fadd_rn(a2.x, a2.y);
-                cur[k] = nxt[k];
-            }
-        }
+        if (sums_by_eight<ANY>(sT)) sum_rows(std::true_type());
+        else if constexpr (ANY != 0) sum_rows(std::false_type());
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
@@ -2561,10 +2571,13 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
         LT.split = tile_split(total_tiles);
         LT.total_units = total_tiles << LT.split;
         const int64_t tg = std::min<int64_t>((int64_t)sm_count() * 8, LT.total_units);
-        if (bf && any) factored_sumsq_tile_kernel<bf16_tag, true><<<(int)tg, 256, 0, cst>>>(LT);
-        else if (any) factored_sumsq_tile_kernel<float, true><<<(int)tg, 256, 0, cst>>>(LT);
-        else if (bf) factored_sumsq_tile_kernel<bf16_tag, false><<<(int)tg, 256, 0, cst>>>(LT);
-        else factored_sumsq_tile_kernel<float, false><<<(int)tg, 256, 0, cst>>>(LT);
+        const int kind = !any ? 0 : cfg->cols_mult8 ? 1 : 2;
+#define AF8_LAUNCH_FSUM(G) do { if (kind == 0) factored_sumsq_tile_kernel<G, 0><<<(int)tg, 256, 0, cst>>>(LT); \
+        else if (kind == 1) factored_sumsq_tile_kernel<G, 1><<<(int)tg, 256, 0, cst>>>(LT); \
+        else factored_sumsq_tile_kernel<G, 2><<<(int)tg, 256, 0, cst>>>(LT); } while (0)
+        if (bf) AF8_LAUNCH_FSUM(bf16_tag);
+        else AF8_LAUNCH_FSUM(float);
+#undef AF8_LAUNCH_FSUM
         AF8_CUDA_TRY(cudaGetLastError());
         return AF8_OK;
     }

@@ -155,6 +155,34 @@ def test_factored_matches_reference_golden(name, oracle):
                                     al16=(ref[key].dtype == np.uint16), zero_reserved=(key != "m_q"))
 
 
+def test_a_matrix_beside_batches_is_the_same(oracle):
+    """Momentum-free matrices share the launch table of batches that hold most of the elements: their norms, and so their clip
+    divisors and parameters, are bit for bit those of a table of their own (the grouping differs between the ranks of a
+    sharded step, and with the parameters that have a gradient)."""
+    from adafactor8bit import Adafactor8Bit
+    hp = dict(cases.CASES["adafactor_factored"]["hp"], enable_fira_for_adafactor=True)
+    gen = torch.Generator().manual_seed(29)
+    flats = [(3 + 7 * i % 40, 8 * (1 + i % 5)) for i in range(60)] + [(64, 264), (530, 1024), (700, 520), (33, 640), (48, 4096)]
+    batch = (6, 600, 512)
+    start = [torch.randn(s, generator=gen) * 0.02 for s in flats + [batch]]
+    grads = [[(torch.randn(s, generator=gen) * torch.randn(s[:-1] + (1,), generator=gen).exp() * 1e-3).bfloat16() for s in flats + [batch]]
+             for _ in range(3)]
+    out = []
+    for n in (len(flats), len(flats) + 1):
+        params = [torch.nn.Parameter(x.clone().cuda()) for x in start[:n]]
+        for p in params:
+            p.grad_dtype = None
+        opt = Adafactor8Bit(params, **hp)
+        for row in grads:
+            for p, g in zip(params, row):
+                p.grad = g.cuda()
+            opt.step()
+        torch.cuda.synchronize()
+        out.append([(p.detach().cpu(), float(opt.state[p]["fira_prev_norm"])) for p in params[:len(flats)]])
+    apart = [(s, na, nb) for s, (a, na), (b, nb) in zip(flats, *out) if na != nb or not torch.equal(a, b)]
+    assert not apart, f"{len(apart)} of {len(flats)} matrices differ: {apart[:3]}"
+
+
 @pytest.mark.parametrize("came", [False, True])
 @pytest.mark.parametrize("shape", [(3, 40, 264), (3, 33, 131), (70, 1001), (3, 40, 256)])
 def test_infinities_and_nans_in_rows_of_any_length(shape, came, oracle):

@@ -1,0 +1,23 @@
+"""Which launch tables the tensors of a group go to (no GPU needed)."""
+import pytest
+import torch
+
+from adafactor8bit import Adafactor8Bit
+
+
+def tensor(shape, shift=0):
+    n = 1
+    for s in shape:
+        n *= s
+    return torch.zeros(n + shift)[shift:].view(shape)
+
+
+@pytest.mark.parametrize("batch,shift_p,shift_g,tables", [((4, 64, 64), 0, 0, 1), ((4, 64, 64), 1, 0, 2), ((4, 64, 64), 0, 1, 2),
+                                                          ((4, 64, 60), 0, 0, 2), ((1, 64, 64), 0, 0, 2)])
+def test_matrices_join_batches(batch, shift_p, shift_g, tables):
+    """Momentum-free matrices share the table of batches that hold most of the elements, unless a batch lies off the 16-byte
+    boundaries or some rows are no whole vectors."""
+    opt = Adafactor8Bit([torch.nn.Parameter(tensor((96, 64)))])
+    entries = [(0, tensor((96, 64)), tensor((96, 64)), {}), (1, tensor(batch, shift_p), tensor(batch, shift_g), {})]
+    launches = opt._sort_group(opt.param_groups[0], entries)
+    assert len(launches) == tables and sorted(e[0] for _, _, items in launches for e in items) == [0, 1]
