@@ -6,6 +6,7 @@ pinned host mirrors.  Each step the optimizer refreshes the host mirror
 (gradient pointers and the step's scalars change) and the plan enqueues the
 passes on the current CUDA stream.
 """
+import collections
 import ctypes
 import math
 
@@ -166,7 +167,28 @@ def ensure_qmap(device):
 # the event behind that copy.  The library's copies are unknown to torch's pinned-memory cache,
 # which would hand a freed block to the next ring at once: the queued copy would then read the
 # new ring's table.  Entries whose event has passed are let go when the next ring is made.
-_RETIRED = []
+# (Only single appends and pops, which are atomic: a ring may be dropped by another thread, or by
+# a garbage collection in the middle of _release_retired.)
+_RETIRED = collections.deque()
+
+
+def _pending(event):
+    """Whether a copy in front of the event may still be queued."""
+    try:
+        return not event.query()
+    except Exception:              # (not to be asked now, as while a stream is captured)
+        return True
+
+
+def _release_retired():
+    """Let go of the retired buffers whose copies have completed."""
+    for _ in range(len(_RETIRED)):
+        try:
+            entry = _RETIRED.popleft()
+        except IndexError:         # (another thread was faster)
+            return
+        if _pending(entry[1]):
+            _RETIRED.append(entry)
 
 
 class _PinnedRing:
@@ -174,7 +196,7 @@ class _PinnedRing:
     copy that read it has completed on the device, also when the ring itself is gone."""
 
     def __init__(self, nbytes, depth=3):
-        _RETIRED[:] = [x for x in _RETIRED if not x[1].query()]
+        _release_retired()
         self.bufs = [torch.empty(max(nbytes, 16), dtype=torch.uint8, pin_memory=True) for _ in range(depth)]
         self.events = [None] * depth
         self.views = [b.numpy() for b in self.bufs]
@@ -202,11 +224,10 @@ class _PinnedRing:
             self.events[self.i] = ev
         ev.record(stream)
 
-    def __del__(self, retired=_RETIRED):
-        try:
-            retired.extend(x for x in zip(self.bufs, self.events) if x[1] is not None and not x[1].query())
-        except Exception:      # (a ring that was never built, or a context that is gone)
-            pass
+    def __del__(self, retired=_RETIRED, pending=_pending):
+        for buf, ev in zip(getattr(self, "bufs", ()), getattr(self, "events", ())):
+            if ev is not None and pending(ev):
+                retired.append((buf, ev))
 
 
 class FullrankKey(tuple):
