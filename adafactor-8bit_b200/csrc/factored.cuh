@@ -111,12 +111,17 @@ __device__ __forceinline__ TilePos tile_pos(const FactoredLaunch &L, const af8_f
     return p;
 }
 
-// Parts per tile, as a power of two: a 512-row tile is 131072 elements, so a table of fewer than about 40 M parameters
-// has fewer tiles than CTAs that are resident together (3 per SM in the kernels with the most registers).  Tiles are
-// halved, down to 64 rows, while the parts still run in one wave: a part costs a fixed 4 us or so (pipeline fill, the
-// reduction over the warps, 256 column atomics), so that more waves of smaller parts lose - 256 tiles of an 8-layer
-// 512 x 1376 model: statistic pass 23 us whole, 42 us in eighths; sum pass 21 and 27 us.  CAME's residual pass spends
-// several times as long on a row, so that up to five waves of parts still gain there: 126 us whole, 98 us in eighths.
+// Parts per tile, as a power of two: a 512-row tile is 131072 elements, so a table of fewer than about 58 M parameters
+// has fewer tiles than three CTAs per SM, what most of these kernels keep resident (the residual pass over any rows, its
+// fp32 statistic and the fp32 write pass over tiles keep two; the same line served them as well).  Tiles are halved, down
+// to 64 rows, while the parts stay within `waves` times that many: a part costs a fixed 4 us or so (pipeline fill, the
+// reduction over the warps, 256 column atomics), so that more waves of smaller parts lose.  One wave for the statistic, sum
+// and write passes; CAME's residual pass spends several times as long on a row and gains up to three.  Measured, bf16
+// gradients, us with whole tiles / halves / quarters / eighths (512 x 1376 layers have 26 tiles, 768 x 2048 ones 64,
+// 1024 x 2752 ones 102):
+//   statistic  104 tiles 26 / 23 / 22 / 25    208 tiles 33 / 28 / 32 / 43    512 tiles 48 / 47 / 60 / 71    612 tiles 53 / 58 / 66 / 82
+//   residual    44 tiles 56 / 52 / 38 / 24    104 tiles 97 / 61 / 42 / 44    208 tiles 130 / 77 / 77 / 81
+//              512 tiles 97 / 97 / 138 / 179  612 tiles 208 / 159 / 175 / 177
 inline int tile_split(int64_t tiles, int waves = 1)
 {
     int sh = 0;
@@ -2451,7 +2456,7 @@ static int af8_factored_stats_impl(const af8_factored_cfg *cfg, const af8_factor
     const bool bf = cfg->grad_dtype == AF8_BF16, res = cfg->mode == AF8_FSTAT_RESIDUAL;
     const bool vec = cfg->aligned8 && cfg->grad_dtype != AF8_F16;      // fp16 gradients take the general kernels
     FactoredLaunch L = make_factored_launch(*cfg, dev_tensors, n_tensors, tiles, dyn, nullptr);
-    L.split = vec ? tile_split(tiles, res ? 5 : 1) : 0;
+    L.split = vec ? tile_split(tiles, res ? 3 : 1) : 0;
     L.total_units = tiles << L.split;
     int64_t grid = (int64_t)sm_count() * 6;
     if (grid > L.total_units) grid = L.total_units;
