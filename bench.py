@@ -12,8 +12,8 @@ copy bandwidth; `cpu_baseline` is the CPU restatement of the reference's step
 timed on this machine's host cores on a bounded sample.
 
 `--impl reference` times the reference's own CPU path alone, with all host threads: the unmodified
-reference package (its pure-PyTorch step, use_cuda_kernel=False) when an offline install of it is
-present under baseline/_ref, else the C restatement under oracle/.
+reference package (its pure-PyTorch step, use_cuda_kernel=False) from an offline install of it under
+baseline/_ref; without one it prints a line that says so.
 
 With N > 1 ranks the step is sharded ZeRO-1 style over the flat parameter space; the parameters
 that travel are a bf16 compute copy written by the update kernels, the fp32 masters stay sharded.
@@ -372,29 +372,33 @@ def reference_package_run(workload, steps, warmup):
 
 
 def run_reference_arm(args):
-    rank = int(os.environ.get("RANK", "0"))
-    if rank != 0:
+    """The unmodified reference package through its own optimizer class; one line that says so where it is not installed."""
+    if int(os.environ.get("RANK", "0")) != 0:
+        return
+    if reference_package_dir() is None:
+        print(json.dumps({"impl": "reference", "unavailable": "the reference package is not installed under baseline/_ref"}))
         return
     wl = WORKLOADS[args.workload]
-    port = cpu_reference_run(args.workload, max(1, min(args.steps, 50)), max(1, min(args.warmup, 5)))
-    if reference_package_dir() is not None:
-        steps = max(1, min(args.steps, 8))       # about 1 s per step on the sample
-        warm = max(1, min(args.warmup, 2))
-        r = reference_package_run(args.workload, steps, warm)
-    else:
-        steps, warm, r = max(1, min(args.steps, 50)), max(1, min(args.warmup, 5)), port
-    cpu = {k: r[k] for k in ("value", "unit", "cores", "kind", "sample")}
-    cpu["port_value"] = port["value"]              # the C + OpenMP restatement (oracle/) on the same sample
-    cpu["port_cores"] = port["cores"]
+    steps, warm = max(1, min(args.steps, 8)), max(1, min(args.warmup, 2))       # about 1 s per step on the sample
+    r = reference_package_run(args.workload, steps, warm)
     line = {
         "impl": "reference", "metric": "optimizer_step_throughput", "value": r["value"], "unit": "Gparams/s",
         "n_gpus": args.gpus, "steps": steps, "warmup": warm, "ms_per_step": r["ms_per_step"],
         "higher_is_better": True, "scaling": "strong", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
         "config": {"workload": args.workload, "grad_dtype": wl["grad"], "sample_params": r["sample_params"]},
-        "cpu_baseline": cpu,
+        "cpu_baseline": {k: r[k] for k in ("value", "unit", "cores", "kind", "sample")},
         "e2e": {"value": r["value"], "unit": "Gparams/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
     }
     print(json.dumps(line))
+
+
+def run_cpu_baseline(args):
+    """The CPU baseline of the GPU arm's line: the reference package where it is installed, else the C restatement under
+    oracle/, whose own figure goes along in either case."""
+    port = cpu_reference_run(args.workload, max(1, min(args.steps, 50)), max(1, min(args.warmup, 5)))
+    r = reference_package_run(args.workload, max(1, min(args.steps, 8)), max(1, min(args.warmup, 2))) if reference_package_dir() else port
+    cpu = {k: r[k] for k in ("value", "unit", "cores", "kind", "sample")}
+    print(json.dumps(dict(cpu, port_value=port["value"], port_cores=port["cores"])))
 
 
 # ---------------------------------------------------------------------------
@@ -634,12 +638,12 @@ def run_gpu_arm(args):
 
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu:
-        # the reference arm in a process of its own (the reference package has the name of this repository's)
-        res = subprocess.run([sys.executable, os.path.abspath(__file__), "--impl", "reference", "--workload", args.workload,
+        # in a process of its own (the reference package has the name of this repository's)
+        res = subprocess.run([sys.executable, os.path.abspath(__file__), "--cpu-baseline", "--workload", args.workload,
                               "--steps", "3", "--warmup", "1"], capture_output=True, text=True, timeout=900)
         for ln in reversed(res.stdout.strip().splitlines()):
             if ln.startswith("{"):
-                cpu = json.loads(ln)["cpu_baseline"]
+                cpu = json.loads(ln)
                 break
         if cpu is None:
             raise RuntimeError("the CPU baseline run printed no result:\n" + res.stderr[-2000:])
@@ -681,12 +685,15 @@ def main():
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--workload", default=DEFAULT_WORKLOAD, choices=sorted(WORKLOADS))
     ap.add_argument("--impl", default="b200", choices=["b200", "reference"])
+    ap.add_argument("--cpu-baseline", action="store_true", help="print the CPU baseline of the workload alone")
     ap.add_argument("--no-e2e", action="store_true")
     ap.add_argument("--no-cpu", action="store_true")
     ap.add_argument("--fp32-gather", action="store_true", help="N > 1: gather the fp32 parameters themselves (no bf16 compute copy)")
     args = ap.parse_args()
-    args.warmup = max(args.warmup, 3) if args.impl == "b200" else args.warmup
-    if args.impl == "reference":
+    args.warmup = max(args.warmup, 3) if args.impl == "b200" and not args.cpu_baseline else args.warmup
+    if args.cpu_baseline:
+        run_cpu_baseline(args)
+    elif args.impl == "reference":
         run_reference_arm(args)
     else:
         run_gpu_arm(args)
