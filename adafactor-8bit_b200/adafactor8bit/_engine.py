@@ -350,9 +350,12 @@ class FullrankPlan:
 
     # -- launches ------------------------------------------------------------
     def kernel_name(self, mode):
+        """The kernel that af8_fullrank_step runs in this mode (fast_covers in csrc/fullrank_api.cuh)."""
         c = self.cfg
-        fast = (c.v_fmt == N.V_AL8 and c.m_fmt == N.M_UF8 and c.block == 2048 and c.m_block == 256
-                and c.use_adam_denom and not c.momentum_only and mode != N.MODE_SUMSQ_M
+        fast = (c.use_adam_denom and not c.momentum_only and c.block == 2048 and mode != N.MODE_SUMSQ_M
+                and c.v_fmt in (N.V_AL8, N.V_AL16)
+                and (c.m_fmt == N.M_NONE or (c.m_block == 256 and c.m_fmt in (N.M_UF8, N.M_UF4)))
+                and (mode != N.MODE_LAG or (c.v_fmt == N.V_AL8 and c.m_fmt == N.M_UF8))
                 and ((c.param_dtype == N.F32 and c.grad_dtype in (N.F32, N.BF16))
                      or (c.param_dtype == N.BF16 and c.grad_dtype == N.BF16)))
         if fast and mode == N.MODE_SUMSQ:

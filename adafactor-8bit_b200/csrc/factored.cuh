@@ -9,13 +9,14 @@
 //
 // Three kernels, each launched once for a whole table of tensors:
 //   factored_stats_kernel   row and column sums of g*g, or of CAME's residual
-//                           (U - M)^2 + eps, over 64 x 256 tiles.  Every product
+//                           (U - M)^2 + eps, over 512 x 256 tiles.  Every product
 //                           is rounded to binary32 as torch does and then
 //                           accumulated in binary64, so the binary32 means do not
 //                           depend on the order of accumulation.
-//   factored_small_kernel   one CTA per tensor: means, EMA into the (tiny) row /
-//                           column AL states with exact requantisation, mean of
-//                           the row state, inverse-std vectors.
+//   factored_small_kernel   one CTA per quantisation block of a row / column state:
+//                           means, EMA into the (tiny) AL states with exact
+//                           requantisation, partial means of the row state; the
+//                           inverse-std vectors follow in factored_inv_kernel.
 //   factored_update_kernel  flat chunks aligned to momentum blocks: the update
 //                           itself, its sum of squares, the parameter write and
 //                           the momentum requantisation.

@@ -105,13 +105,6 @@ __device__ __forceinline__ int find_tensor(const af8_fullrank_tensor *tensors, i
 template <typename T> struct GradLoad;
 
 template <> struct GradLoad<float> {
-    static __device__ __forceinline__ void load8(const void *base, int64_t off, float (&g)[8])
-    {
-        const float4 *p = reinterpret_cast<const float4 *>(static_cast<const float *>(base) + off);
-        float4 a = __ldcs(p), b = __ldcs(p + 1);
-        g[0] = a.x; g[1] = a.y; g[2] = a.z; g[3] = a.w;
-        g[4] = b.x; g[5] = b.y; g[6] = b.z; g[7] = b.w;
-    }
     static __device__ __forceinline__ float load1(const void *base, int64_t off)
     {
         return static_cast<const float *>(base)[off];
@@ -127,15 +120,6 @@ template <> struct GradLoad<f16_tag> {      // (general kernel only)
     }
 };
 template <> struct GradLoad<bf16_tag> {
-    static __device__ __forceinline__ void load8(const void *base, int64_t off, float (&g)[8])
-    {
-        const uint4 *p = reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(base) + off);
-        uint4 a = __ldcs(p);
-        g[0] = __uint_as_float(a.x << 16); g[1] = __uint_as_float(a.x & 0xffff0000u);
-        g[2] = __uint_as_float(a.y << 16); g[3] = __uint_as_float(a.y & 0xffff0000u);
-        g[4] = __uint_as_float(a.z << 16); g[5] = __uint_as_float(a.z & 0xffff0000u);
-        g[6] = __uint_as_float(a.w << 16); g[7] = __uint_as_float(a.w & 0xffff0000u);
-    }
     static __device__ __forceinline__ float load1(const void *base, int64_t off)
     {
         return bf16_bits_to_f32(static_cast<const uint16_t *>(base)[off]);

@@ -2,9 +2,10 @@
 // (V: fp32 / AL8 / AL16; M: none / UF8 / UF4 / d8 / d4 / fp32), block sizes and
 // update rules that the reference's full-rank path accepts
 // (_update_param_8bit, optimizer.py:2076-2194; _fallback_1d_update,
-// optimizer.py:886-917).  The specialised kernel in fullrank_fast.cuh covers
-// the AdamW UF8/AL8 configuration; this one covers the rest and the small
-// fp32-state tensors (numel < min_8bit_size, optimizer.py:1640-1641).
+// optimizer.py:886-917).  The specialised kernels in fullrank_fast.cuh cover the
+// Adam denominator with AL8 / AL16 second moments in blocks of 2048 and UF8 / UF4
+// momentum in blocks of 256 or none (fast_covers); this one covers the rest and the
+// small fp32-state tensors (numel < min_8bit_size, optimizer.py:1640-1641).
 //
 // One CTA owns one V block of `block` elements.  The new second moment (as its
 // log2) and the new momentum are staged in shared memory, because the block

@@ -217,9 +217,8 @@ def test_tensor_core_projection(rows, cols, rank, negate):
 
 
 def test_tensor_core_projection_batch():
-    """af8_apollo_project_batch over mixed shapes: right-case tensors and, through the transposed
-    gradient, left-case ones on the tcgen05 kernel; a rank that is no multiple of 16 on mma.sync;
-    a scratch too small for the last tensor, which then stays on mma.sync as well."""
+    """af8_apollo_project_batch over mixed shapes: right-case tensors and left-case ones (the gradient as an
+    M-major operand) on the tcgen05 kernel, a rank that is no multiple of 16 on mma.sync."""
     from adafactor8bit import _native as N
     lib = N.lib()
     rng = np.random.default_rng(5)
@@ -250,7 +249,7 @@ def test_tensor_core_projection_batch():
     tb = int(lib.af8_apollo_project_task_bytes()) * len(shapes)
     h = torch.empty(tb, dtype=torch.uint8).pin_memory()
     d = torch.empty(tb, dtype=torch.uint8, device="cuda")
-    t_bytes = 200 * 1024                      # fits tensors 1 and 2 one at a time (160 KB, 129 KB), not tensor 4 (384 KB)
+    t_bytes = 200 * 1024                      # (a scratch buffer, as callers had to pass one for left-case tensors: not used)
     t = torch.empty(t_bytes + 256, dtype=torch.uint8, device="cuda")
     N.check(lib.af8_apollo_project_batch(descs.ctypes.data, len(shapes), N.BF16, h.data_ptr(), d.data_ptr(),
                                          (t.data_ptr() + 255) // 256 * 256, t_bytes, stream), "project_batch")
