@@ -245,7 +245,7 @@ inline int dispatch_fast_mode(int mode, FullrankLaunch L, bool eps_hides, cudaSt
 {
     if (mode == AF8_MODE_SUMSQ) return launch_stat<GradT, VB, MF>(L, st);
     if constexpr (VB == 8 && MF == AF8_M_UF8) {
-        if (mode == AF8_MODE_LAG) return launch_fast<GradT, ParamT, VB, MF, SR, true, ROOT_FULL>(L, st);
+        if (mode == AF8_MODE_LAG) return eps_hides ? launch_fast<GradT, ParamT, VB, MF, SR, true, ROOT_FTZ>(L, st) : launch_fast<GradT, ParamT, VB, MF, SR, true, ROOT_FULL>(L, st);
     }
     if (mode == AF8_MODE_NOCLIP) L.dyn = nullptr;        // the step size is the table's
     constexpr int HIDES = root_exact<VB, MF> ? ROOT_REFINED : ROOT_FTZ, SHOWS = root_exact<VB, MF> ? ROOT_EXACT : ROOT_FULL;
