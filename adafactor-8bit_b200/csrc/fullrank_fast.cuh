@@ -15,7 +15,7 @@
 // momentum absmax is a pure warp reduction.  Lane l owns the 4-element groups at
 // 512w+4l, +128, +256 and +384: every shared-memory read and every global store
 // of a warp is one contiguous run.  Sixteen elements per thread halve what a
-// block costs besides its elements against eight (256 threads): 69 -> 54
+// block costs besides its elements against eight (256 threads): 69 -> 56
 // instructions per parameter, and a block-wide barrier joins four warps instead
 // of eight.
 //
@@ -31,7 +31,7 @@
 // the CTA stops at its next block-wide barrier.
 //
 // What bounds it: instruction issue and the latency between dependent
-// instructions (57 % of the issue slots at 24 warps per SM; DRAM 63 % busy), so
+// instructions (62 % of the issue slots with 22 warps resident; DRAM 64 % busy), so
 // the hot loop is kept small (about 14 KB of code): what is rare - tail blocks, uncommon
 // scalars, codes in doubt - is rolled up or handled by a compact general branch.  Inlined
 // between the parts of the loop those copies had put instruction fetches at the top of the
@@ -55,10 +55,10 @@
 //
 // Measured on a B200, before -> after the split by sixteen elements (and, for the formats other
 // than UF8/AL8, against the general kernel): TinyLlama-1.1B update pass 3.23 -> 2.8 ms (5.5 TB/s);
-// bf16 parameters with stochastic rounding 5.0 -> 3.75 ms; UF4/AL16, 176 M parameters 4.17 -> 0.99 ms;
+// bf16 parameters with stochastic rounding 5.0 -> 3.75 ms; UF4/AL16, 176 M parameters 4.17 -> 1.03 ms;
 // AL8 without momentum, fp32 gradients, 110 M parameters 1.95 -> 0.32 ms (4.9 TB/s).  The correctly
-// rounded update of these formats (ROOT_REFINED) costs 5 to 12 % of that against the hardware
-// approximations; with the IEEE functions it cost 30 %.
+// rounded update of these formats (ROOT_REFINED) costs 5 to 12 % against the hardware approximations
+// (30 % with the IEEE functions), the tests for infinities and NaNs (STRICT) up to 4 %.
 #pragma once
 
 #include "common.cuh"
@@ -130,7 +130,8 @@ template <> struct GradLoad<bf16_tag> {
 //   ROOT_EXACT    every operation correctly rounded, as in the general kernel; every format pair but UF8/AL8
 //   ROOT_REFINED  the same numbers from the hardware approximations and one residual step each (Markstein 1990), in packed
 //                 arithmetic: a third of the instructions of the IEEE functions.  Above EPS_HIDES (below) only: a residual
-//                 of v < 2^-100 may be subnormal, but no bit of such a square root survives the addition of eps
+//                 of v < 2^-100 may be subnormal, but no bit of such a square root survives the addition of eps.  (The
+//                 remainder of a gradient below 2^-100 may be, too: the last bit of a quotient below 2^-62)
 //   ROOT_FTZ      hardware approximations in their flush-to-zero forms, one MUFU instruction each (UF8/AL8; relative error
 //                 below 3e-7).  A second moment below 2^-126 has a square root below 2^-63, which an eps of 2^-38
 //                 (EPS_HIDES) or more absorbs whole; below that eps the square root is the denominator and must not be

@@ -21,3 +21,16 @@ def test_matrices_join_batches(batch, shift_p, shift_g, tables):
     entries = [(0, tensor((96, 64)), tensor((96, 64)), {}), (1, tensor(batch, shift_p), tensor(batch, shift_g), {})]
     launches = opt._sort_group(opt.param_groups[0], entries)
     assert len(launches) == tables and sorted(e[0] for _, _, items in launches for e in items) == [0, 1]
+
+
+@pytest.mark.parametrize("v,m,param,grad,mode,name", [
+    ("al8", "uf8", "f32", "bf16", "apply", "fullrank_fast_apply"), ("al16", "uf4", "f32", "f32", "noclip", "fullrank_fast_noclip"),
+    ("al8", None, "bf16", "bf16", "sumsq", "fullrank_stat"), ("al16", "uf8", "f32", "bf16", "lag", "fullrank_generic_lag"),
+    ("al8", "d8", "f32", "bf16", "apply", "fullrank_generic_apply"), ("al8", "uf8", "f32", "f16", "apply", "fullrank_generic_apply"),
+    ("fp32", "uf8", "f32", "f32", "sumsq", "fullrank_generic_sumsq")])
+def test_kernel_names_follow_the_dispatch(v, m, param, grad, mode, name):
+    from adafactor8bit import _engine as E, _native as N
+    plan = object.__new__(E.FullrankPlan)
+    plan.cfg = N.FullrankCfg(block=2048, m_block=256 if m else 0, v_fmt=N.V_FMT[v], m_fmt=N.M_FMT[m], use_adam_denom=1,
+                             param_dtype=getattr(N, param.upper()), grad_dtype=getattr(N, grad.upper()))
+    assert plan.kernel_name(getattr(N, "MODE_" + mode.upper())) == name
