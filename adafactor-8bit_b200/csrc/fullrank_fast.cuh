@@ -55,7 +55,7 @@
 //
 // Measured on a B200, before -> after the split by sixteen elements (and, for the formats other
 // than UF8/AL8, against the general kernel): TinyLlama-1.1B update pass 3.23 -> 2.8 ms (5.5 TB/s);
-// bf16 parameters with stochastic rounding 5.0 -> 3.75 ms; UF4/AL16, 176 M parameters 4.17 -> 1.03 ms;
+// bf16 parameters with stochastic rounding 5.0 -> 3.75 ms; UF4/AL16, 176 M parameters 4.17 -> 1.02 ms;
 // AL8 without momentum, fp32 gradients, 110 M parameters 1.95 -> 0.32 ms (4.9 TB/s).  The correctly
 // rounded update of these formats (ROOT_REFINED) costs 5 to 12 % against the hardware approximations
 // (30 % with the IEEE functions), the tests for infinities and NaNs (STRICT) up to 4 %.
@@ -70,12 +70,12 @@ constexpr int FAST_MBLOCK = 256;
 constexpr int FAST_THREADS = 128;
 constexpr int FAST_EPT = 16;  // elements per thread
 constexpr int FAST_WARPS = FAST_THREADS / 32;
-// resident CTAs asked of the compiler (AL8: 5 -> 6 gave 1-3 %; AL16: 3, 4 and 5 gave 0.93, 0.91 and 0.97 ms on 176 M UF4/AL16 parameters, before ROOT_REFINED)
+// resident CTAs asked of the compiler (AL8: 5 -> 6 gave 1-3 %; AL16: 3, 4 and 5 gave 1.015, 1.03 and 1.11 ms on 176 M UF4/AL16 parameters)
 #ifndef AF8_FAST_CTAS8
 #define AF8_FAST_CTAS8 6
 #endif
 #ifndef AF8_FAST_CTAS16
-#define AF8_FAST_CTAS16 4
+#define AF8_FAST_CTAS16 3
 #endif
 template <int VB> constexpr int fast_min_ctas() { return VB == 8 ? AF8_FAST_CTAS8 : AF8_FAST_CTAS16; }
 
