@@ -55,7 +55,7 @@
 //
 // Measured on a B200, before -> after the split by sixteen elements (and, for the formats other
 // than UF8/AL8, against the general kernel): TinyLlama-1.1B update pass 3.23 -> 2.8 ms (5.5 TB/s);
-// bf16 parameters with stochastic rounding 5.0 -> 3.75 ms; UF4/AL16, 176 M parameters 4.17 -> 1.02 ms;
+// bf16 parameters with stochastic rounding 5.0 -> 3.6 ms; UF4/AL16, 176 M parameters 4.17 -> 0.93 ms;
 // AL8 without momentum, fp32 gradients, 110 M parameters 1.95 -> 0.32 ms (4.9 TB/s).  The correctly
 // rounded update of these formats (ROOT_REFINED) costs 5 to 12 % against the hardware approximations
 // (30 % with the IEEE functions), the tests for infinities and NaNs (STRICT) up to 4 %.
@@ -70,14 +70,23 @@ constexpr int FAST_MBLOCK = 256;
 constexpr int FAST_THREADS = 128;
 constexpr int FAST_EPT = 16;  // elements per thread
 constexpr int FAST_WARPS = FAST_THREADS / 32;
-// resident CTAs asked of the compiler (AL8: 5 -> 6 gave 1-3 %; AL16: 3, 4 and 5 gave 1.015, 1.03 and 1.11 ms on 176 M UF4/AL16 parameters)
+// resident CTAs asked of the compiler (AL8: 5 -> 6 gave 1-3 %; AL16: see fast_stash)
 #ifndef AF8_FAST_CTAS8
 #define AF8_FAST_CTAS8 6
 #endif
 #ifndef AF8_FAST_CTAS16
-#define AF8_FAST_CTAS16 3
+#define AF8_FAST_CTAS16 5
 #endif
 template <int VB> constexpr int fast_min_ctas() { return VB == 8 ? AF8_FAST_CTAS8 : AF8_FAST_CTAS16; }
+
+// Whether the new second moments wait for the block's range in the ring slot, in place of the consumed parameters, instead of
+// in registers, and the two momentum blocks of a warp take turns in one copy of the code.  AL16: the binary64 sequences of
+// sixteen elements at once took 144 registers, three CTAs per SM, and were bound by latency (55 % of the issue slots); eight at
+// a time fit 96 registers and five CTAs (67 M UF4/AL16 parameters 383 -> 346 us; four
+// CTAs 352, six 428).  The slot is then read until the block's
+// last code is written, so that the last warp to leave it has it refilled.  With AL8, where registers suffice, the detour
+// costs more than it gives (fp32 parameters 177 -> 188 us, bf16 ones 174 -> 196).
+template <int VB> __host__ __device__ constexpr bool fast_stash() { return VB == 16; }
 
 struct FullrankLaunch {
     const af8_fullrank_tensor *tensors;
@@ -674,6 +683,54 @@ __device__ __forceinline__ void fast_round8(const float2 (&p)[4], uint64_t sr_ba
     }
 }
 
+// The four new second moments of the group at o, in place of its consumed inputs in the ring slot: 16 bytes of fp32
+// parameters, or 8 of bf16 parameters and 8 of gradients.
+template <int PB, int P_OFF, int G_OFF>
+__device__ __forceinline__ void stash_put(unsigned char *st, int o, float a, float b, float c, float d)
+{
+    if (PB == 4) {
+        *reinterpret_cast<float4 *>(st + P_OFF + o * 4) = make_float4(a, b, c, d);
+    } else {
+        *reinterpret_cast<float2 *>(st + P_OFF + o * 2) = make_float2(a, b);
+        *reinterpret_cast<float2 *>(st + G_OFF + o * 2) = make_float2(c, d);
+    }
+}
+template <int PB, int P_OFF, int G_OFF>
+__device__ __forceinline__ float4 stash_get(const unsigned char *st, int o)
+{
+    if (PB == 4) return *reinterpret_cast<const float4 *>(st + P_OFF + o * 4);
+    const float2 a = *reinterpret_cast<const float2 *>(st + P_OFF + o * 2), b = *reinterpret_cast<const float2 *>(st + G_OFF + o * 2);
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+template <int PB, int P_OFF, int G_OFF>
+__device__ __forceinline__ float *stash_at(unsigned char *st, int e)
+{
+    if (PB == 4) return reinterpret_cast<float *>(st + P_OFF) + e;
+    return reinterpret_cast<float *>(st + ((e & 2) ? G_OFF : P_OFF) + (e & ~3) * 2) + (e & 1);
+}
+
+// Bulk copies of the full blocks b + from * G .. b + (to - 1) * G into their ring slots (one thread).
+template <typename Ring, int MF>
+__device__ __forceinline__ void fast_issue(const af8_fullrank_tensor &sT, unsigned char *ring, uint64_t *full, int b, int G, int n, int from, int to)
+{
+    constexpr int VQ = Ring::VQ_BYTES / (FAST_VBLOCK / 8);       // bits per second-moment code
+    const unsigned char *gp = static_cast<const unsigned char *>(sT.grad);
+    const unsigned char *pp = static_cast<const unsigned char *>(sT.param);
+    const unsigned char *vp = static_cast<const unsigned char *>(sT.v_q);
+    fence_proxy_async();
+    for (int k = from; k < to; ++k) {
+        const int64_t nb = (int64_t)(b + k * G) * FAST_VBLOCK;
+        const int sl = (n + k) % Ring::NST;
+        unsigned char *dst = ring + sl * Ring::STAGE_BYTES;
+        mbar_expect_tx(&full[sl], Ring::STAGE_BYTES);
+        bulk_g2s(dst + Ring::P_OFF, pp + nb * Ring::PB, FAST_VBLOCK * Ring::PB, &full[sl]);
+        bulk_g2s(dst + Ring::G_OFF, gp + nb * Ring::GB, FAST_VBLOCK * Ring::GB, &full[sl]);
+        bulk_g2s(dst + Ring::VQ_OFF, vp + nb * (VQ / 8), Ring::VQ_BYTES, &full[sl]);
+        if (MF != AF8_M_NONE)
+            bulk_g2s(dst + Ring::MQ_OFF, sT.m_q + (MF == AF8_M_UF4 ? nb / 2 : nb), Ring::MQ_BYTES, &full[sl]);
+    }
+}
+
 // SR: bf16 parameters rounded stochastically.  LAG: the scalars are those of the previous step and the
 // sum of squares of this step's raw update goes to block_sumsq.  ROOT_FTZ: every eps of the table is at least EPS_HIDES.
 // (A kernel of its own: chosen per tensor or per block inside one kernel, the two forms cost the common one 2 to 15 %
@@ -690,6 +747,9 @@ fullrank_fast_kernel(const FullrankLaunch L)
     constexpr int QMAX = VB == 16 ? 65535 : 255;
     constexpr float QM1 = VB == 16 ? 65534.0f : 254.0f;
     constexpr bool TABLE = VB == 8;
+    constexpr bool STASH = fast_stash<VB>();
+    constexpr int MB_UNROLL = STASH ? 1 : 2;
+    static_assert(!STASH || NST == 2, "a slot that is left is refilled for the block after the next one");
     // Infinities and NaNs in whole blocks as in the general kernel.  Not with UF8/AL8, where their tests cost 8 % of the
     // update pass: there a NaN is left out of the range and of the largest magnitude.
     constexpr bool STRICT = root_exact<VB, MF>;
@@ -704,6 +764,7 @@ fullrank_fast_kernel(const FullrankLaunch L)
     __shared__ float s_usq[FAST_WARPS];
     __shared__ VRange s_vr;
     __shared__ int s_abort;
+    __shared__ int s_left;                           // STASH: warps that have left a slot, a running count
     __shared__ double s_exp2[TABLE ? 32 : 1];        // copy of the exp2 table of the decode
     __shared__ double2 s_log2[97];                   // copy of the log2 table of the range computation
 
@@ -719,6 +780,7 @@ fullrank_fast_kernel(const FullrankLaunch L)
     if (tid == 0) {
         for (int k = 0; k < NST; ++k) mbar_init(&s_full[k], 1);
         s_abort = 0;
+        s_left = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -782,8 +844,8 @@ fullrank_fast_kernel(const FullrankLaunch L)
             if (want == k && b + k * G < nfull) want = k + 1;
         const bool next_staged = want >= 2;           // the next block gets its table and ranges prepared here
 
-        // ---- issue the bulk copies (one thread) ----
-        if (tid == 0 && ahead < want) {
+        // ---- issue the bulk copies (one thread; STASH: the first ones of a tensor, the others when a slot is left) ----
+        if (tid == 0 && ahead < want && (!STASH || ahead == 0)) {
             const unsigned char *gp = static_cast<const unsigned char *>(sT.grad);
             const unsigned char *pp = static_cast<const unsigned char *>(sT.param);
             const unsigned char *vp = static_cast<const unsigned char *>(sT.v_q);
@@ -860,7 +922,7 @@ fullrank_fast_kernel(const FullrankLaunch L)
         if (SR) counter = sr_counter(sT.sr_base, base, FAST_VBLOCK);
         // (uniform over the CTA; a block that decodes to infinities or NaNs takes the general forms: ROOT_REFINED would lose a NaN)
         const bool hot = full && S.plain && (!root_exact<VB, MF> || range_finite(csc, cml));
-        float v[FAST_EPT];                   // hot blocks: the new second moments
+        float v[STASH ? 8 : FAST_EPT];       // hot blocks: the new second moments (STASH: of one momentum block)
         float usq = 0.0f;                    // LAG: this thread's sum of squares of the raw update
         // Extrema of v.  v >= 0, so the bit patterns order like the values.  The minimum runs over the
         // non-zero elements (optimizer.py:312-313) and travels as bits - 1, which sends "none" to the top.
@@ -868,18 +930,28 @@ fullrank_fast_kernel(const FullrankLaunch L)
 
         if (hot) {
             // ---- two momentum blocks per warp: EMAs, update, parameter, momentum codes ----
-#pragma unroll
+            float fmn = INFINITY, fmx = 0.0f;    // (STRICT: a NaN reaches fmx, else neither)
+#pragma unroll (MB_UNROLL)
             for (int mb = 0; mb < 2; ++mb) {
                 const int oa = ow + mb * FAST_MBLOCK;
                 float2 g[4], p[4], v_old[4], m_old[4], vn[4], mn[4];
-                fast_load8<GradT, ParamT, VB, MF, true>(st, oa, s_tab[stage], csc, cml, cms[mb], LT, p, g, v_old, m_old);
+                fast_load8<GradT, ParamT, VB, MF, true>(st, oa, s_tab[stage], csc, cml, STASH ? (mb ? cms[1] : cms[0]) : cms[mb], LT, p, g, v_old, m_old);
                 if (L.negate_grad) {                              // maximize (optimizer.py:1973-1974)
 #pragma unroll
                     for (int j = 0; j < 4; ++j) g[j] = make_float2(-g[j].x, -g[j].y);
                 }
                 fast_ema8<MF, true, PB == 2 && !SR, LAG, ROOT>(S, g, v_old, m_old, p, vn, mn, 0xffu, usq);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) { v[8 * mb + 2 * j] = vn[j].x; v[8 * mb + 2 * j + 1] = vn[j].y; }
+                for (int j = 0; j < 4; ++j) { v[(STASH ? 0 : 8 * mb) + 2 * j] = vn[j].x; v[(STASH ? 0 : 8 * mb) + 2 * j + 1] = vn[j].y; }
+                if constexpr (STASH) {
+                    stash_put<PB, P_OFF, G_OFF>(st, oa, v[0], v[1], v[2], v[3]);
+                    stash_put<PB, P_OFF, G_OFF>(st, oa + 128, v[4], v[5], v[6], v[7]);
+#pragma unroll
+                    for (int j = 0; j < 8; j += 2) {
+                        fmn = min3(fmn, v[j], v[j + 1]);
+                        fmx = STRICT ? max3_nan(fmx, v[j], v[j + 1]) : max3(fmx, v[j], v[j + 1]);
+                    }
+                }
                 PElem *const pa = static_cast<PElem *>(sT.param) + base + oa;
                 if (PB == 4) {
                     if (!bad) {
@@ -902,23 +974,35 @@ fullrank_fast_kernel(const FullrankLaunch L)
                 if (MF != AF8_M_NONE)
                     fast_store_m<MF, STRICT>(mn, sT.m_q, sT.m_scale + (int64_t)b * MPB + 2 * warp + mb, base + oa, !bad, lane);
             }
-            float fmn = v[0], fmx = v[0];        // (STRICT: a NaN reaches fmx, else neither)
+            if constexpr (!STASH) {
+                fmn = fmx = v[0];
 #pragma unroll
-            for (int j = 1; j + 1 < FAST_EPT; j += 2) {
-                fmn = min3(fmn, v[j], v[j + 1]);
-                fmx = STRICT ? max3_nan(fmx, v[j], v[j + 1]) : max3(fmx, v[j], v[j + 1]);
+                for (int j = 1; j + 1 < FAST_EPT; j += 2) {
+                    fmn = min3(fmn, v[j], v[j + 1]);
+                    fmx = STRICT ? max3_nan(fmx, v[j], v[j + 1]) : max3(fmx, v[j], v[j + 1]);
+                }
+                fmn = fminf(fmn, v[FAST_EPT - 1]);
+                fmx = STRICT ? max3_nan(fmx, v[FAST_EPT - 1], v[FAST_EPT - 1]) : fmaxf(fmx, v[FAST_EPT - 1]);
             }
-            fmn = fminf(fmn, v[FAST_EPT - 1]);
-            fmx = STRICT ? max3_nan(fmx, v[FAST_EPT - 1], v[FAST_EPT - 1]) : fmaxf(fmx, v[FAST_EPT - 1]);
             umin = __reduce_min_sync(0xffffffffu, __float_as_uint(fmn));
             umax = __reduce_max_sync(0xffffffffu, __float_as_uint(fmx));
             if (umin == 0u || (STRICT && umax > 0x7f800000u)) {      // the warp holds a zero (rare after the first steps, except in all-zero regions) or a NaN
                 uint32_t um = 0xffffffffu, ux = 0u;
+                if constexpr (STASH) {
+#pragma unroll 1
+                    for (int q = 0; q < FAST_EPT; ++q) {
+                        float *const x = stash_at<PB, P_OFF, G_OFF>(st, ow + (q >> 2) * 128 + (q & 3));
+                        if (!(*x >= 0.0f)) *x = AF8_TINY;                // (see al_log2)
+                        um = min(um, __float_as_uint(*x) - 1u);
+                        ux = max(ux, __float_as_uint(*x));
+                    }
+                } else {
 #pragma unroll
-                for (int j = 0; j < FAST_EPT; ++j) {
-                    if (STRICT && !(v[j] >= 0.0f)) v[j] = AF8_TINY;      // (see al_log2)
-                    um = min(um, __float_as_uint(v[j]) - 1u);
-                    if (STRICT) ux = max(ux, __float_as_uint(v[j]));
+                    for (int j = 0; j < FAST_EPT; ++j) {
+                        if (STRICT && !(v[j] >= 0.0f)) v[j] = AF8_TINY;
+                        um = min(um, __float_as_uint(v[j]) - 1u);
+                        if (STRICT) ux = max(ux, __float_as_uint(v[j]));
+                    }
                 }
                 umin = __reduce_min_sync(0xffffffffu, um);
                 if (STRICT) umax = __reduce_max_sync(0xffffffffu, ux);
@@ -973,7 +1057,6 @@ fullrank_fast_kernel(const FullrankLaunch L)
                 if (MF != AF8_M_NONE)
                     fast_store_m<MF, STRICT>(mn, sT.m_q, sT.m_scale + (int64_t)b * MPB + 2 * warp + mb, base + oa,
                                      (2 * warp + mb) * FAST_MBLOCK < rem && !bad, lane);
-                // (this thread's own inputs: 16 bytes of fp32 parameters, or 8 of bf16 parameters and 8 of gradients, per group)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int o = oa + 128 * h;
@@ -1043,25 +1126,10 @@ fullrank_fast_kernel(const FullrankLaunch L)
             }
         }
 
-        // ---- what does not need the range: the next block's decode table, or (AL16) this block's log2 ----
+        // ---- what does not need the range: the next block's decode table ----
         if (TABLE && next_staged) {
             s_tab[stage ^ 1][tid] = al8_decode_fast<STRICT>((uint32_t)tid, nsc, nml, s_exp2);
             s_tab[stage ^ 1][tid + 128] = al8_decode_fast<STRICT>((uint32_t)tid + 128u, nsc, nml, s_exp2);
-        }
-        float lv[TABLE ? 1 : FAST_EPT];
-        if (!TABLE && hot) {
-            uint32_t odd = 0u;                                   // subnormal second moments above the floor of 1e-38
-#pragma unroll
-            for (int j = 0; j < FAST_EPT; ++j) {
-                const float l = log2_lane(v[j], LT);             // (shuffles: every lane takes part)
-                lv[TABLE ? 0 : j] = v[j] > AF8_TINY ? l : AF8_LOG2_TINY;
-                if (v[j] > AF8_TINY && v[j] < 1.17549435e-38f) odd |= 1u << j;
-            }
-#pragma unroll 1
-            for (; odd; odd &= odd - 1u) {
-                const int j = __ffs((int)odd) - 1;
-                put(lv, j, log2_cr_fast(pick(v, j), s_log2));
-            }
         }
         __syncthreads();                     // ---- E ----
         if (s_abort) {       // a copy never completed: give the ones still in flight a bounded chance, then stop
@@ -1090,7 +1158,7 @@ fullrank_fast_kernel(const FullrankLaunch L)
             for (int mb = 0; mb < 2; ++mb) {
                 float x[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) x[j] = v[8 * mb + j];
+                for (int j = 0; j < 8; ++j) x[j] = v[STASH ? j : 8 * mb + j];
                 uint32_t kk[8];
                 float dd[8];
                 float dmax = 0.0f;
@@ -1128,7 +1196,7 @@ fullrank_fast_kernel(const FullrankLaunch L)
         } else if (r.thr < 0.0f) {
 #pragma unroll 1
             for (int q = 0; q < FAST_EPT; ++q) {
-                const float x = pick(v, q);
+                const float x = *stash_at<PB, P_OFF, G_OFF>(st, ow + (q >> 2) * 128 + (q & 3));
                 static_cast<uint16_t *>(sT.v_q)[base + ow + (q >> 2) * 128 + (q & 3)] = (uint16_t)al_encode(x, al_log2_fast(x, s_log2), r.min_log, r.scale, QM1, QMAX);
             }
         } else {
@@ -1137,21 +1205,46 @@ fullrank_fast_kernel(const FullrankLaunch L)
 #pragma unroll
             for (int q = 0; q < FAST_EPT / 4; ++q) {
                 uint32_t kk[4];
+                const float4 v4 = stash_get<PB, P_OFF, G_OFF>(st, ow + q * 128);
+                const float x[4] = {v4.x, v4.y, v4.z, v4.w};
+                float lv[4];
+                uint32_t odd = 0u;                               // subnormal second moments above the floor of 1e-38
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float l = log2_lane(x[j], LT);         // (shuffles: every lane takes part)
+                    lv[j] = x[j] > AF8_TINY ? l : AF8_LOG2_TINY;
+                    if (x[j] > AF8_TINY && x[j] < 1.17549435e-38f) odd |= 1u << j;
+                }
+#pragma unroll 1
+                for (; odd; odd &= odd - 1u) {
+                    const int j = __ffs((int)odd) - 1;
+                    put(lv, j, log2_cr_fast(pick(x, j), s_log2));
+                }
 #pragma unroll
                 for (int j = 0; j < 4; j += 2) {
                     // al_encode on a pair: (l - min_log) / scale * 65534, rounded, plus one (optimizer.py:320-321)
-                    const int i = TABLE ? 0 : 4 * q + j;
-                    const float2 d = __fadd2_rn(make_float2(lv[i], lv[TABLE ? 0 : i + 1]), nml2);
+                    const float2 d = __fadd2_rn(make_float2(lv[j], lv[j + 1]), nml2);
                     const float2 q2 = div2_by(d, rc2, nd2);
                     // (below min_log: code 1, which the rounding constant would not give for a quotient of -2^6 and less)
                     const float2 t = make_float2(fmaxf(q2.x, 0.0f), fmaxf(q2.y, 0.0f));
                     // (scalar: the compiler fuses a packed product into a packed sum, which loses the rounding in between)
                     const int k0 = __float_as_int(__fadd_rn(__fmul_rn(t.x, QM1), AF8_MAGIC_F)) - (AF8_MAGIC_I - 1);
                     const int k1 = __float_as_int(__fadd_rn(__fmul_rn(t.y, QM1), AF8_MAGIC_F)) - (AF8_MAGIC_I - 1);
-                    kk[j] = v[4 * q + j] == 0.0f ? 0u : (uint32_t)min(k0, QMAX);
-                    kk[j + 1] = v[4 * q + j + 1] == 0.0f ? 0u : (uint32_t)min(k1, QMAX);
+                    kk[j] = x[j] == 0.0f ? 0u : (uint32_t)min(k0, QMAX);
+                    kk[j + 1] = x[j + 1] == 0.0f ? 0u : (uint32_t)min(k1, QMAX);
                 }
                 *reinterpret_cast<uint2 *>(vp + ow + q * 128) = make_uint2(kk[0] | (kk[1] << 16), kk[2] | (kk[3] << 16));
+            }
+        }
+        if (STASH) {
+            // the last warp to leave the slot has it refilled, for the block after the next one
+            __syncwarp();
+            if (lane == 0 && b + 2 * G < nfull) {
+                __threadfence_block();
+                if ((atomicAdd(&s_left, 1) & (FAST_WARPS - 1)) == FAST_WARPS - 1) {
+                    __threadfence_block();
+                    fast_issue<Ring, MF>(sT, s_ring, s_full, b, G, n, 2, 3);
+                }
             }
         }
         staged = next_staged;
