@@ -1396,6 +1396,9 @@ factored_stats_vec_kernel(const FactoredLaunch L, const int use_ring, const CUte
 // chunk = 2048 elements = 8 warps x 256; requires m_block == 256 when the momentum is quantised
 // PASS 0: a sum-of-squares pass (fewer values live, more resident CTAs); 1: the APPLY pass;
 // 2: the LAG pass (APPLY plus the sums of this step's raw update)
+// PT: the parameters.  0: binary32; 1, 2: bf16, rounded to nearest or stochastically, eight at a time in packed arithmetic (with
+// the element-wise function, whose 64-bit generator is 60 instructions, the momentum-free write pass over the TinyLlama set took
+// 4.25 ms stochastically against 2.32, and 3.75 against 2.54 to nearest with a momentum); 3: any 16-bit format, element by element.
 // CTAS: resident CTAs per SM asked of the compiler.  Measured on B200: 4 for the sum passes; for the
 // writing passes 3 with momentum (CAME, 0.78 ms per Llama-2-7B layer) and 2 without (Adafactor on the
 // TinyLlama set: 2.51 -> 2.21 ms, no register spills).
@@ -1406,7 +1409,7 @@ factored_stats_vec_kernel(const FactoredLaunch L, const int use_ring, const CUte
 // passes enter binary64 one by one, as in factored_update_kernel, which such tensors took before (but see sums_by_eight).  Write pass with bf16
 // gradients: 59 M parameters of odd sizes with a UF8 momentum 1 ms -> 252 us (issue and latency bound, 500 instructions
 // per 256 elements), 138 M in batches without momentum 1.55 ms -> 245 us (325 us with the tests of ANY = 2).
-template <typename GradT, int PASS, int CTAS, int ANY>
+template <typename GradT, int PASS, int CTAS, int ANY, int PT>
 __global__ void __launch_bounds__(FUPD_THREADS, CTAS)
 factored_update_vec_kernel(const FactoredLaunch L)
 {
@@ -1504,7 +1507,7 @@ factored_update_vec_kernel(const FactoredLaunch L)
         uint2 cm = make_uint2(0u, 0u);
         const bool pre_m = has_m && L.m_fmt == AF8_M_UF8 && L.mode != AF8_FUPD_SUMSQ_U;
         float *const pbase = static_cast<float *>(sT.param);
-        const bool lowp = L.param_dtype != AF8_F32;                  // 16-bit parameters: 8 of them in cp0
+        constexpr bool lowp = PT != 0;                               // 16-bit parameters: 8 of them in cp0
         const uint16_t *const hbase = static_cast<const uint16_t *>(sT.param);
         if (have) { cg = ng; cp0 = np0; cp1 = np1; cm = nm; }
         else if (partial) {
@@ -1660,6 +1663,22 @@ factored_update_vec_kernel(const FactoredLaunch L)
                     // stochastically (optimizer.py:873-881, 2033-2039)
                     const uint32_t w[4] = {__float_as_uint(cp0.x), __float_as_uint(cp0.y), __float_as_uint(cp0.z), __float_as_uint(cp0.w)};
                     uint32_t o[4];
+                    if constexpr (PT == 1 || PT == 2) {
+                        const float2 decay2 = bc2(sT.decay), step2 = bc2(step_mul), fira2 = bc2(fira);
+                        float2 x[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            x[j] = __fmul2_rn(make_float2(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xffff0000u)), decay2);
+                            if (PT == 1) {
+                                const uint32_t pk = bf16x2_rn(x[j].x, x[j].y);
+                                x[j] = make_float2(__uint_as_float(pk << 16), __uint_as_float(pk & 0xffff0000u));
+                            }
+                            float2 uu = __fmul2_rn(make_float2(u[2 * j], u[2 * j + 1]), fira2);
+                            if (zero_upd) uu = make_float2(0.0f, 0.0f);
+                            x[j] = __ffma2_rn(step2, uu, x[j]);
+                        }
+                        fast_round8<PT == 2, 0>(x, sT.sr_base, flat, 0, PT == 2 ? sr_counter(sT.sr_base, flat, 8) : SrCounter{}, o);
+                    } else
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
                         const uint32_t h = (j & 1) ? (w[j >> 1] >> 16) : (w[j >> 1] & 0xffffu);
@@ -2626,23 +2645,26 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
         AF8_CUDA_TRY(cudaGetLastError());
         return AF8_OK;
     }
+    // (see PT: bf16 gradients with bf16 parameters have kernels of their own)
+    const int pt = cfg->param_dtype == AF8_F32 ? 0 : (bf && cfg->param_dtype == AF8_BF16 && !lag) ? (cfg->stochastic_round ? 2 : 1) : 3;
+#define AF8_LAUNCH_FUPD(G, P, C, A, T) factored_update_vec_kernel<G, P, C, A, T><<<(int)grid, FUPD_THREADS, 0, cst>>>(L)
+#define AF8_LAUNCH_FUPD_PT(P, C, A) do { \
+        if (bf && pt == 0) AF8_LAUNCH_FUPD(bf16_tag, P, C, A, 0); else if (bf && pt == 3) AF8_LAUNCH_FUPD(bf16_tag, P, C, A, 3); \
+        else if (pt == 0) AF8_LAUNCH_FUPD(float, P, C, A, 0); else if (pt == 3) AF8_LAUNCH_FUPD(float, P, C, A, 3); \
+        else if (P == 1 && pt == 1) AF8_LAUNCH_FUPD(bf16_tag, 1, C, A, 1); else AF8_LAUNCH_FUPD(bf16_tag, 1, C, A, 2); } while (0)
+#define AF8_LAUNCH_FUPD_SUM(C, A) do { if (bf) AF8_LAUNCH_FUPD(bf16_tag, 0, C, A, 0); else AF8_LAUNCH_FUPD(float, 0, C, A, 0); } while (0)
     if (vec && any) {                            // (writing: 2 resident CTAs; the sum pass: 3)
         grid = std::min<int64_t>((int64_t)sm_count() * (apply ? 2 : 3), total_chunks);
-#define AF8_LAUNCH_FUPD(G, P, C) do { if (cfg->cols_mult8) factored_update_vec_kernel<G, P, C, 1><<<(int)grid, FUPD_THREADS, 0, cst>>>(L); \
-        else factored_update_vec_kernel<G, P, C, 2><<<(int)grid, FUPD_THREADS, 0, cst>>>(L); } while (0)
-        if (bf) { if (lag) AF8_LAUNCH_FUPD(bf16_tag, 2, 2); else if (apply) AF8_LAUNCH_FUPD(bf16_tag, 1, 2); else AF8_LAUNCH_FUPD(bf16_tag, 0, 3); }
-        else { if (lag) AF8_LAUNCH_FUPD(float, 2, 2); else if (apply) AF8_LAUNCH_FUPD(float, 1, 2); else AF8_LAUNCH_FUPD(float, 0, 3); }
-#undef AF8_LAUNCH_FUPD
-        AF8_CUDA_TRY(cudaGetLastError());
-        return AF8_OK;
+        if (lag) { if (cfg->cols_mult8) AF8_LAUNCH_FUPD_PT(2, 2, 1); else AF8_LAUNCH_FUPD_PT(2, 2, 2); }
+        else if (apply) { if (cfg->cols_mult8) AF8_LAUNCH_FUPD_PT(1, 2, 1); else AF8_LAUNCH_FUPD_PT(1, 2, 2); }
+        else if (cfg->cols_mult8) AF8_LAUNCH_FUPD_SUM(3, 1);
+        else AF8_LAUNCH_FUPD_SUM(3, 2);
     }
-#define AF8_LAUNCH_FUPD(G, P, C) factored_update_vec_kernel<G, P, C, 0><<<(int)grid, FUPD_THREADS, 0, cst>>>(L)
-    if (vec && bf && lag) { if (no_m) AF8_LAUNCH_FUPD(bf16_tag, 2, 2); else AF8_LAUNCH_FUPD(bf16_tag, 2, 3); }
-    else if (vec && lag) { if (no_m) AF8_LAUNCH_FUPD(float, 2, 2); else AF8_LAUNCH_FUPD(float, 2, 3); }
-    else if (vec && bf && apply) { if (no_m) AF8_LAUNCH_FUPD(bf16_tag, 1, 2); else AF8_LAUNCH_FUPD(bf16_tag, 1, 3); }
-    else if (vec && bf) AF8_LAUNCH_FUPD(bf16_tag, 0, 4);
-    else if (vec && apply) { if (no_m) AF8_LAUNCH_FUPD(float, 1, 2); else AF8_LAUNCH_FUPD(float, 1, 3); }
-    else if (vec) AF8_LAUNCH_FUPD(float, 0, 4);
+    else if (vec && lag) { if (no_m) AF8_LAUNCH_FUPD_PT(2, 2, 0); else AF8_LAUNCH_FUPD_PT(2, 3, 0); }
+    else if (vec && apply) { if (no_m) AF8_LAUNCH_FUPD_PT(1, 2, 0); else AF8_LAUNCH_FUPD_PT(1, 3, 0); }
+    else if (vec) AF8_LAUNCH_FUPD_SUM(4, 0);
+#undef AF8_LAUNCH_FUPD_SUM
+#undef AF8_LAUNCH_FUPD_PT
 #undef AF8_LAUNCH_FUPD
     else factored_update_kernel<<<(int)grid, FUPD_THREADS, smem, static_cast<cudaStream_t>(stream)>>>(L, chunk);
     AF8_CUDA_TRY(cudaGetLastError());

@@ -656,9 +656,9 @@ __device__ __forceinline__ void fast_store_m(const float2 (&m)[4], uint8_t *m_q,
     if (lane == 0) *m_scale = am;
 }
 
-// The 16-bit patterns of eight new bf16 parameters (elements o .. o + 3 and o + 128 .. of the block that starts at base): the
+// The 16-bit patterns of eight new bf16 parameters (elements o .. o + 3 and o + 4 + GAP .. of the run that starts at base): the
 // last rounding, to nearest or stochastic (optimizer.py:873-881).
-template <bool SR>
+template <bool SR, int GAP = 124>
 __device__ __forceinline__ void fast_round8(const float2 (&p)[4], uint64_t sr_base, int64_t base, int o, const SrCounter &counter, uint32_t (&w)[4])
 {
     if (!SR) {
@@ -669,7 +669,7 @@ __device__ __forceinline__ void fast_round8(const float2 (&p)[4], uint64_t sr_ba
     float top = 0.0f;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        const uint32_t k = (uint32_t)(o + (j < 2 ? 0 : 124) + 2 * j);
+        const uint32_t k = (uint32_t)(o + (j < 2 ? 0 : GAP) + 2 * j);
         w[j] = sr_bf16x2(p[j].x, p[j].y, sr_hi32(counter, k), sr_hi32(counter, k + 1u));
         top = max3_nan(top, fabsf(p[j].x), fabsf(p[j].y));
     }
@@ -677,7 +677,7 @@ __device__ __forceinline__ void fast_round8(const float2 (&p)[4], uint64_t sr_ba
         const float x[8] = {p[0].x, p[0].y, p[1].x, p[1].y, p[2].x, p[2].y, p[3].x, p[3].y};
 #pragma unroll 1
         for (int k = 0; k < 4; ++k) {
-            const uint64_t i = (uint64_t)(base + o + (k < 2 ? 0 : 124) + 2 * k);
+            const uint64_t i = (uint64_t)(base + o + (k < 2 ? 0 : GAP) + 2 * k);
             put(w, k, sr_bf16_bits(pick(x, 2 * k), sr_bits24(sr_base, i)) | (sr_bf16_bits(pick(x, 2 * k + 1), sr_bits24(sr_base, i + 1)) << 16));
         }
     }
