@@ -283,6 +283,31 @@ __device__ __forceinline__ float al8_decode_fast(uint32_t code, float scale, flo
     return STRICT && t > 150.0f ? t : exp2_cr_fast(t, tab);
 }
 
+// The tables of the short sequences in global memory, for kernels whose few CTAs copy them into shared memory first: lanes that
+// read different constants take turns, which costs a short kernel more than its work.
+__device__ const double g_exp2_tab[32] = AF8_EXP2_TAB;
+__device__ const double2 g_log2_tab[97] = {
+#include "log2_table.inc"
+};
+struct CodecTables { double exp2[32]; double2 log2[97]; };
+__device__ __forceinline__ void load_codec_tables(CodecTables &t)      // (every thread of the CTA; a barrier follows)
+{
+    if (threadIdx.x < 97) t.log2[threadIdx.x] = g_log2_tab[threadIdx.x];
+    if (threadIdx.x < 32) t.exp2[threadIdx.x] = g_exp2_tab[threadIdx.x];
+}
+// al_decode and al_log2 with the short sequences: the same numbers.  (Exponents beyond the short sequence's range, as of blocks
+// that held infinities, take the library's function; the short logarithm gives 1024 for an infinity.)
+__device__ __forceinline__ float al_decode_tab(uint32_t code, float scale, float min_log, float qm1, const CodecTables &t)
+{
+    if (code == 0) return 0.0f;
+    const float x = __fadd_rn(__fdiv_rn(__fmul_rn((float)(code - 1), scale), qm1), min_log);
+    return fabsf(x) <= 150.0f ? exp2_cr_fast(x, t.exp2) : exp2_cr(x);
+}
+__device__ __forceinline__ float al_log2_tab(float v, const CodecTables &t)
+{
+    return v > 3.402823466e38f ? INFINITY : al_log2_fast(v, t.log2);
+}
+
 // Block range of _log_quantize_nonneg from the reduced extrema
 // (optimizer.py:315-318).  mn = min of log2 over non-zero elements (+inf if
 // none), mx = max over all elements.
@@ -338,6 +363,27 @@ __device__ __forceinline__ float warp_min(float x)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) x = fminf(x, __shfl_xor_sync(0xffffffffu, x, o));
     return x;
+}
+
+__device__ __forceinline__ double warp_sum(double x)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+
+// Sum over the block of f(i), i = 0 .. n - 1, in a fixed order; the value is thread 0's.  Four loads are in flight per thread.
+template <int THREADS, typename F>
+__device__ __forceinline__ double block_sum(int64_t n, F f, double (&part)[THREADS / 32])
+{
+    double acc = 0.0;
+#pragma unroll 4
+    for (int64_t i = threadIdx.x; i < n; i += THREADS) acc += f(i);
+    acc = warp_sum(acc);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x < 32) acc = warp_sum(threadIdx.x < THREADS / 32 ? part[threadIdx.x] : 0.0);
+    return acc;
 }
 
 __device__ __forceinline__ float warp_sum(float x)

@@ -356,12 +356,13 @@ factored_clear_kernel(const af8_factored_tensor *tensors)
 // ---------------------------------------------------------------------------
 // small states
 // ---------------------------------------------------------------------------
-constexpr int SMALL_MAX_THREADS = 512;
+constexpr int SMALL_MAX_THREADS = 1024;
+constexpr int SMALL_KEPT = 2048;        // logarithms of a block that wait for its range in shared memory; those of longer blocks are taken again
 // EMA + requantisation of block b of one small state of n elements (optimizer.py:2232-2238,
 // 937-946, 2248-2251).  `out` receives the un-requantised values.  Returns this thread's partial
 // sum of the block's values (binary64) for the mean of the row state.
-__device__ double small_state_block(const af8_small_state &S, const double *sums, double count, int64_t n, int64_t b,
-                                    float eps_add, float w, float floor_log, float *out, float *s_l, float (*s_red)[SMALL_MAX_THREADS / 32])
+__device__ __forceinline__ double small_state_block(const af8_small_state &S, const double *sums, double count, int64_t n, int64_t b,
+                                    float eps_add, float w, float floor_log, float *out, const CodecTables &tab, float *s_l, float (*s_red)[SMALL_MAX_THREADS / 32])
 {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int block = S.block;
@@ -382,20 +383,23 @@ __device__ double small_state_block(const af8_small_state &S, const double *sums
     const int qmax = bits == 16 ? 65535 : 255;
     const float sc = S.scale[b], ml = S.min_log[b];
     float mn = INFINITY, mx = -INFINITY;
+    // (rolled: the few CTAs of this launch fetch the code for the first time, which unrolled copies made the longest part)
+#pragma unroll 1
     for (int i = tid; i < block; i += blockDim.x) {
         const int64_t e = b * block + i;
         float v = 0.0f;                                       // padding re-enters as zeros (optimizer.py:303-305)
         if (e < n) {
             const uint32_t code = bits == 16 ? static_cast<const uint16_t *>(S.q)[e] : static_cast<const uint8_t *>(S.q)[e];
             const float nv = __fadd_rn(__double2float_rn(sums[e] / count), eps_add);
-            v = lerp_t(al_decode(code, sc, ml, qm1), nv, w);
+            v = lerp_t(al_decode_tab(code, sc, ml, qm1, tab), nv, w);
             out[e] = v;
             acc += (double)v;
         }
-        const float l = al_log2(v);
-        if (v != 0.0f) mn = fminf(mn, l);
+        float l = al_log2_tab(v, tab);
         mx = fmaxf(mx, l);
-        s_l[i] = (v != 0.0f) ? l : -INFINITY;
+        if (v != 0.0f) mn = fminf(mn, l);
+        else l = -INFINITY;
+        if (i < SMALL_KEPT) s_l[i] = l;
     }
     mn = warp_min(mn);
     mx = warp_max(mx);
@@ -404,10 +408,16 @@ __device__ double small_state_block(const af8_small_state &S, const double *sums
     for (int k = 0; k < (int)(blockDim.x >> 5); ++k) { mn = fminf(mn, s_red[0][k]); mx = fmaxf(mx, s_red[1][k]); }
     float min_log, scale;
     al_range(mn, mx, floor_log, min_log, scale);
+#pragma unroll 1
     for (int i = tid; i < block; i += blockDim.x) {
-        const float l = s_l[i];
-        const uint32_t code = (l == -INFINITY) ? 0u : al_encode(1.0f, l, min_log, scale, qm1, qmax);
         const int64_t e = b * block + i;
+        float l;
+        if (i < SMALL_KEPT) l = s_l[i];
+        else {                                                // (this thread's own value again)
+            const float v = e < n ? out[e] : 0.0f;
+            l = v != 0.0f ? al_log2_tab(v, tab) : -INFINITY;
+        }
+        const uint32_t code = (l == -INFINITY) ? 0u : al_encode(1.0f, l, min_log, scale, qm1, qmax);
         if (bits == 16) static_cast<uint16_t *>(S.q)[e] = (uint16_t)code;
         else static_cast<uint8_t *>(S.q)[e] = (uint8_t)code;
     }
@@ -427,33 +437,35 @@ __device__ __forceinline__ int find_factored_small(const af8_factored_tensor *t,
 
 // One CTA per quantisation block of a row or column state: every block of every tensor in
 // parallel (a 32000-row state has 125 blocks of 256; one CTA per tensor walked them in turn).
-// A thread walks block / THREADS elements with binary64 logarithms.
+// A thread walks block / THREADS elements with binary64 exponentials and logarithms: the short sequences with their tables in
+// shared memory (the 3346 units of the TinyLlama set: 39 us with the library's functions and 32 KB of shared memory per CTA, 32).
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS)
 factored_small_kernel(const af8_factored_tensor *tensors, int n_tensors, int conf, float floor_log)
 {
-    extern __shared__ float s_l[];
+    __shared__ CodecTables s_codec;
+    __shared__ float s_l[SMALL_KEPT];
     __shared__ float s_red[2][SMALL_MAX_THREADS / 32];
     __shared__ double s_acc[SMALL_MAX_THREADS / 32];
+    load_codec_tables(s_codec);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int t = find_factored_small(tensors, n_tensors, (int)blockIdx.x);
-    const af8_factored_tensor T = tensors[t];
+    const af8_factored_tensor &T = tensors[t];
     const int block = (conf ? T.conf_row : T.row_var).block;
-    const int64_t nbr = (T.rows + block - 1) / block;
+    const int64_t rows = T.rows, nbr = (rows + block - 1) / block;
     const int64_t local = (int64_t)blockIdx.x - T.first_small;
     const bool is_row = local < nbr;
     const int64_t b = is_row ? local : local - nbr;
-    const float w = conf ? T.c_w : T.v_w;
-    const float eps_add = conf ? 0.0f : T.eps1;                 // optimizer.py:2222-2223 vs 933-934
-    double part;
     // a batch of matrices: the states are flat over the batch (their blocks run across the matrices); a
     // column value is the mean over the rows of its own matrix
-    if (is_row)
-        part = small_state_block(conf ? T.conf_row : T.row_var, T.row_sum, (double)T.cols, T.rows, b, eps_add, w, floor_log,
-                                 conf ? T.inv_row_conf : T.inv_row, s_l, s_red);
-    else
-        part = small_state_block(conf ? T.conf_col : T.col_var, T.col_sum, (double)fact_mat_rows(T), fact_batch(T) * T.cols, b, eps_add, w, floor_log,
-                                 conf ? T.inv_col_conf : T.inv_col, s_l, s_red);
+    const af8_small_state &S = is_row ? (conf ? T.conf_row : T.row_var) : (conf ? T.conf_col : T.col_var);
+    float *const out = is_row ? (conf ? T.inv_row_conf : T.inv_row) : (conf ? T.inv_col_conf : T.inv_col);
+    const double *const sums = is_row ? T.row_sum : T.col_sum;
+    const double count = is_row ? (double)T.cols : (double)fact_mat_rows(T);
+    const float eps_add = conf ? 0.0f : T.eps1;                 // optimizer.py:2222-2223 vs 933-934
+    __syncthreads();
+    double part = small_state_block(S, sums, count, is_row ? rows : fact_batch(T) * T.cols, b, eps_add, conf ? T.c_w : T.v_w, floor_log,
+                                    out, s_codec, s_l, s_red);
     if (!is_row) return;
     // the block's share of the mean of the row state goes where its first row sum was
 #pragma unroll
@@ -502,16 +514,19 @@ factored_inv_kernel(const af8_factored_tensor *tensors, int conf)
         for (int64_t j = first; j < nb * T.cols; j += stride) inv_c[j] = rsqrt_t(inv_c[j]);
         return;
     }
-    if (tid == 0) {
+    if (tid < 32) {                                                         // (fixed order; one thread took 30 us for the 125 blocks of 32000 rows)
         double s = 0.0;
-        for (int64_t e = 0; e < T.rows; e += block) s += T.row_sum[e];      // fixed order
+        for (int64_t e = (int64_t)tid * block; e < T.rows; e += 32 * (int64_t)block) s += T.row_sum[e];
+        s = warp_sum(s);
         float rm = __double2float_rn(s / (double)T.rows);
         if (rm < T.eps1) rm = T.eps1;
-        s_rm = rm;
+        if (tid == 0) s_rm = rm;
     }
     __syncthreads();
     const float rm = s_rm;
+#pragma unroll 4
     for (int64_t i = first; i < T.rows; i += stride) inv_r[i] = rsqrt_t(__fdiv_rn(inv_r[i], rm));
+#pragma unroll 4
     for (int64_t j = first; j < T.cols; j += stride) inv_c[j] = rsqrt_t(inv_c[j]);
 }
 
@@ -2543,12 +2558,11 @@ extern "C" int af8_factored_small(const af8_factored_cfg *cfg, const af8_factore
     if (rc) return rc;
     if (!dev_tensors || n_tensors <= 0 || total_units <= 0) return fail(AF8_ERR_INVALID, "af8_factored_small: null or empty table");
     if (conf && !cfg->came) return fail(AF8_ERR_INVALID, "af8_factored_small: confidence states exist only with CAME");
-    const size_t smem = sizeof(float) * GEN_MAX_BLOCK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // at most one unit per SM (blocks of 2048, few tensors): the launch lasts as long as one CTA, so more threads
-    // (8 layers of 512 x 1376 with CAME: 12.3 -> 10 us a launch; 480 units of 256 elements: 6.2 us with 256, 14 with 512)
-    if (total_units <= sm_count()) factored_small_kernel<SMALL_MAX_THREADS><<<total_units, SMALL_MAX_THREADS, smem, st>>>(dev_tensors, n_tensors, conf, cfg->v_floor);
-    else factored_small_kernel<256><<<total_units, 256, smem, st>>>(dev_tensors, n_tensors, conf, cfg->v_floor);
+    // (8 layers of 512 x 1376 with CAME: 12.3 us a launch with 256, 11.5 with 1024; 480 units of 256 elements: 6.2 us with 256, 14 with 512)
+    if (total_units <= sm_count()) factored_small_kernel<SMALL_MAX_THREADS><<<total_units, SMALL_MAX_THREADS, 0, st>>>(dev_tensors, n_tensors, conf, cfg->v_floor);
+    else factored_small_kernel<256><<<total_units, 256, 0, st>>>(dev_tensors, n_tensors, conf, cfg->v_floor);
     AF8_CUDA_TRY(cudaGetLastError());
     factored_inv_kernel<<<dim3((unsigned)n_tensors, 8), 256, 0, st>>>(dev_tensors, conf);
     AF8_CUDA_TRY(cudaGetLastError());

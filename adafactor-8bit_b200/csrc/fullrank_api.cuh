@@ -19,29 +19,22 @@ namespace af8 {
 // _apply_fira_pytorch / _safe_rms_denom (optimizer.py:805-806, 859-863) and
 // -alpha/denom (optimizer.py:874); in pre_div_mode 1 the RMS clip of the
 // momentum-only rule (optimizer.py:897-899).
-__global__ void __launch_bounds__(256)
+// 1024 threads: the largest tensor of the table decides how long the launch lasts (65.5 M elements, 32000 partial sums:
+// 21 us with 256 threads, 13 with 1024 in binary64).
+constexpr int FINALIZE_THREADS = 1024;
+__global__ void __launch_bounds__(FINALIZE_THREADS)
 norm_finalize_kernel(const af8_norm_tensor *tensors, const void *block_sumsq, af8_dyn_scalars *dyn)
 {
-    __shared__ double s_acc[256];
+    __shared__ double s_part[FINALIZE_THREADS / 32];
     const af8_norm_tensor T = tensors[blockIdx.x];
-    const int tid = threadIdx.x;
-    double acc = 0.0;
-    if (T.partials_f64) {
-        const double *ps = static_cast<const double *>(block_sumsq);
-        for (int64_t i = tid; i < T.n_blocks; i += 256) acc += ps[T.first_block + i];
-    } else {
-        const float *ps = static_cast<const float *>(block_sumsq);
-        for (int64_t i = tid; i < T.n_blocks; i += 256) acc += (double)ps[T.first_block + i];
-    }
-    s_acc[tid] = acc;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (tid < o) s_acc[tid] += s_acc[tid + o];
-        __syncthreads();
-    }
-    if (tid != 0) return;
+    const double *const p64 = static_cast<const double *>(block_sumsq) + T.first_block;
+    const float *const p32 = static_cast<const float *>(block_sumsq) + T.first_block;
+    const double sum = T.n_blocks < 0 ? 0.0
+                     : T.partials_f64 ? block_sum<FINALIZE_THREADS>(T.n_blocks, [=](int64_t i) { return p64[i]; }, s_part)
+                                      : block_sum<FINALIZE_THREADS>(T.n_blocks, [=](int64_t i) { return (double)p32[i]; }, s_part);
+    if (threadIdx.x != 0) return;
 
-    const double total = T.n_blocks < 0 ? *reinterpret_cast<const double *>(static_cast<uintptr_t>(T.first_block)) : s_acc[0];
+    const double total = T.n_blocks < 0 ? *reinterpret_cast<const double *>(static_cast<uintptr_t>(T.first_block)) : sum;
     float norm = __double2float_rn(sqrt(total));
     const float alpha = T.alpha_dev ? *T.alpha_dev : T.alpha;
     af8_dyn_scalars out = dyn[blockIdx.x];
@@ -85,10 +78,10 @@ norm_finalize_kernel(const af8_norm_tensor *tensors, const void *block_sumsq, af
 }
 
 // One CTA per tensor: the scalars of the one-step-lag variant (af8_lag_scalars).
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(FINALIZE_THREADS)
 lag_scalars_kernel(const af8_lag_tensor *tensors, int phase, const void *block_sumsq, af8_dyn_scalars *dyn)
 {
-    __shared__ double s_acc[256];
+    __shared__ double s_part[FINALIZE_THREADS / 32];
     const af8_lag_tensor T = tensors[blockIdx.x];
     const int tid = threadIdx.x;
     if (phase == 0) {
@@ -106,22 +99,12 @@ lag_scalars_kernel(const af8_lag_tensor *tensors, int phase, const void *block_s
         dyn[blockIdx.x] = out;
         return;
     }
-    double acc = 0.0;
-    if (T.partials_f64) {
-        const double *ps = static_cast<const double *>(block_sumsq);
-        for (int64_t i = tid; i < T.n_blocks; i += 256) acc += ps[T.first_block + i];
-    } else {
-        const float *ps = static_cast<const float *>(block_sumsq);
-        for (int64_t i = tid; i < T.n_blocks; i += 256) acc += (double)ps[T.first_block + i];
-    }
-    s_acc[tid] = acc;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (tid < o) s_acc[tid] += s_acc[tid + o];
-        __syncthreads();
-    }
+    const double *const p64 = static_cast<const double *>(block_sumsq) + T.first_block;
+    const float *const p32 = static_cast<const float *>(block_sumsq) + T.first_block;
+    const double sum = T.partials_f64 ? block_sum<FINALIZE_THREADS>(T.n_blocks, [=](int64_t i) { return p64[i]; }, s_part)
+                                      : block_sum<FINALIZE_THREADS>(T.n_blocks, [=](int64_t i) { return (double)p32[i]; }, s_part);
     if (tid != 0) return;
-    const float raw = __double2float_rn(sqrt(s_acc[0]));
+    const float raw = __double2float_rn(sqrt(sum));
     *T.prev_update_norm = raw;                                                              // optimizer.py:1066-1067
     dyn[blockIdx.x].norm = raw;
     if (T.lag_fira_scale == nullptr || T.fira_prev == nullptr) return;
@@ -208,7 +191,7 @@ template <typename GradT, int MODE>
 inline int launch_generic(const FullrankLaunch &L, const GenericCfg &C, cudaStream_t st)
 {
     const bool plain = (C.v_fmt == AF8_V_FP32 || C.v_fmt == AF8_V_NONE) && (C.m_fmt == AF8_M_NONE || C.m_fmt == AF8_M_FP32);
-    return plain && L.total_blocks <= 2 * (int64_t)sm_count() ? launch_generic_threads<GradT, MODE, 1024>(L, C, plain, st)
+    return L.total_blocks <= 2 * (int64_t)sm_count() ? launch_generic_threads<GradT, MODE, 1024>(L, C, plain, st)
                                                               : launch_generic_threads<GradT, MODE, GEN_THREADS>(L, C, plain, st);
 }
 
@@ -449,7 +432,7 @@ extern "C" int af8_lag_scalars(const af8_lag_tensor *tensors, int32_t n_tensors,
     if (n_tensors <= 0) return fail(AF8_ERR_INVALID, "af8_lag_scalars: n_tensors must be positive");
     if (phase != 0 && phase != 1) return fail(AF8_ERR_INVALID, "af8_lag_scalars: phase must be 0 or 1");
     if (phase == 1 && !block_sumsq) return fail(AF8_ERR_INVALID, "af8_lag_scalars: phase 1 needs block_sumsq");
-    lag_scalars_kernel<<<n_tensors, 256, 0, static_cast<cudaStream_t>(stream)>>>(tensors, phase, block_sumsq, dyn);
+    lag_scalars_kernel<<<n_tensors, FINALIZE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(tensors, phase, block_sumsq, dyn);
     AF8_CUDA_TRY(cudaGetLastError());
     return AF8_OK;
 }
@@ -460,7 +443,7 @@ extern "C" int af8_norm_finalize(const af8_norm_tensor *tensors, int32_t n_tenso
     using namespace af8;
     if (!tensors || !block_sumsq || !dyn) return fail(AF8_ERR_INVALID, "af8_norm_finalize: null argument");
     if (n_tensors <= 0) return fail(AF8_ERR_INVALID, "af8_norm_finalize: n_tensors must be positive");
-    norm_finalize_kernel<<<n_tensors, 256, 0, static_cast<cudaStream_t>(stream)>>>(tensors, block_sumsq, dyn);
+    norm_finalize_kernel<<<n_tensors, FINALIZE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(tensors, block_sumsq, dyn);
     AF8_CUDA_TRY(cudaGetLastError());
     return AF8_OK;
 }

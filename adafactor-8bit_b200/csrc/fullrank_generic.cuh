@@ -84,9 +84,10 @@ __device__ __forceinline__ uint32_t m_encode(float m, float a, int fmt)
 // MODE: AF8_MODE_NOCLIP / SUMSQ / APPLY, plus 3 = SUMSQ of the momentum update
 // on the momentum-only path (reads dyn.pre_div like APPLY, writes nothing but
 // the partial sums).
-// THREADS: 256, or 1024 where neither state is quantised and there are at most two blocks per SM (the norm vectors and
-// biases of a model, tensors of a few thousand elements): each of the few CTAs walked its block in eight dependent rounds
-// of loads.  45 vectors of 2048 elements: 23 -> 9 us in one pass, 19 + 16 -> 9 + 8 us in two.
+// THREADS: 256, or 1024 where there are at most two blocks per SM (the norm vectors and biases of a model, tensors of a few
+// thousand elements): each of the few CTAs walked its block in eight dependent rounds of loads.  45 vectors of 2048 elements
+// with binary32 states: 23 -> 9 us in one pass, 19 + 16 -> 9 + 8 us in two; 9 vectors of 4096 elements with UF8 / AL16 states
+// 22 + 32 -> 10 + 14 us in two (the short exponentials and logarithms with their tables in shared memory included).
 template <typename GradT, int MODE, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 fullrank_generic_kernel(const FullrankLaunch L, const GenericCfg C)
@@ -96,6 +97,7 @@ fullrank_generic_kernel(const FullrankLaunch L, const GenericCfg C)
     float *s_m = s_dyn + C.block;       // new momentum
     __shared__ af8_fullrank_tensor sT;
     __shared__ float s_red[3][THREADS / 32];
+    __shared__ CodecTables s_codec;
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
@@ -110,6 +112,7 @@ fullrank_generic_kernel(const FullrankLaunch L, const GenericCfg C)
     const float qm1 = (C.v_fmt == AF8_V_AL16) ? 65534.0f : 254.0f;
     const int qmax = (C.v_fmt == AF8_V_AL16) ? 65535 : 255;
     int cur_t = -1;
+    if (v_quant) load_codec_tables(s_codec);
 
     for (int64_t blk = blockIdx.x; blk < L.total_blocks; blk += gridDim.x) {
         int t = cur_t;
@@ -158,7 +161,7 @@ fullrank_generic_kernel(const FullrankLaunch L, const GenericCfg C)
                     uint32_t code = (C.v_fmt == AF8_V_AL16)
                                         ? static_cast<const uint16_t *>(sT.v_q)[base + i]
                                         : static_cast<const uint8_t *>(sT.v_q)[base + i];
-                    const float v_old = al_decode(code, v_scale, v_min_log, qm1);
+                    const float v_old = al_decode_tab(code, v_scale, v_min_log, qm1, s_codec);
                     const float g2 = __fadd_rn(__fmul_rn(gj, gj), sT.eps_gradsq);
                     vj = lerp_t(v_old, g2, sT.v_w);
                 } else if (sT.v_keep < 0.0f) {   // fp32 state updated with Tensor.lerp_ (APOLLO's low-rank V, optimizer.py:2797-2799)
@@ -226,7 +229,7 @@ fullrank_generic_kernel(const FullrankLaunch L, const GenericCfg C)
             }
             if (writes) {
                 if (v_quant) {
-                    const float l = al_log2(vj);
+                    const float l = al_log2_tab(vj, s_codec);
                     if (vj != 0.0f) mn = fminf(mn, l);
                     mx = fmaxf(mx, l);
                     s_l[i] = (vj != 0.0f) ? l : -INFINITY;

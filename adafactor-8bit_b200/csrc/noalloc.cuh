@@ -171,7 +171,7 @@ extern "C" int af8_fullrank_limited_step_noalloc(const af8_fullrank_cfg *cfg, co
     };
     rc = pass(AF8_MODE_SUMSQ);
     if (rc) return rc;
-    norm_finalize_kernel<<<1, 256, 0, st>>>(d_norm, d_sumsq, d_dyn);
+    norm_finalize_kernel<<<1, FINALIZE_THREADS, 0, st>>>(d_norm, d_sumsq, d_dyn);
     AF8_CUDA_TRY(cudaGetLastError());
     rc = pass(AF8_MODE_APPLY);
     if (rc) return rc;

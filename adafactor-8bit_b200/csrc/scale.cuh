@@ -52,21 +52,20 @@ param_sumsq_kernel(const ScaleLaunch L)
                 acc = __fmaf_rn(v.z, v.z, acc); acc = __fmaf_rn(v.w, v.w, acc);
             }
         } else if (rem >= SCALE_CHUNK) {
-            // bf16 / fp16 parameters enter the norm as binary32 (vector_norm(..., dtype=float32), optimizer.py:850-851)
-            const uint2 *p2 = reinterpret_cast<const uint2 *>(static_cast<const uint16_t *>(p) + base);
+            // bf16 / fp16 parameters enter the norm as binary32 (vector_norm(..., dtype=float32), optimizer.py:850-851);
+            // 128-bit loads as above (64-bit ones: 593 us on the TinyLlama set, 3.7 TB/s)
+            const uint4 *p8 = reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(p) + base);
 #pragma unroll
-            for (int k = 0; k < SCALE_CHUNK / 4 / 256; ++k) {
-                const uint2 w = p2[tid + k * 256];
-                float v[4];
-                if (pdt == AF8_BF16) {
-                    v[0] = __uint_as_float(w.x << 16); v[1] = __uint_as_float(w.x & 0xffff0000u);
-                    v[2] = __uint_as_float(w.y << 16); v[3] = __uint_as_float(w.y & 0xffff0000u);
-                } else {
-                    v[0] = f16_bits_to_f32(w.x & 0xffffu); v[1] = f16_bits_to_f32(w.x >> 16);
-                    v[2] = f16_bits_to_f32(w.y & 0xffffu); v[3] = f16_bits_to_f32(w.y >> 16);
+            for (int k = 0; k < SCALE_CHUNK / 8 / 256; ++k) {
+                const uint4 q = p8[tid + k * 256];
+                const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float lo = pdt == AF8_BF16 ? __uint_as_float(w[j] << 16) : f16_bits_to_f32(w[j] & 0xffffu);
+                    const float hi = pdt == AF8_BF16 ? __uint_as_float(w[j] & 0xffff0000u) : f16_bits_to_f32(w[j] >> 16);
+                    acc = __fmaf_rn(lo, lo, acc);
+                    acc = __fmaf_rn(hi, hi, acc);
                 }
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc = __fmaf_rn(v[j], v[j], acc);
             }
         } else {
             for (int i = tid; i < rem; i += 256) { const float v = param_load(p, base + i, pdt); acc = __fmaf_rn(v, v, acc); }
@@ -84,24 +83,17 @@ param_sumsq_kernel(const ScaleLaunch L)
 }
 
 // one CTA per tensor: fixed-order binary64 reduction, then the scalar chain
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(1024)
 param_scale_finalize_kernel(const af8_scale_tensor *tensors, const float *block_sumsq,
                             uint8_t *table, int64_t stride, int64_t alpha_off, int64_t decay_off)
 {
-    __shared__ double s_acc[256];
+    __shared__ double s_part[32];
     const af8_scale_tensor T = tensors[blockIdx.x];
-    const int tid = threadIdx.x;
     const int64_t n_chunks = (T.numel + SCALE_CHUNK - 1) / SCALE_CHUNK;
-    double acc = 0.0;
-    for (int64_t i = tid; i < n_chunks; i += 256) acc += (double)block_sumsq[T.first_chunk + i];
-    s_acc[tid] = acc;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (tid < o) s_acc[tid] += s_acc[tid + o];
-        __syncthreads();
-    }
-    if (tid != 0) return;
-    const float norm = __double2float_rn(sqrt(T.total ? *T.total : s_acc[0]));
+    const float *const ps = block_sumsq + T.first_chunk;
+    const double sum = block_sum<1024>(n_chunks, [=](int64_t i) { return (double)ps[i]; }, s_part);
+    if (threadIdx.x != 0) return;
+    const float norm = __double2float_rn(sqrt(T.total ? *T.total : sum));
     const float rms = __fdiv_rn(norm, T.sqrt_n);                    // optimizer.py:851-852
     float alpha = __fmul_rn(fmaxf(rms, T.eps2), T.rho);             // optimizer.py:853
     if (T.bc_mode == 1) alpha = __fmul_rn(alpha, T.bc);             // optimizer.py:2026
@@ -158,7 +150,7 @@ extern "C" int af8_param_scale_finish(const af8_scale_tensor *dev_tensors, int32
     if (!dev_tensors || !chunk_sumsq || !dev_table) return fail(AF8_ERR_INVALID, "af8_param_scale_finish: null argument");
     if (n_tensors <= 0) return fail(AF8_ERR_INVALID, "af8_param_scale_finish: n_tensors must be positive");
     if (!param_scale_layout_ok(table_stride, alpha_offset, decay_offset)) return fail(AF8_ERR_INVALID, "af8_param_scale_finish: bad table layout");
-    param_scale_finalize_kernel<<<n_tensors, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+    param_scale_finalize_kernel<<<n_tensors, 1024, 0, static_cast<cudaStream_t>(stream)>>>(
         dev_tensors, chunk_sumsq, static_cast<uint8_t *>(dev_table), table_stride, alpha_offset, decay_offset);
     AF8_CUDA_TRY(cudaGetLastError());
     return AF8_OK;

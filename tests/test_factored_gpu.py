@@ -97,6 +97,12 @@ EXTRA_CASES.update({
                                grad=cases.CASES["adafactor_factored_m"]["grad"], hp=cases.CASES["adafactor_factored_m"]["hp"]),
 })
 
+# small states in blocks longer than what waits in shared memory, of either width, and norm vectors of the general kernel beside them
+EXTRA_CASES["came_long_blocks"] = dict(shapes=[(5000, 16), (40, 9001), (4100,)], steps=3, seed=63, grad=cases.CASES["came_al16"]["grad"],
+                                       hp=dict(cases.CASES["came_al16"]["hp"], block_size=4096))
+EXTRA_CASES["adafactor_long_blocks"] = dict(shapes=[(5000, 16), (40, 9001)], steps=3, seed=64, grad=cases.CASES["adafactor_factored"]["grad"],
+                                            hp=dict(cases.CASES["adafactor_factored"]["hp"], block_size=8192, v_quant_type="al8"))
+
 # lag_norm=True (one pass with the previous step's norm; optimizer.py:1056-1071): the vector kernels, the
 # element-wise kernels (odd column counts) and the limiter on top of the clip
 EXTRA_CASES.update({
