@@ -1011,15 +1011,6 @@ __device__ __forceinline__ void stats_rows(const FactoredLaunch &L, const af8_fa
     }
 }
 
-// The same rows with the inputs of every row slice (256 columns: 512 or 1024 bytes of gradient and,
-// for the residual, 256 momentum codes) requested SR_STAGES slices ahead by the warp's lane 0 with
-// cp.async.bulk into the warp's own ring (one mbarrier per stage).  Needs cols % 256 == 0 (whole
-// slices, 16-byte aligned runs) and, for the residual, a UF8 momentum.  NB rows are consumed per
-// iteration so that their row sums are reduced jointly, as above.  Returns false after a time-out.
-template <typename GradT> __host__ __device__ constexpr int sring_stages() { return sizeof_grad<GradT>() == 2 ? 8 : 4; }
-template <typename GradT, bool RESIDUAL> __host__ __device__ constexpr int sring_stage_bytes() { return 256 * sizeof_grad<GradT>() + (RESIDUAL ? 256 : 0); }
-template <typename GradT, bool RESIDUAL> __host__ __device__ constexpr size_t sring_smem_bytes() { return (size_t)8 * sring_stages<GradT>() * sring_stage_bytes<GradT, RESIDUAL>(); }
-
 // 8 UF8 codes of one momentum block as floats: (code - 128) * mc, two elements per instruction; each
 // component rounds like the scalar form in m_old8
 __device__ __forceinline__ void uf8_decode8(uint2 w, float mc, float2 (&m)[4])
@@ -1040,12 +1031,10 @@ __device__ __forceinline__ void uf8_decode8(uint2 w, float mc, float2 (&m)[4])
 // RMS clip produces: then a finite t = g * r * c has a finite product t * fl(1 / d), and an infinite or NaN t
 // ends as x = NaN with the true quotient as well (U and M are both infinite, U - M is NaN).
 template <bool ONE, bool SMALL>
-__device__ __forceinline__ void residual_x8(const float (&g)[8], uint2 codes, float mc, float ir, const float (&ic)[8],
+__device__ __forceinline__ void residual_m8(const float (&g)[8], const float2 (&mo)[4], float ir, const float (&ic)[8],
                                             const DivBy &D, float ww, float eps, float (&x)[8])
 {
     const float2 ir2 = bc2(ir), r2 = bc2(D.rcp), nd2 = bc2(D.nd), ww2 = bc2(ww), eps2 = bc2(eps);
-    float2 mo[4];
-    uf8_decode8(codes, mc, mo);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const float2 t = __fmul2_rn(__fmul2_rn(make_float2(g[2 * j], g[2 * j + 1]), ir2), make_float2(ic[2 * j], ic[2 * j + 1]));
@@ -1061,127 +1050,229 @@ __device__ __forceinline__ void residual_x8(const float (&g)[8], uint2 codes, fl
     }
 }
 
-// The residual pass over the rows r0 + warp + 8 k of a tile whose 256-column row slices (gradient and UF8 codes,
-// momentum block 256: a slice is one block) come through the warp's ring.  NB rows are consumed per iteration
-// so that their row sums are reduced jointly.  The per-row scalars (inverse row factor, block absmax) of the
-// next iteration are loaded while the current one computes; the sign of a negated gradient rides on the row
-// factor ((-g) * r == g * (-r) bit for bit).  Returns false after a time-out.
-template <typename GradT, int NB, bool ONE, bool SMALL>
-__device__ __forceinline__ bool residual_rows_ring(const FactoredLaunch &L, const af8_factored_tensor &sT, int64_t r0, int64_t r_end, int64_t c0,
-                                                   float pre_div, const float (&ic)[8], double (&cacc)[8],
-                                                   unsigned char *ring, uint64_t *full, uint32_t &cons)
+template <bool ONE, bool SMALL>
+__device__ __forceinline__ void residual_x8(const float (&g)[8], uint2 codes, float mc, float ir, const float (&ic)[8],
+                                            const DivBy &D, float ww, float eps, float (&x)[8])
 {
-    constexpr int GB = sizeof_grad<GradT>(), NS = sring_stages<GradT>(), STAGE = sring_stage_bytes<GradT, true>();
-    static_assert(NS % NB == 0 && (NS & (NS - 1)) == 0, "a ring holds whole groups of rows");
-    static_assert(NB == 2 || NB == 4, "row-sum reduction is written for 2 or 4 rows");
+    float2 mo[4];
+    uf8_decode8(codes, mc, mo);
+    residual_m8<ONE, SMALL>(g, mo, ir, ic, D, ww, eps, x);
+}
+
+// Passes over the rows r0 + warp + 8 k of a tile whose row slices (up to 256 columns of gradient and, with a momentum, its UF8
+// codes) come through the warp's ring, for matrices with rows of any length.  A slice may begin and end anywhere: what is copied
+// are the 16-byte units around it, and the lanes read from its place inside them.  With whole vectors of 8 (VEC) a lane owns 8
+// consecutive columns, as elsewhere; else the columns lane + 32 j, one 2-byte and one 1-byte access each without bank conflicts,
+// which is cheaper than shifting vectors (rows of 1001 and 2731 elements, 59 M parameters: g^2 sums 113 -> 67 us).
+// Requests go out for four rows at a time, by eight lanes with the same instructions (lane 2 i: the gradient of row i, lane
+// 2 i + 1: its codes): a request of one lane for one row costs about 57 issue slots.  Rows are consumed in pairs whose row sums
+// are reduced jointly; the per-row scalars (inverse row factor, block absmax) are loaded a pair ahead.
+//   SLICE_GRADSQ    row and column sums of g^2
+//   SLICE_RESIDUAL  of CAME's residual; the sign of a negated gradient rides on the row factor ((-g) * r == g * (-r) bit for bit)
+//   SLICE_SUM_U     sum of squares of u = g * inv_row * inv_col
+//   SLICE_SUM_M     the same with the momentum after its EMA in place of g
+// The residual wants a momentum weight below 1/2 (the form of lerp) and a clip divisor of at least 1, or NaN.
+enum { SLICE_GRADSQ = 0, SLICE_RESIDUAL = 1, SLICE_SUM_U = 2, SLICE_SUM_M = 3 };
+template <typename GradT> __host__ __device__ constexpr int slice_g_bytes() { return 256 * sizeof_grad<GradT>() + 16; }
+template <typename GradT> __host__ __device__ constexpr int slice_row_bytes() { return slice_g_bytes<GradT>() + 256 + 16; }
+constexpr int SLICE_ROWS = 4, SLICE_STAGES = 2;
+template <typename GradT> __host__ __device__ constexpr size_t slice_warp_bytes() { return (size_t)SLICE_STAGES * SLICE_ROWS * slice_row_bytes<GradT>(); }
+template <typename GradT> __host__ __device__ constexpr size_t slice_smem_bytes() { return 8 * slice_warp_bytes<GradT>(); }
+
+// false after a time-out.  cacc: the lane's column sums; total: the sum of squares (by_eight: eight squares are added in binary32
+// before they enter binary64).  FORM: SLICE_RESIDUAL: the clip divisor is 1; SLICE_SUM_M: the momentum's weight is below 1/2.
+template <typename GradT, int MODE, bool VEC, bool FORM>
+__device__ __forceinline__ bool slice_rows(const FactoredLaunch &L, const af8_factored_tensor &sT, int64_t r0, int64_t r_end, int64_t c0,
+                                           float pre_div, bool by_eight, const float (&ic)[8], double (&cacc)[8], double &total,
+                                           unsigned char *ring, uint64_t *full, uint32_t &cons)
+{
+    constexpr int GB = sizeof_grad<GradT>(), ROWB = slice_row_bytes<GradT>(), STAGE = SLICE_ROWS * ROWB, M_OFF = slice_g_bytes<GradT>();
+    constexpr bool MOM = MODE == SLICE_RESIDUAL || MODE == SLICE_SUM_M, SUM = MODE == SLICE_SUM_U || MODE == SLICE_SUM_M;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t C = sT.cols;
+    const int64_t C = sT.cols, numel = sT.rows * C, step = 8 * C;
+    const int w = (int)min((int64_t)256, C - c0);
     const int64_t row0 = r0 + warp;
-    const int nrows = row0 < r_end ? (int)((r_end - row0 + 7) / 8) : 0;          // rows row0 + 8 k of this warp
-    // lanes 0 and 1 request the next slice: lane 0 its gradients (and the bytes to expect), lane 1 its codes,
-    // both with the same instructions (a copy may complete before the bytes are announced: the phase also
-    // needs lane 0's arrival)
-    const int64_t estep = 8 * C;
-    int64_t eoff = row0 * C + c0;                                // element offset of the next slice
-    const unsigned char *src = lane == 0 ? static_cast<const unsigned char *>(sT.grad) : sT.m_q;
-    const int esz = lane == 0 ? GB : 1;
-    uint32_t prod = cons;                                        // (cons counts the slices consumed before this tile)
-    auto issue = [&]() {                                         // lanes 0 and 1
-        const int sl = (int)(prod & (uint32_t)(NS - 1));
-        ++prod;
-        unsigned char *dst = ring + sl * STAGE;
-        if (lane == 0) mbar_expect_tx(&full[sl], (uint32_t)STAGE);
-        bulk_g2s(dst + lane * (256 * GB), src + eoff * esz, 256 * esz, &full[sl]);
-        eoff += estep;
+    const int nrows = row0 < r_end ? (int)((r_end - row0 + 7) / 8) : 0, ngroups = (nrows + SLICE_ROWS - 1) / SLICE_ROWS;
+    // the gradient's last 16-byte unit, if it is not whole, is not copied: the last row's elements there are fetched one by one
+    const int64_t g_end = (numel * GB) & ~(int64_t)15;
+    const int k_last = nrows - 1;
+    const bool tail = k_last >= 0 && row0 + 8 * (int64_t)k_last == sT.rows - 1 && ((sT.rows - 1) * C + c0 + w) * GB > g_end;
+    int64_t from_off = (row0 + 8 * (int64_t)((lane >> 1) & 3)) * C + c0;      // lanes 0-7: first element of their row's slice in the next group
+    auto issue = [&](int g) {                                        // lanes 0-7: group g into its stage
+        const int sl = (int)((cons + (uint32_t)g) & (SLICE_STAGES - 1));
+        const int i = lane >> 1, k = SLICE_ROWS * g + i;
+        const bool code = lane & 1;
+        int bytes = 0;
+        const int64_t first = code ? from_off : from_off * GB, from = first & ~(int64_t)15;
+        if (k < nrows && (MOM || !code)) {
+            bytes = ((int)(first - from) + (code ? w : w * GB) + 15) & ~15;
+            if (!code && tail && k == k_last) bytes = max((int)min((int64_t)bytes, g_end - from), 0);
+        }
+        from_off += SLICE_ROWS * step;
+        const int both = bytes + (MOM ? __shfl_xor_sync(0xffu, bytes, 1) : 0);
+        if (!code) mbar_expect_tx(&full[sl], (uint32_t)both);        // (four arrivals a phase)
+        if (bytes > 0)
+            bulk_g2s(ring + sl * STAGE + i * ROWB + (code ? M_OFF : 0),
+                     (code ? sT.m_q : static_cast<const unsigned char *>(sT.grad)) + from, (uint32_t)bytes, &full[sl]);
     };
-    if (lane < 2 && nrows > 0) {
+    if (lane < 8 && ngroups > 0) {
         fence_proxy_async();
-        for (int k = 0; k < min(NS, nrows); ++k) issue();
+        for (int g = 0; g < min(SLICE_STAGES, ngroups); ++g) issue(g);
     }
     const DivBy D = make_div(pre_div);
     const LerpW LW = make_lerp(sT.m_w);
-    const float eps = sT.eps_came, sgn = L.negate_grad ? -1.0f : 1.0f;
-    // row row0 + 8 k: inverse row factor at index row0 + 8 k, block absmax at sc0 + k * scstep (both fit 32 bits:
-    // a tensor has fewer than 2^31 rows and momentum blocks)
-    const int scstep = (int)(8 * (C >> 8));
-    const int sc0 = (int)(row0 * (C >> 8) + (c0 >> 8));
-    float nir[NB], nsc[NB];                                      // the scalars of the next NB rows, signed and scaled
-#pragma unroll
-    for (int k = 0; k < NB; ++k) {
-        nir[k] = 0.0f; nsc[k] = 0.0f;
-        if (k < nrows) { nir[k] = __ldg(sT.inv_row + (int)row0 + 8 * k); nsc[k] = __ldg(sT.m_scale + sc0 + k * scstep); }
-    }
-    for (int k0 = 0; k0 < nrows; k0 += NB) {
-        GradRaw8<GradT> cur[NB];
-        uint2 cm[NB];
-        bool landed = true;
-#pragma unroll
-        for (int k = 0; k < NB; ++k) {
-            cm[k] = make_uint2(0u, 0u);
-            if (k0 + k < nrows) {
-                const uint32_t n = cons + (uint32_t)(k0 + k);
-                const int sl = (int)(n & (uint32_t)(NS - 1));
-                landed = landed && mbar_wait_bounded(&full[sl], (n / NS) & 1u);
-                const unsigned char *st = ring + sl * STAGE;
-                cur[k].from_shared(st + lane * (8 * GB));
-                cm[k] = *reinterpret_cast<const uint2 *>(st + 256 * GB + lane * 8);
-            } else cur[k].zero();
-        }
-        if (!__all_sync(0xffffffffu, landed)) return false;
-        __syncwarp();                                            // the stages were read: they may be refilled
-        if (lane < 2) {
-            fence_proxy_async();
-#pragma unroll
-            for (int k = 0; k < NB; ++k)
-                if (k0 + k + NS < nrows) issue();
-        }
-        double rsum[NB];
-#pragma unroll
-        for (int k = 0; k < NB; ++k) {
-            double racc = 0.0;
-            if (k0 + k < nrows) {
-                float g[8], x[8];
-                cur[k].unpack(0, g);
-                // fl(scale / 128): a power-of-two divisor, scale >= 1e-12
-                residual_x8<ONE, SMALL>(g, cm[k], __fmul_rn(nsc[k], 0.0078125f), __fmul_rn(nir[k], sgn), ic, D, LW.ww, eps, x);
-                if (k0 + NB + k < nrows) {                       // this row's successor in the next iteration
-                    nir[k] = __ldg(sT.inv_row + (int)row0 + 8 * (k0 + NB + k));
-                    nsc[k] = __ldg(sT.m_scale + sc0 + (k0 + NB + k) * scstep);
-                }
-                double pr[4];                                   // (pairwise: a short dependency chain)
-#pragma unroll
-                for (int j = 0; j < 8; j += 2) {
-                    const double xa = (double)x[j], xb = (double)x[j + 1];
-                    cacc[j] += xa;
-                    cacc[j + 1] += xb;
-                    pr[j >> 1] = xa + xb;
-                }
-                racc = (pr[0] + pr[1]) + (pr[2] + pr[3]);
+    const float eps = sT.eps_came, sgn = (MODE == SLICE_RESIDUAL && L.negate_grad) ? -1.0f : 1.0f;
+    const bool col_ok = VEC ? lane * 8 < w : true;                   // this lane's columns (VEC: all or none)
+    // the scalars of the next pair of rows
+    const int last_block = (int)((numel - 1) >> 8);
+    const float *pr = sT.inv_row + row0;
+    int64_t soff = row0 * C + c0 + (VEC && col_ok ? lane * 8 : 0);
+    float nir[2], ns0[2], ns1[2];
+    auto scalars = [&](int q, int k) {
+        nir[q] = ns0[q] = ns1[q] = 0.0f;
+        if (k < nrows) {
+            if (MODE != SLICE_GRADSQ) nir[q] = __ldg(pr);
+            if (MOM) {
+                const int block = (int)(soff >> 8);                  // (fewer than 2^31 blocks, as rows)
+                ns0[q] = __ldg(sT.m_scale + block);
+                if (!VEC) ns1[q] = __ldg(sT.m_scale + min(block + 1, last_block));
             }
-            rsum[k] = racc;
         }
-        double v;
-        if (NB == 4) {
-            const bool hi = lane & 16;
-            const double r0x = __shfl_xor_sync(0xffffffffu, hi ? rsum[0] : rsum[2], 16);
-            const double r1x = __shfl_xor_sync(0xffffffffu, hi ? rsum[1] : rsum[NB - 1], 16);
-            const double k0v = (hi ? rsum[2] : rsum[0]) + r0x;
-            const double k1v = (hi ? rsum[NB - 1] : rsum[1]) + r1x;
-            const bool h2 = lane & 8;
-            v = (h2 ? k1v : k0v) + __shfl_xor_sync(0xffffffffu, h2 ? k0v : k1v, 8);
+        pr += 8;
+        soff += step;
+    };
+    scalars(0, 0);
+    scalars(1, 1);
+    uint32_t lo = (uint32_t)(row0 * C + c0);                         // low word of the offset of the row at hand
+    for (int g = 0; g < ngroups; ++g) {
+        const uint32_t n = cons + (uint32_t)g;
+        const int sl = (int)(n & (SLICE_STAGES - 1));
+        const bool landed = mbar_wait_bounded(&full[sl], (n / SLICE_STAGES) & 1u);
+        if (!__all_sync(0xffffffffu, landed)) return false;
+        unsigned char *st = ring + sl * STAGE;
+        if (tail && k_last - SLICE_ROWS * g < SLICE_ROWS) {          // the tensor's last elements
+            const int64_t off = (sT.rows - 1) * C + c0;
+            const int idx = (int)max((int64_t)0, g_end / GB - off) + lane;
+            unsigned char *const to = st + (k_last - SLICE_ROWS * g) * ROWB + ((int)(off * GB) & 15) + idx * GB;
+            if (idx < w) {
+                if (GB == 4) *reinterpret_cast<float *>(to) = static_cast<const float *>(sT.grad)[off + idx];
+                else *reinterpret_cast<uint16_t *>(to) = static_cast<const uint16_t *>(sT.grad)[off + idx];
+            }
+            __syncwarp();
+        }
 #pragma unroll
-            for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if ((lane & 7) == 0 && k0 + (lane >> 3) < nrows) atomicAdd(sT.row_sum + row0 + 8 * (int64_t)(k0 + (lane >> 3)), v);
-        } else {
-            const bool hi = lane & 16;
-            v = (hi ? rsum[1] : rsum[0]) + __shfl_xor_sync(0xffffffffu, hi ? rsum[0] : rsum[1], 16);
+        for (int h = 0; h < SLICE_ROWS / 2; ++h) {
+            float gv[2][8];
+            float2 mo[2][4];
+            float irv[2];
 #pragma unroll
-            for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if ((lane & 15) == 0 && k0 + (lane >> 4) < nrows) atomicAdd(sT.row_sum + row0 + 8 * (int64_t)(k0 + (lane >> 4)), v);
+            for (int q = 0; q < 2; ++q, st += ROWB, lo += (uint32_t)step) {
+                irv[q] = MODE == SLICE_RESIDUAL ? __fmul_rn(nir[q], sgn) : nir[q];
+                const float m0 = __fmul_rn(ns0[q], 0.0078125f), m1 = __fmul_rn(ns1[q], 0.0078125f);      // fl(scale / 128), scale >= 1e-12
+                if (VEC) {
+                    GradRaw8<GradT> raw;
+                    raw.from_shared(st + lane * (8 * GB));
+                    raw.unpack(MODE == SLICE_SUM_M ? L.negate_grad : 0, gv[q]);
+                    if (MOM) uf8_decode8(*reinterpret_cast<const uint2 *>(st + M_OFF + (lo & 8u) + lane * 8), m0, mo[q]);
+                } else {
+                    const unsigned char *const gp = st + ((lo * GB) & 15u) + lane * GB, *const mp = st + M_OFF + (lo & 15u) + lane;
+                    const int bound = 256 - (int)(lo & 255u) - lane;         // 32 j from here on: the next momentum block
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        float x;
+                        if (GB == 4) x = *reinterpret_cast<const float *>(gp + 32 * j * GB);
+                        else x = __uint_as_float((uint32_t)*reinterpret_cast<const uint16_t *>(gp + 32 * j * GB) << 16);
+                        gv[q][j] = (MODE == SLICE_SUM_M && L.negate_grad) ? -x : x;
+                        if (MOM) {
+                            const float y = __fmul_rn(__uint_as_float(0x4b000000u | mp[32 * j]) - 8388736.0f, 32 * j < bound ? m0 : m1);
+                            if (j & 1) mo[q][j >> 1].y = y; else mo[q][j >> 1].x = y;
+                        }
+                    }
+                }
+            }
+            if (h == SLICE_ROWS / 2 - 1) {                           // the stage was read: it may be refilled
+                __syncwarp();
+                if (lane < 8 && g + SLICE_STAGES < ngroups) { fence_proxy_async(); issue(g + SLICE_STAGES); }
+            }
+            const int k0 = SLICE_ROWS * g + 2 * h;
+            scalars(0, k0 + 2);
+            scalars(1, k0 + 3);
+            double rsum[2] = {0.0, 0.0};
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                if (k0 + q >= nrows) continue;                       // (uniform over the warp)
+                float x[8];
+                if (MODE == SLICE_GRADSQ) {
+#pragma unroll
+                    for (int j = 0; j < 8; j += 2) {
+                        const float2 gj = make_float2(gv[q][j], gv[q][j + 1]), xx = __fmul2_rn(gj, gj);
+                        x[j] = xx.x; x[j + 1] = xx.y;
+                    }
+                } else if (MODE == SLICE_RESIDUAL) {
+                    residual_m8<FORM, true>(gv[q], mo[q], irv[q], ic, D, LW.ww, eps, x);
+                } else {
+                    const float2 ir2 = bc2(irv[q]), ww2 = bc2(LW.ww);
+#pragma unroll
+                    for (int j = 0; j < 8; j += 2) {
+                        float2 t = make_float2(gv[q][j], gv[q][j + 1]);
+                        if (MOM) t = __ffma2_rn(ww2, sub2(t, mo[q][j >> 1]), FORM ? mo[q][j >> 1] : t);
+                        const float2 u = __fmul2_rn(__fmul2_rn(t, ir2), make_float2(ic[j], ic[j + 1]));
+                        x[j] = u.x; x[j + 1] = u.y;
+                    }
+                }
+                if (VEC) {                                           // (beyond the slice the stage holds what it held)
+                    if (!col_ok) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) x[j] = 0.0f;
+                    }
+                } else if (w < 256) {                                // (uniform over the warp)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) x[j] = lane + 32 * j < w ? x[j] : 0.0f;
+                }
+                if (SUM && by_eight) {
+                    float2 a2 = __fmul2_rn(make_float2(x[0], x[1]), make_float2(x[0], x[1]));
+#pragma unroll
+                    for (int j = 2; j < 8; j += 2) a2 = __ffma2_rn(make_float2(x[j], x[j + 1]), make_float2(x[j], x[j + 1]), a2);
+                    rsum[q] = (double)__fadd_rn(a2.x, a2.y);
+                } else {
+                    double pr2[4];                                   // (pairwise: a short dependency chain)
+#pragma unroll
+                    for (int j = 0; j < 8; j += 2) {
+                        const double xa = (double)(SUM ? __fmul_rn(x[j], x[j]) : x[j]), xb = (double)(SUM ? __fmul_rn(x[j + 1], x[j + 1]) : x[j + 1]);
+                        if (!SUM) { cacc[j] += xa; cacc[j + 1] += xb; }
+                        pr2[j >> 1] = xa + xb;
+                    }
+                    rsum[q] = (pr2[0] + pr2[1]) + (pr2[2] + pr2[3]);
+                }
+            }
+            if (SUM) {
+                total += rsum[0] + rsum[1];
+            } else {
+                const bool hi = lane & 16;
+                double v = (hi ? rsum[1] : rsum[0]) + __shfl_xor_sync(0xffffffffu, hi ? rsum[0] : rsum[1], 16);
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                const int k = k0 + (lane >> 4);
+                if ((lane & 15) == 0 && k < nrows) atomicAdd(sT.row_sum + row0 + 8 * (int64_t)k, v);
+            }
         }
     }
-    cons += (uint32_t)nrows;
+    cons += (uint32_t)ngroups;
     return true;
+}
+
+// a lane's eight column factors for slice_rows
+template <bool VEC>
+__device__ __forceinline__ void slice_cols(const float *inv_col, int64_t c0, int64_t C, float (&ic)[8])
+{
+    const int lane = threadIdx.x & 31;
+    if (VEC) {
+        if (c0 + lane * 8 < C) load_f8_ro(inv_col + c0 + lane * 8, ic);
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+        if (c0 + lane + 32 * j < C) ic[j] = __ldg(inv_col + c0 + lane + 32 * j);
 }
 
 // The same pass with the input of FBOX_ROWS consecutive rows per copy: one tiled bulk tensor copy brings their
@@ -1189,10 +1280,11 @@ __device__ __forceinline__ bool residual_rows_ring(const FactoredLaunch &L, cons
 // (maps[1]: bytes, same box) into a stage of the warp's two-stage ring, so that the instructions of a request -
 // about 57 issue slots with one lane active - are spent once per FBOX_ROWS rows instead of once per row.  Warp w
 // takes the row groups r0 + FBOX_ROWS (w + 8 k); rows past the end of the unit are skipped (past the end of the tensor they arrive as zeros).
-// bf16 gradients only (a stage is 3 KB; the two stages fill the ring's 6 KB per warp).
+// bf16 gradients only (a stage is 3 KB).
 constexpr int FBOX_ROWS = 4, FBOX_STAGES = 2;
 constexpr int FBOX_G_BYTES = FBOX_ROWS * 512, FBOX_STAGE_BYTES = FBOX_G_BYTES + FBOX_ROWS * 256;
-static_assert(FBOX_STAGES * FBOX_STAGE_BYTES <= sring_stages<bf16_tag>() * sring_stage_bytes<bf16_tag, true>(), "the boxes use the ring's memory");
+static_assert(FBOX_STAGES * FBOX_STAGE_BYTES <= (int)slice_warp_bytes<bf16_tag>() && slice_warp_bytes<bf16_tag>() % 128 == 0, "the boxes use the slices' memory");
+static_assert(FBOX_STAGES == SLICE_STAGES, "and their barriers");
 static_assert(FSTAT_ROWS % (8 * FBOX_ROWS) == 0, "whole row groups per warp and tile");
 
 template <bool ONE, bool SMALL>
@@ -1303,21 +1395,23 @@ __device__ __forceinline__ bool residual_rows_box(const FactoredLaunch &L, const
 #define AF8_FSTAT_MIN_CTAS_RES 3
 #endif
 // ANY: the table has batches of matrices or rows whose length is no multiple of 8 (tensor by tensor)
-template <typename GradT, bool RESIDUAL, bool ANY>
-__global__ void __launch_bounds__(256, ANY && (RESIDUAL || std::is_same<GradT, float>::value) ? 2 : RESIDUAL ? AF8_FSTAT_MIN_CTAS_RES : AF8_FSTAT_MIN_CTAS)
-factored_stats_vec_kernel(const FactoredLaunch L, const int use_ring, const CUtensorMap *__restrict__ maps)
+// IN: how the rows come.  0: direct loads, 1: slices (per tensor, where its form allows), 2: boxes through tensor maps (bf16
+// gradients, cols % 256 == 0; residual pass)
+template <typename GradT, bool RESIDUAL, bool ANY, int IN>
+__global__ void __launch_bounds__(256, (ANY && RESIDUAL) || (std::is_same<GradT, float>::value && (ANY || IN)) ? 2 : RESIDUAL ? AF8_FSTAT_MIN_CTAS_RES : AF8_FSTAT_MIN_CTAS)
+factored_stats_vec_kernel(const FactoredLaunch L, const CUtensorMap *__restrict__ maps)
 {
     __shared__ double s_col[8][FSTAT_COLS];      // [warp][j * 32 + lane]
     __shared__ af8_factored_tensor sT;
     extern __shared__ __align__(128) unsigned char sr_smem[];            // the warps' input rings (use_ring)
-    __shared__ __align__(8) uint64_t s_full[8][sring_stages<GradT>()];
+    __shared__ __align__(8) uint64_t s_full[8][SLICE_STAGES];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int cur_t = -1;
     uint32_t cons = 0;                           // row slices this warp has taken from its ring
     [[maybe_unused]] int mapped = -1;            // tensor whose maps this warp's lane 0 has acquired
-    if (use_ring) {
+    if (IN) {
         if (lane == 0) {
-            for (int k = 0; k < sring_stages<GradT>(); ++k) mbar_init(&s_full[warp][k], 1);
+            for (int k = 0; k < SLICE_STAGES; ++k) mbar_init(&s_full[warp][k], IN == 2 ? 1 : SLICE_ROWS);
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
         __syncthreads();
@@ -1345,64 +1439,67 @@ factored_stats_vec_kernel(const FactoredLaunch L, const int use_ring, const CUte
         float ic[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) ic[j] = 0.0f;
+        // Whole rows of vectors or not; which of the row loops.  Rows of any length take the slices in both passes, whole vectors
+        // in the residual pass (339 M parameters in rows of 2000: direct loads 875 us, slices 472; of 1999: 1189 and 579); the g*g pass over whole vectors was slower through a ring (3.0 -> 4.3 ms on Llama-2-7B) and loads directly.
+        const bool vec = !ANY || (C & 7) == 0;
+        bool slices = IN == 1 && (RESIDUAL || !vec);
         if (RESIDUAL) {
             pre_div = L.dyn[t].pre_div;
-            if (ANY && (C & 7) != 0) load_cols_any(sT.inv_col + P.cb, c, C, ic);
+            slices = slices && L.m_fmt == AF8_M_UF8 && L.m_block == 256 && !(pre_div < 1.0f) && fabsf(sT.m_w) < 0.5f;
+            if (slices && !vec) slice_cols<false>(sT.inv_col + P.cb, c0, C, ic);
+            else if (!vec) load_cols_any(sT.inv_col + P.cb, c, C, ic);
             else if (col_ok) load_f8_ro(sT.inv_col + P.cb + c, ic);
         }
         double cacc[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) cacc[j] = 0.0;
-        // residual: whole 256-column slices of the gradient and the UF8 codes come through the warp's ring
-        // (measured on Llama-2-7B: 11.9 -> 11.4 ms; the g*g pass and the sum passes, which only read the
-        // gradient, were slower through a ring - 3.0 -> 4.3 ms and 4.6 -> 5.9 ms - and load directly)
-        // (the ring's quotient wants a clip divisor >= 1 or NaN, which is what the RMS clip produces)
-        bool done = false;
-        if constexpr (ANY) {
-            if ((C & 7) != 0) {
-                done = true;
-                stats_rows_any<GradT, 4, RESIDUAL>(L, sT, r0, row_end, c, pre_div, ic, cacc);
-            }
-        } else if constexpr (RESIDUAL) {
-            if (use_ring && (C % FSTAT_COLS) == 0 && L.m_fmt == AF8_M_UF8 && L.m_block == 256 && !(pre_div < 1.0f)) {
-                done = true;
-                unsigned char *ring = sr_smem + (size_t)warp * sring_stages<GradT>() * sring_stage_bytes<GradT, true>();
-                constexpr int NB = AF8_FSTAT_RES_NB;
+        bool ok = true, boxes = false;
+        if constexpr (IN == 2) {
+            if (!(pre_div < 1.0f)) {                                             // boxes of rows through tensor maps
+                boxes = true;
                 const bool one = pre_div == 1.0f, small = fabsf(sT.m_w) < 0.5f;  // (uniform over the tensor)
-                bool ok = true, boxes = false;
-                if constexpr (std::is_same<GradT, bf16_tag>::value) {
-                if (use_ring == 2) {                                             // boxes of rows through tensor maps
-                    boxes = true;
-                    const CUtensorMap *mp = maps + 2 * t;
-                    if (lane == 0 && t != mapped) { tensormap_acquire(mp); tensormap_acquire(mp + 1); mapped = t; }
-                    if (one) ok = small ? residual_rows_box<true, true>(L, sT, mp, r0, row_end, c0, pre_div, ic, cacc, ring, s_full[warp], cons)
-                                        : residual_rows_box<true, false>(L, sT, mp, r0, row_end, c0, pre_div, ic, cacc, ring, s_full[warp], cons);
-                    else ok = small ? residual_rows_box<false, true>(L, sT, mp, r0, row_end, c0, pre_div, ic, cacc, ring, s_full[warp], cons)
-                                    : residual_rows_box<false, false>(L, sT, mp, r0, row_end, c0, pre_div, ic, cacc, ring, s_full[warp], cons);
-                }
-                }
-                if (boxes) { }
-                else if (one) ok = small ? residual_rows_ring<GradT, NB, true, true>(L, sT, r0, row_end, c0, pre_div, ic, cacc, ring, s_full[warp], cons)
-                                    : residual_rows_ring<GradT, NB, true, false>(L, sT, r0, row_end, c0, pre_div, ic, cacc, ring, s_full[warp], cons);
-                else ok = small ? residual_rows_ring<GradT, NB, false, true>(L, sT, r0, row_end, c0, pre_div, ic, cacc, ring, s_full[warp], cons)
-                                : residual_rows_ring<GradT, NB, false, false>(L, sT, r0, row_end, c0, pre_div, ic, cacc, ring, s_full[warp], cons);
-                if (!ok) {
-                    atomicExch(&g_device_error, DEVERR_SRING_TIMEOUT);
-                    return;                      // (the whole warp; the others finish their rows and leave at the next barrier)
-                }
+                unsigned char *ring = sr_smem + (size_t)warp * slice_warp_bytes<GradT>();
+                const CUtensorMap *mp = maps + 2 * t;
+                if (lane == 0 && t != mapped) { tensormap_acquire(mp); tensormap_acquire(mp + 1); mapped = t; }
+                if (one) ok = small ? residual_rows_box<true, true>(L, sT, mp, r0, row_end, c0, pre_div, ic, cacc, ring, s_full[warp], cons)
+                                    : residual_rows_box<true, false>(L, sT, mp, r0, row_end, c0, pre_div, ic, cacc, ring, s_full[warp], cons);
+                else ok = small ? residual_rows_box<false, true>(L, sT, mp, r0, row_end, c0, pre_div, ic, cacc, ring, s_full[warp], cons)
+                                : residual_rows_box<false, false>(L, sT, mp, r0, row_end, c0, pre_div, ic, cacc, ring, s_full[warp], cons);
             }
         }
-        if (ANY && done) { }
-        else if (!RESIDUAL) stats_rows<GradT, 4, true, false>(L, sT, r0, row_end, c, col_ok, pre_div, ic, cacc);
-        else if (!done) stats_rows<GradT, AF8_FSTAT_RES_NB, AF8_FSTAT_RES_PREFETCH, true>(L, sT, r0, row_end, c, col_ok, pre_div, ic, cacc);
+        if (boxes) { }
+        else if (slices) {
+            if constexpr (IN == 1) {
+            unsigned char *ring = sr_smem + (size_t)warp * slice_warp_bytes<GradT>();
+            [[maybe_unused]] double none = 0.0;
+            if constexpr (RESIDUAL) {
+                const bool one = pre_div == 1.0f;
+                if (vec) ok = one ? slice_rows<GradT, SLICE_RESIDUAL, true, true>(L, sT, r0, row_end, c0, pre_div, false, ic, cacc, none, ring, s_full[warp], cons)
+                                  : slice_rows<GradT, SLICE_RESIDUAL, true, false>(L, sT, r0, row_end, c0, pre_div, false, ic, cacc, none, ring, s_full[warp], cons);
+                else if constexpr (ANY)
+                    ok = one ? slice_rows<GradT, SLICE_RESIDUAL, false, true>(L, sT, r0, row_end, c0, pre_div, false, ic, cacc, none, ring, s_full[warp], cons)
+                             : slice_rows<GradT, SLICE_RESIDUAL, false, false>(L, sT, r0, row_end, c0, pre_div, false, ic, cacc, none, ring, s_full[warp], cons);
+            } else if constexpr (ANY) {
+                ok = slice_rows<GradT, SLICE_GRADSQ, false, true>(L, sT, r0, row_end, c0, 1.0f, false, ic, cacc, none, ring, s_full[warp], cons);
+            }
+            }
+        } else if (!vec) {
+            if constexpr (ANY) stats_rows_any<GradT, 4, RESIDUAL>(L, sT, r0, row_end, c, pre_div, ic, cacc);
+        } else if (!RESIDUAL) stats_rows<GradT, 4, true, false>(L, sT, r0, row_end, c, col_ok, pre_div, ic, cacc);
+        else stats_rows<GradT, AF8_FSTAT_RES_NB, AF8_FSTAT_RES_PREFETCH, true>(L, sT, r0, row_end, c, col_ok, pre_div, ic, cacc);
+        if (!ok) {
+            atomicExch(&g_device_error, DEVERR_SRING_TIMEOUT);
+            return;                      // (the whole warp; the others finish their rows and leave at the next barrier)
+        }
 #pragma unroll
         for (int j = 0; j < 8; ++j) s_col[warp][j * 32 + lane] = cacc[j];
         __syncthreads();
-        // thread tid owns column c0 + tid = c0 + 8 * (tid >> 3) + (tid & 7)
+        // thread tid owns column c0 + tid = c0 + 8 * (tid >> 3) + (tid & 7) (slices of rows of any length: lane + 32 j as they lie)
+        const int place = slices && !vec ? tid : (tid & 7) * 32 + (tid >> 3);
         if (c0 + tid < C) {
             double sum = 0.0;
 #pragma unroll
-            for (int w = 0; w < 8; ++w) sum += s_col[w][(tid & 7) * 32 + (tid >> 3)];
+            for (int w = 0; w < 8; ++w) sum += s_col[w][place];
             atomicAdd(sT.col_sum + P.cb + c0 + tid, sum);
         }
     }
@@ -2216,6 +2313,74 @@ factored_sumsq_wide_kernel(const FactoredLaunch L)
     }
 }
 
+// The sum of squares of u over the tiles with their rows in slices: with a UF8 momentum (MOM; Adafactor with beta1), or rows of any
+// length.  (With a momentum the flat kernel above re-read the column factors for every element: 1.22 ms for the TinyLlama set's
+// 3.3 GB, 0.79 here; 59 M parameters in rows of 1001 and 2731 elements 132 us, 92.)  Sums as in factored_sumsq_tile_kernel.
+// whole: whether tensors of whole vectors add their squares by eight: 0 none, 1 matrices that are not a batch, 2 all.
+template <typename GradT, bool MOM>
+__global__ void __launch_bounds__(256, sizeof_grad<GradT>() == 2 ? 3 : 2)
+factored_sumsq_slice_kernel(const FactoredLaunch L, const int whole)
+{
+    __shared__ af8_factored_tensor sT;
+    __shared__ double s_acc2[8];
+    extern __shared__ __align__(128) unsigned char sr_smem[];
+    __shared__ __align__(8) uint64_t s_full[8][SLICE_STAGES];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (lane == 0) {
+        for (int k = 0; k < SLICE_STAGES; ++k) mbar_init(&s_full[warp][k], SLICE_ROWS);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    unsigned char *const ring = sr_smem + (size_t)warp * slice_warp_bytes<GradT>();
+    uint32_t cons = 0;
+    int cur_t = -1;
+    for (int64_t id = blockIdx.x; id < L.total_units; id += gridDim.x) {
+        int t = cur_t;
+        const int64_t tile = id >> L.split;
+        if (t < 0) t = find_factored_tile(L.tensors, L.n_tensors, tile);
+        else while (t + 1 < L.n_tensors && __ldg(&L.tensors[t + 1].first_tile) <= tile) ++t;
+        __syncthreads();                                           // s_acc2 of the previous tile was read
+        if (t != cur_t) {
+            if (tid < (int)(sizeof(af8_factored_tensor) / 4))
+                reinterpret_cast<uint32_t *>(&sT)[tid] = __ldg(reinterpret_cast<const uint32_t *>(L.tensors + t) + tid);
+            cur_t = t;
+            __syncthreads();
+        }
+        const int64_t C = sT.cols;
+        const TilePos P = tile_pos(L, sT, id);
+        if (P.r0 >= P.r_end) continue;                             // an empty part of a split tile
+        constexpr int MODE = MOM ? SLICE_SUM_M : SLICE_SUM_U;
+        const bool vec = (C & 7) == 0, by_eight = vec && (whole == 2 || (whole == 1 && sT.batch_rows == 0));
+        const bool small = !MOM || fabsf(sT.m_w) < 0.5f;
+        float ic[8];
+        double none[8], acc = 0.0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) { ic[j] = 0.0f; none[j] = 0.0; }
+        bool ok;
+        if (vec) {
+            slice_cols<true>(sT.inv_col + P.cb, P.c0, C, ic);
+            ok = small ? slice_rows<GradT, MODE, true, true>(L, sT, P.r0, P.r_end, P.c0, 1.0f, by_eight, ic, none, acc, ring, s_full[warp], cons)
+                       : slice_rows<GradT, MODE, true, false>(L, sT, P.r0, P.r_end, P.c0, 1.0f, by_eight, ic, none, acc, ring, s_full[warp], cons);
+        } else {
+            slice_cols<false>(sT.inv_col + P.cb, P.c0, C, ic);
+            ok = small ? slice_rows<GradT, MODE, false, true>(L, sT, P.r0, P.r_end, P.c0, 1.0f, by_eight, ic, none, acc, ring, s_full[warp], cons)
+                       : slice_rows<GradT, MODE, false, false>(L, sT, P.r0, P.r_end, P.c0, 1.0f, by_eight, ic, none, acc, ring, s_full[warp], cons);
+        }
+        if (!ok) {
+            atomicExch(&g_device_error, DEVERR_SRING_TIMEOUT);
+            return;
+        }
+        acc = warp_sum(acc);
+        if (lane == 0) s_acc2[warp] = acc;
+        __syncthreads();
+        if (tid == 0) {
+            double sum = 0.0;
+            for (int w = 0; w < 8; ++w) sum += s_acc2[w];
+            atomicAdd(L.block_sumsq + sT.first_chunk, sum);
+        }
+    }
+}
+
 // The same sum over the 512 x 256 tiles of the statistic pass: a lane keeps the inverse column factors of
 // its 8 columns in registers while its warp walks the tile's rows (the flat kernel above re-reads them for
 // every element, twice the bytes of the gradient itself through L1), four rows' loads in flight.  A CTA adds
@@ -2498,12 +2663,11 @@ static int af8_factored_stats_impl(const af8_factored_cfg *cfg, const af8_factor
     static const bool ring_off = getenv("AF8_NO_FACTORED_RING") != nullptr;
     static const bool box_off = getenv("AF8_NO_FACTORED_BOXES") != nullptr;
     const bool any = cfg->aligned8 == 2;
-    int ring = (ring_off || !res || any) ? 0 : 1;
+    int ring = (ring_off || !(res || any)) ? 0 : 1;
     // residual pass over bf16 gradients and UF8 codes of tensors with cols % 256 == 0: boxes of rows through
-    // tensor maps, when the caller has given room for the maps.  (In tables where only some tensors qualify they were
-    // slower than row copies: 117 against 97 us on an 8-layer 512 x 1376 model.)
+    // tensor maps, when the caller has given room for the maps
     const CUtensorMap *maps = nullptr;
-    if (ring && !box_off && vec && bf && host_maps && dev_maps && cfg->m_fmt == AF8_M_UF8 && cfg->m_block == 256 && cfg->cols_mult256) {
+    if (ring && res && !any && !box_off && vec && bf && host_maps && dev_maps && cfg->m_fmt == AF8_M_UF8 && cfg->m_block == 256 && cfg->cols_mult256) {
         bool ok = (reinterpret_cast<uintptr_t>(dev_maps) & 63) == 0;
         for (int i = 0; i < n_tensors && ok; ++i) {
             const af8_factored_tensor &t = host_tensors[i];
@@ -2521,16 +2685,20 @@ static int af8_factored_stats_impl(const af8_factored_cfg *cfg, const af8_factor
             ring = 2;
         }
     }
+#define AF8_LAUNCH_FSTAT_IN(G, RES, A, I) do { \
+        const size_t sm = (I) ? slice_smem_bytes<G>() : 0; \
+        if (sm > 0) AF8_CUDA_TRY(cudaFuncSetAttribute(factored_stats_vec_kernel<G, RES, A, I>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)); \
+        factored_stats_vec_kernel<G, RES, A, I><<<(int)grid, 256, sm, st>>>(L, maps); } while (0)
 #define AF8_LAUNCH_FSTAT(G, RES) do { \
-        const size_t sm = ring ? sring_smem_bytes<G, RES>() : 0; \
-        if (sm > 0) AF8_CUDA_TRY(cudaFuncSetAttribute(factored_stats_vec_kernel<G, RES, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)); \
-        if (any) factored_stats_vec_kernel<G, RES, true><<<(int)grid, 256, 0, st>>>(L, 0, nullptr); \
-        else factored_stats_vec_kernel<G, RES, false><<<(int)grid, 256, sm, st>>>(L, ring, maps); } while (0)
-    if (vec && bf && res) AF8_LAUNCH_FSTAT(bf16_tag, true);
+        if (any && ring) AF8_LAUNCH_FSTAT_IN(G, RES, true, 1); else if (any) AF8_LAUNCH_FSTAT_IN(G, RES, true, 0); \
+        else if (RES && ring == 1) AF8_LAUNCH_FSTAT_IN(G, RES, false, 1); else AF8_LAUNCH_FSTAT_IN(G, RES, false, 0); } while (0)
+    if (vec && bf && res && ring == 2) AF8_LAUNCH_FSTAT_IN(bf16_tag, true, false, 2);
+    else if (vec && bf && res) AF8_LAUNCH_FSTAT(bf16_tag, true);
     else if (vec && bf) AF8_LAUNCH_FSTAT(bf16_tag, false);
     else if (vec && res) AF8_LAUNCH_FSTAT(float, true);
     else if (vec) AF8_LAUNCH_FSTAT(float, false);
 #undef AF8_LAUNCH_FSTAT
+#undef AF8_LAUNCH_FSTAT_IN
     else factored_stats_kernel<<<(int)grid, 256, 0, st>>>(L);
     AF8_CUDA_TRY(cudaGetLastError());
     return AF8_OK;
@@ -2603,14 +2771,27 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
     static const bool tile_off = getenv("AF8_NO_TILE_SUMS") != nullptr;
     const int64_t total_tiles = cfg->total_tiles;
     const bool any = cfg->aligned8 == 2;         // batches of matrices, rows of any length >= 8
-    if (vec && !apply && !tile_off && total_tiles > 0 && cfg->grad_dtype != AF8_F16 && ((cfg->came && cfg->mode == AF8_FUPD_SUMSQ_U) || no_m)) {
-        // the sum only needs the gradient: over the statistic tiles, column factors in registers
+    const bool only_g = (cfg->came && cfg->mode == AF8_FUPD_SUMSQ_U) || no_m;
+    const bool mom = !cfg->came && cfg->m_fmt == AF8_M_UF8 && cfg->m_block == 256 && !ring_off;
+    if (vec && !apply && !tile_off && total_tiles > 0 && cfg->grad_dtype != AF8_F16 && (only_g || mom)) {
+        // over the statistic tiles, column factors in registers; with a momentum, or rows of any length, in slices
         AF8_CUDA_TRY(cudaMemsetAsync(block_sumsq, 0, sizeof(double) * (size_t)total_chunks, cst));
         FactoredLaunch LT = L;
         LT.split = tile_split(total_tiles);
         LT.total_units = total_tiles << LT.split;
-        const int64_t tg = std::min<int64_t>((int64_t)sm_count() * 8, LT.total_units);
         const int kind = !any ? 0 : cfg->cols_mult8 ? 1 : 2;
+        if (!ring_off && (mom || kind == 2)) {
+            const int64_t sg = std::min<int64_t>((int64_t)sm_count() * (bf ? 3 : 2), LT.total_units);
+#define AF8_LAUNCH_FSLICE(G, M) do { \
+            AF8_CUDA_TRY(cudaFuncSetAttribute(factored_sumsq_slice_kernel<G, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)slice_smem_bytes<G>())); \
+            factored_sumsq_slice_kernel<G, M><<<(int)sg, 256, slice_smem_bytes<G>(), cst>>>(LT, 2 - kind); } while (0)
+            if (bf) { if (mom) AF8_LAUNCH_FSLICE(bf16_tag, true); else AF8_LAUNCH_FSLICE(bf16_tag, false); }
+            else { if (mom) AF8_LAUNCH_FSLICE(float, true); else AF8_LAUNCH_FSLICE(float, false); }
+#undef AF8_LAUNCH_FSLICE
+            AF8_CUDA_TRY(cudaGetLastError());
+            return AF8_OK;
+        }
+        const int64_t tg = std::min<int64_t>((int64_t)sm_count() * 8, LT.total_units);
 #define AF8_LAUNCH_FSUM(G) do { if (kind == 0) factored_sumsq_tile_kernel<G, 0><<<(int)tg, 256, 0, cst>>>(LT); \
         else if (kind == 1) factored_sumsq_tile_kernel<G, 1><<<(int)tg, 256, 0, cst>>>(LT); \
         else factored_sumsq_tile_kernel<G, 2><<<(int)tg, 256, 0, cst>>>(LT); } while (0)

@@ -103,6 +103,19 @@ EXTRA_CASES["came_long_blocks"] = dict(shapes=[(5000, 16), (40, 9001), (4100,)],
 EXTRA_CASES["adafactor_long_blocks"] = dict(shapes=[(5000, 16), (40, 9001)], steps=3, seed=64, grad=cases.CASES["adafactor_factored"]["grad"],
                                             hp=dict(cases.CASES["adafactor_factored"]["hp"], block_size=8192, v_quant_type="al8"))
 
+# row slices through the warps' rings: binary32 gradients, momentum weights of 1/2 and more (the other form of lerp), a last unit
+# of 16 bytes that belongs to one or to two slices of the last row, tiles that end within a group of four rows
+_SLICES = [(700, 257), (131, 273), (39, 264), (1030, 513), (67, 1001)]
+EXTRA_CASES.update({
+    "came_slices_f32": dict(shapes=_SLICES, steps=3, seed=65, grad=_F32, hp=cases.CASES["came_al16"]["hp"]),
+    "came_slices_w": dict(shapes=_SLICES, steps=3, seed=66, grad=cases.CASES["came_al16"]["grad"], hp=dict(cases.CASES["came_al16"]["hp"], beta1=0.4)),
+    "adafactor_m_slices": dict(shapes=_SLICES, steps=3, seed=67, grad=cases.CASES["adafactor_factored_m"]["grad"],
+                               hp=cases.CASES["adafactor_factored_m"]["hp"]),
+    "adafactor_m_slices_f32_w": dict(shapes=_SLICES, steps=3, seed=68, grad=_F32, hp=dict(cases.CASES["adafactor_factored_m"]["hp"], beta1=0.4)),
+    "adafactor_m_slices_8": dict(shapes=[(39, 264), (520, 776), (1030, 520)], steps=3, seed=69, grad=cases.CASES["adafactor_factored_m"]["grad"],
+                                 hp=dict(cases.CASES["adafactor_factored_m"]["hp"], maximize=True)),
+})
+
 # lag_norm=True (one pass with the previous step's norm; optimizer.py:1056-1071): the vector kernels, the
 # element-wise kernels (odd column counts) and the limiter on top of the clip
 EXTRA_CASES.update({
