@@ -194,17 +194,6 @@ __device__ __forceinline__ float u_clipped_fast(float g, float ir, float ic, con
     return div_by(__fmul_rn(__fmul_rn(g, ir), ic), D);
 }
 
-// UF8 code of m for a block absmax a >= 1e-12 (optimizer.py:512): round(m / a * 128) clamped
-// to [-128, 127], plus 128; the division as above
-__device__ __forceinline__ uint32_t uf8_encode_fast(float m, const DivBy &A)
-{
-    const float q = __fmul_rn(m, A.rcp);
-    const float q2 = __fmaf_rn(__fmaf_rn(q, A.nd, m), A.rcp, q);       // |q| <= 1: always finite
-    const float kf = __fmaf_rn(q2, 128.0f, 12582912.0f);               // exact product, round half to even
-    const int k = min(__float_as_int(kf), 0x4b400000 + 127);           // only +128 needs the clamp
-    return (uint32_t)(k - 0x4b400000 + 128);
-}
-
 // The same helpers on pairs of elements with Blackwell's packed binary32 instructions (one
 // instruction per pair; each component rounds exactly like the scalar operation).
 __device__ __forceinline__ float2 div_by2(float2 x, const DivBy &D)
@@ -219,17 +208,6 @@ __device__ __forceinline__ float2 lerp_w2(float2 s, float2 e, const LerpW &l)
 {
     return __ffma2_rn(bc2(l.ww), sub2(e, s), l.small ? s : e);
 }
-// two UF8 codes, the first in the low byte
-__device__ __forceinline__ uint32_t uf8_encode_fast2(float2 m, const DivBy &A)
-{
-    const float2 r2 = bc2(A.rcp);
-    const float2 q = __fmul2_rn(m, r2);
-    const float2 q2 = __ffma2_rn(__ffma2_rn(q, bc2(A.nd), m), r2, q);
-    const float2 kf = __ffma2_rn(q2, bc2(128.0f), bc2(12582912.0f));
-    const int k0 = min(__float_as_int(kf.x), 0x4b400000 + 127), k1 = min(__float_as_int(kf.y), 0x4b400000 + 127);
-    return (uint32_t)(k0 - 0x4b400000 + 128) | ((uint32_t)(k1 - 0x4b400000 + 128) << 8);
-}
-
 // Largest magnitude of a momentum block of 256, 8 elements a lane: at least 1e-12, NaNs left out.  odd: the block holds an
 // infinity or a NaN.  (The bit patterns of non-negative floats are ordered: one REDUX instead of a shuffle tree.)
 __device__ __forceinline__ float m_absmax256(const float (&m)[8], bool &odd)
@@ -261,9 +239,23 @@ __device__ __forceinline__ uint2 uf8_codes8(const float (&m)[8], float am, bool 
         }
         return o;
     }
-    const DivBy A = make_div(am);
-    return make_uint2(uf8_encode_fast2(make_float2(m[0], m[1]), A) | (uf8_encode_fast2(make_float2(m[2], m[3]), A) << 16),
-                      uf8_encode_fast2(make_float2(m[4], m[5]), A) | (uf8_encode_fast2(make_float2(m[6], m[7]), A) << 16));
+    // round(m / am * 128), the quotient from the correctly rounded reciprocal and one residual step (|m / am| <= 1: always finite, the
+    // product exact), half to even by the rounding constant; only + 128 needs the clamp; the low byte is k mod 256, k + 128 with
+    // its top bit flipped
+    const float2 ra2 = bc2(__frcp_rn(am)), nam2 = bc2(-am);
+    uint32_t w[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        uint32_t raw[4];
+#pragma unroll
+        for (int j = 0; j < 4; j += 2) {
+            const float2 kf = __ffma2_rn(div2_by(make_float2(m[4 * h + j], m[4 * h + j + 1]), ra2, nam2), bc2(128.0f), bc2(AF8_MAGIC_F));
+            raw[j] = (uint32_t)min(__float_as_int(kf.x), AF8_MAGIC_I + 127);
+            raw[j + 1] = (uint32_t)min(__float_as_int(kf.y), AF8_MAGIC_I + 127);
+        }
+        w[h] = pack4(raw[0], raw[1], raw[2], raw[3]) ^ 0x80808080u;
+    }
+    return make_uint2(w[0], w[1]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1879,35 +1871,78 @@ factored_update_vec_kernel(const FactoredLaunch L)
 }
 
 // ---------------------------------------------------------------------------
-// The APPLY pass for fp32 parameters with a UF8 momentum (CAME, Adafactor with beta1), inputs
-// through per-warp rings of bulk asynchronous copies.
+// The APPLY pass with a UF8 momentum (CAME, Adafactor with beta1) in flat order, inputs through per-warp rings of bulk
+// asynchronous copies, for rows of any length >= 8, batches of matrices, and binary32 or bf16 parameters.
 //
-// The register-pipelined kernel above has one chunk in flight per thread and was measured
-// latency-bound in this configuration (CAME apply: half of the copy peak, long-scoreboard
-// stalls on top).  Here a warp still owns one momentum block per chunk (256 consecutive
-// elements: gradient, parameter and momentum codes are three contiguous runs of 512 or 1024,
-// 1024 and 256 bytes), but its lane 0 requests them FRING_STAGES - 1 chunks ahead with
-// cp.async.bulk into the warp's own ring; completion is an mbarrier per stage.  Warps do not
-// synchronise with one another except when the CTA moves to its next tensor.  Copies never
+// A warp owns one momentum block per chunk (256 consecutive elements: gradient, parameter and momentum codes are three
+// contiguous runs); lanes 0 to 2 request one run each, FRING_STAGES - 1 chunks ahead, into the warp's own ring; completion is an
+// mbarrier per stage.  Warps do not synchronise with one another except when the CTA moves to its next tensor.  Copies never
 // cross a tensor, and the (at most one) partial chunk at a tensor's end is loaded directly.
-// Same arithmetic, element for element, as factored_update_vec_kernel.
+//
+// What bounds it is instruction issue: the column factors of 8 elements come from memory (L1), at any alignment where rows are no
+// multiple of 8 (ANY), and the row may end among them.  A warp without a row end among its 256 elements takes the form with one row
+// factor.  Two resident CTAs without spills for ANY, three with 90 bytes of them otherwise: 181 and 215 us below.
+// Write pass before (the kernel above for ANY and bf16, one lane's requests else) -> now: 59 M parameters in rows of 1001 and 2731
+// elements 229 -> 180 us, 397 M in rows of 1999 with CAME 1640 -> 1446, 339 M in rows of 2000 with CAME 856 -> 826, 1.1 G bf16
+// parameters 2.54 -> 2.35 ms.
+// PT: the parameters, as above (0: binary32; 1, 2: bf16 to nearest, stochastically).
 // ---------------------------------------------------------------------------
 #ifndef AF8_FRING_STAGES
 #define AF8_FRING_STAGES 4
 #endif
 constexpr int FRING_STAGES = AF8_FRING_STAGES;
 constexpr int DEVERR_FRING_TIMEOUT = 3;
-template <typename GradT> __host__ __device__ constexpr int fring_stage_bytes() { return 256 * sizeof_grad<GradT>() + 1024 + 256; }
-template <typename GradT> constexpr size_t fring_smem_bytes() { return (size_t)(FUPD_THREADS / 32) * FRING_STAGES * fring_stage_bytes<GradT>(); }
+template <typename GradT, int PT = 0> __host__ __device__ constexpr int fring_stage_bytes() { return 256 * sizeof_grad<GradT>() + (PT == 0 ? 1024 : 512) + 256; }
+template <typename GradT, int PT = 0> constexpr size_t fring_smem_bytes() { return (size_t)(FUPD_THREADS / 32) * FRING_STAGES * fring_stage_bytes<GradT, PT>(); }
 
-template <typename GradT, int CTAS>
-__global__ void __launch_bounds__(FUPD_THREADS, CTAS)
-factored_apply_ring_kernel(const FactoredLaunch L)
+// column factors of elements col .. col + 7 of a row, the elements from `left` (1 .. 7) on being the first of the next row
+__device__ __forceinline__ void flat_cols_wrap(const float *v, int64_t cb0, int64_t cb1, int64_t col, int left, float (&x)[8])
 {
-    constexpr int GB = sizeof_grad<GradT>();
-    constexpr int P_OFF = 256 * GB, M_OFF = P_OFF + 1024, STAGE = fring_stage_bytes<GradT>(), NS = FRING_STAGES;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] = __ldg(j < left ? v + cb0 + col + j : v + cb1 + j - left);
+}
+
+// New momentum and update of 8 elements.  ir, irc: row factors of the elements before `left`, irb, ircb of the others (COMMON: no
+// others, and a momentum weight below 1/2).
+template <bool CAME, bool COMMON>
+__device__ __forceinline__ void flat_update8(const float (&g)[8], const float2 (&mo)[4], const float (&ic)[8], const float (&icc)[8], float ir, float irb,
+                                             float irc, float ircb, int left, const DivBy &D, const LerpW &LW, float (&mj)[8], float (&u)[8])
+{
+    const auto row2 = [&](float a, float b, int j) { return COMMON ? bc2(a) : make_float2(j < left ? a : b, j + 1 < left ? a : b); };
+    const float2 ww2 = bc2(LW.ww);
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+        const float2 gj = make_float2(g[j], g[j + 1]), c2 = make_float2(ic[j], ic[j + 1]), m = mo[j >> 1];
+        float2 e = gj;
+        if (CAME) e = div_by2(__fmul2_rn(__fmul2_rn(gj, row2(ir, irb, j)), c2), D);
+        const float2 mm = __ffma2_rn(ww2, sub2(e, m), (COMMON || LW.small) ? m : e);
+        const float2 uj = CAME ? __fmul2_rn(__fmul2_rn(mm, row2(irc, ircb, j)), make_float2(icc[j], icc[j + 1]))
+                               : __fmul2_rn(__fmul2_rn(mm, row2(ir, irb, j)), c2);
+        mj[j] = mm.x; mj[j + 1] = mm.y; u[j] = uj.x; u[j + 1] = uj.y;
+    }
+}
+
+// what a CTA keeps of its current tensor (in shared memory: in registers it costs spills)
+struct FlatTensor {
+    int64_t numel, next_first, full_end, adv_rows, adv_cols;     // chunk ids: the next tensor's first, the first that is not whole; 2048 elements in rows and columns
+    DivBy D;
+    LerpW LW;
+    float step_mul, fira;
+    int32_t zero_upd, whole;                                     // whole: rows are whole vectors
+};
+
+#ifndef FLAT_ANY_CTAS
+#define FLAT_ANY_CTAS 2
+#endif
+template <typename GradT, int PT, bool ANY>
+__global__ void __launch_bounds__(FUPD_THREADS, sizeof_grad<GradT>() == 2 ? (ANY ? FLAT_ANY_CTAS : 3) : 2)
+factored_apply_flat_kernel(const FactoredLaunch L)
+{
+    constexpr int GB = sizeof_grad<GradT>(), PB = PT == 0 ? 4 : 2, NS = FRING_STAGES;
+    constexpr int P_OFF = 256 * GB, M_OFF = P_OFF + 256 * PB, STAGE = fring_stage_bytes<GradT, PT>();
     extern __shared__ __align__(128) unsigned char fr_smem[];
     __shared__ af8_factored_tensor sT;
+    __shared__ FlatTensor sF;
     __shared__ __align__(8) uint64_t s_full[FUPD_THREADS / 32][NS];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     unsigned char *const ring = fr_smem + (size_t)warp * NS * STAGE;
@@ -1921,15 +1956,14 @@ factored_apply_ring_kernel(const FactoredLaunch L)
     const int64_t id_begin = (int64_t)blockIdx.x * per_cta;
     const int64_t id_end = min(id_begin + per_cta, L.total_units);
     int cur_t = -1;
-    int64_t next_first = 0, full_end = 0, flat = 0, row = 0, col = 0;
-    float pre_div = 1.0f, step_mul = 0.0f, fira = 1.0f;
-    bool zero_upd = false;
-    DivBy D = make_div(1.0f);
+    int64_t flat = 0, row = 0, col = 0;
     uint32_t cons = 0;            // chunks this warp has taken from its ring
     int inflight = 0;             // chunks from the current one on whose copies are issued
+    float nsc = 0.0f;             // absmax of this warp's block of the next chunk
+    bool have_sc = false;
 
     for (int64_t id = id_begin; id < id_end; ++id) {
-        if (cur_t < 0 || id >= next_first) {
+        if (cur_t < 0 || id >= sF.next_first) {
             int tn = cur_t;
             if (tn < 0) tn = find_factored_chunk(L.tensors, L.n_tensors, id);
             else while (tn + 1 < L.n_tensors && __ldg(&L.tensors[tn + 1].first_chunk) <= id) ++tn;
@@ -1938,57 +1972,70 @@ factored_apply_ring_kernel(const FactoredLaunch L)
                 reinterpret_cast<uint32_t *>(&sT)[tid] = __ldg(reinterpret_cast<const uint32_t *>(L.tensors + tn) + tid);
             cur_t = tn;
             __syncthreads();
-            next_first = tn + 1 < L.n_tensors ? __ldg(&L.tensors[tn + 1].first_chunk) : L.total_units;
-            full_end = min(id_end, sT.first_chunk + (sT.rows * sT.cols) / 2048);     // chunk ids below it are whole chunks of this tensor
+            const int64_t C = sT.cols;
             flat = (id - sT.first_chunk) * 2048 + tid * 8;
-            row = flat / sT.cols;
-            col = flat - row * sT.cols;
-            pre_div = 1.0f; step_mul = -sT.alpha; fira = 1.0f; zero_upd = false;
-            if (L.dyn != nullptr) {
-                const af8_dyn_scalars ds = L.dyn[tn];
-                if (L.came) pre_div = ds.pre_div;
-                step_mul = ds.step; fira = ds.fira; zero_upd = ds.zero != 0.0f;
+            row = flat / C;
+            col = flat - row * C;
+            if (tid == 0) {
+                FlatTensor F;
+                F.numel = sT.rows * C;
+                F.next_first = tn + 1 < L.n_tensors ? __ldg(&L.tensors[tn + 1].first_chunk) : L.total_units;
+                F.full_end = min(id_end, sT.first_chunk + F.numel / 2048);
+                F.adv_rows = 2048 / C;
+                F.adv_cols = 2048 - F.adv_rows * C;
+                F.whole = !ANY || (C & 7) == 0;
+                float pre_div = 1.0f;
+                F.step_mul = -sT.alpha; F.fira = 1.0f; F.zero_upd = 0;
+                if (L.dyn != nullptr) {
+                    const af8_dyn_scalars ds = L.dyn[tn];
+                    if (L.came) pre_div = ds.pre_div;
+                    F.step_mul = ds.step; F.fira = ds.fira; F.zero_upd = ds.zero != 0.0f;
+                }
+                F.D = make_div(pre_div);
+                F.LW = make_lerp(sT.m_w);
+                sF = F;
             }
-            D = make_div(pre_div);
+            __syncthreads();
             inflight = 0;                                            // (copies never cross a tensor)
+            have_sc = false;
         } else {
             flat += 2048;
-            col += 2048;
-            if (sT.cols >= 2048) {
-                if (col >= sT.cols) { col -= sT.cols; ++row; }
-            } else {
-                const uint32_t q = (uint32_t)col / (uint32_t)sT.cols;
-                row += q;
-                col -= (int64_t)q * sT.cols;
-            }
+            row += sF.adv_rows;
+            col += sF.adv_cols;
+            if (col >= sT.cols) { col -= sT.cols; ++row; }
         }
-        const int64_t numel = sT.rows * sT.cols;
-        const bool full = id < full_end;
+        const int64_t numel = sF.numel;
+        const bool full = id < sF.full_end;
         const bool ok = flat < numel;
-        float *const pbase = static_cast<float *>(sT.param);
+        const int nval = ANY ? (int)min((int64_t)8, numel - flat) : 8;       // (fewer only in a tensor's last vector)
+        const int64_t block = (id - sT.first_chunk) * 8 + warp;              // this warp's momentum block
 
         // ---- request the chunks id .. id + NS - 1 that are whole chunks of this tensor ----
-        int want = (int)min((int64_t)NS, full_end - id);
+        int want = (int)min((int64_t)NS, sF.full_end - id);
         if (want < 0) want = 0;
-        if (lane == 0 && inflight < want) {
+        if (lane < 3 && inflight < want) {
             fence_proxy_async();                                     // this warp's reads of the slots came first
-            const unsigned char *gp = static_cast<const unsigned char *>(sT.grad);
-            const unsigned char *pp = static_cast<const unsigned char *>(sT.param);
+            const unsigned char *const src = lane == 0 ? static_cast<const unsigned char *>(sT.param) : lane == 1 ? static_cast<const unsigned char *>(sT.grad) : sT.m_q;
+            const int size = lane == 0 ? 256 * PB : lane == 1 ? 256 * GB : 256, to = lane == 0 ? P_OFF : lane == 1 ? 0 : M_OFF;
             for (int k = inflight; k < want; ++k) {
-                const int64_t off = (id + k - sT.first_chunk) * 2048 + warp * 256;      // first element of the warp's run
                 const int sl = (int)((cons + (uint32_t)k) % NS);
-                unsigned char *dst = ring + sl * STAGE;
-                mbar_expect_tx(&s_full[warp][sl], (uint32_t)STAGE);
-                bulk_g2s(dst + P_OFF, pp + off * 4, 1024, &s_full[warp][sl]);
-                bulk_g2s(dst, gp + off * GB, 256 * GB, &s_full[warp][sl]);
-                bulk_g2s(dst + M_OFF, sT.m_q + off, 256, &s_full[warp][sl]);
+                if (lane == 0) mbar_expect_tx(&s_full[warp][sl], (uint32_t)STAGE);
+                bulk_g2s(ring + sl * STAGE + to, src + (block + 8 * k) * size, (uint32_t)size, &s_full[warp][sl]);
             }
         }
         inflight = want > 0 ? want - 1 : 0;                          // as seen from the next chunk
 
+        const int64_t w0 = block * 256;                              // (the block exists iff its first element does)
+        float sc = nsc;
+        if (!have_sc) sc = w0 < numel ? __ldg(sT.m_scale + block) : 0.0f;
+        have_sc = id + 1 < id_end && w0 + 2048 < numel;
+        if (have_sc) nsc = __ldg(sT.m_scale + block + 8);
+
         GradRaw8<GradT> cg;
-        float4 cp0 = make_float4(0.f, 0.f, 0.f, 0.f), cp1 = cp0;
-        uint2 cm = make_uint2(0u, 0u);
+        uint4 pa = make_uint4(0u, 0u, 0u, 0u), pb = pa;              // 8 parameters (bf16: in pa)
+        uint2 cm = make_uint2(0x80808080u, 0x80808080u);
+        float *const pbase = static_cast<float *>(sT.param);
+        uint16_t *const hbase = static_cast<uint16_t *>(sT.param);
         if (full) {
             const int sl = (int)(cons % NS);
             const bool landed = mbar_wait_bounded(&s_full[warp][sl], (cons / NS) & 1u);
@@ -1998,82 +2045,137 @@ factored_apply_ring_kernel(const FactoredLaunch L)
             }
             const unsigned char *st = ring + sl * STAGE;
             cg.from_shared(st + lane * (8 * GB));
-            cp0 = *reinterpret_cast<const float4 *>(st + P_OFF + lane * 32);
-            cp1 = *reinterpret_cast<const float4 *>(st + P_OFF + lane * 32 + 16);
+            pa = *reinterpret_cast<const uint4 *>(st + P_OFF + lane * (8 * PB));
+            if (PT == 0) pb = *reinterpret_cast<const uint4 *>(st + P_OFF + lane * 32 + 16);
             cm = *reinterpret_cast<const uint2 *>(st + M_OFF + lane * 8);
             ++cons;
             __syncwarp();                                            // the slot may be refilled from the next iteration on
-        } else if (ok) {
+        } else if (ok && nval == 8) {
             cg.load(sT.grad, flat);
-            cp0 = *reinterpret_cast<const float4 *>(pbase + flat);
-            cp1 = *reinterpret_cast<const float4 *>(pbase + flat + 4);
+            if (PT == 0) {
+                pa = *reinterpret_cast<const uint4 *>(pbase + flat);
+                pb = *reinterpret_cast<const uint4 *>(pbase + flat + 4);
+            } else pa = *reinterpret_cast<const uint4 *>(hbase + flat);
+            cm = *reinterpret_cast<const uint2 *>(sT.m_q + flat);
+        } else if (ok) {                                             // (codes are stored in whole blocks)
+            cg.load_part(sT.grad, flat, nval);
+            uint32_t x[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) x[j] = j < nval ? (PT == 0 ? __float_as_uint(pbase[flat + j]) : (uint32_t)hbase[flat + j]) : 0u;
+            if (PT == 0) { pa = make_uint4(x[0], x[1], x[2], x[3]); pb = make_uint4(x[4], x[5], x[6], x[7]); }
+            else pa = make_uint4(x[0] | (x[1] << 16), x[2] | (x[3] << 16), x[4] | (x[5] << 16), x[6] | (x[7] << 16));
             cm = *reinterpret_cast<const uint2 *>(sT.m_q + flat);
         } else cg.zero();
 
         float mj[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) mj[j] = 0.0f;
+        const bool whole = !ANY || sF.whole;
+        const int left = whole ? 8 : (int)min((int64_t)8, sT.cols - col);     // elements before the row's end
+        const bool common = sF.LW.small && !(ANY && __any_sync(0xffffffffu, left < 8));
         if (ok) {
-            float g[8], ic[8], u[8], mo[8];
-            const LerpW LW = make_lerp(sT.m_w);
+            float g[8], ic[8], icc[8], u[8];
+            float2 mo[4];
             cg.unpack(L.negate_grad, g);
-            load_f8_ro(sT.inv_col + col, ic);
-            const float2 ir2 = bc2(__ldg(sT.inv_row + row));
-            m_old8(sT, AF8_M_UF8, 256, flat, mo, true, cm);
+            uf8_decode8(cm, __fmul_rn(sc, 0.0078125f), mo);          // fl(scale / 128), scale >= 1e-12
+            int64_t cb0 = 0, cb1 = 0, next = row;
+            if (ANY) {
+                next = min(row + 1, sT.rows - 1);                    // (nothing valid follows the last row)
+                if (sT.batch_rows > 0) {                             // (rows < 2^31)
+                    cb0 = (int64_t)((uint32_t)row / (uint32_t)sT.batch_rows) * sT.cols;
+                    if (left < 8) cb1 = (int64_t)((uint32_t)next / (uint32_t)sT.batch_rows) * sT.cols;
+                }
+            }
+            const auto cols8 = [&](const float *v, float (&x)[8]) {
+                if (whole) load_f8_ro(v + cb0 + col, x);
+                else if (left == 8) load_cols8_shifted(v, cb0 + col, x);
+                else flat_cols_wrap(v, cb0, cb1, col, left, x);
+            };
+            cols8(sT.inv_col, ic);
+            const float ir = __ldg(sT.inv_row + row);
             if (L.came) {
-                float icc[8];
-                load_f8_ro(sT.inv_col_conf + col, icc);
-                const float2 irc2 = bc2(__ldg(sT.inv_row_conf + row));
+                cols8(sT.inv_col_conf, icc);
+                const float irc = __ldg(sT.inv_row_conf + row);
+                if (common) flat_update8<true, true>(g, mo, ic, icc, ir, ir, irc, irc, 8, sF.D, sF.LW, mj, u);
+                else flat_update8<true, false>(g, mo, ic, icc, ir, __ldg(sT.inv_row + next), irc, __ldg(sT.inv_row_conf + next), left, sF.D, sF.LW, mj, u);
+            } else {
+                if (common) flat_update8<false, true>(g, mo, ic, ic, ir, ir, ir, ir, 8, sF.D, sF.LW, mj, u);
+                else flat_update8<false, false>(g, mo, ic, ic, ir, __ldg(sT.inv_row + next), ir, ir, left, sF.D, sF.LW, mj, u);
+            }
+            if (ANY && nval < 8) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (j >= nval) { u[j] = 0.0f; mj[j] = 0.0f; }
+            }
+            const float2 decay2 = bc2(sT.decay), step2 = bc2(sF.step_mul), fira2 = bc2(sF.fira);
+            const bool zero_upd = sF.zero_upd;
+            if (PT == 0) {
+                float p[8] = {__uint_as_float(pa.x), __uint_as_float(pa.y), __uint_as_float(pa.z), __uint_as_float(pa.w),
+                              __uint_as_float(pb.x), __uint_as_float(pb.y), __uint_as_float(pb.z), __uint_as_float(pb.w)};
 #pragma unroll
                 for (int j = 0; j < 8; j += 2) {
-                    const float2 ut = div_by2(__fmul2_rn(__fmul2_rn(make_float2(g[j], g[j + 1]), ir2), make_float2(ic[j], ic[j + 1])), D);
-                    const float2 mm = lerp_w2(make_float2(mo[j], mo[j + 1]), ut, LW);
-                    const float2 uj = __fmul2_rn(__fmul2_rn(mm, irc2), make_float2(icc[j], icc[j + 1]));
-                    mj[j] = mm.x; mj[j + 1] = mm.y; u[j] = uj.x; u[j + 1] = uj.y;
+                    float2 pj = __fmul2_rn(make_float2(p[j], p[j + 1]), decay2);
+                    if (!zero_upd) pj = __ffma2_rn(step2, __fmul2_rn(make_float2(u[j], u[j + 1]), fira2), pj);
+                    p[j] = pj.x; p[j + 1] = pj.y;
+                }
+                uint16_t *const copy = static_cast<uint16_t *>(sT.param_copy);        // bf16 compute copy
+                if (!ANY || nval == 8) {
+                    float *pp = pbase + flat;
+                    *reinterpret_cast<float4 *>(pp) = make_float4(p[0], p[1], p[2], p[3]);
+                    *reinterpret_cast<float4 *>(pp + 4) = make_float4(p[4], p[5], p[6], p[7]);
+                    if (copy != nullptr)
+                        *reinterpret_cast<uint4 *>(copy + flat) =
+                            make_uint4(bf16x2_rn(p[0], p[1]), bf16x2_rn(p[2], p[3]), bf16x2_rn(p[4], p[5]), bf16x2_rn(p[6], p[7]));
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (j < nval) {
+                            pbase[flat + j] = p[j];
+                            if (copy != nullptr) copy[flat + j] = (uint16_t)f32_to_bf16_rn_bits(p[j]);
+                        }
                 }
             } else {
+                // rounded to bf16 after the decay and after the update, or once, stochastically (optimizer.py:873-881, 2033-2039)
+                const uint32_t w[4] = {pa.x, pa.y, pa.z, pa.w};
+                uint32_t o[4];
+                float2 x[4];
 #pragma unroll
-                for (int j = 0; j < 8; j += 2) {
-                    const float2 mm = lerp_w2(make_float2(mo[j], mo[j + 1]), make_float2(g[j], g[j + 1]), LW);
-                    const float2 uj = __fmul2_rn(__fmul2_rn(mm, ir2), make_float2(ic[j], ic[j + 1]));
-                    mj[j] = mm.x; mj[j + 1] = mm.y; u[j] = uj.x; u[j + 1] = uj.y;
+                for (int j = 0; j < 4; ++j) {
+                    x[j] = __fmul2_rn(make_float2(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xffff0000u)), decay2);
+                    if (PT == 1) {
+                        const uint32_t pk = bf16x2_rn(x[j].x, x[j].y);
+                        x[j] = make_float2(__uint_as_float(pk << 16), __uint_as_float(pk & 0xffff0000u));
+                    }
+                    float2 uu = __fmul2_rn(make_float2(u[2 * j], u[2 * j + 1]), fira2);
+                    if (zero_upd) uu = make_float2(0.0f, 0.0f);
+                    x[j] = __ffma2_rn(step2, uu, x[j]);
+                }
+                fast_round8<PT == 2, 0>(x, sT.sr_base, flat, 0, PT == 2 ? sr_counter(sT.sr_base, flat, 8) : SrCounter{}, o);
+                if (!ANY || nval == 8) *reinterpret_cast<uint4 *>(hbase + flat) = make_uint4(o[0], o[1], o[2], o[3]);
+                else {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (j < nval) hbase[flat + j] = (uint16_t)(o[j >> 1] >> (16 * (j & 1)));
                 }
             }
-            float *pp = pbase + flat;
-            float p[8] = {cp0.x, cp0.y, cp0.z, cp0.w, cp1.x, cp1.y, cp1.z, cp1.w};
-            const float2 decay2 = bc2(sT.decay), step2 = bc2(step_mul), fira2 = bc2(fira);
-#pragma unroll
-            for (int j = 0; j < 8; j += 2) {
-                float2 pj = __fmul2_rn(make_float2(p[j], p[j + 1]), decay2);
-                if (!zero_upd) pj = __ffma2_rn(step2, __fmul2_rn(make_float2(u[j], u[j + 1]), fira2), pj);
-                p[j] = pj.x; p[j + 1] = pj.y;
-            }
-            *reinterpret_cast<float4 *>(pp) = make_float4(p[0], p[1], p[2], p[3]);
-            *reinterpret_cast<float4 *>(pp + 4) = make_float4(p[4], p[5], p[6], p[7]);
-            if (sT.param_copy != nullptr)                                    // bf16 compute copy
-                *reinterpret_cast<uint4 *>(static_cast<uint16_t *>(sT.param_copy) + flat) =
-                    make_uint4(bf16x2_rn(p[0], p[1]), bf16x2_rn(p[2], p[3]), bf16x2_rn(p[4], p[5]), bf16x2_rn(p[6], p[7]));
-        } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) mj[j] = 0.0f;
         }
-        // one warp = one momentum block of 256 (the block exists iff its first element does)
-        const int64_t w0 = (id - sT.first_chunk) * 2048 + warp * 256;
         bool odd;
         const float am = m_absmax256(mj, odd);
         if (w0 < numel) {
             const uint2 codes = uf8_codes8(mj, am, odd);
-            if (ok) *reinterpret_cast<uint2 *>(sT.m_q + flat) = codes;
-            if (lane == 0) sT.m_scale[w0 / 256] = am;
+            if (ANY || ok) *reinterpret_cast<uint2 *>(sT.m_q + flat) = codes;        // (ANY: what lies beyond the end is coded as zero)
+            if (lane == 0) sT.m_scale[block] = am;
         }
     }
 }
 
 // ---------------------------------------------------------------------------
-// factored_apply_ring_kernel in tile order, for tables whose tensors all have cols % 256 == 0: a CTA takes a
+// The same pass over fp32 parameters in tile order, for tables whose tensors all have cols % 256 == 0: a CTA takes a
 // 512 x 256 statistic tile, warp w its rows r0 + w, r0 + w + 8, ...; a row slice of 256 columns is 256
 // consecutive elements that start on a multiple of 256, i.e. exactly one momentum block, so the warp still owns
 // its block's absmax.  What changes is that a lane works on the same 8 columns for the whole tile and keeps
 // their inverse column factors (and CAME's confidence factors) in registers instead of loading 32 or 64 bytes
-// of them for every 8 elements.  Ring, arithmetic and stores as in factored_apply_ring_kernel; the copies of
+// of them for every 8 elements.  Ring, arithmetic and stores as above; the copies of
 // a warp run FRING_STAGES - 1 rows ahead inside a tile.
 // ---------------------------------------------------------------------------
 template <typename GradT, int CTAS>
@@ -2827,21 +2929,24 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
         AF8_CUDA_TRY(cudaGetLastError());
         return AF8_OK;
     }
-    if (vec && !any && cfg->mode == AF8_FUPD_APPLY && cfg->m_fmt == AF8_M_UF8 && cfg->param_dtype == AF8_F32 && !ring_off) {
-        // fp32 parameters, UF8 momentum: inputs through per-warp rings of bulk copies
-        if (bf) {
-            AF8_CUDA_TRY(cudaFuncSetAttribute(factored_apply_ring_kernel<bf16_tag, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fring_smem_bytes<bf16_tag>()));
-            factored_apply_ring_kernel<bf16_tag, 3><<<(int)grid, FUPD_THREADS, fring_smem_bytes<bf16_tag>(), cst>>>(L);
-        } else {
-            grid = std::min<int64_t>((int64_t)sm_count() * 2, total_chunks);
-            AF8_CUDA_TRY(cudaFuncSetAttribute(factored_apply_ring_kernel<float, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fring_smem_bytes<float>()));
-            factored_apply_ring_kernel<float, 2><<<(int)grid, FUPD_THREADS, fring_smem_bytes<float>(), cst>>>(L);
-        }
+    // (see PT: bf16 gradients with bf16 parameters have kernels of their own)
+    const int pt = cfg->param_dtype == AF8_F32 ? 0 : (bf && cfg->param_dtype == AF8_BF16 && !lag) ? (cfg->stochastic_round ? 2 : 1) : 3;
+    if (vec && cfg->mode == AF8_FUPD_APPLY && cfg->m_fmt == AF8_M_UF8 && pt != 3 && !ring_off) {
+        // UF8 momentum: inputs through per-warp rings of bulk copies
+        grid = std::min<int64_t>((int64_t)sm_count() * (bf ? (any ? FLAT_ANY_CTAS : 3) : 2), total_chunks);
+#define AF8_LAUNCH_FLAT(G, T, A) do { \
+        AF8_CUDA_TRY(cudaFuncSetAttribute(factored_apply_flat_kernel<G, T, A>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fring_smem_bytes<G, T>())); \
+        factored_apply_flat_kernel<G, T, A><<<(int)grid, FUPD_THREADS, fring_smem_bytes<G, T>(), cst>>>(L); } while (0)
+#define AF8_LAUNCH_FLAT_ANY(G, T) do { if (any) AF8_LAUNCH_FLAT(G, T, true); else AF8_LAUNCH_FLAT(G, T, false); } while (0)
+        if (!bf) AF8_LAUNCH_FLAT_ANY(float, 0);
+        else if (pt == 0) AF8_LAUNCH_FLAT_ANY(bf16_tag, 0);
+        else if (pt == 1) AF8_LAUNCH_FLAT_ANY(bf16_tag, 1);
+        else AF8_LAUNCH_FLAT_ANY(bf16_tag, 2);
+#undef AF8_LAUNCH_FLAT_ANY
+#undef AF8_LAUNCH_FLAT
         AF8_CUDA_TRY(cudaGetLastError());
         return AF8_OK;
     }
-    // (see PT: bf16 gradients with bf16 parameters have kernels of their own)
-    const int pt = cfg->param_dtype == AF8_F32 ? 0 : (bf && cfg->param_dtype == AF8_BF16 && !lag) ? (cfg->stochastic_round ? 2 : 1) : 3;
 #define AF8_LAUNCH_FUPD(G, P, C, A, T) factored_update_vec_kernel<G, P, C, A, T><<<(int)grid, FUPD_THREADS, 0, cst>>>(L)
 #define AF8_LAUNCH_FUPD_PT(P, C, A) do { \
         if (bf && pt == 0) AF8_LAUNCH_FUPD(bf16_tag, P, C, A, 0); else if (bf && pt == 3) AF8_LAUNCH_FUPD(bf16_tag, P, C, A, 3); \

@@ -114,6 +114,11 @@ EXTRA_CASES.update({
     "adafactor_m_slices_f32_w": dict(shapes=_SLICES, steps=3, seed=68, grad=_F32, hp=dict(cases.CASES["adafactor_factored_m"]["hp"], beta1=0.4)),
     "adafactor_m_slices_8": dict(shapes=[(39, 264), (520, 776), (1030, 520)], steps=3, seed=69, grad=cases.CASES["adafactor_factored_m"]["grad"],
                                  hp=dict(cases.CASES["adafactor_factored_m"]["hp"], maximize=True)),
+    # the write pass in flat order over whole vectors with that form of lerp; chunks that end a tensor; row ends in a third of the warps
+    "came_flat_w": dict(shapes=[(200, 520), (70, 264), (9, 2056)], steps=3, seed=70, grad=cases.CASES["came_al16"]["grad"],
+                        hp=dict(cases.CASES["came_al16"]["hp"], beta1=0.4)),
+    "came_flat_any": dict(shapes=[(300, 747), (2, 70, 2051), (33, 4099)], steps=3, seed=71, grad=cases.CASES["came_al16"]["grad"],
+                          hp=cases.CASES["came_al16"]["hp"]),
 })
 
 # lag_norm=True (one pass with the previous step's norm; optimizer.py:1056-1071): the vector kernels, the
