@@ -230,6 +230,19 @@ class _PinnedRing:
                 retired.append((buf, ev))
 
 
+def _update_scalars(static, last, scalars, names):
+    """Bring the scalar fields of a launch table's template up to date: those that differ from `last`, what they hold (one value for
+    the table each; arrays of one value per tensor are always written).  Most of them are the same step after step, and storing
+    one into a structured array costs more than comparing it."""
+    for k in names:
+        v = scalars[k]
+        if isinstance(v, np.ndarray):
+            static[k] = v
+            last.pop(k, None)
+        elif last.get(k) != v:
+            static[k] = last[k] = v
+
+
 class FullrankKey(tuple):
     """(grad_dtype, v_fmt, m_fmt, block, m_block, use_adam_denom, momentum_only, negate)"""
 
@@ -335,13 +348,14 @@ class FullrankPlan:
         if self._static is None or sig != self._ptr_sig:
             self._static = self._static_fields()
             self._ptr_sig = sig
+            self._last = {}
+        _update_scalars(self._static, self._last, scalars, ("decay", "alpha", "v_w", "v_keep", "v_eps_add", "m_w", "eps_gradsq", "eps_denom", "eps_sq"))
         buf = self.h_table.next()
         table = self.h_table.table(N.FULLRANK_TENSOR, self.n)
         table[:] = self._static
         table["grad"] = [g.data_ptr() for g in grads]
-        for k in ("decay", "alpha", "v_w", "v_keep", "v_eps_add", "m_w", "eps_gradsq", "eps_denom", "eps_sq"):
-            table[k] = scalars[k]
-        table["sr_base"] = scalars.get("sr_base", 0)
+        if "sr_base" in scalars:
+            table["sr_base"] = scalars["sr_base"]
         if self.cfg.use_adam_denom:
             eps = scalars["eps_denom"]
             eps = float(eps.min()) if isinstance(eps, np.ndarray) else float(eps)
@@ -861,6 +875,8 @@ class FactoredPlan:
         if self._static is None or sig != self._ptr_sig:
             self._static = self._static_fields()
             self._ptr_sig = sig
+            self._last = {}
+        _update_scalars(self._static, self._last, scalars, ("decay", "alpha", "v_w", "m_w", "c_w", "eps1", "eps_came"))
         buf = self.h_table.next()
         tables = self.h_table.table(N.FACTORED_TENSOR, self.n_tables * self.n).reshape(self.n_tables, self.n)
         tables[:] = self._static
@@ -868,12 +884,10 @@ class FactoredPlan:
         table["grad"] = [g.data_ptr() for g in grads]
         if self._any_rows:
             self.cfg.aligned8 = 2 if self._static_aligned and not (table["grad"] & np.uint64(15)).any() else 0
-        for k in ("decay", "alpha", "v_w", "m_w", "c_w", "eps1", "eps_came"):
-            table[k] = scalars[k]
-        table["sr_base"] = scalars.get("sr_base", 0)
+        if "sr_base" in scalars:
+            table["sr_base"] = scalars["sr_base"]
         for k in range(1, self.n_tables):
-            for name in ("grad", "decay", "alpha", "v_w", "m_w", "c_w", "eps1", "eps_came"):
-                tables[k][name] = table[name]
+            tables[k]["grad"] = table["grad"]
         lib = N.lib()
         for k in range(self.n_tables):
             N.check(lib.af8_factored_upload(ctypes.byref(self.cfg), buf.data_ptr() + k * self.n * N.FACTORED_TENSOR.itemsize,

@@ -14,6 +14,7 @@ compatibility and ignored.
 """
 import logging
 import math
+import operator
 from typing import Any, Dict, Iterable, Optional, Tuple, Union
 
 import numpy as np
@@ -39,6 +40,15 @@ _FLOOR = 1.17549435e-38                                   # optimizer.py:23
 _M_TYPES = ("uf4", "uf8", "d4", "d8", "fp32")              # optimizer.py:24
 _V_TYPES = ("al8", "al16", "fp32")                         # optimizer.py:25
 f32 = np.float32
+
+
+class _Launch:
+    """What one launch plan is to step: parameters, their gradients and states.  cached: params and states are the lists of the
+    group's cache, the same objects at every step until the group is sorted again."""
+    __slots__ = ("params", "grads", "states", "cached")
+
+    def __init__(self, params, grads, states, cached):
+        self.params, self.grads, self.states, self.cached = params, grads, states, cached
 
 
 def _pad_to(n, block):
@@ -746,23 +756,16 @@ class Adafactor8Bit(Optimizer):
         params = group["params"]
         gsig = self._group_signature(group) + (bool(group.get("stochastic_round_writeback", False)),)
         c = self._group_cache.get(gi)
-        if c is not None and c["gsig"] == gsig and len(c["params"]) == len(params):
-            grads = []
-            for p, q, kind in zip(params, c["params"], c["kinds"]):
-                g = p.grad
-                if p is not q or ((None if g is None else (g.dim(), g.dtype)) != kind):
-                    grads = None
-                    break
-                grads.append(g)
-            if grads is not None:
-                states = c["states"]
-                return [fn(gi, group, key, [(params[j], grads[j], states[j]) for j in idx])
-                        for fn, key, idx in c["launches"]], ()
-        entries, copy_back, kinds, states, cacheable = [], [], [], [], True
+        if c is not None and c["gsig"] == gsig and len(c["params"]) == len(params) and all(map(operator.is_, params, c["params"])):
+            grads = [p.grad for p in params]
+            if [None if g is None else g.dtype for g in grads] == c["dtypes"] and [None if g is None else g.dim() for g in grads] == c["dims"]:
+                return [fn(gi, group, key, _Launch(ps, [grads[j] for j in idx], sts, True))
+                        for fn, key, idx, ps, sts in c["launches"]], ()
+        entries, copy_back, dtypes, dims, cacheable = [], [], [], [], True
         for j, p in enumerate(params):
             g = p.grad
-            kinds.append(None if g is None else (g.dim(), g.dtype))
-            states.append(None)
+            dtypes.append(None if g is None else g.dtype)
+            dims.append(None if g is None else g.dim())
             if g is None:
                 continue
             if not p.is_cuda:
@@ -781,7 +784,6 @@ class Adafactor8Bit(Optimizer):
                     # launches of this step may be queued already, stay)
                     for k in [k for k in self._plans if k[0] == gi]:
                         del self._plans[k]
-            states[j] = state
             if group.get("stochastic_round_writeback", False) and p.dtype in (torch.bfloat16, torch.float16):
                 self._sr_seed(state, p)     # seeds follow the parameter order of the step (optimizer.py:1889-1892)
             if p.numel() == 0:              # an empty parameter has a state and a step count, nothing to launch
@@ -797,9 +799,11 @@ class Adafactor8Bit(Optimizer):
         launches = self._sort_group(group, entries)
         self._group_cache.pop(gi, None)
         if cacheable:
-            self._group_cache[gi] = dict(gsig=gsig, params=list(params), kinds=kinds, states=states,
-                                         launches=[(fn, key, [e[0] for e in items]) for fn, key, items in launches])
-        return [fn(gi, group, key, [(p, g, st) for _, p, g, st in items]) for fn, key, items in launches], copy_back
+            self._group_cache[gi] = dict(gsig=gsig, params=list(params), dtypes=dtypes, dims=dims,
+                                         launches=[(fn, key, [e[0] for e in items], [e[1] for e in items], [e[3] for e in items])
+                                                   for fn, key, items in launches])
+        return [fn(gi, group, key, _Launch([e[1] for e in items], [e[2] for e in items], [e[3] for e in items], False))
+                for fn, key, items in launches], copy_back
 
     def _sort_group(self, group, entries):
         """Sort (index, parameter, gradient, state) entries into launch groups ->
@@ -892,7 +896,8 @@ class Adafactor8Bit(Optimizer):
             state["_proj_T"] = proj_t      # same values the reference would regenerate each step
         return proj_t
 
-    def _run_apollo(self, gi, group, key, items):
+    def _run_apollo(self, gi, group, key, launch):
+        items = list(zip(launch.params, launch.grads, launch.states))
         rank = int(group["apollo_rank"])
         beta1, beta2 = group.get("beta1"), group["beta2"]
         beta3 = group.get("beta3")
@@ -1035,38 +1040,54 @@ class Adafactor8Bit(Optimizer):
         elif sc["bc_div"] is not None:
             scale["bc"][i], scale["bc_mode"][i] = sc["bc_div"], 2
 
-    def _run_factored(self, gi, group, key, items):
-        device, gdtype, m_fmt, m_block, came, pdtype = key[:6]
-        sr = bool(group.get("stochastic_round_writeback", False)) and pdtype in (torch.bfloat16, torch.float16)
-        ids = tuple(id(p) for p, _, _ in items)
-        pkey = (gi, "factored", key, bool(group["maximize"]), sr)
+    def _plan_of(self, pkey, launch, make):
+        """The launch plan under pkey if it is one for the launch's parameters, else make(pieces).  A launch out of the group's
+        cache knows its plan by the list of parameters that both hold; any other compares the parameters."""
         plan = self._plans.get(pkey)
-        pcs = [self._pieces.get(id(p)) for p, _, _ in items]
+        if plan is not None and launch.cached and plan.owner is launch.params:
+            return plan
+        ids = tuple(map(id, launch.params))
         if plan is None or plan.ids != ids:
-            v_fmts = [(st.get("v_quant_type", "al8") if st.get("is_quantized", False) else "fp32") for _, _, st in items]
-            c_fmts = [(st.get("c_quant_type", st.get("v_quant_type", "al8")) if st.get("is_quantized", False) else "fp32")
-                      for _, _, st in items]
-            plan = FactoredPlan(device, gdtype, m_fmt, m_block, came, group["maximize"],
-                                [p for p, _, _ in items], [s for _, _, s in items], v_fmts, c_fmts, stochastic_round=sr,
-                                pieces=pcs)
+            plan = make([self._pieces.get(i) for i in ids])
             plan.ids = ids
             self._plans[pkey] = plan
-        n = len(items)
-        scale = self._scale_inputs(group, n) if group["scale_parameter"] else None
-        steps = []
-        for _, _, st in items:
-            step = st["step"] + 1
+        plan.owner = launch.params if launch.cached else None
+        return plan
+
+    @staticmethod
+    def _next_steps(states):
+        """Count every state's step -> the step numbers."""
+        steps = [st["step"] + 1 for st in states]
+        for st, step in zip(states, steps):
             st["step"] = step
-            steps.append(step)
+        return steps
+
+    def _sr_bases(self, plan, launch, steps):
+        """Counter origins of the stochastic rounding.  A part of a tensor draws the counters of its elements in the whole tensor."""
+        return np.array([(sr_base(self._sr_seed(st), step) + (pc.elem0 if pc is not None else 0)) & 0xFFFFFFFFFFFFFFFF
+                         for st, step, pc in zip(launch.states, steps, plan.pieces)], dtype=np.uint64)
+
+    def _run_factored(self, gi, group, key, launch):
+        device, gdtype, m_fmt, m_block, came, pdtype = key[:6]
+        sr = bool(group.get("stochastic_round_writeback", False)) and pdtype in (torch.bfloat16, torch.float16)
+
+        def make(pieces):
+            v_fmts = [(st.get("v_quant_type", "al8") if st.get("is_quantized", False) else "fp32") for st in launch.states]
+            c_fmts = [(st.get("c_quant_type", st.get("v_quant_type", "al8")) if st.get("is_quantized", False) else "fp32")
+                      for st in launch.states]
+            return FactoredPlan(device, gdtype, m_fmt, m_block, came, group["maximize"], launch.params, launch.states, v_fmts, c_fmts,
+                                stochastic_round=sr, pieces=pieces)
+
+        plan = self._plan_of((gi, "factored", key, bool(group["maximize"]), sr), launch, make)
+        n = len(launch.params)
+        scale = self._scale_inputs(group, n) if group["scale_parameter"] else None
+        steps = self._next_steps(launch.states)
         uniform = steps.count(steps[0]) == n          # the usual case: every tensor of the group is at the same step
         # (one value per field then, else one per tensor)
         cols = {} if uniform else {k: np.empty(n, dtype=f32) for k in ("decay", "alpha", "v_w", "m_w", "c_w", "eps1", "eps_came")}
-        grads = [g if g.is_contiguous() else g.contiguous() for _, g, _ in items]
-        if sr:                      # a part of a tensor draws the counters of its elements in the whole tensor
-            cols["sr_base"] = np.zeros(n, dtype=np.uint64)
-            for i, (_, _, st) in enumerate(items):
-                first = pcs[i].elem0 if pcs[i] is not None else 0
-                cols["sr_base"][i] = (sr_base(self._sr_seed(st), steps[i]) + first) & 0xFFFFFFFFFFFFFFFF
+        grads = [g if g.is_contiguous() else g.contiguous() for g in launch.grads]
+        if sr:
+            cols["sr_base"] = self._sr_bases(plan, launch, steps)
         for i in ([0] if uniform else range(n)):
             where = slice(None) if uniform else i
             sc = self._step_scalars(group, steps[i])
@@ -1086,7 +1107,7 @@ class Adafactor8Bit(Optimizer):
         return (factored_exchanges(came, d, fira, lag), device,
                 plan.stages(grads, cols, d=d, fira=fira, fira_margin=float(group.get("fira_margin", 0.01)), scale=scale, lag=lag))
 
-    def _run_fullrank(self, gi, group, key, items):
+    def _run_fullrank(self, gi, group, key, launch):
         device, gdtype, v_fmt, m_fmt, block, m_block, pdtype = key
         sr = bool(group.get("stochastic_round_writeback", False)) and pdtype in (torch.bfloat16, torch.float16)
         adam = (not group.get("factored", True)) and group["beta2"] is not None and group.get("beta3") is None   # (as _step_scalars)
@@ -1096,17 +1117,10 @@ class Adafactor8Bit(Optimizer):
         sgd = v_fmt == "none"
         if sgd:
             momentum_only = False
-        ids = tuple(id(p) for p, _, _ in items)
-        pkey = (gi, "fullrank", key, bool(momentum_only), bool(group["maximize"]), sr)
-        plan = self._plans.get(pkey)
-        pcs = [self._pieces.get(id(p)) for p, _, _ in items]
-        if plan is None or plan.ids != ids:
-            plan = FullrankPlan(device, gdtype, v_fmt, m_fmt, block, m_block, adam, momentum_only,
-                                group["maximize"], [p for p, _, _ in items], [s for _, _, s in items],
-                                stochastic_round=sr, pieces=pcs)
-            plan.ids = ids
-            self._plans[pkey] = plan
-        n = len(items)
+        plan = self._plan_of((gi, "fullrank", key, bool(momentum_only), bool(group["maximize"]), sr), launch,
+                             lambda pieces: FullrankPlan(device, gdtype, v_fmt, m_fmt, block, m_block, adam, momentum_only, group["maximize"],
+                                                         launch.params, launch.states, stochastic_round=sr, pieces=pieces))
+        n = len(launch.params)
         scale = None
         if group["scale_parameter"]:
             scale = {k: np.zeros(n, dtype=f32) for k in ("rho", "eps2", "bc", "weight_decay")}
@@ -1122,20 +1136,13 @@ class Adafactor8Bit(Optimizer):
                         f32(1.0 - group["beta1"]) if group.get("beta1") is not None else f32(0.0),
                         f32(sc["eps_gradsq"]), f32(sc["eps_denom"]), f32(sc["eps_sq"]))
 
-        steps = []
-        for _, _, st in items:
-            step = st["step"] + 1
-            st["step"] = step
-            steps.append(step)
+        steps = self._next_steps(launch.states)
         uniform = steps.count(steps[0]) == n          # the usual case: every tensor of the group is at the same step
         # (one value per field then, else one per tensor)
         cols = {} if uniform else {k: np.empty(n, dtype=f32) for k in _FULLRANK_COLS}
-        grads = [g if g.is_contiguous() else g.contiguous() for _, g, _ in items]
-        if sr:                      # a part of a tensor draws the counters of its elements in the whole tensor
-            cols["sr_base"] = np.zeros(n, dtype=np.uint64)
-            for i, (_, _, st) in enumerate(items):
-                first = pcs[i].elem0 if pcs[i] is not None else 0
-                cols["sr_base"][i] = (sr_base(self._sr_seed(st), steps[i]) + first) & 0xFFFFFFFFFFFFFFFF
+        grads = [g if g.is_contiguous() else g.contiguous() for g in launch.grads]
+        if sr:
+            cols["sr_base"] = self._sr_bases(plan, launch, steps)
         cache = {}
         for i in ([0] if uniform else range(n)):
             step = steps[i]

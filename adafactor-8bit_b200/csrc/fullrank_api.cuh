@@ -8,6 +8,8 @@
 #include "fullrank_generic.cuh"
 #include "fullrank_stat.cuh"
 
+#include <atomic>
+
 namespace af8 {
 
 // ---------------------------------------------------------------------------
@@ -126,12 +128,28 @@ lag_scalars_kernel(const af8_lag_tensor *tensors, int phase, const void *block_s
 // ---------------------------------------------------------------------------
 // launch helpers
 // ---------------------------------------------------------------------------
+// Resident CTAs of a kernel launched with fixed threads and shared memory, by device: asked once (the question costs a small step's
+// launch more than the launch itself).
+struct ResidentCtas { std::atomic<int> of_device[64]; };
 template <typename K>
-inline int persistent_grid(K kernel, int threads, size_t smem, int64_t total_blocks, int *grid_out)
+inline int resident_ctas(K kernel, int threads, size_t smem, ResidentCtas *known, int *per_sm)
+{
+    int dev = -1;
+    AF8_CUDA_TRY(cudaGetDevice(&dev));
+    std::atomic<int> *const slot = known && dev >= 0 && dev < 64 ? &known->of_device[dev] : nullptr;
+    *per_sm = slot ? slot->load(std::memory_order_relaxed) : 0;
+    if (*per_sm > 0) return AF8_OK;
+    AF8_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, threads, smem));
+    if (*per_sm < 1) return fail(AF8_ERR_CUDA, "kernel does not fit on an SM (threads=%d smem=%zu)", threads, smem);
+    if (slot) slot->store(*per_sm, std::memory_order_relaxed);
+    return AF8_OK;
+}
+template <typename K>
+inline int persistent_grid(K kernel, int threads, size_t smem, int64_t total_blocks, int *grid_out, ResidentCtas *known = nullptr)
 {
     int per_sm = 0;
-    AF8_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
-    if (per_sm < 1) return fail(AF8_ERR_CUDA, "kernel does not fit on an SM (threads=%d smem=%zu)", threads, smem);
+    const int rc = resident_ctas(kernel, threads, smem, known, &per_sm);
+    if (rc) return rc;
     int64_t g = (int64_t)per_sm * sm_count();
     if (g > total_blocks) g = total_blocks;
     *grid_out = (int)g;
@@ -149,7 +167,8 @@ inline int launch_fast(const FullrankLaunch &L, cudaStream_t st)
     AF8_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                       (int)cudaSharedmemCarveoutMaxShared));
     int grid = 0;
-    int rc = persistent_grid(kernel, FAST_THREADS, Ring::SMEM_BYTES, L.total_blocks, &grid);
+    static ResidentCtas known;
+    int rc = persistent_grid(kernel, FAST_THREADS, Ring::SMEM_BYTES, L.total_blocks, &grid, &known);
     if (rc) return rc;
     kernel<<<grid, FAST_THREADS, Ring::SMEM_BYTES, st>>>(L);
     AF8_CUDA_TRY(cudaGetLastError());
@@ -160,9 +179,10 @@ template <typename GradT, int VB, int MF>
 inline int launch_stat(const FullrankLaunch &L, cudaStream_t st)
 {
     auto kernel = fullrank_stat_kernel<GradT, VB, MF>;
+    static ResidentCtas known;
     int per_sm = 0;
-    AF8_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, STAT_THREADS, 0));
-    if (per_sm < 1) return fail(AF8_ERR_CUDA, "statistic kernel does not fit on an SM");
+    const int rc = resident_ctas(kernel, STAT_THREADS, 0, &known, &per_sm);
+    if (rc) return rc;
     const int64_t warps_per_cta = STAT_THREADS / 32;
     int64_t grid = (int64_t)per_sm * sm_count();
     const int64_t need = (L.total_blocks + warps_per_cta - 1) / warps_per_cta;
@@ -180,7 +200,8 @@ inline int launch_generic_threads(const FullrankLaunch &L, const GenericCfg &C, 
     if (smem > 48 * 1024)
         AF8_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int grid = 0;
-    int rc = persistent_grid(kernel, THREADS, smem, L.total_blocks, &grid);
+    static ResidentCtas known;                        // (of the plain form, whose shared memory is fixed)
+    int rc = persistent_grid(kernel, THREADS, smem, L.total_blocks, &grid, plain ? &known : nullptr);
     if (rc) return rc;
     kernel<<<grid, THREADS, smem, st>>>(L, C);
     AF8_CUDA_TRY(cudaGetLastError());
