@@ -64,6 +64,15 @@ inline int sm_count()
     return cached_sms;
 }
 
+// Lets a kernel be launched with this much dynamic shared memory.  48 KB without the opt-in hold the kernel's static shared memory
+// too; no kernel here has 16 KB of that.
+template <typename K>
+inline int allow_dynamic_smem(K kernel, size_t bytes)
+{
+    if (bytes > 32 * 1024) AF8_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    return AF8_OK;
+}
+
 // ---------------------------------------------------------------------------
 // device: scalar primitives
 // ---------------------------------------------------------------------------

@@ -197,8 +197,8 @@ inline int launch_generic_threads(const FullrankLaunch &L, const GenericCfg &C, 
 {
     const size_t smem = plain ? 0 : (size_t)2 * C.block * sizeof(float);       // (only quantised states are staged)
     auto kernel = fullrank_generic_kernel<GradT, MODE, THREADS>;
-    if (smem > 48 * 1024)
-        AF8_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int rs = allow_dynamic_smem(kernel, smem);
+    if (rs) return rs;
     int grid = 0;
     static ResidentCtas known;                        // (of the plain form, whose shared memory is fixed)
     int rc = persistent_grid(kernel, THREADS, smem, L.total_blocks, &grid, plain ? &known : nullptr);

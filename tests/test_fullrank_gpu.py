@@ -239,6 +239,25 @@ def test_config0_full_size_is_exact(fira, oracle):
         parity.assert_params(param.detach().cpu().numpy(), op, f"step {t} param", tol=1e-6)
 
 
+@pytest.mark.parametrize("v", ["al8", "al16"])
+@pytest.mark.parametrize("blocks", [2, 300])
+@pytest.mark.parametrize("block", [5632, 5888, 6016, 6144, 8192])
+def test_blocks_around_48_kb_of_shared_memory(block, blocks, v, oracle):
+    """A block's logarithms and momentum wait in 8 bytes of dynamic shared memory an element: at 6144 elements 48 KB, the most a
+    launch gets without opting in, less the kernel's static share.  Tables of up to two blocks per SM and larger ones run with
+    different numbers of threads."""
+    hp = dict(cases.CASES["adamw_uf8_al8"]["hp"], block_size=block, m_block_size=128, v_quant_type=v, min_8bit_size=1)
+    case = dict(shapes=[(blocks * block - 77,)], steps=2, seed=81, hp=hp, grad=dict(dist="normal", std=1e-2, zero_frac=0.01))
+    run = OracleRun("long blocks", case=case)
+    params, opt = make_optimizer(run)
+    for t in (1, 2):
+        params[0].grad = to_cuda_grad(run.grads[t][0], params[0].shape)
+        opt.step()
+        run.step()
+        torch.cuda.synchronize()
+        compare_state(f"{block} {v}", t, 0, opt.state[params[0]], run.states[0], params[0], run.params[0], strict=False)
+
+
 def test_device_status_is_clean_after_the_runs_above():
     from adafactor8bit import _native
     assert _native.device_status(torch.cuda.current_stream().cuda_stream) == 0
