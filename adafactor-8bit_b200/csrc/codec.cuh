@@ -137,8 +137,8 @@ extern "C" int af8_al_quant(const float *x, int64_t numel, int32_t block, int32_
     if (numel <= 0 || block <= 0 || (bits != 8 && bits != 16)) return fail(AF8_ERR_INVALID, "af8_al_quant: bad size or bits");
     if (block > 4 * GEN_MAX_BLOCK) return fail(AF8_ERR_UNSUPPORTED, "af8_al_quant: block %d too large", block);
     const size_t smem = sizeof(float) * (size_t)block;
-    if (smem > 48 * 1024)
-        AF8_CUDA_TRY(cudaFuncSetAttribute(al_quant_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int rc = allow_dynamic_smem(al_quant_kernel, smem);
+    if (rc) return rc;
     const int64_t nblocks = (numel + block - 1) / block;
     al_quant_kernel<<<grid_for(nblocks, 1), 256, smem, static_cast<cudaStream_t>(stream)>>>(x, numel, block, bits, floor_log, q, scale, min_log);
     AF8_CUDA_TRY(cudaGetLastError());

@@ -258,6 +258,23 @@ def test_blocks_around_48_kb_of_shared_memory(block, blocks, v, oracle):
         compare_state(f"{block} {v}", t, 0, opt.state[params[0]], run.states[0], params[0], run.params[0], strict=False)
 
 
+@pytest.mark.parametrize("bits", [8, 16])
+@pytest.mark.parametrize("block", [12160, 12288, 12416])
+def test_quantiser_around_48_kb_of_shared_memory(block, bits, oracle):
+    """af8_al_quant keeps a block's logarithms in 4 bytes of dynamic shared memory an element, 48 KB at 12288 elements."""
+    from adafactor8bit import _native as N
+    x = (np.random.default_rng(82).standard_normal(2 * block + 100) ** 2).astype(np.float32)
+    q, scale, min_log, _ = oracle.al_quantize(x, block, bits=bits)
+    d_x = torch.from_numpy(x).cuda()
+    d_q = torch.zeros(q.size, dtype=torch.uint8 if bits == 8 else torch.int16, device="cuda")
+    d_s, d_m = torch.zeros(3, device="cuda"), torch.zeros(3, device="cuda")
+    N.check(N.lib().af8_al_quant(d_x.data_ptr(), x.size, block, bits, -126.0, d_q.data_ptr(), d_s.data_ptr(), d_m.data_ptr(),
+                                 torch.cuda.current_stream().cuda_stream), "af8_al_quant")
+    torch.cuda.synchronize()
+    parity.assert_codes(state_np({"q": d_q}, "q"), q, f"{block}/{bits}", al16=bits == 16)
+    assert int(parity.ulp_diff(d_s.cpu().numpy(), scale).max()) <= 1 and int(parity.ulp_diff(d_m.cpu().numpy(), min_log).max()) <= 1
+
+
 def test_device_status_is_clean_after_the_runs_above():
     from adafactor8bit import _native
     assert _native.device_status(torch.cuda.current_stream().cuda_stream) == 0
