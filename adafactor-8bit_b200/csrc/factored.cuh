@@ -1063,7 +1063,7 @@ __device__ __forceinline__ void residual_x8(const float (&g)[8], uint2 codes, fl
 //   SLICE_RESIDUAL  of CAME's residual; the sign of a negated gradient rides on the row factor ((-g) * r == g * (-r) bit for bit)
 //   SLICE_SUM_U     sum of squares of u = g * inv_row * inv_col
 //   SLICE_SUM_M     the same with the momentum after its EMA in place of g
-// The residual wants a momentum weight below 1/2 (the form of lerp) and a clip divisor of at least 1, or NaN.
+// The residual wants a clip divisor of at least 1, or NaN.
 enum { SLICE_GRADSQ = 0, SLICE_RESIDUAL = 1, SLICE_SUM_U = 2, SLICE_SUM_M = 3 };
 template <typename GradT> __host__ __device__ constexpr int slice_g_bytes() { return 256 * sizeof_grad<GradT>() + 16; }
 template <typename GradT> __host__ __device__ constexpr int slice_row_bytes() { return slice_g_bytes<GradT>() + 256 + 16; }
@@ -1073,7 +1073,8 @@ template <typename GradT> __host__ __device__ constexpr size_t slice_smem_bytes(
 
 // false after a time-out.  cacc: the lane's column sums; total: the sum of squares (by_eight: eight squares are added in binary32
 // before they enter binary64).  FORM: SLICE_RESIDUAL: the clip divisor is 1; SLICE_SUM_M: the momentum's weight is below 1/2.
-template <typename GradT, int MODE, bool VEC, bool FORM>
+// SMALL: SLICE_RESIDUAL: the momentum's weight is below 1/2 (the form of lerp).
+template <typename GradT, int MODE, bool VEC, bool FORM, bool SMALL = true>
 __device__ __forceinline__ bool slice_rows(const FactoredLaunch &L, const af8_factored_tensor &sT, int64_t r0, int64_t r_end, int64_t c0,
                                            float pre_div, bool by_eight, const float (&ic)[8], double (&cacc)[8], double &total,
                                            unsigned char *ring, uint64_t *full, uint32_t &cons)
@@ -1201,7 +1202,7 @@ __device__ __forceinline__ bool slice_rows(const FactoredLaunch &L, const af8_fa
                         x[j] = xx.x; x[j + 1] = xx.y;
                     }
                 } else if (MODE == SLICE_RESIDUAL) {
-                    residual_m8<FORM, true>(gv[q], mo[q], irv[q], ic, D, LW.ww, eps, x);
+                    residual_m8<FORM, SMALL>(gv[q], mo[q], irv[q], ic, D, LW.ww, eps, x);
                 } else {
                     const float2 ir2 = bc2(irv[q]), ww2 = bc2(LW.ww);
 #pragma unroll
@@ -1434,10 +1435,13 @@ factored_stats_vec_kernel(const FactoredLaunch L, const CUtensorMap *__restrict_
         // Whole rows of vectors or not; which of the row loops.  Rows of any length take the slices in both passes, whole vectors
         // in the residual pass (339 M parameters in rows of 2000: direct loads 875 us, slices 472; of 1999: 1189 and 579); the g*g pass over whole vectors was slower through a ring (3.0 -> 4.3 ms on Llama-2-7B) and loads directly.
         const bool vec = !ANY || (C & 7) == 0;
+        // A momentum weight of 1/2 or more takes the other form of lerp.  (Direct loads and slices: 202 M parameters with binary32
+        // gradients in rows of 256 n 528 and 277 us, 235 M bf16 ones in rows of which some are such 638 and 341.)
         bool slices = IN == 1 && (RESIDUAL || !vec);
+        const bool small = !RESIDUAL || fabsf(sT.m_w) < 0.5f;                    // (uniform over the tensor)
         if (RESIDUAL) {
             pre_div = L.dyn[t].pre_div;
-            slices = slices && L.m_fmt == AF8_M_UF8 && L.m_block == 256 && !(pre_div < 1.0f) && fabsf(sT.m_w) < 0.5f;
+            slices = slices && L.m_fmt == AF8_M_UF8 && L.m_block == 256 && !(pre_div < 1.0f) && (!ANY || small);
             if (slices && !vec) slice_cols<false>(sT.inv_col + P.cb, c0, C, ic);
             else if (!vec) load_cols_any(sT.inv_col + P.cb, c, C, ic);
             else if (col_ok) load_f8_ro(sT.inv_col + P.cb + c, ic);
@@ -1449,7 +1453,7 @@ factored_stats_vec_kernel(const FactoredLaunch L, const CUtensorMap *__restrict_
         if constexpr (IN == 2) {
             if (!(pre_div < 1.0f)) {                                             // boxes of rows through tensor maps
                 boxes = true;
-                const bool one = pre_div == 1.0f, small = fabsf(sT.m_w) < 0.5f;  // (uniform over the tensor)
+                const bool one = pre_div == 1.0f;
                 unsigned char *ring = sr_smem + (size_t)warp * slice_warp_bytes<GradT>();
                 const CUtensorMap *mp = maps + 2 * t;
                 if (lane == 0 && t != mapped) { tensormap_acquire(mp); tensormap_acquire(mp + 1); mapped = t; }
@@ -1466,7 +1470,8 @@ factored_stats_vec_kernel(const FactoredLaunch L, const CUtensorMap *__restrict_
             [[maybe_unused]] double none = 0.0;
             if constexpr (RESIDUAL) {
                 const bool one = pre_div == 1.0f;
-                if (vec) ok = one ? slice_rows<GradT, SLICE_RESIDUAL, true, true>(L, sT, r0, row_end, c0, pre_div, false, ic, cacc, none, ring, s_full[warp], cons)
+                if (!ANY && !small) ok = slice_rows<GradT, SLICE_RESIDUAL, true, false, false>(L, sT, r0, row_end, c0, pre_div, false, ic, cacc, none, ring, s_full[warp], cons);
+                else if (vec) ok = one ? slice_rows<GradT, SLICE_RESIDUAL, true, true>(L, sT, r0, row_end, c0, pre_div, false, ic, cacc, none, ring, s_full[warp], cons)
                                   : slice_rows<GradT, SLICE_RESIDUAL, true, false>(L, sT, r0, row_end, c0, pre_div, false, ic, cacc, none, ring, s_full[warp], cons);
                 else if constexpr (ANY)
                     ok = one ? slice_rows<GradT, SLICE_RESIDUAL, false, true>(L, sT, r0, row_end, c0, pre_div, false, ic, cacc, none, ring, s_full[warp], cons)

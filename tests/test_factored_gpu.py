@@ -114,6 +114,11 @@ EXTRA_CASES.update({
     "adafactor_m_slices_f32_w": dict(shapes=_SLICES, steps=3, seed=68, grad=_F32, hp=dict(cases.CASES["adafactor_factored_m"]["hp"], beta1=0.4)),
     "adafactor_m_slices_8": dict(shapes=[(39, 264), (520, 776), (1030, 520)], steps=3, seed=69, grad=cases.CASES["adafactor_factored_m"]["grad"],
                                  hp=dict(cases.CASES["adafactor_factored_m"]["hp"], maximize=True)),
+    # tables of whole vectors without boxes: binary32 gradients, rows of which only some are multiples of 256
+    "came_slices_8_f32_w": dict(shapes=[(700, 256), (131, 520), (1030, 512)], steps=3, seed=72, grad=_F32,
+                                hp=dict(cases.CASES["came_al16"]["hp"], beta1=0.4)),
+    "came_slices_8_w": dict(shapes=[(700, 256), (131, 520), (39, 264)], steps=3, seed=73, grad=cases.CASES["came_al16"]["grad"],
+                            hp=dict(cases.CASES["came_al16"]["hp"], beta1=0.4)),
     # the write pass in flat order over whole vectors with that form of lerp; chunks that end a tensor; row ends in a third of the warps
     "came_flat_w": dict(shapes=[(200, 520), (70, 264), (9, 2056)], steps=3, seed=70, grad=cases.CASES["came_al16"]["grad"],
                         hp=dict(cases.CASES["came_al16"]["hp"], beta1=0.4)),
