@@ -1396,7 +1396,7 @@ factored_stats_vec_kernel(const FactoredLaunch L, const CUtensorMap *__restrict_
 {
     __shared__ double s_col[8][FSTAT_COLS];      // [warp][j * 32 + lane]
     __shared__ af8_factored_tensor sT;
-    extern __shared__ __align__(128) unsigned char sr_smem[];            // the warps' input rings (use_ring)
+    extern __shared__ __align__(128) unsigned char sr_smem[];            // the warps' input rings (IN)
     __shared__ __align__(8) uint64_t s_full[8][SLICE_STAGES];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int cur_t = -1;
@@ -2770,7 +2770,10 @@ static int af8_factored_stats_impl(const af8_factored_cfg *cfg, const af8_factor
     static const bool ring_off = getenv("AF8_NO_FACTORED_RING") != nullptr;
     static const bool box_off = getenv("AF8_NO_FACTORED_BOXES") != nullptr;
     const bool any = cfg->aligned8 == 2;
-    int ring = (ring_off || !(res || any)) ? 0 : 1;
+    // The warps' rings take 51 KB of shared memory a CTA (84 KB with binary32 gradients) from the L1 of the direct loads: only for
+    // tables that have rows to take through them (stacks of
+    // experts, 157 M parameters with binary32 gradients: g^2 pass 144 us with them reserved, 117 without).
+    int ring = (ring_off || !(res ? cfg->m_fmt == AF8_M_UF8 && cfg->m_block == 256 : any && !cfg->cols_mult8)) ? 0 : 1;
     // residual pass over bf16 gradients and UF8 codes of tensors with cols % 256 == 0: boxes of rows through
     // tensor maps, when the caller has given room for the maps
     const CUtensorMap *maps = nullptr;
