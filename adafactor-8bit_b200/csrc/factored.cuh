@@ -2882,7 +2882,17 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
     const int64_t total_tiles = cfg->total_tiles;
     const bool any = cfg->aligned8 == 2;         // batches of matrices, rows of any length >= 8
     const bool only_g = (cfg->came && cfg->mode == AF8_FUPD_SUMSQ_U) || no_m;
-    const bool mom = !cfg->came && cfg->m_fmt == AF8_M_UF8 && cfg->m_block == 256 && !ring_off;
+    // With a UF8 momentum (not CAME's): in slices over the tiles where the table is large and fills its tiles, else in flat order.
+    // Size: the sums that the tiles add to are cleared first, a launch of 2 us (3 of host time).  Slices and flat, bf16 and binary32
+    // gradients: whole vectors 1 M parameters 12.7, 8.6 us; 16.8 M 27.0, 27.0 and 30.4, 29.1; 77 M 81, 107 and 108, 111; 352 M 263,
+    // 404 and 334, 464; ragged rows or batches, whose flat kernel is the slower one, 1 M 14.1, 10.7; 9.4 M 24.1, 25.0 and 26.6,
+    // 27.0; 132 M 184, 271 and 205, 282.
+    // Filling: a warp takes up to 256 columns of a row at a time, and the CTA that gets one tile more decides.  Rows of 16 elements,
+    // 16 M parameters, 189, 29; 30 M bf16 in rows of 192 52, 46, of 224 42, 46, of 117 90, 78, of 165 74, 76, of 205 56, 76; in
+    // matrices of 560 x 560 84, 48.
+    const int64_t slice_from = any ? 4096 : bf ? 8192 : 32768;                                           // chunks of 2048 elements
+    const bool filled = total_chunks * 2048 * 10 >= total_tiles * (FSTAT_ROWS * FSTAT_COLS) * (any ? 5 : 8);
+    const bool mom = !cfg->came && cfg->m_fmt == AF8_M_UF8 && cfg->m_block == 256 && !ring_off && filled && total_chunks >= slice_from;
     if (vec && !apply && !tile_off && total_tiles > 0 && cfg->grad_dtype != AF8_F16 && (only_g || mom)) {
         // over the statistic tiles, column factors in registers; with a momentum, or rows of any length, in slices
         AF8_CUDA_TRY(cudaMemsetAsync(block_sumsq, 0, sizeof(double) * (size_t)total_chunks, cst));

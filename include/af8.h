@@ -367,9 +367,9 @@ typedef struct af8_factored_cfg {
     int32_t stochastic_round; /* as af8_fullrank_cfg.stochastic_round */
     int64_t total_tiles;    /* optional: the table's number of statistic tiles (the last tensor's first_tile plus its
                                own tiles).  With it the sum-of-squares passes that only read the gradient
-                               (AF8_FUPD_SUMSQ_U, AF8_FUPD_SUMSQ without momentum) or the gradient and a UF8 momentum
-                               in blocks of 256 (not CAME's AF8_FUPD_SUMSQ) run over the tiles, with the column factors
-                               in registers; 0: over the flat chunks */
+                               (AF8_FUPD_SUMSQ_U, AF8_FUPD_SUMSQ without momentum) run over the tiles, with the column
+                               factors in registers, and those of large tables of filled tiles that also read a UF8
+                               momentum in blocks of 256 (not CAME's AF8_FUPD_SUMSQ); 0: over the flat chunks */
     int32_t cols_mult256;   /* 1: every tensor of the table has cols % 256 == 0 (with total_tiles: the write pass with a
                                UF8 momentum then also runs over the tiles, a row slice being one momentum block) */
     int32_t cols_mult8;     /* with aligned8 = 2: 1 if every tensor of the table has cols % 8 == 0 (batches of matrices

@@ -104,7 +104,8 @@ EXTRA_CASES["adafactor_long_blocks"] = dict(shapes=[(5000, 16), (40, 9001)], ste
                                             hp=dict(cases.CASES["adafactor_factored"]["hp"], block_size=8192, v_quant_type="al8"))
 
 # row slices through the warps' rings: binary32 gradients, momentum weights of 1/2 and more (the other form of lerp), a last unit
-# of 16 bytes that belongs to one or to two slices of the last row, tiles that end within a group of four rows
+# of 16 bytes that belongs to one or to two slices of the last row, tiles that end within a group of four rows (with a momentum
+# the sums take slices in large tables only, see below)
 _SLICES = [(700, 257), (131, 273), (39, 264), (1030, 513), (67, 1001)]
 EXTRA_CASES.update({
     "came_slices_f32": dict(shapes=_SLICES, steps=3, seed=65, grad=_F32, hp=cases.CASES["came_al16"]["hp"]),
@@ -210,6 +211,46 @@ def test_a_matrix_beside_batches_is_the_same(oracle):
         out.append([(p.detach().cpu(), float(opt.state[p]["fira_prev_norm"])) for p in params[:len(flats)]])
     apart = [(s, na, nb) for s, (a, na), (b, nb) in zip(flats, *out) if na != nb or not torch.equal(a, b)]
     assert not apart, f"{len(apart)} of {len(flats)} matrices differ: {apart[:3]}"
+
+
+_ROWS8, _RAGGED = [(39, 264), (520, 776), (1030, 520)], [(700, 257), (131, 273), (39, 264), (1030, 513), (67, 1001)]
+
+
+@pytest.mark.parametrize("grad,beta1,shapes,sliced", [
+    (torch.bfloat16, 0.9, _ROWS8 + [(2552, 8184)], True), (torch.bfloat16, 0.4, _ROWS8 + [(2552, 8184)], True),
+    (torch.float32, 0.9, _ROWS8 + [(4104, 16392)], True), (torch.float32, 0.4, _ROWS8 + [(4104, 16392)], True),
+    (torch.bfloat16, 0.9, _RAGGED + [(4099, 2067)], True), (torch.bfloat16, 0.4, _RAGGED + [(4099, 2067)], True),
+    (torch.float32, 0.9, _RAGGED + [(4099, 2067)], True), (torch.float32, 0.4, _RAGGED + [(4099, 2067)], True),
+    (torch.bfloat16, 0.9, [(3, 70, 40), (2, 33, 131), (2, 2040, 2100)], True), (torch.float32, 0.9, [(2, 600, 72), (2, 2040, 2104)], True),
+    (torch.bfloat16, 0.9, [(73000, 117)], False), (torch.bfloat16, 0.9, [(132000, 128)], False), (torch.bfloat16, 0.9, [(2040, 8200)], False),
+    (torch.float32, 0.9, [(4088, 16392)], False), (torch.float32, 0.9, [(4000, 2067)], False)])
+def test_sums_with_a_momentum_are_the_same_in_slices_and_flat(grad, beta1, shapes, sliced):
+    """Sums of squares of Adafactor with a UF8 momentum: tables from 2^24 elements on (2^26 with binary32 gradients; 2^23 for rows
+    that are not whole vectors and batches) that fill their tiles take them in row slices, the others in flat order.  The binary32 sums of eight
+    squares are the same in both, so only the order of binary64 additions differs: 2^-53 of the sum for each of the 2^17 that
+    pass through one accumulator at most, 1.5e-11."""
+    from adafactor8bit import Adafactor8Bit, _engine
+    hp = dict(cases.CASES["adafactor_factored_m"]["hp"], beta1=beta1, m_quant_type="uf8", m_block_size=256, min_8bit_size=1)
+    totals = []
+    for flat in (False, True):
+        gen = torch.Generator(device="cuda").manual_seed(33)
+        params = [torch.nn.Parameter(torch.randn(s, generator=gen, device="cuda") * 0.02) for s in shapes]
+        opt = Adafactor8Bit(params, **hp)
+        for t in (1, 2):
+            for p in params:
+                p.grad_dtype = None
+                p.grad = (torch.randn(p.shape, generator=gen, device="cuda") * 1e-3).to(grad)
+            if t == 2:
+                plan, = [x for x in opt._plans.values() if isinstance(x, _engine.FactoredPlan)]
+                assert plan.cfg.total_tiles > 0
+                if flat:
+                    plan.cfg.total_tiles = 0
+            opt.step()
+        sums = [plan.d_sumsq[int(f):int(f) + int(n)] for f, n in zip(plan.first_chunk, plan.nchunks)]
+        assert bool((sums[-1][1:] == 0.0).all()) == (sliced and not flat)
+        totals.append([float(x.sum()) for x in sums])
+    for shape, a, b in zip(shapes, *totals):
+        assert b > 0.0 and abs(a - b) <= 1.5e-11 * b, (shape, a, b)
 
 
 @pytest.mark.parametrize("came", [False, True])
