@@ -85,7 +85,7 @@ __device__ __forceinline__ uint32_t m_encode(float m, float a, int fmt)
 // on the momentum-only path (reads dyn.pre_div like APPLY, writes nothing but
 // the partial sums).
 // THREADS: 256, or 1024 where there are at most two blocks per SM (the norm vectors and biases of a model, tensors of a few
-// thousand elements): each of the few CTAs walked its block in eight dependent rounds of loads.  45 vectors of 2048 elements
+// thousand elements; quantised states in blocks of at least 1024, see the launch): each of the few CTAs walked its block in eight dependent rounds of loads.  45 vectors of 2048 elements
 // with binary32 states: 23 -> 9 us in one pass, 19 + 16 -> 9 + 8 us in two; 9 vectors of 4096 elements with UF8 / AL16 states
 // 22 + 32 -> 10 + 14 us in two (the short exponentials and logarithms with their tables in shared memory included).
 template <typename GradT, int MODE, int THREADS>
