@@ -2837,8 +2837,10 @@ extern "C" int af8_factored_small(const af8_factored_cfg *cfg, const af8_factore
     if (!dev_tensors || n_tensors <= 0 || total_units <= 0) return fail(AF8_ERR_INVALID, "af8_factored_small: null or empty table");
     if (conf && !cfg->came) return fail(AF8_ERR_INVALID, "af8_factored_small: confidence states exist only with CAME");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // at most one unit per SM (blocks of 2048, few tensors): the launch lasts as long as one CTA, so more threads
-    // (8 layers of 512 x 1376 with CAME: 12.3 us a launch with 256, 11.5 with 1024; 480 units of 256 elements: 6.2 us with 256, 14 with 512)
+    // At most one unit per SM (long blocks, few tensors): the launch lasts as long as one CTA, so more threads.  Device time of the
+    // launch and factored_inv_kernel with 256, 512 and 1024 threads, few units: blocks of 256 13.3, 13.3, 14.1 us; of 512 14.0, 13.3,
+    // 14.6; of 1024 15.4, 14.6, 14.4; of 2048 18.4, 15.4, 15.4 (CAME's confidence states 25.0, 20.9, 19.9); of 4096 21.5, 17.4, 17.2.
+    // Many units: 480 of 256 elements 6.2 us with 256 threads, 14 with 512.
     if (total_units <= sm_count()) factored_small_kernel<SMALL_MAX_THREADS><<<total_units, SMALL_MAX_THREADS, 0, st>>>(dev_tensors, n_tensors, conf, cfg->v_floor);
     else factored_small_kernel<256><<<total_units, 256, 0, st>>>(dev_tensors, n_tensors, conf, cfg->v_floor);
     AF8_CUDA_TRY(cudaGetLastError());
