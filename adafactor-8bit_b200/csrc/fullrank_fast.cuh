@@ -203,8 +203,8 @@ __device__ __forceinline__ float lg2_approx(float x)
     return y;
 }
 
-// |lg2.approx(x) - log2(x)| <= 1.22e-7 |log2(x)| + 1.7e-7 for every normal x (all of them measured on a B200: 2.74e-7 for
-// |log2| in [1, 2), 7.78e-6 in [64, 128))
+// |lg2.approx(x) - log2(x)| <= 1.22e-7 |log2(x)| + 1.7e-7 for every normal x (all of them measured on a B200, and by
+// tests/test_lg2_approx_gpu.py: 2.74e-7 for |log2| in [1, 2), 7.78e-6 in [64, 128))
 constexpr float LG2_REL = 1.22e-7f, LG2_ABS = 1.7e-7f;
 
 #define AF8_MAGIC_F 12582912.0f       /* 1.5 * 2^23: adding it rounds to an integer (half to even) */
@@ -845,23 +845,7 @@ fullrank_fast_kernel(const FullrankLaunch L)
         const bool next_staged = want >= 2;           // the next block gets its table and ranges prepared here
 
         // ---- issue the bulk copies (one thread; STASH: the first ones of a tensor, the others when a slot is left) ----
-        if (tid == 0 && ahead < want && (!STASH || ahead == 0)) {
-            const unsigned char *gp = static_cast<const unsigned char *>(sT.grad);
-            const unsigned char *pp = static_cast<const unsigned char *>(sT.param);
-            const unsigned char *vp = static_cast<const unsigned char *>(sT.v_q);
-            fence_proxy_async();
-            for (int k = ahead; k < want; ++k) {
-                const int64_t nb = (int64_t)(b + k * G) * FAST_VBLOCK;
-                const int sl = (n + k) % NST;
-                unsigned char *dst = s_ring + sl * STAGE_BYTES;
-                mbar_expect_tx(&s_full[sl], STAGE_BYTES);
-                bulk_g2s(dst + P_OFF, pp + nb * PB, FAST_VBLOCK * PB, &s_full[sl]);
-                bulk_g2s(dst + G_OFF, gp + nb * GB, FAST_VBLOCK * GB, &s_full[sl]);
-                bulk_g2s(dst + VQ_OFF, vp + nb * (VB / 8), Ring::VQ_BYTES, &s_full[sl]);
-                if (MF != AF8_M_NONE)
-                    bulk_g2s(dst + MQ_OFF, sT.m_q + (MF == AF8_M_UF4 ? nb / 2 : nb), Ring::MQ_BYTES, &s_full[sl]);
-            }
-        }
+        if (tid == 0 && ahead < want && (!STASH || ahead == 0)) fast_issue<Ring, MF>(sT, s_ring, s_full, b, G, n, ahead, want);
         const int in_flight = want;                   // copies outstanding now, this block included
         ahead = want > 0 ? want - 1 : 0;              // ... as seen from the next block
         // ---- ranges of this block (if not prefetched) and of the next one ----
@@ -1151,14 +1135,14 @@ fullrank_fast_kernel(const FullrankLaunch L)
                 else static_cast<uint16_t *>(sT.v_q)[base + o + k] = (uint16_t)c;
             }
             __syncthreads();             // the slot may be refilled from the next iteration on
-        } else if (VB == 8) {
+        } else if constexpr (VB == 8) {
             uint8_t *const vp = static_cast<uint8_t *>(sT.v_q) + base;
             const float2 k2 = bc2(r.k), c2 = bc2(r.c), mg2 = bc2(AF8_MAGIC_F + 1.0f), nmg2 = bc2(-(AF8_MAGIC_F + 1.0f));
 #pragma unroll
             for (int mb = 0; mb < 2; ++mb) {
                 float x[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) x[j] = v[STASH ? j : 8 * mb + j];
+                for (int j = 0; j < 8; ++j) x[j] = v[8 * mb + j];
                 uint32_t kk[8];
                 float dd[8];
                 float dmax = 0.0f;
