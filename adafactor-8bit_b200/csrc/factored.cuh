@@ -849,8 +849,9 @@ __device__ __forceinline__ void load_cols8_shifted(const float *v, int64_t i, fl
     for (int j = 0; j < 8; ++j) x[j] = (s & 1) ? w[j + 1] : w[j];
 }
 
-// stats_rows for rows of any length: elements beyond the row's end count as zeros, all loads through GradAny8
-template <typename GradT, int NB, bool RESIDUAL>
+// The residual pass of stats_rows for rows of any length with a momentum that has no slices (not UF8 in blocks of 256, weights of
+// 1/2 and more): elements beyond the row's end count as zeros, all loads through GradAny8.
+template <typename GradT, int NB>
 __device__ __forceinline__ void stats_rows_any(const FactoredLaunch &L, const af8_factored_tensor &sT, int64_t r0, int64_t r_end, int64_t c,
                                                float pre_div, const float (&ic)[8], double (&cacc)[8])
 {
@@ -870,10 +871,7 @@ __device__ __forceinline__ void stats_rows_any(const FactoredLaunch &L, const af
             const int64_t r = r0 + warp + 8 * (k0 + k);
             float g[8], x[8];
             cur[k].unpack(L.negate_grad, g);
-            if (!RESIDUAL) {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) x[j] = __fmul_rn(g[j], g[j]);
-            } else if (nc > 0 && r < r_end) {
+            if (nc > 0 && r < r_end) {
                 const float ir = sT.inv_row[r];
                 const DivBy D = make_div(pre_div);
                 const LerpW LW = make_lerp(sT.m_w);
@@ -1259,13 +1257,13 @@ template <bool VEC>
 __device__ __forceinline__ void slice_cols(const float *inv_col, int64_t c0, int64_t C, float (&ic)[8])
 {
     const int lane = threadIdx.x & 31;
-    if (VEC) {
+    if constexpr (VEC) {
         if (c0 + lane * 8 < C) load_f8_ro(inv_col + c0 + lane * 8, ic);
-        return;
-    }
+    } else {
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-        if (c0 + lane + 32 * j < C) ic[j] = __ldg(inv_col + c0 + lane + 32 * j);
+        for (int j = 0; j < 8; ++j)
+            if (c0 + lane + 32 * j < C) ic[j] = __ldg(inv_col + c0 + lane + 32 * j);
+    }
 }
 
 // The same pass with the input of FBOX_ROWS consecutive rows per copy: one tiled bulk tensor copy brings their
@@ -1481,7 +1479,7 @@ factored_stats_vec_kernel(const FactoredLaunch L, const CUtensorMap *__restrict_
             }
             }
         } else if (!vec) {
-            if constexpr (ANY) stats_rows_any<GradT, 4, RESIDUAL>(L, sT, r0, row_end, c, pre_div, ic, cacc);
+            if constexpr (ANY && RESIDUAL) stats_rows_any<GradT, 4>(L, sT, r0, row_end, c, pre_div, ic, cacc);
         } else if (!RESIDUAL) stats_rows<GradT, 4, true, false>(L, sT, r0, row_end, c, col_ok, pre_div, ic, cacc);
         else stats_rows<GradT, AF8_FSTAT_RES_NB, AF8_FSTAT_RES_PREFETCH, true>(L, sT, r0, row_end, c, col_ok, pre_div, ic, cacc);
         if (!ok) {
@@ -2492,7 +2490,7 @@ factored_sumsq_slice_kernel(const FactoredLaunch L, const int whole)
 // its 8 columns in registers while its warp walks the tile's rows (the flat kernel above re-reads them for
 // every element, twice the bytes of the gradient itself through L1), four rows' loads in flight.  A CTA adds
 // its tile's sum to the slot of the tensor's first chunk; the caller clears the slots first.
-// ANY = 1: batches of matrices, whole vectors; 2: rows of any length as well (see sums_by_eight).
+// ANY = 1: batches of matrices (see sums_by_eight).  Whole vectors; rows of any length go through factored_sumsq_slice_kernel.
 template <typename GradT, int ANY>
 __global__ void __launch_bounds__(256, ANY ? 3 : 4)
 factored_sumsq_tile_kernel(const FactoredLaunch L)
@@ -2524,32 +2522,6 @@ factored_sumsq_tile_kernel(const FactoredLaunch L)
 #pragma unroll
         for (int j = 0; j < 8; ++j) ic[j] = 0.0f;
         double acc = 0.0;
-        if (ANY == 2 && (C & 7) != 0) {
-            const int nc = (int)max((int64_t)0, min((int64_t)8, C - c));
-            const int64_t numel = sT.rows * C;
-            load_cols_any(sT.inv_col + P.cb, c, C, ic);
-            for (int k0 = 0; r0 + warp + 8 * k0 < R; k0 += NB) {   // (uniform over the warp)
-                GradAny8<GradT> any[NB];
-#pragma unroll
-                for (int k = 0; k < NB; ++k) {
-                    const int64_t r = r0 + warp + 8 * (k0 + k);
-                    if (nc > 0 && r < R) any[k].load(sT.grad, r * C + c, numel);
-                    else any[k].zero();
-                }
-#pragma unroll
-                for (int k = 0; k < NB; ++k) {
-                    const int64_t r = min(r0 + warp + 8 * (int64_t)(k0 + k), R - 1);     // (a row beyond the end carries zeros)
-                    const float ir = __ldg(sT.inv_row + r);
-                    float g[8];
-                    any[k].unpack(0, g);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const float uj = __fmul_rn(__fmul_rn(g[j], ir), ic[j]);
-                        if (j < nc) acc += (double)__fmul_rn(uj, uj);
-                    }
-                }
-            }
-        } else {
         if (col_ok) load_f8_ro(sT.inv_col + P.cb + c, ic);
         const auto sum_rows = [&](auto by_eight) {                 // (a copy of the loop for each: the choice inside cost a third)
             GradRaw8<GradT> cur[NB], nxt[NB];
@@ -2584,7 +2556,6 @@ factored_sumsq_tile_kernel(const FactoredLaunch L)
         };
         if (sums_by_eight<ANY>(sT)) sum_rows(std::true_type());
         else if constexpr (ANY != 0) sum_rows(std::false_type());
-        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
         if (lane == 0) s_acc2[warp] = acc;
@@ -2767,13 +2738,12 @@ static int af8_factored_stats_impl(const af8_factored_cfg *cfg, const af8_factor
     L.total_units = tiles << L.split;
     int64_t grid = (int64_t)sm_count() * 6;
     if (grid > L.total_units) grid = L.total_units;
-    static const bool ring_off = getenv("AF8_NO_FACTORED_RING") != nullptr;
     static const bool box_off = getenv("AF8_NO_FACTORED_BOXES") != nullptr;
     const bool any = cfg->aligned8 == 2;
     // The warps' rings take 51 KB of shared memory a CTA (84 KB with binary32 gradients) from the L1 of the direct loads: only for
     // tables that have rows to take through them (stacks of
     // experts, 157 M parameters with binary32 gradients: g^2 pass 144 us with them reserved, 117 without).
-    int ring = (ring_off || !(res ? cfg->m_fmt == AF8_M_UF8 && cfg->m_block == 256 : any && !cfg->cols_mult8)) ? 0 : 1;
+    int ring = (res ? cfg->m_fmt == AF8_M_UF8 && cfg->m_block == 256 : any && !cfg->cols_mult8) ? 1 : 0;
     // residual pass over bf16 gradients and UF8 codes of tensors with cols % 256 == 0: boxes of rows through
     // tensor maps, when the caller has given room for the maps
     const CUtensorMap *maps = nullptr;
@@ -2878,7 +2848,6 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
     cudaStream_t cst = static_cast<cudaStream_t>(stream);
     const bool bf = cfg->grad_dtype == AF8_BF16;
     const bool no_m = cfg->m_fmt == AF8_M_NONE;
-    static const bool ring_off = getenv("AF8_NO_FACTORED_RING") != nullptr;
     static const bool wide_off = getenv("AF8_NO_WIDE_SUMS") != nullptr;
     static const bool tile_off = getenv("AF8_NO_TILE_SUMS") != nullptr;
     const int64_t total_tiles = cfg->total_tiles;
@@ -2894,7 +2863,7 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
     // matrices of 560 x 560 84, 48.
     const int64_t slice_from = any ? 4096 : bf ? 8192 : 32768;                                           // chunks of 2048 elements
     const bool filled = total_chunks * 2048 * 10 >= total_tiles * (FSTAT_ROWS * FSTAT_COLS) * (any ? 5 : 8);
-    const bool mom = !cfg->came && cfg->m_fmt == AF8_M_UF8 && cfg->m_block == 256 && !ring_off && filled && total_chunks >= slice_from;
+    const bool mom = !cfg->came && cfg->m_fmt == AF8_M_UF8 && cfg->m_block == 256 && filled && total_chunks >= slice_from;
     if (vec && !apply && !tile_off && total_tiles > 0 && cfg->grad_dtype != AF8_F16 && (only_g || mom)) {
         // over the statistic tiles, column factors in registers; with a momentum, or rows of any length, in slices
         AF8_CUDA_TRY(cudaMemsetAsync(block_sumsq, 0, sizeof(double) * (size_t)total_chunks, cst));
@@ -2902,7 +2871,7 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
         LT.split = tile_split(total_tiles);
         LT.total_units = total_tiles << LT.split;
         const int kind = !any ? 0 : cfg->cols_mult8 ? 1 : 2;
-        if (!ring_off && (mom || kind == 2)) {
+        if (mom || kind == 2) {
             const int64_t sg = std::min<int64_t>((int64_t)sm_count() * (bf ? 3 : 2), LT.total_units);
 #define AF8_LAUNCH_FSLICE(G, M) do { \
             AF8_CUDA_TRY(cudaFuncSetAttribute(factored_sumsq_slice_kernel<G, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)slice_smem_bytes<G>())); \
@@ -2915,8 +2884,7 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
         }
         const int64_t tg = std::min<int64_t>((int64_t)sm_count() * 8, LT.total_units);
 #define AF8_LAUNCH_FSUM(G) do { if (kind == 0) factored_sumsq_tile_kernel<G, 0><<<(int)tg, 256, 0, cst>>>(LT); \
-        else if (kind == 1) factored_sumsq_tile_kernel<G, 1><<<(int)tg, 256, 0, cst>>>(LT); \
-        else factored_sumsq_tile_kernel<G, 2><<<(int)tg, 256, 0, cst>>>(LT); } while (0)
+        else factored_sumsq_tile_kernel<G, 1><<<(int)tg, 256, 0, cst>>>(LT); } while (0)
         if (bf) AF8_LAUNCH_FSUM(bf16_tag);
         else AF8_LAUNCH_FSUM(float);
 #undef AF8_LAUNCH_FSUM
@@ -2931,7 +2899,7 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
         return AF8_OK;
     }
     static const bool tile_apply_off = getenv("AF8_NO_TILE_APPLY") != nullptr;
-    if (vec && cfg->mode == AF8_FUPD_APPLY && cfg->m_fmt == AF8_M_UF8 && cfg->param_dtype == AF8_F32 && !ring_off && !tile_apply_off &&
+    if (vec && cfg->mode == AF8_FUPD_APPLY && cfg->m_fmt == AF8_M_UF8 && cfg->param_dtype == AF8_F32 && !tile_apply_off &&
         cfg->total_tiles > 0 && cfg->cols_mult256) {
         // every row slice of 256 columns is one momentum block: tile order, column factors in registers
         FactoredLaunch LT = L;
@@ -2951,7 +2919,7 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
     }
     // (see PT: bf16 gradients with bf16 parameters have kernels of their own)
     const int pt = cfg->param_dtype == AF8_F32 ? 0 : (bf && cfg->param_dtype == AF8_BF16 && !lag) ? (cfg->stochastic_round ? 2 : 1) : 3;
-    if (vec && cfg->mode == AF8_FUPD_APPLY && cfg->m_fmt == AF8_M_UF8 && pt != 3 && !ring_off) {
+    if (vec && cfg->mode == AF8_FUPD_APPLY && cfg->m_fmt == AF8_M_UF8 && pt != 3) {
         // UF8 momentum: inputs through per-warp rings of bulk copies
         grid = std::min<int64_t>((int64_t)sm_count() * (bf ? (any ? FLAT_ANY_CTAS : 3) : 2), total_chunks);
 #define AF8_LAUNCH_FLAT(G, T, A) do { \
