@@ -1151,14 +1151,9 @@ class ApolloPlan:
                 continue
             plan = self._low_plan(idx)
             plan.cfg.v_floor = -126.0 if first else float(floor_later)
-            k = len(idx)
-            cols = dict(decay=np.zeros(k, np.float32), alpha=np.full(k, -1.0, np.float32),
-                        v_w=np.full(k, lowrank_scalars["v_w"], np.float32),
-                        v_keep=np.full(k, -1.0 if self.v_fmt == "fp32" else lowrank_scalars["v_keep"], np.float32),   # fp32 V: lerp_
-                        v_eps_add=np.zeros(k, np.float32),
-                        m_w=np.full(k, lowrank_scalars["m_w"], np.float32), eps_gradsq=np.zeros(k, np.float32),
-                        eps_denom=np.full(k, lowrank_scalars["apollo_eps"], np.float32),
-                        eps_sq=np.full(k, 1.17549435e-38, np.float32))
+            low = lowrank_scalars                   # (one value for the table each)
+            cols = dict(decay=0.0, alpha=-1.0, v_w=low["v_w"], v_keep=-1.0 if self.v_fmt == "fp32" else low["v_keep"],     # fp32 V: lerp_
+                        v_eps_add=0.0, m_w=low["m_w"], eps_gradsq=0.0, eps_denom=low["apollo_eps"], eps_sq=np.float32(1.17549435e-38))
             plan.run([self.g_low[i] for i in idx], cols, d=0.0, fira=False)
         if log is not None:
             ev[2].record(stream)

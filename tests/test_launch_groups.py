@@ -34,3 +34,15 @@ def test_kernel_names_follow_the_dispatch(v, m, param, grad, mode, name):
     plan.cfg = N.FullrankCfg(block=2048, m_block=256 if m else 0, v_fmt=N.V_FMT[v], m_fmt=N.M_FMT[m], use_adam_denom=1,
                              param_dtype=getattr(N, param.upper()), grad_dtype=getattr(N, grad.upper()))
     assert plan.kernel_name(getattr(N, "MODE_" + mode.upper())) == name
+
+
+def test_scalars_of_a_launch_template_follow_every_step():
+    """One value for the table, one per tensor, and the change from either to the other; unchanged values stay."""
+    import numpy as np
+    from adafactor8bit import _engine as E
+    static, last = np.zeros((2, 3), dtype=[("alpha", np.float32), ("decay", np.float32)]), {}
+    array = np.array([1.0, 2.0, 3.0], dtype=np.float32)
+    for alpha, decay in [(0.5, array), (0.5, 0.25), (array, 0.25), (0.5, 0.25), (np.float32(0.1), float("nan")), (np.float32(0.1), 0.0), (0.0, array * 2)]:
+        E._update_scalars(static, last, dict(alpha=alpha, decay=decay), ("alpha", "decay"))
+        for k, v in (("alpha", alpha), ("decay", decay)):
+            np.testing.assert_array_equal(static[k], np.broadcast_to(np.float32(v), (2, 3)), err_msg=k)
