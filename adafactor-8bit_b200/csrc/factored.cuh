@@ -1431,7 +1431,8 @@ factored_stats_vec_kernel(const FactoredLaunch L, const CUtensorMap *__restrict_
 #pragma unroll
         for (int j = 0; j < 8; ++j) ic[j] = 0.0f;
         // Whole rows of vectors or not; which of the row loops.  Rows of any length take the slices in both passes, whole vectors
-        // in the residual pass (339 M parameters in rows of 2000: direct loads 875 us, slices 472; of 1999: 1189 and 579); the g*g pass over whole vectors was slower through a ring (3.0 -> 4.3 ms on Llama-2-7B) and loads directly.
+        // in the residual pass (339 M parameters in rows of 2000: direct loads 875 us, slices 472; of 1999: 1189 and 579); the g*g
+        // pass over whole vectors was slower through a ring (3.0 -> 4.3 ms on Llama-2-7B) and loads directly.
         const bool vec = !ANY || (C & 7) == 0;
         // A momentum weight of 1/2 or more takes the other form of lerp.  (Direct loads and slices: 202 M parameters with binary32
         // gradients in rows of 256 n 528 and 277 us, 235 M bf16 ones in rows of which some are such 638 and 341.)
@@ -2741,8 +2742,8 @@ static int af8_factored_stats_impl(const af8_factored_cfg *cfg, const af8_factor
     static const bool box_off = getenv("AF8_NO_FACTORED_BOXES") != nullptr;
     const bool any = cfg->aligned8 == 2;
     // The warps' rings take 51 KB of shared memory a CTA (84 KB with binary32 gradients) from the L1 of the direct loads: only for
-    // tables that have rows to take through them (stacks of
-    // experts, 157 M parameters with binary32 gradients: g^2 pass 144 us with them reserved, 117 without).
+    // tables that have rows to take through them (g^2 pass over stacks of experts, 157 M parameters with binary32 gradients: 144 us
+    // with the rings reserved, 117 without).
     int ring = (res ? cfg->m_fmt == AF8_M_UF8 && cfg->m_block == 256 : any && !cfg->cols_mult8) ? 1 : 0;
     // residual pass over bf16 gradients and UF8 codes of tensors with cols % 256 == 0: boxes of rows through
     // tensor maps, when the caller has given room for the maps
