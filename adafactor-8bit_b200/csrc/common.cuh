@@ -65,7 +65,7 @@ inline int sm_count()
 }
 
 // Lets a kernel be launched with this much dynamic shared memory.  48 KB without the opt-in hold the kernel's static shared memory
-// too; no kernel here has 16 KB of that.
+// too; none of those that are launched through this has 16 KB of that.
 template <typename K>
 inline int allow_dynamic_smem(K kernel, size_t bytes)
 {
