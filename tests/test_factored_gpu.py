@@ -127,6 +127,16 @@ EXTRA_CASES.update({
                           hp=cases.CASES["came_al16"]["hp"]),
 })
 
+# the write pass without a momentum in units of 2048 elements: tensors that end a unit, just after it or far inside, units with no, one or
+# many row ends, the shortest rows, rows longer than a unit, more tensors than a CTA has stages, matrices of a batch that end in a unit
+_WRITE = [(1, 8), (2, 1024), (1, 2056), (257, 8), (3, 2048), (5, 4104), (100, 24), (1000, 40), (1, 8), (300, 2040), (2, 8)]
+EXTRA_CASES.update({
+    "adafactor_write": dict(shapes=_WRITE, steps=2, seed=81, grad=cases.CASES["adafactor_factored"]["grad"], hp=cases.CASES["adafactor_factored"]["hp"]),
+    "adafactor_write_f32": dict(shapes=_WRITE, steps=2, seed=82, grad=_F32, hp=dict(cases.CASES["adafactor_factored"]["hp"], maximize=True)),
+    "adafactor_write_3d": dict(shapes=[(5, 9, 8), (2, 300, 2056), (7, 33, 64), (3, 1, 2048)], steps=2, seed=83,
+                               grad=cases.CASES["adafactor_factored"]["grad"], hp=cases.CASES["adafactor_factored"]["hp"]),
+})
+
 # lag_norm=True (one pass with the previous step's norm; optimizer.py:1056-1071): the vector kernels, the
 # element-wise kernels (odd column counts) and the limiter on top of the clip
 EXTRA_CASES.update({
