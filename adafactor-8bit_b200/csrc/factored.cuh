@@ -28,8 +28,8 @@
 #include "fullrank_fast.cuh"
 #include "fullrank_generic.cuh"
 #include "fullrank_stat.cuh"
-#include "schedule.cuh"
 #include "tensormap.cuh"
+#include "write_units.cuh"
 
 namespace af8 {
 
@@ -1880,104 +1880,47 @@ factored_update_vec_kernel(const FactoredLaunch L)
 // fp32 or bf16 parameters (PT as above).
 //
 // It moves 10 bytes per parameter (bf16 gradients, fp32 parameters) and computes next to nothing, so the order of its memory
-// accesses decides.  A unit is 2048 consecutive elements.  A CTA takes its units by cluster launch control (schedule.cuh); its fifth
-// warp brings their gradients and parameters in through a ring of WRITE_STAGES stages (two bulk copies a unit, across tensors)
-// and hands the tensor's scalars on with them, the other four write back from registers: a thread owns four groups of four elements,
-// 512 apart, so that every access of a warp is one contiguous run.  Six CTAs per SM, 216 KB requested; two stages, or seven and
-// eight CTAs with fewer registers, are within 3 %.  With the requests made by one of the four warps, whose answers and descriptor it
-// then waits for, the pass was slower than before.
-// Against contiguous runs of units per CTA, loads into registers one unit ahead and requests to L2 three ahead: 134 M parameters
-// in one matrix 218 -> 204 us (6.6 TB/s; a copy of the same streams reaches 6.85), 176 M in 28 matrices of 2048 columns 295 -> 276.
+// accesses decides: write_units.cuh.  Six CTAs per SM, 216 KB requested; two stages, or seven and eight CTAs with fewer registers, are
+// within 3 %.  Against contiguous runs of units per CTA, loads into registers one unit ahead and requests to L2 three ahead: 134 M
+// parameters in one matrix 218 -> 204 us (6.6 TB/s; a copy of the same streams reaches 6.85), 176 M in 28 matrices of 2048 columns
+// 295 -> 276.
 // ---------------------------------------------------------------------------
-constexpr int WRITE_UNIT = 2048, WRITE_THREADS = 128, WRITE_STAGES = 3;      // (and a fifth warp, which requests)
-constexpr int DEVERR_WRITE_TIMEOUT = 6;
-template <typename GradT, int PT> __host__ __device__ constexpr int write_stage_bytes() { return WRITE_UNIT * (sizeof_grad<GradT>() + (PT == 0 ? 4 : 2)); }
-template <typename GradT, int PT> constexpr size_t write_smem_bytes() { return (size_t)WRITE_STAGES * write_stage_bytes<GradT, PT>(); }
-struct __align__(16) WriteUnit {     // a unit, and what its tensor's elements need
-    int64_t base, row;               // flat index and row of its first element
-    int64_t col, cols;               // the first element's column; columns
-    int64_t batch_rows;
-    int count;                       // elements; 0: no unit is left
-    uint32_t magic;                  // floor(2^32 / cols) + 1: quotients by the column count
-    void *param, *copy;
+struct FactoredUnit : WriteUnit {
+    void *copy;
     const float *inv_row, *inv_col;
+    int64_t batch_rows;
     uint64_t sr_base;
     float decay, step, fira, zero;
+};
+struct FactoredUnits {
+    const FactoredLaunch &L;
+    __device__ __forceinline__ int count() const { return L.n_tensors; }
+    __device__ __forceinline__ int64_t first(int t) const { return __ldg(&L.tensors[t].first_chunk); }
+    __device__ __forceinline__ int64_t load(int t, FactoredUnit &U) const
+    {
+        const af8_factored_tensor T = L.tensors[t];
+        U.cols = T.cols; U.param = T.param; U.grad = T.grad; U.copy = T.param_copy; U.inv_row = T.inv_row; U.inv_col = T.inv_col;
+        U.batch_rows = T.batch_rows; U.sr_base = T.sr_base; U.decay = T.decay; U.step = -T.alpha; U.fira = 1.0f; U.zero = 0.0f;
+        if (L.dyn != nullptr) {
+            const af8_dyn_scalars ds = L.dyn[t];
+            U.step = ds.step; U.fira = ds.fira; U.zero = ds.zero;
+        }
+        return T.rows * T.cols;
+    }
 };
 
 template <typename GradT, int PT, bool ANY>
 __global__ void __launch_bounds__(WRITE_THREADS + 32, sizeof_grad<GradT>() == 2 ? 6 : 4)
 factored_write_kernel(const FactoredLaunch L)
 {
-    constexpr int GB = sizeof_grad<GradT>(), PB = PT == 0 ? 4 : 2, P_OFF = WRITE_UNIT * GB, STAGE = write_stage_bytes<GradT, PT>(), NS = WRITE_STAGES;
+    constexpr int GB = sizeof_grad<GradT>(), PB = PT == 0 ? 4 : 2, P_OFF = WRITE_UNIT * GB;
     extern __shared__ __align__(128) unsigned char fw_smem[];
-    __shared__ UnitQueue s_queue;
-    __shared__ __align__(8) uint64_t s_full[NS], s_free[NS];
-    __shared__ WriteUnit s_unit[NS];
-    __shared__ int s_abort;
+    __shared__ __align__(16) WriteShared<FactoredUnit> sh;
     const int tid = threadIdx.x;
-    if (tid == WRITE_THREADS) {
-        for (int k = 0; k < NS; ++k) { mbar_init(&s_full[k], 1); mbar_init(&s_free[k], WRITE_THREADS / 32); }
-        s_abort = 0;
-        unit_start(s_queue);
-    }
-    __syncthreads();
-
-    if (tid >= WRITE_THREADS) {
-        // ---- the fifth warp: units, their tensors' scalars and their copies ----
-        if (tid != WRITE_THREADS) return;
-        int t = -1;
-        int64_t first = 0, end = 0, numel = 0;
-        const unsigned char *grad = nullptr;
-        WriteUnit U = {};
-        int id = (int)blockIdx.x;
-        for (uint32_t n = 0;; ++n) {
-            const int sl = (int)(n % NS);
-            if (n >= NS && !mbar_wait_bounded(&s_free[sl], (n / NS + 1) & 1u)) { s_abort = 1; atomicExch(&g_device_error, DEVERR_WRITE_TIMEOUT); }
-            if (id < 0 || *static_cast<volatile int *>(&s_abort)) {
-                unit_drain(s_queue);
-                s_unit[sl].count = 0;
-                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&s_full[sl])) : "memory");
-                return;
-            }
-            if (t < 0 || id < first || id >= end) {
-                if (t < 0 || id < first) t = find_factored_chunk(L.tensors, L.n_tensors, id);
-                else while (t + 1 < L.n_tensors && __ldg(&L.tensors[t + 1].first_chunk) <= id) ++t;
-                const af8_factored_tensor T = L.tensors[t];
-                numel = T.rows * T.cols; first = T.first_chunk; end = first + (numel + WRITE_UNIT - 1) / WRITE_UNIT;
-                grad = static_cast<const unsigned char *>(T.grad);
-                U.cols = T.cols; U.magic = (uint32_t)(0x100000000ull / (uint64_t)T.cols) + 1u;
-                U.batch_rows = T.batch_rows; U.param = T.param; U.copy = T.param_copy; U.inv_row = T.inv_row; U.inv_col = T.inv_col;
-                U.sr_base = T.sr_base; U.decay = T.decay; U.step = -T.alpha; U.fira = 1.0f; U.zero = 0.0f;
-                if (L.dyn != nullptr) {
-                    const af8_dyn_scalars ds = L.dyn[t];
-                    U.step = ds.step; U.fira = ds.fira; U.zero = ds.zero;
-                }
-            }
-            U.base = (id - first) * WRITE_UNIT;
-            U.count = (int)min((int64_t)WRITE_UNIT, numel - U.base);             // (a multiple of 8)
-            U.row = (numel >> 32) == 0 ? (int64_t)((uint32_t)U.base / (uint32_t)U.cols) : U.base / U.cols;
-            U.col = U.base - U.row * U.cols;
-            s_unit[sl] = U;
-            fence_proxy_async();
-            mbar_expect_tx(&s_full[sl], (uint32_t)(U.count * (GB + PB)));
-            bulk_g2s(fw_smem + sl * STAGE + P_OFF, static_cast<const unsigned char *>(U.param) + U.base * PB, (uint32_t)(U.count * PB), &s_full[sl]);
-            bulk_g2s(fw_smem + sl * STAGE, grad + U.base * GB, (uint32_t)(U.count * GB), &s_full[sl]);
-            id = unit_take(s_queue);
-        }
-    }
-
     const float sgn = L.negate_grad ? -1.0f : 1.0f;                  // ((-g) * r == g * (-r) bit for bit)
-    for (uint32_t n = 0;; ++n) {
-        const int sl = (int)(n % NS);
-        const bool landed = mbar_wait_bounded(&s_full[sl], (n / NS) & 1u);
-        if (!landed) { s_abort = 1; atomicExch(&g_device_error, DEVERR_WRITE_TIMEOUT); }
-        const WriteUnit &U = s_unit[sl];
-        const int count = warp_uniform(U.count);
-        if (count == 0) break;
-        const unsigned char *const st = fw_smem + sl * STAGE;
+    write_units<GB, PB>(FactoredUnits{L}, sh, fw_smem, [&](const FactoredUnit &U, const unsigned char *st, auto release) {
         const int64_t base = U.base;
-        const int64_t C = U.cols;
+        const int count = warp_uniform(U.count);
         float2 x[2][4], u[2][4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -1985,17 +1928,9 @@ factored_write_kernel(const FactoredLaunch L)
             float2 &xa = x[q >> 1][2 * (q & 1)], &xb = x[q >> 1][2 * (q & 1) + 1], &ua = u[q >> 1][2 * (q & 1)], &ub = u[q >> 1][2 * (q & 1) + 1];
             xa = xb = ua = ub = make_float2(0.0f, 0.0f);
             if (o >= count) continue;
-            // the group's row and column: a long row ends once in a unit at most, a short one has columns below 2^12 here
-            int64_t col = U.col + o, row = U.row;
-            if (C >= WRITE_UNIT) {
-                if (col >= C) { col -= C; ++row; }
-            } else {
-                const uint32_t down = __umulhi((uint32_t)col, U.magic);
-                row += down;
-                col = (uint32_t)col - down * (uint32_t)C;
-            }
-            int64_t cb = 0;
-            if (ANY && U.batch_rows > 0) cb = (int64_t)((uint32_t)row / (uint32_t)U.batch_rows) * C;             // (rows < 2^31)
+            int64_t row, col, cb = 0;
+            write_position(U, o, row, col);
+            if (ANY && U.batch_rows > 0) cb = (int64_t)((uint32_t)row / (uint32_t)U.batch_rows) * U.cols;        // (rows < 2^31)
             const float2 ir2 = bc2(__fmul_rn(__ldg(U.inv_row + row), sgn));
             const float4 ic = __ldg(reinterpret_cast<const float4 *>(U.inv_col + cb + col));
             float2 ga, gb;
@@ -2015,9 +1950,7 @@ factored_write_kernel(const FactoredLaunch L)
         void *const param = U.param;
         void *const copy = PT == 0 ? U.copy : nullptr;
         const uint64_t sr_base = PT == 2 ? U.sr_base : 0;
-        __syncwarp();                                                // the stage was read
-        if ((tid & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&s_free[sl])) : "memory");
-        if (!landed) continue;                                       // (nothing is written from a copy that never came)
+        release();
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             float2 (&y)[4] = x[h];
@@ -2051,7 +1984,7 @@ factored_write_kernel(const FactoredLaunch L)
                 }
             }
         }
-    }
+    });
 }
 
 // ---------------------------------------------------------------------------
@@ -3104,8 +3037,8 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
         // no momentum, rows of whole vectors: one CTA per unit
         if (total_chunks > INT32_MAX) return fail(AF8_ERR_UNSUPPORTED, "af8_factored_update: %lld chunks in one launch", (long long)total_chunks);
 #define AF8_LAUNCH_FWRITE(G, T, A) do { \
-        AF8_CUDA_TRY(cudaFuncSetAttribute(factored_write_kernel<G, T, A>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)write_smem_bytes<G, T>())); \
-        factored_write_kernel<G, T, A><<<(int)total_chunks, WRITE_THREADS + 32, write_smem_bytes<G, T>(), cst>>>(L); } while (0)
+        AF8_CUDA_TRY(cudaFuncSetAttribute(factored_write_kernel<G, T, A>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)write_smem_bytes<sizeof_grad<G>(), T == 0 ? 4 : 2>())); \
+        factored_write_kernel<G, T, A><<<(int)total_chunks, WRITE_THREADS + 32, write_smem_bytes<sizeof_grad<G>(), T == 0 ? 4 : 2>(), cst>>>(L); } while (0)
 #define AF8_LAUNCH_FWRITE_ANY(G, T) do { if (any) AF8_LAUNCH_FWRITE(G, T, true); else AF8_LAUNCH_FWRITE(G, T, false); } while (0)
         if (!bf) AF8_LAUNCH_FWRITE_ANY(float, 0);
         else if (pt == 0) AF8_LAUNCH_FWRITE_ANY(bf16_tag, 0);
