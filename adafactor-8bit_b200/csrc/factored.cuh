@@ -900,6 +900,82 @@ __device__ __forceinline__ void stats_rows_any(const FactoredLaunch &L, const af
     }
 }
 
+// Sums over the lanes of a warp of NB values each lane holds, through `buf` (32 * NB doubles of shared memory, this warp's alone): lane l
+// gets the sum of value l / (32 / NB), complete in the first lane of each such group.  Value v of lane l lies at v * 32 + (l ^ (v * G)),
+// so that neither the writes nor the reads of a column of lanes meet in a bank.  (30 instructions for 8 values; exchanging halves of
+// them by shuffles takes 55.)
+template <int NB>
+__device__ __forceinline__ double transpose_sum(const double (&x)[NB], double *buf)
+{
+    constexpr int G = 32 / NB;
+    const int lane = threadIdx.x & 31, v = lane / G;
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < NB; ++k) buf[k * 32 + (lane ^ (k * G))] = x[k];
+    __syncwarp();
+    double t[NB];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) t[i] = buf[v * 32 + (lane & (G - 1)) + G * (i ^ v)];
+#pragma unroll
+    for (int w = NB / 2; w > 0; w >>= 1)
+#pragma unroll
+        for (int i = 0; i < w; ++i) t[i] += t[i + w];
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) t[0] += __shfl_xor_sync(0xffffffffu, t[0], o);
+    return t[0];
+}
+
+// Row and column sums of g^2 over the rows r0 + warp + 8 k of a tile, NB rows at a time, the next NB requested before they are used.
+// buf: 32 * NB doubles of this warp's.
+template <typename GradT, int NB>
+__device__ __forceinline__ void gradsq_rows(const af8_factored_tensor &sT, int64_t r0, int64_t r_end, int64_t c, bool col_ok, double (&cacc)[8], double *buf)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t step = 8 * sT.cols;
+    int64_t off = (r0 + warp) * sT.cols + c;
+    int left = r0 + warp < r_end ? (int)((r_end - (r0 + warp) + 7) / 8) : 0;         // rows from the next group on
+    double *to = sT.row_sum + r0 + warp + 8 * (lane / (32 / NB));
+    const auto load = [&](GradRaw8<GradT> (&raw)[NB], int rows) {
+#pragma unroll
+        for (int k = 0; k < NB; ++k, off += step) {
+            raw[k].zero();
+            if (col_ok && k < rows) raw[k].load(sT.grad, off);
+        }
+    };
+    const auto add = [&](const GradRaw8<GradT> (&raw)[NB]) {
+        double rsum[NB];
+#pragma unroll
+        for (int k = 0; k < NB; ++k) {
+            float g[8];
+            raw[k].unpack(0, g);
+            double t[4];
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) {
+                const float2 gj = make_float2(g[j], g[j + 1]), xx = __fmul2_rn(gj, gj);
+                const double xa = (double)xx.x, xb = (double)xx.y;
+                cacc[j] += xa;
+                cacc[j + 1] += xb;
+                t[j >> 1] = xa + xb;
+            }
+            rsum[k] = (t[0] + t[1]) + (t[2] + t[3]);
+        }
+        const double v = transpose_sum(rsum, buf);
+        if ((lane & (32 / NB - 1)) == 0 && lane / (32 / NB) < left) atomicAdd(to, v);
+        to += 8 * NB;
+        left -= NB;
+    };
+    GradRaw8<GradT> a[NB], b[NB];
+    load(a, left);
+    while (left > 0) {                                               // (uniform over the warp)
+        load(b, left - NB);
+        add(a);
+        if (left <= 0) break;
+        load(a, left - NB);
+        add(b);
+    }
+    __syncwarp();
+}
+
 // Rows r0 + warp + 8k of the tile, NB at a time so that NB independent 128-bit loads per lane
 // are in flight.  Column partials go to a per-warp shared array (no shared-memory atomics).
 template <typename GradT, int NB, bool PREFETCH, bool RESIDUAL>
@@ -1482,7 +1558,7 @@ factored_stats_vec_kernel(const FactoredLaunch L, const CUtensorMap *__restrict_
             }
         } else if (!vec) {
             if constexpr (ANY && RESIDUAL) stats_rows_any<GradT, 4>(L, sT, r0, row_end, c, pre_div, ic, cacc);
-        } else if (!RESIDUAL) stats_rows<GradT, 4, true, false>(L, sT, r0, row_end, c, col_ok, pre_div, ic, cacc);
+        } else if (!RESIDUAL) gradsq_rows<GradT, sizeof_grad<GradT>() == 2 ? 4 : 2>(sT, r0, row_end, c, col_ok, cacc, s_col[warp]);
         else stats_rows<GradT, AF8_FSTAT_RES_NB, AF8_FSTAT_RES_PREFETCH, true>(L, sT, r0, row_end, c, col_ok, pre_div, ic, cacc);
         if (!ok) {
             atomicExch(&g_device_error, DEVERR_SRING_TIMEOUT);
