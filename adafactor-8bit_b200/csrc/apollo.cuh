@@ -343,7 +343,7 @@ __device__ __forceinline__ int find_finish_tensor(const af8_apollo_finish_tensor
     int lo = 0, hi = n - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (__ldg(&t[mid].first_unit) <= unit) lo = mid; else hi = mid - 1;
+        if (t[mid].first_unit <= unit) lo = mid; else hi = mid - 1;
     }
     return lo;
 }
@@ -353,17 +353,18 @@ __device__ __forceinline__ int find_finish_tensor(const af8_apollo_finish_tensor
 // unit are 32 contiguous bytes of every row, so 8 lanes take one row and the 32 groups of a CTA walk
 // the rows together; the sums of a channel are then added over the groups in a fixed order.
 __global__ void __launch_bounds__(256)
-apollo_scales_multi_kernel(const af8_apollo_finish_tensor *__restrict__ T, int n, int64_t total_units)
+apollo_scales_multi_kernel(const af8_apollo_finish_tensor *T, int n, int64_t total_units)
 {
     __shared__ double s_part[8];
     __shared__ double s_nu[8][8], s_ng[8][8];        // left case: [warp][channel of the unit]
+    await_launches();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     for (int64_t unit = blockIdx.x; unit < total_units; unit += gridDim.x) {
         const af8_apollo_finish_tensor *t = T + find_finish_tensor(T, n, unit);
-        const int64_t rows = __ldg(&t->rows), cols = __ldg(&t->cols), rank = __ldg(&t->rank);
+        const int64_t rows = t->rows, cols = t->cols, rank = t->rank;
         const bool right = rows >= cols;
         const int64_t nch = right ? rows : cols;
-        const int64_t ch0 = (unit - __ldg(&t->first_unit)) * 8;
+        const int64_t ch0 = (unit - t->first_unit) * 8;
         const int64_t ch = ch0 + warp;
         const float *upd = t->upd, *g_low = t->g_low;
         double local = 0.0;
@@ -404,7 +405,7 @@ apollo_scales_multi_kernel(const af8_apollo_finish_tensor *__restrict__ T, int n
         }
         if (lane == 0 && ch < nch) {
             float s = __fdiv_rn(__double2float_rn(sqrt(nu)), __fadd_rn(__double2float_rn(sqrt(ng)), 1e-8f));   // optimizer.py:2964
-            if (__ldg(&t->in.scale_front)) s = __fmul_rn(s, __ldg(&t->in.sqrt_scale));                       // optimizer.py:2969-2971
+            if (t->in.scale_front) s = __fmul_rn(s, t->in.sqrt_scale);                       // optimizer.py:2969-2971
             t->sf[ch] = s;
             const float nG = __double2float_rn(sqrt(t->chan_g2[ch]));
             local = (double)__fmul_rn(__fmul_rn(nG, nG), __fmul_rn(s, s));                                   // optimizer.py:2975-2982
@@ -423,6 +424,7 @@ apollo_scales_multi_kernel(const af8_apollo_finish_tensor *__restrict__ T, int n
 __global__ void apollo_finalize_multi_kernel(const af8_apollo_finish_tensor *T, int n)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    await_launches();
     if (i < n) {
         const af8_apollo_scalars_in in = T[i].in;
         apollo_finalize_one(in, T[i].sums, T[i].sf, T[i].fira_prev, T[i].out, T[i].alpha_decay);
@@ -612,7 +614,7 @@ struct ApolloUnits {
     const af8_apollo_apply_tensor *tensors;
     int n;
     __device__ __forceinline__ int count() const { return n; }
-    __device__ __forceinline__ int64_t first(int t) const { return __ldg(&tensors[t].first_chunk); }
+    __device__ __forceinline__ int64_t first(int t) const { return tensors[t].first_chunk; }
     __device__ __forceinline__ int64_t load(int t, ApolloUnit &U) const
     {
         const af8_apollo_apply_tensor T = tensors[t];
@@ -977,8 +979,8 @@ extern "C" int af8_apollo_project_batch(const af8_apollo_proj_desc *descs, int32
             host_u[i].t.first_tile = tile;
             tile += (host_u[i].t.M + UM_BM - 1) / UM_BM;
         }
-        AF8_CUDA_TRY(cudaMemcpyAsync(dev_scratch, host_u, sizeof(UmmaTask) * (size_t)iu, cudaMemcpyHostToDevice, st));
-        int rc = apollo_project_launch_umma(dev_u, iu, tiles_u, st);
+        int rc = upload_table(dev_scratch, host_u, sizeof(UmmaTask) * (size_t)iu, st);
+        if (!rc) rc = apollo_project_launch_umma(dev_u, iu, tiles_u, st);
         if (rc) return rc;
     }
     if (n_mma) {
@@ -1025,6 +1027,9 @@ extern "C" int af8_apollo_scales_batch(const af8_apollo_finish_tensor *host_tens
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int64_t next = 0;
     char *run_begin = nullptr, *run_end = nullptr;
+    const auto clear = [&](char *begin, char *end) {
+        return begin == end ? AF8_OK : clear_doubles(reinterpret_cast<double *>(begin), (end - begin) / 8, nullptr, 0, st);
+    };
     for (int i = 0; i < n; ++i) {
         const af8_apollo_finish_tensor &t = host_tensors[i];
         if (!t.upd || !t.g_low || !t.chan_g2 || !t.sf || !t.sums || !t.out) return fail(AF8_ERR_INVALID, "af8_apollo_scales_batch: tensor %d: null pointer", i);
@@ -1033,21 +1038,24 @@ extern "C" int af8_apollo_scales_batch(const af8_apollo_finish_tensor *host_tens
         if (t.rows <= 0 || t.cols <= 0 || t.rank <= 0) return fail(AF8_ERR_INVALID, "af8_apollo_scales_batch: tensor %d: bad shape", i);
         if (t.first_unit != next) return fail(AF8_ERR_INVALID, "af8_apollo_scales_batch: tensor %d: first_unit %lld, expected %lld", i, (long long)t.first_unit, (long long)next);
         next += ((t.rows >= t.cols ? t.rows : t.cols) + 7) / 8;
-        // clear the three accumulators of every tensor; neighbours in memory share one memset
+        // clear the three accumulators of every tensor; neighbours in memory are cleared together
         char *p = reinterpret_cast<char *>(t.sums);
         if (p == run_end) { run_end += 24; continue; }
-        if (run_end != run_begin) AF8_CUDA_TRY(cudaMemsetAsync(run_begin, 0, (size_t)(run_end - run_begin), st));
+        const int rz = clear(run_begin, run_end);
+        if (rz) return rz;
         run_begin = p;
         run_end = p + 24;
     }
-    if (run_end != run_begin) AF8_CUDA_TRY(cudaMemsetAsync(run_begin, 0, (size_t)(run_end - run_begin), st));
+    const int rz = clear(run_begin, run_end);
+    if (rz) return rz;
     if (next != total_units) return fail(AF8_ERR_INVALID, "af8_apollo_scales_batch: total_units is %lld but the table holds %lld", (long long)total_units, (long long)next);
-    AF8_CUDA_TRY(cudaMemcpyAsync(dev_tensors, host_tensors, sizeof(af8_apollo_finish_tensor) * (size_t)n, cudaMemcpyHostToDevice, st));
+    const int ru = upload_table(dev_tensors, host_tensors, sizeof(af8_apollo_finish_tensor) * (size_t)n, st);
+    if (ru) return ru;
     int64_t grid = (int64_t)sm_count() * 8;
     if (grid > total_units) grid = total_units;
-    apollo_scales_multi_kernel<<<(int)grid, 256, 0, st>>>(dev_tensors, n, total_units);
+    launch_next(apollo_scales_multi_kernel, (unsigned)grid, 256, 0, st, dev_tensors, n, total_units);
     AF8_CUDA_TRY(cudaGetLastError());
-    apollo_finalize_multi_kernel<<<(n + 127) / 128, 128, 0, st>>>(dev_tensors, n);
+    launch_next(apollo_finalize_multi_kernel, (unsigned)((n + 127) / 128), 128, 0, st, dev_tensors, n);
     AF8_CUDA_TRY(cudaGetLastError());
     return AF8_OK;
 }
@@ -1142,13 +1150,14 @@ extern "C" int af8_apollo_apply_batch(const af8_apollo_apply_tensor *host_tensor
         return AF8_OK;
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    AF8_CUDA_TRY(cudaMemcpyAsync(dev_tensors, host_tensors, sizeof(af8_apollo_apply_tensor) * (size_t)n, cudaMemcpyHostToDevice, st));
+    const int ru = upload_table(dev_tensors, host_tensors, sizeof(af8_apollo_apply_tensor) * (size_t)n, st);
+    if (ru) return ru;
     const bool lowp = param_dtype != AF8_F32;
     if (total_chunks > INT32_MAX) return fail(AF8_ERR_UNSUPPORTED, "af8_apollo_apply_batch: %lld chunks in one launch", (long long)total_chunks);
 #define AF8_APOLLO_APPLY_BATCH(B, L) do { \
         constexpr size_t smem = write_smem_bytes<(B) ? 2 : 4, (L) ? 2 : 4>(); \
         AF8_CUDA_TRY(cudaFuncSetAttribute(apollo_write_kernel<B, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-        apollo_write_kernel<B, L><<<(int)total_chunks, WRITE_THREADS + 32, smem, st>>>(dev_tensors, n, negate, param_dtype); \
+        launch_next(apollo_write_kernel<B, L>, (unsigned)total_chunks, WRITE_THREADS + 32, smem, st, dev_tensors, n, negate, param_dtype); \
     } while (0)
     if (grad_dtype == AF8_BF16) { if (lowp) AF8_APOLLO_APPLY_BATCH(true, true); else AF8_APOLLO_APPLY_BATCH(true, false); }
     else { if (lowp) AF8_APOLLO_APPLY_BATCH(false, true); else AF8_APOLLO_APPLY_BATCH(false, false); }

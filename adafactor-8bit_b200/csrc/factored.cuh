@@ -28,6 +28,7 @@
 #include "fullrank_fast.cuh"
 #include "fullrank_generic.cuh"
 #include "fullrank_stat.cuh"
+#include "launch.cuh"
 #include "tensormap.cuh"
 #include "write_units.cuh"
 
@@ -61,7 +62,7 @@ __device__ __forceinline__ int find_factored_tile(const af8_factored_tensor *t, 
     int lo = 0, hi = n - 1;
     while (lo < hi) {
         int mid = (lo + hi + 1) >> 1;
-        if (__ldg(&t[mid].first_tile) <= id) lo = mid; else hi = mid - 1;
+        if (t[mid].first_tile <= id) lo = mid; else hi = mid - 1;
     }
     return lo;
 }
@@ -70,7 +71,7 @@ __device__ __forceinline__ int find_factored_chunk(const af8_factored_tensor *t,
     int lo = 0, hi = n - 1;
     while (lo < hi) {
         int mid = (lo + hi + 1) >> 1;
-        if (__ldg(&t[mid].first_chunk) <= id) lo = mid; else hi = mid - 1;
+        if (t[mid].first_chunk <= id) lo = mid; else hi = mid - 1;
     }
     return lo;
 }
@@ -268,12 +269,13 @@ factored_stats_kernel(const FactoredLaunch L)
     __shared__ double s_col[FSTAT_COLS];
     __shared__ af8_factored_tensor sT;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    await_launches();
 
     for (int64_t id = blockIdx.x; id < L.total_units; id += gridDim.x) {
         const int t = find_factored_tile(L.tensors, L.n_tensors, id);
         __syncthreads();
         if (tid < (int)(sizeof(af8_factored_tensor) / 4))
-            reinterpret_cast<uint32_t *>(&sT)[tid] = __ldg(reinterpret_cast<const uint32_t *>(L.tensors + t) + tid);
+            reinterpret_cast<uint32_t *>(&sT)[tid] = reinterpret_cast<const uint32_t *>(L.tensors + t)[tid];
         s_col[tid] = 0.0;
         __syncthreads();
         const int64_t C = sT.cols;
@@ -338,6 +340,7 @@ factored_stats_kernel(const FactoredLaunch L)
 __global__ void __launch_bounds__(256)
 factored_clear_kernel(const af8_factored_tensor *tensors)
 {
+    await_launches();
     const af8_factored_tensor &T = tensors[blockIdx.x];
     const int64_t stride = (int64_t)blockDim.x * gridDim.y, first = (int64_t)blockIdx.y * blockDim.x + threadIdx.x;
     const int64_t nr = T.rows, nc = fact_batch(T) * T.cols;
@@ -423,7 +426,7 @@ __device__ __forceinline__ int find_factored_small(const af8_factored_tensor *t,
     int lo = 0, hi = n - 1;
     while (lo < hi) {
         int mid = (lo + hi + 1) >> 1;
-        if (__ldg(&t[mid].first_small) <= id) lo = mid; else hi = mid - 1;
+        if (t[mid].first_small <= id) lo = mid; else hi = mid - 1;
     }
     return lo;
 }
@@ -441,6 +444,7 @@ factored_small_kernel(const af8_factored_tensor *tensors, int n_tensors, int con
     __shared__ float s_red[2][SMALL_MAX_THREADS / 32];
     __shared__ double s_acc[SMALL_MAX_THREADS / 32];
     load_codec_tables(s_codec);
+    await_launches();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int t = find_factored_small(tensors, n_tensors, (int)blockIdx.x);
     const af8_factored_tensor &T = tensors[t];
@@ -478,6 +482,7 @@ __global__ void __launch_bounds__(256)
 factored_inv_kernel(const af8_factored_tensor *tensors, int conf)
 {
     __shared__ float s_rm;
+    await_launches();
     const af8_factored_tensor T = tensors[blockIdx.x];
     const int tid = threadIdx.x;
     float *inv_r = conf ? T.inv_row_conf : T.inv_row;
@@ -533,6 +538,7 @@ factored_update_kernel(const FactoredLaunch L, int chunk)
     __shared__ af8_factored_tensor sT;
     __shared__ double s_acc[FUPD_THREADS / 32];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    await_launches();
     const bool has_m = L.m_fmt != AF8_M_NONE;
     const bool m_quant = has_m && L.m_fmt != AF8_M_FP32;
     const bool writes = L.mode == AF8_FUPD_APPLY || L.mode == AF8_FUPD_LAG;
@@ -542,7 +548,7 @@ factored_update_kernel(const FactoredLaunch L, int chunk)
         const int t = find_factored_chunk(L.tensors, L.n_tensors, id);
         __syncthreads();
         if (tid < (int)(sizeof(af8_factored_tensor) / 4))
-            reinterpret_cast<uint32_t *>(&sT)[tid] = __ldg(reinterpret_cast<const uint32_t *>(L.tensors + t) + tid);
+            reinterpret_cast<uint32_t *>(&sT)[tid] = reinterpret_cast<const uint32_t *>(L.tensors + t)[tid];
         __syncthreads();
         const int64_t C = sT.cols, numel = sT.rows * sT.cols;
         const int64_t base = (id - sT.first_chunk) * chunk;
@@ -1484,16 +1490,17 @@ factored_stats_vec_kernel(const FactoredLaunch L, const CUtensorMap *__restrict_
         }
         __syncthreads();
     }
+    await_launches();
 
     for (int64_t id = blockIdx.x; id < L.total_units; id += gridDim.x) {
         int t = cur_t;
         const int64_t tile = id >> L.split;
         if (t < 0) t = find_factored_tile(L.tensors, L.n_tensors, tile);
-        else while (t + 1 < L.n_tensors && __ldg(&L.tensors[t + 1].first_tile) <= tile) ++t;
+        else while (t + 1 < L.n_tensors && L.tensors[t + 1].first_tile <= tile) ++t;
         __syncthreads();                                           // s_col of the previous tile was read
         if (t != cur_t) {
             if (tid < (int)(sizeof(af8_factored_tensor) / 4))
-                reinterpret_cast<uint32_t *>(&sT)[tid] = __ldg(reinterpret_cast<const uint32_t *>(L.tensors + t) + tid);
+                reinterpret_cast<uint32_t *>(&sT)[tid] = reinterpret_cast<const uint32_t *>(L.tensors + t)[tid];
             cur_t = t;
             __syncthreads();
         }
@@ -1603,6 +1610,7 @@ factored_update_vec_kernel(const FactoredLaunch L)
     __shared__ af8_factored_tensor sT;
     __shared__ double s_acc2[1][FUPD_THREADS / 32];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    await_launches();
     const bool has_m = L.m_fmt != AF8_M_NONE;
     const bool m_quant = has_m && L.m_fmt != AF8_M_FP32;
     constexpr bool writes = WRITES;
@@ -1652,13 +1660,13 @@ factored_update_vec_kernel(const FactoredLaunch L)
             run_first = id;
             int tn = cur_t;
             if (tn < 0) tn = find_factored_chunk(L.tensors, L.n_tensors, id);
-            else while (tn + 1 < L.n_tensors && __ldg(&L.tensors[tn + 1].first_chunk) <= id) ++tn;
+            else while (tn + 1 < L.n_tensors && L.tensors[tn + 1].first_chunk <= id) ++tn;
             __syncthreads();
             if (tid < (int)(sizeof(af8_factored_tensor) / 4))
-                reinterpret_cast<uint32_t *>(&sT)[tid] = __ldg(reinterpret_cast<const uint32_t *>(L.tensors + tn) + tid);
+                reinterpret_cast<uint32_t *>(&sT)[tid] = reinterpret_cast<const uint32_t *>(L.tensors + tn)[tid];
             cur_t = tn;
             __syncthreads();
-            next_first = tn + 1 < L.n_tensors ? __ldg(&L.tensors[tn + 1].first_chunk) : L.total_units;
+            next_first = tn + 1 < L.n_tensors ? L.tensors[tn + 1].first_chunk : L.total_units;
             flat = (id - sT.first_chunk) * 2048 + tid * 8;
             row = flat / sT.cols;
             col = flat - row * sT.cols;
@@ -1971,7 +1979,7 @@ struct FactoredUnit : WriteUnit {
 struct FactoredUnits {
     const FactoredLaunch &L;
     __device__ __forceinline__ int count() const { return L.n_tensors; }
-    __device__ __forceinline__ int64_t first(int t) const { return __ldg(&L.tensors[t].first_chunk); }
+    __device__ __forceinline__ int64_t first(int t) const { return L.tensors[t].first_chunk; }
     __device__ __forceinline__ int64_t load(int t, FactoredUnit &U) const
     {
         const af8_factored_tensor T = L.tensors[t];
@@ -2144,6 +2152,7 @@ factored_apply_flat_kernel(const FactoredLaunch L)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    await_launches();
 
     const int64_t per_cta = (L.total_units + gridDim.x - 1) / gridDim.x;
     const int64_t id_begin = (int64_t)blockIdx.x * per_cta;
@@ -2159,10 +2168,10 @@ factored_apply_flat_kernel(const FactoredLaunch L)
         if (cur_t < 0 || id >= sF.next_first) {
             int tn = cur_t;
             if (tn < 0) tn = find_factored_chunk(L.tensors, L.n_tensors, id);
-            else while (tn + 1 < L.n_tensors && __ldg(&L.tensors[tn + 1].first_chunk) <= id) ++tn;
+            else while (tn + 1 < L.n_tensors && L.tensors[tn + 1].first_chunk <= id) ++tn;
             __syncthreads();
             if (tid < (int)(sizeof(af8_factored_tensor) / 4))
-                reinterpret_cast<uint32_t *>(&sT)[tid] = __ldg(reinterpret_cast<const uint32_t *>(L.tensors + tn) + tid);
+                reinterpret_cast<uint32_t *>(&sT)[tid] = reinterpret_cast<const uint32_t *>(L.tensors + tn)[tid];
             cur_t = tn;
             __syncthreads();
             const int64_t C = sT.cols;
@@ -2172,7 +2181,7 @@ factored_apply_flat_kernel(const FactoredLaunch L)
             if (tid == 0) {
                 FlatTensor F;
                 F.numel = sT.rows * C;
-                F.next_first = tn + 1 < L.n_tensors ? __ldg(&L.tensors[tn + 1].first_chunk) : L.total_units;
+                F.next_first = tn + 1 < L.n_tensors ? L.tensors[tn + 1].first_chunk : L.total_units;
                 F.full_end = min(id_end, sT.first_chunk + F.numel / 2048);
                 F.adv_rows = 2048 / C;
                 F.adv_cols = 2048 - F.adv_rows * C;
@@ -2387,6 +2396,7 @@ factored_apply_tile_kernel(const FactoredLaunch L)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    await_launches();
 
     int cur_t = -1;
     float pre_div = 1.0f, step_mul = 0.0f, fira = 1.0f;
@@ -2398,11 +2408,11 @@ factored_apply_tile_kernel(const FactoredLaunch L)
         int t = cur_t;
         const int64_t tile = id >> L.split;
         if (t < 0) t = find_factored_tile(L.tensors, L.n_tensors, tile);
-        else while (t + 1 < L.n_tensors && __ldg(&L.tensors[t + 1].first_tile) <= tile) ++t;
+        else while (t + 1 < L.n_tensors && L.tensors[t + 1].first_tile <= tile) ++t;
         if (t != cur_t) {
             __syncthreads();                                         // every warp has left the previous tensor
             if (tid < (int)(sizeof(af8_factored_tensor) / 4))
-                reinterpret_cast<uint32_t *>(&sT)[tid] = __ldg(reinterpret_cast<const uint32_t *>(L.tensors + t) + tid);
+                reinterpret_cast<uint32_t *>(&sT)[tid] = reinterpret_cast<const uint32_t *>(L.tensors + t)[tid];
             cur_t = t;
             __syncthreads();
             pre_div = 1.0f; step_mul = -sT.alpha; fira = 1.0f; zero_upd = false;
@@ -2575,6 +2585,7 @@ template <typename GradT>
 __global__ void __launch_bounds__(FUPD_THREADS, 4)
 factored_sumsq_wide_kernel(const FactoredLaunch L)
 {
+    await_launches();
     __shared__ af8_factored_tensor sT;
     __shared__ double s_acc2[FUPD_THREADS / 32];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -2584,12 +2595,12 @@ factored_sumsq_wide_kernel(const FactoredLaunch L)
     int tn = -1;
     for (int64_t id = id_begin; id < id_end;) {
         if (tn < 0) tn = find_factored_chunk(L.tensors, L.n_tensors, id);
-        else while (tn + 1 < L.n_tensors && __ldg(&L.tensors[tn + 1].first_chunk) <= id) ++tn;
+        else while (tn + 1 < L.n_tensors && L.tensors[tn + 1].first_chunk <= id) ++tn;
         __syncthreads();
         if (tid < (int)(sizeof(af8_factored_tensor) / 4))
-            reinterpret_cast<uint32_t *>(&sT)[tid] = __ldg(reinterpret_cast<const uint32_t *>(L.tensors + tn) + tid);
+            reinterpret_cast<uint32_t *>(&sT)[tid] = reinterpret_cast<const uint32_t *>(L.tensors + tn)[tid];
         __syncthreads();
-        const int64_t next_first = tn + 1 < L.n_tensors ? __ldg(&L.tensors[tn + 1].first_chunk) : L.total_units;
+        const int64_t next_first = tn + 1 < L.n_tensors ? L.tensors[tn + 1].first_chunk : L.total_units;
         const int64_t run_end = min(id_end, next_first);         // this CTA's chunks of this tensor: id .. run_end - 1
         const int64_t e0 = (id - sT.first_chunk) * 2048;
         const int64_t e1 = min((run_end - sT.first_chunk) * 2048, sT.rows * sT.cols);
@@ -2626,6 +2637,7 @@ factored_sumsq_slice_kernel(const FactoredLaunch L, const int whole)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    await_launches();
     unsigned char *const ring = sr_smem + (size_t)warp * slice_warp_bytes<GradT>();
     uint32_t cons = 0;
     int cur_t = -1;
@@ -2633,11 +2645,11 @@ factored_sumsq_slice_kernel(const FactoredLaunch L, const int whole)
         int t = cur_t;
         const int64_t tile = id >> L.split;
         if (t < 0) t = find_factored_tile(L.tensors, L.n_tensors, tile);
-        else while (t + 1 < L.n_tensors && __ldg(&L.tensors[t + 1].first_tile) <= tile) ++t;
+        else while (t + 1 < L.n_tensors && L.tensors[t + 1].first_tile <= tile) ++t;
         __syncthreads();                                           // s_acc2 of the previous tile was read
         if (t != cur_t) {
             if (tid < (int)(sizeof(af8_factored_tensor) / 4))
-                reinterpret_cast<uint32_t *>(&sT)[tid] = __ldg(reinterpret_cast<const uint32_t *>(L.tensors + t) + tid);
+                reinterpret_cast<uint32_t *>(&sT)[tid] = reinterpret_cast<const uint32_t *>(L.tensors + t)[tid];
             cur_t = t;
             __syncthreads();
         }
@@ -2689,16 +2701,17 @@ factored_sumsq_tile_kernel(const FactoredLaunch L)
     __shared__ af8_factored_tensor sT;
     __shared__ double s_acc2[8];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    await_launches();
     int cur_t = -1;
     for (int64_t id = blockIdx.x; id < L.total_units; id += gridDim.x) {
         int t = cur_t;
         const int64_t tile = id >> L.split;
         if (t < 0) t = find_factored_tile(L.tensors, L.n_tensors, tile);
-        else while (t + 1 < L.n_tensors && __ldg(&L.tensors[t + 1].first_tile) <= tile) ++t;
+        else while (t + 1 < L.n_tensors && L.tensors[t + 1].first_tile <= tile) ++t;
         __syncthreads();                                           // s_acc2 of the previous tile was read
         if (t != cur_t) {
             if (tid < (int)(sizeof(af8_factored_tensor) / 4))
-                reinterpret_cast<uint32_t *>(&sT)[tid] = __ldg(reinterpret_cast<const uint32_t *>(L.tensors + t) + tid);
+                reinterpret_cast<uint32_t *>(&sT)[tid] = reinterpret_cast<const uint32_t *>(L.tensors + t)[tid];
             cur_t = t;
             __syncthreads();
         }
@@ -2860,9 +2873,7 @@ extern "C" int af8_factored_upload(const af8_factored_cfg *cfg, const af8_factor
     if (!host_tensors || !dev_tensors || n_tensors <= 0) return fail(AF8_ERR_INVALID, "af8_factored_upload: null or empty table");
     rc = validate_factored(*cfg, host_tensors, n_tensors);
     if (rc) return rc;
-    AF8_CUDA_TRY(cudaMemcpyAsync(dev_tensors, host_tensors, sizeof(af8_factored_tensor) * (size_t)n_tensors,
-                                 cudaMemcpyHostToDevice, static_cast<cudaStream_t>(stream)));
-    return AF8_OK;
+    return upload_table(dev_tensors, host_tensors, sizeof(af8_factored_tensor) * (size_t)n_tensors, static_cast<cudaStream_t>(stream));
 }
 
 namespace af8 {
@@ -2899,9 +2910,8 @@ static int af8_factored_stats_impl(const af8_factored_cfg *cfg, const af8_factor
     if (cfg->mode == AF8_FSTAT_RESIDUAL && (!cfg->came || !dyn)) return fail(AF8_ERR_INVALID, "af8_factored_stats: the residual needs CAME and dyn");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int64_t tiles = 0;
-    // clear the accumulators: ranges that follow one another in memory form a run; one or two runs take a memset each
-    // (3 us of copy engine and gap apiece), more of them one launch over the table
-    // (29 tensors of odd sizes: 58 memsets, 93 us of a step)
+    // clear the accumulators: ranges that follow one another in memory form a run; one or two runs are cleared as such, more of them by a
+    // launch over the table
     struct { char *begin, *end; } run[2] = {};
     int runs = 0;
     for (int i = 0; i < n_tensors; ++i) {
@@ -2916,9 +2926,11 @@ static int af8_factored_stats_impl(const af8_factored_cfg *cfg, const af8_factor
         tiles += fact_tiles(t);
     }
     if (runs <= 2) {
-        for (int k = 0; k < runs; ++k) AF8_CUDA_TRY(cudaMemsetAsync(run[k].begin, 0, (size_t)(run[k].end - run[k].begin), st));
+        const int rz = clear_doubles(reinterpret_cast<double *>(run[0].begin), (run[0].end - run[0].begin) / 8,
+                                     reinterpret_cast<double *>(run[1].begin), (run[1].end - run[1].begin) / 8, st);
+        if (rz) return rz;
     } else {
-        factored_clear_kernel<<<dim3((unsigned)n_tensors, 4), 256, 0, st>>>(dev_tensors);
+        launch_next(factored_clear_kernel, dim3((unsigned)n_tensors, 4), 256, 0, st, dev_tensors);
         AF8_CUDA_TRY(cudaGetLastError());
     }
     const bool bf = cfg->grad_dtype == AF8_BF16, res = cfg->mode == AF8_FSTAT_RESIDUAL;
@@ -2950,7 +2962,8 @@ static int af8_factored_stats_impl(const af8_factored_cfg *cfg, const af8_factor
                 rc = factored_box_maps(host_tensors[i], hm + 2 * i);
                 if (rc) return rc;
             }
-            AF8_CUDA_TRY(cudaMemcpyAsync(dev_maps, host_maps, sizeof(CUtensorMap) * 2 * (size_t)n_tensors, cudaMemcpyHostToDevice, st));
+            rc = upload_table(dev_maps, host_maps, sizeof(CUtensorMap) * 2 * (size_t)n_tensors, st);
+            if (rc) return rc;
             maps = static_cast<const CUtensorMap *>(dev_maps);
             ring = 2;
         }
@@ -2958,7 +2971,7 @@ static int af8_factored_stats_impl(const af8_factored_cfg *cfg, const af8_factor
 #define AF8_LAUNCH_FSTAT_IN(G, RES, A, I) do { \
         const size_t sm = (I) ? slice_smem_bytes<G>() : 0; \
         if (sm > 0) AF8_CUDA_TRY(cudaFuncSetAttribute(factored_stats_vec_kernel<G, RES, A, I>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)); \
-        factored_stats_vec_kernel<G, RES, A, I><<<(int)grid, 256, sm, st>>>(L, maps); } while (0)
+        launch_next(factored_stats_vec_kernel<G, RES, A, I>, (int)grid, 256, sm, st, L, maps); } while (0)
 #define AF8_LAUNCH_FSTAT(G, RES) do { \
         if (any && ring) AF8_LAUNCH_FSTAT_IN(G, RES, true, 1); else if (any) AF8_LAUNCH_FSTAT_IN(G, RES, true, 0); \
         else if (RES && ring == 1) AF8_LAUNCH_FSTAT_IN(G, RES, false, 1); else AF8_LAUNCH_FSTAT_IN(G, RES, false, 0); } while (0)
@@ -2969,7 +2982,7 @@ static int af8_factored_stats_impl(const af8_factored_cfg *cfg, const af8_factor
     else if (vec) AF8_LAUNCH_FSTAT(float, false);
 #undef AF8_LAUNCH_FSTAT
 #undef AF8_LAUNCH_FSTAT_IN
-    else factored_stats_kernel<<<(int)grid, 256, 0, st>>>(L);
+    else launch_next(factored_stats_kernel, (int)grid, 256, 0, st, L);
     AF8_CUDA_TRY(cudaGetLastError());
     return AF8_OK;
 }
@@ -3001,10 +3014,10 @@ extern "C" int af8_factored_small(const af8_factored_cfg *cfg, const af8_factore
     // launch and factored_inv_kernel with 256, 512 and 1024 threads, few units: blocks of 256 13.3, 13.3, 14.1 us; of 512 14.0, 13.3,
     // 14.6; of 1024 15.4, 14.6, 14.4; of 2048 18.4, 15.4, 15.4 (CAME's confidence states 25.0, 20.9, 19.9); of 4096 21.5, 17.4, 17.2.
     // Many units: 480 of 256 elements 6.2 us with 256 threads, 14 with 512.
-    if (total_units <= sm_count()) factored_small_kernel<SMALL_MAX_THREADS><<<total_units, SMALL_MAX_THREADS, 0, st>>>(dev_tensors, n_tensors, conf, cfg->v_floor);
-    else factored_small_kernel<256><<<total_units, 256, 0, st>>>(dev_tensors, n_tensors, conf, cfg->v_floor);
+    if (total_units <= sm_count()) launch_next(factored_small_kernel<SMALL_MAX_THREADS>, total_units, SMALL_MAX_THREADS, 0, st, dev_tensors, n_tensors, conf, cfg->v_floor);
+    else launch_next(factored_small_kernel<256>, total_units, 256, 0, st, dev_tensors, n_tensors, conf, cfg->v_floor);
     AF8_CUDA_TRY(cudaGetLastError());
-    factored_inv_kernel<<<dim3((unsigned)n_tensors, 8), 256, 0, st>>>(dev_tensors, conf);
+    launch_next(factored_inv_kernel, dim3((unsigned)n_tensors, 8), 256, 0, st, dev_tensors, conf);
     AF8_CUDA_TRY(cudaGetLastError());
     return AF8_OK;
 }
@@ -3056,7 +3069,8 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
     const bool mom = !cfg->came && cfg->m_fmt == AF8_M_UF8 && cfg->m_block == 256 && filled && total_chunks >= slice_from;
     if (vec && !apply && !tile_off && total_tiles > 0 && cfg->grad_dtype != AF8_F16 && (only_g || mom)) {
         // over the statistic tiles, column factors in registers; with a momentum, or rows of any length, in slices
-        AF8_CUDA_TRY(cudaMemsetAsync(block_sumsq, 0, sizeof(double) * (size_t)total_chunks, cst));
+        const int rz = clear_doubles(block_sumsq, total_chunks, nullptr, 0, cst);
+        if (rz) return rz;
         FactoredLaunch LT = L;
         LT.split = tile_split(total_tiles);
         LT.total_units = total_tiles << LT.split;
@@ -3065,7 +3079,7 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
             const int64_t sg = std::min<int64_t>((int64_t)sm_count() * (bf ? 3 : 2), LT.total_units);
 #define AF8_LAUNCH_FSLICE(G, M) do { \
             AF8_CUDA_TRY(cudaFuncSetAttribute(factored_sumsq_slice_kernel<G, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)slice_smem_bytes<G>())); \
-            factored_sumsq_slice_kernel<G, M><<<(int)sg, 256, slice_smem_bytes<G>(), cst>>>(LT, 2 - kind); } while (0)
+            launch_next(factored_sumsq_slice_kernel<G, M>, (int)sg, 256, slice_smem_bytes<G>(), cst, LT, 2 - kind); } while (0)
             if (bf) { if (mom) AF8_LAUNCH_FSLICE(bf16_tag, true); else AF8_LAUNCH_FSLICE(bf16_tag, false); }
             else { if (mom) AF8_LAUNCH_FSLICE(float, true); else AF8_LAUNCH_FSLICE(float, false); }
 #undef AF8_LAUNCH_FSLICE
@@ -3073,8 +3087,8 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
             return AF8_OK;
         }
         const int64_t tg = std::min<int64_t>((int64_t)sm_count() * 8, LT.total_units);
-#define AF8_LAUNCH_FSUM(G) do { if (kind == 0) factored_sumsq_tile_kernel<G, 0><<<(int)tg, 256, 0, cst>>>(LT); \
-        else factored_sumsq_tile_kernel<G, 1><<<(int)tg, 256, 0, cst>>>(LT); } while (0)
+#define AF8_LAUNCH_FSUM(G) do { if (kind == 0) launch_next(factored_sumsq_tile_kernel<G, 0>, (int)tg, 256, 0, cst, LT); \
+        else launch_next(factored_sumsq_tile_kernel<G, 1>, (int)tg, 256, 0, cst, LT); } while (0)
         if (bf) AF8_LAUNCH_FSUM(bf16_tag);
         else AF8_LAUNCH_FSUM(float);
 #undef AF8_LAUNCH_FSUM
@@ -3083,8 +3097,8 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
     }
     if (vec && !any && !apply && !wide_off && cfg->grad_dtype != AF8_F16 && ((cfg->came && cfg->mode == AF8_FUPD_SUMSQ_U) || no_m)) {
         // the sum only needs the gradient: 16 elements per thread, next step's loads in flight
-        if (bf) factored_sumsq_wide_kernel<bf16_tag><<<(int)grid, FUPD_THREADS, 0, cst>>>(L);
-        else factored_sumsq_wide_kernel<float><<<(int)grid, FUPD_THREADS, 0, cst>>>(L);
+        if (bf) launch_next(factored_sumsq_wide_kernel<bf16_tag>, (int)grid, FUPD_THREADS, 0, cst, L);
+        else launch_next(factored_sumsq_wide_kernel<float>, (int)grid, FUPD_THREADS, 0, cst, L);
         AF8_CUDA_TRY(cudaGetLastError());
         return AF8_OK;
     }
@@ -3098,11 +3112,11 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
         if (bf) {
             int64_t tg = std::min<int64_t>((int64_t)sm_count() * 3, LT.total_units);
             AF8_CUDA_TRY(cudaFuncSetAttribute(factored_apply_tile_kernel<bf16_tag, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fring_smem_bytes<bf16_tag>()));
-            factored_apply_tile_kernel<bf16_tag, 3><<<(int)tg, FUPD_THREADS, fring_smem_bytes<bf16_tag>(), cst>>>(LT);
+            launch_next(factored_apply_tile_kernel<bf16_tag, 3>, (int)tg, FUPD_THREADS, fring_smem_bytes<bf16_tag>(), cst, LT);
         } else {
             int64_t tg = std::min<int64_t>((int64_t)sm_count() * 2, LT.total_units);
             AF8_CUDA_TRY(cudaFuncSetAttribute(factored_apply_tile_kernel<float, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fring_smem_bytes<float>()));
-            factored_apply_tile_kernel<float, 2><<<(int)tg, FUPD_THREADS, fring_smem_bytes<float>(), cst>>>(LT);
+            launch_next(factored_apply_tile_kernel<float, 2>, (int)tg, FUPD_THREADS, fring_smem_bytes<float>(), cst, LT);
         }
         AF8_CUDA_TRY(cudaGetLastError());
         return AF8_OK;
@@ -3114,7 +3128,7 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
         if (total_chunks > INT32_MAX) return fail(AF8_ERR_UNSUPPORTED, "af8_factored_update: %lld chunks in one launch", (long long)total_chunks);
 #define AF8_LAUNCH_FWRITE(G, T, A) do { \
         AF8_CUDA_TRY(cudaFuncSetAttribute(factored_write_kernel<G, T, A>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)write_smem_bytes<sizeof_grad<G>(), T == 0 ? 4 : 2>())); \
-        factored_write_kernel<G, T, A><<<(int)total_chunks, WRITE_THREADS + 32, write_smem_bytes<sizeof_grad<G>(), T == 0 ? 4 : 2>(), cst>>>(L); } while (0)
+        launch_next(factored_write_kernel<G, T, A>, (int)total_chunks, WRITE_THREADS + 32, write_smem_bytes<sizeof_grad<G>(), T == 0 ? 4 : 2>(), cst, L); } while (0)
 #define AF8_LAUNCH_FWRITE_ANY(G, T) do { if (any) AF8_LAUNCH_FWRITE(G, T, true); else AF8_LAUNCH_FWRITE(G, T, false); } while (0)
         if (!bf) AF8_LAUNCH_FWRITE_ANY(float, 0);
         else if (pt == 0) AF8_LAUNCH_FWRITE_ANY(bf16_tag, 0);
@@ -3130,7 +3144,7 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
         grid = std::min<int64_t>((int64_t)sm_count() * (bf ? (any ? FLAT_ANY_CTAS : 3) : 2), total_chunks);
 #define AF8_LAUNCH_FLAT(G, T, A) do { \
         AF8_CUDA_TRY(cudaFuncSetAttribute(factored_apply_flat_kernel<G, T, A>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fring_smem_bytes<G, T>())); \
-        factored_apply_flat_kernel<G, T, A><<<(int)grid, FUPD_THREADS, fring_smem_bytes<G, T>(), cst>>>(L); } while (0)
+        launch_next(factored_apply_flat_kernel<G, T, A>, (int)grid, FUPD_THREADS, fring_smem_bytes<G, T>(), cst, L); } while (0)
 #define AF8_LAUNCH_FLAT_ANY(G, T) do { if (any) AF8_LAUNCH_FLAT(G, T, true); else AF8_LAUNCH_FLAT(G, T, false); } while (0)
         if (!bf) AF8_LAUNCH_FLAT_ANY(float, 0);
         else if (pt == 0) AF8_LAUNCH_FLAT_ANY(bf16_tag, 0);
@@ -3141,7 +3155,7 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
         AF8_CUDA_TRY(cudaGetLastError());
         return AF8_OK;
     }
-#define AF8_LAUNCH_FUPD(G, P, C, A, T) factored_update_vec_kernel<G, P, C, A, T><<<(int)grid, FUPD_THREADS, 0, cst>>>(L)
+#define AF8_LAUNCH_FUPD(G, P, C, A, T) launch_next(factored_update_vec_kernel<G, P, C, A, T>, (int)grid, FUPD_THREADS, 0, cst, L)
 #define AF8_LAUNCH_FUPD_PT(P, C, A) do { \
         if (bf && pt == 0) AF8_LAUNCH_FUPD(bf16_tag, P, C, A, 0); else if (bf && pt == 3) AF8_LAUNCH_FUPD(bf16_tag, P, C, A, 3); \
         else if (pt == 0) AF8_LAUNCH_FUPD(float, P, C, A, 0); else if (pt == 3) AF8_LAUNCH_FUPD(float, P, C, A, 3); \
@@ -3161,7 +3175,7 @@ extern "C" int af8_factored_update(const af8_factored_cfg *cfg, const af8_factor
 #undef AF8_LAUNCH_FUPD_SUM
 #undef AF8_LAUNCH_FUPD_PT
 #undef AF8_LAUNCH_FUPD
-    else factored_update_kernel<<<(int)grid, FUPD_THREADS, smem, static_cast<cudaStream_t>(stream)>>>(L, chunk);
+    else launch_next(factored_update_kernel, (int)grid, FUPD_THREADS, smem, static_cast<cudaStream_t>(stream), L, chunk);
     AF8_CUDA_TRY(cudaGetLastError());
     return AF8_OK;
 }

@@ -7,6 +7,7 @@
 #include "fullrank_fast.cuh"
 #include "fullrank_generic.cuh"
 #include "fullrank_stat.cuh"
+#include "launch.cuh"
 
 #include <atomic>
 
@@ -28,6 +29,7 @@ __global__ void __launch_bounds__(FINALIZE_THREADS)
 norm_finalize_kernel(const af8_norm_tensor *tensors, const void *block_sumsq, af8_dyn_scalars *dyn)
 {
     __shared__ double s_part[FINALIZE_THREADS / 32];
+    await_launches();
     const af8_norm_tensor T = tensors[blockIdx.x];
     const double *const p64 = static_cast<const double *>(block_sumsq) + T.first_block;
     const float *const p32 = static_cast<const float *>(block_sumsq) + T.first_block;
@@ -84,6 +86,7 @@ __global__ void __launch_bounds__(FINALIZE_THREADS)
 lag_scalars_kernel(const af8_lag_tensor *tensors, int phase, const void *block_sumsq, af8_dyn_scalars *dyn)
 {
     __shared__ double s_part[FINALIZE_THREADS / 32];
+    await_launches();
     const af8_lag_tensor T = tensors[blockIdx.x];
     const int tid = threadIdx.x;
     if (phase == 0) {
@@ -170,8 +173,7 @@ inline int launch_fast(const FullrankLaunch &L, cudaStream_t st)
     static ResidentCtas known;
     int rc = persistent_grid(kernel, FAST_THREADS, Ring::SMEM_BYTES, L.total_blocks, &grid, &known);
     if (rc) return rc;
-    kernel<<<grid, FAST_THREADS, Ring::SMEM_BYTES, st>>>(L);
-    AF8_CUDA_TRY(cudaGetLastError());
+    AF8_CUDA_TRY(launch_next(kernel, grid, FAST_THREADS, Ring::SMEM_BYTES, st, L));
     return AF8_OK;
 }
 
@@ -187,8 +189,7 @@ inline int launch_stat(const FullrankLaunch &L, cudaStream_t st)
     int64_t grid = (int64_t)per_sm * sm_count();
     const int64_t need = (L.total_blocks + warps_per_cta - 1) / warps_per_cta;
     if (grid > need) grid = need;
-    kernel<<<(int)grid, STAT_THREADS, 0, st>>>(L);
-    AF8_CUDA_TRY(cudaGetLastError());
+    AF8_CUDA_TRY(launch_next(kernel, (unsigned)grid, STAT_THREADS, 0, st, L));
     return AF8_OK;
 }
 
@@ -203,8 +204,7 @@ inline int launch_generic_threads(const FullrankLaunch &L, const GenericCfg &C, 
     static ResidentCtas known;                        // (of the plain form, whose shared memory is fixed)
     int rc = persistent_grid(kernel, THREADS, smem, L.total_blocks, &grid, plain ? &known : nullptr);
     if (rc) return rc;
-    kernel<<<grid, THREADS, smem, st>>>(L, C);
-    AF8_CUDA_TRY(cudaGetLastError());
+    AF8_CUDA_TRY(launch_next(kernel, grid, THREADS, smem, st, L, C));
     return AF8_OK;
 }
 
@@ -348,7 +348,8 @@ extern "C" int af8_fullrank_step(const af8_fullrank_cfg *cfg, const af8_fullrank
     if (host_tensors) {
         int rc = validate_fullrank_table(c, host_tensors, n_tensors, total_blocks);
         if (rc) return rc;
-        AF8_CUDA_TRY(cudaMemcpyAsync(dev_tensors, host_tensors, sizeof(af8_fullrank_tensor) * (size_t)n_tensors, cudaMemcpyHostToDevice, st));
+        rc = upload_table(dev_tensors, host_tensors, sizeof(af8_fullrank_tensor) * (size_t)n_tensors, st);
+        if (rc) return rc;
     }
 
     FullrankLaunch L;
@@ -385,9 +386,7 @@ extern "C" int af8_fullrank_upload(const af8_fullrank_cfg *cfg, const af8_fullra
     if (n_tensors <= 0 || cfg->block < 128 || cfg->block % 128 != 0) return fail(AF8_ERR_INVALID, "af8_fullrank_upload: bad sizes");
     int rc = validate_fullrank_table(*cfg, host_tensors, n_tensors, total_blocks);
     if (rc) return rc;
-    AF8_CUDA_TRY(cudaMemcpyAsync(dev_tensors, host_tensors, sizeof(af8_fullrank_tensor) * (size_t)n_tensors,
-                                 cudaMemcpyHostToDevice, static_cast<cudaStream_t>(stream)));
-    return AF8_OK;
+    return upload_table(dev_tensors, host_tensors, sizeof(af8_fullrank_tensor) * (size_t)n_tensors, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int af8_device_status(int32_t *status_out, void *stream)
@@ -455,8 +454,7 @@ extern "C" int af8_lag_scalars(const af8_lag_tensor *tensors, int32_t n_tensors,
     if (n_tensors <= 0) return fail(AF8_ERR_INVALID, "af8_lag_scalars: n_tensors must be positive");
     if (phase != 0 && phase != 1) return fail(AF8_ERR_INVALID, "af8_lag_scalars: phase must be 0 or 1");
     if (phase == 1 && !block_sumsq) return fail(AF8_ERR_INVALID, "af8_lag_scalars: phase 1 needs block_sumsq");
-    lag_scalars_kernel<<<n_tensors, FINALIZE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(tensors, phase, block_sumsq, dyn);
-    AF8_CUDA_TRY(cudaGetLastError());
+    AF8_CUDA_TRY(launch_next(lag_scalars_kernel, (unsigned)n_tensors, FINALIZE_THREADS, 0, static_cast<cudaStream_t>(stream), tensors, phase, block_sumsq, dyn));
     return AF8_OK;
 }
 
@@ -466,7 +464,6 @@ extern "C" int af8_norm_finalize(const af8_norm_tensor *tensors, int32_t n_tenso
     using namespace af8;
     if (!tensors || !block_sumsq || !dyn) return fail(AF8_ERR_INVALID, "af8_norm_finalize: null argument");
     if (n_tensors <= 0) return fail(AF8_ERR_INVALID, "af8_norm_finalize: n_tensors must be positive");
-    norm_finalize_kernel<<<n_tensors, FINALIZE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(tensors, block_sumsq, dyn);
-    AF8_CUDA_TRY(cudaGetLastError());
+    AF8_CUDA_TRY(launch_next(norm_finalize_kernel, (unsigned)n_tensors, FINALIZE_THREADS, 0, static_cast<cudaStream_t>(stream), tensors, block_sumsq, dyn));
     return AF8_OK;
 }

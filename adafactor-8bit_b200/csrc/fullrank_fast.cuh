@@ -62,6 +62,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "launch.cuh"
 
 namespace af8 {
 
@@ -106,7 +107,7 @@ __device__ __forceinline__ int find_tensor(const af8_fullrank_tensor *tensors, i
     int lo = 0, hi = n - 1;
     while (lo < hi) {
         int mid = (lo + hi + 1) >> 1;
-        if (__ldg(&tensors[mid].first_block) <= blk) lo = mid; else hi = mid - 1;
+        if (tensors[mid].first_block <= blk) lo = mid; else hi = mid - 1;
     }
     return lo;
 }
@@ -784,6 +785,7 @@ fullrank_fast_kernel(const FullrankLaunch L)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    await_launches();
 
     int cur_t = -1;
     int64_t cur_first = 0, cur_end = 0;      // block range of the current tensor
@@ -804,12 +806,12 @@ fullrank_fast_kernel(const FullrankLaunch L)
             if (t < 0) {
                 t = find_tensor(L.tensors, L.n_tensors, blk);
             } else {
-                while (t + 1 < L.n_tensors && __ldg(&L.tensors[t + 1].first_block) <= blk) ++t;
+                while (t + 1 < L.n_tensors && L.tensors[t + 1].first_block <= blk) ++t;
             }
             __syncthreads();
             if (tid < (int)(sizeof(af8_fullrank_tensor) / 4))
                 reinterpret_cast<uint32_t *>(&sT)[tid] =
-                    __ldg(reinterpret_cast<const uint32_t *>(L.tensors + t) + tid);
+                    reinterpret_cast<const uint32_t *>(L.tensors + t)[tid];
             __syncthreads();
             if (tid == 0) {
                 StepScalars S;

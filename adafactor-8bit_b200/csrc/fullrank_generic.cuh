@@ -112,20 +112,21 @@ fullrank_generic_kernel(const FullrankLaunch L, const GenericCfg C)
     const float qm1 = (C.v_fmt == AF8_V_AL16) ? 65534.0f : 254.0f;
     const int qmax = (C.v_fmt == AF8_V_AL16) ? 65535 : 255;
     int cur_t = -1;
-    if (v_quant) load_codec_tables(s_codec);
+    if (v_quant) load_codec_tables(s_codec);              // (constants)
+    await_launches();
 
     for (int64_t blk = blockIdx.x; blk < L.total_blocks; blk += gridDim.x) {
         int t = cur_t;
         if (t < 0) {
             t = find_tensor(L.tensors, L.n_tensors, blk);
         } else {
-            while (t + 1 < L.n_tensors && __ldg(&L.tensors[t + 1].first_block) <= blk) ++t;
+            while (t + 1 < L.n_tensors && L.tensors[t + 1].first_block <= blk) ++t;
         }
         __syncthreads();
         if (t != cur_t) {
             if (tid < (int)(sizeof(af8_fullrank_tensor) / 4))
                 reinterpret_cast<uint32_t *>(&sT)[tid] =
-                    __ldg(reinterpret_cast<const uint32_t *>(L.tensors + t) + tid);
+                    reinterpret_cast<const uint32_t *>(L.tensors + t)[tid];
             cur_t = t;
         }
         __syncthreads();

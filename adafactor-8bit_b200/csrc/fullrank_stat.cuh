@@ -108,6 +108,7 @@ fullrank_stat_kernel(const FullrankLaunch L)
         if (threadIdx.x < 32) s_exp2[threadIdx.x] = c_exp2_tab[threadIdx.x];
         __syncthreads();
     }
+    await_launches();
     float *const dec = s_dec[threadIdx.x >> 5];
     const int64_t warps = (int64_t)gridDim.x * (STAT_THREADS / 32);
     const int64_t w0 = (int64_t)blockIdx.x * (STAT_THREADS / 32) + (threadIdx.x >> 5);
@@ -123,16 +124,16 @@ fullrank_stat_kernel(const FullrankLaunch L)
     for (int64_t blk = w0; blk < L.total_blocks;) {
         // the next tensor (uniform over the warp)
         if (t < 0) t = find_tensor(L.tensors, L.n_tensors, blk);
-        else while (t + 1 < L.n_tensors && __ldg(&L.tensors[t + 1].first_block) <= blk) ++t;
+        else while (t + 1 < L.n_tensors && L.tensors[t + 1].first_block <= blk) ++t;
         const af8_fullrank_tensor *T = L.tensors + t;
-        numel = __ldg(&T->numel);
-        cur_first = __ldg(&T->first_block);
+        numel = T->numel;
+        cur_first = T->first_block;
         cur_end = cur_first + (numel + FAST_VBLOCK - 1) / FAST_VBLOCK;
         grad = T->grad;
         mq = T->m_q; vq = static_cast<const uint8_t *>(T->v_q);
         m_scale = T->m_scale; v_scale = T->v_scale; v_min_log = T->v_min_log;
-        v_w = __ldg(&T->v_w); m_w = MF == AF8_M_NONE ? 0.0f : __ldg(&T->m_w);
-        eps_d = __ldg(&T->eps_denom); eps_g = __ldg(&T->eps_gradsq);
+        v_w = T->v_w; m_w = MF == AF8_M_NONE ? 0.0f : T->m_w;
+        eps_d = T->eps_denom; eps_g = T->eps_gradsq;
         small_w = fabsf(v_w) < 0.5f && fabsf(m_w) < 0.5f;
 
         // The blocks of this warp in this tensor, in one of two copies of the loop (see ROOT_EXACT; TinyLlama-1.1B with UF8/AL8:

@@ -8,6 +8,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "launch.cuh"
 
 namespace af8 {
 
@@ -25,7 +26,7 @@ __device__ __forceinline__ int find_scale_tensor(const af8_scale_tensor *tensors
     int lo = 0, hi = n - 1;
     while (lo < hi) {
         int mid = (lo + hi + 1) >> 1;
-        if (__ldg(&tensors[mid].first_chunk) <= chunk) lo = mid; else hi = mid - 1;
+        if (tensors[mid].first_chunk <= chunk) lo = mid; else hi = mid - 1;
     }
     return lo;
 }
@@ -36,6 +37,7 @@ param_sumsq_kernel(const ScaleLaunch L)
 {
     __shared__ float s_red[8];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    await_launches();
     for (int64_t chunk = blockIdx.x; chunk < L.total_chunks; chunk += gridDim.x) {
         const int t = find_scale_tensor(L.tensors, L.n_tensors, chunk);
         const void *p = L.tensors[t].param;
@@ -88,6 +90,7 @@ param_scale_finalize_kernel(const af8_scale_tensor *tensors, const float *block_
                             uint8_t *table, int64_t stride, int64_t alpha_off, int64_t decay_off)
 {
     __shared__ double s_part[32];
+    await_launches();
     const af8_scale_tensor T = tensors[blockIdx.x];
     const int64_t n_chunks = (T.numel + SCALE_CHUNK - 1) / SCALE_CHUNK;
     const float *const ps = block_sumsq + T.first_chunk;
@@ -133,12 +136,12 @@ extern "C" int af8_param_sumsq(const af8_scale_tensor *host_tensors, af8_scale_t
         next += (t.numel + SCALE_CHUNK - 1) / SCALE_CHUNK;
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    AF8_CUDA_TRY(cudaMemcpyAsync(dev_tensors, host_tensors, sizeof(af8_scale_tensor) * (size_t)n_tensors, cudaMemcpyHostToDevice, st));
+    const int rc = upload_table(dev_tensors, host_tensors, sizeof(af8_scale_tensor) * (size_t)n_tensors, st);
+    if (rc) return rc;
     ScaleLaunch L{dev_tensors, chunk_sumsq, next, n_tensors};
     int64_t grid = (int64_t)sm_count() * 8;
     if (grid > next) grid = next;
-    param_sumsq_kernel<<<(int)grid, 256, 0, st>>>(L);
-    AF8_CUDA_TRY(cudaGetLastError());
+    AF8_CUDA_TRY(launch_next(param_sumsq_kernel, (unsigned)grid, 256, 0, st, L));
     return AF8_OK;
 }
 
@@ -150,9 +153,8 @@ extern "C" int af8_param_scale_finish(const af8_scale_tensor *dev_tensors, int32
     if (!dev_tensors || !chunk_sumsq || !dev_table) return fail(AF8_ERR_INVALID, "af8_param_scale_finish: null argument");
     if (n_tensors <= 0) return fail(AF8_ERR_INVALID, "af8_param_scale_finish: n_tensors must be positive");
     if (!param_scale_layout_ok(table_stride, alpha_offset, decay_offset)) return fail(AF8_ERR_INVALID, "af8_param_scale_finish: bad table layout");
-    param_scale_finalize_kernel<<<n_tensors, 1024, 0, static_cast<cudaStream_t>(stream)>>>(
-        dev_tensors, chunk_sumsq, static_cast<uint8_t *>(dev_table), table_stride, alpha_offset, decay_offset);
-    AF8_CUDA_TRY(cudaGetLastError());
+    AF8_CUDA_TRY(launch_next(param_scale_finalize_kernel, (unsigned)n_tensors, 1024, 0, static_cast<cudaStream_t>(stream),
+                             dev_tensors, chunk_sumsq, static_cast<uint8_t *>(dev_table), table_stride, alpha_offset, decay_offset));
     return AF8_OK;
 }
 

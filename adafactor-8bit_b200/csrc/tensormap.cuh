@@ -26,7 +26,7 @@ inline EncodeTiledFn encode_tiled_fn()
     return fn;
 }
 
-// Orders the uses of a tensor map by the calling thread behind the host's copy that wrote it: a map that lives in
+// Orders the uses of a tensor map by the calling thread behind the copy that wrote it: a map that lives in
 // global memory is read through a proxy of its own, which may still hold what was at that address before.
 __device__ __forceinline__ void tensormap_acquire(const CUtensorMap *map)
 {

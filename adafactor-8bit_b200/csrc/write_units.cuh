@@ -8,6 +8,7 @@
 // of this.)  A thread owns four groups of four elements, 512 apart, so that every access of a warp is one contiguous run.
 #pragma once
 
+#include "launch.cuh"
 #include "schedule.cuh"
 
 namespace af8 {
@@ -63,6 +64,7 @@ __device__ __forceinline__ void write_units(const Tensors &tensors, WriteShared<
         unit_start(sh.queue);
     }
     __syncthreads();
+    await_launches();
 
     if (tid >= WRITE_THREADS) {
         if (tid != WRITE_THREADS) return;

@@ -1,0 +1,75 @@
+"""Uploads of launch tables from any host memory, and calls that are captured into a graph."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+import cases
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(70, 264), (4100,), (3, 2048), (40, 1000)]
+
+
+def make():
+    from adafactor8bit import Adafactor8Bit
+    gen = torch.Generator().manual_seed(3)
+    params = [torch.nn.Parameter((torch.randn(s, generator=gen) * 0.02).cuda()) for s in SHAPES]
+    for p in params:
+        p.grad = (torch.randn(p.shape, generator=gen) * 1e-3).cuda()
+    opt = Adafactor8Bit(params, **dict(cases.CASES["adamw_uf8_al8"]["hp"], min_8bit_size=1))
+    opt.step()
+    plan, = opt._plans.values()
+    ring = plan.h_table
+    torch.cuda.synchronize()
+    return params, opt, plan, np.array(ring.views[ring.i])       # (the launch table of that step)
+
+
+def again(plan, address, stream):
+    from adafactor8bit import _native as N
+    N.check(N.lib().af8_fullrank_step(ctypes.byref(plan.cfg), address, plan.d_table.data_ptr(), plan.n, plan.total_blocks,
+                                      plan.d_dyn.data_ptr(), None, stream.cuda_stream), "af8_fullrank_step")
+
+
+def result(params, opt):
+    torch.cuda.synchronize()
+    return [p.detach().cpu().view(torch.int32) for p in params] + [opt.state[p][k].cpu() for p in params for k in ("m_q", "variance_q")]
+
+
+def test_a_table_comes_from_any_host_memory():
+    """The same second step from a pinned table (copied by a kernel), a pinned one off the 16-byte units, and a pageable one."""
+    out = []
+    for kind in ("pinned", "unaligned", "pageable"):
+        params, opt, plan, table = make()
+        plan.d_table.zero_()
+        room = torch.empty(table.size + 64, dtype=torch.uint8, pin_memory=kind != "pageable")
+        off = -room.data_ptr() % 16 + (8 if kind == "unaligned" else 0)
+        room.numpy()[off:off + table.size] = table
+        again(plan, room.data_ptr() + off, torch.cuda.current_stream())
+        out.append(result(params, opt))
+    for other in out[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(out[0], other))
+
+
+def test_a_captured_step_replays():
+    """Two steps captured into a graph, upload included, are the two steps launched one by one."""
+    out = []
+    for graph in (False, True):
+        params, opt, plan, table = make()
+        room = torch.empty(table.size, dtype=torch.uint8, pin_memory=True)
+        room.numpy()[:] = table
+        stream = torch.cuda.Stream()
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            if graph:
+                g = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(g, stream=stream):
+                    again(plan, room.data_ptr(), stream)
+                    again(plan, room.data_ptr(), stream)
+                g.replay()
+            else:
+                again(plan, room.data_ptr(), stream)
+                again(plan, room.data_ptr(), stream)
+        out.append(result(params, opt))
+    assert all(torch.equal(a, b) for a, b in zip(*out))
