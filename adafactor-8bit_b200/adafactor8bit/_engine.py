@@ -103,6 +103,17 @@ def dynamic_map(total_bits):
 
 _QMAP_DEVICES = set()
 
+_STREAMS = {}         # device index -> the stream object handed out last
+
+
+def stream_of(device):
+    """torch.cuda.current_stream(device), whose making costs a small step as much as a launch: the object of the last call while the
+    device's current stream is the same."""
+    s = _STREAMS.get(device.index)
+    if s is None or s.cuda_stream != torch._C._cuda_getCurrentRawStream(device.index):
+        s = _STREAMS[device.index] = torch.cuda.current_stream(device)
+    return s
+
 # When set to a list, every kernel launch appends (name, parameters covered,
 # start event, end event), recorded on the launch stream.  Used by bench.py to
 # time individual kernels inside its timed region; None disables it.
@@ -206,7 +217,7 @@ class _PinnedRing:
     def next(self):
         self.i = (self.i + 1) % len(self.bufs)
         ev = self.events[self.i]
-        if ev is not None:
+        if ev is not None and not ev.query():
             ev.synchronize()
         return self.bufs[self.i]
 
@@ -216,6 +227,11 @@ class _PinnedRing:
         if t is None:
             t = self.tables[self.i, dtype.itemsize, n] = self.views[self.i][: n * dtype.itemsize].view(dtype)
         return t
+
+    def fill(self, table):
+        """Copy a table into the current buffer, as bytes: records are copied field by field (14 of them in 4 us)."""
+        raw = table.reshape(-1).view(np.uint8)
+        self.views[self.i][: raw.size] = raw
 
     def mark(self, stream):
         ev = self.events[self.i]
@@ -294,6 +310,8 @@ class FullrankPlan:
 
         self.d_table = torch.empty(n * N.FULLRANK_TENSOR.itemsize, dtype=torch.uint8, device=self.device)
         self.d_dyn = torch.zeros(n * N.DYN_SCALARS.itemsize, dtype=torch.uint8, device=self.device)
+        self._cfg_ref = ctypes.byref(self.cfg)
+        self._table_args = (self.d_table.data_ptr(), n, self.total_blocks, self.d_dyn.data_ptr())
         self._norm_tables = {}       # (pre_div_mode, exchange) -> (inputs, limiter pointers, device table) of norm_finalize
         self.d_sumsq = None
         self.h_table = _PinnedRing(n * N.FULLRANK_TENSOR.itemsize)
@@ -352,7 +370,7 @@ class FullrankPlan:
         _update_scalars(self._static, self._last, scalars, ("decay", "alpha", "v_w", "v_keep", "v_eps_add", "m_w", "eps_gradsq", "eps_denom", "eps_sq"))
         buf = self.h_table.next()
         table = self.h_table.table(N.FULLRANK_TENSOR, self.n)
-        table[:] = self._static
+        self.h_table.fill(self._static)
         table["grad"] = [g.data_ptr() for g in grads]
         if "sr_base" in scalars:
             table["sr_base"] = scalars["sr_base"]
@@ -384,10 +402,10 @@ class FullrankPlan:
             e1 = torch.cuda.Event(enable_timing=True)
             e0.record(stream)
         rc = N.lib().af8_fullrank_step(
-            ctypes.byref(self.cfg), host_buf.data_ptr() if host_buf is not None else None,
-            self.d_table.data_ptr(), self.n, self.total_blocks, self.d_dyn.data_ptr(),
+            self._cfg_ref, host_buf.data_ptr() if host_buf is not None else None, *self._table_args,
             self.d_sumsq.data_ptr() if self.d_sumsq is not None else None, stream.cuda_stream)
-        N.check(rc, "af8_fullrank_step")
+        if rc != N.OK:
+            N.check(rc, "af8_fullrank_step")
         if log is not None:
             e1.record(stream)
             log.append((self.kernel_name(mode), self.total_numel, e0, e1))
@@ -407,20 +425,12 @@ class FullrankPlan:
     def _scale_table(self, buf, scale, stream):
         """Upload the launch table and fill the host table of the parameter-RMS passes
         (scale_parameter=True, optimizer.py:850-853)."""
-        chunk = N.lib().af8_scale_chunk()
-        nchunks = (self.numel + chunk - 1) // chunk
-        if self.h_scale is None:
-            self.h_scale = _PinnedRing(self.n * N.SCALE_TENSOR.itemsize)
-            self.d_scale = torch.empty(self.n * N.SCALE_TENSOR.itemsize, dtype=torch.uint8, device=self.device)
-            self.d_chunks = torch.empty(int(nchunks.sum()), dtype=torch.float32, device=self.device)
         rc = N.lib().af8_fullrank_upload(ctypes.byref(self.cfg), buf.data_ptr(), self.d_table.data_ptr(), self.n,
                                          self.total_blocks, stream.cuda_stream)
         N.check(rc, "af8_fullrank_upload")
         self.h_table.mark(stream)
-        hb = self.h_scale.next()
-        t = hb.numpy()[: self.n * N.SCALE_TENSOR.itemsize].view(N.SCALE_TENSOR)
-        fill_scale_table(t, self.params, self.numel, self.full_numel, nchunks, self.cfg.param_dtype, scale)
-        self._scale_first, self._scale_count = t["first_chunk"].copy(), nchunks
+        hb, t = plan_scale_table(self, scale)
+        self._scale_first, self._scale_count = self.scale_static["first_chunk"], self.scale_chunks
         return hb, t
 
     def _param_scale(self, buf, scale, stream, x=None):
@@ -483,7 +493,7 @@ class FullrankPlan:
         scale: per-tensor inputs of af8_param_scale when alpha depends on the
         parameter RMS; the table's alpha / decay are then produced on the device.
         lag: lag_norm=True; the momentum-only rule keeps its exact passes."""
-        stream = stream or torch.cuda.current_stream(self.device)
+        stream = stream or stream_of(self.device)
         buf, table = self.fill_table(grads, scalars)
         self._alpha_on_device = scale is not None
         mom_only = bool(self.cfg.momentum_only)
@@ -613,14 +623,35 @@ def fira_state_pointers(plan):
 
 def fill_scale_table(t, params, numel, full_numel, nchunks, param_dtype, scale):
     """Fill an af8_scale_tensor table (host view `t`)."""
-    t["param"] = [p.data_ptr() for p in params]
     t["numel"] = numel
     t["first_chunk"] = np.concatenate([[0], np.cumsum(nchunks)[:-1]])
     t["sqrt_n"] = np.sqrt(full_numel.astype(np.float64)).astype(np.float32)
     t["param_dtype"] = param_dtype
     t["total"] = 0
+    _scale_step_fields(t, params, scale)
+
+
+def _scale_step_fields(t, params, scale):
+    t["param"] = [p.data_ptr() for p in params]
     for k in ("rho", "eps2", "bc", "weight_decay", "bc_mode", "scale_weight_decay"):
         t[k] = scale[k]
+
+
+def plan_scale_table(plan, scale):
+    """This step's af8_scale_tensor table of a full-rank or factored plan, in the plan's current pinned buffer -> (buffer, table).  Sizes
+    and counts stay in a template."""
+    if plan.h_scale is None:
+        chunk = N.lib().af8_scale_chunk()
+        plan.scale_chunks = (plan.numel + chunk - 1) // chunk
+        plan.h_scale = _PinnedRing(plan.n * N.SCALE_TENSOR.itemsize)
+        plan.d_scale = torch.empty(plan.n * N.SCALE_TENSOR.itemsize, dtype=torch.uint8, device=plan.device)
+        plan.d_chunks = torch.empty(int(plan.scale_chunks.sum()), dtype=torch.float32, device=plan.device)
+        plan.scale_static = np.zeros(plan.n, dtype=N.SCALE_TENSOR)
+        fill_scale_table(plan.scale_static, plan.params, plan.numel, plan.full_numel, plan.scale_chunks, plan.cfg.param_dtype, scale)
+    _scale_step_fields(plan.scale_static, plan.params, scale)
+    hb = plan.h_scale.next()
+    plan.h_scale.fill(plan.scale_static)
+    return hb, plan.h_scale.table(N.SCALE_TENSOR, plan.n)
 
 
 def _small_state_fields(row, st, prefix, fmt, block):
@@ -870,7 +901,7 @@ class FactoredPlan:
     def stages(self, grads, scalars, d=0.0, fira=False, fira_margin=0.01, scale=None, stream=None, lag=False):
         """The step as a generator (optimizer.py:2202-2552) that yields at its factored_exchanges(...)
         exchange points, like FullrankPlan.stages; the last segment writes the parameters."""
-        stream = stream or torch.cuda.current_stream(self.device)
+        stream = stream or stream_of(self.device)
         sig = self._pointer_signature()
         if self._static is None or sig != self._ptr_sig:
             self._static = self._static_fields()
@@ -879,7 +910,7 @@ class FactoredPlan:
         _update_scalars(self._static, self._last, scalars, ("decay", "alpha", "v_w", "m_w", "c_w", "eps1", "eps_came"))
         buf = self.h_table.next()
         tables = self.h_table.table(N.FACTORED_TENSOR, self.n_tables * self.n).reshape(self.n_tables, self.n)
-        tables[:] = self._static
+        self.h_table.fill(self._static)
         table = tables[0]
         table["grad"] = [g.data_ptr() for g in grads]
         if self._any_rows:
@@ -942,15 +973,7 @@ class FactoredPlan:
             self._update(N.FUPD_APPLY, False, stream)
 
     def _param_scale(self, scale, stream, x=None):
-        chunk = N.lib().af8_scale_chunk()
-        nchunks = (self.numel + chunk - 1) // chunk
-        if self.h_scale is None:
-            self.h_scale = _PinnedRing(self.n * N.SCALE_TENSOR.itemsize)
-            self.d_scale = torch.empty(self.n * N.SCALE_TENSOR.itemsize, dtype=torch.uint8, device=self.device)
-            self.d_chunks = torch.empty(int(nchunks.sum()), dtype=torch.float32, device=self.device)
-        hb = self.h_scale.next()
-        t = hb.numpy()[: self.n * N.SCALE_TENSOR.itemsize].view(N.SCALE_TENSOR)
-        fill_scale_table(t, self.params, self.numel, self.full_numel, nchunks, self.cfg.param_dtype, scale)
+        hb, t = plan_scale_table(self, scale)
         if x is not None:
             for i in self.cut:
                 t["total"][i] = self.pieces[i].slots[x].data_ptr()
@@ -961,7 +984,7 @@ class FactoredPlan:
         if x is not None:
             first = t["first_chunk"]
             for i in self.cut:
-                _add_to_slot(self.pieces[i].slots[x], 0, self.d_chunks[int(first[i]):int(first[i]) + int(nchunks[i])])
+                _add_to_slot(self.pieces[i].slots[x], 0, self.d_chunks[int(first[i]):int(first[i]) + int(self.scale_chunks[i])])
 
     def _param_finish(self, stream):
         N.check(N.lib().af8_param_scale_finish(
@@ -1114,7 +1137,7 @@ class ApolloPlan:
         (scale_parameter=True); alpha and the decay factor then come from the device.
         versions: one hashable per tensor that changes whenever its projection matrix does; while it stays
         the same the bf16 planes of the matrix are kept in the workspace instead of being rebuilt."""
-        stream = stream or torch.cuda.current_stream(self.device)
+        stream = stream or stream_of(self.device)
         if params is not None:
             self.params = list(params)
         lib = N.lib()

@@ -133,7 +133,15 @@ lag_scalars_kernel(const af8_lag_tensor *tensors, int phase, const void *block_s
 // ---------------------------------------------------------------------------
 // Resident CTAs of a kernel launched with fixed threads and shared memory, by device: asked once (the question costs a small step's
 // launch more than the launch itself).
-struct ResidentCtas { std::atomic<int> of_device[64]; };
+struct ResidentCtas {
+    std::atomic<int> of_device[64];
+    // whether they are known for the current device (and the kernel's attributes set there)
+    bool asked() const
+    {
+        int dev = -1;
+        return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && of_device[dev].load(std::memory_order_relaxed) > 0;
+    }
+};
 template <typename K>
 inline int resident_ctas(K kernel, int threads, size_t smem, ResidentCtas *known, int *per_sm)
 {
@@ -164,13 +172,15 @@ inline int launch_fast(const FullrankLaunch &L, cudaStream_t st)
 {
     using Ring = FastRing<GradT, ParamT, VB, MF>;
     auto kernel = fullrank_fast_kernel<GradT, ParamT, VB, MF, SR, LAG, ROOT>;
-    // the ring lives in dynamic shared memory (up to 44 KB per CTA): opt in and ask for the large
-    // shared-memory carve-out
-    AF8_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring::SMEM_BYTES));
-    AF8_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                      (int)cudaSharedmemCarveoutMaxShared));
     int grid = 0;
     static ResidentCtas known;
+    if (!known.asked()) {
+        // the ring lives in dynamic shared memory (up to 44 KB per CTA): opt in and ask for the large
+        // shared-memory carve-out
+        AF8_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring::SMEM_BYTES));
+        AF8_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                          (int)cudaSharedmemCarveoutMaxShared));
+    }
     int rc = persistent_grid(kernel, FAST_THREADS, Ring::SMEM_BYTES, L.total_blocks, &grid, &known);
     if (rc) return rc;
     AF8_CUDA_TRY(launch_next(kernel, grid, FAST_THREADS, Ring::SMEM_BYTES, st, L));
