@@ -22,7 +22,7 @@ import numpy as np
 import torch
 from torch import Tensor
 from torch.optim import Optimizer
-from torch.optim import optimizer as _torch_optimizer
+from torch.optim.optimizer import _global_optimizer_post_hooks, _global_optimizer_pre_hooks
 
 from . import _native as N
 from ._engine import ApolloPlan, FactoredPlan, FullrankPlan, factored_exchanges, fullrank_exchanges, sr_base
@@ -48,7 +48,7 @@ def _step_hooks(func):
     """torch.optim's wrapper around step, which runs the step hooks inside a range for the profiler, where there are hooks or a profiler
     records; the step itself otherwise (the wrapper costs 14 us, a sixth of a small step)."""
     full = Optimizer.profile_hook_step(func)
-    before, after = _torch_optimizer._global_optimizer_pre_hooks, _torch_optimizer._global_optimizer_post_hooks
+    before, after = _global_optimizer_pre_hooks, _global_optimizer_post_hooks
 
     @functools.wraps(func)
     def wrapper(*args, **kwargs):

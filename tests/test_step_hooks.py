@@ -1,6 +1,7 @@
 """The step's own wrapper: hooks run, and a profiler sees the step, as with torch.optim's."""
 import pytest
 import torch
+from torch.optim.optimizer import register_optimizer_step_post_hook, register_optimizer_step_pre_hook
 
 from adafactor8bit import Adafactor8Bit
 
@@ -22,8 +23,7 @@ def test_hooks_run_around_the_step(kind):
     if kind == "own":
         handles = [opt.register_step_pre_hook(before), opt.register_step_post_hook(after)]
     else:
-        handles = [torch.optim.optimizer.register_optimizer_step_pre_hook(before),
-                   torch.optim.optimizer.register_optimizer_step_post_hook(after)]
+        handles = [register_optimizer_step_pre_hook(before), register_optimizer_step_post_hook(after)]
     opt.step(grad_ready=[None])
     for h in handles:
         h.remove()
