@@ -348,68 +348,98 @@ __device__ __forceinline__ int find_finish_tensor(const af8_apollo_finish_tensor
     return lo;
 }
 
-// unit = 8 channels of one tensor.  Right case (a channel is a row of rank contiguous values): one
-// warp per channel.  Left case (a channel is a column of the rank x cols array): the 8 channels of the
-// unit are 32 contiguous bytes of every row, so 8 lanes take one row and the 32 groups of a CTA walk
-// the rows together; the sums of a channel are then added over the groups in a fixed order.
-__global__ void __launch_bounds__(256)
+// unit = 8 channels of one tensor.  A CTA takes a run of neighbouring units, up to SCALES_UNITS of one tensor at a time.  Right case (a
+// channel is a row of rank contiguous values): one warp per channel, a channel of each unit after another.  Left case (a channel is a column of
+// the rank x cols array): a lane per channel, so that a warp reads 128 contiguous bytes of a row, and the 8 warps walk the rows together; the
+// sums of a channel are then added over the warps in a fixed order.
+// What a unit (16 KB at rank 256) waits for decides: a run needs one search of the table and one sum over the CTA with one atomic per
+// tensor, where each unit had them; rows come in 128-bit loads, lines whole where a column unit read 32 bytes of each, and the square
+// roots and divisions of a step are made by as many threads as it has channels: 61 M projected elements 187 -> 110 us.
+constexpr int SCALES_UNITS = 4;
+__global__ void __launch_bounds__(256, 8)
 apollo_scales_multi_kernel(const af8_apollo_finish_tensor *T, int n, int64_t total_units)
 {
+    __shared__ double s_nu[2][8][SCALES_UNITS * 8], s_ng[2][8][SCALES_UNITS * 8];       // by parity of the step, [warp][channel]
     __shared__ double s_part[8];
-    __shared__ double s_nu[8][8], s_ng[8][8];        // left case: [warp][channel of the unit]
-    await_launches();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    for (int64_t unit = blockIdx.x; unit < total_units; unit += gridDim.x) {
-        const af8_apollo_finish_tensor *t = T + find_finish_tensor(T, n, unit);
+    const int64_t steps = (total_units + SCALES_UNITS - 1) / SCALES_UNITS;
+    int64_t unit = steps * blockIdx.x / gridDim.x * SCALES_UNITS;
+    const int64_t last = steps * (blockIdx.x + 1) / gridDim.x * SCALES_UNITS, end = last < total_units ? last : total_units;
+    int parity = 0;
+    await_launches();
+    while (unit < end) {
+        const af8_apollo_finish_tensor *const t = T + find_finish_tensor(T, n, unit);
         const int64_t rows = t->rows, cols = t->cols, rank = t->rank;
         const bool right = rows >= cols;
         const int64_t nch = right ? rows : cols;
-        const int64_t ch0 = (unit - t->first_unit) * 8;
-        const int64_t ch = ch0 + warp;
-        const float *upd = t->upd, *g_low = t->g_low;
+        const int64_t stop_t = t->first_unit + (nch + 7) / 8, stop = stop_t < end ? stop_t : end;
+        const float *const upd = t->upd, *const g_low = t->g_low;
+        const bool wide = (rank & 3) == 0 && ((reinterpret_cast<uintptr_t>(upd) | reinterpret_cast<uintptr_t>(g_low)) & 15) == 0;
         double local = 0.0;
-        double nu = 0.0, ng = 0.0;
-        if (right) {
-            if (ch < nch) {
-                for (int64_t k = lane; k < rank; k += 32) {
-                    const int64_t idx = ch * rank + k;
-                    const float u = upd[idx], g = g_low[idx];
-                    nu += (double)__fmul_rn(u, u);
-                    ng += (double)__fmul_rn(g, g);
-                }
-            }
+        int64_t ch0 = (unit - t->first_unit) * 8;
+        while (unit < stop) {
+            const int m = (int)(stop - unit < SCALES_UNITS ? stop - unit : SCALES_UNITS);
+            double nu = 0.0, ng = 0.0;               // of channel ch (lane j < m: channel warp * m + j of the step)
+            const int64_t ch = ch0 + warp * m + lane;
+            if (right) {
+                for (int j = 0; j < m; ++j) {
+                    const int64_t c = ch0 + warp * m + j;
+                    double u2 = 0.0, g2 = 0.0;
+                    if (c < nch && wide) {
+                        const float4 *const u4 = reinterpret_cast<const float4 *>(upd + c * rank);
+                        const float4 *const g4 = reinterpret_cast<const float4 *>(g_low + c * rank);
+#pragma unroll 2
+                        for (int64_t k = lane; k < (rank >> 2); k += 32) {
+                            const float4 u = u4[k], g = g4[k];
+                            u2 += ((double)__fmul_rn(u.x, u.x) + (double)__fmul_rn(u.y, u.y)) + ((double)__fmul_rn(u.z, u.z) + (double)__fmul_rn(u.w, u.w));
+                            g2 += ((double)__fmul_rn(g.x, g.x) + (double)__fmul_rn(g.y, g.y)) + ((double)__fmul_rn(g.z, g.z) + (double)__fmul_rn(g.w, g.w));
+                        }
+                    } else if (c < nch) {
+                        for (int64_t k = lane; k < rank; k += 32) {
+                            const float u = upd[c * rank + k], g = g_low[c * rank + k];
+                            u2 += (double)__fmul_rn(u, u);
+                            g2 += (double)__fmul_rn(g, g);
+                        }
+                    }
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                nu += __shfl_xor_sync(0xffffffffu, nu, o);
-                ng += __shfl_xor_sync(0xffffffffu, ng, o);
-            }
-        } else {
-            const int64_t c = ch0 + (lane & 7);
-            if (c < nch) {
-                for (int64_t k = warp * 4 + (lane >> 3); k < rank; k += 32) {
-                    const int64_t idx = k * nch + c;
-                    const float u = upd[idx], g = g_low[idx];
-                    nu += (double)__fmul_rn(u, u);
-                    ng += (double)__fmul_rn(g, g);
+                    for (int o = 16; o > 0; o >>= 1) {
+                        u2 += __shfl_xor_sync(0xffffffffu, u2, o);
+                        g2 += __shfl_xor_sync(0xffffffffu, g2, o);
+                    }
+                    if (lane == j) { nu = u2; ng = g2; }
                 }
-            }
-            nu += __shfl_xor_sync(0xffffffffu, nu, 8);  ng += __shfl_xor_sync(0xffffffffu, ng, 8);
-            nu += __shfl_xor_sync(0xffffffffu, nu, 16); ng += __shfl_xor_sync(0xffffffffu, ng, 16);
-            if (lane < 8) { s_nu[warp][lane] = nu; s_ng[warp][lane] = ng; }
-            __syncthreads();
-            nu = ng = 0.0;
-            if (lane == 0) {
+            } else {
+                const int64_t c = ch0 + lane;
+                double u2 = 0.0, g2 = 0.0;
+                if (lane < m * 8 && c < nch) {
+#pragma unroll 4
+                    for (int64_t k = warp; k < rank; k += 8) {
+                        const float u = upd[k * nch + c], g = g_low[k * nch + c];
+                        u2 += (double)__fmul_rn(u, u);
+                        g2 += (double)__fmul_rn(g, g);
+                    }
+                }
+                s_nu[parity][warp][lane] = u2;
+                s_ng[parity][warp][lane] = g2;
+                __syncthreads();                     // (the next step writes the other half)
+                if (lane < m) {
 #pragma unroll
-                for (int w = 0; w < 8; ++w) { nu += s_nu[w][warp]; ng += s_ng[w][warp]; }
+                    for (int w = 0; w < 8; ++w) { nu += s_nu[parity][w][warp * m + lane]; ng += s_ng[parity][w][warp * m + lane]; }
+                }
+                parity ^= 1;
             }
+            if (lane < m && ch < nch) {
+                float s = __fdiv_rn(__double2float_rn(sqrt(nu)), __fadd_rn(__double2float_rn(sqrt(ng)), 1e-8f));   // optimizer.py:2964
+                if (t->in.scale_front) s = __fmul_rn(s, t->in.sqrt_scale);                                       // optimizer.py:2969-2971
+                t->sf[ch] = s;
+                const float nG = __double2float_rn(sqrt(t->chan_g2[ch]));
+                local += (double)__fmul_rn(__fmul_rn(nG, nG), __fmul_rn(s, s));                                  // optimizer.py:2975-2982
+            }
+            unit += m;
+            ch0 += m * 8;
         }
-        if (lane == 0 && ch < nch) {
-            float s = __fdiv_rn(__double2float_rn(sqrt(nu)), __fadd_rn(__double2float_rn(sqrt(ng)), 1e-8f));   // optimizer.py:2964
-            if (t->in.scale_front) s = __fmul_rn(s, t->in.sqrt_scale);                       // optimizer.py:2969-2971
-            t->sf[ch] = s;
-            const float nG = __double2float_rn(sqrt(t->chan_g2[ch]));
-            local = (double)__fmul_rn(__fmul_rn(nG, nG), __fmul_rn(s, s));                                   // optimizer.py:2975-2982
-        }
+#pragma unroll
+        for (int o = SCALES_UNITS / 2; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
         __syncthreads();
         if (lane == 0) s_part[warp] = local;
         __syncthreads();
