@@ -288,6 +288,48 @@ def test_projection_is_correctly_rounded():
         assert np.allclose(chan.cpu().numpy(), want_ch, rtol=1e-12)
 
 
+@pytest.mark.parametrize("rank", [1, 6, 40, 256])
+@pytest.mark.parametrize("many", [False, True], ids=["few_tensors", "runs_over_tensors"])
+def test_scales_batch_equals_per_tensor_calls(rank, many):
+    """af8_apollo_scales_batch against af8_apollo_scales tensor by tensor: rows and columns as channels, channel counts off the
+    units of 8 and the steps of 32, ranks off the 128-bit loads, arrays off the 16-byte grid, and runs of a CTA that span
+    tensors.  Both add squares in binary64 in another order, so a norm may round the other way once: 2 ulp of a quotient."""
+    import ctypes
+    from adafactor8bit import _native as N
+    lib = N.lib()
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device="cpu").manual_seed(rank)
+    shapes = [(300, 17), (5, 33), (1000, 1000), (64, 1027), (9, 8), (24, 4100), (1, 1)] * (40 if many else 1)
+    n, nch = len(shapes), [max(s) for s in shapes]
+    off = [i % 3 == 2 for i in range(n)]
+    upd, low = ([torch.randn(c * rank + o, generator=gen).to(dev)[o:] for c, o in zip(nch, off)] for _ in range(2))
+    g2 = [torch.rand(c, generator=gen, dtype=torch.float64).to(dev) for c in nch]
+    want, got = ([torch.zeros(c, device=dev) for c in nch] for _ in range(2))
+    sums, out_w, out_g = torch.ones(n, 3, dtype=torch.float64, device=dev), *(torch.zeros(n, 4, device=dev) for _ in range(2))
+    host = torch.zeros(n * N.APOLLO_FINISH_TENSOR.itemsize, dtype=torch.uint8).pin_memory()
+    devt = torch.empty_like(host, device=dev)
+    t = np.frombuffer(host.numpy(), dtype=N.APOLLO_FINISH_TENSOR, count=n)
+    s = torch.cuda.current_stream(dev).cuda_stream
+    first = 0
+    for i, (r, c) in enumerate(shapes):
+        sin = N.ApolloScalarsIn()
+        sin.alpha, sin.bc, sin.d, sin.clip_div, sin.sqrt_scale, sin.scale_front = 1e-2, 1.0, 1.0, 3.0, 1.25, int(i % 2)
+        N.check(lib.af8_apollo_scales(upd[i].data_ptr(), low[i].data_ptr(), g2[i].data_ptr(), r, c, rank, ctypes.byref(sin),
+                                      want[i].data_ptr(), sums.data_ptr() + 24 * i, None, out_w.data_ptr() + 16 * i, None, s),
+                "af8_apollo_scales")
+        t["upd"][i], t["g_low"][i], t["chan_g2"][i] = upd[i].data_ptr(), low[i].data_ptr(), g2[i].data_ptr()
+        t["sf"][i], t["sums"][i], t["out"][i] = got[i].data_ptr(), sums.data_ptr() + 24 * i, out_g.data_ptr() + 16 * i
+        t["rows"][i], t["cols"][i], t["rank"][i], t["first_unit"][i] = r, c, rank, first
+        first += (nch[i] + 7) // 8
+        for k in ("alpha", "bc", "d", "clip_div", "sqrt_scale", "scale_front"):
+            t[k][i] = getattr(sin, k)
+    N.check(lib.af8_apollo_scales_batch(host.data_ptr(), devt.data_ptr(), n, first, s), "af8_apollo_scales_batch")
+    torch.cuda.synchronize(dev)
+    assert all(bool((w > 0).all()) for w in want)
+    assert torch.allclose(torch.cat(got), torch.cat(want), rtol=2.5e-7, atol=0.0)
+    assert torch.allclose(out_g, out_w, rtol=5e-7, atol=0.0)
+
+
 @pytest.mark.parametrize("param_dtype,grad_dtype", [("f32", "bf16"), ("f32", "f32"), ("bf16", "bf16")])
 @pytest.mark.parametrize("aligned", [True, False], ids=["vector_path", "one_odd_tensor"])
 def test_apply_batch_equals_per_tensor_calls(param_dtype, grad_dtype, aligned):
