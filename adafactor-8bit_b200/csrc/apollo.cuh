@@ -814,6 +814,10 @@ inline bool apollo_umma_eligible(const af8_apollo_proj_desc &d)
     return !disabled && d.rank % 16 == 0 && d.rank >= 16 && d.rank <= UM_MAXN;
 }
 
+// Whether two SMs share a tile of 256 rows (each holds its rows of G and half of the columns of Pt).  They read half as much of the planes
+// from L2 and from shared memory as two alone: four Llama-3-8B layers 1164 us against 1308.  The instruction takes ranks of whole 32s.
+inline bool apollo_umma_paired(int64_t rank) { return rank % UM_PAIR_N == 0; }
+
 inline int apollo_project_prepare(const af8_apollo_proj_desc &d, int32_t grad_dtype, ProjTask &task, int &next_tile, bool umma,
                                   cudaStream_t st)
 {
@@ -850,7 +854,7 @@ inline int apollo_project_prepare(const af8_apollo_proj_desc &d, int32_t grad_dt
     task.first_tile = next_tile;
     task.tiles_n = umma ? 1 : (task.N + MM_BN - 1) / MM_BN;
     task.reserved = 0;
-    const int64_t tiles = (int64_t)((task.M + MM_BM - 1) / MM_BM) * task.tiles_n;      // MM_BM == UM_BM
+    const int64_t tiles = (int64_t)((task.M + MM_BM - 1) / MM_BM) * task.tiles_n;      // (tcgen05: apollo_umma_number counts again)
     if (tiles + next_tile >= (1ll << 31)) return fail(AF8_ERR_UNSUPPORTED, "af8_apollo_project: too many tiles in one launch");
     next_tile += (int)tiles;
     return AF8_OK;
@@ -859,7 +863,7 @@ inline int apollo_project_prepare(const af8_apollo_proj_desc &d, int32_t grad_dt
 // the two tensor maps of a tcgen05 task: G as [M][K] with boxes of 128 x 32 and the 64-byte swizzle (left: as [K][M] with
 // boxes of 32 x 64 and the 128-byte swizzle), the planes as [3][N][K] with boxes of 3 x N x 32 and the 64-byte swizzle;
 // zero fill outside
-inline int apollo_umma_maps(UmmaTask &u)
+inline int apollo_umma_maps(UmmaTask &u, bool pair)
 {
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return fail(AF8_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
@@ -876,7 +880,7 @@ inline int apollo_umma_maps(UmmaTask &u)
     {
         const cuuint64_t dim[3] = {(cuuint64_t)t.K, (cuuint64_t)t.N, 3};
         const cuuint64_t stride[2] = {(cuuint64_t)t.K * 2, (cuuint64_t)t.K * t.N * 2};
-        const cuuint32_t box[3] = {UM_BK, (cuuint32_t)t.N, 3}, es[3] = {1, 1, 1};
+        const cuuint32_t box[3] = {UM_BK, (cuuint32_t)(pair ? t.N / 2 : t.N), 3}, es[3] = {1, 1, 1};
         const CUresult r = enc(&u.map_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<__nv_bfloat16 *>(t.planes), dim, stride, box, es,
                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -885,15 +889,39 @@ inline int apollo_umma_maps(UmmaTask &u)
     return AF8_OK;
 }
 
+// numbers the tiles of the tasks; their total
+inline int apollo_umma_number(UmmaTask *tasks, int n, bool pair)
+{
+    const int height = pair ? 2 * UM_BM : UM_BM;
+    int tile = 0;
+    for (int i = 0; i < n; ++i) {
+        tasks[i].t.first_tile = tile;
+        tile += (tasks[i].t.M + height - 1) / height;
+    }
+    return tile;
+}
+
+template <int CG>
 inline int apollo_project_launch_umma(const UmmaTask *dev_tasks, int n, int total_tiles, cudaStream_t st)
 {
-    static_assert(MM_BM == UM_BM, "tile height");
-    auto kernel = apollo_project_umma_kernel;
-    AF8_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)um_smem_bytes()));
-    int grid = sm_count();
-    if (grid > total_tiles) grid = total_tiles;
-    kernel<<<grid, UM_THREADS, um_smem_bytes(), st>>>(dev_tasks, n, total_tiles);
-    AF8_CUDA_TRY(cudaGetLastError());
+    auto kernel = apollo_project_umma_kernel<CG>;
+    AF8_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)um_smem_bytes<CG>()));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(sm_count() / CG * CG));
+    cfg.blockDim = dim3(UM_THREADS);
+    cfg.dynamicSmemBytes = um_smem_bytes<CG>();
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CG;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int tiles_at_once = 0;             // (the SMs of a processing cluster need not be even in number: one of a pair may be left over)
+    AF8_CUDA_TRY(cudaOccupancyMaxActiveClusters(&tiles_at_once, kernel, &cfg));
+    if (tiles_at_once > total_tiles) tiles_at_once = total_tiles;
+    cfg.gridDim = dim3((unsigned)(tiles_at_once * CG));
+    AF8_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, dev_tasks, n, total_tiles));
     return AF8_OK;
 }
 
@@ -949,10 +977,13 @@ extern "C" int af8_apollo_project_ws(const void *grad, int32_t grad_dtype, int32
         memset(&u, 0, sizeof(u));
         u.t = task;
         u.chan_g2 = chan_g2;
-        rc = apollo_umma_maps(u);
+        const bool pair = apollo_umma_paired(rank);
+        rc = apollo_umma_maps(u, pair);
         if (rc) return rc;
+        tiles = apollo_umma_number(&u, 1, pair);
         AF8_CUDA_TRY(cudaMemcpyAsync(slot, &u, sizeof(UmmaTask), cudaMemcpyHostToDevice, st));
-        return apollo_project_launch_umma(reinterpret_cast<const UmmaTask *>(slot), 1, tiles, st);
+        const UmmaTask *const dev = reinterpret_cast<const UmmaTask *>(slot);
+        return pair ? apollo_project_launch_umma<2>(dev, 1, tiles, st) : apollo_project_launch_umma<1>(dev, 1, tiles, st);
     }
     AF8_CUDA_TRY(cudaMemcpyAsync(slot, &task, sizeof(ProjTask), cudaMemcpyHostToDevice, st));
     return apollo_project_launch(reinterpret_cast<const ProjTask *>(slot), 1, tiles, st);
@@ -975,10 +1006,11 @@ extern "C" int af8_apollo_project_batch(const af8_apollo_proj_desc *descs, int32
     if (transpose_bytes > 0 && (!transpose_scratch || (reinterpret_cast<uintptr_t>(transpose_scratch) & 255u)))
         return fail(AF8_ERR_INVALID, "af8_apollo_project_batch: transpose_scratch must be 256-byte aligned");      // (no longer used)
     int n_umma = 0, n_mma = 0;
+    bool pair = true;                  // (one launch for all of them)
     for (int i = 0; i < n; ++i) {
         int rc = apollo_check_desc(descs[i], grad_dtype);
         if (rc) return rc;
-        if (apollo_tc_eligible(descs[i], grad_dtype)) { if (apollo_umma_eligible(descs[i])) ++n_umma; else ++n_mma; }
+        if (apollo_tc_eligible(descs[i], grad_dtype)) { if (apollo_umma_eligible(descs[i])) { ++n_umma; pair = pair && apollo_umma_paired(descs[i].rank); } else ++n_mma; }
     }
     UmmaTask *host_u = static_cast<UmmaTask *>(host_scratch);
     const UmmaTask *dev_u = static_cast<const UmmaTask *>(dev_scratch);
@@ -993,7 +1025,7 @@ extern "C" int af8_apollo_project_batch(const af8_apollo_proj_desc *descs, int32
             memset(&u, 0, sizeof(u));
             rc = apollo_project_prepare(descs[i], grad_dtype, u.t, tiles_u, true, st);
             u.chan_g2 = descs[i].chan_g2;
-            if (!rc) rc = apollo_umma_maps(u);
+            if (!rc) rc = apollo_umma_maps(u, pair);
         } else {
             rc = apollo_project_prepare(descs[i], grad_dtype, host_m[im++], tiles_m, false, st);
         }
@@ -1004,13 +1036,9 @@ extern "C" int af8_apollo_project_batch(const af8_apollo_proj_desc *descs, int32
         // is one of short ones (four Llama-3-8B layers: 1600 tiles of K = 4096 and 256 of K = 1024 over 148 CTAs:
         // 1466 -> 1328 us).
         std::sort(host_u, host_u + iu, [](const UmmaTask &a, const UmmaTask &b) { return a.t.K > b.t.K; });
-        int tile = 0;
-        for (int i = 0; i < iu; ++i) {
-            host_u[i].t.first_tile = tile;
-            tile += (host_u[i].t.M + UM_BM - 1) / UM_BM;
-        }
+        tiles_u = apollo_umma_number(host_u, iu, pair);
         int rc = upload_table(dev_scratch, host_u, sizeof(UmmaTask) * (size_t)iu, st);
-        if (!rc) rc = apollo_project_launch_umma(dev_u, iu, tiles_u, st);
+        if (!rc) rc = pair ? apollo_project_launch_umma<2>(dev_u, iu, tiles_u, st) : apollo_project_launch_umma<1>(dev_u, iu, tiles_u, st);
         if (rc) return rc;
     }
     if (n_mma) {

@@ -15,6 +15,15 @@
 // 128-byte swizzle), an M-major operand.  (A separate transposition of such gradients, 52 us per Llama-3-8B layer, and
 // their second trip through memory are gone with it.)
 //
+// Two SMs share a tile of 256 rows wherever the instruction allows it (cta_group::2, ranks of whole 32s; CG = 2 below): each holds its 128
+// rows of the gradient, half of the columns of Pt and the totals of its rows; the first CTA of the pair issues the MMAs for both.  One SM
+// alone reads 56 KB of operands a stage from L2 and 72 KB from shared memory, one of a pair 32 and 48.  That alone changed
+// nothing (four Llama-3-8B layers, rank 256: 1308 -> 1307 us): the stage was as long as the workers' pass over it, a chain of a
+// wait, loads, eight dependent sums, conversion and addition in binary64, 1170 of 1700 cycles.  They now read two
+// stages at a time, whose chains overlap: 1164 us (four at a time spill registers: 1209; two in one SM alone, which has four stages: 1273).
+// Without the pass 1106, without copies of the planes either 1030; at the 1.3 to 1.5 GHz that the power limit leaves the
+// MMAs themselves, at the measured bf16 rate, take 800 (a burst) to 960 us.
+//
 // CTA = 320 threads, one CTA per SM, persistent over (task, M tile) pairs:
 //   warps 0-7  read every gradient tile from shared memory before its MMAs: they add up the
 //              squares of each row of M (the channel norms ||G_row||^2 that the scaling step needs,
@@ -23,9 +32,9 @@
 //              128 (w / 4) .. +127, 128 totals per thread; then store g_low and the norms.
 //   warp 8     allocates / frees TMEM; its lane 0 issues the MMAs and the commits
 //   warp 9     lane 0 issues the copies
-// Four 56 KB stages; a "full" barrier completes on the copies' transaction bytes, a "clean"
-// barrier when the 256 workers have read (and, rarely, repaired) the gradient tile, an "empty"
-// barrier on tcgen05.commit.
+// Four 56 KB stages, of a pair seven of 32 KB; a "full" barrier completes on the copies' transaction bytes, a "clean"
+// barrier of the issuing CTA when the worker warps (of both) have read (and, rarely, repaired) the gradient tile, an "empty"
+// barrier (of both) on tcgen05.commit.
 //
 // The tensor cores add into their binary32 accumulators with truncation, whose error grows
 // linearly with K (measured 1.4e-5 relative at K = 4096, as with mma.sync).  The accumulation
@@ -35,7 +44,7 @@
 // Every wait is bounded (two seconds of %globaltimer); on a time-out the thread raises the
 // device error flag and leaves; the others follow at their next wait or tile, and the tensor
 // memory is freed after all have reported (or after a bounded wait).  After the start-up
-// barrier no block-wide barrier is used, so a lost role cannot hang the others.  No copy
+// barrier no block-wide barrier is used, so a lost role cannot hang the others (a pair meets once more at the end, when every wait is over).  No copy
 // uses cluster multicast.
 #pragma once
 
@@ -49,20 +58,23 @@
 
 namespace af8 {
 
-constexpr int UM_BM = 128, UM_BK = 32, UM_STAGES = 4, UM_THREADS = 320, UM_WORKERS = 256, UM_MMA_WARP = 8, UM_TMA_WARP = 9;
+constexpr int UM_BM = 128, UM_BK = 32, UM_THREADS = 320, UM_WORKERS = 256, UM_MMA_WARP = 8, UM_TMA_WARP = 9;
+template <int CG> __host__ __device__ constexpr int um_stages() { return CG == 2 ? 7 : 4; }
+template <int CG> __host__ __device__ constexpr int um_scan() { return CG == 2 ? 2 : 1; }      // stages that the workers read at a time
+constexpr int UM_PAIR_N = 32;      // a pair takes ranks that are multiples of this
 constexpr int UM_FLUSH = 8;        // stages (256 values of K) per accumulator chunk
 constexpr int UM_MAXN = 256;
 constexpr int UM_ROW_BYTES = UM_BK * 2;                       // 64
 constexpr int UM_A_BYTES = UM_BM * UM_ROW_BYTES;              // 8 KB (a multiple of 1024, like a stage: the 128-byte swizzle's period)
 constexpr int UM_B_BYTES = UM_MAXN * UM_ROW_BYTES;            // 16 KB per plane at N = 256
-constexpr int UM_STAGE_BYTES = UM_A_BYTES + 3 * UM_B_BYTES;   // 56 KB
+template <int CG> __host__ __device__ constexpr int um_stage_bytes() { return UM_A_BYTES + 3 * UM_B_BYTES / CG; }   // 56 KB; of a pair: 32 KB in each SM
 constexpr int UM_SBO = 8 * UM_ROW_BYTES;                      // 512 bytes between 8-row groups
 constexpr int DEVERR_UMMA_TIMEOUT = 2;
 
 // One projection of a tcgen05 launch: the mma.sync task plus the two tensor maps
 struct __align__(64) UmmaTask {
     CUtensorMap map_a;       // right: G as [M][K], box 128 x 32; left: G as [K][M], box 32 x 64
-    CUtensorMap map_b;       // planes as [3][N][K], box 3 x N x 32
+    CUtensorMap map_b;       // planes as [3][N][K], box 3 x N x 32 (of a pair: 3 x N/2 x 32)
     ProjTask t;
     double *chan_g2;         // [M] sums of squares of the rows of G (non-finite entries count as zero)
     unsigned char pad[384 - 2 * sizeof(CUtensorMap) - sizeof(ProjTask) - sizeof(double *)];
@@ -84,21 +96,55 @@ __device__ __forceinline__ uint64_t umma_smem_desc_left(uint32_t smem_addr)
     return (uint64_t)((smem_addr >> 4) & 0x3fffu) | ((uint64_t)(UM_LEFT_BOX_BYTES >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
            (1ull << 46) | (2ull << 61);
 }
-// kind::f16 instruction descriptor: D = F32, A = B = BF16, B K-major, A K-major or (bit 15) M-major, M = 128, N = n
+// kind::f16 instruction descriptor: D = F32, A = B = BF16, B K-major, A K-major or (bit 15) M-major, M = 128 (a pair: 256), N = n
+template <int CG>
 __device__ __forceinline__ uint32_t umma_instr_desc(int n, bool a_m_major)
 {
-    return (1u << 4) | (1u << 7) | (1u << 10) | (a_m_major ? 1u << 15 : 0u) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(UM_BM >> 4) << 24);
+    return (1u << 4) | (1u << 7) | (1u << 10) | (a_m_major ? 1u << 15 : 0u) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(CG * UM_BM >> 4) << 24);
 }
+template <int CG>
 __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
 {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+    if (CG == 2)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                     ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+    else
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                     ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
+// arrives on the barrier (of a pair: on that of both CTAs) when the MMAs issued so far are done
+template <int CG>
 __device__ __forceinline__ void umma_commit(uint64_t *bar)
 {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+    if (CG == 2)
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                     ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
+    else
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+__device__ __forceinline__ uint32_t cluster_rank()
+{
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// every thread of both CTAs
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+// Arrives on the same barrier of the pair's first CTA.  At the default scope: what the other side reads after it was written by copies
+// that this thread has seen complete, in the SM that reads it; a generic write before it takes fence_cluster.  (With release and acquire at
+// cluster scope each arrival waits for the thread's other accesses: 1.3 ms become 2.4.)
+__device__ __forceinline__ void mbar_arrive_first(uint64_t *bar)
+{
+    asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, 0;\n\t"
+                 "mbarrier.arrive.shared::cluster.b64 _, [a];\n\t}" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void fence_cluster() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar)
 {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -140,10 +186,9 @@ __device__ __forceinline__ int volatile_load(const int *p) { return *reinterpret
 // case is eight binary32 multiply-adds; when that sum is not finite (a NaN or an infinity in the
 // chunk, or squares beyond binary32) the non-finite entries are zeroed in shared memory, as the
 // reference zeroes them in the gradient (optimizer.py:2606), and the sum is redone in binary64.
-__device__ __forceinline__ double umma_chunk_sumsq(unsigned char *p, bool &wrote)
+__device__ __forceinline__ float umma_chunk_sum(uint4 v)
 {
-    uint4 v = *reinterpret_cast<uint4 *>(p);
-    uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
     float s = 0.0f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -151,6 +196,13 @@ __device__ __forceinline__ double umma_chunk_sumsq(unsigned char *p, bool &wrote
         s = __fmaf_rn(lo, lo, s);
         s = __fmaf_rn(hi, hi, s);
     }
+    return s;
+}
+__device__ __noinline__ double umma_chunk_sumsq(unsigned char *p, bool &wrote)
+{
+    const uint4 v = *reinterpret_cast<uint4 *>(p);
+    uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    const float s = umma_chunk_sum(v);
     if (s <= 3.0e38f) return (double)s;                          // false for NaN and infinity
     bool changed = false;
     double d = 0.0;
@@ -172,18 +224,23 @@ __device__ __forceinline__ double umma_chunk_sumsq(unsigned char *p, bool &wrote
 // Left case: the 4 values of half a 16-byte chunk belong to 4 rows of M.  Their squares are added to acc[4] in binary32 (the
 // caller passes the sums on to binary64 after at most 8 values); where a magnitude from 2^60 up makes squares that might
 // leave binary32, they go into wide[4] in binary64, and non-finite entries are zeroed in shared memory as above.
+__device__ __forceinline__ void umma_quad_add(uint2 v, float (&acc)[4])
+{
+    const uint32_t w[2] = {v.x, v.y};
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const float lo = __uint_as_float(w[i] << 16), hi = __uint_as_float(w[i] & 0xffff0000u);
+        acc[2 * i] = __fmaf_rn(lo, lo, acc[2 * i]);
+        acc[2 * i + 1] = __fmaf_rn(hi, hi, acc[2 * i + 1]);
+    }
+}
 __device__ __forceinline__ void umma_quad_squares(unsigned char *p, float (&acc)[4], double (&wide)[4], bool &wrote)
 {
     const uint2 v = *reinterpret_cast<const uint2 *>(p);
     uint32_t w[2] = {v.x, v.y};
     const uint32_t top = __vmaxu2(w[0] & 0x7fff7fffu, w[1] & 0x7fff7fffu);
     if ((top >> 16) < 0x5d80u && (top & 0xffffu) < 0x5d80u) {
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const float lo = __uint_as_float(w[i] << 16), hi = __uint_as_float(w[i] & 0xffff0000u);
-            acc[2 * i] = __fmaf_rn(lo, lo, acc[2 * i]);
-            acc[2 * i + 1] = __fmaf_rn(hi, hi, acc[2 * i + 1]);
-        }
+        umma_quad_add(v, acc);
         return;
     }
     bool changed = false;
@@ -201,9 +258,11 @@ __device__ __forceinline__ void umma_quad_squares(unsigned char *p, float (&acc)
     }
 }
 
+template <int CG>
 __global__ void __launch_bounds__(UM_THREADS, 1)
 apollo_project_umma_kernel(const UmmaTask *__restrict__ tasks, int n_tasks, int total_tiles)
 {
+    constexpr int UM_STAGES = um_stages<CG>(), UM_STAGE_BYTES = um_stage_bytes<CG>(), UM_SCAN = um_scan<CG>();
     extern __shared__ __align__(1024) unsigned char um_smem[];
     __shared__ __align__(8) uint64_t s_full[UM_STAGES], s_clean[UM_STAGES], s_empty[UM_STAGES], s_acc_full[2], s_acc_empty[2], s_done;
     __shared__ uint32_t s_tmem;
@@ -211,19 +270,31 @@ apollo_project_umma_kernel(const UmmaTask *__restrict__ tasks, int n_tasks, int 
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
-        for (int s = 0; s < UM_STAGES; ++s) { mbar_init(&s_full[s], 1); mbar_init(&s_clean[s], UM_WORKERS); mbar_init(&s_empty[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&s_acc_full[b], 1); mbar_init(&s_acc_empty[b], UM_WORKERS); }
+        for (int s = 0; s < UM_STAGES; ++s) { mbar_init(&s_full[s], 1); mbar_init(&s_clean[s], CG * UM_WORKERS / 32); mbar_init(&s_empty[s], 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&s_acc_full[b], 1); mbar_init(&s_acc_empty[b], CG * UM_WORKERS / 32); }
         mbar_init(&s_done, UM_THREADS);
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == UM_MMA_WARP) {   // all 512 columns of tensor memory: two 128 x 256 binary32 accumulators
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(512u) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (CG == 2) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(512u) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(512u) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     tc_fence_before();
     __syncthreads();             // the only block-wide barrier: after it the roles run on mbarriers alone
+    if (CG == 2) cluster_sync(); // (the other CTA's barriers are set up, and both have allocated)
     tc_fence_after();
+    const int cta = CG == 2 ? (int)cluster_rank() : 0;
+    // one arrival of a warp, on the barrier of the CTA that issues the MMAs
+    const auto arrive_issuer = [&](uint64_t *bar) {
+        __syncwarp();
+        if (lane == 0) { if (CG == 2) mbar_arrive_first(bar); else mbar_arrive(bar); }
+    };
     const uint32_t tmem = s_tmem;
     const uint32_t smem_base = smem_u32(um_smem);
 
@@ -234,7 +305,7 @@ apollo_project_umma_kernel(const UmmaTask *__restrict__ tasks, int n_tasks, int 
     int issued = 0;                 // producer only: stage fills issued so far
     int mapped = -1;                // producer only: task whose tensor maps it has acquired
 
-    for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
+    for (int tile = blockIdx.x / CG; tile < total_tiles; tile += gridDim.x / CG) {
         if (volatile_load(&s_abort)) break;
         int lo = 0, hi = n_tasks - 1;
         while (lo < hi) {
@@ -244,10 +315,10 @@ apollo_project_umma_kernel(const UmmaTask *__restrict__ tasks, int n_tasks, int 
         const UmmaTask *U = tasks + lo;
         const ProjTask *T = &U->t;
         const int M = __ldg(&T->M), N = __ldg(&T->N), K = __ldg(&T->K);
-        const int m0 = (tile - __ldg(&T->first_tile)) * UM_BM;
+        const int m0 = (tile - __ldg(&T->first_tile)) * CG * UM_BM + cta * UM_BM;       // rows of this CTA
         const int ksteps = (K + UM_BK - 1) / UM_BK;
         const int nchunks = (ksteps + UM_FLUSH - 1) / UM_FLUSH;
-        const int plane_bytes = N * UM_ROW_BYTES;
+        const int plane_bytes = N / CG * UM_ROW_BYTES;                     // (of a pair each CTA has half of the columns)
         const bool right = __ldg(&T->right) != 0;
         bool failed = false;
 
@@ -262,7 +333,7 @@ apollo_project_umma_kernel(const UmmaTask *__restrict__ tasks, int n_tasks, int 
             // add accumulator chunk c of this tile into the totals, with rounding, and hand the buffer back
             auto flush = [&](int c) -> bool {
                 const int g = gchunk + c, buf = g & 1;
-                if (!mbar_wait_bounded(&s_acc_full[buf], (uint32_t)(g >> 1) & 1u)) return false;
+                if (!__all_sync(0xffffffffu, mbar_wait_bounded(&s_acc_full[buf], (uint32_t)(g >> 1) & 1u))) return false;
                 tc_fence_after();
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
@@ -279,7 +350,7 @@ apollo_project_umma_kernel(const UmmaTask *__restrict__ tasks, int n_tasks, int 
                     }
                 }
                 tc_fence_before();
-                mbar_arrive(&s_acc_empty[buf]);
+                arrive_issuer(&s_acc_empty[buf]);
                 return true;
             };
             // The 8 KB gradient tile of a stage is 512 chunks of 16 bytes, two per thread.  rs: this thread's share
@@ -289,35 +360,75 @@ apollo_project_umma_kernel(const UmmaTask *__restrict__ tasks, int n_tasks, int 
             // of two of the four groups of 8.  The 128-byte swizzle puts chunk c of a box row k at c ^ (k & 7): the 16
             // lanes of an access hit 16 different pairs of banks.
             double rs[4];
-            float rq[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { rs[i] = 0.0; rq[i] = 0.0f; }
+            for (int i = 0; i < 4; ++i) rs[i] = 0.0;
             const int lk = 2 * ((lane >> 2) & 3), lc = 2 * (warp & 3) + ((lane >> 1) & 1);
             const int lbase = (warp >> 2) * UM_LEFT_BOX_BYTES + (lane >> 4) * 2048 + (lane & 1) * 8;
             const int left0 = lbase + lk * 128 + ((lc ^ lk) << 4), left1 = lbase + (lk + 1) * 128 + ((lc ^ (lk + 1)) << 4);
-            auto scan = [&](int c) -> bool {
-                const int k_end = min(ksteps, (c + 1) * UM_FLUSH);
-                for (int ks = c * UM_FLUSH; ks < k_end; ++ks) {
-                    const int f = fills + ks, slot = f % UM_STAGES;
-                    if (!mbar_wait_bounded(&s_full[slot], (uint32_t)(f / UM_STAGES) & 1u)) return false;
-                    unsigned char *st = um_smem + slot * UM_STAGE_BYTES;
-                    bool wrote = false;
-                    if (right) {
-                        rs[0] += umma_chunk_sumsq(st + tid * 16, wrote);
-                        rs[1] += umma_chunk_sumsq(st + (tid + UM_WORKERS) * 16, wrote);
-                    } else {
-                        umma_quad_squares(st + left0, rq, rs, wrote);
-                        umma_quad_squares(st + left1, rq, rs, wrote);
-                        umma_quad_squares(st + left0 + 1024, rq, rs, wrote);
-                        umma_quad_squares(st + left1 + 1024, rq, rs, wrote);
-                        if ((ks & 1) == 1 || ks + 1 == ksteps) {     // (8 values)
+            // NS stages from stage ks of the tile on
+            const auto scan_stages = [&](int ks, auto count) -> bool {
+                constexpr int NS = decltype(count)::value;
+                unsigned char *st[NS];
+                bool wrote = false;
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) { rs[i] += (double)rq[i]; rq[i] = 0.0f; }
+                for (int i = 0; i < NS; ++i) {
+                    const int f = fills + ks + i, slot = f % UM_STAGES;
+                    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&s_full[slot], (uint32_t)(f / UM_STAGES) & 1u))) return false;
+                    st[i] = um_smem + slot * UM_STAGE_BYTES;
+                }
+                if (right) {
+                    uint4 v[2 * NS];
+                    float sum[2 * NS];
+                    bool finite = true;
+#pragma unroll
+                    for (int i = 0; i < 2 * NS; ++i) v[i] = *reinterpret_cast<const uint4 *>(st[i >> 1] + (tid + (i & 1) * UM_WORKERS) * 16);
+#pragma unroll
+                    for (int i = 0; i < 2 * NS; ++i) { sum[i] = umma_chunk_sum(v[i]); finite = finite && sum[i] <= 3.0e38f; }
+                    if (finite) {
+#pragma unroll
+                        for (int i = 0; i < 2 * NS; ++i) rs[i & 1] += (double)sum[i];
+                    } else {
+#pragma unroll 1
+                        for (int i = 0; i < NS; ++i) {
+                            unsigned char *const p = um_smem + ((fills + ks + i) % UM_STAGES) * UM_STAGE_BYTES + tid * 16;
+                            rs[0] += umma_chunk_sumsq(p, wrote);
+                            rs[1] += umma_chunk_sumsq(p + UM_WORKERS * 16, wrote);
                         }
                     }
-                    if (wrote) fence_proxy_async();              // repaired entries must be visible to the MMAs
-                    mbar_arrive(&s_clean[slot]);
+                } else {
+                    float rq[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                    uint2 v[4 * NS];
+                    uint32_t top = 0;
+#pragma unroll
+                    for (int i = 0; i < 4 * NS; ++i) v[i] = *reinterpret_cast<const uint2 *>(st[i >> 2] + ((i & 1) ? left1 : left0) + ((i >> 1) & 1) * 1024);
+#pragma unroll
+                    for (int i = 0; i < 4 * NS; ++i) top = __vmaxu2(top, __vmaxu2(v[i].x & 0x7fff7fffu, v[i].y & 0x7fff7fffu));
+                    if ((top >> 16) < 0x5d80u && (top & 0xffffu) < 0x5d80u) {
+#pragma unroll
+                        for (int i = 0; i < 4 * NS; ++i) umma_quad_add(v[i], rq);
+                    } else {
+#pragma unroll 1
+                        for (int i = 0; i < 4 * NS; ++i)
+                            umma_quad_squares(um_smem + ((fills + ks + (i >> 2)) % UM_STAGES) * UM_STAGE_BYTES + ((i & 1) ? left1 : left0) + ((i >> 1) & 1) * 1024, rq, rs, wrote);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) rs[i] += (double)rq[i];      // (at most 8 values each)
                 }
+                if (wrote) {                                 // repaired entries must be visible to the MMAs
+                    if (CG == 2) fence_cluster();
+                    fence_proxy_async();
+                }
+#pragma unroll
+                for (int i = 0; i < NS; ++i) arrive_issuer(&s_clean[(fills + ks + i) % UM_STAGES]);
+                return true;
+            };
+            auto scan = [&](int c) -> bool {
+                const int k_end = min(ksteps, (c + 1) * UM_FLUSH);
+                int ks = c * UM_FLUSH;
+                for (; ks + UM_SCAN <= k_end; ks += UM_SCAN)
+                    if (!scan_stages(ks, std::integral_constant<int, UM_SCAN>())) return false;
+                for (; ks < k_end; ++ks)
+                    if (!scan_stages(ks, std::integral_constant<int, 1>())) return false;
                 return true;
             };
             for (int c = 0; c < nchunks && !failed; ++c) {
@@ -368,9 +479,9 @@ apollo_project_umma_kernel(const UmmaTask *__restrict__ tasks, int n_tasks, int 
                     }
                 }
             }
-        } else if (warp == UM_MMA_WARP && lane == 0) {
+        } else if (warp == UM_MMA_WARP && lane == 0 && cta == 0) {
             // ---------------- MMA issuer ----------------
-            const uint32_t idesc = umma_instr_desc(N, !right);
+            const uint32_t idesc = umma_instr_desc<CG>(N, !right);
             for (int ks = 0; ks < ksteps; ++ks) {
                 const int g = gchunk + ks / UM_FLUSH, buf = g & 1;
                 const bool chunk_start = (ks % UM_FLUSH) == 0;
@@ -391,11 +502,11 @@ apollo_project_umma_kernel(const UmmaTask *__restrict__ tasks, int n_tasks, int 
 #pragma unroll
                     for (int t = 2; t >= 0; --t) {              // smallest plane first
                         const uint64_t bd = umma_smem_desc(a0 + UM_A_BYTES + t * plane_bytes + k16 * 32);
-                        umma_bf16(d, ad, bd, idesc, (!chunk_start || k16 > 0 || t < 2) ? 1u : 0u);
+                        umma_bf16<CG>(d, ad, bd, idesc, (!chunk_start || k16 > 0 || t < 2) ? 1u : 0u);
                     }
                 }
-                umma_commit(&s_empty[slot]);                    // frees the slot when these MMAs are done
-                if ((ks % UM_FLUSH) == UM_FLUSH - 1 || ks == ksteps - 1) umma_commit(&s_acc_full[buf]);
+                umma_commit<CG>(&s_empty[slot]);                    // frees the slot when these MMAs are done
+                if ((ks % UM_FLUSH) == UM_FLUSH - 1 || ks == ksteps - 1) umma_commit<CG>(&s_acc_full[buf]);
             }
         } else if (warp == UM_TMA_WARP && lane == 0) {
             // ---------------- copies ----------------
@@ -415,7 +526,7 @@ apollo_project_umma_kernel(const UmmaTask *__restrict__ tasks, int n_tasks, int 
                     tma_load_2d(st, &U->map_a, m0, ks * UM_BK, &s_full[slot]);
                     tma_load_2d(st + UM_LEFT_BOX_BYTES, &U->map_a, m0 + UM_LEFT_BOX_M, ks * UM_BK, &s_full[slot]);
                 }
-                tma_load_3d(st + UM_A_BYTES, &U->map_b, ks * UM_BK, 0, 0, &s_full[slot]);
+                tma_load_3d(st + UM_A_BYTES, &U->map_b, ks * UM_BK, cta * (N / CG), 0, &s_full[slot]);
                 issued = f + 1;
             }
         }
@@ -443,10 +554,16 @@ apollo_project_umma_kernel(const UmmaTask *__restrict__ tasks, int n_tasks, int 
     if (warp == UM_MMA_WARP) {
         mbar_wait_bounded(&s_done, 0u);
         __syncwarp();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
     }
+    // (a pair: no CTA ends, or frees, while the other may still arrive on its barriers or use its memory; every wait before has an end)
+    if (CG == 2) { __syncwarp(); cluster_sync(); }
+    if (warp == UM_MMA_WARP) {
+        if (CG == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    }
+    if (CG == 2) { __syncwarp(); cluster_sync(); }
 }
 
-constexpr size_t um_smem_bytes() { return (size_t)UM_STAGES * UM_STAGE_BYTES + 1024; }
+template <int CG> constexpr size_t um_smem_bytes() { return (size_t)um_stages<CG>() * um_stage_bytes<CG>() + 1024; }
 
 }  // namespace af8

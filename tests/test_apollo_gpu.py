@@ -216,13 +216,29 @@ def test_tensor_core_projection(rows, cols, rank, negate):
     assert np.allclose(chan.cpu().numpy(), want_ch, rtol=1e-6)
 
 
+@pytest.mark.parametrize("rows,cols,rank", [(104, 40, 32), (264, 72, 64), (392, 264, 96), (136, 1288, 224), (40, 128, 32), (640, 640, 256),
+                                            (136, 264, 48)])
+def test_projection_tiles_of_two_sms(rows, cols, rank):
+    """Ranks of whole 32s: tiles of 256 rows over two SMs (second half empty, partly filled, full; odd numbers of stages; one
+    accumulator chunk and several).  The last rank is none: one SM for each tile."""
+    test_tensor_core_projection(rows, cols, rank, 0)
+
+
 def test_tensor_core_projection_batch():
     """af8_apollo_project_batch over mixed shapes: right-case tensors and left-case ones (the gradient as an
     M-major operand) on the tcgen05 kernel, a rank that is no multiple of 16 on mma.sync."""
+    _projection_batch([(512, 256, 64), (128, 640, 64), (64, 1032, 32), (264, 136, 24), (96, 2048, 256)])
+
+
+def test_tensor_core_projection_batch_of_single_tiles():
+    """One rank that is no multiple of 32 gives the whole launch tiles of one SM."""
+    _projection_batch([(512, 256, 64), (128, 640, 48), (64, 1032, 32)])
+
+
+def _projection_batch(shapes):
     from adafactor8bit import _native as N
     lib = N.lib()
     rng = np.random.default_rng(5)
-    shapes = [(512, 256, 64), (128, 640, 64), (64, 1032, 32), (264, 136, 24), (96, 2048, 256)]
     stream = torch.cuda.current_stream().cuda_stream
     descs = np.zeros(len(shapes), dtype=N.APOLLO_PROJ_DESC)
     keep, wants, outs, chans, want_chs = [], [], [], [], []
