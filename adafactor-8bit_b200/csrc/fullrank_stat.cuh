@@ -17,7 +17,15 @@
 // special-function pipe was the busiest unit with the decode per element (3 operations,
 // 70 % busy): the table took the pass from 1.04 to 0.93 ms on the TinyLlama set.
 // (Replacing the reciprocal by rsqrt and a short series was measured slower; so were requests for the
-// next block's lines in L2, 0.972 against 0.955 ms.)  AL16 has too many codes for a table: an element
+// next block's lines in L2, 0.972 against 0.955 ms.)
+//
+// What it waits for then is its loads (8 of 13 stall cycles an instruction).  With bf16 gradients, UF8 and AL8 each lane copies what it will
+// read into a ring of its own in shared memory (cp.async; no other thread reads it, so nothing but its own groups is waited for), three
+// steps of 256 elements ahead and on into the warp's next block, whose ranges are loaded a block ahead as well.  The ring takes the
+// place of load registers: 64 without spills at four CTAs of 256 threads.  270 M parameters 223 -> 204 us (5.3 TB/s); with four steps of a
+// block unrolled instead of eight 220, with five CTAs 232 and more (spills), five CTAs without the ring 223 and four 227.
+//
+// AL16 has too many codes for a table: an element
 // costs a polynomial more (176 M UF4/AL16 parameters: 0.30 ms; 0.55 with the binary64 sequence of exp2_lane).
 #pragma once
 
@@ -36,8 +44,26 @@ constexpr int STAT_THREADS = 256;
 #ifndef AF8_STAT_UNROLL
 #define AF8_STAT_UNROLL 4
 #endif
-#define AF8_PRAGMA_(x) _Pragma(#x)
-#define AF8_UNROLL_(n) AF8_PRAGMA_(unroll n)
+constexpr int STAT_RING = 4, STAT_SLOT = FAST_MBLOCK * 4;    // steps in flight; bytes of one: gradients, momentum and second-moment codes
+template <typename GradT, int VB, int MF> __host__ __device__ constexpr bool stat_ring() { return std::is_same<GradT, bf16_tag>::value && VB == 8 && MF == AF8_M_UF8; }
+#ifndef AF8_STAT_MIN_CTAS_RING
+#define AF8_STAT_MIN_CTAS_RING 4
+#endif
+template <typename GradT, int VB, int MF> __host__ __device__ constexpr int stat_min_ctas()
+{
+    return stat_ring<GradT, VB, MF>() ? AF8_STAT_MIN_CTAS_RING : VB == 16 ? AF8_STAT_MIN_CTAS16 : AF8_STAT_MIN_CTAS;
+}
+
+__device__ __forceinline__ void copy_async16(void *dst, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async8(void *dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 template <int ROOT>
 __device__ __forceinline__ float ex2_approx(float x)
@@ -82,18 +108,21 @@ __device__ __forceinline__ void stat_load_g<float>(const void *grad, int64_t off
     g[0] = a.x; g[1] = a.y; g[2] = a.z; g[3] = a.w; g[4] = b.x; g[5] = b.y; g[6] = b.z; g[7] = b.w;
 }
 
-template <>
-__device__ __forceinline__ void stat_load_g<bf16_tag>(const void *grad, int64_t off, float (&g)[8])
+__device__ __forceinline__ void stat_widen(uint4 a, float (&g)[8])
 {
-    const uint4 a = __ldcs(reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(grad) + off));
     g[0] = __uint_as_float(a.x << 16); g[1] = __uint_as_float(a.x & 0xffff0000u);
     g[2] = __uint_as_float(a.y << 16); g[3] = __uint_as_float(a.y & 0xffff0000u);
     g[4] = __uint_as_float(a.z << 16); g[5] = __uint_as_float(a.z & 0xffff0000u);
     g[6] = __uint_as_float(a.w << 16); g[7] = __uint_as_float(a.w & 0xffff0000u);
 }
+template <>
+__device__ __forceinline__ void stat_load_g<bf16_tag>(const void *grad, int64_t off, float (&g)[8])
+{
+    stat_widen(__ldcs(reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(grad) + off)), g);
+}
 
 template <typename GradT, int VB, int MF>
-__global__ void __launch_bounds__(STAT_THREADS, VB == 16 ? AF8_STAT_MIN_CTAS16 : AF8_STAT_MIN_CTAS)
+__global__ void __launch_bounds__(STAT_THREADS, (stat_min_ctas<GradT, VB, MF>()))
 fullrank_stat_kernel(const FullrankLaunch L)
 {
     // per-warp decode table of the block's 256 second-moment codes: 8 exponentials per lane and block
@@ -103,6 +132,9 @@ fullrank_stat_kernel(const FullrankLaunch L)
     constexpr bool EXACT = root_exact<VB, MF>;
     __shared__ float s_dec[STAT_THREADS / 32][TABLE ? 256 : 1];
     __shared__ double s_exp2[EXACT && TABLE ? 32 : 1];       // copy of the exp2 table of the exact decode
+    constexpr bool RING = stat_ring<GradT, VB, MF>();
+    constexpr int STEPS = FAST_VBLOCK / FAST_MBLOCK, UNROLL = RING ? STEPS : AF8_STAT_UNROLL;
+    __shared__ __align__(16) unsigned char s_ring[STAT_THREADS / 32][RING ? STAT_RING * STAT_SLOT : 16];
     const int lane = threadIdx.x & 31;
     if (EXACT && TABLE) {
         if (threadIdx.x < 32) s_exp2[threadIdx.x] = c_exp2_tab[threadIdx.x];
@@ -141,12 +173,31 @@ fullrank_stat_kernel(const FullrankLaunch L)
         const int64_t stop = min(cur_end, L.total_blocks);
         const auto blocks = [&](auto root) {
             constexpr int ROOT = decltype(root)::value;
+            // the ring: this lane's 8 elements of a step lie in its own 32 bytes of the step's slot
+            unsigned char *const ring = s_ring[threadIdx.x >> 5];
+            const auto request = [&](int64_t first, int step) {
+                const int64_t o = first + step * FAST_MBLOCK + lane * 8;
+                unsigned char *const r = ring + step % STAT_RING * STAT_SLOT;
+                copy_async16(r + lane * 16, static_cast<const uint16_t *>(grad) + o);
+                copy_async8(r + FAST_MBLOCK * 2 + lane * 8, mq + o);
+                copy_async8(r + FAST_MBLOCK * 3 + lane * 8, vq + o);
+            };
+            bool ahead = false;                 // the first steps of the block at hand are requested, its ranges loaded
+            [[maybe_unused]] float next_sc = 0.0f, next_ml = 0.0f, next_ms = 0.0f;
             for (; blk < stop; blk += warps) {
                 const int64_t b = blk - cur_first;
                 const int64_t base = b * FAST_VBLOCK;
                 const int64_t rem = numel - base;
                 // decode v = 2^((code-1)*scale/levels + min_log) as 2^(code*a + c)
-                const float sc = __ldg(v_scale + b), ml = __ldg(v_min_log + b);
+                const bool requested = RING && ahead;
+                const float sc = requested ? next_sc : __ldg(v_scale + b), ml = requested ? next_ml : __ldg(v_min_log + b);
+                // (lane s: the momentum scale of step s)
+                [[maybe_unused]] const float ms = requested ? next_ms : RING && rem >= FAST_VBLOCK ? __ldg(m_scale + b * STEPS + (lane & (STEPS - 1))) : 0.0f;
+                if (RING) {
+                    const int64_t nb = b + warps;
+                    ahead = blk + warps < stop && numel - nb * FAST_VBLOCK >= FAST_VBLOCK && small_w;
+                    if (ahead) { next_sc = __ldg(v_scale + nb); next_ml = __ldg(v_min_log + nb); next_ms = __ldg(m_scale + nb * STEPS + (lane & (STEPS - 1))); }
+                }
                 [[maybe_unused]] const float a = sc * (VB == 16 ? 1.0f / 65534.0f : 1.0f / 254.0f);
                 [[maybe_unused]] const float c = ml - a;
                 float acc = 0.0f;
@@ -165,30 +216,45 @@ fullrank_stat_kernel(const FullrankLaunch L)
                         }
                         __syncwarp();
                     }
+                    if (RING && !requested) {
+#pragma unroll
+                        for (int q = 0; q < STAT_RING - 1; ++q) { request(base, q); copy_async_commit(); }
+                    }
                     const float2 wv2 = bc2(v_w), wm2 = bc2(m_w), ed2 = bc2(eps_d);
                     float2 acc2 = make_float2(0.0f, 0.0f);
-AF8_UNROLL_(AF8_STAT_UNROLL)
-                    for (int s = 0; s < FAST_VBLOCK / FAST_MBLOCK; ++s) {
+#pragma unroll UNROLL
+                    for (int s = 0; s < STEPS; ++s) {
                         const int64_t off = base + s * FAST_MBLOCK + lane * 8;
                         float g[8];
-                        stat_load_g<GradT>(grad, off, g);
+                        [[maybe_unused]] const unsigned char *const slot = ring + s % STAT_RING * STAT_SLOT;
+                        if (RING) {
+                            const int q = s + STAT_RING - 1;         // (into the slot that the step before has left)
+                            if (q < STEPS) request(base, q);
+                            else if (ahead) request(base + warps * FAST_VBLOCK, q - STEPS);
+                            copy_async_commit();
+                            copy_async_wait<STAT_RING - 1>();
+                            stat_widen(*reinterpret_cast<const uint4 *>(slot + lane * 16), g);
+                        } else {
+                            stat_load_g<GradT>(grad, off, g);
+                        }
                         if (L.negate_grad) {                       // maximize (optimizer.py:1973-1974)
 #pragma unroll
                             for (int j = 0; j < 8; ++j) g[j] = -g[j];
                         }
                         uint2 mw = make_uint2(0u, 0u);
                         uint32_t vw[VB / 4];
-                        if (MF == AF8_M_UF8) mw = __ldcs(reinterpret_cast<const uint2 *>(mq + off));
+                        if (RING) mw = *reinterpret_cast<const uint2 *>(slot + FAST_MBLOCK * 2 + lane * 8);
+                        else if (MF == AF8_M_UF8) mw = __ldcs(reinterpret_cast<const uint2 *>(mq + off));
                         if (MF == AF8_M_UF4) mw.x = __ldcs(reinterpret_cast<const uint32_t *>(mq + off / 2));
                         if (VB == 8) {
-                            const uint2 w = __ldcs(reinterpret_cast<const uint2 *>(vq + off));
+                            const uint2 w = RING ? *reinterpret_cast<const uint2 *>(slot + FAST_MBLOCK * 3 + lane * 8) : __ldcs(reinterpret_cast<const uint2 *>(vq + off));
                             vw[0] = w.x; vw[1] = w.y;
                         } else {
                             const uint4 w = __ldcs(reinterpret_cast<const uint4 *>(vq + off * 2));
                             vw[0] = w.x; vw[1] = w.y; vw[VB / 4 - 2] = w.z; vw[VB / 4 - 1] = w.w;
                         }
                         float2 sum8 = make_float2(0.0f, 0.0f);
-                        const float2 mc2 = bc2(MF == AF8_M_NONE ? 0.0f : __ldg(m_scale + b * (FAST_VBLOCK / FAST_MBLOCK) + s) * M_UNIT);
+                        const float2 mc2 = bc2(RING ? __shfl_sync(0xffffffffu, ms, s) * M_UNIT : MF == AF8_M_NONE ? 0.0f : __ldg(m_scale + b * STEPS + s) * M_UNIT);
 #pragma unroll
                         for (int j = 0; j < 8; j += 2) {
                             const float2 gj = make_float2(g[j], g[j + 1]);
