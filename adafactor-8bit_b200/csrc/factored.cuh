@@ -1592,8 +1592,8 @@ factored_stats_vec_kernel(const FactoredLaunch L, const CUtensorMap *__restrict_
 // the element-wise function, whose 64-bit generator is 60 instructions, the momentum-free write pass over the TinyLlama set took
 // 4.25 ms stochastically against 2.32, and 3.75 against 2.54 to nearest with a momentum); 3: any 16-bit format, element by element.
 // CTAS: resident CTAs per SM asked of the compiler.  Measured on B200: 4 for the sum passes; for the
-// writing passes 3 with momentum (CAME, 0.78 ms per Llama-2-7B layer) and 2 without (Adafactor on the
-// TinyLlama set: 2.51 -> 2.21 ms, no register spills).
+// writing passes 3 with momentum (CAME, 0.78 ms per Llama-2-7B layer) and 2 without (which the write kernel below has
+// taken over wherever it can: see factored_write_kernel).
 // ANY = 1: batches of matrices, rows of a multiple of 8.  ANY = 2: rows of any length >= 8 as well.  The flat vectors of
 // 8 stay aligned; a vector crosses at most one row end, so its elements take one of two row factors, and column factors
 // from three aligned vectors that are shifted (one by one in a lane with a row end).  Only a tensor's last vector may be
