@@ -44,22 +44,6 @@ _V_TYPES = ("al8", "al16", "fp32")                         # optimizer.py:25
 f32 = np.float32
 
 
-def _step_hooks(func):
-    """torch.optim's wrapper around step, which runs the step hooks inside a range for the profiler, where there are hooks or a profiler
-    records; the step itself otherwise (the wrapper costs 14 us, a sixth of a small step)."""
-    full = Optimizer.profile_hook_step(func)
-    before, after = _global_optimizer_pre_hooks, _global_optimizer_post_hooks
-
-    @functools.wraps(func)
-    def wrapper(*args, **kwargs):
-        self = args[0]
-        if self._optimizer_step_pre_hooks or self._optimizer_step_post_hooks or before or after or torch.autograd.profiler._is_profiler_enabled:
-            return full(*args, **kwargs)
-        return func(*args, **kwargs)
-    wrapper.hooked = True        # (torch.optim wraps the step of a class without this mark)
-    return wrapper
-
-
 class _Launch:
     """What one launch plan is to step: parameters, their gradients and states.  cached: params and states are the lists of the
     group's cache, the same objects at every step until the group is sorted again."""
@@ -669,7 +653,36 @@ class Adafactor8Bit(Optimizer):
     # ------------------------------------------------------------------
     # step
     # ------------------------------------------------------------------
-    @_step_hooks
+    # torch.optim wraps the step of a class when the first instance of it is made, by this method.
+    _stepping = False             # a step of this instance is under way
+
+    @staticmethod
+    def profile_hook_step(func):
+        """torch.optim's wrapper around step: the hooks, inside a range named after the step.  Where there is no hook and no profiler
+        records, the range alone, by torch's shorter call, whose range every record-function observer sees as well (2 us against 8; a
+        small step takes 70).  Hooks and range come once a step: the wrapped step that the step of a subclass calls has neither."""
+        full = Optimizer.profile_hook_step(func)
+        before, after = _global_optimizer_pre_hooks, _global_optimizer_post_hooks
+        enter, leave = torch._C._autograd._record_function_with_args_enter, torch._C._autograd._record_function_with_args_exit
+
+        @functools.wraps(func)
+        def wrapper(*args, **kwargs):
+            self = args[0]
+            if self._stepping:
+                return func(*args, **kwargs)
+            self._stepping = True
+            try:
+                if self._optimizer_step_pre_hooks or self._optimizer_step_post_hooks or before or after or torch.autograd.profiler._is_profiler_enabled:
+                    return full(*args, **kwargs)
+                mark = enter(f"Optimizer.step#{self.__class__.__name__}.step")
+                try:
+                    return func(*args, **kwargs)
+                finally:
+                    leave(mark)
+            finally:
+                self._stepping = False
+        return wrapper
+
     @torch.no_grad()
     def step(self, closure=None, *, grad_ready=None):
         """One optimization step (optimizer.py:1866-1938).
