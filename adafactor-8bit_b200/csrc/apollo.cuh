@@ -681,9 +681,9 @@ apollo_write_kernel(const af8_apollo_apply_tensor *tensors, int n, int negate, i
             write_position(U, o, row, col);
             float2 f[2];
             if (scale_tensor) f[0] = f[1] = bc2(U.st);
-            else if (right) f[0] = f[1] = bc2(__ldg(U.sf + row));
+            else if (right) f[0] = f[1] = bc2(load_state(U.sf + row));
             else {
-                const float4 a = __ldg(reinterpret_cast<const float4 *>(U.sf + col));
+                const float4 a = load_state(reinterpret_cast<const float4 *>(U.sf + col));
                 f[0] = make_float2(a.x, a.y); f[1] = make_float2(a.z, a.w);
             }
             float2 g[2], p[2];

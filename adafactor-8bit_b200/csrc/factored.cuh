@@ -143,7 +143,7 @@ __device__ __forceinline__ float load_grad_any(const void *g, int dtype, int64_t
 __device__ __forceinline__ float m_old_at(const af8_factored_tensor &T, int m_fmt, int m_block, int64_t flat)
 {
     if (m_fmt == AF8_M_FP32) return T.m_f32[flat];
-    return m_decode(T.m_q, __ldg(T.m_scale + flat / m_block), flat, m_fmt);
+    return m_decode(T.m_q, load_state(T.m_scale + flat / m_block), flat, m_fmt);
 }
 
 // Tensor.lerp_ with a weight that is the same for many elements: the choice between ATen's two
@@ -730,9 +730,9 @@ __device__ __forceinline__ void load_f8(const float *p, float (&x)[8])
     x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
 }
 
-__device__ __forceinline__ void load_f8_ro(const float *p, float (&x)[8])     // read-only data, kept in L1
+__device__ __forceinline__ void load_f8_ro(const float *p, float (&x)[8])
 {
-    const float4 a = __ldg(reinterpret_cast<const float4 *>(p)), b = __ldg(reinterpret_cast<const float4 *>(p + 4));
+    const float4 a = load_state(reinterpret_cast<const float4 *>(p)), b = load_state(reinterpret_cast<const float4 *>(p + 4));
     x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
 }
 
@@ -742,7 +742,7 @@ __device__ __forceinline__ void m_old8(const af8_factored_tensor &T, int m_fmt, 
                                        bool have_pre = false, uint2 pre = make_uint2(0u, 0u))
 {
     if (m_fmt == AF8_M_FP32) { load_f8(T.m_f32 + flat, m); return; }
-    const float sc = __ldg(T.m_scale + (m_block == 256 ? flat >> 8 : flat / m_block));
+    const float sc = load_state(T.m_scale + (m_block == 256 ? flat >> 8 : flat / m_block));
     if (m_fmt == AF8_M_UF8) {
         const uint2 w = have_pre ? pre : *reinterpret_cast<const uint2 *>(T.m_q + flat);
         const float mc = __fmul_rn(sc, 0.0078125f);      // fl(scale / 128): a power-of-two divisor, scale >= 1e-12
@@ -764,7 +764,7 @@ template <> struct GradAny8<bf16_tag> {
     int s;
     __device__ __forceinline__ static uint4 vec(const uint16_t *p, int64_t off, int64_t numel)
     {
-        if (off + 8 <= numel) return __ldg(reinterpret_cast<const uint4 *>(p + off));
+        if (off + 8 <= numel) return load_state(reinterpret_cast<const uint4 *>(p + off));
         GradRaw8<bf16_tag> t;
         t.load_part(p, off, (int)(numel - off));                 // (none for a negative count)
         return t.a;
@@ -805,7 +805,7 @@ template <> struct GradAny8<float> {
     {
         const float *p = static_cast<const float *>(grad) + off;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = off + j < numel ? __ldg(p + j) : 0.0f;
+        for (int j = 0; j < 8; ++j) v[j] = off + j < numel ? load_state(p + j) : 0.0f;
     }
     __device__ __forceinline__ void unpack(int negate, float (&g)[8]) const
     {
@@ -820,7 +820,7 @@ __device__ __forceinline__ void m_old8_any(const af8_factored_tensor &T, int m_f
     if (m_fmt == AF8_M_UF8 && m_block == 256) {
         const int64_t b = flat >> 8, last = (numel - 1) >> 8;
         const int left = 256 - (int)(flat & 255);                // elements of the first block
-        const float s0 = __fmul_rn(__ldg(T.m_scale + b), 0.0078125f), s1 = __fmul_rn(__ldg(T.m_scale + min(b + 1, last)), 0.0078125f);
+        const float s0 = __fmul_rn(load_state(T.m_scale + b), 0.0078125f), s1 = __fmul_rn(load_state(T.m_scale + min(b + 1, last)), 0.0078125f);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const uint32_t code = flat + j < numel ? (uint32_t)T.m_q[flat + j] : 128u;
@@ -836,7 +836,7 @@ __device__ __forceinline__ void m_old8_any(const af8_factored_tensor &T, int m_f
 __device__ __forceinline__ void load_cols_any(const float *p, int64_t col, int64_t C, float (&x)[8])
 {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) x[j] = col + j < C ? __ldg(p + col + j) : 0.0f;
+    for (int j = 0; j < 8; ++j) x[j] = col + j < C ? load_state(p + col + j) : 0.0f;
 }
 
 // values i .. i + 7 of a 16-byte aligned array, i of any alignment: the two or three aligned vectors around them, shifted
@@ -846,9 +846,9 @@ __device__ __forceinline__ void load_cols8_shifted(const float *v, int64_t i, fl
 {
     const int s = (int)(i & 3);
     const float4 *p = reinterpret_cast<const float4 *>(v + (i - s));
-    const float4 a = __ldg(p), b = __ldg(p + 1);
+    const float4 a = load_state(p), b = load_state(p + 1);
     float4 c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (s) c = __ldg(p + 2);
+    if (s) c = load_state(p + 2);
     float w[11] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z};
 #pragma unroll
     for (int j = 0; j < 9; ++j) w[j] = (s & 2) ? w[j + 2] : w[j];
@@ -1205,11 +1205,11 @@ __device__ __forceinline__ bool slice_rows(const FactoredLaunch &L, const af8_fa
     auto scalars = [&](int q, int k) {
         nir[q] = ns0[q] = ns1[q] = 0.0f;
         if (k < nrows) {
-            if (MODE != SLICE_GRADSQ) nir[q] = __ldg(pr);
+            if (MODE != SLICE_GRADSQ) nir[q] = load_state(pr);
             if (MOM) {
                 const int block = (int)(soff >> 8);                  // (fewer than 2^31 blocks, as rows)
-                ns0[q] = __ldg(sT.m_scale + block);
-                if (!VEC) ns1[q] = __ldg(sT.m_scale + min(block + 1, last_block));
+                ns0[q] = load_state(sT.m_scale + block);
+                if (!VEC) ns1[q] = load_state(sT.m_scale + min(block + 1, last_block));
             }
         }
         pr += 8;
@@ -1345,7 +1345,7 @@ __device__ __forceinline__ void slice_cols(const float *inv_col, int64_t c0, int
     } else {
 #pragma unroll
         for (int j = 0; j < 8; ++j)
-            if (c0 + lane + 32 * j < C) ic[j] = __ldg(inv_col + c0 + lane + 32 * j);
+            if (c0 + lane + 32 * j < C) ic[j] = load_state(inv_col + c0 + lane + 32 * j);
     }
 }
 
@@ -1392,7 +1392,7 @@ __device__ __forceinline__ bool residual_rows_box(const FactoredLaunch &L, const
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
         nir[k] = 0.0f; nsc[k] = 0.0f;
-        if (row0 + k < r_end) { nir[k] = __ldg(sT.inv_row + row0 + k); nsc[k] = __ldg(sT.m_scale + (row0 + k) * scrow + scoff); }
+        if (row0 + k < r_end) { nir[k] = load_state(sT.inv_row + row0 + k); nsc[k] = load_state(sT.m_scale + (row0 + k) * scrow + scoff); }
     }
     for (int g = 0; g < ngroups; ++g) {
         const uint32_t n = cons + (uint32_t)g;
@@ -1422,7 +1422,7 @@ __device__ __forceinline__ bool residual_rows_box(const FactoredLaunch &L, const
                 const float ir = __fmul_rn(nir[k], sgn), mc = __fmul_rn(nsc[k], 0.0078125f);   // fl(scale / 128), scale >= 1e-12
                 {   // this row's successor: the same place of the next pair
                     const int rn = (h == BR / 2 - 1) ? r + 8 * BR - (BR - 2) : r + 2;
-                    if (rn < r_end) { nir[k] = __ldg(sT.inv_row + rn); nsc[k] = __ldg(sT.m_scale + rn * scrow + scoff); }
+                    if (rn < r_end) { nir[k] = load_state(sT.inv_row + rn); nsc[k] = load_state(sT.m_scale + rn * scrow + scoff); }
                 }
                 if (r < r_end) {
                     float gg[8], x[8];
@@ -1782,13 +1782,13 @@ factored_update_vec_kernel(const FactoredLaunch L)
                 if (wrap == 8) { load_cols8_shifted(v, cb0 + col, x); return; }
                 const float *va = v + cb0 + col, *vb = v + cb1 - wrap;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) x[j] = __ldg((j < wrap ? va : vb) + j);
+                for (int j = 0; j < 8; ++j) x[j] = load_state((j < wrap ? va : vb) + j);
             };
             auto row2 = [&](float a, float b, int j) {               // the row factors of elements j, j + 1
                 return ANY == 2 ? make_float2(j < wrap ? a : b, j + 1 < wrap ? a : b) : bc2(a);
             };
             cols8(sT.inv_col, ic);
-            const float ir = __ldg(sT.inv_row + row), irb = ANY == 2 ? __ldg(sT.inv_row + irow1) : 0.0f;
+            const float ir = load_state(sT.inv_row + row), irb = ANY == 2 ? load_state(sT.inv_row + irow1) : 0.0f;
             // pairs of elements in packed binary32 arithmetic (bit-identical to the element-wise form)
             if (L.came) {
                 if (L.mode == AF8_FUPD_SUMSQ_U) {
@@ -1804,7 +1804,7 @@ factored_update_vec_kernel(const FactoredLaunch L)
                         for (int j = 0; j < 8; ++j) mo[j] = j < nval ? sT.m_f32[flat + j] : 0.0f;
                     } else m_old8(sT, L.m_fmt, 256, flat, mo, pre_m, cm);
                     cols8(sT.inv_col_conf, icc);
-                    const float irc = __ldg(sT.inv_row_conf + row), ircb = ANY == 2 ? __ldg(sT.inv_row_conf + irow1) : 0.0f;
+                    const float irc = load_state(sT.inv_row_conf + row), ircb = ANY == 2 ? load_state(sT.inv_row_conf + irow1) : 0.0f;
 #pragma unroll
                     for (int j = 0; j < 8; j += 2) {
                         const float2 ut = div_by2(__fmul2_rn(__fmul2_rn(make_float2(g[j], g[j + 1]), row2(ir, irb, j)), make_float2(ic[j], ic[j + 1])), D);
@@ -2015,8 +2015,8 @@ factored_write_kernel(const FactoredLaunch L)
             int64_t row, col, cb = 0;
             write_position(U, o, row, col);
             if (ANY && U.batch_rows > 0) cb = (int64_t)((uint32_t)row / (uint32_t)U.batch_rows) * U.cols;        // (rows < 2^31)
-            const float2 ir2 = bc2(__fmul_rn(__ldg(U.inv_row + row), sgn));
-            const float4 ic = __ldg(reinterpret_cast<const float4 *>(U.inv_col + cb + col));
+            const float2 ir2 = bc2(__fmul_rn(load_state(U.inv_row + row), sgn));
+            const float4 ic = load_state(reinterpret_cast<const float4 *>(U.inv_col + cb + col));
             float2 ga, gb;
             if (GB == 4) {
                 const float4 g = *reinterpret_cast<const float4 *>(st + o * 4);
@@ -2100,7 +2100,7 @@ template <typename GradT, int PT = 0> constexpr size_t fring_smem_bytes() { retu
 __device__ __forceinline__ void flat_cols_wrap(const float *v, int64_t cb0, int64_t cb1, int64_t col, int left, float (&x)[8])
 {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) x[j] = __ldg(j < left ? v + cb0 + col + j : v + cb1 + j - left);
+    for (int j = 0; j < 8; ++j) x[j] = load_state(j < left ? v + cb0 + col + j : v + cb1 + j - left);
 }
 
 // New momentum and update of 8 elements.  ir, irc: row factors of the elements before `left`, irb, ircb of the others (COMMON: no
@@ -2229,9 +2229,9 @@ factored_apply_flat_kernel(const FactoredLaunch L)
 
         const int64_t w0 = block * 256;                              // (the block exists iff its first element does)
         float sc = nsc;
-        if (!have_sc) sc = w0 < numel ? __ldg(sT.m_scale + block) : 0.0f;
+        if (!have_sc) sc = w0 < numel ? load_state(sT.m_scale + block) : 0.0f;
         have_sc = id + 1 < id_end && w0 + 2048 < numel;
-        if (have_sc) nsc = __ldg(sT.m_scale + block + 8);
+        if (have_sc) nsc = load_state(sT.m_scale + block + 8);
 
         GradRaw8<GradT> cg;
         uint4 pa = make_uint4(0u, 0u, 0u, 0u), pb = pa;              // 8 parameters (bf16: in pa)
@@ -2294,15 +2294,15 @@ factored_apply_flat_kernel(const FactoredLaunch L)
                 else flat_cols_wrap(v, cb0, cb1, col, left, x);
             };
             cols8(sT.inv_col, ic);
-            const float ir = __ldg(sT.inv_row + row);
+            const float ir = load_state(sT.inv_row + row);
             if (L.came) {
                 cols8(sT.inv_col_conf, icc);
-                const float irc = __ldg(sT.inv_row_conf + row);
+                const float irc = load_state(sT.inv_row_conf + row);
                 if (common) flat_update8<true, true>(g, mo, ic, icc, ir, ir, irc, irc, 8, sF.D, sF.LW, mj, u);
-                else flat_update8<true, false>(g, mo, ic, icc, ir, __ldg(sT.inv_row + next), irc, __ldg(sT.inv_row_conf + next), left, sF.D, sF.LW, mj, u);
+                else flat_update8<true, false>(g, mo, ic, icc, ir, load_state(sT.inv_row + next), irc, load_state(sT.inv_row_conf + next), left, sF.D, sF.LW, mj, u);
             } else {
                 if (common) flat_update8<false, true>(g, mo, ic, ic, ir, ir, ir, ir, 8, sF.D, sF.LW, mj, u);
-                else flat_update8<false, false>(g, mo, ic, ic, ir, __ldg(sT.inv_row + next), ir, ir, left, sF.D, sF.LW, mj, u);
+                else flat_update8<false, false>(g, mo, ic, ic, ir, load_state(sT.inv_row + next), ir, ir, left, sF.D, sF.LW, mj, u);
             }
             if (ANY && nval < 8) {
 #pragma unroll
@@ -2458,8 +2458,8 @@ factored_apply_tile_kernel(const FactoredLaunch L)
         const float sgn = (L.came && L.negate_grad) ? -1.0f : 1.0f;
         float n_ir = 0.0f, n_irc = 0.0f, n_sc = 0.0f;
         if (nrows > 0) {
-            n_ir = __ldg(sT.inv_row + row0); n_sc = __ldg(scp);
-            if (L.came) n_irc = __ldg(sT.inv_row_conf + row0);
+            n_ir = load_state(sT.inv_row + row0); n_sc = load_state(scp);
+            if (L.came) n_irc = load_state(sT.inv_row_conf + row0);
         }
         for (int k = 0; k < nrows; ++k) {
             const uint32_t n = cons + (uint32_t)k;
@@ -2486,8 +2486,8 @@ factored_apply_tile_kernel(const FactoredLaunch L)
             const float2 ir2 = bc2(__fmul_rn(n_ir, sgn)), irc2 = bc2(n_irc);
             uf8_decode8(cm, __fmul_rn(n_sc, 0.0078125f), mo);                    // fl(scale / 128), scale >= 1e-12
             if (k + 1 < nrows) {
-                n_ir = __ldg(sT.inv_row + row + 8); n_sc = __ldg(scp + (k + 1) * scstep);
-                if (L.came) n_irc = __ldg(sT.inv_row_conf + row + 8);
+                n_ir = load_state(sT.inv_row + row + 8); n_sc = load_state(scp + (k + 1) * scstep);
+                if (L.came) n_irc = load_state(sT.inv_row_conf + row + 8);
             }
             if (L.came) {
 #pragma unroll
@@ -2557,7 +2557,7 @@ __device__ __forceinline__ double sumsq_span(const FactoredLaunch &L, const af8_
 #pragma unroll
             for (int v = 0; v < NV; ++v) nxt[v].load(sT.grad, e + STEP + 8 * v);
         }
-        const float2 ir2 = bc2(__ldg(sT.inv_row + row));
+        const float2 ir2 = bc2(load_state(sT.inv_row + row));
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
             float g[8], ic[8];
@@ -2742,7 +2742,7 @@ factored_sumsq_tile_kernel(const FactoredLaunch L)
 #pragma unroll
                 for (int k = 0; k < NB; ++k) {
                     const int64_t r = min(r0 + warp + 8 * (int64_t)(k0 + k), R - 1);     // (a row beyond the end carries zeros)
-                    const float2 ir2 = bc2(__ldg(sT.inv_row + r));
+                    const float2 ir2 = bc2(load_state(sT.inv_row + r));
                     float g[8];
                     cur[k].unpack(0, g);                           // (the sign does not matter for the square)
                     float2 a2 = make_float2(0.0f, 0.0f);

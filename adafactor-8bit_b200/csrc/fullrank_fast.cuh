@@ -852,12 +852,12 @@ fullrank_fast_kernel(const FullrankLaunch L)
         ahead = want > 0 ? want - 1 : 0;              // ... as seen from the next block
         // ---- ranges of this block (if not prefetched) and of the next one ----
         if (!staged) {
-            csc = __ldg(sT.v_scale + b);
-            cml = __ldg(sT.v_min_log + b);
+            csc = load_state(sT.v_scale + b);
+            cml = load_state(sT.v_min_log + b);
             if (MF != AF8_M_NONE) {
 #pragma unroll
                 for (int k = 0; k < 2; ++k)           // (momentum blocks beyond the tensor are not allocated)
-                    cms[k] = (2 * warp + k) * FAST_MBLOCK < rem ? __ldg(sT.m_scale + (int64_t)b * MPB + 2 * warp + k) : 0.0f;
+                    cms[k] = (2 * warp + k) * FAST_MBLOCK < rem ? load_state(sT.m_scale + (int64_t)b * MPB + 2 * warp + k) : 0.0f;
             }
             if (TABLE) {
                 s_tab[stage][tid] = al8_decode_fast<STRICT>((uint32_t)tid, csc, cml, s_exp2);   // optimizer.py:341-349
@@ -866,10 +866,10 @@ fullrank_fast_kernel(const FullrankLaunch L)
             __syncthreads();
         }
         if (next_staged) {
-            nsc = __ldg(sT.v_scale + b_next);
-            nml = __ldg(sT.v_min_log + b_next);
+            nsc = load_state(sT.v_scale + b_next);
+            nml = load_state(sT.v_min_log + b_next);
             if (MF != AF8_M_NONE) {
-                const float2 x = make_float2(__ldg(sT.m_scale + (int64_t)b_next * MPB + 2 * warp), __ldg(sT.m_scale + (int64_t)b_next * MPB + 2 * warp + 1));
+                const float2 x = make_float2(load_state(sT.m_scale + (int64_t)b_next * MPB + 2 * warp), load_state(sT.m_scale + (int64_t)b_next * MPB + 2 * warp + 1));
                 nms[0] = x.x; nms[1] = x.y;
             }
         }

@@ -138,7 +138,7 @@ fullrank_generic_kernel(const FullrankLaunch L, const GenericCfg C)
         const int subs_per_block = has_m && m_quant ? C.block / C.m_block : 0;
 
         float v_scale = 1.0f, v_min_log = 0.0f;
-        if (v_quant) { v_scale = __ldg(sT.v_scale + b); v_min_log = __ldg(sT.v_min_log + b); }
+        if (v_quant) { v_scale = load_state(sT.v_scale + b); v_min_log = load_state(sT.v_min_log + b); }
 
         float step_mul = -sT.alpha, fira = 1.0f, pre_div = 1.0f;
         bool zero_upd = false;
@@ -192,7 +192,7 @@ fullrank_generic_kernel(const FullrankLaunch L, const GenericCfg C)
                     float m_old;
                     if (m_quant) {
                         const int64_t sb = (base + i) / C.m_block;
-                        m_old = m_decode(sT.m_q, __ldg(sT.m_scale + sb), base + i, C.m_fmt);
+                        m_old = m_decode(sT.m_q, load_state(sT.m_scale + sb), base + i, C.m_fmt);
                     } else {
                         m_old = sT.m_f32[base + i];
                     }

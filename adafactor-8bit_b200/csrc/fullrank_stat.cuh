@@ -190,13 +190,13 @@ fullrank_stat_kernel(const FullrankLaunch L)
                 const int64_t rem = numel - base;
                 // decode v = 2^((code-1)*scale/levels + min_log) as 2^(code*a + c)
                 const bool requested = RING && ahead;
-                const float sc = requested ? next_sc : __ldg(v_scale + b), ml = requested ? next_ml : __ldg(v_min_log + b);
+                const float sc = requested ? next_sc : load_state(v_scale + b), ml = requested ? next_ml : load_state(v_min_log + b);
                 // (lane s: the momentum scale of step s)
-                [[maybe_unused]] const float ms = requested ? next_ms : RING && rem >= FAST_VBLOCK ? __ldg(m_scale + b * STEPS + (lane & (STEPS - 1))) : 0.0f;
+                [[maybe_unused]] const float ms = requested ? next_ms : RING && rem >= FAST_VBLOCK ? load_state(m_scale + b * STEPS + (lane & (STEPS - 1))) : 0.0f;
                 if (RING) {
                     const int64_t nb = b + warps;
                     ahead = blk + warps < stop && numel - nb * FAST_VBLOCK >= FAST_VBLOCK && small_w;
-                    if (ahead) { next_sc = __ldg(v_scale + nb); next_ml = __ldg(v_min_log + nb); next_ms = __ldg(m_scale + nb * STEPS + (lane & (STEPS - 1))); }
+                    if (ahead) { next_sc = load_state(v_scale + nb); next_ml = load_state(v_min_log + nb); next_ms = load_state(m_scale + nb * STEPS + (lane & (STEPS - 1))); }
                 }
                 [[maybe_unused]] const float a = sc * (VB == 16 ? 1.0f / 65534.0f : 1.0f / 254.0f);
                 [[maybe_unused]] const float c = ml - a;
@@ -254,7 +254,7 @@ fullrank_stat_kernel(const FullrankLaunch L)
                             vw[0] = w.x; vw[1] = w.y; vw[VB / 4 - 2] = w.z; vw[VB / 4 - 1] = w.w;
                         }
                         float2 sum8 = make_float2(0.0f, 0.0f);
-                        const float2 mc2 = bc2(RING ? __shfl_sync(0xffffffffu, ms, s) * M_UNIT : MF == AF8_M_NONE ? 0.0f : __ldg(m_scale + b * STEPS + s) * M_UNIT);
+                        const float2 mc2 = bc2(RING ? __shfl_sync(0xffffffffu, ms, s) * M_UNIT : MF == AF8_M_NONE ? 0.0f : load_state(m_scale + b * STEPS + s) * M_UNIT);
 #pragma unroll
                         for (int j = 0; j < 8; j += 2) {
                             const float2 gj = make_float2(g[j], g[j + 1]);
@@ -301,7 +301,7 @@ fullrank_stat_kernel(const FullrankLaunch L)
                         float mj = gj;
                         if (MF != AF8_M_NONE) {
                             const int k = MF == AF8_M_UF8 ? (int)mq[e] - 128 : (int)((e & 1) ? (mq[e >> 1] & 15u) : (mq[e >> 1] >> 4)) - 8;
-                            mj = lerp_t(__fmul_rn((float)k, __ldg(m_scale + e / FAST_MBLOCK) * M_UNIT), gj, m_w);
+                            mj = lerp_t(__fmul_rn((float)k, load_state(m_scale + e / FAST_MBLOCK) * M_UNIT), gj, m_w);
                         }
                         const float u = root_update2<MF, EXACT ? ROOT_EXACT : ROOT>(make_float2(mj, 0.0f), make_float2(vj, 0.0f), bc2(eps_d)).x;
                         acc = __fmaf_rn(u, u, acc);

@@ -6,8 +6,9 @@
 // kernels of 10 us with 888 CTAs: 14.3 us a kernel with plain launches, 11.8 at best.)  Every CTA calls await_launches() before it
 // touches global memory, so that a kernel is complete only after all before it are, and whatever follows in the stream
 // without the attribute (copies, events, other libraries' kernels) waits for it as always.  No more than two kernels overlap.
-// What a kernel reads first, tables and scalars, it reads with plain loads: the compiler may move a load that it holds for
-// read-only (__ldg) in front of the wait.
+// These kernels read with ordinary loads alone.  A read-only load (__ldg, a const __restrict__ parameter) asks that nobody writes the
+// memory during the reading kernel's lifetime, which begins here while the kernel before may still write it, and the compiler may move
+// it in front of the wait.
 //
 // A table copied by the copy engine between two kernels holds them up for 13 us (6 below 1 KB); read from pinned memory by a kernel, before
 // it waits, 1.5 to 4 us for 1 to 52 KB.  A memset costs 5 us there, a kernel that clears 2.
@@ -21,6 +22,28 @@ __device__ __forceinline__ void await_launches()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// An ordinary load that stores in between need not hold up, as a read-only one: what the kernels load a block or a row ahead, and what
+// no thread writes before it was used.  (As *p the UF8/AL8 update spills 30 to 80 bytes and the sums over ragged rows take 94 us instead of 90;
+// without `volatile` the general kernel's sums take 48 registers instead of 32, 638 -> 774 us for 67 M parameters.)
+__device__ __forceinline__ float load_state(const float *p)
+{
+    float x;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(x) : "l"(p));
+    return x;
+}
+__device__ __forceinline__ float4 load_state(const float4 *p)
+{
+    float4 x;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "l"(p));
+    return x;
+}
+__device__ __forceinline__ uint4 load_state(const uint4 *p)
+{
+    uint4 x;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w) : "l"(p));
+    return x;
 }
 
 template <typename... Params, typename... Args>

@@ -1,0 +1,58 @@
+"""Rules that kernels launched while the kernel before them still runs have to keep, read off the sources: a breach shows on a GPU only
+when the timing is bad."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "adafactor-8bit_b200", "csrc")
+
+
+def sources():
+    out = {}
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith((".cu", ".cuh")):
+            with open(os.path.join(CSRC, name)) as f:
+                out[name] = re.sub(r"//[^\n]*", "", f.read())
+    return out
+
+
+def kernels_after_others():
+    """name -> text of the kernels that launch_next launches (by name, or as `kernel`, a name given a line or two before)."""
+    src = sources()
+    names = set()
+    for text in src.values():
+        for m in re.finditer(r"launch_next\((\w+)", text):
+            names.add(m.group(1))
+        if "launch_next(kernel" in text:
+            names.update(re.findall(r"auto kernel = (\w+)", text))
+    names -= {"kernel", "void"}
+    out = {}
+    for text in src.values():
+        for m in re.finditer(r"^(?:template[^\n]*\n)?__global__.*?^\}", text, re.S | re.M):
+            name = re.search(r"(\w+)\s*\((?!\()(?:const|void|double|FullrankLaunch|ScaleLaunch|\w+ \*)", re.sub(r"__launch_bounds__\([^\n]*", "", m.group(0))).group(1)
+            if name in names:
+                out[name] = m.group(0)
+    return names, out
+
+
+def test_every_kernel_is_found():
+    names, found = kernels_after_others()
+    assert len(names) >= 20 and names == set(found)
+
+
+def test_kernels_wait_before_they_run_on():
+    for name, text in kernels_after_others()[1].items():
+        assert "await_launches()" in text or "write_units<" in text, name
+
+
+# what these kernels call lies in these files or is no memory access
+_CALLED = ("factored.cuh", "fullrank_fast.cuh", "fullrank_generic.cuh", "fullrank_stat.cuh", "fullrank_api.cuh", "launch.cuh", "scale.cuh",
+           "schedule.cuh", "tensormap.cuh", "write_units.cuh", "common.cuh")
+
+
+def test_no_read_only_loads():
+    """The memory may still be written when the kernel starts: no __ldg, no ld.global.nc, no const __restrict__ parameter."""
+    src = sources()
+    for name in _CALLED:
+        assert not re.search(r"__ldg\(|ld\.global\.nc", src[name]), name
+    for name, text in kernels_after_others()[1].items():
+        assert not re.search(r"__ldg\(|ld\.global\.nc|const (?!CUtensorMap)\w+ \*__restrict__", text), name
