@@ -1037,7 +1037,7 @@ extern "C" int af8_apollo_project_batch(const af8_apollo_proj_desc *descs, int32
         // 1466 -> 1328 us).
         std::sort(host_u, host_u + iu, [](const UmmaTask &a, const UmmaTask &b) { return a.t.K > b.t.K; });
         tiles_u = apollo_umma_number(host_u, iu, pair);
-        int rc = upload_table(dev_scratch, host_u, sizeof(UmmaTask) * (size_t)iu, st);
+        int rc = upload_table<true>(dev_scratch, host_u, sizeof(UmmaTask) * (size_t)iu, st);
         if (!rc) rc = pair ? apollo_project_launch_umma<2>(dev_u, iu, tiles_u, st) : apollo_project_launch_umma<1>(dev_u, iu, tiles_u, st);
         if (rc) return rc;
     }

@@ -2962,7 +2962,7 @@ static int af8_factored_stats_impl(const af8_factored_cfg *cfg, const af8_factor
                 rc = factored_box_maps(host_tensors[i], hm + 2 * i);
                 if (rc) return rc;
             }
-            rc = upload_table(dev_maps, host_maps, sizeof(CUtensorMap) * 2 * (size_t)n_tensors, st);
+            rc = upload_table<true>(dev_maps, host_maps, sizeof(CUtensorMap) * 2 * (size_t)n_tensors, st);
             if (rc) return rc;
             maps = static_cast<const CUtensorMap *>(dev_maps);
             ring = 2;

@@ -62,6 +62,9 @@ inline cudaError_t launch_next(void (*kernel)(Params...), dim3 grid, int block, 
     return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
 }
 
+// MAPS: the table holds tensor maps.  They are read through a proxy of their own, which tensormap_acquire on the reading side orders behind
+// a release on this one.
+template <bool MAPS>
 __global__ void __launch_bounds__(256)
 upload_kernel(const uint4 *host, uint4 *dev, int n)
 {
@@ -70,10 +73,12 @@ upload_kernel(const uint4 *host, uint4 *dev, int n)
     if (i < n) asm volatile("ld.global.cv.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(host + i));
     await_launches();                                        // (kernels before this one may still read the table)
     if (i < n) dev[i] = v;
+    if (MAPS) asm volatile("fence.proxy.tensormap::generic.release.sys;" ::: "memory");
 }
 
 // Enqueues the copy of a table.  `host` stays as it is until the copy has run.  Pinned tables of whole 16-byte units that the device can
 // read are copied by a kernel, any other memory by the copy engine.
+template <bool MAPS = false>
 inline int upload_table(void *dev, const void *host, size_t bytes, cudaStream_t st)
 {
     cudaPointerAttributes a;
@@ -81,7 +86,7 @@ inline int upload_table(void *dev, const void *host, size_t bytes, cudaStream_t 
     if ((low & 15) == 0 && bytes < (1u << 20) && cudaPointerGetAttributes(&a, host) == cudaSuccess && a.type == cudaMemoryTypeHost &&
         a.devicePointer != nullptr) {
         const int n = (int)(bytes / 16);
-        AF8_CUDA_TRY(launch_next(upload_kernel, (n + 255) / 256, 256, 0, st, static_cast<const uint4 *>(a.devicePointer), static_cast<uint4 *>(dev), n));
+        AF8_CUDA_TRY(launch_next(upload_kernel<MAPS>, (n + 255) / 256, 256, 0, st, static_cast<const uint4 *>(a.devicePointer), static_cast<uint4 *>(dev), n));
         return AF8_OK;
     }
     cudaGetLastError();

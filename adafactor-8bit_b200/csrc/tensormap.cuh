@@ -26,8 +26,9 @@ inline EncodeTiledFn encode_tiled_fn()
     return fn;
 }
 
-// Orders the uses of a tensor map by the calling thread behind the copy that wrote it: a map that lives in
-// global memory is read through a proxy of its own, which may still hold what was at that address before.
+// Orders the uses of a tensor map by the calling thread behind what wrote it, a copy of the copy engine or an upload_kernel, which ends with
+// the release that belongs to this: a map that lives in global memory is read through a proxy of its own, which may still hold
+// what was at that address before.
 __device__ __forceinline__ void tensormap_acquire(const CUtensorMap *map)
 {
     asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");

@@ -56,3 +56,15 @@ def test_no_read_only_loads():
         assert not re.search(r"__ldg\(|ld\.global\.nc", src[name]), name
     for name, text in kernels_after_others()[1].items():
         assert not re.search(r"__ldg\(|ld\.global\.nc|const (?!CUtensorMap)\w+ \*__restrict__", text), name
+
+
+def test_tables_with_tensor_maps_are_released():
+    """An upload by a kernel whose table holds tensor maps ends with the release that the acquire of their readers belongs to."""
+    src = sources()
+    assert "fence.proxy.tensormap::generic.acquire" in src["tensormap.cuh"]
+    kernel = re.search(r"upload_kernel\(.*?^\}", src["launch.cuh"], re.S | re.M).group(0)
+    assert re.search(r"dev\[i\] = v;\s*if \(MAPS\) asm volatile\(\"fence\.proxy\.tensormap::generic\.release", kernel)
+    calls = [c for text in src.values() for c in re.findall(r"upload_table[^;]*;", text) if "MAPS" not in c]
+    assert len(calls) >= 8
+    maps = [c for c in calls if "CUtensorMap" in c or "UmmaTask" in c]
+    assert len(maps) == 2 and all(c.startswith("upload_table<true>") for c in maps)

@@ -1,4 +1,4 @@
-"""Uploads of launch tables from any host memory, and calls that are captured into a graph."""
+"""Uploads of launch tables from any host memory, tensor maps that are written anew at every step, and calls that are captured into a graph."""
 import ctypes
 
 import numpy as np
@@ -73,3 +73,32 @@ def test_a_captured_step_replays():
                 again(plan, room.data_ptr(), stream)
         out.append(result(params, opt))
     assert all(torch.equal(a, b) for a, b in zip(*out))
+
+
+@pytest.mark.parametrize("name", ["came_al16", "apollo_r32"])
+def test_gradients_that_move(name):
+    """The tensor maps of a step lie where those of the last step lay.  Gradients at another address at every step, the steps queued
+    behind one another, against the same gradients copied to one place, step by step.  Sums by binary64 atomics differ in their order, so
+    that a stored code may tip: a few elements off by 1e-2 of an update, 1e-6 of the norm.  One step with another step's gradients: 1e-3 and more."""
+    from adafactor8bit import Adafactor8Bit
+    shapes = [(512, 1024), (1024, 256), (768, 512)]
+    hp = dict(cases.CASES[name]["hp"], min_8bit_size=1)
+    out = []
+    for moving in (False, True):
+        gen = torch.Generator().manual_seed(11)
+        torch.manual_seed(0)
+        params = [torch.nn.Parameter((torch.randn(s, generator=gen) * 0.02).cuda()) for s in shapes]
+        opt = Adafactor8Bit(params, **hp)
+        grads = [[(torch.randn(s, generator=gen) * 1e-3 * 4.0 ** k).bfloat16().cuda() for s in shapes] for k in range(4)]
+        home = [torch.empty_like(g) for g in grads[0]]
+        for p in params:
+            p.grad_dtype = None
+        for k in range(8):
+            for i, p in enumerate(params):
+                p.grad = grads[k % 4][i] if moving else home[i].copy_(grads[k % 4][i])
+            opt.step()
+            if not moving:
+                torch.cuda.synchronize()
+        out.append([p.detach().clone() for p in params])
+    for a, b in zip(*out):
+        assert float((a - b).norm() / a.norm()) < 1e-4
