@@ -81,15 +81,18 @@ upload_kernel(const uint4 *host, uint4 *dev, int n)
 template <bool MAPS = false>
 inline int upload_table(void *dev, const void *host, size_t bytes, cudaStream_t st)
 {
-    cudaPointerAttributes a;
+    cudaPointerAttributes a = {};
     const uintptr_t low = reinterpret_cast<uintptr_t>(dev) | reinterpret_cast<uintptr_t>(host) | bytes;
-    if ((low & 15) == 0 && bytes < (1u << 20) && cudaPointerGetAttributes(&a, host) == cudaSuccess && a.type == cudaMemoryTypeHost &&
-        a.devicePointer != nullptr) {
+    const bool units = (low & 15) == 0 && bytes < (1u << 20);
+    if (units && cudaPointerGetAttributes(&a, host) != cudaSuccess) {
+        cudaGetLastError();                                  // (the question's own error, not one that is waiting for the caller)
+        a = {};
+    }
+    if (units && a.type == cudaMemoryTypeHost && a.devicePointer != nullptr) {
         const int n = (int)(bytes / 16);
         AF8_CUDA_TRY(launch_next(upload_kernel<MAPS>, (n + 255) / 256, 256, 0, st, static_cast<const uint4 *>(a.devicePointer), static_cast<uint4 *>(dev), n));
         return AF8_OK;
     }
-    cudaGetLastError();
     AF8_CUDA_TRY(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, st));
     return AF8_OK;
 }

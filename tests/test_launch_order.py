@@ -68,3 +68,9 @@ def test_tables_with_tensor_maps_are_released():
     assert len(calls) >= 8
     maps = [c for c in calls if "CUtensorMap" in c or "UmmaTask" in c]
     assert len(maps) == 2 and all(c.startswith("upload_table<true>") for c in maps)
+
+
+def test_an_upload_clears_no_error_but_its_own():
+    body = re.search(r"upload_table\(void \*dev.*?^\}", sources()["launch.cuh"], re.S | re.M).group(0)
+    assert body.count("cudaGetLastError") == 1
+    assert re.search(r"cudaPointerGetAttributes\(&a, host\) != cudaSuccess\) \{\s*cudaGetLastError\(\);", body)
