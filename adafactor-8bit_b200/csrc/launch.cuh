@@ -66,31 +66,32 @@ inline cudaError_t launch_next(void (*kernel)(Params...), dim3 grid, int block, 
 // a release on this one.
 template <bool MAPS>
 __global__ void __launch_bounds__(256)
-upload_kernel(const uint4 *host, uint4 *dev, int n)
+upload_kernel(const uint2 *host, uint2 *dev, int n)         // n units of 8 bytes
 {
-    const int i = blockIdx.x * 256 + threadIdx.x;
+    const int i = 2 * (blockIdx.x * 256 + threadIdx.x);
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (i < n) asm volatile("ld.global.cv.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(host + i));
+    if (i + 1 < n) asm volatile("ld.global.cv.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(host + i));
+    else if (i < n) asm volatile("ld.global.cv.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(host + i));
     await_launches();                                        // (kernels before this one may still read the table)
-    if (i < n) dev[i] = v;
+    if (i + 1 < n) *reinterpret_cast<uint4 *>(dev + i) = v;
+    else if (i < n) dev[i] = make_uint2(v.x, v.y);
     if (MAPS) asm volatile("fence.proxy.tensormap::generic.release.sys;" ::: "memory");
 }
 
-// Enqueues the copy of a table.  `host` stays as it is until the copy has run.  Pinned tables of whole 16-byte units that the device can
-// read are copied by a kernel, any other memory by the copy engine.
+// Enqueues the copy of a table.  `host` stays as it is until the copy has run.  Pinned tables on 16-byte boundaries that the device can
+// read are copied by a kernel, any other memory by the copy engine.  (APOLLO's write-back table has 104 bytes a tensor: whole units of 8.)
 template <bool MAPS = false>
 inline int upload_table(void *dev, const void *host, size_t bytes, cudaStream_t st)
 {
     cudaPointerAttributes a = {};
-    const uintptr_t low = reinterpret_cast<uintptr_t>(dev) | reinterpret_cast<uintptr_t>(host) | bytes;
-    const bool units = (low & 15) == 0 && bytes < (1u << 20);
+    const bool units = ((reinterpret_cast<uintptr_t>(dev) | reinterpret_cast<uintptr_t>(host)) & 15) == 0 && (bytes & 7) == 0 && bytes < (1u << 20);
     if (units && cudaPointerGetAttributes(&a, host) != cudaSuccess) {
         cudaGetLastError();                                  // (the question's own error, not one that is waiting for the caller)
         a = {};
     }
     if (units && a.type == cudaMemoryTypeHost && a.devicePointer != nullptr) {
-        const int n = (int)(bytes / 16);
-        AF8_CUDA_TRY(launch_next(upload_kernel<MAPS>, (n + 255) / 256, 256, 0, st, static_cast<const uint4 *>(a.devicePointer), static_cast<uint4 *>(dev), n));
+        const int n = (int)(bytes / 8);
+        AF8_CUDA_TRY(launch_next(upload_kernel<MAPS>, (n + 511) / 512, 256, 0, st, static_cast<const uint2 *>(a.devicePointer), static_cast<uint2 *>(dev), n));
         return AF8_OK;
     }
     AF8_CUDA_TRY(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, st));

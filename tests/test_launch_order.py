@@ -63,7 +63,7 @@ def test_tables_with_tensor_maps_are_released():
     src = sources()
     assert "fence.proxy.tensormap::generic.acquire" in src["tensormap.cuh"]
     kernel = re.search(r"upload_kernel\(.*?^\}", src["launch.cuh"], re.S | re.M).group(0)
-    assert re.search(r"dev\[i\] = v;\s*if \(MAPS\) asm volatile\(\"fence\.proxy\.tensormap::generic\.release", kernel)
+    assert re.search(r"dev\[i\] = [^;]*;\s*if \(MAPS\) asm volatile\(\"fence\.proxy\.tensormap::generic\.release", kernel)
     calls = [c for text in src.values() for c in re.findall(r"upload_table[^;]*;", text) if "MAPS" not in c]
     assert len(calls) >= 8
     maps = [c for c in calls if "CUtensorMap" in c or "UmmaTask" in c]

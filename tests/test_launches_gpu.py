@@ -52,6 +52,27 @@ def test_a_table_comes_from_any_host_memory():
         assert all(torch.equal(a, b) for a, b in zip(out[0], other))
 
 
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5])
+def test_no_table_of_an_apollo_step_takes_the_copy_engine(n):
+    """The write-back table has 104 bytes a tensor: odd numbers of tensors end in half a 16-byte unit."""
+    from adafactor8bit import Adafactor8Bit
+    gen = torch.Generator().manual_seed(n)
+    params = [torch.nn.Parameter((torch.randn(256, 128 + 64 * i, generator=gen) * 0.02).cuda()) for i in range(n)]
+    opt = Adafactor8Bit(params, **dict(cases.CASES["apollo_r32"]["hp"], apollo_update_proj_gap=100))
+    for p in params:
+        p.grad_dtype = None
+        p.grad = (torch.randn(p.shape, generator=gen) * 1e-3).bfloat16().cuda()
+    before = [p.detach().clone() for p in params]
+    opt.step()
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        opt.step()
+        torch.cuda.synchronize()
+    names = [e.name for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+    assert any("apollo_write_kernel" in k for k in names) and not any("Memcpy HtoD" in k for k in names)
+    assert all(bool((p != b).any(1).all()) for p, b in zip(params, before))
+
+
 def test_a_captured_step_replays():
     """Two steps captured into a graph, upload included, are the two steps launched one by one."""
     out = []
