@@ -353,15 +353,27 @@ def test_apply_batch_equals_per_tensor_calls(param_dtype, grad_dtype, aligned):
     left-case tensors, channel- and tensor-wise scaling, every decay mode, a bf16 compute copy, a tensor that
     ends inside a 2048-element chunk; with one tensor whose columns are no multiple of 8 the table takes the
     per-tensor route."""
+    shapes = [(512, 256), (64, 1032), (264, 136), (96, 2048), (40, 72)]
+    if not aligned:
+        shapes[2] = (250, 36)
+    _apply_batch(shapes, param_dtype, grad_dtype)
+
+
+@pytest.mark.parametrize("param_dtype,grad_dtype", [("f32", "bf16"), ("f32", "f32"), ("bf16", "bf16"), ("bf16", "f32"), ("f16", "bf16")])
+def test_apply_batch_of_many_chunks(param_dtype, grad_dtype):
+    """Over 4000 chunks, four to seven for each resident CTA: CTAs take chunk after chunk, within a tensor and across tensors of a few
+    elements, and use every stage of their rings again."""
+    _apply_batch([(40, 72), (1500, 2048), (64, 1032), (8, 8), (264, 136)] + [(9, 16)] * 10 + [(2056, 2000), (96, 8), (1, 8), (300, 4104)],
+                 param_dtype, grad_dtype)
+
+
+def _apply_batch(shapes, param_dtype, grad_dtype):
     import ctypes
     from adafactor8bit import _native as N
     lib = N.lib()
     dev = torch.device("cuda:0")
     gen = torch.Generator(device="cpu").manual_seed(77)
-    shapes = [(512, 256), (64, 1032), (264, 136), (96, 2048), (40, 72)]
-    if not aligned:
-        shapes[2] = (250, 36)
-    pdt = dict(f32=torch.float32, bf16=torch.bfloat16)[param_dtype]
+    pdt = dict(f32=torch.float32, bf16=torch.bfloat16, f16=torch.float16)[param_dtype]
     gdt = dict(f32=torch.float32, bf16=torch.bfloat16)[grad_dtype]
     n = len(shapes)
     p0 = [torch.randn(s, generator=gen).to(pdt).to(dev) for s in shapes]
@@ -376,14 +388,14 @@ def test_apply_batch_equals_per_tensor_calls(param_dtype, grad_dtype, aligned):
     sins = []
     for i in range(n):
         sin = N.ApolloScalarsIn()
-        sin.scale_tensor, sin.fira, sin.scale_front, sin.sqrt_scale = int(i == 3), int(i % 2 == 0), int(i == 1), 1.25
+        sin.scale_tensor, sin.fira, sin.scale_front, sin.sqrt_scale = int(i % 5 == 3), int(i % 2 == 0), int(i % 5 == 1), 1.25
         sins.append(sin)
-    decay = [0.999, 0.0, 0.98, 0.0, 0.97]
-    has_decay = [1, 0, 2, 0, 1]
-    sr = [int(param_dtype != "f32" and i == 4) for i in range(n)]
-    copies = [torch.zeros(s, dtype=torch.bfloat16, device=dev) if (param_dtype == "f32" and i in (0, 3)) else None
+    decay = [(0.999, 0.0, 0.98, 0.0, 0.97)[i % 5] for i in range(n)]
+    has_decay = [(1, 0, 2, 0, 1)[i % 5] for i in range(n)]
+    sr = [int(param_dtype != "f32" and i % 5 == 4) for i in range(n)]
+    copies = [torch.zeros(s, dtype=torch.bfloat16, device=dev) if (param_dtype == "f32" and i % 5 in (0, 3)) else None
               for i, s in enumerate(shapes)]
-    PD, GD = dict(f32=N.F32, bf16=N.BF16)[param_dtype], dict(f32=N.F32, bf16=N.BF16)[grad_dtype]
+    PD, GD = dict(f32=N.F32, bf16=N.BF16, f16=N.F16)[param_dtype], dict(f32=N.F32, bf16=N.BF16)[grad_dtype]
     s = torch.cuda.current_stream(dev).cuda_stream
 
     want_p = [p.clone() for p in p0]
@@ -410,9 +422,9 @@ def test_apply_batch_equals_per_tensor_calls(param_dtype, grad_dtype, aligned):
     N.check(lib.af8_apollo_apply_batch(host.data_ptr(), devt.data_ptr(), n, first, PD, GD, 1, s), "af8_apollo_apply_batch")
     torch.cuda.synchronize(dev)
     for i in range(n):
-        assert not torch.equal(want_p[i], p0[i])
-        assert torch.equal(got_p[i].view(torch.int16 if pdt == torch.bfloat16 else torch.int32),
-                           want_p[i].view(torch.int16 if pdt == torch.bfloat16 else torch.int32)), shapes[i]
+        assert want_p[i].numel() < 1000 or not torch.equal(want_p[i], p0[i])      # (a few 16-bit values may all round to themselves)
+        bits = torch.int32 if pdt == torch.float32 else torch.int16
+        assert torch.equal(got_p[i].view(bits), want_p[i].view(bits)), shapes[i]
         if want_c[i] is not None:
             assert torch.equal(got_c[i].view(torch.int16), want_c[i].view(torch.int16)), shapes[i]
     # a table whose chunk numbering is wrong is refused before anything is launched

@@ -128,7 +128,8 @@ EXTRA_CASES.update({
 })
 
 # the write pass without a momentum in units of 2048 elements: tensors that end a unit, just after it or far inside, units with no, one or
-# many row ends, the shortest rows, rows longer than a unit, more tensors than a CTA has stages, matrices of a batch that end in a unit
+# many row ends, the shortest rows, rows longer than a unit, matrices of a batch that end in a unit (a CTA has one unit here at most;
+# test_write_pass_of_many_units gives it several)
 _WRITE = [(1, 8), (2, 1024), (1, 2056), (257, 8), (3, 2048), (5, 4104), (100, 24), (1000, 40), (1, 8), (300, 2040), (2, 8)]
 EXTRA_CASES.update({
     "adafactor_write": dict(shapes=_WRITE, steps=2, seed=81, grad=cases.CASES["adafactor_factored"]["grad"], hp=cases.CASES["adafactor_factored"]["hp"]),
@@ -221,6 +222,48 @@ def test_a_matrix_beside_batches_is_the_same(oracle):
         out.append([(p.detach().cpu(), float(opt.state[p]["fira_prev_norm"])) for p in params[:len(flats)]])
     apart = [(s, na, nb) for s, (a, na), (b, nb) in zip(flats, *out) if na != nb or not torch.equal(a, b)]
     assert not apart, f"{len(apart)} of {len(flats)} matrices differ: {apart[:3]}"
+
+
+_UNITS = [(1, 8), (1500, 2048), (257, 8), (1, 2056)] + [(2, 24)] * 12 + [(700, 4104), (8, 8), (1000, 1000), (40, 40000)]
+
+
+@pytest.mark.parametrize("param,grad,sr", [(torch.float32, torch.bfloat16, False), (torch.float32, torch.float32, False),
+                                           (torch.bfloat16, torch.bfloat16, False), (torch.bfloat16, torch.bfloat16, True)])
+@pytest.mark.parametrize("shapes", [_UNITS, [(600, 9, 8), (5, 900, 1032), (3, 1, 2048), (7, 33, 64), (2, 300, 2056), (2, 1000, 1000)]], ids=["matrices", "batches"])
+def test_write_pass_of_many_units(param, grad, sr, shapes):
+    """About 4000 units, four to seven for each resident CTA of the write pass without a momentum: units within a
+    tensor and across tensors of a few elements, every stage of the ring used again.  From the same factors the general kernel writes the
+    same bits."""
+    from adafactor8bit import Adafactor8Bit, _engine, _native as N
+    hp = dict(cases.CASES["adafactor_factored"]["hp"], min_8bit_size=1, weight_decay=0.01, stochastic_round_writeback=sr)
+    gen = torch.Generator().manual_seed(91)
+    params = [torch.nn.Parameter((torch.randn(s, generator=gen) * 0.02).to(param).cuda()) for s in shapes]
+    for p in params:
+        p.grad_dtype = None
+        p.grad = (torch.randn(p.shape, generator=gen) * 1e-3).to(grad).cuda()
+    opt = Adafactor8Bit(params, **hp)
+    opt.step()
+    plan = max((x for x in opt._plans.values() if isinstance(x, _engine.FactoredPlan)), key=lambda x: x.total_chunks)
+    params, update, seen = plan.params, plan._update, []
+
+    def both(mode, *args):
+        if mode != N.FUPD_APPLY:
+            return update(mode, *args)
+        assert plan.cfg.aligned8 and plan.total_chunks > 3500 and len(params) > 4
+        before, route = [p.detach().clone() for p in params], plan.cfg.aligned8
+        for plan.cfg.aligned8 in (0, route):
+            for p, b in zip(params, before):
+                p.detach().copy_(b)
+            update(mode, *args)
+            seen.append([p.detach().clone() for p in params])
+        assert not any(torch.equal(a, b) for a, b in zip(seen[0], before) if a.numel() >= 1000)
+
+    plan._update = both
+    opt.step()
+    torch.cuda.synchronize()
+    bits = torch.int32 if param == torch.float32 else torch.int16
+    for a, b in zip(*seen):
+        assert torch.equal(a.view(bits), b.view(bits)), (a.shape, int((a != b).sum()))
 
 
 _ROWS8, _RAGGED = [(39, 264), (520, 776), (1030, 520)], [(700, 257), (131, 273), (39, 264), (1030, 513), (67, 1001)]
