@@ -647,7 +647,7 @@ factored_update_kernel(const FactoredLaunch L, int chunk)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 #ifndef AF8_FUPD_PREFETCH_AHEAD
-#define AF8_FUPD_PREFETCH_AHEAD 3      /* chunks ahead that the momentum-free write pass requests from L2; 0: off */
+#define AF8_FUPD_PREFETCH_AHEAD 3      /* chunks ahead that the write passes named below request from L2; 0: off */
 #endif
 template <typename GradT> __host__ __device__ constexpr int sizeof_grad() { return std::is_same<GradT, float>::value ? 4 : 2; }
 
@@ -856,7 +856,7 @@ __device__ __forceinline__ void load_cols8_shifted(const float *v, int64_t i, fl
     for (int j = 0; j < 8; ++j) x[j] = (s & 1) ? w[j + 1] : w[j];
 }
 
-// The residual pass of stats_rows for rows of any length with a momentum that has no slices (not UF8 in blocks of 256, weights of
+// The residual pass of residual_rows for rows of any length with a momentum that has no slices (not UF8 in blocks of 256, weights of
 // 1/2 and more): elements beyond the row's end count as zeros, all loads through GradAny8.
 template <typename GradT, int NB>
 __device__ __forceinline__ void stats_rows_any(const FactoredLaunch &L, const af8_factored_tensor &sT, int64_t r0, int64_t r_end, int64_t c,
@@ -982,15 +982,16 @@ __device__ __forceinline__ void gradsq_rows(const af8_factored_tensor &sT, int64
     __syncwarp();
 }
 
-// Rows r0 + warp + 8k of the tile, NB at a time so that NB independent 128-bit loads per lane
-// are in flight.  Column partials go to a per-warp shared array (no shared-memory atomics).
-template <typename GradT, int NB, bool PREFETCH, bool RESIDUAL>
-__device__ __forceinline__ void stats_rows(const FactoredLaunch &L, const af8_factored_tensor &sT, int64_t r0, int64_t r_end, int64_t c,
-                                           bool col_ok, float pre_div, const float (&ic)[8], double (&cacc)[8])
+// The residual pass over whole vectors of 8 without a ring (a momentum that is not UF8 in blocks of 256, a clip divisor below 1, momentum
+// weights of 1/2 and more in tables with batches or rows of any length): rows r0 + warp + 8 k of the tile, two at a time, the loads of the next
+// two issued before these are used.
+template <typename GradT>
+__device__ __forceinline__ void residual_rows(const FactoredLaunch &L, const af8_factored_tensor &sT, int64_t r0, int64_t r_end, int64_t c,
+                                              bool col_ok, float pre_div, const float (&ic)[8], double (&cacc)[8])
 {
+    constexpr int NB = 2;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t R = r_end, C = sT.cols;            // r_end: end of the unit's rows
-    // PREFETCH: the loads of the next NB rows are issued before the current ones are processed
     GradRaw8<GradT> cur[NB], nxt[NB];
     auto fetch = [&](GradRaw8<GradT> (&dst)[NB], int k0) {
 #pragma unroll
@@ -1000,30 +1001,22 @@ __device__ __forceinline__ void stats_rows(const FactoredLaunch &L, const af8_fa
             else dst[k].zero();
         }
     };
-    if (PREFETCH) fetch(cur, 0);
+    fetch(cur, 0);
     for (int k0 = 0; r0 + warp + 8 * k0 < R; k0 += NB) {          // (uniform over the warp)
-        if (PREFETCH) fetch(nxt, k0 + NB);
-        else fetch(cur, k0);
+        fetch(nxt, k0 + NB);
         float g[NB][8];
         double rsum[NB];
 #pragma unroll
         for (int k = 0; k < NB; ++k) {
             cur[k].unpack(L.negate_grad, g[k]);
-            if (PREFETCH) cur[k] = nxt[k];
+            cur[k] = nxt[k];
         }
 #pragma unroll
         for (int k = 0; k < NB; ++k) {
             const int64_t r = r0 + warp + 8 * (k0 + k);
             const bool live = col_ok && r < R;
             float x[8];
-            if (!RESIDUAL) {
-#pragma unroll
-                for (int j = 0; j < 8; j += 2) {
-                    const float2 gj = make_float2(g[k][j], g[k][j + 1]);
-                    const float2 xx = __fmul2_rn(gj, gj);
-                    x[j] = xx.x; x[j + 1] = xx.y;
-                }
-            } else if (live) {
+            if (live) {
                 const int64_t flat = r * C + c;
                 const float2 ir2 = bc2(sT.inv_row[r]);
                 const DivBy D = make_div(pre_div);
@@ -1052,34 +1045,14 @@ __device__ __forceinline__ void stats_rows(const FactoredLaunch &L, const af8_fa
             }
             rsum[k] = racc;
         }
-        // The NB row sums of the warp are reduced together: each exchange halves the number of
-        // values a lane carries, so NB rows cost NB - 1 + (5 - log2 NB) shuffles instead of 5 NB.
-        // The sum of row k0 + i ends up in lane 32 i / NB.
-        static_assert(NB == 2 || NB == 4, "row-sum reduction is written for 2 or 4 rows");
-        double v;
-        if (NB == 4) {
-            const bool hi = lane & 16;
-            const double r0x = __shfl_xor_sync(0xffffffffu, hi ? rsum[0] : rsum[2], 16);
-            const double r1x = __shfl_xor_sync(0xffffffffu, hi ? rsum[1] : rsum[NB - 1], 16);
-            const double k0v = (hi ? rsum[2] : rsum[0]) + r0x;
-            const double k1v = (hi ? rsum[NB - 1] : rsum[1]) + r1x;
-            const bool h2 = lane & 8;
-            v = (h2 ? k1v : k0v) + __shfl_xor_sync(0xffffffffu, h2 ? k0v : k1v, 8);
+        // the two row sums of the warp are reduced together: the first exchange leaves one value a lane; row k0 + i ends in lane 16 i
+        const bool hi = lane & 16;
+        double v = (hi ? rsum[1] : rsum[0]) + __shfl_xor_sync(0xffffffffu, hi ? rsum[0] : rsum[1], 16);
 #pragma unroll
-            for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if ((lane & 7) == 0) {
-                const int64_t r = r0 + warp + 8 * (k0 + (lane >> 3));
-                if (r < R) atomicAdd(sT.row_sum + r, v);
-            }
-        } else {
-            const bool hi = lane & 16;
-            v = (hi ? rsum[1] : rsum[0]) + __shfl_xor_sync(0xffffffffu, hi ? rsum[0] : rsum[1], 16);
-#pragma unroll
-            for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if ((lane & 15) == 0) {
-                const int64_t r = r0 + warp + 8 * (k0 + (lane >> 4));
-                if (r < R) atomicAdd(sT.row_sum + r, v);
-            }
+        for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if ((lane & 15) == 0) {
+            const int64_t r = r0 + warp + 8 * (k0 + (lane >> 4));
+            if (r < R) atomicAdd(sT.row_sum + r, v);
         }
     }
 }
@@ -1459,12 +1432,6 @@ __device__ __forceinline__ bool residual_rows_box(const FactoredLaunch &L, const
 #ifndef AF8_FSTAT_MIN_CTAS
 #define AF8_FSTAT_MIN_CTAS 3
 #endif
-#ifndef AF8_FSTAT_RES_NB
-#define AF8_FSTAT_RES_NB 2
-#endif
-#ifndef AF8_FSTAT_RES_PREFETCH
-#define AF8_FSTAT_RES_PREFETCH true
-#endif
 #ifndef AF8_FSTAT_MIN_CTAS_RES
 #define AF8_FSTAT_MIN_CTAS_RES 3
 #endif
@@ -1566,7 +1533,7 @@ factored_stats_vec_kernel(const FactoredLaunch L, const CUtensorMap *__restrict_
         } else if (!vec) {
             if constexpr (ANY && RESIDUAL) stats_rows_any<GradT, 4>(L, sT, r0, row_end, c, pre_div, ic, cacc);
         } else if (!RESIDUAL) gradsq_rows<GradT, sizeof_grad<GradT>() == 2 ? 4 : 2>(sT, r0, row_end, c, col_ok, cacc, s_col[warp]);
-        else stats_rows<GradT, AF8_FSTAT_RES_NB, AF8_FSTAT_RES_PREFETCH, true>(L, sT, r0, row_end, c, col_ok, pre_div, ic, cacc);
+        else residual_rows<GradT>(L, sT, r0, row_end, c, col_ok, pre_div, ic, cacc);
         if (!ok) {
             atomicExch(&g_device_error, DEVERR_SRING_TIMEOUT);
             return;                      // (the whole warp; the others finish their rows and leave at the next barrier)
@@ -1728,10 +1695,11 @@ factored_update_vec_kernel(const FactoredLaunch L)
         } else cg.zero();
 #if AF8_FUPD_PREFETCH_AHEAD > 0
         if (writes && (!has_m || ANY == 2)) {
-            // The momentum-free write pass asks L2 for the chunk a few iterations ahead (same tensor), one
-            // request per 128-byte line.  The passes with momentum and the sum passes were measured slower with it (CAME apply
-            // 24.9 -> 25.6 ms, sums 0.87 -> 0.94 ms), so they go without; rows of any length, whose loads wait longer, gain with one
-            // too (252 -> 238 us, 59 M parameters).
+            // What is left of the momentum-free write passes beside factored_write_kernel (with the previous step's norm, 16-bit
+            // parameters element by element, rows of any length) asks L2 for the chunk a few iterations ahead (same tensor), one request
+            // per 128-byte line.  Passes with momentum and the sum passes were measured slower with it (CAME apply 24.9 -> 25.6 ms, sums
+            // 0.87 -> 0.94 ms), so they go without; rows of any length, whose loads wait longer, gain with one too (252 -> 238 us,
+            // 59 M parameters).
             const int64_t pf = flat + (int64_t)AF8_FUPD_PREFETCH_AHEAD * 2048;
             if (id + AF8_FUPD_PREFETCH_AHEAD < id_end && pf < numel) {
                 constexpr int GB = sizeof_grad<GradT>();
