@@ -77,6 +77,8 @@ __device__ __forceinline__ void write_units(const Tensors &tensors, WriteShared<
             if (n >= NS && !mbar_wait_bounded(&sh.free[sl], (n / NS + 1) & 1u)) { sh.abort = 1; atomicExch(&g_device_error, DEVERR_WRITE_TIMEOUT); }
             if (id < 0 || *static_cast<volatile int *>(&sh.abort)) {
                 unit_drain(sh.queue);
+                if (id >= 0)                                         // given up: the copies in flight get a bounded chance to land before the CTA may end
+                    for (uint32_t k = n > NS ? n - NS : 0; k < n; ++k) mbar_wait_bounded(&sh.full[k % NS], (k / NS) & 1u);
                 sh.unit[sl].count = 0;
                 asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&sh.full[sl])) : "memory");
                 return;

@@ -87,8 +87,15 @@ AF8_API int32_t af8_struct_size(int32_t index);
 /* Device-side health: waits inside the kernels (on asynchronous copies) are
  * bounded; a wait that ran out sets a sticky flag on the device instead of
  * hanging.  This call synchronises `stream` and returns the flag of the current
- * device in *status_out: 0 = healthy, 1 = an asynchronous copy never completed
- * (results of that launch are invalid).  No counterpart in the reference. */
+ * device in *status_out: 0 = healthy, else the wait that ran out last (results of
+ * that launch are invalid):
+ *   1  full-rank update: a copy of a block's inputs
+ *   2  APOLLO's projection on the tensor cores: a copy, an MMA or another warp
+ *   3  factored write pass with a momentum: a copy of its ring
+ *   4  sums of the factored passes: a copy of their rings
+ *   5  write pass without a momentum, APOLLO's write-back: the answer to a request for a unit
+ *   6  the same passes: a copy of their ring, or a stage that was not given back
+ * No counterpart in the reference. */
 AF8_API int af8_device_status(int32_t *status_out, void *stream);
 /* Reset that flag to 0 (synchronises `stream`).  No counterpart in the reference. */
 AF8_API int af8_device_status_clear(void *stream);

@@ -74,3 +74,11 @@ def test_an_upload_clears_no_error_but_its_own():
     body = re.search(r"upload_table\(void \*dev.*?^\}", sources()["launch.cuh"], re.S | re.M).group(0)
     assert body.count("cudaGetLastError") == 1
     assert re.search(r"cudaPointerGetAttributes\(&a, host\) != cudaSuccess\) \{\s*cudaGetLastError\(\);", body)
+
+
+def test_a_write_pass_that_gives_up_waits_for_its_copies():
+    """What the warp that copies has requested may still write shared memory: bounded waits for the stages come before the last arrival,
+    on which the other warps leave."""
+    text = sources()["write_units.cuh"]
+    leave = re.search(r"if \(id < 0 \|\| \*static_cast<volatile int \*>\(&sh\.abort\)\) \{.*?return;", text, re.S).group(0)
+    assert re.search(r"mbar_wait_bounded\(&sh\.full\[k % NS\], \(k / NS\) & 1u\);.*mbarrier\.arrive", leave, re.S)
