@@ -354,7 +354,7 @@ __device__ __forceinline__ int find_finish_tensor(const af8_apollo_finish_tensor
 // sums of a channel are then added over the warps in a fixed order.
 // What a unit (16 KB at rank 256) waits for decides: a run needs one search of the table and one sum over the CTA with one atomic per
 // tensor, where each unit had them; rows come in 128-bit loads, lines whole where a column unit read 32 bytes of each, and the square
-// roots and divisions of a step are made by as many threads as it has channels: 61 M projected elements 187 -> 110 us.
+// roots and divisions of a step are made by as many threads as it has channels: 61 M projected elements 184 -> 108 us.
 constexpr int SCALES_UNITS = 4;
 __global__ void __launch_bounds__(256, 8)
 apollo_scales_multi_kernel(const af8_apollo_finish_tensor *T, int n, int64_t total_units)
@@ -631,8 +631,8 @@ apollo_apply_vec_kernel(void *__restrict__ param_v, const void *__restrict__ gra
 
 // All tensors of a table in one launch, in units of 2048 elements (write_units.cuh); every tensor has cols % 8 == 0 and arrays on 16-byte
 // boundaries, fewer than 2^34 elements.  The arithmetic of apollo_apply_group.
-// CTAs that walked the table with the grid's stride took 1450 us for four Llama-3-8B layers (872 M parameters, 10 bytes each; 6.0 TB/s),
-// this takes 1340.
+// CTAs that walked the table with the grid's stride took 1445 us for four Llama-3-8B layers (872 M parameters, 10 bytes each; 6.0 TB/s),
+// this takes 1255 (6.9 TB/s).
 struct ApolloUnit : WriteUnit {
     void *copy;
     const float *sf;
@@ -1033,8 +1033,8 @@ extern "C" int af8_apollo_project_batch(const af8_apollo_proj_desc *descs, int32
     }
     if (iu) {
         // The persistent CTAs deal the tiles out in turn and a tile costs its K: long ones first, so that the last round
-        // is one of short ones (four Llama-3-8B layers: 1600 tiles of K = 4096 and 256 of K = 1024 over 148 CTAs:
-        // 1466 -> 1328 us).
+        // is one of short ones (four Llama-3-8B layers: 1600 tiles of K = 4096 and 256 of K = 1024 over 148 CTAs,
+        // each SM a tile of its own: 1466 -> 1328 us; as measured later, before pairs, 1308).
         std::sort(host_u, host_u + iu, [](const UmmaTask &a, const UmmaTask &b) { return a.t.K > b.t.K; });
         tiles_u = apollo_umma_number(host_u, iu, pair);
         int rc = upload_table<true>(dev_scratch, host_u, sizeof(UmmaTask) * (size_t)iu, st);

@@ -152,7 +152,7 @@ NCU_TRAFFIC_BPP = {
     ("fullrank_fast_apply", "bf16"): (13.72, "profiles/fullrank_fast_apply_tinyllama_4layers.txt"),
     ("fullrank_stat", "bf16"): (4.12, "profiles/fullrank_stat_tinyllama_4layers.txt"),
     # the factored write pass: without momentum (Adafactor, 10 B/param) and with a UF8 momentum (CAME, 12 B/param)
-    ("factored_apply", "bf16", 10): (9.68, "profiles/factored_update_nomomentum_tinyllama_4layers.txt"),
+    ("factored_apply", "bf16", 10): (9.68, "profiles/factored_write_tinyllama_4layers.txt"),
     ("factored_apply", "bf16", 12): (11.82, "profiles/factored_kernels_llama2_layer_came.txt"),
 }
 
