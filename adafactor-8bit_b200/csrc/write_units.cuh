@@ -75,9 +75,10 @@ __device__ __forceinline__ void write_units(const Tensors &tensors, WriteShared<
         for (uint32_t n = 0;; ++n) {
             const int sl = (int)(n % NS);
             if (n >= NS && !mbar_wait_bounded(&sh.free[sl], (n / NS + 1) & 1u)) { sh.abort = 1; atomicExch(&g_device_error, DEVERR_WRITE_TIMEOUT); }
-            if (id < 0 || *static_cast<volatile int *>(&sh.abort)) {
+            const bool given_up = *static_cast<volatile int *>(&sh.abort) != 0;
+            if (id < 0 || given_up) {
                 unit_drain(sh.queue);
-                if (id >= 0)                                         // given up: the copies in flight get a bounded chance to land before the CTA may end
+                if (given_up)                                        // the copies in flight get a bounded chance to land before the CTA may end
                     for (uint32_t k = n > NS ? n - NS : 0; k < n; ++k) mbar_wait_bounded(&sh.full[k % NS], (k / NS) & 1u);
                 sh.unit[sl].count = 0;
                 asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&sh.full[sl])) : "memory");

@@ -80,5 +80,5 @@ def test_a_write_pass_that_gives_up_waits_for_its_copies():
     """What the warp that copies has requested may still write shared memory: bounded waits for the stages come before the last arrival,
     on which the other warps leave."""
     text = sources()["write_units.cuh"]
-    leave = re.search(r"if \(id < 0 \|\| \*static_cast<volatile int \*>\(&sh\.abort\)\) \{.*?return;", text, re.S).group(0)
-    assert re.search(r"mbar_wait_bounded\(&sh\.full\[k % NS\], \(k / NS\) & 1u\);.*mbarrier\.arrive", leave, re.S)
+    leave = re.search(r"if \(id < 0 \|\| given_up\) \{.*?return;", text, re.S).group(0)
+    assert re.search(r"if \(given_up\)\s*for [^;]*;[^;]*;[^;]*mbar_wait_bounded\(&sh\.full\[k % NS\], \(k / NS\) & 1u\);.*mbarrier\.arrive", leave, re.S)
